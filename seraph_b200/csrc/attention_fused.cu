@@ -1,4 +1,4 @@
-// attention_fused.cu - causal attention forward in one kernel (head size 128, FP16 hi/lo parts, FP32-level accuracy).
+// attention_fused.cu - causal attention forward in one kernel (head sizes 64 and 128, FP16 hi/lo parts, FP32-level accuracy).
 //
 // One CTA owns 128 consecutive queries of one (sequence, query head) and walks over that sequence's keys in
 // blocks of 64, up to the diagonal.  Nothing of size S x S ever reaches memory:
@@ -16,32 +16,42 @@
 // Warps: 0 TMA producer, 1 MMA issuer (owns the tensor-memory allocation), 4-7 softmax, 8-15 O accumulation
 // (two warps per lane quarter, 64 columns each).  Shared memory: Q parts 64 KB, K and V parts 2 x 32 KB each
 // (double buffered), P parts 32 KB.  Tensor memory: 2 x (64 + 64) columns for S, 2 x 128 for P V.
+// 64-wide heads run the same kernel with half of everything but the score block (one accumulator of twelve instructions per S).  What
+// bounds them is the softmax warps and, on short sequences, the launch: evaluation of 64 samples of up to 256 tokens on the 33M model went
+// from 7.2 to 0.65 ms of attention per call when they left the launch-per-product path.
 // Every mbarrier wait is bounded; a wait that runs out sets the status word and the CTA drains and frees its
 // tensor memory.
 #include "attention_fused.cuh"
 
+template <int HD>
 __global__ void __launch_bounds__(AF_THREADS, 1)
 at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant__ CUtensorMap mQ2,
                     const __grid_constant__ CUtensorMap mK1, const __grid_constant__ CUtensorMap mK2,
                     const __grid_constant__ CUtensorMap mV1, const __grid_constant__ CUtensorMap mV2,
-                    const __grid_constant__ AfSeqs seqs, float* __restrict__ O, float* __restrict__ lse,
+                    const AfSeqTab seqs, float* __restrict__ O, float* __restrict__ lse,
                     const float* __restrict__ amax_q, const float* __restrict__ amax_k, const float* __restrict__ amax_v,
                     int Hq, int g, int nqb_max, float scale, int* status, unsigned* amax_o) {
+    constexpr int NH = HD / 64;                              // 64-column halves of the head dimension (one 128-byte row of halfs each)
+    constexpr int Q_BYTES = NH * 32768, KV_STAGE = NH * 16384, Q_PART = NH * 16384, KV_PART = NH * 8192;
+    constexpr int OFF_K = Q_BYTES, OFF_V = OFF_K + 2 * KV_STAGE, OFF_P = OFF_V + 2 * KV_STAGE, OFF_BAR = OFF_P + 32768;
+    constexpr int COL_PV = 2 * NH * AF_BKV;                  // tensor memory: two S buffers of NH x 64 columns, then two P V buffers of HD
+    constexpr int TMEM_COLS = COL_PV + 2 * HD;               // 512 or 256
+    constexpr int OC = HD / 2;                               // columns of O per accumulation thread
     // which (query block, sequence, head): blocks with the most keys first, the query heads of one K/V head side by side
     const int per_i = seqs.n * Hq;
     const int qb = nqb_max - 1 - (int)blockIdx.x / per_i;
     const int rem = (int)blockIdx.x % per_i;
     const int b = rem / Hq, h = rem % Hq;
-    const int t0 = seqs.start[b], S = seqs.start[b + 1] - t0;
+    const int t0 = (int)seqs.start[b], S = (int)seqs.start[b + 1] - t0;
     if (qb * AF_BQ >= S) return;
     if (*(volatile int*)status != 0) return;                 // an earlier CTA gave up: do not queue behind its cause
     const int nkv = min((S + AF_BKV - 1) / AF_BKV, 2 * qb + 2);
     const int kvh = h / g;
-    const int qd = Hq * AF_HD;
+    const int qd = Hq * HD;
 
     extern __shared__ uint8_t af_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)af_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* bars = (uint64_t*)(smem + AF_OFF_BAR);
+    uint64_t* bars = (uint64_t*)(smem + OFF_BAR);
     uint64_t* q_full = bars;            // 1
     uint64_t* k_full = bars + 1;        // 2
     uint64_t* k_empty = bars + 3;       // 2
@@ -56,7 +66,7 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
     uint64_t* a_full = bars + 19;       // 2
     uint64_t* fin_full = bars + 21;     // 1
     uint32_t* tmem_slot = (uint32_t*)(bars + 24);
-    float* alpha_s = (float*)(smem + AF_OFF_BAR + 256);          // [2][128]
+    float* alpha_s = (float*)(smem + OFF_BAR + 256);          // [2][128]
     float* fin_s = alpha_s + 256;                                 // [128]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -71,7 +81,7 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     tc_fence_before();
@@ -83,10 +93,10 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (elect_one()) {
-            mbar_expect_tx(q_full, AF_Q_BYTES);
-            for (int p = 0; p < 2; p++) {
-                af_tma_2d(smem + p * 16384, &mQ1, q_full, h * AF_HD + p * 64, t0 + qb * AF_BQ);
-                af_tma_2d(smem + 32768 + p * 16384, &mQ2, q_full, h * AF_HD + p * 64, t0 + qb * AF_BQ);
+            mbar_expect_tx(q_full, Q_BYTES);
+            for (int p = 0; p < NH; p++) {
+                af_tma_2d(smem + p * 16384, &mQ1, q_full, h * HD + p * 64, t0 + qb * AF_BQ);
+                af_tma_2d(smem + Q_PART + p * 16384, &mQ2, q_full, h * HD + p * 64, t0 + qb * AF_BQ);
             }
             // order of need: K_0, K_1, V_0, K_2, V_1, ...
             for (int jj = -1; jj < nkv && ok; jj++) {
@@ -95,22 +105,22 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
                     const int s = jk & 1, u = jk >> 1;
                     ok = mbar_wait(&k_empty[s], (u & 1) ^ 1);
                     if (!ok) break;
-                    uint8_t* dst = smem + AF_OFF_K + s * AF_KV_STAGE;
-                    mbar_expect_tx(&k_full[s], AF_KV_STAGE);
-                    for (int p = 0; p < 2; p++) {
-                        af_tma_2d(dst + p * 8192, &mK1, &k_full[s], kvh * AF_HD + p * 64, t0 + jk * AF_BKV);
-                        af_tma_2d(dst + 16384 + p * 8192, &mK2, &k_full[s], kvh * AF_HD + p * 64, t0 + jk * AF_BKV);
+                    uint8_t* dst = smem + OFF_K + s * KV_STAGE;
+                    mbar_expect_tx(&k_full[s], KV_STAGE);
+                    for (int p = 0; p < NH; p++) {
+                        af_tma_2d(dst + p * 8192, &mK1, &k_full[s], kvh * HD + p * 64, t0 + jk * AF_BKV);
+                        af_tma_2d(dst + KV_PART + p * 8192, &mK2, &k_full[s], kvh * HD + p * 64, t0 + jk * AF_BKV);
                     }
                 }
                 if (jj >= 0) {
                     const int s = jj & 1, u = jj >> 1;
                     ok = mbar_wait(&v_empty[s], (u & 1) ^ 1);
                     if (!ok) break;
-                    uint8_t* dst = smem + AF_OFF_V + s * AF_KV_STAGE;
-                    mbar_expect_tx(&v_full[s], AF_KV_STAGE);
-                    for (int p = 0; p < 2; p++) {
-                        af_tma_2d(dst + p * 8192, &mV1, &v_full[s], kvh * AF_HD + p * 64, t0 + jj * AF_BKV);
-                        af_tma_2d(dst + 16384 + p * 8192, &mV2, &v_full[s], kvh * AF_HD + p * 64, t0 + jj * AF_BKV);
+                    uint8_t* dst = smem + OFF_V + s * KV_STAGE;
+                    mbar_expect_tx(&v_full[s], KV_STAGE);
+                    for (int p = 0; p < NH; p++) {
+                        af_tma_2d(dst + p * 8192, &mV1, &v_full[s], kvh * HD + p * 64, t0 + jj * AF_BKV);
+                        af_tma_2d(dst + KV_PART + p * 8192, &mV2, &v_full[s], kvh * HD + p * 64, t0 + jj * AF_BKV);
                     }
                 }
             }
@@ -120,7 +130,7 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
         // ---------------- MMA issuer ----------------
         if (elect_one()) {
             const uint32_t idesc_s = (1u << 4) | ((uint32_t)(AF_BKV >> 3) << 17) | ((uint32_t)(AF_BQ >> 4) << 24);
-            const uint32_t idesc_o = (1u << 4) | (1u << 16) | ((uint32_t)(AF_HD >> 3) << 17) | ((uint32_t)(AF_BQ >> 4) << 24);
+            const uint32_t idesc_o = (1u << 4) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(AF_BQ >> 4) << 24);
             const uint32_t sq = smem_u32(smem);
             ok = mbar_wait(q_full, 0);
             for (int jj = -1; jj < nkv && ok; jj++) {
@@ -131,12 +141,12 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
                     ok = mbar_wait(&k_full[s], u & 1) && mbar_wait(&s_empty[s], (u & 1) ^ 1);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t sk = smem_u32(smem + AF_OFF_K + s * AF_KV_STAGE);
+                    const uint32_t sk = smem_u32(smem + OFF_K + s * KV_STAGE);
 #pragma unroll
-                    for (int p = 0; p < 2; p++) {
-                        const uint64_t a1 = make_kmajor_desc<128>(sq + p * 16384), a2 = make_kmajor_desc<128>(sq + 32768 + p * 16384);
-                        const uint64_t b1 = make_kmajor_desc<128>(sk + p * 8192), b2 = make_kmajor_desc<128>(sk + 16384 + p * 8192);
-                        const uint32_t d = tmem_base + (uint32_t)(s * 128 + p * 64);
+                    for (int p = 0; p < NH; p++) {
+                        const uint64_t a1 = make_kmajor_desc<128>(sq + p * 16384), a2 = make_kmajor_desc<128>(sq + Q_PART + p * 16384);
+                        const uint64_t b1 = make_kmajor_desc<128>(sk + p * 8192), b2 = make_kmajor_desc<128>(sk + KV_PART + p * 8192);
+                        const uint32_t d = tmem_base + (uint32_t)(s * (NH * AF_BKV) + p * AF_BKV);
 #pragma unroll
                         for (int kk = 0; kk < 4; kk++) {
                             const uint64_t adv = (uint64_t)(kk * 2);
@@ -154,10 +164,10 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
                     ok = mbar_wait(p_full, jj & 1) && mbar_wait(&v_full[s], u & 1) && mbar_wait(&pv_empty[s], (u & 1) ^ 1);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t sp = smem_u32(smem + AF_OFF_P), sv = smem_u32(smem + AF_OFF_V + s * AF_KV_STAGE);
+                    const uint32_t sp = smem_u32(smem + OFF_P), sv = smem_u32(smem + OFF_V + s * KV_STAGE);
                     const uint64_t a1 = make_kmajor_desc<128>(sp), a2 = make_kmajor_desc<128>(sp + 16384);
-                    const uint64_t b1 = make_mn16_desc<AF_BKV>(sv), b2 = make_mn16_desc<AF_BKV>(sv + 16384);
-                    const uint32_t d = tmem_base + (uint32_t)(256 + s * 128);
+                    const uint64_t b1 = make_mn16_desc<AF_BKV>(sv), b2 = make_mn16_desc<AF_BKV>(sv + KV_PART);
+                    const uint32_t d = tmem_base + (uint32_t)(COL_PV + s * HD);
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++) {
                         const uint64_t adva = (uint64_t)(kk * 2), advb = (uint64_t)(kk * 128);
@@ -178,7 +188,7 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
         const int qi = qb * AF_BQ + r;                        // position of this row inside the sequence
         const float cs = tc_pow2(-tc_f16_shift(__ldg(amax_q))) * tc_pow2(-tc_f16_shift(__ldg(amax_k))) * (scale * 1.4426950408889634f);
         float m = -INFINITY, l = 0.f;
-        uint8_t* prow = smem + AF_OFF_P + r * 128;
+        uint8_t* prow = smem + OFF_P + r * 128;
         for (int j = 0; j < nkv && ok; j++) {
             const int s = j & 1, u = j >> 1;
             ok = mbar_wait(&s_full[s], u & 1);
@@ -186,15 +196,16 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
             tc_fence_after();
             float y[64];                                        // raw scores (the two accumulators added)
             {
-                const uint32_t ta = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(s * 128);
+                const uint32_t ta = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(s * (NH * AF_BKV));
                 uint32_t a[32], c[32];
 #pragma unroll
                 for (int hh = 0; hh < 2; hh++) {
                     af_ld32_issue(ta + hh * 32, a);
-                    af_ld32_issue(ta + 64 + hh * 32, c);
-                    af_ld_wait(a); af_ld_dep(c);
+                    if constexpr (NH == 2) af_ld32_issue(ta + 64 + hh * 32, c);
+                    af_ld_wait(a);
+                    if constexpr (NH == 2) af_ld_dep(c);
 #pragma unroll
-                    for (int i = 0; i < 32; i++) y[hh * 32 + i] = __uint_as_float(a[i]) + __uint_as_float(c[i]);
+                    for (int i = 0; i < 32; i++) y[hh * 32 + i] = NH == 2 ? __uint_as_float(a[i]) + __uint_as_float(c[i]) : __uint_as_float(a[i]);
                 }
             }
             tc_fence_before();
@@ -211,10 +222,13 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
             const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * cs;      // cs > 0
             const float m_new = fmaxf(m, mx);                 // finite from block 0 on: key 0 counts for every row
             const float alpha = af_ex2(m - m_new);
-            const float off = 14.f - m_new;                   // P leaves as P * 2^14
+            // P leaves as P * 2^14.  128-wide heads: the 14 rides on the exponent, which costs nothing and rounds an exponent of up to 14;
+            // 64-wide heads have the issue slots for an exact multiplication instead
+            constexpr bool EXACT = HD == 64;
+            const float off = EXACT ? -m_new : 14.f - m_new;
             float sm4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int i = 0; i < 64; i++) { y[i] = af_ex2(fmaf(y[i], cs, off)); sm4[i & 3] += y[i]; }
+            for (int i = 0; i < 64; i++) { y[i] = af_ex2(fmaf(y[i], cs, off)); if (EXACT) y[i] *= 16384.f; sm4[i & 3] += y[i]; }
             l = l * alpha + ((sm4[0] + sm4[1]) + (sm4[2] + sm4[3]));          // in units of 2^-14
             m = m_new;
             // alpha to the O warps (the slot was last read for block j - 2)
@@ -243,32 +257,36 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
         }
         if (ok) {
             fin_s[r] = l > 0.f ? 1.0f / l : 0.f;
-            if (lse && qi < S) lse[(size_t)(t0 + qi) * Hq + h] = (m + log2f(l) - 14.f) * 0.6931471805599453f;
+            if (lse && qi < S) lse[(size_t)(t0 + qi) * Hq + h] = fmaf(m, 0.6931471805599453f, logf(l * (1.0f / 16384.f)));
         }
         __syncwarp();
         if (lane == 0) af_arrive(fin_full);
         if (!ok && lane == 0) atomicExch(status, SB_ERR_TIMEOUT);
     } else if (warp >= 8) {
-        // ---------------- O accumulation: one row and 64 columns per thread ----------------
+        // ---------------- O accumulation: one row and half of the columns per thread ----------------
         const int q = warp & 3, r = q * 32 + lane, ch = (warp - 8) >> 2;
         const int qi = qb * AF_BQ + r;
-        float o[64];
+        float o[OC];
 #pragma unroll
-        for (int i = 0; i < 64; i++) o[i] = 0.f;
+        for (int i = 0; i < OC; i++) o[i] = 0.f;
         for (int j = 0; j < nkv && ok; j++) {
             const int s = j & 1, u = j >> 1;
             ok = mbar_wait(&a_full[s], u & 1) && mbar_wait(&pv_full[s], u & 1);
             if (!ok) break;
             tc_fence_after();
             const float alpha = alpha_s[s * 128 + r];
-            const uint32_t ta = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(256 + s * 128 + ch * 64);
+            const uint32_t ta = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(COL_PV + s * HD + ch * OC);
             {
                 uint32_t t[32], t2[32];
                 af_ld32_issue(ta, t);
-                af_ld32_issue(ta + 32, t2);
-                af_ld_wait(t); af_ld_dep(t2);
+                if constexpr (OC == 64) af_ld32_issue(ta + 32, t2);
+                af_ld_wait(t);
+                if constexpr (OC == 64) af_ld_dep(t2);
 #pragma unroll
-                for (int i = 0; i < 32; i++) { o[i] = fmaf(o[i], alpha, __uint_as_float(t[i])); o[32 + i] = fmaf(o[32 + i], alpha, __uint_as_float(t2[i])); }
+                for (int i = 0; i < 32; i++) {
+                    o[i] = fmaf(o[i], alpha, __uint_as_float(t[i]));
+                    if constexpr (OC == 64) o[32 + i] = fmaf(o[32 + i], alpha, __uint_as_float(t2[i]));
+                }
             }
             tc_fence_before();
             __syncwarp();
@@ -278,9 +296,9 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
         float am = 0.f;
         if (ok && qi < S) {
             const float f = fin_s[r] * tc_pow2(-tc_f16_shift(__ldg(amax_v)));      // fin = 1 / l with l in units of 2^-14, O holds (P * 2^14) V' products
-            float4* dst = (float4*)(O + (size_t)(t0 + qi) * qd + (size_t)h * AF_HD + ch * 64);
+            float4* dst = (float4*)(O + (size_t)(t0 + qi) * qd + (size_t)h * HD + ch * OC);
 #pragma unroll
-            for (int i = 0; i < 16; i++) {
+            for (int i = 0; i < OC / 4; i++) {
                 const float4 v = make_float4(o[4 * i] * f, o[4 * i + 1] * f, o[4 * i + 2] * f, o[4 * i + 3] * f);
                 dst[i] = v;
                 am = sb_amax4(am, v);
@@ -296,7 +314,7 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
     }
 }
 
@@ -524,37 +542,43 @@ at_score_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
     }
 }
 
-// q1/q2, k1/k2, v1/v2: the FP16 parts of Q [T, Hq*128], K and V [T, Hkv*128]; amax_*: the device words their scales derive from.
+template <int HD>
+static int af_launch_fwd(sb_ctx_t* c, const void* q1, const void* q2, const void* k1, const void* k2, const void* v1, const void* v2,
+                         const float* amax_q, const float* amax_k, const float* amax_v, float* O, float* lse, int T, int Hq, int Hkv) {
+    constexpr int smem = HD / 64 * (32768 + 4 * 16384) + 32768 + 2048 + 1024;
+    auto kern = at_fused_fwd_kernel<HD>;
+    static bool attr_done = false;
+    if (!attr_done) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) { cudaGetLastError(); return 1; }
+        attr_done = true;
+    }
+    int Smax = 0;
+    for (int b = 0; b < c->h_seq_n; b++) Smax = max(Smax, c->h_seq[b + 1] - c->h_seq[b]);
+    if (Smax <= 0) return 1;
+    const AfSeqTab seqs = {c->h_seq_n, c->attn_seq_starts};
+    const int nqb = (Smax + AF_BQ - 1) / AF_BQ;
+    const int qd = Hq * HD, kvd = Hkv * HD;
+    CUtensorMap mQ1, mQ2, mK1, mK2, mV1, mV2;
+    if (!af_make_map(c, &mQ1, q1, T, qd, AF_BQ) || !af_make_map(c, &mQ2, q2, T, qd, AF_BQ) ||
+        !af_make_map(c, &mK1, k1, T, kvd, AF_BKV) || !af_make_map(c, &mK2, k2, T, kvd, AF_BKV) ||
+        !af_make_map(c, &mV1, v1, T, kvd, AF_BKV) || !af_make_map(c, &mV2, v2, T, kvd, AF_BKV)) return 1;
+    const long blocks = (long)nqb * seqs.n * Hq;
+    if (blocks > 0x7fffffffL) return 1;
+    kern<<<(unsigned)blocks, AF_THREADS, smem, (cudaStream_t)c->pub.stream>>>(
+        mQ1, mQ2, mK1, mK2, mV1, mV2, seqs, O, lse, amax_q, amax_k, amax_v, Hq, Hq / Hkv, nqb, 1.0f / sqrtf((float)HD), c->d_status,
+        sb_amax_take(c, O, (size_t)T * qd));
+    c->launches++;
+    return cudaGetLastError() == cudaSuccess ? 0 : 1;
+}
+// q1/q2, k1/k2, v1/v2: the FP16 parts of Q [T, Hq*hd], K and V [T, Hkv*hd]; amax_*: the device words their scales derive from.
 // Returns 0 when the kernel was launched, 1 when this path does not take the call.
 extern "C" int sb_attention_fused_forward(sb_ctx_t* c, const void* q1, const void* q2, const void* k1, const void* k2,
                                           const void* v1, const void* v2, const float* amax_q, const float* amax_k, const float* amax_v,
                                           float* O, float* lse, int T, int Hq, int Hkv, int hd) {
-    if (hd != AF_HD || c->h_seq_n <= 0 || c->h_seq_n > AF_MAXSEQ || Hq % Hkv) return 1;
-    if (!tc_aligned16(O) || !tc_load_encode()) return 1;
-    static bool attr_done = false;
-    if (!attr_done) {
-        if (cudaFuncSetAttribute(at_fused_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AF_SMEM) != cudaSuccess) { cudaGetLastError(); return 1; }
-        attr_done = true;
-    }
-    AfSeqs seqs;
-    seqs.n = c->h_seq_n;
-    int Smax = 0;
-    for (int b = 0; b <= c->h_seq_n; b++) seqs.start[b] = c->h_seq[b];
-    for (int b = 0; b < c->h_seq_n; b++) Smax = max(Smax, c->h_seq[b + 1] - c->h_seq[b]);
-    if (Smax <= 0) return 1;
-    const int nqb = (Smax + AF_BQ - 1) / AF_BQ;
-    const int qd = Hq * hd, kvd = Hkv * hd;
-    CUtensorMap mQ1, mQ2, mK1, mK2, mV1, mV2;
-    if (!af_make_map(&mQ1, q1, T, qd, AF_BQ) || !af_make_map(&mQ2, q2, T, qd, AF_BQ) ||
-        !af_make_map(&mK1, k1, T, kvd, AF_BKV) || !af_make_map(&mK2, k2, T, kvd, AF_BKV) ||
-        !af_make_map(&mV1, v1, T, kvd, AF_BKV) || !af_make_map(&mV2, v2, T, kvd, AF_BKV)) return 1;
-    const long blocks = (long)nqb * seqs.n * Hq;
-    if (blocks > 0x7fffffffL) return 1;
-    at_fused_fwd_kernel<<<(unsigned)blocks, AF_THREADS, AF_SMEM, (cudaStream_t)c->pub.stream>>>(
-        mQ1, mQ2, mK1, mK2, mV1, mV2, seqs, O, lse, amax_q, amax_k, amax_v, Hq, Hq / Hkv, nqb, 1.0f / sqrtf((float)hd), c->d_status,
-        sb_amax_take(c, O, (size_t)T * qd));
-    c->launches++;
-    return cudaGetLastError() == cudaSuccess ? 0 : 1;
+    if (c->h_seq_n <= 0 || !c->attn_seq_starts || Hq % Hkv || !tc_aligned16(O) || !tc_load_encode()) return 1;
+    if (hd == 128) return af_launch_fwd<128>(c, q1, q2, k1, k2, v1, v2, amax_q, amax_k, amax_v, O, lse, T, Hq, Hkv);
+    if (hd == 64) return af_launch_fwd<64>(c, q1, q2, k1, k2, v1, v2, amax_q, amax_k, amax_v, O, lse, T, Hq, Hkv);
+    return 1;
 }
 
 // The backward score kernel.  nb > 0: one sequence [t0, t0 + S) and the heads head0, head0 + head_step, ... (nb of them), the
@@ -584,10 +608,10 @@ extern "C" int sb_attention_fused_scores(sb_ctx_t* c, const void* q1, const void
     }
     const int qd = Hq * hd, kvd = Hkv * hd, nqb = (Smax + AF_BQ - 1) / AF_BQ;
     CUtensorMap mQ1, mQ2, mD1, mD2, mK1, mK2, mV1, mV2;
-    if (!af_make_map(&mQ1, q1, T, qd, AF_BQ) || !af_make_map(&mQ2, q2, T, qd, AF_BQ) ||
-        !af_make_map(&mD1, do1, T, qd, AF_BQ) || !af_make_map(&mD2, do2, T, qd, AF_BQ) ||
-        !af_make_map(&mK1, k1, T, kvd, AF_BKV) || !af_make_map(&mK2, k2, T, kvd, AF_BKV) ||
-        !af_make_map(&mV1, v1, T, kvd, AF_BKV) || !af_make_map(&mV2, v2, T, kvd, AF_BKV)) return 1;
+    if (!af_make_map(c, &mQ1, q1, T, qd, AF_BQ) || !af_make_map(c, &mQ2, q2, T, qd, AF_BQ) ||
+        !af_make_map(c, &mD1, do1, T, qd, AF_BQ) || !af_make_map(c, &mD2, do2, T, qd, AF_BQ) ||
+        !af_make_map(c, &mK1, k1, T, kvd, AF_BKV) || !af_make_map(c, &mK2, k2, T, kvd, AF_BKV) ||
+        !af_make_map(c, &mV1, v1, T, kvd, AF_BKV) || !af_make_map(c, &mV2, v2, T, kvd, AF_BKV)) return 1;
     const long blocks = (long)nqb * seqs.n * (nb > 0 ? nb : Hq);
     if (blocks > 0x7fffffffL) return 1;
     at_score_bwd_kernel<<<(unsigned)blocks, AS_THREADS, AS_SMEM, (cudaStream_t)c->pub.stream>>>(

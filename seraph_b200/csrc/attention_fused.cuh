@@ -12,13 +12,20 @@
 
 struct AfSeqs { int n; int start[AF_MAXSEQ + 1]; };
 
+struct AfSeqTab { int n; const uint32_t* start; };      // sequence boundaries in device memory, n + 1 of them
+
+// First row of (sequence b, head h) in the backward's per-head scratch (rows of dS^T are keys; of LT and DT the row's one value).
+// pitch > 0: every slot has `pitch` rows.  pitch == 0: slots have the sequence's own length rounded up to 128, so that short sequences
+// packed beside a long one cost what they need; 128 (t0 / 128 + b) is at least the sum of the rounded lengths before sequence b.
+__host__ __device__ __forceinline__ int af_slot_row(int pitch, int Hq, int b, int h, int t0, int S) {
+    return pitch > 0 ? (b * Hq + h) * pitch : Hq * (((t0 >> 7) + b) << 7) + h * ((S + 127) & ~127);
+}
+static inline size_t af_slot_rows(int pitch, int Hq, int n, int T) {
+    return pitch > 0 ? (size_t)n * Hq * pitch : (size_t)Hq * ((((size_t)T >> 7) + n + 1) << 7);
+}
+
 #define AF_Q_BYTES 65536
 #define AF_KV_STAGE 32768
-#define AF_OFF_K AF_Q_BYTES
-#define AF_OFF_V (AF_OFF_K + 2 * AF_KV_STAGE)
-#define AF_OFF_P (AF_OFF_V + 2 * AF_KV_STAGE)
-#define AF_OFF_BAR (AF_OFF_P + 32768)
-#define AF_SMEM (AF_OFF_BAR + 2048 + 1024)
 
 __device__ __forceinline__ void af_tma_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -93,12 +100,22 @@ __device__ __forceinline__ void af_quad_transpose(uint4 (&w)[4], int lane) {
 
 
 // 2-D FP16 tensor map over a token-major array [T, cols]: boxes of 64 columns x box_rows tokens, 128-byte swizzle
-static inline bool af_make_map(CUtensorMap* m, const void* base, int T, int cols, int box_rows) {
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)T};
-    cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-    cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    return g_tc_encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+static inline bool af_make_map(sb_ctx_t* c, CUtensorMap* m, const void* base, int T, int cols, int box_rows) {
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)T}, strides[1] = {(cuuint64_t)cols * 2};
+    const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
+    return tc_encode(c, m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+// The backward with dK and dV kept on chip.  q, do, k, v: the FP16 parts of Q, dO [T, Hq*hd] and K, V [T, Hkv*hd]; amax_*: the device words
+// their scales derive from; ds_bound: the device word that bounds |dS|.  dS1/dS2: the parts of dS^T, laid out
+// [slot of (sequence, head): af_slot_row][Sp] (key rows, query columns).  LT, DT: the log-sum-exp and D, one value per row of the
+// slots (row = query), in the form at_bwd_prep2_kernel writes.  accumulate: dK and dV are added into, else written.  dQ given: dQ = dS K follows in a second launch
+// (Sp a multiple of 128, slots of the sequences' own lengths); NULL: the caller forms it (Sp a multiple of 256, slots of Sp rows).
+struct AbCall {
+    const void *q1, *q2, *do1, *do2, *k1, *k2, *v1, *v2;
+    const float *amax_q, *amax_k, *amax_v, *amax_do, *ds_bound, *LT, *DT;
+    void *dS1, *dS2;
+    float *dK, *dV, *dQ;
+    int accumulate, Sp, T, Hq, Hkv;
+};
+int sb_attention_fused_dkv(sb_ctx_t* c, const AbCall& p, int hd);

@@ -25,7 +25,7 @@
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
-#include "gemm_tc.cuh"
+#include "attention_fused.cuh"
 
 #define AT_ROWTILE 256                            // rows of a CTA pair's tile: P and dS are zeroed up to this boundary past the diagonal
 #define AT_ALL_SCORES_BYTES ((size_t)0)           // > 0: the backward scores of all sequences and heads in one launch when their parts fit this many bytes
@@ -195,36 +195,86 @@ __global__ void at_delta_kernel(const float* __restrict__ dO, const float* __res
     if (lane == 0) D[w] = s;
 }
 
-// The same D for 128-wide heads, together with what the FP16 split of dO and the bound of dS need from the same rows:
-// the largest |dO| (amax) and the largest row norm of dO (norm_max), both raised with integer atomicMax on the float
-// bits (order-free; zeroed before).  One warp per four (t,h) rows, a float4 per lane and row.
-__global__ void __launch_bounds__(256) at_bwd_prep128_kernel(const float* __restrict__ dO, const float* __restrict__ O, float* __restrict__ D,
-                                                             int n_th, unsigned* __restrict__ norm_max, unsigned* __restrict__ amax) {
-    const int lane = threadIdx.x & 31, nwarps = (gridDim.x * blockDim.x) >> 5;
+// D for 64- and 128-wide heads, together with what the FP16 split of dO and the bound of dS need from the same rows: the largest |dO|
+// (amax) and the largest row norms of dO (norm_do; blockIdx.y == 0) and of V (norm_v; blockIdx.y == 1), all raised with integer atomicMax
+// on the float bits (order-free; zeroed before).  HD/4 lanes per (t,h) row, four passes of rows in flight.
+template <int HD>
+__global__ void __launch_bounds__(256) at_bwd_prep_kernel(const float* __restrict__ dO, const float* __restrict__ O, float* __restrict__ D, int n_do,
+                                                          const float* __restrict__ V, int n_v,
+                                                          unsigned* __restrict__ norm_do, unsigned* __restrict__ amax, unsigned* __restrict__ norm_v) {
+    constexpr int LPR = HD / 4, RPW = 32 / LPR;
+    const int lane = threadIdx.x & 31, sub = lane / LPR, l = lane % LPR, nwarps = (gridDim.x * blockDim.x) >> 5;
+    const bool is_v = blockIdx.y != 0;
+    const int n = is_v ? n_v : n_do;
     float bn = 0.f, ba = 0.f;
-    for (int r0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4; r0 < n_th; r0 += nwarps * 4) {
+    for (int r0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (4 * RPW); r0 < n; r0 += nwarps * (4 * RPW)) {
         float d[4], n2[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             d[i] = 0.f; n2[i] = 0.f;
-            if (r0 + i < n_th) {
-                const float4 g = __ldg((const float4*)(dO + (size_t)(r0 + i) * 128) + lane);
-                const float4 o = __ldg((const float4*)(O + (size_t)(r0 + i) * 128) + lane);
-                d[i] = g.x * o.x + g.y * o.y + g.z * o.z + g.w * o.w;
+            const int r = r0 + i * RPW + sub;
+            if (r < n) {
+                const float4 g = __ldg((const float4*)((is_v ? V : dO) + (size_t)r * HD) + l);
                 n2[i] = g.x * g.x + g.y * g.y + g.z * g.z + g.w * g.w;
-                ba = sb_amax4(ba, g);
+                if (!is_v) {
+                    const float4 o = __ldcs((const float4*)(O + (size_t)r * HD) + l);      // dO is read again by the next kernel, O is not
+                    d[i] = g.x * o.x + g.y * o.y + g.z * o.z + g.w * o.w;
+                    ba = sb_amax4(ba, g);
+                }
             }
         }
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const float ds = warp_sum_f(d[i]);
-            bn = fmaxf(bn, warp_sum_f(n2[i]));
-            if (lane == 0 && r0 + i < n_th) D[r0 + i] = ds;
+            const int r = r0 + i * RPW + sub;
+            for (int o = LPR / 2; o > 0; o >>= 1) { d[i] += __shfl_xor_sync(0xffffffffu, d[i], o); n2[i] += __shfl_xor_sync(0xffffffffu, n2[i], o); }
+            bn = fmaxf(bn, n2[i]);
+            if (!is_v && l == 0 && r < n) D[r] = d[i];
         }
     }
-    sb_block_amax(sqrtf(bn), norm_max);
+    sb_block_amax(sqrtf(bn), is_v ? norm_v : norm_do);
     __syncthreads();
-    sb_block_amax(ba, amax);
+    if (!is_v) sb_block_amax(ba, amax);
+}
+// Second step, once those maxima are known.  blockIdx.y == 0: the FP16 parts of dO; also the constants (consts[0] = 1, consts[1] = the
+// bound of dS as in at_consts_kernel).  blockIdx.y == 1: lse and D, [token][head], moved to the rows of the (sequence, head) slots (zeros up
+// to a multiple of 32 queries) in the form the backward's elementwise warps use: 14 - lse log2(e) for 128-wide heads (the
+// probabilities are formed times 2^14, by the exponent), -lse for 64-wide ones (those have the issue slots to multiply by log2(e) and 2^14
+// after the subtraction, which keeps the rounding of the large terms out of the exponent), and D times the factor that takes
+// P 2^14 (dP - D) to the scaled dS.
+__global__ void __launch_bounds__(256) at_bwd_prep2_kernel(const float4* __restrict__ dO, size_t n4, uint2* __restrict__ h1, uint2* __restrict__ h2,
+                                                           const float* __restrict__ amax, float* consts, const float* __restrict__ norms, float scale,
+                                                           const float* __restrict__ lse, const float* __restrict__ D, float* __restrict__ LT, float* __restrict__ DT,
+                                                           const AfSeqTab seqs, int Hq, int Smax, int slot_pitch, int natural) {
+    const float bound = 2.0f * __ldg(norms) * __ldg(norms + 1) * scale;
+    if (blockIdx.y == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) { consts[0] = 1.0f; consts[1] = bound; }
+        const float sc = tc_pow2(tc_f16_shift(__ldg(amax)));
+        const size_t nth = (size_t)gridDim.x * blockDim.x;
+        for (size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n4; i0 += 2 * nth) {
+            float4 v[2];
+#pragma unroll
+            for (int u = 0; u < 2; u++) if (i0 + u * nth < n4) v[u] = __ldg(dO + (n4 - 1 - i0 - u * nth));      // backwards: the end is still in L2
+#pragma unroll
+            for (int u = 0; u < 2; u++) if (i0 + u * nth < n4) {
+                uint2 a, b;
+                sb_split2(v[u].x * sc, v[u].y * sc, a.x, b.x); sb_split2(v[u].z * sc, v[u].w * sc, a.y, b.y);
+                h1[n4 - 1 - i0 - u * nth] = a; h2[n4 - 1 - i0 - u * nth] = b;
+            }
+        }
+        return;
+    }
+    const float dsc = tc_pow2(tc_f16_shift(bound)) * scale * (1.0f / 16384.f);
+    const int qblocks = (Smax + 31) >> 5, lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    const long items = (long)seqs.n * qblocks * Hq;
+    for (long w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < items; w += nw) {
+        const int h = (int)(w % Hq), bq = (int)(w / Hq), b = bq / qblocks, q = (bq % qblocks) * 32 + lane;
+        const int t0 = (int)__ldg(seqs.start + b), S = (int)__ldg(seqs.start + b + 1) - t0;
+        if (q - lane >= S) continue;
+        float a = 0.f, d = 0.f;
+        if (q < S) { const float L = __ldg(&lse[(size_t)(t0 + q) * Hq + h]); a = natural ? -L : 14.f - L * 1.4426950408889634f; d = __ldg(&D[(size_t)(t0 + q) * Hq + h]) * dsc; }
+        const size_t o = (size_t)af_slot_row(slot_pitch, Hq, b, h, t0, S) + q;
+        LT[o] = a; DT[o] = d;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -234,13 +284,24 @@ static bool at_f16(sb_ctx_t* c, int hd) {
     int mode = c->pub.use_bf16 ? SB_GEMM_BF16 : c->gemm_mode;
     return mode == SB_GEMM_FP16X3 && (hd % 32) == 0 && !c->attn_fused;
 }
+// The kernels of attention_fused.cu and attention_bwd_fused.cu take the call: 64- and 128-wide heads, any lengths.  Their products are
+// FP32-accurate whatever the mode of the plain products, so the reduced-precision modes take them too (their attention was the
+// TF32 split before: as accurate, twice the tensor-core cycles and a launch per product).
+static bool at_one_kernel(sb_ctx_t* c, int Hq, int Hkv, int hd) {
+    const int mode = c->pub.use_bf16 ? SB_GEMM_BF16 : c->gemm_mode;
+    if (mode == SB_GEMM_SIMT || mode == SB_GEMM_FP32X3 || !c->gemm_pair || !c->attn_flash || c->attn_fused || (hd != 64 && hd != 128)) return false;
+    return Hkv > 0 && Hq % Hkv == 0 && c->attn_seq_starts && tc_load_encode();
+}
+// the boundaries on the host: usable for the tensor-core paths?  (waits for them if they are still on their way)
+static bool at_have_seq(sb_ctx_t* c, int T) {
+    sb_resolve_host_seq(c);
+    return c->h_seq_n > 0 && c->h_seq && c->h_seq[c->h_seq_n] == T;
+}
 static bool at_eligible(sb_ctx_t* c, int T, int Hq, int Hkv, int hd) {
     int mode = c->pub.use_bf16 ? SB_GEMM_BF16 : c->gemm_mode;
     if (mode == SB_GEMM_SIMT || !c->gemm_pair) return false;
-    if (c->h_seq_n <= 0 || !c->h_seq) return false;
     if (hd % 4 || hd < 16 || hd > 256 || Hkv <= 0 || Hq % Hkv) return false;
-    if (T < 128) return false;
-    if (c->h_seq[c->h_seq_n] != T) return false;
+    if (T < 128 || !at_have_seq(c, T)) return false;
     return tc_load_encode();
 }
 
@@ -277,7 +338,7 @@ static bool at_gemm(sb_ctx_t* c, const TcOperand& A, const TcOperand& B, float* 
     return tc_launch(c, p, 3);
 }
 // FP16 parts of x[n] into h[0..n) and h[n..2n), its largest magnitude into *amax
-static AtParts at_make_parts(sb_ctx_t* c, const float* x, size_t n, __half* h, float* amax, bool amax_known = false) {
+static AtParts at_make_parts(sb_ctx_t* c, const float* x, size_t n, __half* h, float* amax) {
     cudaStream_t st = (cudaStream_t)c->pub.stream;
     void* kept; float* kept_amax; int fresh;
     if (sb_parts_find(c, x, n, &kept, &kept_amax, &fresh)) {          // q, k, v of a training step: made in the forward pass, read again here
@@ -287,7 +348,7 @@ static AtParts at_make_parts(sb_ctx_t* c, const float* x, size_t n, __half* h, f
     const dim3 pg(tc_ew_blocks(c, n / 4), 1);
     float* left = sb_amax_lookup(c, x, n);                            // the kernel that wrote x may have left its largest magnitude
     if (left) { amax = left; sb_parts_set_amax(c, x, left); }
-    else if (!amax_known) {
+    else {
         cudaMemsetAsync(amax, 0, sizeof(float), st);
         tc_amax_kernel<<<pg, 256, 0, st>>>(x, n / 4, (unsigned*)amax, nullptr, 0, nullptr);
         c->launches++;
@@ -296,6 +357,38 @@ static AtParts at_make_parts(sb_ctx_t* c, const float* x, size_t n, __half* h, f
     c->launches++;
     AtParts p = {h, h + n, amax};
     return p;
+}
+// The same for several tensors, in one maximum and one split launch; their words are consecutive from need[0].amax (zeroed: by the caller)
+struct AtNeed { const float* x; size_t n; __half* h; float* amax; };
+static void at_make_parts_multi(sb_ctx_t* c, const AtNeed* need, int count, AtParts* out, bool zeroed) {
+    TcMulti am, sp;
+    cudaStream_t st = (cudaStream_t)c->pub.stream;
+    am.n = sp.n = 0; am.chunks = sp.chunks = 0;
+    for (int i = 0; i < count; i++) {
+        __half* h = need[i].h; float* amax = need[i].amax;
+        const float* x = need[i].x; const size_t n = need[i].n;
+        void* kept; float* kept_amax; int fresh = 1;
+        const bool reg = sb_parts_find(c, x, n, &kept, &kept_amax, &fresh) != 0;
+        if (reg) { h = (__half*)kept; amax = kept_amax; }
+        if (fresh) {
+            float* left = sb_amax_lookup(c, x, n);
+            if (left) { amax = left; sb_parts_set_amax(c, x, left); }
+            else {
+                if (reg) cudaMemsetAsync(amax, 0, sizeof(float), st);
+                else if (!zeroed) { cudaMemsetAsync(need[0].amax, 0, count * sizeof(float), st); zeroed = true; }
+                tc_multi_add(&am, x, n, nullptr, amax);
+            }
+            tc_multi_add(&sp, x, n, h, amax);
+        }
+        out[i] = {h, h + n, amax};
+        // large tensors one by one, so that the split finds most of what the maximum pass read in L2 (126 MB): three tensors of 134 MB
+        // prepared together cost 2 % of a forward and backward call at 8 x 2048 tokens, 16 heads of 128
+        if ((size_t)(am.chunks + sp.chunks) * TC_MULTI_CHUNK * 16 > ((size_t)64 << 20) || i + 1 == count) {
+            tc_multi_amax(c, am);
+            tc_multi_split(c, sp);
+            am.n = sp.n = 0; am.chunks = sp.chunks = 0;
+        }
+    }
 }
 // per-(token, head) vector (lse or D, laid out [token][Hq]) as seen by a launch over heads head0, head0+step, ...
 static TcEpi at_epi(int mode, float scale, const float* vec, int tok0, int Hq, int head0, int head_step, const float* aux) {
@@ -344,8 +437,28 @@ static void at_join(sb_ctx_t* c, int ns, void* main_stream) {
     }
 }
 
+// 64- and 128-wide heads: the operands' parts, then one kernel over all sequences and heads
+static int at_forward_one_kernel(sb_ctx_t* c, const float* Q, const float* K, const float* V, float* O, float* lse, int T, int Hq, int Hkv, int hd) {
+    const size_t n_q = (size_t)T * Hq * hd, n_kv = (size_t)T * Hkv * hd;
+    float* consts = (float*)sb_gemm_stage(c, 2, (n_q + 2 * n_kv) * 2 * sizeof(__half) + 64 * sizeof(float));
+    if (!consts) return 1;
+    int tk = sb_tick_begin(c, SB_CLS_ATTN_FWD);
+    __half* hb = (__half*)(consts + 64);
+    const AtNeed need[3] = {{Q, n_q, hb, consts + 8}, {K, n_kv, hb + 2 * n_q, consts + 9}, {V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10}};
+    AtParts p[3];
+    at_make_parts_multi(c, need, 3, p, false);
+    if (!at_have_seq(c, T)) { sb_tick_end(c, tk, 0.0, 0.0); return 1; }
+    double fl = 0;
+    for (int b = 0; b < c->h_seq_n; b++) { const double S = c->h_seq[b + 1] - c->h_seq[b]; fl += 2.0 * Hq * S * S * hd; }
+    const int rc = sb_attention_fused_forward(c, p[0].h1, p[0].h2, p[1].h1, p[1].h2, p[2].h1, p[2].h2, p[0].amax, p[1].amax, p[2].amax, O, lse, T, Hq, Hkv, hd);
+    sb_tick_end(c, tk, fl, 0.0);
+    return rc;
+}
+
 extern "C" int sb_attention_tc_forward(sb_ctx_t* c, const float* Q, const float* K, const float* V, float* O, float* lse,
                                        int T, int Hq, int Hkv, int hd) {
+    if (at_one_kernel(c, Hq, Hkv, hd) && tc_aligned16(Q) && tc_aligned16(K) && tc_aligned16(V) && tc_aligned16(O) &&
+        at_forward_one_kernel(c, Q, K, V, O, lse, T, Hq, Hkv, hd) == 0) return 0;
     if (!at_eligible(c, T, Hq, Hkv, hd)) return 1;
     const int qd = Hq * hd, kvd = Hkv * hd, g = Hq / Hkv;
     const float scale = 1.0f / sqrtf((float)hd);
@@ -357,9 +470,8 @@ extern "C" int sb_attention_tc_forward(sb_ctx_t* c, const float* Q, const float*
     const int G = at_group(Sp, f16 ? 2 : 1, Hkv);
     const size_t n_s = (size_t)G * Sp * Sp;
     const size_t per_stream = f16 ? 2 * n_s : n_s;                   // floats: S, then (FP16) the two parts of P
-    const bool one_kernel = f16 && c->attn_flash && hd == 128 && c->h_seq_n <= 240;      // no score scratch at all
-    float* Sb0 = one_kernel ? nullptr : (float*)sb_gemm_stage(c, 3, AT_SIDE * per_stream * sizeof(float));
-    if (!Sb0 && !one_kernel) return 1;
+    float* Sb0 = (float*)sb_gemm_stage(c, 3, AT_SIDE * per_stream * sizeof(float));
+    if (!Sb0) return 1;
     const size_t n_q = (size_t)T * qd, n_kv = (size_t)T * kvd;
     AtParts pq = AT_NOPARTS, pk = AT_NOPARTS, pv = AT_NOPARTS;
     float* consts = nullptr;
@@ -372,16 +484,6 @@ extern "C" int sb_attention_tc_forward(sb_ctx_t* c, const float* Q, const float*
         pq = at_make_parts(c, Q, n_q, hb, consts + 8);
         pk = at_make_parts(c, K, n_kv, hb + 2 * n_q, consts + 9);
         pv = at_make_parts(c, V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10);
-        if (one_kernel) {
-            double fl = 0;
-            for (int b = 0; b < c->h_seq_n; b++) { const double S = c->h_seq[b + 1] - c->h_seq[b]; fl += 2.0 * Hq * S * S * hd; }
-            if (sb_attention_fused_forward(c, pq.h1, pq.h2, pk.h1, pk.h2, pv.h1, pv.h2, pq.amax, pk.amax, pv.amax, O, lse, T, Hq, Hkv, hd) == 0) {
-                sb_tick_end(c, tk, fl, 0.0);
-                return 0;
-            }
-            Sb0 = (float*)sb_gemm_stage(c, 3, AT_SIDE * per_stream * sizeof(float));
-            if (!Sb0) { sb_tick_end(c, tk, 0.0, 0.0); return 1; }
-        }
         at_consts_kernel<<<1, 1, 0, (cudaStream_t)c->pub.stream>>>(consts, consts + 2, scale);       // only consts[0] is used here
         c->launches++;
     }
@@ -416,9 +518,84 @@ extern "C" int sb_attention_tc_forward(sb_ctx_t* c, const float* Q, const float*
     return 0;
 }
 
+// 64- and 128-wide heads: D and the maxima, then the parts of dO and the row vectors, then dK and dV on chip, then dQ
+static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, const float* V, const float* O, const float* lse, const float* dO,
+                               float* dQ, float* dK, float* dV, int accumulate_kv, int T, int Hq, int Hkv, int hd) {
+    const int qd = Hq * hd, kvd = Hkv * hd, g = Hq / Hkv;
+    const float scale = 1.0f / sqrtf((float)hd);
+    const size_t n_q = (size_t)T * qd, n_kv = (size_t)T * kvd, d_floats = ((size_t)T * Hq + 63) & ~(size_t)63;
+    float* D = (float*)sb_gemm_stage(c, 2, (d_floats + 64) * sizeof(float) + (2 * n_q + 2 * n_kv) * 2 * sizeof(__half));
+    if (!D) return 1;
+    float* consts = D + d_floats;                                    // [0] 1.0, [1] dS bound, [2] max |dO row|, [3] max |V row|, [8..11] amax of Q, K, V, dO
+    __half* hb = (__half*)(consts + 64);
+    cudaStream_t st = (cudaStream_t)c->pub.stream;
+    int tk = sb_tick_begin(c, SB_CLS_ATTN_BWD);
+    cudaMemsetAsync(consts, 0, 64 * sizeof(float), st);
+    const AtNeed need[3] = {{Q, n_q, hb, consts + 8}, {K, n_kv, hb + 2 * n_q, consts + 9}, {V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10}};
+    AtParts p[3];
+    at_make_parts_multi(c, need, 3, p, true);
+    __half* hdo = hb + 2 * n_q + 4 * n_kv;
+    {
+        const int rpb = 8 * 4 * (128 / hd);                          // rows a CTA takes per pass
+        const int cap = c->pub.gpu_sm_count * 8, want = (T * Hq + rpb - 1) / rpb;
+        const dim3 pg(want < cap ? want : cap, 2);
+        if (hd == 128) at_bwd_prep_kernel<128><<<pg, 256, 0, st>>>(dO, O, D, T * Hq, V, T * Hkv, (unsigned*)(consts + 2), (unsigned*)(consts + 11), (unsigned*)(consts + 3));
+        else at_bwd_prep_kernel<64><<<pg, 256, 0, st>>>(dO, O, D, T * Hq, V, T * Hkv, (unsigned*)(consts + 2), (unsigned*)(consts + 11), (unsigned*)(consts + 3));
+        c->launches++;
+    }
+    // from here on the launches depend on the boundaries
+    int Smax = 0, n = 0;
+    double flops = 0;
+    if (at_have_seq(c, T)) n = c->h_seq_n;
+    for (int b = 0; b < n; b++) { const int S = c->h_seq[b + 1] - c->h_seq[b]; Smax = max(Smax, S); flops += 5.0 * Hq * (double)S * S * hd; }
+    if (Smax <= 0) { sb_tick_end(c, tk, 0.0, 0.0); return 1; }
+    // Long sequences of 128-wide heads: dQ from the CTA-pair GEMM kernel (256-row tiles read K half as often), a launch per sequence.
+    // Shorter ones and 64-wide heads: at_dq_bwd_kernel, one launch for all.  8 x 2048 tokens, 16 heads: 1.57 against 1.67 ms for the whole
+    // call; 5 sequences of 1080 on average: equal; 33M model, 24 sequences of 240: a launch instead of 24.
+    const bool dq_gemm = hd == 128 && (long)n * 1024 <= T;
+    const int Sp = round_up(Smax, dq_gemm ? AT_ROWTILE : 128), slot_pitch = dq_gemm ? Sp : 0;
+    const size_t rows = af_slot_rows(slot_pitch, Hq, n, T), n_ds = rows * (size_t)Sp, row_floats = (rows + 63) & ~(size_t)63;
+    float* bb = (float*)sb_gemm_stage(c, 3, n_ds * 4 + 2 * row_floats * sizeof(float));
+    if (!bb) { sb_tick_end(c, tk, 0.0, 0.0); return 1; }
+    float* LT = bb + n_ds; float* DT = LT + row_floats;
+    {
+        const AfSeqTab seqs = {n, c->attn_seq_starts};
+        at_bwd_prep2_kernel<<<dim3(tc_ew_blocks(c, n_q / 8), 2), 256, 0, st>>>((const float4*)dO, n_q / 4, (uint2*)hdo, (uint2*)(hdo + n_q), consts + 11,
+                                                                            consts, consts + 2, scale, lse, D, LT, DT, seqs, Hq, Smax, slot_pitch, hd == 64 ? 1 : 0);
+        c->launches++;
+    }
+    __half* a = (__half*)bb;
+    AbCall call = {p[0].h1, p[0].h2, hdo, hdo + n_q, p[1].h1, p[1].h2, p[2].h1, p[2].h2, p[0].amax, p[1].amax, p[2].amax, consts + 11, consts + 1, LT, DT,
+                   a, a + n_ds, dK, dV, dq_gemm ? nullptr : dQ, accumulate_kv, Sp, T, Hq, Hkv};
+    bool ok = sb_attention_fused_dkv(c, call, hd) == 0;
+    if (ok && dq_gemm) {
+        void* main_stream = c->pub.stream;
+        const int ns = at_fork(c, n);
+        const long sb = (long)Sp * Sp;
+        for (int b = 0; b < n && ok; b++) {
+            const int t0 = c->h_seq[b], S = c->h_seq[b + 1] - t0;
+            if (S <= 0) continue;
+            if (ns > 1) c->pub.stream = c->side_stream[b % ns];
+            // all query heads of the sequence in one launch: head h reads slot b Hq + h of dS^T and K/V head h / g
+            const AtParts pds = {a + (size_t)b * Hq * sb, a + n_ds + (size_t)b * Hq * sb, consts + 1};
+            TcOperand kop = op_tokens_mn(K, p[1], t0, kvd, Hkv, hd, 0, 1);
+            kop.c2_div = g;
+            ok = ok && at_gemm(c, op_scratch(bb, pds, S, Sp, Hq, 1), kop, dQ + (size_t)t0 * qd, qd, (long)hd, S, hd, S, 0, Hq,
+                               TC_CAUSAL_K_UPTO_M, nullptr, pds.amax, p[1].amax);
+        }
+        at_join(c, ns, main_stream);
+    }
+    sb_tick_end(c, tk, flops, 0.0);
+    if (!ok) sb_set_status(c, SB_ERR_CUDA);
+    return ok ? 0 : 1;
+}
+
 extern "C" int sb_attention_tc_backward(sb_ctx_t* c, const float* Q, const float* K, const float* V, const float* O, const float* lse,
                                         const float* dO, float* dQ, float* dK, float* dV, int accumulate_kv,
                                         int T, int Hq, int Hkv, int hd) {
+    if (at_one_kernel(c, Hq, Hkv, hd) && c->attn_flash != 2 && tc_aligned16(Q) && tc_aligned16(K) && tc_aligned16(V) && tc_aligned16(O) &&
+        tc_aligned16(dO) && tc_aligned16(dQ) && tc_aligned16(dK) && tc_aligned16(dV) &&
+        at_backward_on_chip(c, Q, K, V, O, lse, dO, dQ, dK, dV, accumulate_kv, T, Hq, Hkv, hd) == 0) return 0;
     if (!at_eligible(c, T, Hq, Hkv, hd)) return 1;
     const int qd = Hq * hd, kvd = Hkv * hd, g = Hq / Hkv;
     const float scale = 1.0f / sqrtf((float)hd);
@@ -438,31 +615,15 @@ extern "C" int sb_attention_tc_backward(sb_ctx_t* c, const float* Q, const float
     const size_t n_all = (size_t)c->h_seq_n * Hq * Sp * Sp;
     size_t all_limit = AT_ALL_SCORES_BYTES;                          // SERAPH_B200_ATTN_ALL_SCORES_MB overrides (0, the default: one launch per sequence and head group)
     { const char* e = getenv("SERAPH_B200_ATTN_ALL_SCORES_MB"); if (e && e[0]) all_limit = (size_t)atol(e) << 20; }
-    const bool all_scores = f16 && c->attn_flash && !c->attn_fused && hd == 128 && c->h_seq_n <= 240 && n_all * 8 <= all_limit;
+    const bool all_scores = f16 && c->attn_flash && !c->attn_fused && hd == 128 && c->h_seq_n <= AF_MAXSEQ && n_all * 8 <= all_limit;
     const size_t group_bytes = AT_SIDE * per_stream * sizeof(float);
-    // 128-wide heads, default mode: dK and dV accumulate on chip in one launch over all sequences and K/V heads that leaves only
-    // the FP16 parts of dS^T (4 bytes per score, [sequence][K-V head][group member][key][query]); dQ is then one product per
-    // sequence over all its query heads.  seraph_b200_set_attn_flash(ctx, 2) or SERAPH_B200_ATTN_FLASH=2 selects the older
-    // score-materialising path, 3 this one, for every shape.
-    // attn_flash 1 (default) and 3 take this path (it measured faster at every shape tried: 16 % at 2048 tokens with two query heads
-    // per K/V head, 30 % without head grouping)
-    const bool dkv_fused = f16 && (c->attn_flash == 3 || c->attn_flash == 1) && !c->attn_fused && hd == 128 &&
-                           c->h_seq_n <= 240 && !all_scores;
-    size_t need = all_scores ? (n_all * 8 > group_bytes ? n_all * 8 : group_bytes) : group_bytes;
-    const size_t n_rows = (size_t)c->h_seq_n * Hq * Sp;             // log-sum-exp and D by [sequence][head][query] for the on-chip kernel
-    if (dkv_fused && n_all * 4 + 2 * n_rows * sizeof(float) > need) need = n_all * 4 + 2 * n_rows * sizeof(float);
-    float* bb = (float*)sb_gemm_stage(c, 3, need);
+    float* bb = (float*)sb_gemm_stage(c, 3, all_scores && n_all * 8 > group_bytes ? n_all * 8 : group_bytes);
     if (!st0 || !bb) return 1;
     float* D = st0;
     float* consts = st0 + d_floats;                                  // [0] 1.0, [1] dS bound, [2] max |dO row|, [3] max |V row|, [8..11] amax of Q, K, V, dO
     AtParts pq = AT_NOPARTS, pk = AT_NOPARTS, pv = AT_NOPARTS, pdo = AT_NOPARTS;
     cudaStream_t s0 = (cudaStream_t)c->pub.stream;
     int tk = sb_tick_begin(c, SB_CLS_ATTN_BWD);
-    const bool prep128 = f16 && hd == 128 && tc_aligned16(dO) && tc_aligned16(O);      // D, max |dO| and its largest row norm in one pass
-    if (prep128) {
-        cudaMemsetAsync(consts + 2, 0, 10 * sizeof(float), s0);
-        at_bwd_prep128_kernel<<<at_rn_blocks(c, T * Hq), 256, 0, s0>>>(dO, O, D, T * Hq, (unsigned*)(consts + 2), (unsigned*)(consts + 11));
-    } else
     at_delta_kernel<<<(T * Hq * 32 + 255) / 256, 256, 0, s0>>>(dO, O, D, T * Hq, hd);
     c->launches++;
     if (f16) {
@@ -470,15 +631,12 @@ extern "C" int sb_attention_tc_backward(sb_ctx_t* c, const float* Q, const float
         pq = at_make_parts(c, Q, n_q, hb, consts + 8);
         pk = at_make_parts(c, K, n_kv, hb + 2 * n_q, consts + 9);
         pv = at_make_parts(c, V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10);
-        pdo = at_make_parts(c, dO, n_q, hb + 2 * n_q + 4 * n_kv, consts + 11, prep128);
-        if (!prep128) {
-            cudaMemsetAsync(consts + 2, 0, 2 * sizeof(float), s0);
-            at_rownorm_max_kernel<<<at_rn_blocks(c, T * Hq), 256, 0, s0>>>(dO, T * Hq, hd, (unsigned*)(consts + 2));
-            c->launches++;
-        }
+        pdo = at_make_parts(c, dO, n_q, hb + 2 * n_q + 4 * n_kv, consts + 11);
+        cudaMemsetAsync(consts + 2, 0, 2 * sizeof(float), s0);
+        at_rownorm_max_kernel<<<at_rn_blocks(c, T * Hq), 256, 0, s0>>>(dO, T * Hq, hd, (unsigned*)(consts + 2));
         at_rownorm_max_kernel<<<at_rn_blocks(c, T * Hkv), 256, 0, s0>>>(V, T * Hkv, hd, (unsigned*)(consts + 3));
         at_consts_kernel<<<1, 1, 0, s0>>>(consts, consts + 2, scale);
-        c->launches += 2;
+        c->launches += 3;
     }
     bool ok = true;
     double flops = 0;
@@ -488,37 +646,6 @@ extern "C" int sb_attention_tc_backward(sb_ctx_t* c, const float* Q, const float
         __half* a = (__half*)bb;
         have_all = sb_attention_fused_scores(c, pq.h1, pq.h2, pdo.h1, pdo.h2, pk.h1, pk.h2, pv.h1, pv.h2, pq.amax, pk.amax, pv.amax, pdo.amax,
                                              consts + 1, lse, D, a, a + n_all, a + 2 * n_all, a + 3 * n_all, 0, 0, Sp, T, Hq, Hkv, hd, 0, 0, 0) == 0;
-    }
-    if (dkv_fused) {
-        __half* a = (__half*)bb;
-        if (!accumulate_kv) {
-            cudaMemsetAsync(dK, 0, n_kv * sizeof(float), s0);
-            cudaMemsetAsync(dV, 0, n_kv * sizeof(float), s0);
-        }
-        if (sb_attention_fused_dkv(c, pq.h1, pq.h2, pdo.h1, pdo.h2, pk.h1, pk.h2, pv.h1, pv.h2, pq.amax, pk.amax, pv.amax, pdo.amax,
-                                   consts + 1, lse, D, a, a + n_all, (float*)(a + 2 * n_all), (float*)(a + 2 * n_all) + n_rows, dK, dV, Sp, T, Hq, Hkv, hd) == 0) {
-            const int ns2 = at_fork(c, c->h_seq_n);
-            const long sb = (long)Sp * Sp;
-            for (int b = 0; b < c->h_seq_n && ok; b++) {
-                const int t0 = c->h_seq[b], S = c->h_seq[b + 1] - t0;
-                if (S <= 0) continue;
-                flops += 5.0 * Hq * (double)S * S * hd;
-                if (ns2 > 1) c->pub.stream = c->side_stream[b % ns2];
-                {
-                    // all query heads of the sequence in one launch: head h reads slot b Hq + h of dS^T and K/V head h / g
-                    __half* d1 = a + ((size_t)b * Hq) * (size_t)sb;
-                    const AtParts pds = {d1, d1 + n_all, consts + 1};
-                    TcOperand kop = op_tokens_mn(K, pk, t0, kvd, Hkv, hd, 0, 1);
-                    kop.c2_div = g;
-                    ok = ok && at_gemm(c, op_scratch(bb, pds, S, Sp, Hq, 1), kop, dQ + (size_t)t0 * qd, qd, (long)hd, S, hd, S, 0, Hq,
-                                       TC_CAUSAL_K_UPTO_M, nullptr, pds.amax, pk.amax);                                       // dQ = dS K
-                }
-            }
-            at_join(c, ns2, main_stream);
-            sb_tick_end(c, tk, flops, 0.0);
-            if (!ok) { sb_set_status(c, SB_ERR_CUDA); return 1; }
-            return 0;
-        }
     }
     const int Gl = have_all ? Hkv : G;                               // K-V heads per launch of the long products
     const int ns = at_fork(c, c->h_seq_n);

@@ -905,6 +905,93 @@ static __global__ void __launch_bounds__(256) tc_split_f16_kernel(const float* _
     }
 }
 
+// The same two passes over up to TC_MULTI tensors in one launch each: the tensors are cut into chunks of TC_MULTI_CHUNK float4, a CTA takes
+// an equal run of chunks.  Preparing a small model's operands is launches, not bytes: one launch instead of one or two per tensor.
+#define TC_MULTI 64
+#define TC_MULTI_CHUNK 1024
+struct TcMultiJob { const float* x; __half* h; float* amax; uint32_t n4, first; };      // h: hi parts, lo parts behind them; first: its first chunk
+struct TcMulti { int n; uint32_t chunks; TcMultiJob j[TC_MULTI]; };
+static inline void tc_multi_add(TcMulti* m, const float* x, size_t n, void* h, float* amax) {
+    TcMultiJob* j = &m->j[m->n++];
+    j->x = x; j->h = (__half*)h; j->amax = amax; j->n4 = (uint32_t)(n / 4); j->first = m->chunks;
+    m->chunks += (j->n4 + TC_MULTI_CHUNK - 1) / TC_MULTI_CHUNK;
+}
+__device__ __forceinline__ int tc_multi_find(const TcMulti& m, uint32_t chunk) {
+    int lo = 0, hi = m.n - 1;
+    while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (m.j[mid].first <= chunk) lo = mid; else hi = mid - 1; }
+    return lo;
+}
+static __global__ void __launch_bounds__(256) tc_amax_multi_kernel(const __grid_constant__ TcMulti m) {
+    __shared__ float red[8];
+    const uint32_t per = (m.chunks + gridDim.x - 1) / gridDim.x;
+    uint32_t ck = blockIdx.x * per;
+    const uint32_t end = min(m.chunks, ck + per);
+    while (ck < end) {
+        const int jb = tc_multi_find(m, ck);
+        const TcMultiJob& j = m.j[jb];
+        const uint32_t last = min(end, jb + 1 < m.n ? m.j[jb + 1].first : m.chunks);
+        const float4* x = (const float4*)j.x;
+        float mx = 0.f;
+        for (; ck < last; ck++) {
+            const uint32_t base = (ck - j.first) * TC_MULTI_CHUNK + threadIdx.x;
+            float4 v[TC_MULTI_CHUNK / 256];
+#pragma unroll
+            for (int u = 0; u < TC_MULTI_CHUNK / 256; u++) v[u] = base + u * 256 < j.n4 ? __ldg(x + base + u * 256) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < TC_MULTI_CHUNK / 256; u++) mx = sb_amax4(mx, v[u]);
+        }
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[w]);
+            if (mx > 0.f) atomicMax((unsigned*)j.amax, __float_as_uint(mx));
+        }
+        __syncthreads();
+    }
+}
+// walks each CTA's run backwards: what the maximum pass read last is still in L2
+static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid_constant__ TcMulti m) {
+    const uint32_t per = (m.chunks + gridDim.x - 1) / gridDim.x;
+    const uint32_t begin = blockIdx.x * per;
+    uint32_t ck = min(m.chunks, begin + per);
+    while (ck > begin) {
+        const int jb = tc_multi_find(m, ck - 1);
+        const TcMultiJob& j = m.j[jb];
+        const uint32_t stop = max(begin, j.first);
+        const float4* x = (const float4*)j.x;
+        uint2* h1 = (uint2*)j.h; uint2* h2 = h1 + j.n4;
+        const float sc = tc_pow2(tc_f16_shift(*j.amax));
+        while (ck > stop) {
+            ck--;
+            const uint32_t base = (ck - j.first) * TC_MULTI_CHUNK + threadIdx.x;
+            float4 v[TC_MULTI_CHUNK / 256];
+#pragma unroll
+            for (int u = 0; u < TC_MULTI_CHUNK / 256; u++) if (base + u * 256 < j.n4) v[u] = __ldg(x + base + u * 256);
+#pragma unroll
+            for (int u = 0; u < TC_MULTI_CHUNK / 256; u++) if (base + u * 256 < j.n4) {
+                uint2 a, b;
+                sb_split2(v[u].x * sc, v[u].y * sc, a.x, b.x); sb_split2(v[u].z * sc, v[u].w * sc, a.y, b.y);
+                h1[base + u * 256] = a; h2[base + u * 256] = b;
+            }
+        }
+    }
+}
+static inline unsigned tc_multi_grid(sb_ctx_t* c, const TcMulti& m) {
+    const unsigned cap = (unsigned)(c->pub.gpu_sm_count > 0 ? c->pub.gpu_sm_count : 148) * 8;
+    return m.chunks < cap ? (m.chunks ? m.chunks : 1) : cap;
+}
+static inline void tc_multi_amax(sb_ctx_t* c, const TcMulti& m) {      // the words are zero before
+    if (!m.n) return;
+    tc_amax_multi_kernel<<<tc_multi_grid(c, m), 256, 0, (cudaStream_t)c->pub.stream>>>(m);
+    c->launches++;
+}
+static inline void tc_multi_split(sb_ctx_t* c, const TcMulti& m) {
+    if (!m.n) return;
+    tc_split_multi_kernel<<<tc_multi_grid(c, m), 256, 0, (cudaStream_t)c->pub.stream>>>(m);
+    c->launches++;
+}
+
 // --------------------------------------------------------------------------- operand preparation kernels
 // lo[i] = x[i] - tf32_trunc(x[i]);  8 bytes per element
 static __global__ void __launch_bounds__(256) split_lo_kernel(const float* __restrict__ x, float* __restrict__ lo, size_t n4) {
@@ -956,60 +1043,57 @@ static inline bool tc_swapped(const TcOperand& op) { return op.c2_dim > 1 && op.
 
 // Encoding a tensor map costs a few microseconds on the host and a training step re-issues the same
 // (pointer, shape) combinations every layer and every step, so encoded maps are kept in a small
-// direct-mapped cache keyed by everything that goes into the encoding.
-struct TcMapKey { const void* base; long pitch, c2_stride; int K, rows, c2_dim, BK, box_rows, mn, elt; };
+// direct-mapped cache of the context, keyed by everything that goes into the encoding.
+struct TcMapKey { uint64_t base, dims[3], strides[2], box01, box2_rank, dt_swz; };
 struct TcMapEntry { TcMapKey key; CUtensorMap map; bool valid; };
-#define TC_MAP_CACHE 8192
-static TcMapEntry* g_tc_map_cache = nullptr;
+#define TC_MAP_CACHE 4096
+
+static bool tc_encode(sb_ctx_t* c, CUtensorMap* m, CUtensorMapDataType dt, int rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
+                      const cuuint32_t* box, CUtensorMapSwizzle swz, CUtensorMapL2promotion promo = CU_TENSOR_MAP_L2_PROMOTION_L2_256B) {
+    TcMapKey key;
+    memset(&key, 0, sizeof key);
+    key.base = (uint64_t)(uintptr_t)base;
+    for (int i = 0; i < rank; i++) key.dims[i] = dims[i];
+    for (int i = 0; i + 1 < rank; i++) key.strides[i] = strides[i];
+    key.box01 = (uint64_t)box[0] | ((uint64_t)(rank > 1 ? box[1] : 0u) << 32);
+    key.box2_rank = (uint64_t)(rank > 2 ? box[2] : 0u) | ((uint64_t)rank << 32);
+    key.dt_swz = (uint64_t)dt | ((uint64_t)swz << 16) | ((uint64_t)promo << 32);
+    if (!c->map_cache) c->map_cache = calloc(TC_MAP_CACHE, sizeof(TcMapEntry));
+    TcMapEntry* e = nullptr;
+    if (c->map_cache) {
+        const uint64_t* w = (const uint64_t*)&key;
+        uint64_t h = 1469598103934665603ull;
+        for (size_t i = 0; i < sizeof key / 8; i++) { h ^= w[i]; h *= 0x9E3779B97F4A7C15ull; h ^= h >> 29; }
+        e = (TcMapEntry*)c->map_cache + h % TC_MAP_CACHE;
+        if (e->valid && memcmp(&e->key, &key, sizeof key) == 0) { *m = e->map; return true; }
+    }
+    const cuuint32_t estr[3] = {1, 1, 1};
+    if (g_tc_encode(m, dt, (cuuint32_t)rank, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, promo,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return false;
+    if (e) { e->key = key; e->map = *m; e->valid = true; }
+    return true;
+}
 
 // 3-D FP32 tensor {K, rows, slots} (or {K, slots, rows}); box = BK x box_rows x 1; reads beyond the extents give zero
 // elt = 2: the same for an FP16 array of the same shape (BK halfs per box; MN-major boxes are 64 rows, plain 128-byte swizzle)
-static bool tc_make_map(CUtensorMap* m, const void* base, const TcOperand& op, int K, int BK, int box_rows, int elt = 4) {
-    TcMapKey key;
-    memset(&key, 0, sizeof key);
-    key.elt = elt;
+static bool tc_make_map(sb_ctx_t* c, CUtensorMap* m, const void* base, const TcOperand& op, int K, int BK, int box_rows, int elt = 4) {
     const CUtensorMapDataType dt = elt == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    key.base = base; key.pitch = op.pitch; key.c2_stride = op.c2_dim > 1 ? op.c2_stride : 0; key.K = K; key.rows = op.rows;
-    key.c2_dim = op.c2_dim > 1 ? op.c2_dim : 1; key.BK = BK; key.box_rows = box_rows; key.mn = op.mn;
-    if (!g_tc_map_cache) g_tc_map_cache = (TcMapEntry*)calloc(TC_MAP_CACHE, sizeof(TcMapEntry));
-    TcMapEntry* e = nullptr;
-    if (g_tc_map_cache) {
-        uint64_t h = 1469598103934665603ull;
-        const unsigned char* kb = (const unsigned char*)&key;
-        for (size_t i = 0; i < sizeof key; i++) { h ^= kb[i]; h *= 1099511628211ull; }
-        e = &g_tc_map_cache[h % TC_MAP_CACHE];
-        if (e->valid && memcmp(&e->key, &key, sizeof key) == 0) { *m = e->map; return true; }
-    }
+    const bool sw = tc_swapped(op);
+    const cuuint64_t nslot = (cuuint64_t)(op.c2_dim > 1 ? op.c2_dim : 1);
     if (op.mn) {
-        // the array is [K, rows] with rows contiguous: {rows, K, 1}, boxes of 32 floats x BK k-rows, 128-byte swizzle of 32-byte units
-        const bool swm = tc_swapped(op);
-        const cuuint64_t nsl = (cuuint64_t)(op.c2_dim > 1 ? op.c2_dim : 1);
+        // the array is [K, rows] with rows contiguous: {rows, K, 1}, boxes of 128 bytes x BK k-rows, 128-byte swizzle (of 32-byte units for FP32)
         const cuuint64_t krow = (cuuint64_t)op.pitch * elt;
         const cuuint64_t sl = op.c2_dim > 1 ? (cuuint64_t)op.c2_stride * elt : krow * (cuuint64_t)K;
-        cuuint64_t dims[3] = {(cuuint64_t)op.rows, swm ? nsl : (cuuint64_t)K, swm ? (cuuint64_t)K : nsl};
-        cuuint64_t strides[2] = {swm ? sl : krow, swm ? krow : sl};
-        cuuint32_t box[3] = {(cuuint32_t)(128 / elt), swm ? 1u : (cuuint32_t)BK, swm ? (cuuint32_t)BK : 1u};
-        cuuint32_t estr[3] = {1, 1, 1};
-        CUresult r = g_tc_encode(m, dt, 3, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                 elt == 2 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return false;
-        if (e) { e->key = key; e->map = *m; e->valid = true; }
-        return true;
+        const cuuint64_t dims[3] = {(cuuint64_t)op.rows, sw ? nslot : (cuuint64_t)K, sw ? (cuuint64_t)K : nslot};
+        const cuuint64_t strides[2] = {sw ? sl : krow, sw ? krow : sl};
+        const cuuint32_t box[3] = {(cuuint32_t)(128 / elt), sw ? 1u : (cuuint32_t)BK, sw ? (cuuint32_t)BK : 1u};
+        return tc_encode(c, m, dt, 3, base, dims, strides, box, elt == 2 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
     }
-    const bool sw = tc_swapped(op);
-    const cuuint64_t nslot = (cuuint64_t)(op.c2_dim > 0 ? op.c2_dim : 1);
     const cuuint64_t slot_stride = (cuuint64_t)(op.c2_dim > 1 ? op.c2_stride : (long)op.pitch * op.rows) * elt;
-    cuuint64_t dims[3] = {(cuuint64_t)K, sw ? nslot : (cuuint64_t)op.rows, sw ? (cuuint64_t)op.rows : nslot};
-    cuuint64_t strides[2] = {sw ? slot_stride : (cuuint64_t)op.pitch * elt, sw ? (cuuint64_t)op.pitch * elt : slot_stride};
-    cuuint32_t box[3] = {(cuuint32_t)BK, sw ? 1u : (cuuint32_t)box_rows, sw ? (cuuint32_t)box_rows : 1u};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = g_tc_encode(m, dt, 3, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             BK * elt == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return false;
-    if (e) { e->key = key; e->map = *m; e->valid = true; }
-    return true;
+    const cuuint64_t dims[3] = {(cuuint64_t)K, sw ? nslot : (cuuint64_t)op.rows, sw ? (cuuint64_t)op.rows : nslot};
+    const cuuint64_t strides[2] = {sw ? slot_stride : (cuuint64_t)op.pitch * elt, sw ? (cuuint64_t)op.pitch * elt : slot_stride};
+    const cuuint32_t box[3] = {(cuuint32_t)BK, sw ? 1u : (cuuint32_t)box_rows, sw ? (cuuint32_t)box_rows : 1u};
+    return tc_encode(c, m, dt, 3, base, dims, strides, box, BK * elt == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 static inline bool tc_aligned16(const void* p) { return (((uintptr_t)p) & 15) == 0; }
@@ -1021,11 +1105,11 @@ static bool tc_launch_t(sb_ctx_t* c, const TcProblem& p) {
     constexpr bool CONV = (CTAS == 2 && NTERMS == 3);
     constexpr int BKE = PREP ? 2 * BK : BK;
     if (PREP) {
-        if (!tc_make_map(&mAh, p.A.h1, p.A, p.K, BKE, TC_BM, 2) || !tc_make_map(&mBh, p.B.h1, p.B, p.K, BKE, BROWS, 2) ||
-            !tc_make_map(&mAl, p.A.h2, p.A, p.K, BKE, TC_BM, 2) || !tc_make_map(&mBl, p.B.h2, p.B, p.K, BKE, BROWS, 2)) return false;
+        if (!tc_make_map(c, &mAh, p.A.h1, p.A, p.K, BKE, TC_BM, 2) || !tc_make_map(c, &mBh, p.B.h1, p.B, p.K, BKE, BROWS, 2) ||
+            !tc_make_map(c, &mAl, p.A.h2, p.A, p.K, BKE, TC_BM, 2) || !tc_make_map(c, &mBl, p.B.h2, p.B, p.K, BKE, BROWS, 2)) return false;
     } else
-    if (!tc_make_map(&mAh, p.A.hi, p.A, p.K, BK, TC_BM) || !tc_make_map(&mBh, p.B.hi, p.B, p.K, BK, BROWS)) return false;
-    if (!PREP && NTERMS == 3 && !CONV) { if (!tc_make_map(&mAl, p.A.lo, p.A, p.K, BK, TC_BM) || !tc_make_map(&mBl, p.B.lo, p.B, p.K, BK, BROWS)) return false; }
+    if (!tc_make_map(c, &mAh, p.A.hi, p.A, p.K, BK, TC_BM) || !tc_make_map(c, &mBh, p.B.hi, p.B, p.K, BK, BROWS)) return false;
+    if (!PREP && NTERMS == 3 && !CONV) { if (!tc_make_map(c, &mAl, p.A.lo, p.A, p.K, BK, TC_BM) || !tc_make_map(c, &mBl, p.B.lo, p.B, p.K, BK, BROWS)) return false; }
     else if (!PREP) { mAl = mAh; mBl = mBh; }
     constexpr int STAGE_BYTES = (NTERMS == 3 ? 2 : 1) * (TC_BM + BROWS) * BK * 4;
     constexpr size_t stg_bytes = (size_t)TC_STG_ROWS * (BN + 4) * 4;

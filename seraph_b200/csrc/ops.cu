@@ -51,23 +51,58 @@ int sb_set_host_seq(sb_ctx_t* c, const int* starts, int B) {
     return 0;
 }
 
-// index tables for one packed batch described by a device seq_starts array; the boundaries are also read back
-// to the host (small synchronous copy) because the tensor-core attention builds its tile maps per sequence
+// index tables for one packed batch described by a device seq_starts array (no host copy of the boundaries: these ops read the tables only)
 static int index_from_device_starts(sb_ctx_t* c, const uint32_t* d_starts, int B, int T) {
     if (sb_ensure_tokens(c, T, B)) return 1;
     sb_seq_index(c, d_starts, B, T, c->pos_ids, c->seq_ids);
     c->h_seq_n = 0;
-    if (B > 0 && B < (1 << 20)) {
-        int* tmp = (int*)malloc(sizeof(int) * (size_t)(B + 1));
-        if (tmp) {
-            cudaStreamSynchronize((cudaStream_t)c->pub.stream);
-            if (cudaMemcpy(tmp, d_starts, sizeof(int) * (size_t)(B + 1), cudaMemcpyDeviceToHost) == cudaSuccess && tmp[0] == 0 && tmp[B] == T)
-                sb_set_host_seq(c, tmp, B);
-            free(tmp);
-        }
-    }
     return 0;
 }
+// The packed attention ops: the tensor-core paths size their launches from the boundaries, so these are read back to the host.  The copy goes
+// through a stream of its own that waits only for what was queued before the call: the operand preparation, which does not depend on the
+// boundaries, is queued meanwhile, and the host waits for the copy (sb_resolve_host_seq) with the GPU at work instead of draining it.
+// The per-token tables are made only if the CUDA-core kernels end up taking the call.
+static int starts_for_attention(sb_ctx_t* c, const uint32_t* d_starts, int B, int T) {
+    if (sb_ensure_tokens(c, T, B)) return 1;
+    c->h_seq_n = 0; c->seq_pending = 0;
+    c->lazy_starts = d_starts; c->lazy_B = B; c->lazy_T = T;
+    if (B <= 0 || B >= (1 << 20)) return 0;
+    if (!c->seq_copy_stream) {
+        cudaStream_t st; cudaEvent_t e0, e1;
+        if (sb_check(c, cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "copy stream")) return 1;
+        c->seq_copy_stream = st;
+        if (sb_check(c, cudaEventCreateWithFlags(&e0, cudaEventDisableTiming), "copy event")) return 1;
+        c->seq_copy_ev[0] = e0;
+        if (sb_check(c, cudaEventCreateWithFlags(&e1, cudaEventDisableTiming), "copy event")) return 1;
+        c->seq_copy_ev[1] = e1;
+    }
+    if (!c->seq_copy_ev[0] || !c->seq_copy_ev[1]) return 1;
+    if (c->h_seq_pin_cap < B + 1) {
+        if (c->h_seq_pin) cudaFreeHost(c->h_seq_pin);
+        c->h_seq_pin = NULL; c->h_seq_pin_cap = 0;
+        const int cap = B + 1 < 1024 ? 1024 : B + 1;
+        if (sb_check(c, cudaMallocHost((void**)&c->h_seq_pin, sizeof(int) * (size_t)cap), "pinned sequence boundaries")) return 1;
+        c->h_seq_pin_cap = cap;
+    }
+    cudaEventRecord((cudaEvent_t)c->seq_copy_ev[0], (cudaStream_t)c->pub.stream);
+    cudaStreamWaitEvent((cudaStream_t)c->seq_copy_stream, (cudaEvent_t)c->seq_copy_ev[0], 0);
+    if (cudaMemcpyAsync(c->h_seq_pin, d_starts, sizeof(int) * (size_t)(B + 1), cudaMemcpyDeviceToHost, (cudaStream_t)c->seq_copy_stream) == cudaSuccess &&
+        cudaEventRecord((cudaEvent_t)c->seq_copy_ev[1], (cudaStream_t)c->seq_copy_stream) == cudaSuccess) c->seq_pending = 1;
+    return 0;
+}
+// waits for the boundaries of the call in flight, if they are still on their way
+void sb_resolve_host_seq(sb_ctx_t* c) {
+    if (!c->seq_pending) return;
+    c->seq_pending = 0;
+    if (sb_check(c, cudaEventSynchronize((cudaEvent_t)c->seq_copy_ev[1]), "sequence boundaries")) return;
+    if (c->h_seq_pin[0] == 0 && c->h_seq_pin[c->lazy_B] == c->lazy_T) sb_set_host_seq(c, c->h_seq_pin, c->lazy_B);
+}
+// the per-token tables of the call in flight, when the call did not make them
+void sb_resolve_seq_index(sb_ctx_t* c) {
+    if (c->lazy_starts) sb_seq_index(c, c->lazy_starts, c->lazy_B, c->lazy_T, c->pos_ids, c->seq_ids);
+    c->lazy_starts = NULL;
+}
+static void attention_done(sb_ctx_t* c) { sb_resolve_host_seq(c); c->lazy_starts = NULL; }
 // single sequence of `len` rows (len may exceed T so that no row counts as "last")
 static int index_single(sb_ctx_t* c, int T, int len) {
     if (sb_ensure_tokens(c, T, 1)) return 1;
@@ -194,10 +229,11 @@ void cuda_train_batch_attention_packed(cuda_train_context_t* ctx, cuda_buffer_t*
                                        cuda_buffer_t* lse_out, cuda_buffer_t* seq_starts, int total_tokens, int batch_size,
                                        int num_heads, int kv_heads, int head_dim, int max_seq_in_batch) {
     CTX_OR_RETURN(ctx); NEED(Q, K, V, out, seq_starts);
-    if (total_tokens <= 0 || index_from_device_starts(c, (const uint32_t*)seq_starts->data, batch_size, total_tokens)) return;
+    if (total_tokens <= 0 || starts_for_attention(c, (const uint32_t*)seq_starts->data, batch_size, total_tokens)) return;
     int op = sb_prof_begin(c, "attention_packed");
     sb_attention(c, Q->data, K->data, V->data, out->data, lse_out ? lse_out->data : NULL, (const uint32_t*)seq_starts->data, c->seq_ids,
                  total_tokens, num_heads, kv_heads, head_dim);
+    attention_done(c);
     sb_prof_end(c, op, (size_t)2 * total_tokens * max_seq_in_batch * num_heads * head_dim, 0);
 }
 
@@ -288,10 +324,11 @@ void cuda_train_batch_attention_backward_packed(cuda_train_context_t* ctx, cuda_
                                                 cuda_buffer_t* seq_starts, int total_tokens, int batch_size,
                                                 int num_heads, int kv_heads, int head_dim, int max_seq_in_batch) {
     CTX_OR_RETURN(ctx); NEED(Q, K, V, attn_out, lse, grad_out, grad_Q, grad_K, grad_V, seq_starts);
-    if (total_tokens <= 0 || index_from_device_starts(c, (const uint32_t*)seq_starts->data, batch_size, total_tokens)) return;
+    if (total_tokens <= 0 || starts_for_attention(c, (const uint32_t*)seq_starts->data, batch_size, total_tokens)) return;
     int op = sb_prof_begin(c, "attention_bwd_packed");
     sb_attention_backward(c, Q->data, K->data, V->data, attn_out->data, lse->data, grad_out->data, grad_Q->data, grad_K->data,
                           grad_V->data, 1, (const uint32_t*)seq_starts->data, c->seq_ids, batch_size, total_tokens, num_heads, kv_heads, head_dim);
+    attention_done(c);
     sb_prof_end(c, op, (size_t)5 * total_tokens * max_seq_in_batch * num_heads * head_dim, 0);
 }
 void cuda_train_embedding_backward(cuda_train_context_t* ctx, cuda_buffer_t* tokens_u32, cuda_buffer_t* grad_hidden, cuda_buffer_t* grad_embed,

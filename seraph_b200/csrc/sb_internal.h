@@ -130,6 +130,9 @@ typedef struct sb_ctx {
     uint32_t *tokens, *targets, *seq_starts, *pos_ids, *seq_ids;
     int seq_cap, seq_starts_cap;
     int* h_seq; int h_seq_n, h_seq_cap;   /* host copy of the current batch's sequence starts (h_seq_n + 1 entries); 0 = unknown */
+    /* boundaries of an op-level packed attention call on their way to the host (ops.cu), and the tables it did not make yet */
+    void* seq_copy_stream; void* seq_copy_ev[2]; int* h_seq_pin; int h_seq_pin_cap; int seq_pending;
+    const uint32_t* lazy_starts; int lazy_B, lazy_T;
     int res_T, res_B, res_max_seq;   /* geometry of the batch currently resident on the device */
     float* d_loss;                   /* device scalar */
     float* d_gnorm;                  /* device scalar: sum of squares of all gradients */
@@ -139,6 +142,8 @@ typedef struct sb_ctx {
     void* scratch; size_t scratch_bytes;
     /* operand staging of the tensor-core GEMM (hi/lo, transposed copies) */
     void* gemm_stage[5]; size_t gemm_stage_bytes[5];
+    void* map_cache;                 /* encoded tensor maps (gemm_tc.cuh) */
+    const uint32_t* attn_seq_starts; /* device sequence boundaries of the attention call in flight (h_seq_n + 1 entries) */
     /* rope cos/sin table */
     float* rope_tab; int rope_tab_pos, rope_tab_hd; float rope_tab_theta;
 
@@ -246,6 +251,8 @@ void sb_copy(sb_ctx_t*, void* dst, const void* src, size_t bytes);
 
 /* host copy of the sequence boundaries of the batch the index tables describe */
 int  sb_set_host_seq(sb_ctx_t* c, const int* starts, int B);
+void sb_resolve_host_seq(sb_ctx_t* c);
+void sb_resolve_seq_index(sb_ctx_t* c);
 /* tensor-core attention (attention_tc.cu); nonzero = not eligible, caller uses the CUDA-core kernels */
 int  sb_attention_fused_forward(sb_ctx_t*, const void* q1, const void* q2, const void* k1, const void* k2, const void* v1, const void* v2,
                                 const float* amax_q, const float* amax_k, const float* amax_v, float* O, float* lse, int T, int Hq, int Hkv, int hd);
@@ -253,10 +260,6 @@ int  sb_attention_fused_scores(sb_ctx_t*, const void* q1, const void* q2, const 
                                const void* v1, const void* v2, const float* amax_q, const float* amax_k, const float* amax_v, const float* amax_do,
                                const float* ds_bound, const float* lse, const float* D, void* P1, void* P2, void* dS1, void* dS2,
                                int t0, int S, int Sp, int T, int Hq, int Hkv, int hd, int head0, int head_step, int nb);
-int  sb_attention_fused_dkv(sb_ctx_t*, const void* q1, const void* q2, const void* do1, const void* do2, const void* k1, const void* k2,
-                            const void* v1, const void* v2, const float* amax_q, const float* amax_k, const float* amax_v, const float* amax_do,
-                            const float* ds_bound, const float* lse, const float* D, void* dS1, void* dS2, float* lse_rows, float* d_rows, float* dK, float* dV,
-                            int Sp, int T, int Hq, int Hkv, int hd);     /* lse_rows, d_rows: scratch of sequences x Hq x Sp floats each */
 int  sb_attention_tc_forward(sb_ctx_t*, const float* Q, const float* K, const float* V, float* O, float* lse, int T, int Hq, int Hkv, int hd);
 int  sb_attention_tc_backward(sb_ctx_t*, const float* Q, const float* K, const float* V, const float* O, const float* lse, const float* dO,
                               float* dQ, float* dK, float* dV, int accumulate_kv, int T, int Hq, int Hkv, int hd);

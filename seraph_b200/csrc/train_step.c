@@ -681,6 +681,7 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
         sb_gemm_keep_begin(c);
         linear_fwd(c, use_lora, l, 0, a->x_norm_attn, c->W + o->q, c->head_norm ? a->q_pre : a->q, T, d, qd, 0);
         linear_fwd(c, use_lora, l, 1, a->x_norm_attn, c->W + o->k, c->head_norm ? a->k_pre : a->k, T, d, kvd, 0);
+        sb_amax_announce(c, a->v, (size_t)T * kvd);           /* nothing rewrites v before attention splits it */
         linear_fwd(c, use_lora, l, 2, a->x_norm_attn, c->W + o->v, a->v, T, d, kvd, 0);
         sb_gemm_keep_end(c);
         if (c->head_norm) {       /* learned RMSNorm over each head (rows of head_dim), before RoPE */
@@ -1211,6 +1212,10 @@ void cuda_train_free(cuda_train_context_t* ctx) {
         for (int i = 0; i < 5; i++) cudaEventDestroy((cudaEvent_t)c->side_ev[i]);
     }
     if (c->rope_tab) cudaFree(c->rope_tab);
+    free(c->map_cache);
+    if (c->seq_copy_stream) cudaStreamDestroy((cudaStream_t)c->seq_copy_stream);
+    for (int i = 0; i < 2; i++) if (c->seq_copy_ev[i]) cudaEventDestroy((cudaEvent_t)c->seq_copy_ev[i]);
+    if (c->h_seq_pin) cudaFreeHost(c->h_seq_pin);
     sb_parts_free(c);
     if (c->d_amax) cudaFree(c->d_amax);
     for (int i = 0; i < SB_F16_SLOTS; i++) if (c->f16_slot[i].h) cudaFree(c->f16_slot[i].h);

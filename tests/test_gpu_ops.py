@@ -238,6 +238,32 @@ def test_attention_head128_one_kernel_paths(ctx, ss, Hq, Hkv, flash):
     ctx.release(bq, bk, bv, bdo, bs)
 
 
+@pytest.mark.parametrize("ss,Hq,Hkv,hd", [([0, 1, 3, 66, 194, 450, 963], 4, 2, 64), (list(range(0, 301 * 7, 7)), 2, 1, 64), ([0, 61], 8, 8, 64),
+                                          ([0, 128, 256, 1280], 8, 2, 64), ([0, 5, 133, 900, 901], 4, 2, 128), ([0, 17], 2, 2, 128)])
+def test_attention_on_chip_short_and_ragged(ctx, ss, Hq, Hkv, hd):
+    """The kernels that keep scores on chip at both head sizes: sequences shorter than a tile, tile edges, more sequences than fit a kernel
+    parameter table, dK and dV added to what is there."""
+    ss = np.array(ss, np.uint32)
+    T, B = int(ss[-1]), len(ss) - 1
+    r = rng(T + Hq + hd)
+    Q, K, V = f32(r.standard_normal((T, Hq * hd))), f32(r.standard_normal((T, Hkv * hd))), f32(r.standard_normal((T, Hkv * hd)))
+    dO, dK0, dV0 = f32(r.standard_normal(Q.shape)), f32(r.standard_normal(K.shape)), f32(r.standard_normal(V.shape))
+    out_ref, lse_ref, dQ_ref, dK_ref, dV_ref = np.empty_like(Q), np.empty((T, Hq), np.float32), np.empty_like(Q), dK0.copy(), dV0.copy()
+    O.lib().ref_attention(Q, K, V, out_ref, lse_ref, ss, T, B, Hq, Hkv, hd)
+    O.lib().ref_attention_backward(Q, K, V, dO, dQ_ref, dK_ref, dV_ref, ss, T, B, Hq, Hkv, hd)
+    bq, bk, bv, bdo, bs = ctx.upload(Q), ctx.upload(K), ctx.upload(V), ctx.upload(dO), ctx.upload(ss)
+    bout, blse, bdq, bdk, bdv = ctx.zeros(Q.size), ctx.zeros(T * Hq), ctx.empty(Q.size), ctx.upload(dK0), ctx.upload(dV0)
+    n0, longest = ctx.launches(), int(np.diff(ss).max())
+    ctx.lib.cuda_train_batch_attention_packed(ctx.h, bq.b, bk.b, bv.b, bout.b, blse.b, bs.b, T, B, Hq, Hkv, hd, longest)
+    ctx.lib.cuda_train_batch_attention_backward_packed(ctx.h, bq.b, bk.b, bv.b, bout.b, blse.b, bdo.b, bdq.b, bdk.b, bdv.b, bs.b,
+                                                       T, B, Hq, Hkv, hd, longest)
+    ctx.check()
+    assert ctx.launches() - n0 <= 12
+    for got, ref in zip((bout, blse, bdq, bdk, bdv), (out_ref, lse_ref, dQ_ref, dK_ref, dV_ref)):
+        assert rel_l2(got.numpy(), ref) < TOL
+    ctx.release(bq, bk, bv, bdo, bs, bout, blse, bdq, bdk, bdv)
+
+
 def test_attention_unpacked_single_sequence(ctx):
     T, Hq, Hkv, hd = 70, 4, 4, 32
     r = rng(70)
