@@ -1,0 +1,754 @@
+// gemm_group.cu - several independent products in one persistent launch, on FP16 operand parts.
+//
+//   C_p[M,N] (+)= sum over segments s of p of  A_s[M,K_s] B_s[N,K_s]^T        p = 0 .. nprob-1
+//
+// The plain products of a training step come in groups that share operands or a destination: q, k and v; gate and up; a
+// projection's weight gradient with its input gradient; the input gradients that are summed (three for q, k, v).  As launches of their
+// own each pays for a ramp, a tail and (when its tiles do not fill the SMs) a split-K pass; a small model's step was mostly that.  Here a
+// group is one launch: the tiles of all its products are dealt together, and products that are added into one destination are
+// segments of one k loop, so their sum never leaves the accumulators.
+//
+// As in gemm_tc_kernel's prepared-FP16 form (gemm_tc.cuh), CTA pairs (cta_group::2) compute 256 x BN tiles, and accumulation in tensor memory
+// is cut every 64 k (twelve instructions) and added into registers with round-to-nearest adds.  What differs:
+//   * a stage is 64 k (one such chunk) of the hi or of the lo parts: rows of 128 bytes, whole lines, where 32 k of both asked L2 twice for each;
+//   * an operand's hi and lo parts are the third dimension of one tensor map; either operand may be K-major or MN-major, per segment, at
+//     run time;
+//   * the power-of-two scales of the two operands are applied as a chunk is added (an fma), since segments have their own;
+//   * work items are handed out at run time: one warp of the pair's leader takes the next item from a counter and passes it to the
+//     roles of both CTAs through a ring in shared memory.  Items are ordered longest first, so the schedule is a greedy one whatever the mix
+//     of products; the order of the additions inside a tile does not depend on it;
+//   * each epilogue warp sends its 32 rows out itself, 32 columns at a time, through two 4 KB buffers and tensor stores (or reductions).
+//     An SM writes about 32 bytes a cycle to L2, 4096 cycles for its half of a 256 x 256 tile; with buffers that are refilled as they drain the
+//     warps are back at the next tile's chunks after about 2900 cycles, which is what the two accumulators hide of it.  (Whole rows through
+//     one buffer of 64 rows and store warps: 4900 cycles, a stall of 1.3 us a tile.)
+// NT = 3: FP32-accurate (hi hi + lo hi + hi lo).  NT = 1: hi parts only, the 11 leading significant bits (what a TF32 instruction reads of an
+// FP32 word, at twice its rate): the reduced-precision mode.
+#include <stdio.h>
+#include "gemm_tc.cuh"
+
+#define GG_MAXP 10               // products per launch
+#define GG_MAXS 10               // segments per launch
+#define GG_MAXE (2 * GG_MAXP)    // runs of items: whole tiles, then pieces, of each product
+#define GG_RING 4                // items the slowest role may lag behind the scheduling warp
+#define GG_AHEAD 8               // k blocks left to load of an item when the next one is asked for: enough to hide the hand-over, not more, so
+                                 // that items go to the pairs that really are free first
+#define GG_THREADS 512
+#define GG_EMPTY_ARRIVALS 19     // roles that take an item: producer and 8 epilogue warps in both CTAs, the MMA warp in the leader
+
+struct __align__(64) GgSeg {
+    CUtensorMap a, b;            // parts: K-major {K, rows, part}, MN-major {rows, K, part}
+    const float *amax_a, *amax_b;
+    int K, kb;                   // kb: k blocks of 64
+    int mn;                      // bit 0: A is MN-major, bit 1: B is
+};
+struct __align__(64) GgProb {
+    CUtensorMap c;               // FP32 {N, M}, boxes of 32 columns x 32 rows, 128-byte swizzle
+    unsigned* out_amax;          // largest |C| is left here (whole tiles; the fix-up leaves it for split ones), or NULL
+    int M, N, tiles_m, tiles_n, seg0, nseg, kb, acc;
+};
+struct GgRun { int item0, prob, tile0, split, slot0; };      // items item0 .. : tiles tile0 .. of the product, `split` pieces each
+struct GgParams {
+    int nruns, items, nsegs;
+    unsigned* counter; int* status;
+    CUtensorMap partial;         // workspace of the split tiles: {BN, 256 rows per piece}, the same boxes
+    GgRun run[GG_MAXE];
+    GgProb prob[GG_MAXP];
+    GgSeg seg[GG_MAXS];
+};
+
+__device__ __forceinline__ bool gg_wait_cluster(uint64_t* bar, uint32_t parity) {      // as mbar_wait, for data written by the other CTA of the pair
+    uint32_t addr = smem_u32(bar), done = 0;
+    long long t0 = clock64();
+    for (;;) {
+        asm volatile("{\n\t.reg .pred P;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}"
+                     : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+        if (done) return true;
+        if (clock64() - t0 > TC_SPIN_CYCLES) return false;
+    }
+}
+__device__ __forceinline__ void gg_arrive_release(uint32_t bar_cluster) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
+}
+
+__device__ __forceinline__ void af_arrive_local(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+struct GgWork { int prob, m0, n0, nb0, kb0, kb1, slot; bool split; };
+template <int BN>
+__device__ __forceinline__ void gg_decode(const GgParams& p, int item, int rank, GgWork& w) {
+    int r = 0;
+    while (r + 1 < p.nruns && p.run[r + 1].item0 <= item) r++;
+    const GgRun& run = p.run[r];
+    const GgProb& pr = p.prob[run.prob];
+    const int local = item - run.item0;
+    const int t = run.split > 1 ? local / run.split : local, piece = run.split > 1 ? local % run.split : 0;
+    int mt, nt;
+    tc_raster(run.tile0 + t, pr.tiles_m, pr.tiles_n, TC_GROUP_M / 2, &mt, &nt);
+    w.prob = run.prob;
+    w.m0 = mt * 256 + rank * 128; w.n0 = nt * BN; w.nb0 = w.n0 + rank * (BN / 2);
+    w.split = run.split > 1;
+    w.slot = run.slot0 + local;
+    w.kb0 = 0; w.kb1 = pr.kb;
+    if (w.split) {
+        const int per = (pr.kb + run.split - 1) / run.split;
+        w.kb0 = min(pr.kb, piece * per); w.kb1 = min(pr.kb, w.kb0 + per);
+    }
+}
+
+template <int BN, int NT>
+struct GgShape {
+    static constexpr int NP = NT == 3 ? 2 : 1;                     // parts per operand
+    static constexpr int A_PART = 128 * 128, B_PART = (BN / 2) * 128;
+    static constexpr int STAGE = A_PART + B_PART;                  // one part of both operands
+    // A load takes about a microsecond under load: 1.5 (BN = 256) to 3 (BN = 128) chunks of MMA time ahead of the one being multiplied.  With the
+    // narrow tile six stages and two buffers per warp were 13 % slower than eight and one.
+    static constexpr int STAGES = BN == 256 ? 5 : 8;
+    static constexpr int NBUF = BN == 256 ? 2 : 1;                 // output staging: blocks of 32 rows x 32 columns per epilogue warp
+    static constexpr int STG = 8 * NBUF * 4096;
+    static constexpr int SMEM = STAGES * STAGE + STG + 1024 + 512;
+};
+
+template <int BN, int NT>
+__global__ void __launch_bounds__(GG_THREADS, 1)
+gg_kernel(const __grid_constant__ GgParams p) {
+    using Sh = GgShape<BN, NT>;
+    constexpr int NP = Sh::NP, A_PART = Sh::A_PART, STAGE = Sh::STAGE, STAGES = Sh::STAGES;
+    constexpr uint32_t TMEM_COLS = 2 * BN;
+    constexpr int COLS = BN / 2;                                   // columns per epilogue thread
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* stg = smem + STAGES * STAGE;
+    uint64_t* full = (uint64_t*)(stg + Sh::STG);
+    uint64_t* empty = full + STAGES;
+    uint64_t* acc_full = empty + STAGES;          // [2]
+    uint64_t* acc_empty = acc_full + 2;           // [2]
+    uint64_t* item_full = acc_empty + 2;          // [GG_RING]
+    uint64_t* item_empty = item_full + GG_RING;   // [GG_RING] (the leader's are used)
+    uint64_t* item_req = item_empty + GG_RING;    // 1: the leader's producer asks for the next item
+    int* item_slot = (int*)(item_req + 1);
+    uint32_t* tmem_slot = (uint32_t*)(item_slot + GG_RING);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();
+    const bool leader = rank == 0;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int b = 0; b < 2; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }
+        mbar_init(item_req, 1);
+        for (int b = 0; b < GG_RING; b++) { mbar_init(&item_full[b], 1); mbar_init(&item_empty[b], GG_EMPTY_ARRIVALS); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 3 && lane < p.nsegs) {            // the tensor maps on their way to the cache
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&p.seg[lane].a) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&p.seg[lane].b) : "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();                           // the peer's barriers exist before anything signals them
+    sb_pdl_enter();                               // up to here nothing was read that the kernel before may still write
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    bool ok = true;
+    // the n-th item of this CTA's roles: the first is the pair's number, the others are waited for, read, and their slot handed back; -1 after the last
+    auto next_item = [&](int n, bool arrive) -> int {
+        if (n == 0) return (int)(blockIdx.x >> 1);
+        const int s = (n - 1) % GG_RING;
+        if (!gg_wait_cluster(&item_full[s], ((n - 1) / GG_RING) & 1)) { ok = false; return -1; }
+        const int item = *(volatile int*)&item_slot[s];
+        __syncwarp(__activemask());
+        if (arrive) gg_arrive_release(mapa_u32(smem_u32(&item_empty[s]), 0));
+        return item;
+    };
+
+    const bool is_epi = warp >= 4 && warp < 12;
+    if (!is_epi) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REGS_LIGHT));
+        if (warp == 0) {
+            // ---------------- TMA producer ----------------
+            if (elect_one()) {
+                uint32_t git = 0;
+                for (int n = 0; ok; n++) {
+                    const int item = next_item(n, true);
+                    if (item < 0) break;
+                    GgWork w;
+                    gg_decode<BN>(p, item, (int)rank, w);
+                    const GgProb& pr = p.prob[w.prob];
+                    int off = 0, left = w.kb1 - w.kb0;
+                    const int ask = min(left, GG_AHEAD);
+                    if (left == 0 && leader) af_arrive_local(item_req);
+                    for (int sg = pr.seg0; sg < pr.seg0 + pr.nseg && ok; sg++) {
+                        const GgSeg& g = p.seg[sg];
+                        const int lo = max(w.kb0, off) - off, hi = min(w.kb1, off + g.kb) - off;
+                        off += g.kb;
+                        const bool amn = (g.mn & 1) != 0, bmn = (g.mn & 2) != 0;
+                        for (int kb = lo; kb < hi && ok; kb++) {
+                            if (left-- == ask && leader) af_arrive_local(item_req);
+                            for (int part = 0; part < NP; part++, git++) {
+                                const int s = git % STAGES;
+                                ok = mbar_wait(&empty[s], ((git / STAGES) & 1) ^ 1);
+                                if (!ok) break;
+                                uint8_t* st = smem + s * STAGE;
+                                if (leader) mbar_expect_tx(&full[s], STAGE * 2);      // both CTAs' bytes land on the leader's barrier
+                                const uint32_t fb = mapa_u32(smem_u32(&full[s]), 0);
+                                if (amn) {
+#pragma unroll
+                                    for (int j = 0; j < 2; j++) tma_load_3d_pair(st + j * 8192, &g.a, fb, w.m0 + 64 * j, kb * 64, part);
+                                } else tma_load_3d_pair(st, &g.a, fb, kb * 64, w.m0, part);
+                                if (bmn) {
+#pragma unroll
+                                    for (int j = 0; j < BN / 128; j++) tma_load_3d_pair(st + A_PART + j * 8192, &g.b, fb, w.nb0 + 64 * j, kb * 64, part);
+                                } else tma_load_3d_pair(st + A_PART, &g.b, fb, kb * 64, w.nb0, part);
+                            }
+                        }
+                    }
+                }
+                if (!ok) atomicExch(p.status, SB_ERR_TIMEOUT);
+            }
+        } else if (warp == 1) {
+            // ---------------- MMA issuer ----------------
+            if (leader && elect_one()) {
+                uint32_t git = 0, gch = 0;
+                for (int n = 0; ok; n++) {
+                    const int item = next_item(n, true);
+                    if (item < 0) break;
+                    GgWork w;
+                    gg_decode<BN>(p, item, 0, w);
+                    const GgProb& pr = p.prob[w.prob];
+                    int off = 0;
+                    for (int sg = pr.seg0; sg < pr.seg0 + pr.nseg && ok; sg++) {
+                        const GgSeg& g = p.seg[sg];
+                        const int lo = max(w.kb0, off) - off, hi = min(w.kb1, off + g.kb) - off;
+                        off += g.kb;
+                        const bool amn = (g.mn & 1) != 0, bmn = (g.mn & 2) != 0;
+                        const uint32_t idesc = (1u << 4) | ((amn ? 1u : 0u) << 15) | ((bmn ? 1u : 0u) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+                        const uint64_t adva = amn ? 128 : 2, advb = bmn ? 128 : 2;      // 16 k in 16-byte units
+                        for (int kb = lo; kb < hi && ok; kb++, git += NP, gch++) {
+                            const int buf = gch & 1, s = git % STAGES, s2 = (git + 1) % STAGES;
+                            ok = mbar_wait(&acc_empty[buf], ((gch >> 1) & 1) ^ 1) && mbar_wait(&full[s], (git / STAGES) & 1);
+                            if (!ok) break;
+                            tc_fence_after();
+                            const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BN);
+                            const uint32_t sa = smem_u32(smem + s * STAGE), sb = sa + A_PART;
+                            const uint64_t a1 = amn ? make_mn16_desc<64>(sa) : make_kmajor_desc<128>(sa);
+                            const uint64_t b1 = bmn ? make_mn16_desc<64>(sb) : make_kmajor_desc<128>(sb);
+                            const int nkk = min(4, (g.K - kb * 64 + 15) >> 4);      // the rest of a short last block is zeros
+                            if (NT == 3) {
+                                // consecutive instructions share an operand (hi hi, lo hi, hi lo): with the narrow tile, whose operand reads take as long
+                                // as its arithmetic, all of hi hi first was 40 % slower
+                                ok = mbar_wait(&full[s2], ((git + 1) / STAGES) & 1);
+                                if (!ok) break;
+                                tc_fence_after();
+                                const uint64_t a2 = a1 + (uint64_t)((s2 - s) * (STAGE >> 4)), b2 = b1 + (uint64_t)((s2 - s) * (STAGE >> 4));
+                                for (int kk = 0; kk < nkk; kk++) {
+                                    tc_mma_f16_pair(tmem_d, a1 + kk * adva, b1 + kk * advb, idesc, kk ? 1u : 0u);
+                                    tc_mma_f16_pair(tmem_d, a2 + kk * adva, b1 + kk * advb, idesc, 1);
+                                    tc_mma_f16_pair(tmem_d, a1 + kk * adva, b2 + kk * advb, idesc, 1);
+                                }
+                            } else {
+                                for (int kk = 0; kk < nkk; kk++) tc_mma_f16_pair(tmem_d, a1 + kk * adva, b1 + kk * advb, idesc, kk ? 1u : 0u);
+                            }
+                            tc_commit_pair(&empty[s]);
+                            if (NT == 3) tc_commit_pair(&empty[s2]);
+                            tc_commit_pair(&acc_full[buf]);
+                        }
+                    }
+                }
+                if (!ok) atomicExch(p.status, SB_ERR_TIMEOUT);
+            }
+        } else if (warp == 2) {
+            // ---------------- scheduler: hands the next item to the roles of both CTAs ----------------
+            if (leader && elect_one()) {
+                const int G = gridDim.x / 2;
+                const uint32_t slot1 = mapa_u32(smem_u32(item_slot), 1), full1 = mapa_u32(smem_u32(item_full), 1), full0 = mapa_u32(smem_u32(item_full), 0);
+                for (int n = 0; ok; n++) {
+                    const int s = n % GG_RING;
+                    ok = mbar_wait(item_req, n & 1) && gg_wait_cluster(&item_empty[s], ((n / GG_RING) & 1) ^ 1);
+                    if (!ok) break;
+                    const int item = G + (int)atomicAdd(p.counter, 1u);
+                    const int v = item < p.items ? item : -1;
+                    *(volatile int*)&item_slot[s] = v;
+                    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(slot1 + (uint32_t)(s * 4)), "r"(v) : "memory");
+                    gg_arrive_release(full0 + (uint32_t)(s * 8));
+                    gg_arrive_release(full1 + (uint32_t)(s * 8));
+                    if (v < 0) break;
+                }
+                if (!ok) atomicExch(p.status, SB_ERR_TIMEOUT);
+            }
+        }
+    } else {
+        // ---------------- epilogue: chunks from tensor memory, scaled, into register accumulators; tiles to the staging buffer ----------------
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TC_REGS_EPI));
+        const int q = warp & 3, col0 = ((warp - 4) >> 2) * COLS;
+        const uint32_t sbuf = smem_u32(stg + (warp - 4) * Sh::NBUF * 4096);
+        uint32_t gch = 0, pieces = 0;
+        for (int n = 0; ok; n++) {
+            const int item = next_item(n, lane == 0);
+            if (item < 0) break;
+            GgWork w;
+            gg_decode<BN>(p, item, (int)rank, w);
+            const GgProb& pr = p.prob[w.prob];
+            float accr[COLS];
+#pragma unroll
+            for (int j = 0; j < COLS; j++) accr[j] = 0.f;
+            int off = 0;
+            for (int sg = pr.seg0; sg < pr.seg0 + pr.nseg && ok; sg++) {
+                const GgSeg& g = p.seg[sg];
+                const int lo = max(w.kb0, off) - off, hi = min(w.kb1, off + g.kb) - off;
+                off += g.kb;
+                if (lo >= hi) continue;
+                // undo the operands' power-of-two scales; their product may leave the float range, then it takes two multiplications
+                const int e = -tc_f16_shift(sb_word(g.amax_a)) - tc_f16_shift(sb_word(g.amax_b));
+                const bool far = e < -120 || e > 120;
+                const float s1 = far ? tc_pow2(e / 2) : tc_pow2(e), s2 = far ? tc_pow2(e - e / 2) : 1.f;
+                for (int kb = lo; kb < hi && ok; kb++, gch++) {
+                    const int buf = gch & 1;
+                    ok = mbar_wait(&acc_full[buf], (gch >> 1) & 1);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + col0);
+#pragma unroll
+                    for (int gi = 0; gi < COLS / 32; gi++) {
+                        uint32_t r[32];
+                        tc_ld32(taddr + (uint32_t)(gi * 32), r);
+                        if (gi == COLS / 32 - 1) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[buf]), 0));
+                        }
+                        if (!far) {
+#pragma unroll
+                            for (int j = 0; j < 32; j++) accr[gi * 32 + j] = fmaf(__uint_as_float(r[j]), s1, accr[gi * 32 + j]);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; j++) accr[gi * 32 + j] += __uint_as_float(r[j]) * s1 * s2;
+                        }
+                    }
+                }
+            }
+            if (pr.out_amax && !w.split) {
+                float m = 0.f;
+#pragma unroll
+                for (int j = 0; j < COLS; j++) m = fmaxf(m, fabsf(accr[j]));
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+                if (lane == 0 && m > 0.f) atomicMax(pr.out_amax, __float_as_uint(m));
+            }
+            if (!ok) break;
+            const CUtensorMap* map = w.split ? &p.partial : &pr.c;
+            const int x0 = (w.split ? 0 : w.n0) + col0, y0 = (w.split ? (w.slot * 2 + (int)rank) * 128 : w.m0) + q * 32;
+            const bool inside = w.split || y0 < pr.M, accf = !w.split && pr.acc;
+#pragma unroll
+            for (int g = 0; g < COLS / 32; g++, pieces++) {
+                if (!inside || !(w.split || x0 + g * 32 < pr.N)) continue;
+                const uint32_t buf = sbuf + (pieces % Sh::NBUF) * 4096;
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(Sh::NBUF - 1) : "memory");      // what was staged here before has been read
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (uint32_t)(lane * 128 + ((i ^ (lane & 7)) << 4))),
+                                 "f"(accr[g * 32 + 4 * i]), "f"(accr[g * 32 + 4 * i + 1]), "f"(accr[g * 32 + 4 * i + 2]), "f"(accr[g * 32 + 4 * i + 3]) : "memory");
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    if (accf) asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x0 + g * 32), "r"(y0), "r"(buf) : "memory");
+                    else      asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x0 + g * 32), "r"(y0), "r"(buf) : "memory");
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
+            }
+        }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the buffers are read out before the CTA gives its shared memory back
+        if (!ok && lane == 0) atomicExch(p.status, SB_ERR_TIMEOUT);
+        tc_fence_before();
+    }
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");      // neither CTA leaves while the other may still signal it or read its operands
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
+    }
+}
+
+// Adds the pieces of the split tiles into C in piece order: one thread per four columns of one row, all products of the launch.
+struct GgFixRun { float* C; long ldc; unsigned* out_amax; int M, N, tiles_m, tiles_n, acc, tile0, split, slot0, block0; };
+struct GgFixParams { int n, blocks, bn; const float* partial; GgFixRun f[GG_MAXP]; };
+static __global__ void __launch_bounds__(256) gg_fixup_kernel(const __grid_constant__ GgFixParams p) {
+    sb_pdl_enter();
+    const int bn4 = p.bn >> 2;
+    const long item = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int blk = (int)(item / (128 * bn4)), i = (int)(item % (128 * bn4));
+    if (blk >= p.blocks) return;
+    int k = 0;
+    while (k + 1 < p.n && p.f[k + 1].block0 <= blk) k++;
+    const GgFixRun& f = p.f[k];
+    const int t = (blk - f.block0) >> 1, rank = (blk - f.block0) & 1;
+    int mt, nt;
+    tc_raster(f.tile0 + t, f.tiles_m, f.tiles_n, TC_GROUP_M / 2, &mt, &nt);
+    const int r = i / bn4, col = (i % bn4) * 4;
+    const int row = mt * 256 + rank * 128 + r, c0 = nt * p.bn + col;
+    if (row >= f.M || c0 >= f.N) return;                        // N is a multiple of 4: a group of columns is inside or outside
+    const size_t block = (size_t)128 * p.bn;
+    const float* p0 = p.partial + ((size_t)(f.slot0 + t * f.split) * 2 + rank) * block + (size_t)r * p.bn + col;
+    float4* cp = (float4*)(f.C + (size_t)row * f.ldc + c0);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (f.acc) v = *cp;
+    float4 o[8];
+#pragma unroll
+    for (int s = 0; s < 8; s++) if (s < f.split) o[s] = __ldcg((const float4*)(p0 + (size_t)s * 2 * block));
+#pragma unroll
+    for (int s = 0; s < 8; s++) if (s < f.split) { v.x += o[s].x; v.y += o[s].y; v.z += o[s].z; v.w += o[s].w; }
+    *cp = v;
+    if (f.out_amax) {
+        const float m = sb_amax4(0.f, v);
+        const unsigned live = __activemask();
+        const unsigned wm = __reduce_max_sync(live, __float_as_uint(m));
+        if ((int)(threadIdx.x & 31) == __ffs(live) - 1 && wm != 0u) atomicMax(f.out_amax, wm);
+    }
+}
+
+// --------------------------------------------------------------------------- the schedule of a group
+// Whole tiles of 256 x 256 or 256 x 128, the last of them cut into pieces of the k range when that shortens the launch.  The cost of an item is
+// its k blocks plus an epilogue that the next item's first two chunks hide part of; a launch is the greedy schedule of its items on the CTA
+// pairs.  The constants (microseconds per k block of 64 at BN = 256 and 128, per epilogue, for the fix-up launch) are measured.
+struct GgPlanRun { int prob, tile0, tiles, split; };
+struct GgPlan { int bn, nruns; GgPlanRun run[GG_MAXE]; };
+struct GgPlanKey { int nprob, nt, G; int mnk[GG_MAXP][3]; };
+struct GgPlanEntry { GgPlanKey key; GgPlan plan; bool valid; };
+#define GG_PLANS 128
+
+static const float gg_t_kb[2][2] = {{0.95f, 0.50f}, {0.36f, 0.25f}}, gg_t_epi[2] = {4.0f, 2.4f}, gg_t_fix = 3.5f;      // [nt == 1][bn == 128]
+
+struct GgSim { float t[64]; int c[64]; int n; };
+// `count` items of one cost, each to the pair that is free first
+static void gg_sim_add(GgSim* s, int count, float cost) {
+    while (count > 0) {
+        int lo = 0;
+        for (int i = 1; i < s->n; i++) if (s->t[i] < s->t[lo]) lo = i;
+        const int a = count < s->c[lo] ? count : s->c[lo];
+        const float nt = s->t[lo] + cost;
+        count -= a; s->c[lo] -= a;
+        int hit = -1;
+        for (int i = 0; i < s->n; i++) if (s->t[i] == nt || (s->n >= 60 && s->t[i] > nt - 0.5f * cost && s->t[i] < nt + 0.5f * cost)) { hit = i; break; }
+        if (hit >= 0) s->c[hit] += a;
+        else if (s->c[lo] == 0) { s->t[lo] = nt; s->c[lo] = a; continue; }
+        else { s->t[s->n] = nt; s->c[s->n] = a; s->n++; }
+        if (s->c[lo] == 0) { s->n--; s->t[lo] = s->t[s->n]; s->c[lo] = s->c[s->n]; }
+    }
+}
+static int gg_tiles(const int* mnk, int bn) { return ((mnk[0] + 255) / 256) * ((mnk[1] + bn - 1) / bn); }
+static void gg_make_plan(const GgPlanKey* k, GgPlan* best) {
+    float best_t = 0.f;
+    best->nruns = 0;
+    for (int wide = 1; wide >= 0; wide--) {
+        const int bn = wide ? 256 : 128;
+        const float tk = gg_t_kb[k->nt == 1][!wide], te = gg_t_epi[!wide];
+        int order[GG_MAXP], total = 0;
+        for (int i = 0; i < k->nprob; i++) {
+            int j = i;
+            for (; j > 0 && k->mnk[order[j - 1]][2] < k->mnk[i][2]; j--) order[j] = order[j - 1];
+            order[j] = i;
+            total += gg_tiles(k->mnk[i], bn);
+        }
+        // what is cut: nothing; the last `cut` tiles of the last products into s pieces; or everything into pieces of at most q k blocks
+        for (int kind = 0; kind < 12; kind++) {
+            GgPlan p;
+            p.bn = bn; p.nruns = 0;
+            GgPlanRun pieces[GG_MAXP]; int np = 0;
+            int cut_left = 0, s_tail = 1, q = 0;
+            if (kind >= 1 && kind <= 6) {
+                static const int ss[6] = {2, 3, 4, 5, 6, 8};
+                s_tail = ss[kind - 1];
+                cut_left = total % k->G;
+                if (cut_left == 0) continue;
+            } else if (kind > 6) {
+                static const int qs[5] = {3, 5, 8, 12, 20};
+                q = qs[kind - 7];
+                if (total >= k->G) continue;
+            }
+            // the tail is taken from the products with the shortest k, last in the order
+            int cut[GG_MAXP], spl[GG_MAXP];
+            for (int i = 0; i < k->nprob; i++) { cut[i] = 0; spl[i] = 1; }
+            bool any = false, bad = false;
+            for (int o = k->nprob - 1; o >= 0; o--) {
+                const int i = order[o], t = gg_tiles(k->mnk[i], bn), kb = k->mnk[i][2];
+                int s = s_tail;
+                if (q) { s = (kb + q - 1) / q; if (s > 8) s = 8; }
+                const int per = (kb + s - 1) / s;
+                if (s > 1 && (per * (s - 1) >= kb || per < 2)) { if (q) { s = 1; } else if (cut_left > 0) { bad = true; break; } }
+                if (q) { if (s > 1) { cut[i] = t; spl[i] = s; any = true; } }
+                else if (cut_left > 0 && s > 1) { cut[i] = t < cut_left ? t : cut_left; spl[i] = s; cut_left -= cut[i]; any = true; }
+            }
+            if (bad || (kind > 0 && !any)) continue;
+            GgSim sim;
+            sim.n = 1; sim.t[0] = 0.f; sim.c[0] = k->G;
+            for (int o = 0; o < k->nprob; o++) {
+                const int i = order[o], t = gg_tiles(k->mnk[i], bn), kb = k->mnk[i][2];
+                if (t > cut[i]) {
+                    p.run[p.nruns++] = {i, 0, t - cut[i], 1};
+                    gg_sim_add(&sim, t - cut[i], kb * tk + te);
+                }
+                if (cut[i]) pieces[np++] = {i, t - cut[i], cut[i], spl[i]};
+            }
+            for (int a = 1; a < np; a++)                         // longest pieces first
+                for (int b = a; b > 0; b--) {
+                    const int ka = (k->mnk[pieces[b].prob][2] + pieces[b].split - 1) / pieces[b].split, kp = (k->mnk[pieces[b - 1].prob][2] + pieces[b - 1].split - 1) / pieces[b - 1].split;
+                    if (ka > kp) { GgPlanRun x = pieces[b]; pieces[b] = pieces[b - 1]; pieces[b - 1] = x; } else break;
+                }
+            for (int a = 0; a < np; a++) {
+                const int kb = k->mnk[pieces[a].prob][2], per = (kb + pieces[a].split - 1) / pieces[a].split;
+                p.run[p.nruns++] = pieces[a];
+                gg_sim_add(&sim, pieces[a].tiles * pieces[a].split, per * tk + te);
+            }
+            float t = 0.f;
+            for (int i = 0; i < sim.n; i++) if (sim.t[i] > t) t = sim.t[i];
+            if (np) t = (t + gg_t_fix) * 1.03f;
+            if (best->nruns == 0 || t < best_t) { *best = p; best_t = t; }
+        }
+    }
+}
+static const GgPlan* gg_plan(sb_ctx_t* c, const GgPlanKey* key) {
+    if (!c->gg_plans) c->gg_plans = calloc(GG_PLANS + 1, sizeof(GgPlanEntry));
+    if (!c->gg_plans) return nullptr;
+    uint64_t h = 1469598103934665603ull;
+    const int* w = (const int*)key;
+    for (size_t i = 0; i < sizeof *key / sizeof(int); i++) { h ^= (uint64_t)(uint32_t)w[i]; h *= 0x9E3779B97F4A7C15ull; h ^= h >> 29; }
+    GgPlanEntry* e = (GgPlanEntry*)c->gg_plans + h % GG_PLANS;
+    if (!e->valid || memcmp(&e->key, key, sizeof *key) != 0) { gg_make_plan(key, &e->plan); e->key = *key; e->valid = true; }
+    return &e->plan;
+}
+
+template <int BN, int NT>
+static bool gg_launch_t(sb_ctx_t* c, const GgParams& p, int G) {
+    auto kern = gg_kernel<BN, NT>;
+    constexpr int smem = GgShape<BN, NT>::SMEM;
+    static_assert(smem <= 232448, "shared memory of one CTA");
+    static bool attr_set = false;
+    if (!attr_set) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return false;
+        attr_set = true;
+    }
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDim = dim3((unsigned)(2 * G)); cfg.blockDim = dim3(GG_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = (cudaStream_t)c->pub.stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 2;
+    c->launches++;
+    return cudaLaunchKernelEx(&cfg, kern, p) == cudaSuccess;
+}
+
+// --------------------------------------------------------------------------- host side
+bool gg_shape_ok(int M, int N, int K, int tA, int tB) {
+    if (M < 8 || N < 16 || K < 8 || (N & 3) || (double)M * N * K < (double)(1 << 19)) return false;      // smaller: the CUDA-core kernel
+    if (tA && tB) tA = tB = 0;
+    return (tA ? (M & 7) == 0 : (K & 7) == 0) && (tB ? (K & 7) == 0 : (N & 7) == 0);
+}
+static bool gg_mode(const sb_ctx_t* c, int* nt) {
+    const int mode = c->pub.use_bf16 ? SB_GEMM_BF16 : c->gemm_mode;
+    *nt = mode == SB_GEMM_BF16 ? 1 : 3;
+    return c->gemm_pair && (mode == SB_GEMM_FP16X3 || mode == SB_GEMM_BF16) && tc_load_encode();
+}
+extern "C" int sb_gemm_group_takes(sb_ctx_t* c, int M, int N, int K, int tA, int tB) {
+    int nt;
+    return gg_mode(c, &nt) && gg_shape_ok(M, N, K, tA, tB) ? 1 : 0;
+}
+
+struct GgOperand { const float* x; size_t n; __half* h; float* amax; bool fresh; int slot; };
+// the parts of an operand: those a producer or an earlier product of the step left, or a slot to make them in
+static int gg_operand(sb_ctx_t* c, GgOperand* ops, int* nops, const float* x, size_t n) {
+    for (int i = 0; i < *nops; i++) if (ops[i].x == x && ops[i].n == n) return i;
+    GgOperand* o = &ops[*nops];
+    o->x = x; o->n = n; o->slot = -1;
+    void* h; int fresh;
+    if (sb_parts_find(c, x, n, &h, &o->amax, &fresh)) { o->h = (__half*)h; o->fresh = fresh != 0; }
+    else {
+        bool fr;
+        const int s = sb_f16_slot(c, x, n, -1, &fr);
+        if (s < 0) return -1;
+        o->h = (__half*)c->f16_slot[s].h; o->fresh = fr; o->slot = s;
+        if (fr) c->f16_slot[s].amax = c->d_amax + s;
+        o->amax = c->f16_slot[s].amax;
+    }
+    return (*nops)++;
+}
+// Parts of the operands that have none yet: one maximum launch for those whose producer left none, one split launch.  Large ones in runs that
+// fit L2, so that the split finds what the maximum pass read.
+static void gg_prepare(sb_ctx_t* c, GgOperand* ops, int n) {
+    cudaStream_t st = (cudaStream_t)c->pub.stream;
+    TcMulti am, sp;
+    am.n = sp.n = 0; am.chunks = sp.chunks = 0;
+    double bytes = 0;
+    int tk = -1;
+    bool any = false;
+    for (int i = 0; i < n; i++) {
+        GgOperand* o = &ops[i];
+        if (o->fresh) {
+            if (!any) { tk = sb_tick_begin(c, SB_CLS_GEMM_PREP); any = true; }
+            float* left = sb_amax_lookup(c, o->x, o->n);
+            if (left) {
+                o->amax = left;
+                if (o->slot >= 0) c->f16_slot[o->slot].amax = left; else sb_parts_set_amax(c, o->x, left);
+            } else {
+                float* word = sb_zero_word(c);                  // zero already; outside a step the operand's own word
+                if (word) { o->amax = word; if (o->slot >= 0) c->f16_slot[o->slot].amax = word; else sb_parts_set_amax(c, o->x, word); }
+                else cudaMemsetAsync(o->amax, 0, sizeof(float), st);
+                tc_multi_add(&am, o->x, o->n, nullptr, o->amax);
+                bytes += 4.0 * o->n;
+            }
+            tc_multi_add(&sp, o->x, o->n, o->h, o->amax);
+            bytes += 8.0 * o->n;
+        }
+        if (sp.n == TC_MULTI || (sp.n && (i + 1 == n || (size_t)(am.chunks + sp.chunks) * TC_MULTI_CHUNK * 16 > ((size_t)64 << 20)))) {
+            tc_multi_amax(c, am);
+            tc_multi_split(c, sp);
+            am.n = sp.n = 0; am.chunks = sp.chunks = 0;
+        }
+    }
+    if (any) sb_tick_end(c, tk, 0.0, bytes);
+}
+// Parts of registered tensors (weights) ahead of the products that read them: one pair of launches instead of one or two per tensor
+extern "C" void sb_parts_prepare(sb_ctx_t* c, const float* const* x, const size_t* n, int count) {
+    GgOperand ops[TC_MULTI];
+    for (int i0 = 0; i0 < count; ) {
+        int k = 0;
+        for (; i0 < count && k < TC_MULTI; i0++) {
+            void* h; int fresh;
+            if (!sb_parts_find(c, x[i0], n[i0], &h, &ops[k].amax, &fresh)) return;      // no arena: every product prepares its own operands
+            ops[k].x = x[i0]; ops[k].n = n[i0]; ops[k].h = (__half*)h; ops[k].fresh = fresh != 0; ops[k].slot = -1;
+            k++;
+        }
+        gg_prepare(c, ops, k);
+    }
+}
+
+static bool gg_map(sb_ctx_t* c, CUtensorMap* m, const __half* h, size_t n, int rows, int K, bool mn, int box_rows) {
+    // parts are n halfs apart; K-major [rows, K]: {K, rows, part}; MN-major [K, rows]: {rows, K, part}
+    const cuuint64_t dims[3] = {(cuuint64_t)(mn ? rows : K), (cuuint64_t)(mn ? K : rows), 2};
+    const cuuint64_t strides[2] = {(cuuint64_t)(mn ? rows : K) * 2, (cuuint64_t)n * 2};
+    const cuuint32_t box[3] = {64u, mn ? 64u : (cuuint32_t)box_rows, 1u};
+    return tc_encode(c, m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, h, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+static bool gg_map_out(sb_ctx_t* c, CUtensorMap* m, const float* C, int M, int N) {
+    const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M}, strides[1] = {(cuuint64_t)N * 4};
+    const cuuint32_t box[2] = {32u, 32u};
+    return tc_encode(c, m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, C, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+}
+
+// one launch (and the fix-up pass of its split tiles); jobs with the same destination as the one before are its further segments
+static bool gg_run(sb_ctx_t* c, const sb_gemm_job_t* jobs, int njobs, int nt) {
+    GgOperand ops[2 * GG_MAXS];
+    int nops = 0, ia[GG_MAXS], ib[GG_MAXS];
+    for (int j = 0; j < njobs; j++) {
+        ia[j] = gg_operand(c, ops, &nops, jobs[j].A, (size_t)jobs[j].M * jobs[j].K);
+        ib[j] = gg_operand(c, ops, &nops, jobs[j].B, (size_t)jobs[j].N * jobs[j].K);
+        if (ia[j] < 0 || ib[j] < 0) return false;
+    }
+    gg_prepare(c, ops, nops);
+    GgParams p;
+    memset(&p, 0, sizeof p);
+    GgPlanKey key;
+    memset(&key, 0, sizeof key);
+    int np = 0;
+    double flops = 0, bytes = 0;
+    for (int j = 0; j < njobs; j++) {
+        const sb_gemm_job_t* b = &jobs[j];
+        const bool more = j > 0 && b->C == jobs[j - 1].C && b->acc;
+        flops += 2.0 * b->M * b->N * b->K;
+        bytes += 4.0 * ((double)b->M * b->K + (double)b->N * b->K + (more ? 0.0 : (double)b->M * b->N * (b->acc ? 2 : 1)));
+        if (!more) {
+            GgProb* q = &p.prob[np++];
+            q->M = b->M; q->N = b->N; q->seg0 = j; q->nseg = 0; q->kb = 0; q->acc = b->acc;
+        }
+        GgProb* q = &p.prob[np - 1];
+        p.seg[j].K = b->K; p.seg[j].kb = (b->K + 63) / 64;
+        q->nseg++; q->kb += p.seg[j].kb;
+    }
+    const int sms = c->pub.gpu_sm_count > 0 ? c->pub.gpu_sm_count : 148;
+    key.nprob = np; key.nt = nt; key.G = max(1, (sms - (c->gemm_reserve_sms < sms ? c->gemm_reserve_sms : 0)) / 2);
+    for (int i = 0; i < np; i++) { key.mnk[i][0] = p.prob[i].M; key.mnk[i][1] = p.prob[i].N; key.mnk[i][2] = p.prob[i].kb; }
+    const GgPlan* plan = gg_plan(c, &key);
+    if (!plan) return false;
+    const int bn = plan->bn;
+    for (int j = 0; j < njobs; j++) {
+        const sb_gemm_job_t* b = &jobs[j];
+        int tA = b->tA, tB = b->tB;
+        if (tA && tB) tA = tB = 0;
+        const GgOperand *oa = &ops[ia[j]], *ob = &ops[ib[j]];
+        p.seg[j].mn = (tA ? 1 : 0) | (tB ? 0 : 2);
+        p.seg[j].amax_a = oa->amax; p.seg[j].amax_b = ob->amax;
+        if (!gg_map(c, &p.seg[j].a, oa->h, oa->n, b->M, b->K, tA != 0, 128) ||
+            !gg_map(c, &p.seg[j].b, ob->h, ob->n, b->N, b->K, !tB, bn / 2)) return false;
+    }
+    GgFixParams fx;
+    fx.n = fx.blocks = 0; fx.bn = bn;
+    int slots = 0;
+    for (int i = 0; i < np; i++) {
+        GgProb* q = &p.prob[i];
+        q->tiles_m = (q->M + 255) / 256; q->tiles_n = (q->N + bn - 1) / bn;
+        float* C = jobs[q->seg0].C;
+        if (!q->acc) q->out_amax = sb_amax_take(c, C, (size_t)q->M * q->N);      // an announced output: the epilogue leaves max |C|
+        if (!gg_map_out(c, &q->c, C, q->M, q->N)) return false;
+    }
+    for (int r = 0; r < plan->nruns; r++) {
+        const GgPlanRun* pr = &plan->run[r];
+        GgProb* q = &p.prob[pr->prob];
+        p.run[r].item0 = p.items; p.run[r].prob = pr->prob; p.run[r].tile0 = pr->tile0; p.run[r].split = pr->split; p.run[r].slot0 = slots;
+        p.items += pr->tiles * pr->split;
+        if (pr->split > 1) {
+            GgFixRun* f = &fx.f[fx.n++];
+            f->C = jobs[q->seg0].C; f->ldc = q->N; f->out_amax = q->out_amax; f->M = q->M; f->N = q->N; f->tiles_m = q->tiles_m; f->tiles_n = q->tiles_n;
+            f->acc = q->acc; f->tile0 = pr->tile0; f->split = pr->split; f->slot0 = slots; f->block0 = fx.blocks;
+            fx.blocks += pr->tiles * 2;
+            slots += pr->tiles * pr->split;
+        }
+    }
+    p.nruns = plan->nruns; p.nsegs = njobs;
+    float* partial = nullptr;
+    if (slots) {
+        partial = (float*)sb_gemm_stage(c, 4, (size_t)slots * 2 * 128 * bn * sizeof(float));
+        if (!partial || !gg_map_out(c, &p.partial, partial, slots * 256, bn)) return false;
+    }
+    p.counter = sb_item_counter(c);
+    if (!p.counter) return false;
+    p.status = c->d_status;
+    int tg = sb_tick_begin(c, SB_CLS_GEMM);
+    const int G = p.items < key.G ? p.items : key.G;
+    bool ok = bn == 256 ? (nt == 3 ? gg_launch_t<256, 3>(c, p, G) : gg_launch_t<256, 1>(c, p, G))
+                        : (nt == 3 ? gg_launch_t<128, 3>(c, p, G) : gg_launch_t<128, 1>(c, p, G));
+    if (ok && fx.blocks) {
+        fx.partial = partial;
+        const long items = (long)fx.blocks * 128 * (bn / 4);
+        sb_launch(gg_fixup_kernel, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, (cudaStream_t)c->pub.stream, fx);
+        c->launches++;
+    }
+    sb_tick_end(c, tg, flops, bytes);
+    return ok && cudaGetLastError() == cudaSuccess;
+}
+
+// Returns 0 when the products were launched, 1 when some are not for this kernel (nothing has been launched then).
+extern "C" int sb_gemm_group_try(sb_ctx_t* c, const sb_gemm_job_t* jobs, int njobs) {
+    int nt;
+    if (njobs <= 0 || !gg_mode(c, &nt)) return 1;
+    for (int j = 0; j < njobs; j++)
+        if (!gg_shape_ok(jobs[j].M, jobs[j].N, jobs[j].K, jobs[j].tA, jobs[j].tB) || !tc_aligned16(jobs[j].A) || !tc_aligned16(jobs[j].B) || !tc_aligned16(jobs[j].C)) return 1;
+    const int keep = c->f16_keep;
+    if (!keep) c->f16_keep = 1;                                   // operands of one group never share a slot
+    bool ok = true;
+    for (int j = 0; j < njobs && ok; ) {
+        int k = j + 1;
+        while (k < njobs && k - j < GG_MAXS) k++;
+        if (k < njobs) while (k > j + 1 && jobs[k].C == jobs[k - 1].C && jobs[k].acc) k--;      // a sum stays in one launch
+        ok = gg_run(c, jobs + j, k - j, nt);
+        j = k;
+    }
+    if (!keep) sb_gemm_keep_end(c);
+    if (!ok) sb_set_status(c, SB_ERR_CUDA);
+    return 0;
+}

@@ -4,7 +4,7 @@
 // accumulate) map onto C (+)= A^[M,K] B^[N,K]^T:
 //   * large, 16-byte-aligned products go to the CTA-pair kernel as they are: it reads either
 //     operand in either layout and makes the lo parts of the FP32-accurate mode itself, so
-//     nothing is prepared in HBM;
+//     nothing is prepared in HBM (the FP16-part modes run on the grouped kernel of gemm_group.cu);
 //   * the rest are brought to the single-CTA kernel's one form (both operands K-major) by an
 //     operand-preparation pass: an operand that already is K-major is used in place (only its lo
 //     part is written, 8 bytes per element); an operand that is not gets a transposed hi copy and
@@ -44,7 +44,7 @@ static bool prep_operand(sb_ctx_t* c, const float* src, int rows, int K, bool km
 // Slot holding (or about to hold) the FP16 parts of operand x[n].  Inside a keep region the kept slots are searched
 // first and the least recently used one is taken on a miss; outside, the call's own slot `own` is used.  *fresh: the
 // parts must be made.  Returns the slot index, -1 on allocation failure.
-static int f16_slot(sb_ctx_t* c, const float* x, size_t n, int own, bool* fresh) {
+int sb_f16_slot(sb_ctx_t* c, const float* x, size_t n, int own, bool* fresh) {
     if (!c->d_amax && sb_check(c, cudaMalloc(&c->d_amax, SB_F16_SLOTS * sizeof(float)), "amax alloc")) return -1;
     int s = own;
     *fresh = true;
@@ -127,6 +127,25 @@ extern "C" void sb_parts_unregister(sb_ctx_t* c, int kind) {
     parts_drop_arena(c);
 }
 #define SB_HINT_CAP 4096
+// a device word that is zero until the current step ends; NULL outside a step or when they are used up
+float* sb_zero_word(sb_ctx_t* c) {
+    if (!c->parts_open || !c->hint_pool || c->hint_n >= c->hint_cap) return NULL;
+    c->hint_tab[c->hint_n].ptr = NULL; c->hint_tab[c->hint_n].n = 0;
+    return c->hint_pool + c->hint_n++;
+}
+// The item counter of one grouped launch, zero when that launch starts: taken in turn from a ring that is cleared as a whole, in stream order
+#define SB_COUNTERS 1024
+unsigned* sb_item_counter(sb_ctx_t* c) {
+    if (!c->item_counters) {
+        if (sb_check(c, cudaMalloc((void**)&c->item_counters, SB_COUNTERS * sizeof(unsigned)), "item counters")) { c->item_counters = NULL; return NULL; }
+        c->item_counter_n = SB_COUNTERS;
+    }
+    if (c->item_counter_n == SB_COUNTERS) {
+        if (cudaMemsetAsync(c->item_counters, 0, SB_COUNTERS * sizeof(unsigned), (cudaStream_t)c->pub.stream) != cudaSuccess) return NULL;
+        c->item_counter_n = 0;
+    }
+    return c->item_counters + c->item_counter_n++;
+}
 extern "C" void sb_parts_open(sb_ctx_t* c) {
     c->parts_gen++; c->parts_open = 1;
     c->hint_n = 0; c->hint_npending = 0;
@@ -238,6 +257,7 @@ static bool tc_f16_direct(const sb_ctx_t* c, int mode, int M, int N, int K, bool
 }
 extern "C" int sb_gemm_reads_f16_parts(sb_ctx_t* c, int M, int N, int K, int tA, int tB) {
     const int mode = c->pub.use_bf16 ? SB_GEMM_BF16 : c->gemm_mode;
+    if (sb_gemm_group_takes(c, M, N, K, tA, tB)) return 1;
     if (K <= 0 || M < 32 || N < 32 || (double)M * N * K < (double)(1 << 21)) return 0;
     if (tA && tB) { tA = 0; tB = 0; }
     const bool a_kmajor = !tA, b_kmajor = tB != 0;
@@ -252,6 +272,7 @@ static bool tc_out_amax_on() {
     return on != 0;
 }
 extern "C" int sb_gemm_tc(sb_ctx_t* c, const float* A, const float* B, float* C, int M, int N, int K, int tA, int tB, int acc, int mode) {
+    { const sb_gemm_job_t job = {A, B, C, M, N, K, tA, tB, acc}; if (sb_gemm_group_try(c, &job, 1) == 0) return 0; }
     if (K <= 0 || M < 32 || N < 32) return 1;
     if ((double)M * N * K < (double)(1 << 21)) return 1;                 // too small to pay for the pipeline
     if (!tc_aligned16(A) || !tc_aligned16(B) || !tc_aligned16(C)) return 1;
@@ -278,9 +299,9 @@ extern "C" int sb_gemm_tc(sb_ctx_t* c, const float* A, const float* B, float* C,
             __half *ha, *hb; float *ma, *mb;
             void* hv; int fr; int sa = -1, sb = -1;
             if (sb_parts_find(c, A, na, &hv, &ma, &fr)) { ha = (__half*)hv; fa = fr != 0; }
-            else { sa = f16_slot(c, A, na, SB_F16_KEPT, &fa); if (sa < 0) return 1; ha = (__half*)c->f16_slot[sa].h; if (fa) c->f16_slot[sa].amax = c->d_amax + sa; ma = c->f16_slot[sa].amax; }
+            else { sa = sb_f16_slot(c, A, na, SB_F16_KEPT, &fa); if (sa < 0) return 1; ha = (__half*)c->f16_slot[sa].h; if (fa) c->f16_slot[sa].amax = c->d_amax + sa; ma = c->f16_slot[sa].amax; }
             if (sb_parts_find(c, B, nb, &hv, &mb, &fr)) { hb = (__half*)hv; fb = fr != 0; }
-            else { sb = f16_slot(c, B, nb, SB_F16_KEPT + 1, &fb); if (sb < 0) return 1; hb = (__half*)c->f16_slot[sb].h; if (fb) c->f16_slot[sb].amax = c->d_amax + sb; mb = c->f16_slot[sb].amax; }
+            else { sb = sb_f16_slot(c, B, nb, SB_F16_KEPT + 1, &fb); if (sb < 0) return 1; hb = (__half*)c->f16_slot[sb].h; if (fb) c->f16_slot[sb].amax = c->d_amax + sb; mb = c->f16_slot[sb].amax; }
             if (fa || fb) {
                 cudaStream_t st = (cudaStream_t)c->pub.stream;
                 int tp = sb_tick_begin(c, SB_CLS_GEMM_PREP);

@@ -910,7 +910,7 @@ static __global__ void __launch_bounds__(256) tc_split_f16_kernel(const float* _
 #define TC_MULTI 64
 #define TC_MULTI_CHUNK 1024
 struct TcMultiJob { const float* x; __half* h; float* amax; uint32_t n4, first; };      // h: hi parts, lo parts behind them; first: its first chunk
-struct TcMulti { int n; uint32_t chunks; TcMultiJob j[TC_MULTI]; };
+struct TcMulti { int n; uint32_t chunks; unsigned keep; TcMultiJob j[TC_MULTI]; };
 static inline void tc_multi_add(TcMulti* m, const float* x, size_t n, void* h, float* amax) {
     TcMultiJob* j = &m->j[m->n++];
     j->x = x; j->h = (__half*)h; j->amax = amax; j->n4 = (uint32_t)(n / 4); j->first = m->chunks;
@@ -922,6 +922,7 @@ __device__ __forceinline__ int tc_multi_find(const TcMulti& m, uint32_t chunk) {
     return lo;
 }
 static __global__ void __launch_bounds__(256) tc_amax_multi_kernel(const __grid_constant__ TcMulti m) {
+    sb_pdl_enter();
     __shared__ float red[8];
     const uint32_t per = (m.chunks + gridDim.x - 1) / gridDim.x;
     uint32_t ck = blockIdx.x * per;
@@ -952,6 +953,7 @@ static __global__ void __launch_bounds__(256) tc_amax_multi_kernel(const __grid_
 }
 // walks each CTA's run backwards: what the maximum pass read last is still in L2
 static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid_constant__ TcMulti m) {
+    sb_pdl_enter();
     const uint32_t per = (m.chunks + gridDim.x - 1) / gridDim.x;
     const uint32_t begin = blockIdx.x * per;
     uint32_t ck = min(m.chunks, begin + per);
@@ -961,7 +963,7 @@ static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid
         const uint32_t stop = max(begin, j.first);
         const float4* x = (const float4*)j.x;
         uint2* h1 = (uint2*)j.h; uint2* h2 = h1 + j.n4;
-        const float sc = tc_pow2(tc_f16_shift(*j.amax));
+        const float sc = tc_pow2(tc_f16_shift(sb_word(j.amax)));
         while (ck > stop) {
             ck--;
             const uint32_t base = (ck - j.first) * TC_MULTI_CHUNK + threadIdx.x;
@@ -971,7 +973,7 @@ static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid
 #pragma unroll
             for (int u = 0; u < TC_MULTI_CHUNK / 256; u++) if (base + u * 256 < j.n4) {
                 uint2 a, b;
-                sb_split2(v[u].x * sc, v[u].y * sc, a.x, b.x); sb_split2(v[u].z * sc, v[u].w * sc, a.y, b.y);
+                sb_split2(v[u].x * sc, v[u].y * sc, a.x, b.x, m.keep); sb_split2(v[u].z * sc, v[u].w * sc, a.y, b.y, m.keep);
                 h1[base + u * 256] = a; h2[base + u * 256] = b;
             }
         }
@@ -983,12 +985,13 @@ static inline unsigned tc_multi_grid(sb_ctx_t* c, const TcMulti& m) {
 }
 static inline void tc_multi_amax(sb_ctx_t* c, const TcMulti& m) {      // the words are zero before
     if (!m.n) return;
-    tc_amax_multi_kernel<<<tc_multi_grid(c, m), 256, 0, (cudaStream_t)c->pub.stream>>>(m);
+    sb_launch(tc_amax_multi_kernel, dim3(tc_multi_grid(c, m)), dim3(256), 0, (cudaStream_t)c->pub.stream, m);
     c->launches++;
 }
-static inline void tc_multi_split(sb_ctx_t* c, const TcMulti& m) {
+static inline void tc_multi_split(sb_ctx_t* c, TcMulti& m) {
     if (!m.n) return;
-    tc_split_multi_kernel<<<tc_multi_grid(c, m), 256, 0, (cudaStream_t)c->pub.stream>>>(m);
+    m.keep = sb_parts_keep(c);
+    sb_launch(tc_split_multi_kernel, dim3(tc_multi_grid(c, m)), dim3(256), 0, (cudaStream_t)c->pub.stream, m);
     c->launches++;
 }
 

@@ -130,6 +130,12 @@ void sb_gemm(sb_ctx_t* c, const float* A, const float* B, float* C, int M, int N
     sb_tick_end(c, t, 2.0 * M * N * K, 4.0 * ((double)M * K + (double)N * K + (double)M * N * (acc ? 2 : 1)));
 }
 
+void sb_gemm_group(sb_ctx_t* c, const sb_gemm_job_t* jobs, int n) {
+    for (int j = 0; j < n; j++) sb_amax_forget(c, jobs[j].C);
+    if (sb_gemm_group_try(c, jobs, n) == 0) return;
+    for (int j = 0; j < n; j++) sb_gemm(c, jobs[j].A, jobs[j].B, jobs[j].C, jobs[j].M, jobs[j].N, jobs[j].K, jobs[j].tA, jobs[j].tB, jobs[j].acc);
+}
+
 // reference: cuda_train_matmul, src/cuda_train_context.cu:2697
 void cuda_train_matmul(cuda_train_context_t* ctx, cuda_buffer_t* A, cuda_buffer_t* B, cuda_buffer_t* C, int M, int N, int K) {
     CTX_OR_RETURN(ctx); NEED(A, B, C);

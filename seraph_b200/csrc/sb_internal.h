@@ -16,8 +16,8 @@ extern "C" {
 #endif
 
 #define SB_MAGIC 0x53423230u   /* "SB20" */
-#define SB_F16_KEPT 10          /* operand-part slots kept across the products of a keep region */
-#define SB_F16_SLOTS 12         /* plus one per operand for products outside a region */
+#define SB_F16_KEPT 22          /* operand-part slots kept across the products of a keep region */
+#define SB_F16_SLOTS 24         /* plus one per operand for products outside a region */
 
 /* status codes (seraph_b200_last_status) */
 enum {
@@ -62,8 +62,8 @@ typedef struct sb_ctx {
     int* d_status;                   /* device status word (bounds checks, bounded waits) */
     int gemm_mode;                   /* SB_GEMM_* (use_bf16 in pub overrides to BF16) */
     float* d_amax;                   /* FP16 split: max |x| of the operand held by each part slot */
-    struct { void* h; size_t cap; const float* ptr; size_t n; unsigned stamp; int valid; float* amax; } f16_slot[SB_F16_SLOTS];   /* FP16 parts of GEMM operands: 0-9 kept across
-                                        calls inside a keep region (train_step.c marks runs of GEMMs that share operands), 10-11 for one call */
+    struct { void* h; size_t cap; const float* ptr; size_t n; unsigned stamp; int valid; float* amax; } f16_slot[SB_F16_SLOTS];   /* FP16 parts of GEMM operands: all but the last two kept across
+                                        calls inside a keep region (train_step.c marks runs of GEMMs that share operands), the last two for one call */
     int f16_keep; unsigned f16_clock;
     /* FP16 parts of registered tensors (weights, saved activations), valid from their first use inside a training or
        evaluation step until that step returns: made once, then shared by every product of the step that reads the tensor */
@@ -142,6 +142,8 @@ typedef struct sb_ctx {
     void* scratch; size_t scratch_bytes;
     /* operand staging of the tensor-core GEMM (hi/lo, transposed copies) */
     void* gemm_stage[5]; size_t gemm_stage_bytes[5];
+    void* gg_plans;                  /* schedules of grouped products (gemm_group.cu) */
+    unsigned* item_counters; int item_counter_n;
     void* map_cache;                 /* encoded tensor maps (gemm_tc.cuh) */
     const uint32_t* attn_seq_starts; /* device sequence boundaries of the attention call in flight (h_seq_n + 1 entries) */
     /* rope cos/sin table */
@@ -240,6 +242,13 @@ void sb_sumsq(sb_ctx_t*, const float* g, size_t n, float* d_out);               
 void sb_nan_check(sb_ctx_t*, const float* x, size_t n, uint32_t* flags, uint32_t idx);
 /* C[M,N] (+)= op(A) op(B); same semantics as the reference's matmul_dispatch */
 void sb_gemm(sb_ctx_t*, const float* A, const float* B, float* C, int M, int N, int K, int tA, int tB, int acc);
+/* Several products that do not depend on one another, as if by sb_gemm in this order; a product with the destination of the one before it and
+   acc set is added to it.  On FP16 parts they run as one launch. */
+typedef struct { const float *A, *B; float* C; int M, N, K, tA, tB, acc; } sb_gemm_job_t;
+void sb_gemm_group(sb_ctx_t*, const sb_gemm_job_t* jobs, int n);
+int  sb_gemm_group_try(sb_ctx_t*, const sb_gemm_job_t* jobs, int n);      /* 0: launched as a group */
+int  sb_gemm_group_takes(sb_ctx_t*, int M, int N, int K, int tA, int tB);
+void sb_parts_prepare(sb_ctx_t*, const float* const* x, const size_t* n, int count);
 int  sb_gemm_reads_f16_parts(sb_ctx_t*, int M, int N, int K, int tA, int tB);      /* 1: that product takes prepared FP16 parts of its operands */
 void sb_gemm_simt(sb_ctx_t*, const float* A, const float* B, float* C, int M, int N, int K, int tA, int tB, int acc);
 /* returns 0 if the tensor-core path took the call, nonzero if the shape is not eligible */
@@ -270,10 +279,37 @@ void sb_prof_end(sb_ctx_t*, int op, size_t flops, size_t bytes);
 
 #ifdef __cplusplus
 }
+/* the `keep` mask of sb_split2 for operands of the plain products */
+static inline unsigned sb_parts_keep(const sb_ctx_t* c) { return c->pub.use_bf16 || c->gemm_mode == SB_GEMM_BF16 ? 0xffffe000u : 0xffffffffu; }
+float* sb_zero_word(sb_ctx_t* c);
+unsigned* sb_item_counter(sb_ctx_t* c);
+int sb_f16_slot(sb_ctx_t* c, const float* x, size_t n, int own, bool* fresh);
 #endif
 #endif
 
 #ifdef __CUDACC__
+/* Programmatic dependent launch.  A training step is a few hundred short kernels in one stream; the gap between two of them (the drain of the
+   one, the launch and the start-up of the other) costs 2 to 4 us, as much as many of them run.  sb_launch lets a kernel start while its
+   predecessor drains; every kernel launched by it waits (sb_pdl_wait: until the predecessor has completed and its writes are visible)
+   before it touches global memory, in every thread, so completion stays ordered along the stream. */
+static __device__ __forceinline__ void sb_pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+static __device__ __forceinline__ void sb_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+/* The successor is let in only after the wait: its launch then also follows the end of the kernel before this one, so that an SM's L1
+   holds no line that was read back then. */
+static __device__ __forceinline__ void sb_pdl_enter() { sb_pdl_wait(); sb_pdl_trigger(); }
+/* A word another kernel leaves behind (a largest magnitude, a bound), from L2: words of different producers share cache lines, and a successor
+   that is already resident must not take its line from an L1 that the producer's other reads filled. */
+static __device__ __forceinline__ float sb_word(const float* p) { float v; asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory"); return v; }
+template <typename... E, typename... A>
+static inline cudaError_t sb_launch(void (*kernel)(E...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
 /* Largest magnitude seen by a CTA (each thread passes its own maximum, >= 0) raised into *out with an integer atomicMax on the
    float bits; every thread of the CTA must call it, CTAs of at most 1024 threads.  out == NULL: nothing happens. */
 static __device__ __forceinline__ void sb_block_amax(float v, unsigned* out) {
@@ -303,15 +339,18 @@ static __device__ __forceinline__ int sb_f16_shift(float amax) {
     return sh < -100 ? -100 : (sh > 100 ? 100 : sh);
 }
 static __device__ __forceinline__ float sb_pow2(int sh) { return __uint_as_float((unsigned)(127 + sh) << 23); }
+/* keep: all bits, or SB_KEEP_TF32: hi is cut to 11 significant bits instead of rounded.  The single-pass mode reads only the hi parts, and cut
+   they are the operands a TF32 instruction takes from the FP32 words. */
+#define SB_KEEP_TF32 0xffffe000u
 /* two scaled values as packed parts (x0 in the low half); x - hi by the mixed-precision fma hi * -1 + x, exact */
-static __device__ __forceinline__ void sb_split2(float x0, float x1, unsigned& hi, unsigned& lo) {
+static __device__ __forceinline__ void sb_split2(float x0, float x1, unsigned& hi, unsigned& lo, unsigned keep = 0xffffffffu) {
     asm("{\n\t.reg .b16 h0, h1, m1;\n\t.reg .f32 l0, l1;\n\t"
-        "cvt.rn.f16x2.f32 %0, %3, %2;\n\t"
+        "cvt.rn.f16x2.f32 %0, %5, %4;\n\t"
         "mov.b32 {h0, h1}, %0;\n\t"
         "mov.b16 m1, 0xBC00;\n\t"
         "fma.rn.f32.f16 l0, h0, m1, %2;\n\t"
         "fma.rn.f32.f16 l1, h1, m1, %3;\n\t"
         "cvt.rn.f16x2.f32 %1, l1, l0;\n\t}"
-        : "=&r"(hi), "=r"(lo) : "f"(x0), "f"(x1));
+        : "=&r"(hi), "=r"(lo) : "f"(x0), "f"(x1), "f"(__uint_as_float(__float_as_uint(x0) & keep)), "f"(__uint_as_float(__float_as_uint(x1) & keep)));
 }
 #endif

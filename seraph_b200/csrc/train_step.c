@@ -653,6 +653,32 @@ static int nan_tripped(sb_ctx_t* c, const train_state_t* st, int T) {
     return any;
 }
 
+/* The FP16 parts of every weight matrix the pass reads, in a few launches (tensors that fit L2 together share a maximum and a split
+   launch) instead of one or two per matrix at its first product. */
+#define PREP_BATCH_FLOATS ((size_t)10 << 20)
+static void prepare_weights(sb_ctx_t* c, int T) {
+    const int d = c->d, F = c->F, qd = c->qd, kvd = c->kvd;
+    if (!sb_gemm_group_takes(c, T, qd, d, 0, 1) || !sb_gemm_group_takes(c, T, kvd, d, 0, 1) || !sb_gemm_group_takes(c, T, F, d, 0, 1) ||
+        !sb_gemm_group_takes(c, T, d, F, 0, 1) || !sb_gemm_group_takes(c, T, d, qd, 0, 1) || !sb_gemm_group_takes(c, T, c->V, d, 0, 1)) return;
+    const float* x[64]; size_t n[64], sum = 0; int k = 0;
+    for (int l = -1; l < c->L; l++) {
+        const sb_layer_off_t* o = l >= 0 ? &c->off[l] : NULL;
+        const float* w[7]; size_t m[7]; int nw = 0;
+        if (l < 0) { w[0] = c->untied ? c->XW + extras_lm_off(c) : c->W; m[0] = (size_t)c->V * d; nw = 1; }
+        else {
+            const size_t off[7] = {o->q, o->k, o->v, o->o, o->gate, o->up, o->down};
+            const size_t len[7] = {(size_t)qd * d, (size_t)kvd * d, (size_t)kvd * d, (size_t)qd * d, (size_t)F * d, (size_t)F * d, (size_t)F * d};
+            for (int i = 0; i < 7; i++) { w[i] = c->W + off[i]; m[i] = len[i]; }
+            nw = 7;
+        }
+        for (int i = 0; i < nw; i++) {
+            if (k && (k == 64 || sum + m[i] > PREP_BATCH_FLOATS)) { sb_parts_prepare(c, x, n, k); k = 0; sum = 0; }
+            x[k] = w[i]; n[k] = m[i]; sum += m[i]; k++;
+        }
+    }
+    if (k) sb_parts_prepare(c, x, n, k);
+}
+
 static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_lora) {
     const int d = c->d, F = c->F, qd = c->qd, kvd = c->kvd, L = c->L;
     const size_t Td = (size_t)T * d;
@@ -667,6 +693,7 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
                          sb_gemm_reads_f16_parts(c, T, F, d, 0, 1) && sb_gemm_reads_f16_parts(c, F, d, T, 1, 0);
     const int hn_parts = !c->nan_on && sb_gemm_reads_f16_parts(c, T, c->V, d, 0, 1) && sb_gemm_reads_f16_parts(c, c->V, d, T, 1, 0);
     nan_mark(c, c->W, (size_t)c->V * d, nan_weight_idx(c));
+    prepare_weights(c, T);
     sb_embed_lookup(c, c->tokens, c->W, c->act[0].layer_in, T, d, c->V);
     nan_mark(c, c->act[0].layer_in, Td, 7);
     for (int l = 0; l < L; l++) {
@@ -679,10 +706,17 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
         }
         /* runs of products that share an operand keep its prepared parts (the adapters' scratch, rewritten in between, is dropped from the kept set at every write) */
         sb_gemm_keep_begin(c);
-        linear_fwd(c, use_lora, l, 0, a->x_norm_attn, c->W + o->q, c->head_norm ? a->q_pre : a->q, T, d, qd, 0);
-        linear_fwd(c, use_lora, l, 1, a->x_norm_attn, c->W + o->k, c->head_norm ? a->k_pre : a->k, T, d, kvd, 0);
+        float* yq = c->head_norm ? a->q_pre : a->q; float* yk = c->head_norm ? a->k_pre : a->k;
         sb_amax_announce(c, a->v, (size_t)T * kvd);           /* nothing rewrites v before attention splits it */
-        linear_fwd(c, use_lora, l, 2, a->x_norm_attn, c->W + o->v, a->v, T, d, kvd, 0);
+        if (!(use_lora && (c->lora_mask & 0x07))) {
+            const sb_gemm_job_t jobs[3] = {{a->x_norm_attn, c->W + o->q, yq, T, qd, d, 0, 1, 0}, {a->x_norm_attn, c->W + o->k, yk, T, kvd, d, 0, 1, 0},
+                                           {a->x_norm_attn, c->W + o->v, a->v, T, kvd, d, 0, 1, 0}};
+            sb_gemm_group(c, jobs, 3);
+        } else {
+            linear_fwd(c, use_lora, l, 0, a->x_norm_attn, c->W + o->q, yq, T, d, qd, 0);
+            linear_fwd(c, use_lora, l, 1, a->x_norm_attn, c->W + o->k, yk, T, d, kvd, 0);
+            linear_fwd(c, use_lora, l, 2, a->x_norm_attn, c->W + o->v, a->v, T, d, kvd, 0);
+        }
         sb_gemm_keep_end(c);
         if (c->head_norm) {       /* learned RMSNorm over each head (rows of head_dim), before RoPE */
             const float* wn = c->XW + (size_t)l * 2 * c->hd;
@@ -706,9 +740,14 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
         }
         sb_gemm_keep_begin(c);
         sb_amax_announce(c, a->gate, (size_t)T * F);        /* the products' epilogues leave max |gate|, max |up| for the bound below */
-        linear_fwd(c, use_lora, l, 4, a->x_norm_ffn, c->W + o->gate, a->gate, T, d, F, 0);
         sb_amax_announce(c, a->up, (size_t)T * F);
-        linear_fwd(c, use_lora, l, 5, a->x_norm_ffn, c->W + o->up, a->up, T, d, F, 0);
+        if (!(use_lora && (c->lora_mask & 0x30))) {
+            const sb_gemm_job_t jobs[2] = {{a->x_norm_ffn, c->W + o->gate, a->gate, T, F, d, 0, 1, 0}, {a->x_norm_ffn, c->W + o->up, a->up, T, F, d, 0, 1, 0}};
+            sb_gemm_group(c, jobs, 2);
+        } else {
+            linear_fwd(c, use_lora, l, 4, a->x_norm_ffn, c->W + o->gate, a->gate, T, d, F, 0);
+            linear_fwd(c, use_lora, l, 5, a->x_norm_ffn, c->W + o->up, a->up, T, d, F, 0);
+        }
         sb_gemm_keep_end(c);
         /* silu(gate) * up is read only as an operand (down projection, its weight gradient): when those products take FP16 parts
            the kernel writes the parts and no FP32 copy */
@@ -740,8 +779,11 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
     float* norm_sink = c->g_tmp;                 /* LoRA mode: norm-scale gradients are discarded */
     if (!full) sb_memset(c, norm_sink, 0, (size_t)d * sizeof(float));
     sb_gemm_keep_begin(c);
-    sb_gemm(c, c->dlogits, c->untied ? c->XW + extras_lm_off(c) : c->W, gx, T, d, V, 0, 0, 0);
-    if (full) sb_gemm(c, c->dlogits, c->hidden_norm, c->untied ? c->XG + extras_lm_off(c) : Gd, V, d, T, 1, 0, 1);
+    {
+        const sb_gemm_job_t jobs[2] = {{c->dlogits, c->untied ? c->XW + extras_lm_off(c) : c->W, gx, T, d, V, 0, 0, 0},
+                                       {c->dlogits, c->hidden_norm, c->untied ? c->XG + extras_lm_off(c) : Gd, V, d, T, 1, 0, 1}};
+        sb_gemm_group(c, jobs, full ? 2 : 1);
+    }
     sb_gemm_keep_end(c);
     nan_mark(c, c->dlogits, (size_t)T * V, 3); nan_mark(c, gx, (size_t)T * d, 4);
     sb_amax_announce(c, gh, (size_t)T * d);
@@ -754,9 +796,11 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
         sb_layer_act_t* a = &c->act[l];
         /* FFN */
         sb_gemm_keep_begin(c);                       /* gh (and, with adapters, what they read) is split once for the whole group */
-        if (full) sb_gemm(c, gh, a->ffn_hidden, Gd + o->down, d, F, T, 1, 0, 1);
         sb_amax_announce(c, c->g_ffn, (size_t)T * F);
-        sb_gemm(c, gh, c->W + o->down, c->g_ffn, T, F, d, 0, 0, 0);
+        {
+            const sb_gemm_job_t jobs[2] = {{gh, c->W + o->down, c->g_ffn, T, F, d, 0, 0, 0}, {gh, a->ffn_hidden, Gd + o->down, d, F, T, 1, 0, 1}};
+            sb_gemm_group(c, jobs, full ? 2 : 1);
+        }
         if (!full) lora_bwd(c, l, 6, gh, a->ffn_hidden, c->g_ffn, T);
         sb_gemm_keep_end(c);
         if (!(ffn_parts_bwd && sb_swiglu_backward_parts(c, a->gate, a->up, c->g_ffn, c->g_gate, c->g_up, (size_t)T * F))) {
@@ -764,20 +808,21 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
             sb_swiglu_backward(c, a->gate, a->up, c->g_ffn, c->g_gate, c->g_up, (size_t)T * F);
         }
         sb_gemm_keep_begin(c);
-        if (full) {
-            sb_gemm(c, c->g_gate, a->x_norm_ffn, Gd + o->gate, F, d, T, 1, 0, 1);
-            sb_gemm(c, c->g_up, a->x_norm_ffn, Gd + o->up, F, d, T, 1, 0, 1);
+        {
+            const sb_gemm_job_t jobs[4] = {{c->g_gate, c->W + o->gate, gx, T, d, F, 0, 0, 0}, {c->g_up, c->W + o->up, gx, T, d, F, 0, 0, 1},
+                                           {c->g_gate, a->x_norm_ffn, Gd + o->gate, F, d, T, 1, 0, 1}, {c->g_up, a->x_norm_ffn, Gd + o->up, F, d, T, 1, 0, 1}};
+            sb_gemm_group(c, jobs, full ? 4 : 2);
         }
-        sb_gemm(c, c->g_gate, c->W + o->gate, gx, T, d, F, 0, 0, 0);
-        sb_gemm(c, c->g_up, c->W + o->up, gx, T, d, F, 0, 0, 1);
         if (!full) { lora_bwd(c, l, 4, c->g_gate, a->x_norm_ffn, gx, T); lora_bwd(c, l, 5, c->g_up, a->x_norm_ffn, gx, T); }
         sb_gemm_keep_end(c);
         sb_amax_announce(c, gh, (size_t)T * d);
         sb_rmsnorm_backward(c, a->post_attn_in, c->W + o->post_norm, gx, gh, gh, full ? Gd + o->post_norm : norm_sink, T, d, RMS_EPS);
         /* attention */
         sb_gemm_keep_begin(c);
-        if (full) sb_gemm(c, gh, a->attn_out, Gd + o->o, d, qd, T, 1, 0, 1);
-        sb_gemm(c, gh, c->W + o->o, c->g_attn, T, qd, d, 0, 0, 0);
+        {
+            const sb_gemm_job_t jobs[2] = {{gh, c->W + o->o, c->g_attn, T, qd, d, 0, 0, 0}, {gh, a->attn_out, Gd + o->o, d, qd, T, 1, 0, 1}};
+            sb_gemm_group(c, jobs, full ? 2 : 1);
+        }
         if (!full) lora_bwd(c, l, 3, gh, a->attn_out, c->g_attn, T);
         sb_gemm_keep_end(c);
         nan_mark(c, c->g_attn, (size_t)T * qd, nan_bwd_base(c) + 5u * (uint32_t)l);
@@ -803,14 +848,12 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
             gq = c->g_q2; gk = c->g_k2;
         }
         sb_gemm_keep_begin(c);
-        if (full) {
-            sb_gemm(c, gq, a->x_norm_attn, Gd + o->q, qd, d, T, 1, 0, 1);
-            sb_gemm(c, gk, a->x_norm_attn, Gd + o->k, kvd, d, T, 1, 0, 1);
-            sb_gemm(c, c->g_v, a->x_norm_attn, Gd + o->v, kvd, d, T, 1, 0, 1);
+        {
+            const sb_gemm_job_t jobs[6] = {{gq, c->W + o->q, gx, T, d, qd, 0, 0, 0}, {gk, c->W + o->k, gx, T, d, kvd, 0, 0, 1}, {c->g_v, c->W + o->v, gx, T, d, kvd, 0, 0, 1},
+                                           {gq, a->x_norm_attn, Gd + o->q, qd, d, T, 1, 0, 1}, {gk, a->x_norm_attn, Gd + o->k, kvd, d, T, 1, 0, 1},
+                                           {c->g_v, a->x_norm_attn, Gd + o->v, kvd, d, T, 1, 0, 1}};
+            sb_gemm_group(c, jobs, full ? 6 : 3);
         }
-        sb_gemm(c, gq, c->W + o->q, gx, T, d, qd, 0, 0, 0);
-        sb_gemm(c, gk, c->W + o->k, gx, T, d, kvd, 0, 0, 1);
-        sb_gemm(c, c->g_v, c->W + o->v, gx, T, d, kvd, 0, 0, 1);
         if (!full) { lora_bwd(c, l, 0, gq, a->x_norm_attn, gx, T); lora_bwd(c, l, 1, gk, a->x_norm_attn, gx, T); lora_bwd(c, l, 2, c->g_v, a->x_norm_attn, gx, T); }
         sb_gemm_keep_end(c);
         sb_amax_announce(c, gh, (size_t)T * d);
@@ -1213,6 +1256,8 @@ void cuda_train_free(cuda_train_context_t* ctx) {
     }
     if (c->rope_tab) cudaFree(c->rope_tab);
     free(c->map_cache);
+    free(c->gg_plans);
+    if (c->item_counters) cudaFree(c->item_counters);
     if (c->seq_copy_stream) cudaStreamDestroy((cudaStream_t)c->seq_copy_stream);
     for (int i = 0; i < 2; i++) if (c->seq_copy_ev[i]) cudaEventDestroy((cudaEvent_t)c->seq_copy_ev[i]);
     if (c->h_seq_pin) cudaFreeHost(c->h_seq_pin);
