@@ -121,6 +121,7 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
                   const float* __restrict__ amax_q, const float* __restrict__ amax_k, const float* __restrict__ amax_v,
                   const float* __restrict__ amax_do, const float* __restrict__ ds_bound,
                   const AfSeqTab seqs, int Sp, int Hq, int g, int nkb, int chunk, int accumulate, int slot_pitch, float scale, int* status) {
+    sb_pdl_enter();
     constexpr int NH = HD / 64;
     constexpr int KV_PART = NH * 16384, ST_PART = NH * 4096;
     constexpr int COL_DK = 0, COL_DV = HD, COL_K = 2 * HD, COL_S0 = 3 * HD, COL_V = COL_S0 + 128;
@@ -312,8 +313,8 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
             const int q = warp & 3, r = q * 32 + lane, kg = k0 + r;
             const bool live = kg < S;
             // dV accumulates (P 2^14) (dO 2^s_do), dK accumulates (dS 2^s_ds) (Q 2^s_q)
-            const float fv = tc_pow2(-14) * tc_pow2(-tc_f16_shift(__ldg(amax_do)));
-            const float fk = tc_pow2(-tc_f16_shift(__ldg(ds_bound))) * tc_pow2(-tc_f16_shift(__ldg(amax_q)));
+            const float fv = tc_pow2(-14) * tc_pow2(-tc_f16_shift(sb_word(amax_do)));
+            const float fk = tc_pow2(-tc_f16_shift(sb_word(ds_bound))) * tc_pow2(-tc_f16_shift(sb_word(amax_q)));
             float* rowk = dK + (size_t)(t0 + (live ? kg : 0)) * kvd + (size_t)kvh * HD;
             float* rowv = dV + (size_t)(t0 + (live ? kg : 0)) * kvd + (size_t)kvh * HD;
             const uint32_t ta = tmem_base + ((uint32_t)(q * 32) << 16);
@@ -418,9 +419,9 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
         // ---------------- elementwise: one key row and 16 of the step's 32 queries per thread (warps 4-7: queries 0..15, 8-11: 16..31) ----------------
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(AB_REGS_EW));
         const int ch = (warp - 4) >> 2, q = warp & 3, r = q * 32 + lane, kg = k0 + r;
-        const float cs = tc_pow2(-tc_f16_shift(__ldg(amax_q))) * tc_pow2(-tc_f16_shift(__ldg(amax_k))) * (HD == 64 ? scale : scale * 1.4426950408889634f);
-        const float cp = tc_pow2(-tc_f16_shift(__ldg(amax_do))) * tc_pow2(-tc_f16_shift(__ldg(amax_v)));
-        const float cpd = cp * (tc_pow2(tc_f16_shift(__ldg(ds_bound))) * scale * (1.0f / 16384.f));      // p holds P * 2^14
+        const float cs = tc_pow2(-tc_f16_shift(sb_word(amax_q))) * tc_pow2(-tc_f16_shift(sb_word(amax_k))) * (HD == 64 ? scale : scale * 1.4426950408889634f);
+        const float cp = tc_pow2(-tc_f16_shift(sb_word(amax_do))) * tc_pow2(-tc_f16_shift(sb_word(amax_v)));
+        const float cpd = cp * (tc_pow2(tc_f16_shift(sb_word(ds_bound))) * scale * (1.0f / 16384.f));      // p holds P * 2^14
         const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
         // This key row's parts of K from shared memory (128-byte-swizzled tiles: hi and lo part of each half of the head
         // dimension) into tensor memory: head-dimension k-steps ch*4 .. ch*4+3 are half `ch`, two consecutive halfs per column.
@@ -584,6 +585,7 @@ at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant_
                  const __grid_constant__ CUtensorMap mK1, const __grid_constant__ CUtensorMap mK2,
                  const AfSeqTab seqs, float* __restrict__ dQ, const float* __restrict__ ds_bound, const float* __restrict__ amax_k,
                  int Sp, int Hq, int g, int nqb_max, int* status) {
+    sb_pdl_enter();
     constexpr int NH = HD / 64, OC = HD / 2;
     const int per_i = seqs.n * Hq;
     const int qb = nqb_max - 1 - (int)blockIdx.x / per_i;
@@ -690,7 +692,7 @@ at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant_
             }
         }
         if (ok && qi < S) {
-            const float f1 = tc_pow2(-tc_f16_shift(__ldg(ds_bound))), f2 = tc_pow2(-tc_f16_shift(__ldg(amax_k)));
+            const float f1 = tc_pow2(-tc_f16_shift(sb_word(ds_bound))), f2 = tc_pow2(-tc_f16_shift(sb_word(amax_k)));
             float4* dst = (float4*)(dQ + (size_t)(t0 + qi) * Hq * HD + (size_t)h * HD + ch * OC);
 #pragma unroll
             for (int i = 0; i < OC / 4; i++)
@@ -752,12 +754,11 @@ static int ab_launch(sb_ctx_t* c, const AbCall& p) {
     chunk = max(1, min(chunk, seqs.n * p.Hkv));
     if (qblocks > 0x7fffffffL) return 1;
     cudaStream_t st = (cudaStream_t)c->pub.stream;
-    kern<<<(unsigned)blocks, AB_THREADS, AB_SMEM(NH), st>>>(
-        mQ1, mQ2, mD1, mD2, mK1, mK2, mV1, mV2, mS1, mS2, mdK, mdV, p.LT, p.DT, (__half*)p.dS1, (__half*)p.dS2, p.dK, p.dV,
+    sb_launch(kern, dim3((unsigned)blocks), dim3(AB_THREADS), AB_SMEM(NH), st, mQ1, mQ2, mD1, mD2, mK1, mK2, mV1, mV2, mS1, mS2, mdK, mdV, p.LT, p.DT, (__half*)p.dS1, (__half*)p.dS2, p.dK, p.dV,
         p.amax_q, p.amax_k, p.amax_v, p.amax_do, p.ds_bound, seqs, p.Sp, p.Hq, g, nkb, chunk, p.accumulate, slot_pitch, 1.0f / sqrtf((float)HD), c->d_status);
     c->launches++;
     if (p.dQ) {
-        at_dq_bwd_kernel<HD><<<(unsigned)qblocks, AQ_THREADS, AQ_SMEM(NH), st>>>(mA1, mA2, mB1, mB2, seqs, p.dQ, p.ds_bound, p.amax_k, p.Sp, p.Hq, g, nkb, c->d_status);
+        sb_launch(at_dq_bwd_kernel<HD>, dim3((unsigned)qblocks), dim3(AQ_THREADS), AQ_SMEM(NH), st, mA1, mA2, mB1, mB2, seqs, p.dQ, p.ds_bound, p.amax_k, p.Sp, p.Hq, g, nkb, c->d_status);
         c->launches++;
     }
     return cudaGetLastError() == cudaSuccess ? 0 : 1;

@@ -31,6 +31,7 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
                     const AfSeqTab seqs, float* __restrict__ O, float* __restrict__ lse,
                     const float* __restrict__ amax_q, const float* __restrict__ amax_k, const float* __restrict__ amax_v,
                     int Hq, int g, int nqb_max, float scale, int* status, unsigned* amax_o) {
+    sb_pdl_enter();
     constexpr int NH = HD / 64;                              // 64-column halves of the head dimension (one 128-byte row of halfs each)
     constexpr int Q_BYTES = NH * 32768, KV_STAGE = NH * 16384, Q_PART = NH * 16384, KV_PART = NH * 8192;
     constexpr int OFF_K = Q_BYTES, OFF_V = OFF_K + 2 * KV_STAGE, OFF_P = OFF_V + 2 * KV_STAGE, OFF_BAR = OFF_P + 32768;
@@ -186,7 +187,7 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
         // ---------------- softmax: one query row per thread ----------------
         const int q = warp & 3, r = q * 32 + lane;
         const int qi = qb * AF_BQ + r;                        // position of this row inside the sequence
-        const float cs = tc_pow2(-tc_f16_shift(__ldg(amax_q))) * tc_pow2(-tc_f16_shift(__ldg(amax_k))) * (scale * 1.4426950408889634f);
+        const float cs = tc_pow2(-tc_f16_shift(sb_word(amax_q))) * tc_pow2(-tc_f16_shift(sb_word(amax_k))) * (scale * 1.4426950408889634f);
         float m = -INFINITY, l = 0.f;
         uint8_t* prow = smem + OFF_P + r * 128;
         for (int j = 0; j < nkv && ok; j++) {
@@ -295,7 +296,7 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
         if (ok) ok = mbar_wait(fin_full, 0);
         float am = 0.f;
         if (ok && qi < S) {
-            const float f = fin_s[r] * tc_pow2(-tc_f16_shift(__ldg(amax_v)));      // fin = 1 / l with l in units of 2^-14, O holds (P * 2^14) V' products
+            const float f = fin_s[r] * tc_pow2(-tc_f16_shift(sb_word(amax_v)));      // fin = 1 / l with l in units of 2^-14, O holds (P * 2^14) V' products
             float4* dst = (float4*)(O + (size_t)(t0 + qi) * qd + (size_t)h * HD + ch * OC);
 #pragma unroll
             for (int i = 0; i < OC / 4; i++) {
@@ -344,6 +345,7 @@ at_score_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
                     const float* __restrict__ amax_q, const float* __restrict__ amax_k, const float* __restrict__ amax_v,
                     const float* __restrict__ amax_do, const float* __restrict__ ds_bound,
                     const __grid_constant__ AfSeqs seqs, int Sp, int Hq, int g, int head0, int head_step, int nb, int nqb, float scale, int* status) {
+    sb_pdl_enter();
     // nb > 0: one sequence, heads head0 + i * head_step, output slot i.  nb == 0: every sequence and head of the call,
     // output slot ((sequence * g + head % g) * Hkv + head / g), i.e. the Hkv heads of one (sequence, group member) side by side
     const int nheads = nb > 0 ? nb : Hq;
@@ -469,9 +471,9 @@ at_score_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
         const int q = warp & 3, r = q * 32 + lane, half = (warp - 4) >> 2;
         const int qi = qb * AF_BQ + r;
         const bool live = qi < S;
-        const float cs = tc_pow2(-tc_f16_shift(__ldg(amax_q))) * tc_pow2(-tc_f16_shift(__ldg(amax_k))) * (scale * 1.4426950408889634f);
-        const float cp = tc_pow2(-tc_f16_shift(__ldg(amax_do))) * tc_pow2(-tc_f16_shift(__ldg(amax_v)));
-        const float dsc = tc_pow2(tc_f16_shift(__ldg(ds_bound))) * scale * (1.0f / 16384.f);      // pr holds P * 2^14
+        const float cs = tc_pow2(-tc_f16_shift(sb_word(amax_q))) * tc_pow2(-tc_f16_shift(sb_word(amax_k))) * (scale * 1.4426950408889634f);
+        const float cp = tc_pow2(-tc_f16_shift(sb_word(amax_do))) * tc_pow2(-tc_f16_shift(sb_word(amax_v)));
+        const float dsc = tc_pow2(tc_f16_shift(sb_word(ds_bound))) * scale * (1.0f / 16384.f);      // pr holds P * 2^14
         const float L2 = live ? lse[(size_t)(t0 + qi) * Hq + h] * 1.4426950408889634f : 0.f;
         const float Dq = live ? D[(size_t)(t0 + qi) * Hq + h] : 0.f;
         // after the transpose: lane (a, c) = (lane / 4, lane % 4) writes chunk c of the warp's rows 4a + t, t = 0..3
@@ -564,8 +566,7 @@ static int af_launch_fwd(sb_ctx_t* c, const void* q1, const void* q2, const void
         !af_make_map(c, &mV1, v1, T, kvd, AF_BKV) || !af_make_map(c, &mV2, v2, T, kvd, AF_BKV)) return 1;
     const long blocks = (long)nqb * seqs.n * Hq;
     if (blocks > 0x7fffffffL) return 1;
-    kern<<<(unsigned)blocks, AF_THREADS, smem, (cudaStream_t)c->pub.stream>>>(
-        mQ1, mQ2, mK1, mK2, mV1, mV2, seqs, O, lse, amax_q, amax_k, amax_v, Hq, Hq / Hkv, nqb, 1.0f / sqrtf((float)HD), c->d_status,
+    sb_launch(kern, dim3((unsigned)blocks), dim3(AF_THREADS), smem, (cudaStream_t)c->pub.stream, mQ1, mQ2, mK1, mK2, mV1, mV2, seqs, O, lse, amax_q, amax_k, amax_v, Hq, Hq / Hkv, nqb, 1.0f / sqrtf((float)HD), c->d_status,
         sb_amax_take(c, O, (size_t)T * qd));
     c->launches++;
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
@@ -614,8 +615,7 @@ extern "C" int sb_attention_fused_scores(sb_ctx_t* c, const void* q1, const void
         !af_make_map(c, &mV1, v1, T, kvd, AF_BKV) || !af_make_map(c, &mV2, v2, T, kvd, AF_BKV)) return 1;
     const long blocks = (long)nqb * seqs.n * (nb > 0 ? nb : Hq);
     if (blocks > 0x7fffffffL) return 1;
-    at_score_bwd_kernel<<<(unsigned)blocks, AS_THREADS, AS_SMEM, (cudaStream_t)c->pub.stream>>>(
-        mQ1, mQ2, mD1, mD2, mK1, mK2, mV1, mV2, lse, D, (__half*)P1, (__half*)P2, (__half*)dS1, (__half*)dS2,
+    sb_launch(at_score_bwd_kernel, dim3((unsigned)blocks), dim3(AS_THREADS), AS_SMEM, (cudaStream_t)c->pub.stream, mQ1, mQ2, mD1, mD2, mK1, mK2, mV1, mV2, lse, D, (__half*)P1, (__half*)P2, (__half*)dS1, (__half*)dS2,
         amax_q, amax_k, amax_v, amax_do, ds_bound, seqs, Sp, Hq, Hq / Hkv, head0, head_step, nb, nqb, 1.0f / sqrtf((float)hd), c->d_status);
     c->launches++;
     return cudaGetLastError() == cudaSuccess ? 0 : 1;

@@ -70,6 +70,7 @@ __device__ __forceinline__ void at_put_parts(__half* __restrict__ h1, __half* __
 __global__ void __launch_bounds__(256) at_softmax_rows(float* __restrict__ Sb, float* __restrict__ lse,
                                                        int S, int Sp, int Hq, int head0, int head_step, int tok0, float scale,
                                                        __half* __restrict__ P1, __half* __restrict__ P2) {
+    sb_pdl_enter();
     __shared__ float red[8];
     const int q = blockIdx.x, i = blockIdx.y, h = head0 + i * head_step;
     float* row = Sb + ((size_t)i * Sp + q) * Sp;
@@ -127,13 +128,14 @@ __global__ void __launch_bounds__(256) at_ds_rows(float* __restrict__ buf_s, flo
                                                   const float* __restrict__ D, int S, int Sp, int Hq, int head0, int head_step,
                                                   int tok0, float scale, __half* __restrict__ P1, __half* __restrict__ P2,
                                                   __half* __restrict__ dS1, __half* __restrict__ dS2, const float* __restrict__ ds_bound) {
+    sb_pdl_enter();
     const int q = blockIdx.x, i = blockIdx.y, h = head0 + i * head_step;
     float* srow = buf_s + ((size_t)i * Sp + q) * Sp;
     float* drow = buf_dp + ((size_t)i * Sp + q) * Sp;
     const float L = lse[(size_t)(tok0 + q) * Hq + h], Dq = D[(size_t)(tok0 + q) * Hq + h];
     const int zend = min(Sp, (q / AT_ROWTILE + 1) * AT_ROWTILE);
     const size_t rbase = ((size_t)i * Sp + q) * Sp;
-    const float dsc = P1 ? tc_pow2(tc_f16_shift(*ds_bound)) : 1.f;
+    const float dsc = P1 ? tc_pow2(tc_f16_shift(sb_word(ds_bound))) : 1.f;
     for (int k = threadIdx.x; k < zend; k += blockDim.x) {
         float p = 0.f, ds = 0.f;
         if (k <= q) { p = expf(srow[k] * scale - L); ds = p * (drow[k] - Dq) * scale; }
@@ -144,6 +146,7 @@ __global__ void __launch_bounds__(256) at_ds_rows(float* __restrict__ buf_s, flo
 
 // largest row norm of x[n_rows, hd] (one warp per row), as float bits through an integer atomicMax; out zeroed before
 __global__ void at_rownorm_max_kernel(const float* __restrict__ x, int n_rows, int hd, unsigned* __restrict__ out) {
+    sb_pdl_enter();
     const int lane = threadIdx.x & 31, nwarps = (gridDim.x * blockDim.x) >> 5;
     int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     float best = 0.f;
@@ -180,12 +183,14 @@ static inline int at_rn_blocks(sb_ctx_t* c, int n_rows) {
 // consts[0] = 1 (the largest possible P); consts[1] = 2 * max|dO row| * max|V row| * scale >= |dS| everywhere:
 // |dP| = |dO_q . V_k| <= the product of the norms, D_q is a convex combination of the dP_qk, P <= 1
 __global__ void at_consts_kernel(float* consts, const float* norms, float scale) {
+    sb_pdl_enter();
     consts[0] = 1.0f;
     consts[1] = 2.0f * norms[0] * norms[1] * scale;
 }
 
 // D[t,h] = sum_d dO[t,h,d] * O[t,h,d]; one warp per (t,h)
 __global__ void at_delta_kernel(const float* __restrict__ dO, const float* __restrict__ O, float* __restrict__ D, int n_th, int hd) {
+    sb_pdl_enter();
     int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (w >= n_th) return;
     const float* a = dO + (size_t)w * hd; const float* b = O + (size_t)w * hd;
@@ -202,6 +207,7 @@ template <int HD>
 __global__ void __launch_bounds__(256) at_bwd_prep_kernel(const float* __restrict__ dO, const float* __restrict__ O, float* __restrict__ D, int n_do,
                                                           const float* __restrict__ V, int n_v,
                                                           unsigned* __restrict__ norm_do, unsigned* __restrict__ amax, unsigned* __restrict__ norm_v) {
+    sb_pdl_enter();
     constexpr int LPR = HD / 4, RPW = 32 / LPR;
     const int lane = threadIdx.x & 31, sub = lane / LPR, l = lane % LPR, nwarps = (gridDim.x * blockDim.x) >> 5;
     const bool is_v = blockIdx.y != 0;
@@ -245,10 +251,11 @@ __global__ void __launch_bounds__(256) at_bwd_prep2_kernel(const float4* __restr
                                                            const float* __restrict__ amax, float* consts, const float* __restrict__ norms, float scale,
                                                            const float* __restrict__ lse, const float* __restrict__ D, float* __restrict__ LT, float* __restrict__ DT,
                                                            const AfSeqTab seqs, int Hq, int Smax, int slot_pitch, int natural) {
-    const float bound = 2.0f * __ldg(norms) * __ldg(norms + 1) * scale;
+    sb_pdl_enter();
+    const float bound = 2.0f * sb_word(norms) * sb_word(norms + 1) * scale;
     if (blockIdx.y == 0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) { consts[0] = 1.0f; consts[1] = bound; }
-        const float sc = tc_pow2(tc_f16_shift(__ldg(amax)));
+        const float sc = tc_pow2(tc_f16_shift(sb_word(amax)));
         const size_t nth = (size_t)gridDim.x * blockDim.x;
         for (size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n4; i0 += 2 * nth) {
             float4 v[2];
@@ -484,7 +491,7 @@ extern "C" int sb_attention_tc_forward(sb_ctx_t* c, const float* Q, const float*
         pq = at_make_parts(c, Q, n_q, hb, consts + 8);
         pk = at_make_parts(c, K, n_kv, hb + 2 * n_q, consts + 9);
         pv = at_make_parts(c, V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10);
-        at_consts_kernel<<<1, 1, 0, (cudaStream_t)c->pub.stream>>>(consts, consts + 2, scale);       // only consts[0] is used here
+        sb_launch(at_consts_kernel, dim3(1), dim3(1), 0, (cudaStream_t)c->pub.stream, consts, consts + 2, scale);       // only consts[0] is used here
         c->launches++;
     }
     bool ok = true;
@@ -505,7 +512,7 @@ extern "C" int sb_attention_tc_forward(sb_ctx_t* c, const float* Q, const float*
                 const int nb = min(G, Hkv - i0), qh0 = r + i0 * g;
                 ok = ok && at_gemm(c, op_tokens(Q, pq, t0, S, qd, Hq, hd, qh0, g), op_tokens(K, pk, t0, S, kvd, Hkv, hd, i0, 1),
                                    Sb, Sp, (long)Sp * Sp, S, S, hd, 0, nb, TC_CAUSAL_SKIP_UPPER, nullptr, pq.amax, pk.amax);
-                at_softmax_rows<<<dim3(S, nb), 256, 0, s>>>(Sb, lse, S, Sp, Hq, qh0, g, t0, scale, P1, P2);
+                sb_launch(at_softmax_rows, dim3(dim3(S, nb)), dim3(256), 0, s, Sb, lse, S, Sp, Hq, qh0, g, t0, scale, P1, P2);
                 c->launches++;
                 ok = ok && at_gemm(c, op_scratch(Sb, pp, S, Sp, nb, 0), op_tokens_mn(V, pv, t0, kvd, Hkv, hd, i0, 1),
                                    O + (size_t)t0 * qd + (size_t)qh0 * hd, qd, (long)g * hd, S, hd, S, 0, nb, TC_CAUSAL_K_UPTO_M,
@@ -539,8 +546,8 @@ static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, cons
         const int rpb = 8 * 4 * (128 / hd);                          // rows a CTA takes per pass
         const int cap = c->pub.gpu_sm_count * 8, want = (T * Hq + rpb - 1) / rpb;
         const dim3 pg(want < cap ? want : cap, 2);
-        if (hd == 128) at_bwd_prep_kernel<128><<<pg, 256, 0, st>>>(dO, O, D, T * Hq, V, T * Hkv, (unsigned*)(consts + 2), (unsigned*)(consts + 11), (unsigned*)(consts + 3));
-        else at_bwd_prep_kernel<64><<<pg, 256, 0, st>>>(dO, O, D, T * Hq, V, T * Hkv, (unsigned*)(consts + 2), (unsigned*)(consts + 11), (unsigned*)(consts + 3));
+        if (hd == 128) sb_launch(at_bwd_prep_kernel<128>, dim3(pg), dim3(256), 0, st, dO, O, D, T * Hq, V, T * Hkv, (unsigned*)(consts + 2), (unsigned*)(consts + 11), (unsigned*)(consts + 3));
+        else sb_launch(at_bwd_prep_kernel<64>, dim3(pg), dim3(256), 0, st, dO, O, D, T * Hq, V, T * Hkv, (unsigned*)(consts + 2), (unsigned*)(consts + 11), (unsigned*)(consts + 3));
         c->launches++;
     }
     // from here on the launches depend on the boundaries
@@ -560,7 +567,7 @@ static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, cons
     float* LT = bb + n_ds; float* DT = LT + row_floats;
     {
         const AfSeqTab seqs = {n, c->attn_seq_starts};
-        at_bwd_prep2_kernel<<<dim3(tc_ew_blocks(c, n_q / 8), 2), 256, 0, st>>>((const float4*)dO, n_q / 4, (uint2*)hdo, (uint2*)(hdo + n_q), consts + 11,
+        sb_launch(at_bwd_prep2_kernel, dim3(dim3(tc_ew_blocks(c, n_q / 8), 2)), dim3(256), 0, st, (const float4*)dO, n_q / 4, (uint2*)hdo, (uint2*)(hdo + n_q), consts + 11,
                                                                             consts, consts + 2, scale, lse, D, LT, DT, seqs, Hq, Smax, slot_pitch, hd == 64 ? 1 : 0);
         c->launches++;
     }
@@ -624,7 +631,7 @@ extern "C" int sb_attention_tc_backward(sb_ctx_t* c, const float* Q, const float
     AtParts pq = AT_NOPARTS, pk = AT_NOPARTS, pv = AT_NOPARTS, pdo = AT_NOPARTS;
     cudaStream_t s0 = (cudaStream_t)c->pub.stream;
     int tk = sb_tick_begin(c, SB_CLS_ATTN_BWD);
-    at_delta_kernel<<<(T * Hq * 32 + 255) / 256, 256, 0, s0>>>(dO, O, D, T * Hq, hd);
+    sb_launch(at_delta_kernel, dim3((T * Hq * 32 + 255) / 256), dim3(256), 0, s0, dO, O, D, T * Hq, hd);
     c->launches++;
     if (f16) {
         __half* hb = (__half*)(consts + 64);
@@ -633,9 +640,9 @@ extern "C" int sb_attention_tc_backward(sb_ctx_t* c, const float* Q, const float
         pv = at_make_parts(c, V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10);
         pdo = at_make_parts(c, dO, n_q, hb + 2 * n_q + 4 * n_kv, consts + 11);
         cudaMemsetAsync(consts + 2, 0, 2 * sizeof(float), s0);
-        at_rownorm_max_kernel<<<at_rn_blocks(c, T * Hq), 256, 0, s0>>>(dO, T * Hq, hd, (unsigned*)(consts + 2));
-        at_rownorm_max_kernel<<<at_rn_blocks(c, T * Hkv), 256, 0, s0>>>(V, T * Hkv, hd, (unsigned*)(consts + 3));
-        at_consts_kernel<<<1, 1, 0, s0>>>(consts, consts + 2, scale);
+        sb_launch(at_rownorm_max_kernel, dim3(at_rn_blocks(c, T * Hq)), dim3(256), 0, s0, dO, T * Hq, hd, (unsigned*)(consts + 2));
+        sb_launch(at_rownorm_max_kernel, dim3(at_rn_blocks(c, T * Hkv)), dim3(256), 0, s0, V, T * Hkv, hd, (unsigned*)(consts + 3));
+        sb_launch(at_consts_kernel, dim3(1), dim3(1), 0, s0, consts, consts + 2, scale);
         c->launches += 3;
     }
     bool ok = true;
@@ -685,7 +692,7 @@ extern "C" int sb_attention_tc_backward(sb_ctx_t* c, const float* Q, const float
                                        b0, Sp, sb, S, S, hd, 0, nb, TC_CAUSAL_SKIP_UPPER, nullptr, pq.amax, pk.amax);     // S
                     ok = ok && at_gemm(c, op_tokens(dO, pdo, t0, S, qd, Hq, hd, qh0, g), op_tokens(V, pv, t0, S, kvd, Hkv, hd, i0, 1),
                                        b1, Sp, sb, S, S, hd, 0, nb, TC_CAUSAL_SKIP_UPPER, nullptr, pdo.amax, pv.amax);    // dP
-                    at_ds_rows<<<dim3(S, nb), 256, 0, s>>>(b0, b1, lse, D, S, Sp, Hq, qh0, g, t0, scale, P1, P2, dS1, dS2, consts + 1);   // P, dS
+                    sb_launch(at_ds_rows, dim3(dim3(S, nb)), dim3(256), 0, s, b0, b1, lse, D, S, Sp, Hq, qh0, g, t0, scale, P1, P2, dS1, dS2, consts + 1);   // P, dS
                     c->launches++;
                 }
                 const int acc = (r > 0 || accumulate_kv) ? 1 : 0;

@@ -40,6 +40,7 @@ __device__ __forceinline__ float ew_apply(float a, float b) {
 template <int OP, bool BINARY>
 __global__ void __launch_bounds__(EW_THREADS) ew_kernel(const float* __restrict__ a, const float* __restrict__ b,
                                                         float* __restrict__ c, size_t n, int vec_ok, unsigned* amax_out) {
+    sb_pdl_enter();
     size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
     float am = 0.f;                                       // largest |output| of this thread (asked for by the next GEMM's operand split)
     if (vec_ok) {
@@ -66,12 +67,13 @@ static void ew_launch(sb_ctx_t* c, const float* a, const float* b, float* o, siz
     if (!n) return;
     int vec = aligned16(a) && aligned16(o) && (!BINARY || aligned16(b));
     int tk = sb_tick_begin(c, OP == OP_SWIGLU ? SB_CLS_SWIGLU : SB_CLS_OTHER);
-    ew_kernel<OP, BINARY><<<ew_grid(c, (n + 3) / 4), EW_THREADS, 0, (cudaStream_t)c->pub.stream>>>(a, b, o, n, vec, OP == OP_SWIGLU ? sb_amax_take(c, o, n) : (unsigned*)nullptr);
+    sb_launch(ew_kernel<OP, BINARY>, dim3(ew_grid(c, (n + 3) / 4)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, a, b, o, n, vec, OP == OP_SWIGLU ? sb_amax_take(c, o, n) : (unsigned*)nullptr);
     sb_tick_end(c, tk, 0.0, (BINARY ? 12.0 : 8.0) * (double)n);
     c->launches++;
 }
 
 __global__ void __launch_bounds__(EW_THREADS) scale_kernel(float* x, size_t n, float alpha) {
+    sb_pdl_enter();
     size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
     for (size_t i = tid; i < n; i += nth) x[i] *= alpha;
 }
@@ -80,6 +82,7 @@ __global__ void __launch_bounds__(EW_THREADS) scale_kernel(float* x, size_t n, f
 __global__ void __launch_bounds__(EW_THREADS) mul_bwd_kernel(const float* __restrict__ A, const float* __restrict__ B,
                                                              const float* __restrict__ dC, float* __restrict__ dA,
                                                              float* __restrict__ dB, size_t n) {
+    sb_pdl_enter();
     size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
     for (size_t i = tid; i < n; i += nth) { float g = dC[i], a = A[i], b = B[i]; dA[i] = g * b; dB[i] = g * a; }
 }
@@ -92,6 +95,7 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_kernel(const float* __r
                                                                 const float* __restrict__ dout, float* __restrict__ dgate,
                                                                 float* __restrict__ dup, size_t n, int vec_ok,
                                                                 unsigned* amax_dgate, unsigned* amax_dup) {
+    sb_pdl_enter();
     size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
     float amg = 0.f, amu = 0.f;
 #define SWIGLU_BWD_ONE(g, u, d, dg, du) { float sg = sigmoidf_(g); float si = (g) * sg; \
@@ -122,8 +126,9 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_kernel(const float* __r
 __global__ void __launch_bounds__(EW_THREADS) swiglu_parts_kernel(const float4* __restrict__ gate, const float4* __restrict__ up,
                                                                   uint2* __restrict__ h1, uint2* __restrict__ h2, size_t n4,
                                                                   const float* __restrict__ amax_g, const float* __restrict__ amax_u,
-                                                                  float* __restrict__ bound_out) {
-    const float bound = fminf(__ldg(amax_g) * __ldg(amax_u), 3.0e38f);
+                                                                  float* __restrict__ bound_out, unsigned keep) {
+    sb_pdl_enter();
+    const float bound = fminf(sb_word(amax_g) * sb_word(amax_u), 3.0e38f);
     const float sc = sb_pow2(sb_f16_shift(bound));
     if (blockIdx.x == 0 && threadIdx.x == 0) *bound_out = bound;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
@@ -131,7 +136,7 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_parts_kernel(const float4* 
         const float r0 = ew_apply<OP_SWIGLU>(g.x, u.x) * sc, r1 = ew_apply<OP_SWIGLU>(g.y, u.y) * sc;
         const float r2 = ew_apply<OP_SWIGLU>(g.z, u.z) * sc, r3 = ew_apply<OP_SWIGLU>(g.w, u.w) * sc;
         uint2 a, b;
-        sb_split2(r0, r1, a.x, b.x); sb_split2(r2, r3, a.y, b.y);
+        sb_split2(r0, r1, a.x, b.x, keep); sb_split2(r2, r3, a.y, b.y, keep);
         h1[i] = a; h2[i] = b;
     }
 }
@@ -141,9 +146,10 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_parts_kernel(const floa
                                                                       uint2* __restrict__ du1, uint2* __restrict__ du2, size_t n4,
                                                                       const float* __restrict__ amax_g, const float* __restrict__ amax_u,
                                                                       const float* __restrict__ amax_d,
-                                                                      float* __restrict__ bound_dg, float* __restrict__ bound_du) {
-    const float ad = __ldg(amax_d);
-    const float bg = fminf(1.1f * ad * __ldg(amax_u), 3.0e38f), bu = fminf(ad * __ldg(amax_g), 3.0e38f);
+                                                                      float* __restrict__ bound_dg, float* __restrict__ bound_du, unsigned keep) {
+    sb_pdl_enter();
+    const float ad = sb_word(amax_d);
+    const float bg = fminf(1.1f * ad * sb_word(amax_u), 3.0e38f), bu = fminf(ad * sb_word(amax_g), 3.0e38f);
     const float sg_ = sb_pow2(sb_f16_shift(bg)), su = sb_pow2(sb_f16_shift(bu));
     if (blockIdx.x == 0 && threadIdx.x == 0) { *bound_dg = bg; *bound_du = bu; }
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
@@ -152,8 +158,8 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_parts_kernel(const floa
         SWIGLU_BWD_ONE(g.x, u.x, d.x, dg.x, du.x) SWIGLU_BWD_ONE(g.y, u.y, d.y, dg.y, du.y)
         SWIGLU_BWD_ONE(g.z, u.z, d.z, dg.z, du.z) SWIGLU_BWD_ONE(g.w, u.w, d.w, dg.w, du.w)
         uint2 a, b, e, f;
-        sb_split2(dg.x * sg_, dg.y * sg_, a.x, b.x); sb_split2(dg.z * sg_, dg.w * sg_, a.y, b.y);
-        sb_split2(du.x * su, du.y * su, e.x, f.x); sb_split2(du.z * su, du.w * su, e.y, f.y);
+        sb_split2(dg.x * sg_, dg.y * sg_, a.x, b.x, keep); sb_split2(dg.z * sg_, dg.w * sg_, a.y, b.y, keep);
+        sb_split2(du.x * su, du.y * su, e.x, f.x, keep); sb_split2(du.z * su, du.w * su, e.y, f.y, keep);
         dg1[i] = a; dg2[i] = b; du1[i] = e; du2[i] = f;
     }
 }
@@ -162,6 +168,7 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_parts_kernel(const floa
 // beyond the table set the status word and read row 0 instead of faulting.
 __global__ void __launch_bounds__(EW_THREADS) embed_lookup_kernel(const uint32_t* __restrict__ tok, const float* __restrict__ E,
                                                                   float* __restrict__ out, int T, int d, int V, int vec, int* status) {
+    sb_pdl_enter();
     for (int t = blockIdx.x; t < T; t += gridDim.x) {
         uint32_t id = tok[t];
         if (id >= (uint32_t)V) { if (threadIdx.x == 0) atomicExch(status, SB_ERR_TOKEN_RANGE); id = 0; }
@@ -176,6 +183,7 @@ __global__ void __launch_bounds__(EW_THREADS) embed_lookup_kernel(const uint32_t
 
 // position of each packed row inside its sequence, and the sequence index
 __global__ void seq_index_kernel(const uint32_t* __restrict__ ss, int B, int T, uint32_t* pos_ids, uint32_t* seq_ids) {
+    sb_pdl_enter();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T) return;
     int lo = 0, hi = B;
@@ -188,6 +196,7 @@ __global__ void seq_index_kernel(const uint32_t* __restrict__ ss, int B, int T, 
 // cos/sin table [max_pos, hd/2] built with the same FP32 expression the
 // reference evaluates per element: angle = pos * (1/powf(theta, 2p/hd)).
 __global__ void rope_table_kernel(float2* tab, int max_pos, int half, int hd, float theta) {
+    sb_pdl_enter();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= max_pos * half) return;
     int pos = i / half, p = i % half;
@@ -206,6 +215,7 @@ __global__ void __launch_bounds__(EW_THREADS) rope_kernel(const float* qin, floa
                                                           const uint32_t* __restrict__ pos_ids, const float2* __restrict__ tab,
                                                           int T, int Hq, int Hkv, int hd, int backward,
                                                           unsigned* amax_q, unsigned* amax_k) {
+    sb_pdl_enter();
     float amq = 0.f, amk = 0.f;
     const uint32_t quads = (uint32_t)hd >> 2, rq = (uint32_t)Hq * quads, rk = kin ? (uint32_t)Hkv * quads : 0u, row_quads = rq + rk;
     const uint32_t total = (uint32_t)T * row_quads;
@@ -252,6 +262,7 @@ __global__ void __launch_bounds__(EW_THREADS) rope_kernel(const float* qin, floa
 // pair-at-a-time variant for head_dim not divisible by 4 or unaligned buffers
 __global__ void rope_pair_kernel(const float* __restrict__ in, float* __restrict__ out, const uint32_t* __restrict__ pos_ids,
                                  const float2* __restrict__ tab, int T, int H, int hd, int backward) {
+    sb_pdl_enter();
     int half = hd >> 1;
     size_t total = (size_t)T * H * half;
     size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
@@ -266,6 +277,7 @@ __global__ void rope_pair_kernel(const float* __restrict__ in, float* __restrict
 }
 
 __global__ void __launch_bounds__(EW_THREADS) nan_check_kernel(const float* __restrict__ x, size_t n, uint32_t* flags, uint32_t idx) {
+    sb_pdl_enter();
     size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
     bool bad = false;
     for (size_t i = tid; i < n; i += nth) { float v = x[i]; bad |= (isnan(v) || isinf(v)); }
@@ -282,13 +294,13 @@ void sb_swiglu(sb_ctx_t* c, const float* g, const float* u, float* o, size_t n) 
 
 void sb_scale(sb_ctx_t* c, float* a, size_t n, float alpha) {
     if (!n) return;
-    scale_kernel<<<ew_grid(c, n), EW_THREADS, 0, (cudaStream_t)c->pub.stream>>>(a, n, alpha);
+    sb_launch(scale_kernel, dim3(ew_grid(c, n)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, a, n, alpha);
     c->launches++;
 }
 
 void sb_mul_backward(sb_ctx_t* c, const float* A, const float* B, const float* dC, float* dA, float* dB, size_t n) {
     if (!n) return;
-    mul_bwd_kernel<<<ew_grid(c, n), EW_THREADS, 0, (cudaStream_t)c->pub.stream>>>(A, B, dC, dA, dB, n);
+    sb_launch(mul_bwd_kernel, dim3(ew_grid(c, n)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, A, B, dC, dA, dB, n);
     c->launches++;
 }
 
@@ -297,7 +309,7 @@ void sb_swiglu_backward(sb_ctx_t* c, const float* gate, const float* up, const f
     int vec = aligned16(gate) && aligned16(up) && aligned16(dout) && aligned16(dgate) && aligned16(dup);
     sb_parts_invalidate(c, dgate); sb_parts_invalidate(c, dup);
     int tk = sb_tick_begin(c, SB_CLS_SWIGLU);
-    swiglu_bwd_kernel<<<ew_grid(c, (n + 3) / 4), EW_THREADS, 0, (cudaStream_t)c->pub.stream>>>(gate, up, dout, dgate, dup, n, vec,
+    sb_launch(swiglu_bwd_kernel, dim3(ew_grid(c, (n + 3) / 4)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, gate, up, dout, dgate, dup, n, vec,
                                                                                                   sb_amax_take(c, dgate, n), sb_amax_take(c, dup, n));
     sb_tick_end(c, tk, 0.0, 20.0 * (double)n);
     c->launches++;
@@ -311,8 +323,8 @@ int sb_swiglu_parts(sb_ctx_t* c, const float* gate, const float* up, float* out,
     if (!sb_parts_find(c, out, n, &h, &bound, &fresh)) return 0;
     sb_amax_forget(c, out);
     int tk = sb_tick_begin(c, SB_CLS_SWIGLU);
-    swiglu_parts_kernel<<<ew_grid(c, n / 4), EW_THREADS, 0, (cudaStream_t)c->pub.stream>>>((const float4*)gate, (const float4*)up, (uint2*)h,
-                                                                                         (uint2*)((uint16_t*)h + n), n / 4, ag, au, bound);
+    sb_launch(swiglu_parts_kernel, dim3(ew_grid(c, n / 4)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (const float4*)gate, (const float4*)up, (uint2*)h,
+                                                                                         (uint2*)((uint16_t*)h + n), n / 4, ag, au, bound, sb_parts_keep(c));
     sb_tick_end(c, tk, 0.0, 12.0 * (double)n);
     c->launches++;
     return 1;
@@ -325,9 +337,8 @@ int sb_swiglu_backward_parts(sb_ctx_t* c, const float* gate, const float* up, co
     if (!sb_parts_find(c, dgate, n, &hg, &bg, &fresh) || !sb_parts_find(c, dup, n, &hu, &bu, &fresh)) return 0;
     sb_amax_forget(c, dgate); sb_amax_forget(c, dup);
     int tk = sb_tick_begin(c, SB_CLS_SWIGLU);
-    swiglu_bwd_parts_kernel<<<ew_grid(c, n / 4), EW_THREADS, 0, (cudaStream_t)c->pub.stream>>>(
-        (const float4*)gate, (const float4*)up, (const float4*)dout, (uint2*)hg, (uint2*)((uint16_t*)hg + n), (uint2*)hu, (uint2*)((uint16_t*)hu + n),
-        n / 4, ag, au, ad, bg, bu);
+    sb_launch(swiglu_bwd_parts_kernel, dim3(ew_grid(c, n / 4)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (const float4*)gate, (const float4*)up, (const float4*)dout, (uint2*)hg, (uint2*)((uint16_t*)hg + n), (uint2*)hu, (uint2*)((uint16_t*)hu + n),
+        n / 4, ag, au, ad, bg, bu, sb_parts_keep(c));
     sb_tick_end(c, tk, 0.0, 20.0 * (double)n);
     c->launches++;
     return 1;
@@ -339,14 +350,14 @@ void sb_embed_lookup(sb_ctx_t* c, const uint32_t* tok, const float* E, float* ou
     int grid = T < sms * 8 ? T : sms * 8;
     int vec = ((d & 3) == 0) && aligned16(E) && aligned16(out);
     int tk = sb_tick_begin(c, SB_CLS_EMBED);
-    embed_lookup_kernel<<<grid, EW_THREADS, 0, (cudaStream_t)c->pub.stream>>>(tok, E, out, T, d, V, vec, c->d_status);
+    sb_launch(embed_lookup_kernel, dim3(grid), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, tok, E, out, T, d, V, vec, c->d_status);
     sb_tick_end(c, tk, 0.0, 8.0 * T * d);
     c->launches++;
 }
 
 void sb_seq_index(sb_ctx_t* c, const uint32_t* seq_starts, int B, int T, uint32_t* pos_ids, uint32_t* seq_ids) {
     if (T <= 0) return;
-    seq_index_kernel<<<(T + 255) / 256, 256, 0, (cudaStream_t)c->pub.stream>>>(seq_starts, B, T, pos_ids, seq_ids);
+    sb_launch(seq_index_kernel, dim3((T + 255) / 256), dim3(256), 0, (cudaStream_t)c->pub.stream, seq_starts, B, T, pos_ids, seq_ids);
     c->launches++;
 }
 
@@ -361,7 +372,7 @@ static bool rope_ensure_table(sb_ctx_t* c, int hd, float theta, int max_pos) {
     if (sb_check(c, cudaMalloc(&c->rope_tab, (size_t)cap * half * sizeof(float2)), "rope table")) return false;
     c->rope_tab_pos = cap; c->rope_tab_hd = hd; c->rope_tab_theta = theta;
     int n = cap * half;
-    rope_table_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)c->pub.stream>>>((float2*)c->rope_tab, cap, half, hd, theta);
+    sb_launch(rope_table_kernel, dim3((n + 255) / 256), dim3(256), 0, (cudaStream_t)c->pub.stream, (float2*)c->rope_tab, cap, half, hd, theta);
     c->launches++;
     return true;
 }
@@ -374,10 +385,10 @@ void sb_rope(sb_ctx_t* c, const float* in, float* out, const uint32_t* pos_ids, 
     int tk = sb_tick_begin(c, SB_CLS_ROPE);
     if ((hd & 3) == 0 && aligned16(in) && aligned16(out) && aligned16(c->rope_tab) && (double)T * H * (hd / 4) < 2147483648.0) {
         size_t work = ((size_t)T * H * (hd / 4) + ROPE_UNROLL - 1) / ROPE_UNROLL;
-        rope_kernel<<<ew_grid(c, work), EW_THREADS, 0, (cudaStream_t)c->pub.stream>>>(in, out, nullptr, nullptr, pos_ids, (const float2*)c->rope_tab, T, H, 0, hd, backward, nullptr, nullptr);
+        sb_launch(rope_kernel, dim3(ew_grid(c, work)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, in, out, nullptr, nullptr, pos_ids, (const float2*)c->rope_tab, T, H, 0, hd, backward, nullptr, nullptr);
     } else {
         size_t work = (size_t)T * H * half;
-        rope_pair_kernel<<<ew_grid(c, work), EW_THREADS, 0, (cudaStream_t)c->pub.stream>>>(in, out, pos_ids, (const float2*)c->rope_tab, T, H, hd, backward);
+        sb_launch(rope_pair_kernel, dim3(ew_grid(c, work)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, in, out, pos_ids, (const float2*)c->rope_tab, T, H, hd, backward);
     }
     sb_tick_end(c, tk, 0.0, 8.0 * T * H * hd);
     c->launches++;
@@ -395,7 +406,7 @@ void sb_rope2(sb_ctx_t* c, float* q, float* k, const uint32_t* pos_ids, int T, i
     if (!rope_ensure_table(c, hd, theta, max_pos)) return;
     int tk = sb_tick_begin(c, SB_CLS_ROPE);
     size_t work = ((size_t)nq + ROPE_UNROLL - 1) / ROPE_UNROLL;
-    rope_kernel<<<ew_grid(c, work), EW_THREADS, 0, (cudaStream_t)c->pub.stream>>>(q, q, k, k, pos_ids, (const float2*)c->rope_tab, T, Hq, Hkv, hd, backward,
+    sb_launch(rope_kernel, dim3(ew_grid(c, work)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, q, q, k, k, pos_ids, (const float2*)c->rope_tab, T, Hq, Hkv, hd, backward,
                                                                                    sb_amax_take(c, q, (size_t)T * Hq * hd), sb_amax_take(c, k, (size_t)T * Hkv * hd));
     sb_tick_end(c, tk, 0.0, 8.0 * T * (Hq + Hkv) * hd);
     c->launches++;
@@ -403,7 +414,7 @@ void sb_rope2(sb_ctx_t* c, float* q, float* k, const uint32_t* pos_ids, int T, i
 
 void sb_nan_check(sb_ctx_t* c, const float* x, size_t n, uint32_t* flags, uint32_t idx) {
     if (!n) return;
-    nan_check_kernel<<<ew_grid(c, n), EW_THREADS, 0, (cudaStream_t)c->pub.stream>>>(x, n, flags, idx);
+    sb_launch(nan_check_kernel, dim3(ew_grid(c, n)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, x, n, flags, idx);
     c->launches++;
 }
 

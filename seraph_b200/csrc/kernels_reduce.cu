@@ -42,6 +42,7 @@ __device__ __forceinline__ void block_sum2(float& a, float& b, float* red) {
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(RB_THREADS) rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                              float* __restrict__ y, int rows, int cols, float eps, int vec) {
+    sb_pdl_enter();
     __shared__ float red[64];
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
         const float* xr = x + (size_t)r * cols; float* yr = y + (size_t)r * cols;
@@ -70,6 +71,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_bwd_kernel(const float* __
                                                                  const float* __restrict__ dy, const float* __restrict__ resid,
                                                                  float* __restrict__ dx, float* __restrict__ partial,
                                                                  int rows, int cols, float eps, int vec) {
+    sb_pdl_enter();
     __shared__ float red[64];
     float acc[RN_MAX_SWEEP * 4];
 #pragma unroll
@@ -136,6 +138,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_bwd_kernel(const float* __
 template <int NV>
 __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                   float* __restrict__ y, int rows, int cols, float eps, unsigned* amax_out) {
+    sb_pdl_enter();
     const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int c4 = cols >> 2;
     float am = 0.f;
@@ -170,6 +173,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_kernel(const float* _
 // flight together, so that a warp has 2 KB of loads outstanding instead of 512 bytes.
 __global__ void __launch_bounds__(RB_THREADS) rmsnorm_w128_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y,
                                                                   int rows, float eps, unsigned* amax_out) {
+    sb_pdl_enter();
     const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const float4 s = ((const float4*)w)[lane];
     float am = 0.f;
@@ -268,6 +272,7 @@ template <int NC>
 __global__ void __launch_bounds__(RB_THREADS, 2) rmsnorm_bwd_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                          const float* __restrict__ dy, const float* resid, float* dx,
                                                                          float* __restrict__ partial, int rows, int cols, float eps, unsigned* amax_dx) {
+    sb_pdl_enter();
     float am = 0.f;
     __shared__ float s_red[2][RB_THREADS / 32][2 * RNB_ROWS];
     __shared__ float s_tot[2][2 * RNB_ROWS];
@@ -306,6 +311,7 @@ __global__ void __launch_bounds__(RB_THREADS, 2) rmsnorm_bwd_rows_kernel(const f
 __global__ void __launch_bounds__(RB_THREADS, 4) rmsnorm_bwd_w128_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                          const float* __restrict__ dy, const float* resid, float* dx,
                                                                          float* __restrict__ partial, int rows, float eps, unsigned* amax_dx) {
+    sb_pdl_enter();
     __shared__ float4 s_acc[RB_THREADS / 32][32];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = (gridDim.x * RB_THREADS) >> 5;
     const float4 sc = ((const float4*)w)[lane];
@@ -354,6 +360,7 @@ __global__ void __launch_bounds__(RB_THREADS, 4) rmsnorm_bwd_w128_kernel(const f
 #define CS_GROUPS 32
 #define CS_BATCH 10
 __global__ void __launch_bounds__(32 * CS_GROUPS) colsum_partials_kernel(const float* __restrict__ partial, float* __restrict__ dscale, int nblocks, int cols) {
+    sb_pdl_enter();
     __shared__ float s_part[CS_GROUPS][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int cidx = blockIdx.x * 32 + tx;
@@ -384,6 +391,7 @@ __global__ void __launch_bounds__(32 * CS_GROUPS) colsum_partials_kernel(const f
 // Row softmax (kept for API completeness; no training step uses it)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(RB_THREADS) softmax_kernel(const float* __restrict__ x, float* __restrict__ y, int rows, int cols) {
+    sb_pdl_enter();
     __shared__ float red[64];
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
         const float* xr = x + (size_t)r * cols; float* yr = y + (size_t)r * cols;
@@ -415,7 +423,8 @@ __global__ void __launch_bounds__(RB_THREADS) softmax_kernel(const float* __rest
 template <int NV>
 __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                         uint2* __restrict__ h1, uint2* __restrict__ h2, int rows, int cols, float eps,
-                                                                        float* __restrict__ bound_out) {
+                                                                        float* __restrict__ bound_out, unsigned keep) {
+    sb_pdl_enter();
     const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int c4 = cols >> 2;
     float wm = 0.f;                       // (w is read again from cache in the output loop: keeping it would double the registers)
@@ -450,7 +459,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const fl
                 const float4 s = ((const float4*)w)[j];
                 const float y0 = v[i].x * inv * s.x, y1 = v[i].y * inv * s.y, y2 = v[i].z * inv * s.z, y3 = v[i].w * inv * s.w;
                 uint2 a, b;
-                sb_split2(y0 * sc, y1 * sc, a.x, b.x); sb_split2(y2 * sc, y3 * sc, a.y, b.y);
+                sb_split2(y0 * sc, y1 * sc, a.x, b.x, keep); sb_split2(y2 * sc, y3 * sc, a.y, b.y, keep);
                 o1[j] = a; o2[j] = b;
             }
         }
@@ -458,6 +467,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const fl
 }
 template <int NV>
 __global__ void __launch_bounds__(RB_THREADS) qk_norm_warp_kernel(float* __restrict__ x, float* __restrict__ rms_out, int rows, int cols, float eps) {
+    sb_pdl_enter();
     const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int c4 = cols >> 2;
     for (int r = warp; r < rows; r += nwarps) {
@@ -484,6 +494,7 @@ __global__ void __launch_bounds__(RB_THREADS) qk_norm_warp_kernel(float* __restr
 template <int NV>
 __global__ void __launch_bounds__(RB_THREADS) qk_norm_bwd_warp_kernel(const float* __restrict__ y, const float* __restrict__ rms,
                                                                       const float* dy, float* dx, int rows, int cols, float eps) {
+    sb_pdl_enter();
     const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int c4 = cols >> 2;
     for (int r = warp; r < rows; r += nwarps) {
@@ -513,6 +524,7 @@ __global__ void __launch_bounds__(RB_THREADS) qk_norm_bwd_warp_kernel(const floa
 // any shape: one CTA per row, two passes over the row
 __global__ void __launch_bounds__(RB_THREADS) qk_norm_row_kernel(float* __restrict__ x, float* __restrict__ rms_out, const float* __restrict__ rms_in,
                                                                  const float* dy, float* dx, int rows, int cols, float eps) {
+    sb_pdl_enter();
     __shared__ float red[RB_THREADS / 32];
     __shared__ float tot;
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -552,7 +564,8 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(const float* 
                                                                    const uint32_t* __restrict__ pos_ids, const uint32_t* __restrict__ seq_ids,
                                                                    const uint32_t* __restrict__ seq_starts,
                                                                    int T, int V, float inv_valid, int vec, int* status, unsigned* amax_grad,
-                                                                   __half* __restrict__ g1, __half* __restrict__ g2, float part_scale, float* part_amax) {
+                                                                   __half* __restrict__ g1, __half* __restrict__ g2, float part_scale, float* part_amax, unsigned keep) {
+    sb_pdl_enter();
     // g1 != NULL (vec only): the gradient leaves as the two FP16 parts the LM-head backward products read, h1 = fp16(g * part_scale),
     // h2 = fp16(g * part_scale - h1), laid out like grad; nothing is written to grad.  |g| <= inv_valid everywhere (softmax minus
     // one-hot, over the number of predictions), so the parts' scale is known before a single logit is read: *part_amax = inv_valid.
@@ -603,10 +616,9 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(const float* 
         g.x *= inv_valid; g.y *= inv_valid; g.z *= inv_valid; g.w *= inv_valid;
         if (g1) {
             const float q0 = g.x * part_scale, q1 = g.y * part_scale, q2 = g.z * part_scale, q3 = g.w * part_scale;
-            const __half2 ha = __floats2half2_rn(q0, q1), hb = __floats2half2_rn(q2, q3);
-            const float2 fa = __half22float2(ha), fb = __half22float2(hb);
-            const __half2 la = __floats2half2_rn(q0 - fa.x, q1 - fa.y), lb = __floats2half2_rn(q2 - fb.x, q3 - fb.y);
-            p1[i] = make_uint2(*(const uint32_t*)&ha, *(const uint32_t*)&hb); p2[i] = make_uint2(*(const uint32_t*)&la, *(const uint32_t*)&lb);
+            uint2 h, l;
+            sb_split2(q0, q1, h.x, l.x, keep); sb_split2(q2, q3, h.y, l.y, keep);
+            p1[i] = h; p2[i] = l;
         } else {
             ((float4*)gr)[i] = g;
             am = sb_amax4(am, g);
@@ -625,6 +637,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(const float* 
 // ---------------------------------------------------------------------------
 template <bool SQUARE>
 __global__ void __launch_bounds__(RB_THREADS) partial_sum_kernel(const float* __restrict__ x, size_t n, float* __restrict__ partial, int vec) {
+    sb_pdl_enter();
     __shared__ float red[64];
     size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
     float s = 0.f, d0 = 0.f;
@@ -640,6 +653,7 @@ __global__ void __launch_bounds__(RB_THREADS) partial_sum_kernel(const float* __
     if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 __global__ void final_sum_kernel(const float* __restrict__ partial, int n, float* out) {
+    sb_pdl_enter();
     __shared__ float red[64];
     float s = 0.f, d0 = 0.f;
     for (int i = threadIdx.x; i < n; i += blockDim.x) s += partial[i];
@@ -660,6 +674,7 @@ __global__ void final_sum_kernel(const float* __restrict__ partial, int n, float
 #define EB_CHUNK 1024
 __global__ void __launch_bounds__(EB_CHUNK) eb_count_kernel(const uint32_t* __restrict__ tok, int T, int V,
                                                             int* __restrict__ chunk_cnt, int* __restrict__ cnt, int* status) {
+    sb_pdl_enter();
     int t = blockIdx.x * EB_CHUNK + threadIdx.x;
     if (t >= T) return;
     uint32_t id = tok[t];
@@ -671,6 +686,7 @@ __global__ void __launch_bounds__(EB_CHUNK) eb_count_kernel(const uint32_t* __re
 // single CTA: exclusive scan of cnt[V] -> start[V]; compaction of rows with cnt>0 -> rows[], meta[0] = U
 __global__ void __launch_bounds__(1024) eb_scan_kernel(const int* __restrict__ cnt, int V, int* __restrict__ start,
                                                        int* __restrict__ rows, int* __restrict__ meta) {
+    sb_pdl_enter();
     __shared__ int s_cnt[1024], s_u[1024];
     int per = (V + 1023) / 1024, b = threadIdx.x * per, e = min(b + per, V);
     int c = 0, u = 0;
@@ -696,6 +712,7 @@ __global__ void __launch_bounds__(1024) eb_scan_kernel(const int* __restrict__ c
 __global__ void __launch_bounds__(EB_CHUNK) eb_place_kernel(const uint32_t* __restrict__ tok, int T, int V,
                                                             const int* __restrict__ chunk_cnt, const int* __restrict__ start,
                                                             int* __restrict__ sorted_pos) {
+    sb_pdl_enter();
     __shared__ uint32_t s_tok[EB_CHUNK];
     int t = blockIdx.x * EB_CHUNK + threadIdx.x;
     uint32_t id = t < T ? tok[t] : 0xffffffffu;
@@ -712,6 +729,7 @@ __global__ void __launch_bounds__(RB_THREADS) eb_segsum_kernel(const float* __re
                                                                const int* __restrict__ rows, const int* __restrict__ start,
                                                                const int* __restrict__ cnt, const int* __restrict__ sorted_pos,
                                                                const int* __restrict__ meta, int d, int vec) {
+    sb_pdl_enter();
     int U = meta[0];
     for (int u = blockIdx.x; u < U; u += gridDim.x) {
         int row = rows[u], s0 = start[row], n = cnt[row];
@@ -737,6 +755,7 @@ __global__ void __launch_bounds__(RB_THREADS) adamw_kernel(float* __restrict__ w
                                                            float* __restrict__ v, size_t n, float lr, float b1, float b2, float wd,
                                                            float eps, float c1, float c2, float grad_scale,
                                                            const float* __restrict__ sumsq, float clip, int vec) {
+    sb_pdl_enter();
     float gs = grad_scale;
     if (clip > 0.f && sumsq) {
         float norm = sqrtf(sumsq[0]) * grad_scale;
@@ -773,14 +792,14 @@ void sb_rmsnorm(sb_ctx_t* c, const float* x, const float* w, float* y, int rows,
         unsigned* am = sb_amax_take(c, y, (size_t)rows * cols);
         if (cols == 128 && rows >= 1024) {
             int g4 = (rows + 31) / 32; if (g4 > sm_count(c) * 4) g4 = sm_count(c) * 4;      // 8 warps x 4 rows per CTA and pass
-            rmsnorm_w128_kernel<<<g4, RB_THREADS, 0, st>>>(x, w, y, rows, eps, am);
+            sb_launch(rmsnorm_w128_kernel, dim3(g4), dim3(RB_THREADS), 0, st, x, w, y, rows, eps, am);
         } else
-        if (cols <= 512)       rmsnorm_warp_kernel<4><<<wgrid, RB_THREADS, 0, st>>>(x, w, y, rows, cols, eps, am);
-        else if (cols <= 1024) rmsnorm_warp_kernel<8><<<wgrid, RB_THREADS, 0, st>>>(x, w, y, rows, cols, eps, am);
-        else if (cols <= 2048) rmsnorm_warp_kernel<16><<<wgrid, RB_THREADS, 0, st>>>(x, w, y, rows, cols, eps, am);
-        else                   rmsnorm_warp_kernel<32><<<wgrid, RB_THREADS, 0, st>>>(x, w, y, rows, cols, eps, am);
+        if (cols <= 512)       sb_launch(rmsnorm_warp_kernel<4>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, rows, cols, eps, am);
+        else if (cols <= 1024) sb_launch(rmsnorm_warp_kernel<8>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, rows, cols, eps, am);
+        else if (cols <= 2048) sb_launch(rmsnorm_warp_kernel<16>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, rows, cols, eps, am);
+        else                   sb_launch(rmsnorm_warp_kernel<32>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, rows, cols, eps, am);
     } else
-    rmsnorm_kernel<<<grid, RB_THREADS, 0, (cudaStream_t)c->pub.stream>>>(x, w, y, rows, cols, eps, vec);
+    sb_launch(rmsnorm_kernel, dim3(grid), dim3(RB_THREADS), 0, (cudaStream_t)c->pub.stream, x, w, y, rows, cols, eps, vec);
     sb_tick_end(c, tk, 0.0, 8.0 * rows * cols);
     c->launches++;
 }
@@ -797,10 +816,10 @@ int sb_rmsnorm_parts(sb_ctx_t* c, const float* x, const float* w, float* y, int 
     cudaStream_t st = (cudaStream_t)c->pub.stream;
     uint2* h1 = (uint2*)h; uint2* h2 = (uint2*)((uint16_t*)h + n);
     int tk = sb_tick_begin(c, SB_CLS_NORM_FWD);
-    if (cols <= 512)       rmsnorm_warp_parts_kernel<4><<<wgrid, RB_THREADS, 0, st>>>(x, w, h1, h2, rows, cols, eps, bound);
-    else if (cols <= 1024) rmsnorm_warp_parts_kernel<8><<<wgrid, RB_THREADS, 0, st>>>(x, w, h1, h2, rows, cols, eps, bound);
-    else if (cols <= 2048) rmsnorm_warp_parts_kernel<16><<<wgrid, RB_THREADS, 0, st>>>(x, w, h1, h2, rows, cols, eps, bound);
-    else                   rmsnorm_warp_parts_kernel<32><<<wgrid, RB_THREADS, 0, st>>>(x, w, h1, h2, rows, cols, eps, bound);
+    if (cols <= 512)       sb_launch(rmsnorm_warp_parts_kernel<4>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c));
+    else if (cols <= 1024) sb_launch(rmsnorm_warp_parts_kernel<8>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c));
+    else if (cols <= 2048) sb_launch(rmsnorm_warp_parts_kernel<16>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c));
+    else                   sb_launch(rmsnorm_warp_parts_kernel<32>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c));
     sb_tick_end(c, tk, 0.0, 8.0 * rows * cols);
     c->launches++;
     return 1;
@@ -814,8 +833,8 @@ void sb_rmsnorm_backward_with_partials(sb_ctx_t* c, const float* x, const float*
     int vec = (cols % 4 == 0) && aligned16(x) && aligned16(w) && aligned16(dy) && aligned16(dx_out) && (!resid || aligned16(resid));
     cudaStream_t s = (cudaStream_t)c->pub.stream;
     int tk = sb_tick_begin(c, SB_CLS_NORM_BWD);
-    rmsnorm_bwd_kernel<<<grid, RB_THREADS, 0, s>>>(x, w, dy, resid, dx_out, partial, rows, cols, eps, vec);
-    colsum_partials_kernel<<<(cols + 31) / 32, 32 * CS_GROUPS, 0, s>>>(partial, dscale, grid, cols);
+    sb_launch(rmsnorm_bwd_kernel, dim3(grid), dim3(RB_THREADS), 0, s, x, w, dy, resid, dx_out, partial, rows, cols, eps, vec);
+    sb_launch(colsum_partials_kernel, dim3((cols + 31) / 32), dim3(32 * CS_GROUPS), 0, s, partial, dscale, grid, cols);
     sb_tick_end(c, tk, 0.0, (resid ? 16.0 : 12.0) * rows * cols);
     c->launches += 2;
 }
@@ -833,8 +852,8 @@ void sb_rmsnorm_backward(sb_ctx_t* c, const float* x, const float* w, const floa
         cudaStream_t st = (cudaStream_t)c->pub.stream;
         int tk = sb_tick_begin(c, SB_CLS_NORM_BWD);
         unsigned* am = sb_amax_take(c, dx_out, (size_t)rows * cols);
-        rmsnorm_bwd_w128_kernel<<<wgrid, RB_THREADS, 0, st>>>(x, w, dy, resid, dx_out, partial, rows, eps, am);
-        colsum_partials_kernel<<<(cols + 31) / 32, 32 * CS_GROUPS, 0, st>>>(partial, dscale, wgrid, cols);
+        sb_launch(rmsnorm_bwd_w128_kernel, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, eps, am);
+        sb_launch(colsum_partials_kernel, dim3((cols + 31) / 32), dim3(32 * CS_GROUPS), 0, st, partial, dscale, wgrid, cols);
         sb_tick_end(c, tk, 0.0, (resid ? 16.0 : 12.0) * rows * cols);
         c->launches += 2;
         return;
@@ -847,9 +866,9 @@ void sb_rmsnorm_backward(sb_ctx_t* c, const float* x, const float* w, const floa
         cudaStream_t st = (cudaStream_t)c->pub.stream;
         int tk = sb_tick_begin(c, SB_CLS_NORM_BWD);
         unsigned* am = sb_amax_take(c, dx_out, (size_t)rows * cols);
-        if (cols <= 1024) rmsnorm_bwd_rows_kernel<1><<<wgrid, RB_THREADS, 0, st>>>(x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
-        else              rmsnorm_bwd_rows_kernel<2><<<wgrid, RB_THREADS, 0, st>>>(x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
-        colsum_partials_kernel<<<(cols + 31) / 32, 32 * CS_GROUPS, 0, st>>>(partial, dscale, wgrid, cols);
+        if (cols <= 1024) sb_launch(rmsnorm_bwd_rows_kernel<1>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
+        else              sb_launch(rmsnorm_bwd_rows_kernel<2>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
+        sb_launch(colsum_partials_kernel, dim3((cols + 31) / 32), dim3(32 * CS_GROUPS), 0, st, partial, dscale, wgrid, cols);
         sb_tick_end(c, tk, 0.0, (resid ? 16.0 : 12.0) * rows * cols);
         c->launches += 2;
         return;
@@ -863,7 +882,7 @@ void sb_rmsnorm_backward(sb_ctx_t* c, const float* x, const float* w, const floa
 void sb_softmax(sb_ctx_t* c, const float* x, float* y, int rows, int cols) {
     if (rows <= 0 || cols <= 0) return;
     int grid = rows < sm_count(c) * 8 ? rows : sm_count(c) * 8;
-    softmax_kernel<<<grid, RB_THREADS, 0, (cudaStream_t)c->pub.stream>>>(x, y, rows, cols);
+    sb_launch(softmax_kernel, dim3(grid), dim3(RB_THREADS), 0, (cudaStream_t)c->pub.stream, x, y, rows, cols);
     c->launches++;
 }
 
@@ -878,13 +897,13 @@ void sb_qk_norm(sb_ctx_t* c, float* x, float* rms_out, int rows, int cols, float
     int tk = sb_tick_begin(c, SB_CLS_NORM_FWD);
     if ((cols % 4) == 0 && cols <= 4096 && aligned16(x) && rows >= 64) {
         const int g = qk_wgrid(c, rows);
-        if (cols <= 512)       qk_norm_warp_kernel<4><<<g, RB_THREADS, 0, st>>>(x, rms_out, rows, cols, eps);
-        else if (cols <= 1024) qk_norm_warp_kernel<8><<<g, RB_THREADS, 0, st>>>(x, rms_out, rows, cols, eps);
-        else if (cols <= 2048) qk_norm_warp_kernel<16><<<g, RB_THREADS, 0, st>>>(x, rms_out, rows, cols, eps);
-        else                   qk_norm_warp_kernel<32><<<g, RB_THREADS, 0, st>>>(x, rms_out, rows, cols, eps);
+        if (cols <= 512)       sb_launch(qk_norm_warp_kernel<4>, dim3(g), dim3(RB_THREADS), 0, st, x, rms_out, rows, cols, eps);
+        else if (cols <= 1024) sb_launch(qk_norm_warp_kernel<8>, dim3(g), dim3(RB_THREADS), 0, st, x, rms_out, rows, cols, eps);
+        else if (cols <= 2048) sb_launch(qk_norm_warp_kernel<16>, dim3(g), dim3(RB_THREADS), 0, st, x, rms_out, rows, cols, eps);
+        else                   sb_launch(qk_norm_warp_kernel<32>, dim3(g), dim3(RB_THREADS), 0, st, x, rms_out, rows, cols, eps);
     } else {
         int grid = rows < sm_count(c) * 8 ? rows : sm_count(c) * 8;
-        qk_norm_row_kernel<<<grid, RB_THREADS, 0, st>>>(x, rms_out, NULL, NULL, NULL, rows, cols, eps);
+        sb_launch(qk_norm_row_kernel, dim3(grid), dim3(RB_THREADS), 0, st, x, rms_out, nullptr, nullptr, nullptr, rows, cols, eps);
     }
     sb_tick_end(c, tk, 0.0, 8.0 * rows * cols);
     c->launches++;
@@ -895,13 +914,13 @@ void sb_qk_norm_backward(sb_ctx_t* c, const float* y, const float* rms, const fl
     int tk = sb_tick_begin(c, SB_CLS_NORM_BWD);
     if ((cols % 4) == 0 && cols <= 4096 && aligned16(y) && aligned16(dy) && aligned16(dx) && rows >= 64) {
         const int g = qk_wgrid(c, rows);
-        if (cols <= 512)       qk_norm_bwd_warp_kernel<4><<<g, RB_THREADS, 0, st>>>(y, rms, dy, dx, rows, cols, eps);
-        else if (cols <= 1024) qk_norm_bwd_warp_kernel<8><<<g, RB_THREADS, 0, st>>>(y, rms, dy, dx, rows, cols, eps);
-        else if (cols <= 2048) qk_norm_bwd_warp_kernel<16><<<g, RB_THREADS, 0, st>>>(y, rms, dy, dx, rows, cols, eps);
-        else                   qk_norm_bwd_warp_kernel<32><<<g, RB_THREADS, 0, st>>>(y, rms, dy, dx, rows, cols, eps);
+        if (cols <= 512)       sb_launch(qk_norm_bwd_warp_kernel<4>, dim3(g), dim3(RB_THREADS), 0, st, y, rms, dy, dx, rows, cols, eps);
+        else if (cols <= 1024) sb_launch(qk_norm_bwd_warp_kernel<8>, dim3(g), dim3(RB_THREADS), 0, st, y, rms, dy, dx, rows, cols, eps);
+        else if (cols <= 2048) sb_launch(qk_norm_bwd_warp_kernel<16>, dim3(g), dim3(RB_THREADS), 0, st, y, rms, dy, dx, rows, cols, eps);
+        else                   sb_launch(qk_norm_bwd_warp_kernel<32>, dim3(g), dim3(RB_THREADS), 0, st, y, rms, dy, dx, rows, cols, eps);
     } else {
         int grid = rows < sm_count(c) * 8 ? rows : sm_count(c) * 8;
-        qk_norm_row_kernel<<<grid, RB_THREADS, 0, st>>>((float*)y, NULL, rms, dy, dx, rows, cols, eps);
+        sb_launch(qk_norm_row_kernel, dim3(grid), dim3(RB_THREADS), 0, st, (float*)y, nullptr, rms, dy, dx, rows, cols, eps);
     }
     sb_tick_end(c, tk, 0.0, 12.0 * rows * cols);
     c->launches++;
@@ -912,9 +931,9 @@ void sb_cross_entropy(sb_ctx_t* c, const float* logits, const uint32_t* targets,
     if (T <= 0 || V <= 0) return;
     int vec = (V % 4 == 0) && aligned16(logits) && aligned16(grad);
     int tk = sb_tick_begin(c, SB_CLS_CE);
-    cross_entropy_kernel<<<T, CE_THREADS, 0, (cudaStream_t)c->pub.stream>>>(logits, targets, grad, loss_rows, pos_ids, seq_ids,
+    sb_launch(cross_entropy_kernel, dim3(T), dim3(CE_THREADS), 0, (cudaStream_t)c->pub.stream, logits, targets, grad, loss_rows, pos_ids, seq_ids,
                                                                           seq_starts, T, V, 1.0f / (float)num_valid, vec, c->d_status, sb_amax_take(c, grad, (size_t)T * V),
-                                                                          NULL, NULL, 0.f, NULL);
+                                                                          nullptr, nullptr, 0.f, nullptr, 0u);
     sb_tick_end(c, tk, 0.0, 12.0 * T * V);
     c->launches++;
 }
@@ -935,8 +954,8 @@ int sb_cross_entropy_parts(sb_ctx_t* c, const float* logits, const uint32_t* tar
     int sh = ce_shift(inv_valid); sh = sh < -100 ? -100 : (sh > 100 ? 100 : sh);      // the rule the products apply to *amax
     const float sc = ldexpf(1.0f, sh);
     int tk = sb_tick_begin(c, SB_CLS_CE);
-    cross_entropy_kernel<<<T, CE_THREADS, 0, (cudaStream_t)c->pub.stream>>>(logits, targets, grad, loss_rows, pos_ids, seq_ids, seq_starts, T, V,
-                                                                          inv_valid, 1, c->d_status, NULL, (__half*)h, (__half*)h + (size_t)T * V, sc, amax);
+    sb_launch(cross_entropy_kernel, dim3(T), dim3(CE_THREADS), 0, (cudaStream_t)c->pub.stream, logits, targets, grad, loss_rows, pos_ids, seq_ids, seq_starts, T, V,
+                                                                          inv_valid, 1, c->d_status, nullptr, (__half*)h, (__half*)h + (size_t)T * V, sc, amax, sb_parts_keep(c));
     sb_tick_end(c, tk, 0.0, 12.0 * T * V);
     c->launches++;
     return 1;
@@ -952,9 +971,9 @@ static void sum_impl(sb_ctx_t* c, const float* in, float* out, size_t n, bool sq
     if (!partial) return;
     int vec = aligned16(in);
     int tk = sb_tick_begin(c, SB_CLS_OTHER);
-    if (square) partial_sum_kernel<true><<<grid, RB_THREADS, 0, s>>>(in, n, partial, vec);
-    else        partial_sum_kernel<false><<<grid, RB_THREADS, 0, s>>>(in, n, partial, vec);
-    final_sum_kernel<<<1, RB_THREADS, 0, s>>>(partial, grid, out);
+    if (square) sb_launch(partial_sum_kernel<true>, dim3(grid), dim3(RB_THREADS), 0, s, in, n, partial, vec);
+    else        sb_launch(partial_sum_kernel<false>, dim3(grid), dim3(RB_THREADS), 0, s, in, n, partial, vec);
+    sb_launch(final_sum_kernel, dim3(1), dim3(RB_THREADS), 0, s, partial, grid, out);
     sb_tick_end(c, tk, 0.0, 4.0 * (double)n);
     c->launches += 2;
 }
@@ -978,13 +997,13 @@ void sb_embedding_backward(sb_ctx_t* c, const uint32_t* tok, const float* g, flo
     int tk = sb_tick_begin(c, SB_CLS_EMBED);
     cudaMemsetAsync(cnt, 0, (size_t)V * sizeof(int), s);
     cudaMemsetAsync(chunk_cnt, 0, (size_t)nchunk * V * sizeof(int), s);
-    eb_count_kernel<<<nchunk, EB_CHUNK, 0, s>>>(tok, T, V, chunk_cnt, cnt, c->d_status);
-    eb_scan_kernel<<<1, 1024, 0, s>>>(cnt, V, start, rows, meta);
-    eb_place_kernel<<<nchunk, EB_CHUNK, 0, s>>>(tok, T, V, chunk_cnt, start, sorted_pos);
+    sb_launch(eb_count_kernel, dim3(nchunk), dim3(EB_CHUNK), 0, s, tok, T, V, chunk_cnt, cnt, c->d_status);
+    sb_launch(eb_scan_kernel, dim3(1), dim3(1024), 0, s, cnt, V, start, rows, meta);
+    sb_launch(eb_place_kernel, dim3(nchunk), dim3(EB_CHUNK), 0, s, tok, T, V, chunk_cnt, start, sorted_pos);
     int grid = T < V ? T : V;
     if (grid > sm_count(c) * 8) grid = sm_count(c) * 8;
     int vec = (d % 4 == 0) && aligned16(g) && aligned16(dE);
-    eb_segsum_kernel<<<grid, RB_THREADS, 0, s>>>(g, dE, rows, start, cnt, sorted_pos, meta, d, vec);
+    sb_launch(eb_segsum_kernel, dim3(grid), dim3(RB_THREADS), 0, s, g, dE, rows, start, cnt, sorted_pos, meta, d, vec);
     sb_tick_end(c, tk, 0.0, 12.0 * T * d);      // upper bound: every token a distinct row
     c->launches += 4;
 }
@@ -1022,7 +1041,7 @@ void sb_adamw(sb_ctx_t* c, float* w, const float* g, float* m, float* v, size_t 
     size_t grid = (size_t)sm_count(c) * 8;
     if (grid > need) grid = need;
     int tk = sb_tick_begin(c, SB_CLS_ADAMW);
-    adamw_kernel<<<(int)grid, RB_THREADS, 0, (cudaStream_t)c->pub.stream>>>(w, g, m, v, n, lr, b1, b2, wd, eps, c1, c2,
+    sb_launch(adamw_kernel, dim3((int)grid), dim3(RB_THREADS), 0, (cudaStream_t)c->pub.stream, w, g, m, v, n, lr, b1, b2, wd, eps, c1, c2,
                                                                          grad_scale, d_sumsq, clip, vec);
     sb_tick_end(c, tk, 0.0, 28.0 * (double)n);
     c->launches++;
@@ -1096,6 +1115,7 @@ extern "C" int seraph_b200_rmsnorm_backward_static(const float* input, const flo
     cudaStream_t s = (cudaStream_t)stream;
     // every CTA overwrites its whole row of partials before the column sum reads it,
     // so nothing left over from an earlier call is ever read and no clearing is needed
+    // plain launches on the caller's stream, which may be under capture
     rmsnorm_bwd_kernel<<<grid, RB_THREADS, 0, s>>>(input, scale, grad_output, nullptr, grad_input, partial, rows, cols, eps, vec);
     colsum_partials_kernel<<<(cols + 31) / 32, 32 * CS_GROUPS, 0, s>>>(partial, grad_scale, grid, cols);
     cudaError_t e = cudaGetLastError();
