@@ -39,6 +39,7 @@ struct __align__(64) GgSeg {
     CUtensorMap a, b;            // parts: K-major {K, rows, part}, MN-major {rows, K, part}
     const float *amax_a, *amax_b;
     int K, kb;                   // kb: k blocks of 64
+    float alpha;                 // factor of this segment
     int mn;                      // bit 0: A is MN-major, bit 1: B is
 };
 struct __align__(64) GgProb {
@@ -303,7 +304,7 @@ gg_kernel(const __grid_constant__ GgParams p) {
                 // undo the operands' power-of-two scales; their product may leave the float range, then it takes two multiplications
                 const int e = -tc_f16_shift(sb_word(g.amax_a)) - tc_f16_shift(sb_word(g.amax_b));
                 const bool far = e < -120 || e > 120;
-                const float s1 = far ? tc_pow2(e / 2) : tc_pow2(e), s2 = far ? tc_pow2(e - e / 2) : 1.f;
+                const float s1 = (far ? tc_pow2(e / 2) : tc_pow2(e)) * g.alpha, s2 = far ? tc_pow2(e - e / 2) : 1.f;
                 for (int kb = lo; kb < hi && ok; kb++, gch++) {
                     const int buf = gch & 1;
                     ok = mbar_wait(&acc_full[buf], (gch >> 1) & 1);
@@ -545,7 +546,7 @@ static bool gg_launch_t(sb_ctx_t* c, const GgParams& p, int G) {
 
 // --------------------------------------------------------------------------- host side
 bool gg_shape_ok(int M, int N, int K, int tA, int tB) {
-    if (M < 8 || N < 16 || K < 8 || (N & 3) || (double)M * N * K < (double)(1 << 19)) return false;      // smaller: the CUDA-core kernel
+    if (M < 8 || N < 8 || K < 8 || (N & 3) || (double)M * N * K < (double)(1 << 19)) return false;      // smaller: the CUDA-core kernel
     if (tA && tB) tA = tB = 0;
     return (tA ? (M & 7) == 0 : (K & 7) == 0) && (tB ? (K & 7) == 0 : (N & 7) == 0);
 }
@@ -559,12 +560,12 @@ extern "C" int sb_gemm_group_takes(sb_ctx_t* c, int M, int N, int K, int tA, int
     return gg_mode(c, &nt) && gg_shape_ok(M, N, K, tA, tB) ? 1 : 0;
 }
 
-struct GgOperand { const float* x; size_t n; __half* h; float* amax; bool fresh; int slot; };
+struct GgOperand { const float* x; size_t n; __half* h; float* amax; bool fresh, kept; int slot; };      // kept: the parts outlive the step
 // the parts of an operand: those a producer or an earlier product of the step left, or a slot to make them in
 static int gg_operand(sb_ctx_t* c, GgOperand* ops, int* nops, const float* x, size_t n) {
     for (int i = 0; i < *nops; i++) if (ops[i].x == x && ops[i].n == n) return i;
     GgOperand* o = &ops[*nops];
-    o->x = x; o->n = n; o->slot = -1;
+    o->x = x; o->n = n; o->slot = -1; o->kept = false;
     void* h; int fresh;
     if (sb_parts_find(c, x, n, &h, &o->amax, &fresh)) { o->h = (__half*)h; o->fresh = fresh != 0; }
     else {
@@ -595,7 +596,7 @@ static void gg_prepare(sb_ctx_t* c, GgOperand* ops, int n) {
                 o->amax = left;
                 if (o->slot >= 0) c->f16_slot[o->slot].amax = left; else sb_parts_set_amax(c, o->x, left);
             } else {
-                float* word = sb_zero_word(c);                  // zero already; outside a step the operand's own word
+                float* word = o->kept ? NULL : sb_zero_word(c); // zero already; outside a step the operand's own word
                 if (word) { o->amax = word; if (o->slot >= 0) c->f16_slot[o->slot].amax = word; else sb_parts_set_amax(c, o->x, word); }
                 else cudaMemsetAsync(o->amax, 0, sizeof(float), st);
                 tc_multi_add(&am, o->x, o->n, nullptr, o->amax);
@@ -620,7 +621,7 @@ extern "C" void sb_parts_prepare(sb_ctx_t* c, const float* const* x, const size_
         for (; i0 < count && k < TC_MULTI; i0++) {
             void* h; int fresh;
             if (!sb_parts_find(c, x[i0], n[i0], &h, &ops[k].amax, &fresh)) return;      // no arena: every product prepares its own operands
-            ops[k].x = x[i0]; ops[k].n = n[i0]; ops[k].h = (__half*)h; ops[k].fresh = fresh != 0; ops[k].slot = -1;
+            ops[k].x = x[i0]; ops[k].n = n[i0]; ops[k].h = (__half*)h; ops[k].fresh = fresh != 0; ops[k].kept = c->weights_fixed != 0; ops[k].slot = -1;
             k++;
         }
         gg_prepare(c, ops, k);
@@ -667,7 +668,7 @@ static bool gg_run(sb_ctx_t* c, const sb_gemm_job_t* jobs, int njobs, int nt) {
             q->M = b->M; q->N = b->N; q->seg0 = j; q->nseg = 0; q->kb = 0; q->acc = b->acc;
         }
         GgProb* q = &p.prob[np - 1];
-        p.seg[j].K = b->K; p.seg[j].kb = (b->K + 63) / 64;
+        p.seg[j].K = b->K; p.seg[j].alpha = b->alpha == 0.f ? 1.f : b->alpha; p.seg[j].kb = (b->K + 63) / 64;
         q->nseg++; q->kb += p.seg[j].kb;
     }
     const int sms = c->pub.gpu_sm_count > 0 ? c->pub.gpu_sm_count : 148;

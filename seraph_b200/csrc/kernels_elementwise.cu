@@ -259,6 +259,20 @@ __global__ void __launch_bounds__(EW_THREADS) rope_kernel(const float* qin, floa
     sb_block_amax(amk, amax_k);
 }
 
+// Adapters between their compact form (A [r,in], B [out,r]) and the working copies of rank R (A [R,in], B [out,R]): blockIdx.y = adapter,
+// blockIdx.z = layer.  Only the live part moves; the padding of the working copies stays zero.
+struct LoraShapes { int n, r, R; int in[7], out[7]; size_t off[7], off_pad[7], per_layer, per_layer_pad; };
+__global__ void __launch_bounds__(EW_THREADS) lora_repad_kernel(float* __restrict__ compact, float* __restrict__ pad, int to_pad, const __grid_constant__ LoraShapes s) {
+    sb_pdl_enter();
+    const int a = blockIdx.y;
+    float* c = compact + (size_t)blockIdx.z * s.per_layer + s.off[a]; float* p = pad + (size_t)blockIdx.z * s.per_layer_pad + s.off_pad[a];
+    const size_t nA = (size_t)s.r * s.in[a], nB = (size_t)s.out[a] * s.r, pA = (size_t)s.R * s.in[a];
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nA + nB; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t j = i - nA, q = i < nA ? i : pA + (j / s.r) * s.R + j % s.r;
+        if (to_pad) p[q] = c[i]; else c[i] = p[q];
+    }
+}
+
 // pair-at-a-time variant for head_dim not divisible by 4 or unaligned buffers
 __global__ void rope_pair_kernel(const float* __restrict__ in, float* __restrict__ out, const uint32_t* __restrict__ pos_ids,
                                  const float2* __restrict__ tab, int T, int H, int hd, int backward) {
@@ -295,6 +309,27 @@ void sb_swiglu(sb_ctx_t* c, const float* g, const float* u, float* o, size_t n) 
 void sb_scale(sb_ctx_t* c, float* a, size_t n, float alpha) {
     if (!n) return;
     sb_launch(scale_kernel, dim3(ew_grid(c, n)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, a, n, alpha);
+    c->launches++;
+}
+
+void sb_lora_repad(sb_ctx_t* c, float* compact, float* pad, int to_pad, int l0, int layers) {
+    LoraShapes s;
+    s.n = 0; s.r = c->lora_rank; s.R = c->lora_R; s.per_layer = s.per_layer_pad = 0;
+    size_t most = 0;
+    for (int a = 0; a < 7; a++) {
+        if (!(c->lora_mask & (1 << a))) continue;
+        const int in = a == 3 ? c->qd : a == 6 ? c->F : c->d, out = a == 0 ? c->qd : (a == 1 || a == 2) ? c->kvd : (a == 4 || a == 5) ? c->F : c->d;
+        s.in[s.n] = in; s.out[s.n] = out; s.off[s.n] = s.per_layer; s.off_pad[s.n] = s.per_layer_pad; s.n++;
+        const size_t n = (size_t)s.r * ((size_t)in + out);
+        s.per_layer += n; s.per_layer_pad += (size_t)s.R * ((size_t)in + out);
+        if (n > most) most = n;
+    }
+    if (!s.n || layers <= 0) return;
+    int tk = sb_tick_begin(c, SB_CLS_COPY);
+    size_t g = (most + EW_THREADS * 4 - 1) / (EW_THREADS * 4);
+    sb_launch(lora_repad_kernel, dim3((unsigned)(g > 64 ? 64 : g), (unsigned)s.n, (unsigned)layers), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream,
+              compact + (size_t)l0 * s.per_layer, pad + (size_t)l0 * s.per_layer_pad, to_pad, s);
+    sb_tick_end(c, tk, 0.0, 8.0 * (double)s.per_layer * layers);
     c->launches++;
 }
 

@@ -834,7 +834,7 @@ void sb_rmsnorm_backward_with_partials(sb_ctx_t* c, const float* x, const float*
     cudaStream_t s = (cudaStream_t)c->pub.stream;
     int tk = sb_tick_begin(c, SB_CLS_NORM_BWD);
     sb_launch(rmsnorm_bwd_kernel, dim3(grid), dim3(RB_THREADS), 0, s, x, w, dy, resid, dx_out, partial, rows, cols, eps, vec);
-    sb_launch(colsum_partials_kernel, dim3((cols + 31) / 32), dim3(32 * CS_GROUPS), 0, s, partial, dscale, grid, cols);
+    if (dscale) sb_launch(colsum_partials_kernel, dim3((cols + 31) / 32), dim3(32 * CS_GROUPS), 0, s, partial, dscale, grid, cols);
     sb_tick_end(c, tk, 0.0, (resid ? 16.0 : 12.0) * rows * cols);
     c->launches += 2;
 }
@@ -853,7 +853,7 @@ void sb_rmsnorm_backward(sb_ctx_t* c, const float* x, const float* w, const floa
         int tk = sb_tick_begin(c, SB_CLS_NORM_BWD);
         unsigned* am = sb_amax_take(c, dx_out, (size_t)rows * cols);
         sb_launch(rmsnorm_bwd_w128_kernel, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, eps, am);
-        sb_launch(colsum_partials_kernel, dim3((cols + 31) / 32), dim3(32 * CS_GROUPS), 0, st, partial, dscale, wgrid, cols);
+        if (dscale) sb_launch(colsum_partials_kernel, dim3((cols + 31) / 32), dim3(32 * CS_GROUPS), 0, st, partial, dscale, wgrid, cols);
         sb_tick_end(c, tk, 0.0, (resid ? 16.0 : 12.0) * rows * cols);
         c->launches += 2;
         return;
@@ -868,7 +868,7 @@ void sb_rmsnorm_backward(sb_ctx_t* c, const float* x, const float* w, const floa
         unsigned* am = sb_amax_take(c, dx_out, (size_t)rows * cols);
         if (cols <= 1024) sb_launch(rmsnorm_bwd_rows_kernel<1>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
         else              sb_launch(rmsnorm_bwd_rows_kernel<2>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
-        sb_launch(colsum_partials_kernel, dim3((cols + 31) / 32), dim3(32 * CS_GROUPS), 0, st, partial, dscale, wgrid, cols);
+        if (dscale) sb_launch(colsum_partials_kernel, dim3((cols + 31) / 32), dim3(32 * CS_GROUPS), 0, st, partial, dscale, wgrid, cols);
         sb_tick_end(c, tk, 0.0, (resid ? 16.0 : 12.0) * rows * cols);
         c->launches += 2;
         return;

@@ -113,7 +113,7 @@ static int index_single(sb_ctx_t* c, int T, int len) {
     return 0;
 }
 
-#define CTX_OR_RETURN(ctx) sb_ctx_t* c = sb_priv(ctx); if (!c) { fprintf(stderr, "seraph_b200: invalid context\n"); return; }
+#define CTX_OR_RETURN(ctx) sb_ctx_t* c = sb_priv(ctx); if (!c) { fprintf(stderr, "seraph_b200: invalid context\n"); return; } c->weights_gen++;      /* its output may be a view of the weights */
 #define NEED(...) do { const void* ptrs_[] = {__VA_ARGS__}; for (size_t i_ = 0; i_ < sizeof(ptrs_) / sizeof(ptrs_[0]); i_++) \
         if (!ptrs_[i_]) { sb_set_status(c, SB_ERR_ARG); return; } } while (0)
 
@@ -133,7 +133,10 @@ void sb_gemm(sb_ctx_t* c, const float* A, const float* B, float* C, int M, int N
 void sb_gemm_group(sb_ctx_t* c, const sb_gemm_job_t* jobs, int n) {
     for (int j = 0; j < n; j++) sb_amax_forget(c, jobs[j].C);
     if (sb_gemm_group_try(c, jobs, n) == 0) return;
-    for (int j = 0; j < n; j++) sb_gemm(c, jobs[j].A, jobs[j].B, jobs[j].C, jobs[j].M, jobs[j].N, jobs[j].K, jobs[j].tA, jobs[j].tB, jobs[j].acc);
+    for (int j = 0; j < n; j++) {
+        if (jobs[j].alpha != 0.f && jobs[j].alpha != 1.f) { sb_set_status(c, SB_ERR_ARG); return; }      // only groups that sb_gemm_group_takes take a factor
+        sb_gemm(c, jobs[j].A, jobs[j].B, jobs[j].C, jobs[j].M, jobs[j].N, jobs[j].K, jobs[j].tA, jobs[j].tB, jobs[j].acc);
+    }
 }
 
 // reference: cuda_train_matmul, src/cuda_train_context.cu:2697

@@ -75,6 +75,7 @@ typedef struct sb_ctx {
        the operand preparation then skips its own pass over the tensor */
     struct { const float* ptr; size_t n; } *hint_tab; int hint_n, hint_cap; float* hint_pool;
     struct { const float* ptr; size_t n; } hint_pending[4]; int hint_npending;
+    int weights_fixed, in_evaluate; unsigned weights_gen;      /* the weights' parts outlive the call while weights_gen stands */
     unsigned parts_gen; int parts_open; int parts_cache;   /* parts_cache 0: off (switch, or the arena did not fit) */
     int eval_batch_tokens;           /* cuda_evaluate packs samples up to this many tokens per forward pass; 0: one sample per pass */
     int attn_flash;                  /* 128-wide heads: 0 a launch per product over a score scratch; otherwise the forward is one kernel and the backward
@@ -112,14 +113,17 @@ typedef struct sb_ctx {
     int lora_rank, lora_mask; float lora_alpha;
     size_t n_lora;
     float *LW, *LG, *LM, *LV;
-    /* The rank-r products are far too thin for the tensor-core kernel's tiles (and ran 40 times slower on the CUDA-core GEMM),
-       so the step works on copies of A and B whose rank is padded with zero rows / columns to lora_R, a multiple of 128 (the
-       narrow tile of the CTA-pair kernel):
+    /* The rank-r products are far too thin for the CTA-pair kernel of the TF32 modes (and ran 40 times slower on the CUDA-core GEMM),
+       so there the step works on copies of A and B whose rank is padded with zero rows / columns to lora_R, a multiple of 128 (the
+       narrow tile of that kernel).  The grouped kernel of the FP16-part modes takes any multiple of 8: lora_R is that, and where it is
+       the rank itself the working copies are the adapters themselves (LWp == LW, LGp == LG).
        LWp [per adapter: A (R, in) then B (out, R)] is refreshed from LW before a step when the adapters changed, the gradient
        products accumulate into LGp and the live part is copied to LG layer by layer.  Padding changes no value: the extra rows of
        A and columns of B are zero, so the extra columns of X A^T are zero and the extra gradient rows / columns are never read. */
     int lora_R; size_t n_lora_pad; float *LWp, *LGp; int lora_pad_stale;
     float* lora_tmp; size_t lora_tmp_cap;
+    float* lora_h; size_t lora_h_cap; int lora_h_T;      /* X A^T of every layer and adapter, kept for the backward pass [T, lora_R] */
+    int lora_grouped;                /* the step in flight runs its adapters' products in groups */
 
     /* activations */
     int T_cap;
@@ -186,6 +190,8 @@ void sb_rmsnorm_backward(sb_ctx_t*, const float* x, const float* w, const float*
 void sb_add(sb_ctx_t*, const float* a, const float* b, float* c, size_t n);
 void sb_mul(sb_ctx_t*, const float* a, const float* b, float* c, size_t n);
 void sb_scale(sb_ctx_t*, float* a, size_t n, float alpha);
+/* between compact adapters (rank r) and working copies (rank R), all layers: to_pad 1: pad <- compact, 0: compact <- pad */
+void sb_lora_repad(sb_ctx_t*, float* compact, float* pad, int to_pad, int l0, int layers);
 void sb_silu(sb_ctx_t*, const float* x, float* y, size_t n);
 void sb_softmax(sb_ctx_t*, const float* x, float* y, int rows, int cols);
 void sb_silu_backward(sb_ctx_t*, const float* x, const float* dy, float* dx, size_t n);
@@ -243,8 +249,8 @@ void sb_nan_check(sb_ctx_t*, const float* x, size_t n, uint32_t* flags, uint32_t
 /* C[M,N] (+)= op(A) op(B); same semantics as the reference's matmul_dispatch */
 void sb_gemm(sb_ctx_t*, const float* A, const float* B, float* C, int M, int N, int K, int tA, int tB, int acc);
 /* Several products that do not depend on one another, as if by sb_gemm in this order; a product with the destination of the one before it and
-   acc set is added to it.  On FP16 parts they run as one launch. */
-typedef struct { const float *A, *B; float* C; int M, N, K, tA, tB, acc; } sb_gemm_job_t;
+   acc set is added to it.  On FP16 parts they run as one launch.  Jobs with a factor only where sb_gemm_group_takes says so. */
+typedef struct { const float *A, *B; float* C; int M, N, K, tA, tB, acc; float alpha; } sb_gemm_job_t;      /* alpha: factor of the product, 0 means 1 */
 void sb_gemm_group(sb_ctx_t*, const sb_gemm_job_t* jobs, int n);
 int  sb_gemm_group_try(sb_ctx_t*, const sb_gemm_job_t* jobs, int n);      /* 0: launched as a group */
 int  sb_gemm_group_takes(sb_ctx_t*, int M, int N, int K, int tA, int tB);

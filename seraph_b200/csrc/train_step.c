@@ -307,6 +307,7 @@ static int ensure_model(sb_ctx_t* c, const train_state_t* st, int frozen_base) {
         sb_parts_register(c, 0, c->W + o->gate, (size_t)F * d); sb_parts_register(c, 0, c->W + o->up, (size_t)F * d);
         sb_parts_register(c, 0, c->W + o->down, (size_t)F * d);
     }
+    c->weights_gen++;
     if (st->full_weights) for_each_tensor(c, st->full_weights, up_tensor, NULL);
     else if (upload_base_from_model(c, (const seraph_model_t*)st->model)) { sb_set_status(c, SB_ERR_ARG); return 1; }
     publish_views(c);
@@ -326,6 +327,7 @@ static int ensure_extras(sb_ctx_t* c, int full) {
         }
         if (sb_check(c, cudaMalloc((void**)&c->XW, n * 4), "extra parameters")) { c->status = SB_ERR_OOM; return 1; }
         c->n_extras = n;
+        c->weights_gen++;
         cudaMemcpyAsync(c->XW, c->h_extras, n * 4, cudaMemcpyHostToDevice, S(c));
         if (c->untied) sb_parts_register(c, 0, c->XW + extras_lm_off(c), (size_t)c->V * c->d);
         if (sb_check(c, cudaStreamSynchronize(S(c)), "extra parameter upload")) return 1;
@@ -383,13 +385,15 @@ static cuda_lora_gpu_adapter_t* lora_pub(cuda_lora_gpu_state_t* s, int a) {
                  case 4: return &s->gate; case 5: return &s->up; default: return &s->down; }
 }
 static void free_lora(sb_ctx_t* c) {
+    if (c->LWp && c->LWp != c->LW) { cudaFree(c->LWp); cudaFree(c->LGp); }
     if (c->LW) cudaFree(c->LW);
     if (c->LG) cudaFree(c->LG);
     if (c->LM) cudaFree(c->LM);
     if (c->LV) cudaFree(c->LV);
     if (c->lora_tmp) cudaFree(c->lora_tmp);
-    if (c->LWp) cudaFree(c->LWp);
-    if (c->LGp) cudaFree(c->LGp);
+    sb_parts_unregister(c, 2); sb_parts_unregister(c, 3);
+    if (c->lora_h) cudaFree(c->lora_h);
+    c->lora_h = NULL; c->lora_h_cap = 0; c->lora_h_T = 0;
     c->LW = c->LG = c->LM = c->LV = c->lora_tmp = c->LWp = c->LGp = NULL; c->lora_tmp_cap = 0; c->n_lora_pad = 0; c->lora_R = 0;
     cuda_lora_gpu_state_t* s = (cuda_lora_gpu_state_t*)c->pub.lora_gpu;
     if (s) {
@@ -421,13 +425,7 @@ static int ensure_lora(sb_ctx_t* c, const lora_model_t* m) {
     cudaStreamSynchronize(S(c));
     free_lora(c);
     c->lora_rank = m->rank; c->lora_mask = mask; c->lora_alpha = m->alpha;
-    c->lora_R = (m->rank + 127) / 128 * 128;
     c->n_lora = lora_layer_params(c) * (size_t)c->L;
-    c->n_lora_pad = lora_layer_params_pad(c) * (size_t)c->L;
-    if (sb_check(c, cudaMalloc((void**)&c->LWp, c->n_lora_pad * sizeof(float)), "lora padded weights") ||
-        sb_check(c, cudaMalloc((void**)&c->LGp, c->n_lora_pad * sizeof(float)), "lora padded grads")) { c->status = SB_ERR_OOM; return 1; }
-    cudaMemsetAsync(c->LWp, 0, c->n_lora_pad * sizeof(float), S(c)); cudaMemsetAsync(c->LGp, 0, c->n_lora_pad * sizeof(float), S(c));
-    c->lora_pad_stale = 1;
     size_t bytes = c->n_lora * sizeof(float);
     if (sb_check(c, cudaMalloc((void**)&c->LW, bytes), "lora weights") || sb_check(c, cudaMalloc((void**)&c->LG, bytes), "lora grads") ||
         sb_check(c, cudaMalloc((void**)&c->LM, bytes), "lora m") || sb_check(c, cudaMalloc((void**)&c->LV, bytes), "lora v")) {
@@ -464,6 +462,77 @@ static int ensure_lora(sb_ctx_t* c, const lora_model_t* m) {
     }
     c->pub.lora_gpu = s;
     return sb_check(c, cudaStreamSynchronize(S(c)), "lora upload");
+}
+
+/* The working copies of the adapters for the context's present GEMM mode (see sb_ctx_t): made or remade when the rank they are padded to
+ * changes, registered as operands whose parts are made together. */
+static int ensure_lora_working(sb_ctx_t* c) {
+    const int mode = c->pub.use_bf16 ? SB_GEMM_BF16 : c->gemm_mode;
+    const int grouped = c->gemm_pair && (mode == SB_GEMM_FP16X3 || mode == SB_GEMM_BF16);
+    const int R = grouped ? (c->lora_rank + 7) / 8 * 8 : (c->lora_rank + 127) / 128 * 128;
+    if (c->LWp && c->lora_R == R) return 0;
+    cudaStreamSynchronize(S(c));
+    sb_parts_unregister(c, 2); sb_parts_unregister(c, 3);
+    if (c->LWp && c->LWp != c->LW) { cudaFree(c->LWp); cudaFree(c->LGp); }
+    c->LWp = c->LGp = NULL; c->lora_h_T = 0;
+    c->lora_R = R;
+    c->n_lora_pad = lora_layer_params_pad(c) * (size_t)c->L;
+    if (R == c->lora_rank) { c->LWp = c->LW; c->LGp = c->LG; c->lora_pad_stale = 0; }
+    else {
+        const size_t bytes = c->n_lora_pad * sizeof(float);
+        if (sb_check(c, cudaMalloc((void**)&c->LWp, bytes), "lora padded weights") || sb_check(c, cudaMalloc((void**)&c->LGp, bytes), "lora padded grads")) {
+            if (c->LWp) cudaFree(c->LWp);
+            c->LWp = c->LGp = NULL; c->status = SB_ERR_OOM;
+            return 1;
+        }
+        cudaMemsetAsync(c->LWp, 0, bytes, S(c)); cudaMemsetAsync(c->LGp, 0, bytes, S(c));
+        sb_lora_repad(c, c->LG, c->LGp, 1, 0, c->L);            /* an accumulation cycle may be under way */
+        c->lora_pad_stale = 1;
+    }
+    for (int l = 0; l < c->L; l++)
+        for (int a = 0; a < 7; a++) {
+            if (!(c->lora_mask & (1 << a))) continue;
+            int in, out; lora_dims(c, a, &in, &out);
+            const size_t o = lora_off_pad(c, l, a), nA = (size_t)R * in;
+            sb_parts_register(c, 2, c->LWp + o, nA); sb_parts_register(c, 2, c->LWp + o + nA, (size_t)out * R);
+        }
+    return 0;
+}
+static int lora_count_adapters(const sb_ctx_t* c) { int n = 0; for (int a = 0; a < 7; a++) n += (c->lora_mask >> a) & 1; return n; }
+static float* lora_h_of(const sb_ctx_t* c, int l, int a) {
+    int i = 0;
+    for (int b = 0; b < a; b++) i += (c->lora_mask >> b) & 1;
+    return c->lora_h + ((size_t)l * lora_count_adapters(c) + i) * (((size_t)c->lora_h_T * c->lora_R + 63) & ~(size_t)63);
+}
+/* May this step run its adapters' products in groups?  Then X A^T of every adapter is kept for the backward pass (lora_h, sized here for T
+ * tokens); otherwise the products run one after the other over lora_tmp. */
+static int ensure_lora_grouped(sb_ctx_t* c, int T) {
+    c->lora_grouped = 0;
+    const int R = c->lora_R;
+    for (int a = 0; a < 7; a++) {
+        if (!(c->lora_mask & (1 << a))) continue;
+        int in, out; lora_dims(c, a, &in, &out);
+        if (!sb_gemm_group_takes(c, T, R, in, 0, 1) || !sb_gemm_group_takes(c, T, out, R, 0, 1) || !sb_gemm_group_takes(c, T, out, in, 0, 1) ||
+            !sb_gemm_group_takes(c, T, in, out, 0, 0) || !sb_gemm_group_takes(c, out, R, T, 1, 0) || !sb_gemm_group_takes(c, T, R, out, 0, 0) ||
+            !sb_gemm_group_takes(c, R, in, T, 1, 0) || !sb_gemm_group_takes(c, T, in, R, 0, 0)) return 0;
+    }
+    const int n = lora_count_adapters(c);
+    const size_t one = ((size_t)T * R + 63) & ~(size_t)63, need = one * (size_t)n * (size_t)c->L;
+    if (c->lora_h_T != T) {
+        sb_parts_unregister(c, 3);
+        c->lora_h_T = 0;
+        if (c->lora_h_cap < need) {
+            cudaStreamSynchronize(S(c));
+            if (c->lora_h) cudaFree(c->lora_h);
+            c->lora_h = NULL; c->lora_h_cap = 0;
+            if (sb_check(c, cudaMalloc((void**)&c->lora_h, need * sizeof(float)), "lora activations")) { c->status = SB_ERR_OOM; return 1; }
+            c->lora_h_cap = need;
+        }
+        c->lora_h_T = T;
+        for (size_t i = 0; i < (size_t)n * (size_t)c->L; i++) sb_parts_register(c, 3, c->lora_h + i * one, (size_t)T * R);
+    }
+    c->lora_grouped = 1;
+    return 0;
 }
 
 /* ------------------------------------------------------------------------ */
@@ -538,41 +607,76 @@ static int ensure_pinned(sb_ctx_t* c, size_t bytes) {
 /* ------------------------------------------------------------------------ */
 /* the step                                                                  */
 /* ------------------------------------------------------------------------ */
-typedef struct { const float *A, *B; float *gA, *gB; int in, out; } lora_ref_t;
+typedef struct { const float *A, *B; float *gA, *gB, *h; int in, out; } lora_ref_t;
 /* the rank-padded working copies of adapter a of layer l */
 static int lora_get(sb_ctx_t* c, int l, int a, lora_ref_t* r) {
     if (!c->LW || !(c->lora_mask & (1 << a))) return 0;
     lora_dims(c, a, &r->in, &r->out);
     size_t o = lora_off_pad(c, l, a), nA = (size_t)c->lora_R * r->in;
     r->A = c->LWp + o; r->B = c->LWp + o + nA; r->gA = c->LGp + o; r->gB = c->LGp + o + nA;
+    r->h = c->lora_grouped ? lora_h_of(c, l, a) : NULL;
     return 1;
 }
-/* LWp <- LW (all layers) when the adapters changed: A's r rows are the head of the padded block, B's r columns a strided copy */
+/* LWp <- LW (all layers) when the adapters changed */
 static void lora_refresh_padded(sb_ctx_t* c) {
-    if (!c->lora_pad_stale || !c->LWp) return;
-    const int r = c->lora_rank, R = c->lora_R;
-    for (int l = 0; l < c->L; l++)
-        for (int a = 0; a < 7; a++) {
-            if (!(c->lora_mask & (1 << a))) continue;
-            int in, out; lora_dims(c, a, &in, &out);
-            const size_t o = lora_off(c, l, a), op = lora_off_pad(c, l, a);
-            cudaMemcpyAsync(c->LWp + op, c->LW + o, (size_t)r * in * 4, cudaMemcpyDeviceToDevice, S(c));
-            cudaMemcpy2DAsync(c->LWp + op + (size_t)R * in, (size_t)R * 4, c->LW + o + (size_t)r * in, (size_t)r * 4, (size_t)r * 4, (size_t)out,
-                              cudaMemcpyDeviceToDevice, S(c));
-        }
+    if (!c->lora_pad_stale || !c->LWp || c->LWp == c->LW) return;
+    sb_lora_repad(c, c->LW, c->LWp, 1, 0, c->L);
     c->lora_pad_stale = 0;
 }
-/* LG <- live part of LGp for layer l (the running total of this accumulation cycle) */
-static void lora_compact_grads(sb_ctx_t* c, int l) {
-    const int r = c->lora_rank, R = c->lora_R;
-    for (int a = 0; a < 7; a++) {
-        if (!(c->lora_mask & (1 << a))) continue;
-        int in, out; lora_dims(c, a, &in, &out);
-        const size_t o = lora_off(c, l, a), op = lora_off_pad(c, l, a);
-        cudaMemcpyAsync(c->LG + o, c->LGp + op, (size_t)r * in * 4, cudaMemcpyDeviceToDevice, S(c));
-        cudaMemcpy2DAsync(c->LG + o + (size_t)r * in, (size_t)r * 4, c->LGp + op + (size_t)R * in, (size_t)R * 4, (size_t)r * 4, (size_t)out,
-                          cudaMemcpyDeviceToDevice, S(c));
+/* LG <- live part of LGp (the running total of this accumulation cycle) */
+static void lora_compact_grads(sb_ctx_t* c, int l0, int layers) {
+    if (c->LGp != c->LG) sb_lora_repad(c, c->LG, c->LGp, 0, l0, layers);
+}
+
+/* Projections of one input, Y_i (+)= X W_i^T plus their adapters' s (X A_i^T) B_i^T, in two launches: X A^T of all adapters, then every
+ * projection with its adapter as a second segment of its k loop. */
+typedef struct { int a; const float* W; float* Y; int out, acc; } proj_t;
+static void lora_fwd_group(sb_ctx_t* c, int l, const float* X, const proj_t* p, int n, int T, int in) {
+    const float s = c->lora_alpha / (float)c->lora_rank;
+    sb_gemm_job_t jobs[8]; int k = 0;
+    lora_ref_t r;
+    for (int i = 0; i < n; i++)
+        if (lora_get(c, l, p[i].a, &r)) {
+            const sb_gemm_job_t j = {X, r.A, r.h, T, c->lora_R, in, 0, 1, 0, 1.f};
+            sb_amax_announce(c, r.h, (size_t)T * c->lora_R);
+            jobs[k++] = j;
+        }
+    if (k) sb_gemm_group(c, jobs, k);
+    k = 0;
+    for (int i = 0; i < n; i++) {
+        const sb_gemm_job_t j = {X, p[i].W, p[i].Y, T, p[i].out, in, 0, 1, p[i].acc, 1.f};
+        jobs[k++] = j;
+        if (lora_get(c, l, p[i].a, &r)) { const sb_gemm_job_t b = {r.h, r.B, p[i].Y, T, p[i].out, c->lora_R, 0, 1, 1, s}; jobs[k++] = b; }
     }
+    sb_gemm_group(c, jobs, k);
+}
+/* The backward of the same projections: with dX (may be NULL) = sum_i dY_i W_i in a first launch go gB_i += s dY_i^T (X A_i^T) and gh_i = dY_i B_i, in a
+ * second gA_i += s gh_i^T X and, in exact mode, dX += s gh_i A_i. */
+static void lora_bwd_group(sb_ctx_t* c, int l, const int* ads, const float* const* dY, const float* const* W, int n, const float* X, float* dX, int T, int in) {
+    const float s = c->lora_alpha / (float)c->lora_rank;
+    sb_gemm_job_t jobs[10]; int k = 0;
+    lora_ref_t r;
+    const size_t one = ((size_t)T * c->lora_R + 63) & ~(size_t)63;
+    for (int i = 0; i < n && dX; i++) {
+        int in_, out_; lora_dims(c, ads[i], &in_, &out_);
+        const sb_gemm_job_t j = {dY[i], W[i], dX, T, in, out_, 0, 0, i > 0, 1.f};
+        jobs[k++] = j;
+    }
+    for (int i = 0; i < n; i++)
+        if (lora_get(c, l, ads[i], &r)) {
+            float* gh = c->lora_tmp + (size_t)i * one;
+            const sb_gemm_job_t j = {dY[i], r.B, gh, T, c->lora_R, r.out, 0, 0, 0, 1.f}, b = {dY[i], r.h, r.gB, r.out, c->lora_R, T, 1, 0, 1, s};
+            sb_gemm_keep_forget(c, gh);
+            sb_amax_announce(c, gh, (size_t)T * c->lora_R);
+            jobs[k++] = j; jobs[k++] = b;
+        }
+    if (k) sb_gemm_group(c, jobs, k);
+    k = 0;
+    for (int i = 0; i < n; i++)
+        if (lora_get(c, l, ads[i], &r)) { const sb_gemm_job_t j = {c->lora_tmp + (size_t)i * one, X, r.gA, c->lora_R, r.in, T, 1, 0, 1, s}; jobs[k++] = j; }
+    for (int i = 0; i < n && dX && c->lora_exact; i++)
+        if (lora_get(c, l, ads[i], &r)) { const sb_gemm_job_t j = {c->lora_tmp + (size_t)i * one, r.A, dX, T, r.in, c->lora_R, 0, 0, 1, s}; jobs[k++] = j; }
+    if (k) sb_gemm_group(c, jobs, k);
 }
 
 /* Y[T,out] (+)= X[T,in] W[out,in]^T, plus the adapter's (s X A^T) B^T when one is active */
@@ -676,6 +780,13 @@ static void prepare_weights(sb_ctx_t* c, int T) {
             x[k] = w[i]; n[k] = m[i]; sum += m[i]; k++;
         }
     }
+    for (int l = 0; l < c->L && c->lora_grouped; l++)
+        for (int a = 0; a < 7; a++) {
+            lora_ref_t r;
+            if (!lora_get(c, l, a, &r)) continue;
+            if (k > 62) { sb_parts_prepare(c, x, n, k); k = 0; }
+            x[k] = r.A; n[k++] = (size_t)c->lora_R * r.in; x[k] = r.B; n[k++] = (size_t)r.out * c->lora_R;
+        }
     if (k) sb_parts_prepare(c, x, n, k);
 }
 
@@ -712,6 +823,9 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
             const sb_gemm_job_t jobs[3] = {{a->x_norm_attn, c->W + o->q, yq, T, qd, d, 0, 1, 0}, {a->x_norm_attn, c->W + o->k, yk, T, kvd, d, 0, 1, 0},
                                            {a->x_norm_attn, c->W + o->v, a->v, T, kvd, d, 0, 1, 0}};
             sb_gemm_group(c, jobs, 3);
+        } else if (c->lora_grouped) {
+            const proj_t p[3] = {{0, c->W + o->q, yq, qd, 0}, {1, c->W + o->k, yk, kvd, 0}, {2, c->W + o->v, a->v, kvd, 0}};
+            lora_fwd_group(c, l, a->x_norm_attn, p, 3, T, d);
         } else {
             linear_fwd(c, use_lora, l, 0, a->x_norm_attn, c->W + o->q, yq, T, d, qd, 0);
             linear_fwd(c, use_lora, l, 1, a->x_norm_attn, c->W + o->k, yk, T, d, kvd, 0);
@@ -733,7 +847,8 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
         sb_amax_announce(c, a->attn_out, (size_t)T * qd);
         sb_attention(c, a->q, a->k, a->v, a->attn_out, a->lse, c->seq_starts, c->seq_ids, T, c->Hq, c->Hkv, c->hd);
         sb_copy(c, a->post_attn_in, a->layer_in, Td * sizeof(float));
-        linear_fwd(c, use_lora, l, 3, a->attn_out, c->W + o->o, a->post_attn_in, T, qd, d, 1);
+        if (use_lora && c->lora_grouped) { const proj_t p = {3, c->W + o->o, a->post_attn_in, d, 1}; sb_gemm_keep_begin(c); lora_fwd_group(c, l, a->attn_out, &p, 1, T, qd); sb_gemm_keep_end(c); }
+        else linear_fwd(c, use_lora, l, 3, a->attn_out, c->W + o->o, a->post_attn_in, T, qd, d, 1);
         if (!(xf_parts && sb_rmsnorm_parts(c, a->post_attn_in, c->W + o->post_norm, a->x_norm_ffn, T, d, RMS_EPS))) {
             sb_amax_announce(c, a->x_norm_ffn, Td);
             sb_rmsnorm(c, a->post_attn_in, c->W + o->post_norm, a->x_norm_ffn, T, d, RMS_EPS);
@@ -744,6 +859,9 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
         if (!(use_lora && (c->lora_mask & 0x30))) {
             const sb_gemm_job_t jobs[2] = {{a->x_norm_ffn, c->W + o->gate, a->gate, T, F, d, 0, 1, 0}, {a->x_norm_ffn, c->W + o->up, a->up, T, F, d, 0, 1, 0}};
             sb_gemm_group(c, jobs, 2);
+        } else if (c->lora_grouped) {
+            const proj_t p[2] = {{4, c->W + o->gate, a->gate, F, 0}, {5, c->W + o->up, a->up, F, 0}};
+            lora_fwd_group(c, l, a->x_norm_ffn, p, 2, T, d);
         } else {
             linear_fwd(c, use_lora, l, 4, a->x_norm_ffn, c->W + o->gate, a->gate, T, d, F, 0);
             linear_fwd(c, use_lora, l, 5, a->x_norm_ffn, c->W + o->up, a->up, T, d, F, 0);
@@ -756,7 +874,8 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
             sb_swiglu(c, a->gate, a->up, a->ffn_hidden, (size_t)T * F);
         }
         sb_copy(c, next_in, a->post_attn_in, Td * sizeof(float));
-        linear_fwd(c, use_lora, l, 6, a->ffn_hidden, c->W + o->down, next_in, T, F, d, 1);
+        if (use_lora && c->lora_grouped) { const proj_t p = {6, c->W + o->down, next_in, d, 1}; sb_gemm_keep_begin(c); lora_fwd_group(c, l, a->ffn_hidden, &p, 1, T, F); sb_gemm_keep_end(c); }
+        else linear_fwd(c, use_lora, l, 6, a->ffn_hidden, c->W + o->down, next_in, T, F, d, 1);
         nan_mark(c, next_in, Td, nan_fwd_base(c) + (uint32_t)l);
     }
     if (!(hn_parts && sb_rmsnorm_parts(c, c->final_in, c->W + (size_t)c->V * d, c->hidden_norm, T, d, RMS_EPS))) {
@@ -776,8 +895,8 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
     const int d = c->d, F = c->F, qd = c->qd, kvd = c->kvd, L = c->L, V = c->V;
     float* gh = c->g_hidden; float* gx = c->g_xnorm;
     float* Gd = full ? c->G : NULL;
-    float* norm_sink = c->g_tmp;                 /* LoRA mode: norm-scale gradients are discarded */
-    if (!full) sb_memset(c, norm_sink, 0, (size_t)d * sizeof(float));
+    float* norm_sink = NULL;                     /* LoRA mode: norm-scale gradients are not formed */
+    const int grouped = !full && c->lora_grouped;
     sb_gemm_keep_begin(c);
     {
         const sb_gemm_job_t jobs[2] = {{c->dlogits, c->untied ? c->XW + extras_lm_off(c) : c->W, gx, T, d, V, 0, 0, 0},
@@ -797,34 +916,44 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
         /* FFN */
         sb_gemm_keep_begin(c);                       /* gh (and, with adapters, what they read) is split once for the whole group */
         sb_amax_announce(c, c->g_ffn, (size_t)T * F);
-        {
+        if (grouped) {
+            const int ad = 6; const float *dy = gh, *w = c->W + o->down;
+            lora_bwd_group(c, l, &ad, &dy, &w, 1, a->ffn_hidden, c->g_ffn, T, F);
+        } else {
             const sb_gemm_job_t jobs[2] = {{gh, c->W + o->down, c->g_ffn, T, F, d, 0, 0, 0}, {gh, a->ffn_hidden, Gd + o->down, d, F, T, 1, 0, 1}};
             sb_gemm_group(c, jobs, full ? 2 : 1);
         }
-        if (!full) lora_bwd(c, l, 6, gh, a->ffn_hidden, c->g_ffn, T);
+        if (!full && !grouped) lora_bwd(c, l, 6, gh, a->ffn_hidden, c->g_ffn, T);
         sb_gemm_keep_end(c);
         if (!(ffn_parts_bwd && sb_swiglu_backward_parts(c, a->gate, a->up, c->g_ffn, c->g_gate, c->g_up, (size_t)T * F))) {
             sb_amax_announce(c, c->g_gate, (size_t)T * F); sb_amax_announce(c, c->g_up, (size_t)T * F);
             sb_swiglu_backward(c, a->gate, a->up, c->g_ffn, c->g_gate, c->g_up, (size_t)T * F);
         }
         sb_gemm_keep_begin(c);
-        {
+        if (grouped) {
+            const int ads[2] = {4, 5}; const float *dy[2] = {c->g_gate, c->g_up}, *w[2] = {c->W + o->gate, c->W + o->up};
+            lora_bwd_group(c, l, ads, dy, w, 2, a->x_norm_ffn, gx, T, d);
+        } else {
             const sb_gemm_job_t jobs[4] = {{c->g_gate, c->W + o->gate, gx, T, d, F, 0, 0, 0}, {c->g_up, c->W + o->up, gx, T, d, F, 0, 0, 1},
                                            {c->g_gate, a->x_norm_ffn, Gd + o->gate, F, d, T, 1, 0, 1}, {c->g_up, a->x_norm_ffn, Gd + o->up, F, d, T, 1, 0, 1}};
             sb_gemm_group(c, jobs, full ? 4 : 2);
         }
-        if (!full) { lora_bwd(c, l, 4, c->g_gate, a->x_norm_ffn, gx, T); lora_bwd(c, l, 5, c->g_up, a->x_norm_ffn, gx, T); }
+        if (!full && !grouped) { lora_bwd(c, l, 4, c->g_gate, a->x_norm_ffn, gx, T); lora_bwd(c, l, 5, c->g_up, a->x_norm_ffn, gx, T); }
         sb_gemm_keep_end(c);
         sb_amax_announce(c, gh, (size_t)T * d);
         sb_rmsnorm_backward(c, a->post_attn_in, c->W + o->post_norm, gx, gh, gh, full ? Gd + o->post_norm : norm_sink, T, d, RMS_EPS);
         /* attention */
         sb_gemm_keep_begin(c);
-        {
+        if (grouped) {
+            const int ad = 3; const float *dy = gh, *w = c->W + o->o;
+            lora_bwd_group(c, l, &ad, &dy, &w, 1, a->attn_out, l > 0 || (c->lora_mask & 7) ? c->g_attn : NULL, T, qd);
+        } else {
             const sb_gemm_job_t jobs[2] = {{gh, c->W + o->o, c->g_attn, T, qd, d, 0, 0, 0}, {gh, a->attn_out, Gd + o->o, d, qd, T, 1, 0, 1}};
             sb_gemm_group(c, jobs, full ? 2 : 1);
         }
-        if (!full) lora_bwd(c, l, 3, gh, a->attn_out, c->g_attn, T);
+        if (!full && !grouped) lora_bwd(c, l, 3, gh, a->attn_out, c->g_attn, T);
         sb_gemm_keep_end(c);
+        if (grouped && !c->nan_on && l == 0 && !(c->lora_mask & 7)) break;      /* below the first layer's o projection nothing is trained */
         nan_mark(c, c->g_attn, (size_t)T * qd, nan_bwd_base(c) + 5u * (uint32_t)l);
         sb_attention_backward(c, a->q, a->k, a->v, a->attn_out, a->lse, c->g_attn, c->g_q, c->g_k, c->g_v, 0,
                               c->seq_starts, c->seq_ids, B, T, c->Hq, c->Hkv, c->hd);
@@ -848,23 +977,30 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
             gq = c->g_q2; gk = c->g_k2;
         }
         sb_gemm_keep_begin(c);
-        {
+        const int last = grouped && !c->nan_on && l == 0;      /* nothing below the first layer's projections is trained: their input gradient is not formed */
+        if (grouped) {
+            const int ads[3] = {0, 1, 2}; const float *dy[3] = {gq, gk, c->g_v}, *w[3] = {c->W + o->q, c->W + o->k, c->W + o->v};
+            lora_bwd_group(c, l, ads, dy, w, 3, a->x_norm_attn, last ? NULL : gx, T, d);
+        } else {
             const sb_gemm_job_t jobs[6] = {{gq, c->W + o->q, gx, T, d, qd, 0, 0, 0}, {gk, c->W + o->k, gx, T, d, kvd, 0, 0, 1}, {c->g_v, c->W + o->v, gx, T, d, kvd, 0, 0, 1},
                                            {gq, a->x_norm_attn, Gd + o->q, qd, d, T, 1, 0, 1}, {gk, a->x_norm_attn, Gd + o->k, kvd, d, T, 1, 0, 1},
                                            {c->g_v, a->x_norm_attn, Gd + o->v, kvd, d, T, 1, 0, 1}};
             sb_gemm_group(c, jobs, full ? 6 : 3);
         }
-        if (!full) { lora_bwd(c, l, 0, gq, a->x_norm_attn, gx, T); lora_bwd(c, l, 1, gk, a->x_norm_attn, gx, T); lora_bwd(c, l, 2, c->g_v, a->x_norm_attn, gx, T); }
+        if (!full && !grouped) { lora_bwd(c, l, 0, gq, a->x_norm_attn, gx, T); lora_bwd(c, l, 1, gk, a->x_norm_attn, gx, T); lora_bwd(c, l, 2, c->g_v, a->x_norm_attn, gx, T); }
         sb_gemm_keep_end(c);
-        sb_amax_announce(c, gh, (size_t)T * d);
-        sb_rmsnorm_backward(c, a->layer_in, c->W + o->in_norm, gx, gh, gh, full ? Gd + o->in_norm : norm_sink, T, d, RMS_EPS);
+        if (!last) {
+            sb_amax_announce(c, gh, (size_t)T * d);
+            sb_rmsnorm_backward(c, a->layer_in, c->W + o->in_norm, gx, gh, gh, full ? Gd + o->in_norm : norm_sink, T, d, RMS_EPS);
+        }
         nan_mark(c, gh, (size_t)T * d, nan_ghid_base(c) + (uint32_t)l);
-        if (!full && c->LW) lora_compact_grads(c, l);
+        if (!full && c->LW && reduce) lora_compact_grads(c, l, 1);
         if (reduce) {
             if (full) sb_dp_bucket_ready(c, Gd + o->q, o->post_norm + (size_t)d - o->q);
             else { size_t per = lora_layer_params(c); sb_dp_bucket_ready(c, c->LG + per * (size_t)l, per); }
         }
     }
+    if (!full && c->LW && !reduce) lora_compact_grads(c, 0, L);
     if (full) {
         nan_mark(c, gh, (size_t)T * d, 8);
         sb_embedding_backward(c, c->tokens, gh, Gd, T, d, V);
@@ -936,12 +1072,18 @@ static float step_body(train_state_t* st, int* tokens, int T, int* seq_starts, i
     if (use_lora && ensure_lora(c, st->lora)) return -1.0f;
     if (ensure_extras(c, full && train)) return -1.0f;
     if (ensure_activations(c, T, train)) return -1.0f;
-    if (use_lora && c->lora_tmp_cap < (size_t)T * c->lora_R) {
-        cudaStreamSynchronize(S(c));
-        if (c->lora_tmp) cudaFree(c->lora_tmp);
-        c->lora_tmp = NULL;
-        if (sb_check(c, cudaMalloc((void**)&c->lora_tmp, (size_t)T * c->lora_R * sizeof(float)), "lora tmp")) return -1.0f;
-        c->lora_tmp_cap = (size_t)T * c->lora_R;
+    c->weights_fixed = c->frozen_base || c->in_evaluate;
+    c->lora_grouped = 0;
+    if (use_lora) {
+        if (ensure_lora_working(c) || ensure_lora_grouped(c, T)) return -1.0f;
+        const size_t need = (((size_t)T * c->lora_R + 63) & ~(size_t)63) * 3;      /* up to three projections of one group */
+        if (c->lora_tmp_cap < need) {
+            cudaStreamSynchronize(S(c));
+            if (c->lora_tmp) cudaFree(c->lora_tmp);
+            c->lora_tmp = NULL; c->lora_tmp_cap = 0;
+            if (sb_check(c, cudaMalloc((void**)&c->lora_tmp, need * sizeof(float)), "lora tmp")) return -1.0f;
+            c->lora_tmp_cap = need;
+        }
     }
     if (use_lora) lora_refresh_padded(c);
     float theta = st->config->rope_theta > 0 ? st->config->rope_theta : 10000.0f;
@@ -959,7 +1101,7 @@ static float step_body(train_state_t* st, int* tokens, int T, int* seq_starts, i
     if (nan_begin(c, train && st->debug_nan_check)) return -1.0f;
     if (train && st->accumulation_counter == 0) {
         if (full) sb_memset(c, c->G, 0, c->n_params * sizeof(float));
-        else { sb_memset(c, c->LG, 0, c->n_lora * sizeof(float)); sb_memset(c, c->LGp, 0, c->n_lora_pad * sizeof(float)); }
+        else { sb_memset(c, c->LG, 0, c->n_lora * sizeof(float)); if (c->LGp != c->LG) sb_memset(c, c->LGp, 0, c->n_lora_pad * sizeof(float)); }
         if (full && c->XG) sb_memset(c, c->XG, 0, c->n_extras * sizeof(float));
     }
     forward_pass(c, T, max_seq, theta, use_lora);
@@ -1109,6 +1251,7 @@ float cuda_evaluate(train_state_t* state, int* val_tokens, int num_val_tokens, i
     }
     int full = state->lora == NULL;
     int B = 0;
+    if (c) { c->weights_gen++; c->in_evaluate = 1; }      /* nothing changes the weights between the passes of this call */
     if (budget > 0) ss[0] = 0;
     for (int s = 0; s < num_samples; s += stride) {
         int start = offsets[s], end = (s + 1 < num_samples) ? offsets[s + 1] : num_val_tokens;
@@ -1129,6 +1272,7 @@ float cuda_evaluate(train_state_t* state, int* val_tokens, int num_val_tokens, i
         eval_flush(state, ctx, pk, ss, B, full, rows, &total, &valid);
         free(pk); free(ss); free(rows);
     }
+    if (c) c->in_evaluate = 0;
     float avg = valid > 0 ? (float)(total / valid) : -1.0f;
     if (out_perplexity) *out_perplexity = avg > 0.0f ? expf(avg) : 0.0f;
     return avg;
@@ -1181,7 +1325,7 @@ void cuda_train_zero_lora_grads(cuda_train_context_t* ctx) {
     sb_ctx_t* c = sb_priv(ctx);
     if (!c || !c->LG) return;
     sb_memset(c, c->LG, 0, c->n_lora * sizeof(float));
-    if (c->LGp) sb_memset(c, c->LGp, 0, c->n_lora_pad * sizeof(float));
+    if (c->LGp && c->LGp != c->LG) sb_memset(c, c->LGp, 0, c->n_lora_pad * sizeof(float));
 }
 
 /* Extension: repeat the full-weight step on the batch the previous step call left on the device.
