@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_bwd_kernel(const float* __
 // ---------------------------------------------------------------------------
 template <int NV>
 __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                                  float* __restrict__ y, int rows, int cols, float eps, unsigned* amax_out) {
+                                                                  float* __restrict__ y, float* __restrict__ copy, int rows, int cols, float eps, unsigned* amax_out) {
     sb_pdl_enter();
     const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int c4 = cols >> 2;
@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_kernel(const float* _
         for (int i = 0; i < NV; i++) {
             int j = lane + 32 * i;
             v[i] = j < c4 ? xr[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (copy && j < c4) ((float4*)(copy + (size_t)r * cols))[j] = v[i];
             ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
         }
         ss = warp_sum(ss);
@@ -194,20 +195,19 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_w128_kernel(const float* _
     sb_block_amax(am, amax_out);
 }
 
-// RMSNorm backward for a 256-thread CTA that visits row groups of RNB_ROWS rows.  Thread t owns the float4 column
+// RMSNorm backward for a 256-thread CTA that visits groups of ROWS rows.  Thread t owns the float4 column
 // chunks t, t+256, ... (NC of them) of every row the CTA visits, so its dscale partial stays in NC float4
 // registers.  The loads of the next group (x, dy, residual) are issued before the current group is reduced,
 // so memory requests are in flight during the two CTA-wide reductions (sum x^2 and sum dy*w*x of each row);
 // two CTAs share an SM.  One dscale partial row per CTA, summed in CTA order by colsum_partials_kernel.
-#define RNB_ROWS 2
-template <int NC>
-struct RnbSet { float4 v[RNB_ROWS][NC], g[RNB_ROWS][NC], q[RNB_ROWS][NC]; };
+template <int NC, int ROWS>
+struct RnbSet { float4 v[ROWS][NC], g[ROWS][NC], q[ROWS][NC]; };
 
-template <int NC>
-__device__ __forceinline__ void rnb_load(RnbSet<NC>& s, const float* __restrict__ x, const float* __restrict__ dy, const float* resid,
+template <int NC, int ROWS>
+__device__ __forceinline__ void rnb_load(RnbSet<NC, ROWS>& s, const float* __restrict__ x, const float* __restrict__ dy, const float* resid,
                                          int r0, int rows, int c4) {
 #pragma unroll
-    for (int rr = 0; rr < RNB_ROWS; rr++)
+    for (int rr = 0; rr < ROWS; rr++)
 #pragma unroll
         for (int i = 0; i < NC; i++) {
             const int j = threadIdx.x + RB_THREADS * i;
@@ -219,28 +219,36 @@ __device__ __forceinline__ void rnb_load(RnbSet<NC>& s, const float* __restrict_
         }
 }
 
+// the row's scales: in registers, or with four chunks a thread read from cache again where they are used (registers are what limits it)
 template <int NC>
-__device__ __forceinline__ void rnb_compute(const RnbSet<NC>& s, const float4 (&sc)[NC], float4 (&acc)[NC], float* dx, int r0, int rows,
-                                            int cols, int c4, float eps, float (*s_red)[2 * RNB_ROWS], float* s_tot, float& am) {
+__device__ __forceinline__ float4 rnb_scale(const float4 (&scr)[NC], const float* __restrict__ w, int i, int c4) {
+    if constexpr (NC < 4) return scr[i];
+    const int j = threadIdx.x + RB_THREADS * i;
+    return j < c4 ? __ldg((const float4*)w + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+template <int NC, int ROWS>
+__device__ __forceinline__ void rnb_compute(const RnbSet<NC, ROWS>& s, const float4 (&scr)[NC], const float* __restrict__ w, float4 (&acc)[NC], float* dx, int r0, int rows,
+                                            int cols, int c4, float eps, float (*s_red)[2 * ROWS], float* s_tot, float& am) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    float part[2 * RNB_ROWS];
+    float part[2 * ROWS];
 #pragma unroll
-    for (int rr = 0; rr < RNB_ROWS; rr++) {
+    for (int rr = 0; rr < ROWS; rr++) {
         float ss = 0.f, cp = 0.f;
 #pragma unroll
         for (int i = 0; i < NC; i++) {
-            const float4 v = s.v[rr][i], g = s.g[rr][i];
+            const float4 v = s.v[rr][i], g = s.g[rr][i], sc = rnb_scale<NC>(scr, w, i, c4);
             ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            cp += g.x * sc[i].x * v.x + g.y * sc[i].y * v.y + g.z * sc[i].z * v.z + g.w * sc[i].w * v.w;
+            cp += g.x * sc.x * v.x + g.y * sc.y * v.y + g.z * sc.z * v.z + g.w * sc.w * v.w;
         }
         part[2 * rr] = warp_sum(ss); part[2 * rr + 1] = warp_sum(cp);
     }
     if (lane == 0) {
 #pragma unroll
-        for (int k = 0; k < 2 * RNB_ROWS; k++) s_red[wib][k] = part[k];
+        for (int k = 0; k < 2 * ROWS; k++) s_red[wib][k] = part[k];
     }
     __syncthreads();
-    if (threadIdx.x < 2 * RNB_ROWS) {
+    if (threadIdx.x < 2 * ROWS) {
         float t = 0.f;
 #pragma unroll
         for (int wv = 0; wv < RB_THREADS / 32; wv++) t += s_red[wv][threadIdx.x];
@@ -248,7 +256,7 @@ __device__ __forceinline__ void rnb_compute(const RnbSet<NC>& s, const float4 (&
     }
     __syncthreads();
 #pragma unroll
-    for (int rr = 0; rr < RNB_ROWS; rr++) {
+    for (int rr = 0; rr < ROWS; rr++) {
         if (r0 + rr >= rows) break;
         const float inv = 1.0f / sqrtf(s_tot[2 * rr] / cols + eps);
         const float k = inv * inv * inv / cols * s_tot[2 * rr + 1];
@@ -256,11 +264,11 @@ __device__ __forceinline__ void rnb_compute(const RnbSet<NC>& s, const float4 (&
         for (int i = 0; i < NC; i++) {
             const int j = threadIdx.x + RB_THREADS * i;
             if (j < c4) {
-                const float4 v = s.v[rr][i], g = s.g[rr][i], q = s.q[rr][i];
+                const float4 v = s.v[rr][i], g = s.g[rr][i], q = s.q[rr][i], sc = rnb_scale<NC>(scr, w, i, c4);
                 float4 o;
                 acc[i].x += g.x * v.x * inv; acc[i].y += g.y * v.y * inv; acc[i].z += g.z * v.z * inv; acc[i].w += g.w * v.w * inv;
-                o.x = g.x * sc[i].x * inv - v.x * k + q.x; o.y = g.y * sc[i].y * inv - v.y * k + q.y;
-                o.z = g.z * sc[i].z * inv - v.z * k + q.z; o.w = g.w * sc[i].w * inv - v.w * k + q.w;
+                o.x = g.x * sc.x * inv - v.x * k + q.x; o.y = g.y * sc.y * inv - v.y * k + q.y;
+                o.z = g.z * sc.z * inv - v.z * k + q.z; o.w = g.w * sc.w * inv - v.w * k + q.w;
                 ((float4*)dx)[(size_t)(r0 + rr) * c4 + j] = o;
                 am = sb_amax4(am, o);
             }
@@ -268,14 +276,14 @@ __device__ __forceinline__ void rnb_compute(const RnbSet<NC>& s, const float4 (&
     }
 }
 
-template <int NC>
+template <int NC, int ROWS>
 __global__ void __launch_bounds__(RB_THREADS, 2) rmsnorm_bwd_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                          const float* __restrict__ dy, const float* resid, float* dx,
                                                                          float* __restrict__ partial, int rows, int cols, float eps, unsigned* amax_dx) {
     sb_pdl_enter();
     float am = 0.f;
-    __shared__ float s_red[2][RB_THREADS / 32][2 * RNB_ROWS];
-    __shared__ float s_tot[2][2 * RNB_ROWS];
+    __shared__ float s_red[2][RB_THREADS / 32][2 * ROWS];
+    __shared__ float s_tot[2][2 * ROWS];
     const int c4 = cols >> 2;
     float4 acc[NC], sc[NC];
 #pragma unroll
@@ -284,17 +292,17 @@ __global__ void __launch_bounds__(RB_THREADS, 2) rmsnorm_bwd_rows_kernel(const f
         const int j = threadIdx.x + RB_THREADS * i;
         sc[i] = j < c4 ? ((const float4*)w)[j] : acc[i];
     }
-    const int ngroups = (rows + RNB_ROWS - 1) / RNB_ROWS, stride = gridDim.x;
-    RnbSet<NC> a, b;
+    const int ngroups = (rows + ROWS - 1) / ROWS, stride = gridDim.x;
+    RnbSet<NC, ROWS> a, b;
     int gidx = blockIdx.x;
-    if (gidx < ngroups) rnb_load<NC>(a, x, dy, resid, gidx * RNB_ROWS, rows, c4);
+    if (gidx < ngroups) rnb_load<NC, ROWS>(a, x, dy, resid, gidx * ROWS, rows, c4);
     while (gidx < ngroups) {
-        if (gidx + stride < ngroups) rnb_load<NC>(b, x, dy, resid, (gidx + stride) * RNB_ROWS, rows, c4);
-        rnb_compute<NC>(a, sc, acc, dx, gidx * RNB_ROWS, rows, cols, c4, eps, s_red[0], s_tot[0], am);
+        if (gidx + stride < ngroups) rnb_load<NC, ROWS>(b, x, dy, resid, (gidx + stride) * ROWS, rows, c4);
+        rnb_compute<NC, ROWS>(a, sc, w, acc, dx, gidx * ROWS, rows, cols, c4, eps, s_red[0], s_tot[0], am);
         gidx += stride;
         if (gidx >= ngroups) break;
-        if (gidx + stride < ngroups) rnb_load<NC>(a, x, dy, resid, (gidx + stride) * RNB_ROWS, rows, c4);
-        rnb_compute<NC>(b, sc, acc, dx, gidx * RNB_ROWS, rows, cols, c4, eps, s_red[1], s_tot[1], am);
+        if (gidx + stride < ngroups) rnb_load<NC, ROWS>(a, x, dy, resid, (gidx + stride) * ROWS, rows, c4);
+        rnb_compute<NC, ROWS>(b, sc, w, acc, dx, gidx * ROWS, rows, cols, c4, eps, s_red[1], s_tot[1], am);
         gidx += stride;
     }
 #pragma unroll
@@ -359,8 +367,14 @@ __global__ void __launch_bounds__(RB_THREADS, 4) rmsnorm_bwd_w128_kernel(const f
 // sums then added in group order.
 #define CS_GROUPS 32
 #define CS_BATCH 10
-__global__ void __launch_bounds__(32 * CS_GROUPS) colsum_partials_kernel(const float* __restrict__ partial, float* __restrict__ dscale, int nblocks, int cols) {
+#define CS_TAB 64
+struct CsEntry { const float* partial; float* dscale; int nblocks, cols; };
+struct CsTab { int store; CsEntry e[CS_TAB]; };      // blockIdx.y = entry; store: dscale is written, not added to
+__global__ void __launch_bounds__(32 * CS_GROUPS) colsum_partials_kernel(const __grid_constant__ CsTab tab) {
     sb_pdl_enter();
+    const float* __restrict__ partial = tab.e[blockIdx.y].partial; float* __restrict__ dscale = tab.e[blockIdx.y].dscale;
+    const int nblocks = tab.e[blockIdx.y].nblocks, cols = tab.e[blockIdx.y].cols;
+    if ((int)blockIdx.x * 32 >= cols) return;
     __shared__ float s_part[CS_GROUPS][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int cidx = blockIdx.x * 32 + tx;
@@ -383,7 +397,7 @@ __global__ void __launch_bounds__(32 * CS_GROUPS) colsum_partials_kernel(const f
         float t = s_part[0][tx];
 #pragma unroll
         for (int g = 1; g < CS_GROUPS; g++) t += s_part[g][tx];
-        dscale[cidx] += t;
+        dscale[cidx] = tab.store ? t : dscale[cidx] + t;
     }
 }
 
@@ -423,7 +437,7 @@ __global__ void __launch_bounds__(RB_THREADS) softmax_kernel(const float* __rest
 template <int NV>
 __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                         uint2* __restrict__ h1, uint2* __restrict__ h2, int rows, int cols, float eps,
-                                                                        float* __restrict__ bound_out, unsigned keep) {
+                                                                        float* __restrict__ bound_out, unsigned keep, float* __restrict__ copy) {
     sb_pdl_enter();
     const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int c4 = cols >> 2;
@@ -446,6 +460,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const fl
         for (int i = 0; i < NV; i++) {
             int j = lane + 32 * i;
             v[i] = j < c4 ? xr[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (copy && j < c4) ((float4*)(copy + (size_t)r * cols))[j] = v[i];
             ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
         }
         ss = warp_sum(ss);
@@ -778,13 +793,15 @@ __global__ void __launch_bounds__(RB_THREADS) adamw_kernel(float* __restrict__ w
 
 extern "C" {
 
-void sb_rmsnorm(sb_ctx_t* c, const float* x, const float* w, float* y, int rows, int cols, float eps) {
+// `copy` (may be NULL) receives the rows x as well: the residual stream that the layer's next product adds into, written while x is in registers
+void sb_rmsnorm_copy(sb_ctx_t* c, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps) {
     if (rows <= 0 || cols <= 0) return;
     sb_parts_invalidate(c, y);
     int grid = rows < sm_count(c) * 8 ? rows : sm_count(c) * 8;
     int vec = (cols % 4 == 0) && aligned16(x) && aligned16(w) && aligned16(y);
+    if (copy && !(vec && aligned16(copy) && cols <= 4096 && !(cols == 128 && rows >= 1024))) { sb_copy(c, copy, x, (size_t)rows * cols * sizeof(float)); copy = NULL; }
     int tk = sb_tick_begin(c, SB_CLS_NORM_FWD);
-    if (vec && cols <= 4096 && rows >= 64) {
+    if (vec && cols <= 4096) {
         // warp per row, 8 warps per CTA, two CTAs resident per SM: every warp gets the same number of rows (no tail)
         int wgrid = (rows + 7) / 8;
         { int cap = sm_count(c) * 2, k = (wgrid + cap - 1) / cap; wgrid = (wgrid + k - 1) / k; }
@@ -794,19 +811,20 @@ void sb_rmsnorm(sb_ctx_t* c, const float* x, const float* w, float* y, int rows,
             int g4 = (rows + 31) / 32; if (g4 > sm_count(c) * 4) g4 = sm_count(c) * 4;      // 8 warps x 4 rows per CTA and pass
             sb_launch(rmsnorm_w128_kernel, dim3(g4), dim3(RB_THREADS), 0, st, x, w, y, rows, eps, am);
         } else
-        if (cols <= 512)       sb_launch(rmsnorm_warp_kernel<4>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, rows, cols, eps, am);
-        else if (cols <= 1024) sb_launch(rmsnorm_warp_kernel<8>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, rows, cols, eps, am);
-        else if (cols <= 2048) sb_launch(rmsnorm_warp_kernel<16>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, rows, cols, eps, am);
-        else                   sb_launch(rmsnorm_warp_kernel<32>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, rows, cols, eps, am);
+        if (cols <= 512)       sb_launch(rmsnorm_warp_kernel<4>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am);
+        else if (cols <= 1024) sb_launch(rmsnorm_warp_kernel<8>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am);
+        else if (cols <= 2048) sb_launch(rmsnorm_warp_kernel<16>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am);
+        else                   sb_launch(rmsnorm_warp_kernel<32>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am);
     } else
     sb_launch(rmsnorm_kernel, dim3(grid), dim3(RB_THREADS), 0, (cudaStream_t)c->pub.stream, x, w, y, rows, cols, eps, vec);
-    sb_tick_end(c, tk, 0.0, 8.0 * rows * cols);
+    sb_tick_end(c, tk, 0.0, (copy ? 12.0 : 8.0) * rows * cols);
     c->launches++;
 }
+void sb_rmsnorm(sb_ctx_t* c, const float* x, const float* w, float* y, int rows, int cols, float eps) { sb_rmsnorm_copy(c, x, w, y, NULL, rows, cols, eps); }
 
 // y only as the FP16 parts of the registered tensor `y`; 1 = done, 0 = not possible here (call sb_rmsnorm)
-int sb_rmsnorm_parts(sb_ctx_t* c, const float* x, const float* w, float* y, int rows, int cols, float eps) {
-    if (rows < 64 || cols <= 0 || (cols & 7) || cols > 4096 || !aligned16(x) || !aligned16(w)) return 0;
+int sb_rmsnorm_parts(sb_ctx_t* c, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps) {
+    if (rows < 1 || cols <= 0 || (cols & 7) || cols > 4096 || !aligned16(x) || !aligned16(w) || (copy && !aligned16(copy))) return 0;
     void* h; float* bound; int fresh;
     const size_t n = (size_t)rows * cols;
     if (!sb_parts_find(c, y, n, &h, &bound, &fresh)) return 0;
@@ -816,16 +834,79 @@ int sb_rmsnorm_parts(sb_ctx_t* c, const float* x, const float* w, float* y, int 
     cudaStream_t st = (cudaStream_t)c->pub.stream;
     uint2* h1 = (uint2*)h; uint2* h2 = (uint2*)((uint16_t*)h + n);
     int tk = sb_tick_begin(c, SB_CLS_NORM_FWD);
-    if (cols <= 512)       sb_launch(rmsnorm_warp_parts_kernel<4>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c));
-    else if (cols <= 1024) sb_launch(rmsnorm_warp_parts_kernel<8>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c));
-    else if (cols <= 2048) sb_launch(rmsnorm_warp_parts_kernel<16>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c));
-    else                   sb_launch(rmsnorm_warp_parts_kernel<32>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c));
-    sb_tick_end(c, tk, 0.0, 8.0 * rows * cols);
+    if (cols <= 512)       sb_launch(rmsnorm_warp_parts_kernel<4>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy);
+    else if (cols <= 1024) sb_launch(rmsnorm_warp_parts_kernel<8>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy);
+    else if (cols <= 2048) sb_launch(rmsnorm_warp_parts_kernel<16>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy);
+    else                   sb_launch(rmsnorm_warp_parts_kernel<32>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy);
+    sb_tick_end(c, tk, 0.0, (copy ? 12.0 : 8.0) * rows * cols);
     c->launches++;
     return 1;
 }
 
 // number of CTAs the rmsnorm backward uses for `rows` rows (also the row count of its partial buffer)
+// The sums of dscale partials: at once, or (between sb_colsum_defer and sb_colsum_flush) noted and formed together, up to CS_TAB norms in one
+// launch.  A sum is 3 us of work in a launch of its own; a training step of an eight-layer model has 17 of them.
+struct CsPending { CsTab tab; int n, maxcols; float* arena; size_t cap, used; };
+#define CS_ARENA ((size_t)8 << 20)      // floats (32 MB): 13 norms of 2048 columns; filling up only means a launch
+static void cs_launch(sb_ctx_t* c, const CsTab& t, int n, int maxcols) {
+    sb_launch(colsum_partials_kernel, dim3((maxcols + 31) / 32, n), dim3(32 * CS_GROUPS), 0, (cudaStream_t)c->pub.stream, t);
+    c->launches++;
+}
+extern "C" void sb_colsum_flush(sb_ctx_t* c) {
+    CsPending* p = (CsPending*)c->cs_pending;
+    if (!p) return;
+    if (p->n) {
+        int tk = sb_tick_begin(c, SB_CLS_NORM_BWD);
+        cs_launch(c, p->tab, p->n, p->maxcols);
+        sb_tick_end(c, tk, 0.0, 0.0);
+    }
+    p->n = 0; p->maxcols = 0; p->used = 0;
+}
+extern "C" void sb_colsum_defer(sb_ctx_t* c, int on, int store, size_t floats) {
+    sb_colsum_flush(c);
+    c->cs_defer = 0; c->cs_store = store;
+    if (!on) return;
+    CsPending* p = (CsPending*)c->cs_pending;
+    if (!p) { p = (CsPending*)calloc(1, sizeof *p); c->cs_pending = p; }
+    if (!p) return;
+    if (floats > CS_ARENA) floats = CS_ARENA;
+    if (p->cap < floats) {
+        cudaStreamSynchronize((cudaStream_t)c->pub.stream);
+        if (p->arena) cudaFree(p->arena);
+        p->arena = NULL; p->cap = 0;
+        if (cudaMalloc((void**)&p->arena, floats * sizeof(float)) != cudaSuccess) { cudaGetLastError(); return; }      // no room: one launch per sum
+        p->cap = floats;
+    }
+    c->cs_defer = 1;
+}
+extern "C" void sb_colsum_free(sb_ctx_t* c) {
+    CsPending* p = (CsPending*)c->cs_pending;
+    if (p) { if (p->arena) cudaFree(p->arena); free(p); }
+    c->cs_pending = NULL; c->cs_defer = 0;
+}
+// room for the partials of one norm
+static float* rn_partials(sb_ctx_t* c, size_t floats) {
+    CsPending* p = (CsPending*)c->cs_pending;
+    if (c->cs_defer && floats <= p->cap) {
+        if (p->n == CS_TAB || p->used + floats > p->cap) sb_colsum_flush(c);
+        float* r = p->arena + p->used;
+        p->used += (floats + 31) & ~(size_t)31;
+        return r;
+    }
+    return (float*)sb_scratch(c, floats * sizeof(float));
+}
+static void rn_dscale(sb_ctx_t* c, const float* partial, float* dscale, int nblocks, int cols) {
+    CsPending* p = (CsPending*)c->cs_pending;
+    const CsEntry e = {partial, dscale, nblocks, cols};
+    if (c->cs_defer && partial >= p->arena && partial < p->arena + p->cap) {
+        p->tab.store = c->cs_store; p->tab.e[p->n++] = e;
+        if (cols > p->maxcols) p->maxcols = cols;
+        return;
+    }
+    CsTab t; t.store = c->cs_store; t.e[0] = e;
+    cs_launch(c, t, 1, cols);
+}
+
 static int rn_bwd_grid(sb_ctx_t* c, int rows) { int cap = sm_count(c) * 2; return rows < cap ? rows : cap; }
 
 void sb_rmsnorm_backward_with_partials(sb_ctx_t* c, const float* x, const float* w, const float* dy, const float* resid,
@@ -834,9 +915,9 @@ void sb_rmsnorm_backward_with_partials(sb_ctx_t* c, const float* x, const float*
     cudaStream_t s = (cudaStream_t)c->pub.stream;
     int tk = sb_tick_begin(c, SB_CLS_NORM_BWD);
     sb_launch(rmsnorm_bwd_kernel, dim3(grid), dim3(RB_THREADS), 0, s, x, w, dy, resid, dx_out, partial, rows, cols, eps, vec);
-    if (dscale) sb_launch(colsum_partials_kernel, dim3((cols + 31) / 32), dim3(32 * CS_GROUPS), 0, s, partial, dscale, grid, cols);
+    c->launches++;
+    if (dscale) rn_dscale(c, partial, dscale, grid, cols);
     sb_tick_end(c, tk, 0.0, (resid ? 16.0 : 12.0) * rows * cols);
-    c->launches += 2;
 }
 
 void sb_rmsnorm_backward(sb_ctx_t* c, const float* x, const float* w, const float* dy, const float* resid,
@@ -847,34 +928,37 @@ void sb_rmsnorm_backward(sb_ctx_t* c, const float* x, const float* w, const floa
     if (vec && cols == 128 && rows >= 1024) {
         // many short rows (the per-head norm): a warp per row
         int wgrid = (rows + 31) / 32; if (wgrid > 4 * sm_count(c)) wgrid = 4 * sm_count(c);
-        float* partial = (float*)sb_scratch(c, (size_t)wgrid * cols * sizeof(float));
+        float* partial = rn_partials(c, (size_t)wgrid * cols);
         if (!partial) return;
         cudaStream_t st = (cudaStream_t)c->pub.stream;
         int tk = sb_tick_begin(c, SB_CLS_NORM_BWD);
         unsigned* am = sb_amax_take(c, dx_out, (size_t)rows * cols);
         sb_launch(rmsnorm_bwd_w128_kernel, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, eps, am);
-        if (dscale) sb_launch(colsum_partials_kernel, dim3((cols + 31) / 32), dim3(32 * CS_GROUPS), 0, st, partial, dscale, wgrid, cols);
+        c->launches++;
+        if (dscale) rn_dscale(c, partial, dscale, wgrid, cols);
         sb_tick_end(c, tk, 0.0, (resid ? 16.0 : 12.0) * rows * cols);
-        c->launches += 2;
         return;
     }
-    if (vec && cols <= 2048 && rows >= 64) {
-        // row groups with the next group's loads in flight, two CTAs per SM; one dscale partial per CTA, summed in CTA order
-        int wgrid = (rows + RNB_ROWS - 1) / RNB_ROWS; if (wgrid > 2 * sm_count(c)) wgrid = 2 * sm_count(c);
-        float* partial = (float*)sb_scratch(c, (size_t)wgrid * cols * sizeof(float));
+    if (vec && cols <= 4096) {
+        // row groups with the next group's loads in flight, two CTAs per SM; one dscale partial per CTA, summed in CTA order.  Groups of two
+        // rows, of one above 2048 columns (a thread then holds four chunks of a row, and two rows would not fit its registers).
+        const int per = cols <= 2048 ? 2 : 1;
+        int wgrid = (rows + per - 1) / per; if (wgrid > 2 * sm_count(c)) wgrid = 2 * sm_count(c);
+        float* partial = rn_partials(c, (size_t)wgrid * cols);
         if (!partial) return;
         cudaStream_t st = (cudaStream_t)c->pub.stream;
         int tk = sb_tick_begin(c, SB_CLS_NORM_BWD);
         unsigned* am = sb_amax_take(c, dx_out, (size_t)rows * cols);
-        if (cols <= 1024) sb_launch(rmsnorm_bwd_rows_kernel<1>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
-        else              sb_launch(rmsnorm_bwd_rows_kernel<2>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
-        if (dscale) sb_launch(colsum_partials_kernel, dim3((cols + 31) / 32), dim3(32 * CS_GROUPS), 0, st, partial, dscale, wgrid, cols);
+        if (cols <= 1024)      sb_launch(rmsnorm_bwd_rows_kernel<1, 2>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
+        else if (cols > 2048)  sb_launch(rmsnorm_bwd_rows_kernel<4, 1>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
+        else                   sb_launch(rmsnorm_bwd_rows_kernel<2, 2>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
+        c->launches++;
+        if (dscale) rn_dscale(c, partial, dscale, wgrid, cols);
         sb_tick_end(c, tk, 0.0, (resid ? 16.0 : 12.0) * rows * cols);
-        c->launches += 2;
         return;
     }
     int grid = rn_bwd_grid(c, rows);
-    float* partial = (float*)sb_scratch(c, (size_t)grid * cols * sizeof(float));
+    float* partial = rn_partials(c, (size_t)grid * cols);
     if (!partial) return;
     sb_rmsnorm_backward_with_partials(c, x, w, dy, resid, dx_out, dscale, rows, cols, eps, partial, grid);
 }
@@ -1117,7 +1201,9 @@ extern "C" int seraph_b200_rmsnorm_backward_static(const float* input, const flo
     // so nothing left over from an earlier call is ever read and no clearing is needed
     // plain launches on the caller's stream, which may be under capture
     rmsnorm_bwd_kernel<<<grid, RB_THREADS, 0, s>>>(input, scale, grad_output, nullptr, grad_input, partial, rows, cols, eps, vec);
-    colsum_partials_kernel<<<(cols + 31) / 32, 32 * CS_GROUPS, 0, s>>>(partial, grad_scale, grid, cols);
+    CsTab tab;
+    tab.store = 0; tab.e[0] = {partial, grad_scale, grid, cols};
+    colsum_partials_kernel<<<(cols + 31) / 32, 32 * CS_GROUPS, 0, s>>>(tab);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         fprintf(stderr, "seraph_b200_rmsnorm_backward_static: launch failed: %s\n", cudaGetErrorString(e));

@@ -75,6 +75,7 @@ typedef struct sb_ctx {
        the operand preparation then skips its own pass over the tensor */
     struct { const float* ptr; size_t n; } *hint_tab; int hint_n, hint_cap; float* hint_pool;
     struct { const float* ptr; size_t n; } hint_pending[4]; int hint_npending;
+    void* cs_pending; int cs_defer, cs_store;      /* dscale sums waiting for their common launch */
     int weights_fixed, in_evaluate; unsigned weights_gen;      /* the weights' parts outlive the call while weights_gen stands */
     unsigned parts_gen; int parts_open; int parts_cache;   /* parts_cache 0: off (switch, or the arena did not fit) */
     int eval_batch_tokens;           /* cuda_evaluate packs samples up to this many tokens per forward pass; 0: one sample per pass */
@@ -182,6 +183,10 @@ void sb_tick_end(sb_ctx_t* c, int slot, double flops, double bytes);
 /* ---- kernel launchers (raw pointers) ---- */
 void sb_embed_lookup(sb_ctx_t*, const uint32_t* tok, const float* E, float* out, int T, int d, int V);
 void sb_rmsnorm(sb_ctx_t*, const float* x, const float* w, float* y, int rows, int cols, float eps);
+void sb_rmsnorm_copy(sb_ctx_t*, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps);
+void sb_colsum_defer(sb_ctx_t*, int on, int store, size_t floats);      /* dscale sums of sb_rmsnorm_backward in one launch at the flush */
+void sb_colsum_flush(sb_ctx_t*);
+void sb_colsum_free(sb_ctx_t*);
 /* dx = rmsnorm'(x; dy); if resid != NULL, dx_out = resid + dx (fused residual-gradient add) */
 void sb_qk_norm(sb_ctx_t*, float* x, float* rms_out, int rows, int cols, float eps);
 void sb_qk_norm_backward(sb_ctx_t*, const float* y, const float* rms, const float* dy, float* dx, int rows, int cols, float eps);
@@ -201,7 +206,7 @@ void sb_swiglu_backward(sb_ctx_t*, const float* gate, const float* up, const flo
 /* The same two, writing `out` (dgate, dup) only as the FP16 parts of registered tensors, scaled by bounds formed from the largest
    magnitudes their producers left for the inputs; 1 = done, 0 = not possible here (no parts, no hints): call the plain one */
 int  sb_swiglu_parts(sb_ctx_t*, const float* gate, const float* up, float* out, size_t n);
-int  sb_rmsnorm_parts(sb_ctx_t*, const float* x, const float* w, float* y, int rows, int cols, float eps);      /* bound: sqrt(cols) max|w| */
+int  sb_rmsnorm_parts(sb_ctx_t*, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps);      /* bound: sqrt(cols) max|w| */
 int  sb_swiglu_backward_parts(sb_ctx_t*, const float* gate, const float* up, const float* dout, float* dgate, float* dup, size_t n);
 void sb_amax_forget(sb_ctx_t*, const float* x);      /* x is written by something that leaves no maximum: earlier hints for it are void */
 void sb_seq_index(sb_ctx_t*, const uint32_t* seq_starts, int B, int T, uint32_t* pos_ids, uint32_t* seq_ids);

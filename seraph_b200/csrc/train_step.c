@@ -811,9 +811,10 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
         const sb_layer_off_t* o = &c->off[l];
         sb_layer_act_t* a = &c->act[l];
         float* next_in = (l + 1 < L) ? c->act[l + 1].layer_in : c->final_in;
-        if (!(xa_parts && sb_rmsnorm_parts(c, a->layer_in, c->W + o->in_norm, a->x_norm_attn, T, d, RMS_EPS))) {
+        /* the norms also write the rows they read to where the residual stream goes on: the o and down projections add into that copy */
+        if (!(xa_parts && sb_rmsnorm_parts(c, a->layer_in, c->W + o->in_norm, a->x_norm_attn, a->post_attn_in, T, d, RMS_EPS))) {
             sb_amax_announce(c, a->x_norm_attn, Td);       /* producers of GEMM operands leave max |x| behind for the operand split */
-            sb_rmsnorm(c, a->layer_in, c->W + o->in_norm, a->x_norm_attn, T, d, RMS_EPS);
+            sb_rmsnorm_copy(c, a->layer_in, c->W + o->in_norm, a->x_norm_attn, a->post_attn_in, T, d, RMS_EPS);
         }
         /* runs of products that share an operand keep its prepared parts (the adapters' scratch, rewritten in between, is dropped from the kept set at every write) */
         sb_gemm_keep_begin(c);
@@ -846,12 +847,11 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
         }
         sb_amax_announce(c, a->attn_out, (size_t)T * qd);
         sb_attention(c, a->q, a->k, a->v, a->attn_out, a->lse, c->seq_starts, c->seq_ids, T, c->Hq, c->Hkv, c->hd);
-        sb_copy(c, a->post_attn_in, a->layer_in, Td * sizeof(float));
         if (use_lora && c->lora_grouped) { const proj_t p = {3, c->W + o->o, a->post_attn_in, d, 1}; sb_gemm_keep_begin(c); lora_fwd_group(c, l, a->attn_out, &p, 1, T, qd); sb_gemm_keep_end(c); }
         else linear_fwd(c, use_lora, l, 3, a->attn_out, c->W + o->o, a->post_attn_in, T, qd, d, 1);
-        if (!(xf_parts && sb_rmsnorm_parts(c, a->post_attn_in, c->W + o->post_norm, a->x_norm_ffn, T, d, RMS_EPS))) {
+        if (!(xf_parts && sb_rmsnorm_parts(c, a->post_attn_in, c->W + o->post_norm, a->x_norm_ffn, next_in, T, d, RMS_EPS))) {
             sb_amax_announce(c, a->x_norm_ffn, Td);
-            sb_rmsnorm(c, a->post_attn_in, c->W + o->post_norm, a->x_norm_ffn, T, d, RMS_EPS);
+            sb_rmsnorm_copy(c, a->post_attn_in, c->W + o->post_norm, a->x_norm_ffn, next_in, T, d, RMS_EPS);
         }
         sb_gemm_keep_begin(c);
         sb_amax_announce(c, a->gate, (size_t)T * F);        /* the products' epilogues leave max |gate|, max |up| for the bound below */
@@ -873,12 +873,11 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
             sb_amax_announce(c, a->ffn_hidden, (size_t)T * F);
             sb_swiglu(c, a->gate, a->up, a->ffn_hidden, (size_t)T * F);
         }
-        sb_copy(c, next_in, a->post_attn_in, Td * sizeof(float));
         if (use_lora && c->lora_grouped) { const proj_t p = {6, c->W + o->down, next_in, d, 1}; sb_gemm_keep_begin(c); lora_fwd_group(c, l, a->ffn_hidden, &p, 1, T, F); sb_gemm_keep_end(c); }
         else linear_fwd(c, use_lora, l, 6, a->ffn_hidden, c->W + o->down, next_in, T, F, d, 1);
         nan_mark(c, next_in, Td, nan_fwd_base(c) + (uint32_t)l);
     }
-    if (!(hn_parts && sb_rmsnorm_parts(c, c->final_in, c->W + (size_t)c->V * d, c->hidden_norm, T, d, RMS_EPS))) {
+    if (!(hn_parts && sb_rmsnorm_parts(c, c->final_in, c->W + (size_t)c->V * d, c->hidden_norm, NULL, T, d, RMS_EPS))) {
         sb_amax_announce(c, c->hidden_norm, Td);
         sb_rmsnorm(c, c->final_in, c->W + (size_t)c->V * d, c->hidden_norm, T, d, RMS_EPS);
     }
@@ -891,16 +890,21 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
 typedef struct { int on, done, step; float lr, gscale; } early_adamw_t;
 
 /* `reduce`: hand every finished gradient range to the data-parallel all-reduce as soon as it is complete */
-static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, int full, int reduce, early_adamw_t* early) {
+/* store: the gradients of this pass are the first of their accumulation cycle; products and norm sums write them instead of adding to zeros */
+static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, int full, int store, int reduce, early_adamw_t* early) {
     const int d = c->d, F = c->F, qd = c->qd, kvd = c->kvd, L = c->L, V = c->V;
     float* gh = c->g_hidden; float* gx = c->g_xnorm;
     float* Gd = full ? c->G : NULL;
     float* norm_sink = NULL;                     /* LoRA mode: norm-scale gradients are not formed */
+    const int add = !store;
     const int grouped = !full && c->lora_grouped;
+    /* the gradients of all norm scales are summed in one launch at the end, unless the layers' buckets are handed to the all-reduce as they come */
+    const size_t sms = (size_t)(c->pub.gpu_sm_count > 0 ? c->pub.gpu_sm_count : 148);
+    sb_colsum_defer(c, full && !reduce, store, sms * ((size_t)(2 * L + 1) * 2 * ((size_t)d + 32) + (c->head_norm ? (size_t)2 * L * 4 * ((size_t)c->hd + 32) : 0)));
     sb_gemm_keep_begin(c);
     {
         const sb_gemm_job_t jobs[2] = {{c->dlogits, c->untied ? c->XW + extras_lm_off(c) : c->W, gx, T, d, V, 0, 0, 0},
-                                       {c->dlogits, c->hidden_norm, c->untied ? c->XG + extras_lm_off(c) : Gd, V, d, T, 1, 0, 1}};
+                                       {c->dlogits, c->hidden_norm, c->untied ? c->XG + extras_lm_off(c) : Gd, V, d, T, 1, 0, add}};
         sb_gemm_group(c, jobs, full ? 2 : 1);
     }
     sb_gemm_keep_end(c);
@@ -920,7 +924,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
             const int ad = 6; const float *dy = gh, *w = c->W + o->down;
             lora_bwd_group(c, l, &ad, &dy, &w, 1, a->ffn_hidden, c->g_ffn, T, F);
         } else {
-            const sb_gemm_job_t jobs[2] = {{gh, c->W + o->down, c->g_ffn, T, F, d, 0, 0, 0}, {gh, a->ffn_hidden, Gd + o->down, d, F, T, 1, 0, 1}};
+            const sb_gemm_job_t jobs[2] = {{gh, c->W + o->down, c->g_ffn, T, F, d, 0, 0, 0}, {gh, a->ffn_hidden, Gd + o->down, d, F, T, 1, 0, add}};
             sb_gemm_group(c, jobs, full ? 2 : 1);
         }
         if (!full && !grouped) lora_bwd(c, l, 6, gh, a->ffn_hidden, c->g_ffn, T);
@@ -935,7 +939,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
             lora_bwd_group(c, l, ads, dy, w, 2, a->x_norm_ffn, gx, T, d);
         } else {
             const sb_gemm_job_t jobs[4] = {{c->g_gate, c->W + o->gate, gx, T, d, F, 0, 0, 0}, {c->g_up, c->W + o->up, gx, T, d, F, 0, 0, 1},
-                                           {c->g_gate, a->x_norm_ffn, Gd + o->gate, F, d, T, 1, 0, 1}, {c->g_up, a->x_norm_ffn, Gd + o->up, F, d, T, 1, 0, 1}};
+                                           {c->g_gate, a->x_norm_ffn, Gd + o->gate, F, d, T, 1, 0, add}, {c->g_up, a->x_norm_ffn, Gd + o->up, F, d, T, 1, 0, add}};
             sb_gemm_group(c, jobs, full ? 4 : 2);
         }
         if (!full && !grouped) { lora_bwd(c, l, 4, c->g_gate, a->x_norm_ffn, gx, T); lora_bwd(c, l, 5, c->g_up, a->x_norm_ffn, gx, T); }
@@ -948,12 +952,12 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
             const int ad = 3; const float *dy = gh, *w = c->W + o->o;
             lora_bwd_group(c, l, &ad, &dy, &w, 1, a->attn_out, l > 0 || (c->lora_mask & 7) ? c->g_attn : NULL, T, qd);
         } else {
-            const sb_gemm_job_t jobs[2] = {{gh, c->W + o->o, c->g_attn, T, qd, d, 0, 0, 0}, {gh, a->attn_out, Gd + o->o, d, qd, T, 1, 0, 1}};
+            const sb_gemm_job_t jobs[2] = {{gh, c->W + o->o, c->g_attn, T, qd, d, 0, 0, 0}, {gh, a->attn_out, Gd + o->o, d, qd, T, 1, 0, add}};
             sb_gemm_group(c, jobs, full ? 2 : 1);
         }
         if (!full && !grouped) lora_bwd(c, l, 3, gh, a->attn_out, c->g_attn, T);
         sb_gemm_keep_end(c);
-        if (grouped && !c->nan_on && l == 0 && !(c->lora_mask & 7)) break;      /* below the first layer's o projection nothing is trained */
+        if (grouped && !c->nan_on && l == 0 && !(c->lora_mask & 7)) goto layer_done;      /* below the first layer's o projection nothing is trained */
         nan_mark(c, c->g_attn, (size_t)T * qd, nan_bwd_base(c) + 5u * (uint32_t)l);
         sb_attention_backward(c, a->q, a->k, a->v, a->attn_out, a->lse, c->g_attn, c->g_q, c->g_k, c->g_v, 0,
                               c->seq_starts, c->seq_ids, B, T, c->Hq, c->Hkv, c->hd);
@@ -983,8 +987,8 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
             lora_bwd_group(c, l, ads, dy, w, 3, a->x_norm_attn, last ? NULL : gx, T, d);
         } else {
             const sb_gemm_job_t jobs[6] = {{gq, c->W + o->q, gx, T, d, qd, 0, 0, 0}, {gk, c->W + o->k, gx, T, d, kvd, 0, 0, 1}, {c->g_v, c->W + o->v, gx, T, d, kvd, 0, 0, 1},
-                                           {gq, a->x_norm_attn, Gd + o->q, qd, d, T, 1, 0, 1}, {gk, a->x_norm_attn, Gd + o->k, kvd, d, T, 1, 0, 1},
-                                           {c->g_v, a->x_norm_attn, Gd + o->v, kvd, d, T, 1, 0, 1}};
+                                           {gq, a->x_norm_attn, Gd + o->q, qd, d, T, 1, 0, add}, {gk, a->x_norm_attn, Gd + o->k, kvd, d, T, 1, 0, add},
+                                           {c->g_v, a->x_norm_attn, Gd + o->v, kvd, d, T, 1, 0, add}};
             sb_gemm_group(c, jobs, full ? 6 : 3);
         }
         if (!full && !grouped) { lora_bwd(c, l, 0, gq, a->x_norm_attn, gx, T); lora_bwd(c, l, 1, gk, a->x_norm_attn, gx, T); lora_bwd(c, l, 2, c->g_v, a->x_norm_attn, gx, T); }
@@ -993,6 +997,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
             sb_amax_announce(c, gh, (size_t)T * d);
             sb_rmsnorm_backward(c, a->layer_in, c->W + o->in_norm, gx, gh, gh, full ? Gd + o->in_norm : norm_sink, T, d, RMS_EPS);
         }
+    layer_done:
         nan_mark(c, gh, (size_t)T * d, nan_ghid_base(c) + (uint32_t)l);
         if (!full && c->LW && reduce) lora_compact_grads(c, l, 1);
         if (reduce) {
@@ -1001,6 +1006,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
         }
     }
     if (!full && c->LW && !reduce) lora_compact_grads(c, 0, L);
+    sb_colsum_defer(c, 0, 0, 0);
     if (full) {
         nan_mark(c, gh, (size_t)T * d, 8);
         sb_embedding_backward(c, c->tokens, gh, Gd, T, d, V);
@@ -1058,6 +1064,11 @@ static float lr_for_step(const train_state_t* st, int accum) {
     return lr / accum;
 }
 
+static int grads_can_store(const sb_ctx_t* c, int T) {
+    sb_ctx_t* m = (sb_ctx_t*)c;
+    return sb_gemm_group_takes(m, c->V, c->d, T, 1, 0) && sb_gemm_group_takes(m, c->qd, c->d, T, 1, 0) && sb_gemm_group_takes(m, c->kvd, c->d, T, 1, 0) &&
+           sb_gemm_group_takes(m, c->d, c->qd, T, 1, 0) && sb_gemm_group_takes(m, c->F, c->d, T, 1, 0) && sb_gemm_group_takes(m, c->d, c->F, T, 1, 0);
+}
 static float step_body(train_state_t* st, int* tokens, int T, int* seq_starts, int B, cuda_train_context_t* ctx, int full, int train, int resident) {
     sb_ctx_t* c = sb_priv(ctx);
     if (!st || !st->config || !c || T <= 0 || B <= 0) return -1.0f;
@@ -1099,10 +1110,14 @@ static float step_body(train_state_t* st, int* tokens, int T, int* seq_starts, i
     c->pub.batch_size = B;
 
     if (nan_begin(c, train && st->debug_nan_check)) return -1.0f;
+    /* the first pass of a cycle writes every gradient when all weight gradients come from the grouped products: no clearing, no read-modify-write */
+    int store = 0;
     if (train && st->accumulation_counter == 0) {
-        if (full) sb_memset(c, c->G, 0, c->n_params * sizeof(float));
+        store = full && !c->nan_on && grads_can_store(c, T);
+        if (store) { if (c->untied) sb_memset(c, c->G, 0, (size_t)c->V * c->d * sizeof(float)); }
+        else if (full) sb_memset(c, c->G, 0, c->n_params * sizeof(float));
         else { sb_memset(c, c->LG, 0, c->n_lora * sizeof(float)); if (c->LGp != c->LG) sb_memset(c, c->LGp, 0, c->n_lora_pad * sizeof(float)); }
-        if (full && c->XG) sb_memset(c, c->XG, 0, c->n_extras * sizeof(float));
+        if (full && c->XG && !store) sb_memset(c, c->XG, 0, c->n_extras * sizeof(float));
     }
     forward_pass(c, T, max_seq, theta, use_lora);
     /* training: the gradient of the logits leaves the loss kernel as the FP16 parts the two LM-head backward products read (its
@@ -1127,7 +1142,7 @@ static float step_body(train_state_t* st, int* tokens, int T, int* seq_starts, i
             train_state_t tmp = *st; tmp.optimizer_step = early.step;
             early.lr = lr_for_step(&tmp, accum);
         }
-        backward_pass(c, T, B, max_seq, theta, full, last_micro && c->dp_world > 1, &early);
+        backward_pass(c, T, B, max_seq, theta, full, store, last_micro && c->dp_world > 1, &early);
         if (c->nan_on) {
             /* the reference reads its flags back before the optimizer and skips it when one is set, leaving the counters alone
                (src/train_cuda.c:1086-1187).  Data parallel: the buckets are already in flight, so every rank first waits for them and
@@ -1405,7 +1420,7 @@ void cuda_train_free(cuda_train_context_t* ctx) {
     if (c->seq_copy_stream) cudaStreamDestroy((cudaStream_t)c->seq_copy_stream);
     for (int i = 0; i < 2; i++) if (c->seq_copy_ev[i]) cudaEventDestroy((cudaEvent_t)c->seq_copy_ev[i]);
     if (c->h_seq_pin) cudaFreeHost(c->h_seq_pin);
-    sb_parts_free(c);
+    sb_parts_free(c); sb_colsum_free(c);
     if (c->d_amax) cudaFree(c->d_amax);
     for (int i = 0; i < SB_F16_SLOTS; i++) if (c->f16_slot[i].h) cudaFree(c->f16_slot[i].h);
     if (c->d_status) cudaFree(c->d_status);
