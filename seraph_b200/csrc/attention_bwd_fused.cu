@@ -120,7 +120,8 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
                   __half* __restrict__ dS1, __half* __restrict__ dS2, float* __restrict__ dK, float* __restrict__ dV,
                   const float* __restrict__ amax_q, const float* __restrict__ amax_k, const float* __restrict__ amax_v,
                   const float* __restrict__ amax_do, const float* __restrict__ ds_bound,
-                  const AfSeqTab seqs, int Sp, int Hq, int g, int nkb, int chunk, int accumulate, int slot_pitch, float scale, int* status) {
+                  const AfSeqTab seqs, int Sp, int Hq, int g, int nkb, int chunk, int accumulate, int slot_pitch, float scale, int* status,
+                  unsigned* amax_dk, unsigned* amax_dv) {
     sb_pdl_enter();
     constexpr int NH = HD / 64;
     constexpr int KV_PART = NH * 16384, ST_PART = NH * 4096;
@@ -386,6 +387,18 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
                     add(a3, v);
                 }
                 if (ok) { emit(0, !accumulate, a0, a1, a0, a1); emit(1, !accumulate, a2, a3, a2, a3); }
+                if (amax_dk && amax_dv) {
+                    float mk = 0.f, mv = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 32; i++) {
+                        mk = fmaxf(mk, fmaxf(fabsf(__uint_as_float(a0[i])), fabsf(__uint_as_float(a1[i]))));
+                        mv = fmaxf(mv, fmaxf(fabsf(__uint_as_float(a2[i])), fabsf(__uint_as_float(a3[i]))));
+                    }
+                    mk = live ? mk * fk : 0.f; mv = live ? mv * fv : 0.f;
+                    for (int d = 16; d > 0; d >>= 1) { mk = fmaxf(mk, __shfl_xor_sync(0xffffffffu, mk, d)); mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, d)); }
+                    if (lane == 0 && mk > 0.f) atomicMax(amax_dk, __float_as_uint(mk));
+                    if (lane == 0 && mv > 0.f) atomicMax(amax_dv, __float_as_uint(mv));
+                }
             } else {
                 for (int c = 0; c < nchains && ok; c++) {
                     ok = mbar_wait(acc_ready, c & 1);
@@ -584,7 +597,7 @@ __global__ void __launch_bounds__(AQ_THREADS, 1)
 at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant__ CUtensorMap mS2,
                  const __grid_constant__ CUtensorMap mK1, const __grid_constant__ CUtensorMap mK2,
                  const AfSeqTab seqs, float* __restrict__ dQ, const float* __restrict__ ds_bound, const float* __restrict__ amax_k,
-                 int Sp, int Hq, int g, int nqb_max, int* status) {
+                 int Sp, int Hq, int g, int nqb_max, int* status, unsigned* amax_dq) {
     sb_pdl_enter();
     constexpr int NH = HD / 64, OC = HD / 2;
     const int per_i = seqs.n * Hq;
@@ -691,12 +704,20 @@ at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant_
                 if constexpr (OC == 64) o[32 + i] += __uint_as_float(t2[i]);
             }
         }
+        float am = 0.f;
         if (ok && qi < S) {
             const float f1 = tc_pow2(-tc_f16_shift(sb_word(ds_bound))), f2 = tc_pow2(-tc_f16_shift(sb_word(amax_k)));
             float4* dst = (float4*)(dQ + (size_t)(t0 + qi) * Hq * HD + (size_t)h * HD + ch * OC);
 #pragma unroll
-            for (int i = 0; i < OC / 4; i++)
-                dst[i] = make_float4(o[4 * i] * f1 * f2, o[4 * i + 1] * f1 * f2, o[4 * i + 2] * f1 * f2, o[4 * i + 3] * f1 * f2);
+            for (int i = 0; i < OC / 4; i++) {
+                const float4 v = make_float4(o[4 * i] * f1 * f2, o[4 * i + 1] * f1 * f2, o[4 * i + 2] * f1 * f2, o[4 * i + 3] * f1 * f2);
+                dst[i] = v;
+                am = sb_amax4(am, v);
+            }
+        }
+        if (amax_dq) {
+            for (int d = 16; d > 0; d >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, d));
+            if (lane == 0 && am > 0.f) atomicMax(amax_dq, __float_as_uint(am));
         }
         if (!ok && lane == 0) atomicExch(status, SB_ERR_TIMEOUT);
     }
@@ -755,10 +776,10 @@ static int ab_launch(sb_ctx_t* c, const AbCall& p) {
     if (qblocks > 0x7fffffffL) return 1;
     cudaStream_t st = (cudaStream_t)c->pub.stream;
     sb_launch(kern, dim3((unsigned)blocks), dim3(AB_THREADS), AB_SMEM(NH), st, mQ1, mQ2, mD1, mD2, mK1, mK2, mV1, mV2, mS1, mS2, mdK, mdV, p.LT, p.DT, (__half*)p.dS1, (__half*)p.dS2, p.dK, p.dV,
-        p.amax_q, p.amax_k, p.amax_v, p.amax_do, p.ds_bound, seqs, p.Sp, p.Hq, g, nkb, chunk, p.accumulate, slot_pitch, 1.0f / sqrtf((float)HD), c->d_status);
+        p.amax_q, p.amax_k, p.amax_v, p.amax_do, p.ds_bound, seqs, p.Sp, p.Hq, g, nkb, chunk, p.accumulate, slot_pitch, 1.0f / sqrtf((float)HD), c->d_status, p.amax_dk, p.amax_dv);
     c->launches++;
     if (p.dQ) {
-        sb_launch(at_dq_bwd_kernel<HD>, dim3((unsigned)qblocks), dim3(AQ_THREADS), AQ_SMEM(NH), st, mA1, mA2, mB1, mB2, seqs, p.dQ, p.ds_bound, p.amax_k, p.Sp, p.Hq, g, nkb, c->d_status);
+        sb_launch(at_dq_bwd_kernel<HD>, dim3((unsigned)qblocks), dim3(AQ_THREADS), AQ_SMEM(NH), st, mA1, mA2, mB1, mB2, seqs, p.dQ, p.ds_bound, p.amax_k, p.Sp, p.Hq, g, nkb, c->d_status, p.amax_dq);
         c->launches++;
     }
     return cudaGetLastError() == cudaSuccess ? 0 : 1;

@@ -30,8 +30,9 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
                     const __grid_constant__ CUtensorMap mV1, const __grid_constant__ CUtensorMap mV2,
                     const AfSeqTab seqs, float* __restrict__ O, float* __restrict__ lse,
                     const float* __restrict__ amax_q, const float* __restrict__ amax_k, const float* __restrict__ amax_v,
-                    int Hq, int g, int nqb_max, float scale, int* status, unsigned* amax_o) {
+                    int Hq, int g, int nqb_max, float scale, int* status, float* bound_o, uint4* __restrict__ Oh, size_t n_o, unsigned keep) {
     sb_pdl_enter();
+    if (bound_o && blockIdx.x == 0 && threadIdx.x == 0) *bound_o = sb_word(amax_v);
     constexpr int NH = HD / 64;                              // 64-column halves of the head dimension (one 128-byte row of halfs each)
     constexpr int Q_BYTES = NH * 32768, KV_STAGE = NH * 16384, Q_PART = NH * 16384, KV_PART = NH * 8192;
     constexpr int OFF_K = Q_BYTES, OFF_V = OFF_K + 2 * KV_STAGE, OFF_P = OFF_V + 2 * KV_STAGE, OFF_BAR = OFF_P + 32768;
@@ -294,20 +295,24 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
             if (lane == 0) af_arrive(&pv_empty[s]);
         }
         if (ok) ok = mbar_wait(fin_full, 0);
-        float am = 0.f;
+        // O is a weighted mean of rows of V, so max |V| bounds it: its word for the output projection's operand, and the scale of the parts that
+        // are written here beside O (a split pass over O less)
         if (ok && qi < S) {
             const float f = fin_s[r] * tc_pow2(-tc_f16_shift(sb_word(amax_v)));      // fin = 1 / l with l in units of 2^-14, O holds (P * 2^14) V' products
-            float4* dst = (float4*)(O + (size_t)(t0 + qi) * qd + (size_t)h * HD + ch * OC);
+            const size_t at = (size_t)(t0 + qi) * qd + (size_t)h * HD + ch * OC;
+            float4* dst = (float4*)(O + at);
 #pragma unroll
-            for (int i = 0; i < OC / 4; i++) {
-                const float4 v = make_float4(o[4 * i] * f, o[4 * i + 1] * f, o[4 * i + 2] * f, o[4 * i + 3] * f);
-                dst[i] = v;
-                am = sb_amax4(am, v);
+            for (int i = 0; i < OC / 4; i++) dst[i] = make_float4(o[4 * i] * f, o[4 * i + 1] * f, o[4 * i + 2] * f, o[4 * i + 3] * f);
+            if (Oh) {
+                const float sc = tc_pow2(tc_f16_shift(sb_word(amax_v)));
+#pragma unroll
+                for (int i = 0; i < OC / 8; i++) {
+                    uint4 a, b;
+                    sb_split2(o[8 * i] * f * sc, o[8 * i + 1] * f * sc, a.x, b.x, keep); sb_split2(o[8 * i + 2] * f * sc, o[8 * i + 3] * f * sc, a.y, b.y, keep);
+                    sb_split2(o[8 * i + 4] * f * sc, o[8 * i + 5] * f * sc, a.z, b.z, keep); sb_split2(o[8 * i + 6] * f * sc, o[8 * i + 7] * f * sc, a.w, b.w, keep);
+                    Oh[at / 8 + i] = a; Oh[(n_o + at) / 8 + i] = b;
+                }
             }
-        }
-        if (amax_o) {                                          // largest |O|, for the split of the output projection's operand
-            for (int d = 16; d > 0; d >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, d));
-            if (lane == 0 && am > 0.f) atomicMax(amax_o, __float_as_uint(am));
         }
         if (!ok && lane == 0) atomicExch(status, SB_ERR_TIMEOUT);
     }
@@ -566,8 +571,12 @@ static int af_launch_fwd(sb_ctx_t* c, const void* q1, const void* q2, const void
         !af_make_map(c, &mV1, v1, T, kvd, AF_BKV) || !af_make_map(c, &mV2, v2, T, kvd, AF_BKV)) return 1;
     const long blocks = (long)nqb * seqs.n * Hq;
     if (blocks > 0x7fffffffL) return 1;
+    const size_t n_o = (size_t)T * qd;
+    void* oh; float* own; int fresh;
+    float* bound_o = (float*)sb_amax_take(c, O, n_o);
+    if (sb_parts_find(c, O, n_o, &oh, &own, &fresh)) sb_parts_set_amax(c, O, (float*)amax_v); else oh = nullptr;      // O of a training step is an operand
     sb_launch(kern, dim3((unsigned)blocks), dim3(AF_THREADS), smem, (cudaStream_t)c->pub.stream, mQ1, mQ2, mK1, mK2, mV1, mV2, seqs, O, lse, amax_q, amax_k, amax_v, Hq, Hq / Hkv, nqb, 1.0f / sqrtf((float)HD), c->d_status,
-        sb_amax_take(c, O, (size_t)T * qd));
+        bound_o, (uint4*)oh, n_o, sb_parts_keep(c));
     c->launches++;
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }

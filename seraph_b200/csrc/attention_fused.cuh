@@ -117,5 +117,6 @@ struct AbCall {
     void *dS1, *dS2;
     float *dK, *dV, *dQ;
     int accumulate, Sp, T, Hq, Hkv;
+    unsigned *amax_dq, *amax_dk, *amax_dv;      // max |dQ|, |dK|, |dV| of this call are left there (64-wide heads, whose outputs pass through registers whole; else NULL)
 };
 int sb_attention_fused_dkv(sb_ctx_t* c, const AbCall& p, int hd);

@@ -248,11 +248,11 @@ __global__ void __launch_bounds__(256) at_bwd_prep_kernel(const float* __restric
 // after the subtraction, which keeps the rounding of the large terms out of the exponent), and D times the factor that takes
 // P 2^14 (dP - D) to the scaled dS.
 __global__ void __launch_bounds__(256) at_bwd_prep2_kernel(const float4* __restrict__ dO, size_t n4, uint2* __restrict__ h1, uint2* __restrict__ h2,
-                                                           const float* __restrict__ amax, float* consts, const float* __restrict__ norms, float scale,
+                                                           const float* __restrict__ amax, float* consts, const float* __restrict__ norm_do, const float* __restrict__ norm_v, float scale,
                                                            const float* __restrict__ lse, const float* __restrict__ D, float* __restrict__ LT, float* __restrict__ DT,
                                                            const AfSeqTab seqs, int Hq, int Smax, int slot_pitch, int natural) {
     sb_pdl_enter();
-    const float bound = 2.0f * sb_word(norms) * sb_word(norms + 1) * scale;
+    const float bound = 2.0f * sb_word(norm_do) * sb_word(norm_v) * scale;
     if (blockIdx.y == 0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) { consts[0] = 1.0f; consts[1] = bound; }
         const float sc = tc_pow2(tc_f16_shift(sb_word(amax)));
@@ -298,6 +298,10 @@ static bool at_one_kernel(sb_ctx_t* c, int Hq, int Hkv, int hd) {
     const int mode = c->pub.use_bf16 ? SB_GEMM_BF16 : c->gemm_mode;
     if (mode == SB_GEMM_SIMT || mode == SB_GEMM_FP32X3 || !c->gemm_pair || !c->attn_flash || c->attn_fused || (hd != 64 && hd != 128)) return false;
     return Hkv > 0 && Hq % Hkv == 0 && c->attn_seq_starts && tc_load_encode();
+}
+extern "C" int sb_attention_reads_parts(sb_ctx_t* c, int Hq, int Hkv, int hd) {
+    const int mode = c->pub.use_bf16 ? SB_GEMM_BF16 : c->gemm_mode;
+    return mode != SB_GEMM_SIMT && mode != SB_GEMM_FP32X3 && c->gemm_pair && c->attn_flash == 1 && !c->attn_fused && (hd == 64 || hd == 128) && Hkv > 0 && Hq % Hkv == 0;
 }
 // the boundaries on the host: usable for the tensor-core paths?  (waits for them if they are still on their way)
 static bool at_have_seq(sb_ctx_t* c, int T) {
@@ -537,17 +541,20 @@ static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, cons
     __half* hb = (__half*)(consts + 64);
     cudaStream_t st = (cudaStream_t)c->pub.stream;
     int tk = sb_tick_begin(c, SB_CLS_ATTN_BWD);
-    cudaMemsetAsync(consts, 0, 64 * sizeof(float), st);
+    // words that start from zero: inside a step from its pool, else cleared here (a launch)
+    float *am_do = sb_zero_word(c), *norm_do = sb_zero_word(c), *norm_v = sb_zero_word(c);
+    const bool cleared = !norm_v;
+    if (cleared) { cudaMemsetAsync(consts, 0, 64 * sizeof(float), st); norm_do = consts + 2; norm_v = consts + 3; am_do = consts + 11; }
     const AtNeed need[3] = {{Q, n_q, hb, consts + 8}, {K, n_kv, hb + 2 * n_q, consts + 9}, {V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10}};
     AtParts p[3];
-    at_make_parts_multi(c, need, 3, p, true);
+    at_make_parts_multi(c, need, 3, p, cleared);
     __half* hdo = hb + 2 * n_q + 4 * n_kv;
     {
         const int rpb = 8 * 4 * (128 / hd);                          // rows a CTA takes per pass
         const int cap = c->pub.gpu_sm_count * 8, want = (T * Hq + rpb - 1) / rpb;
         const dim3 pg(want < cap ? want : cap, 2);
-        if (hd == 128) sb_launch(at_bwd_prep_kernel<128>, dim3(pg), dim3(256), 0, st, dO, O, D, T * Hq, V, T * Hkv, (unsigned*)(consts + 2), (unsigned*)(consts + 11), (unsigned*)(consts + 3));
-        else sb_launch(at_bwd_prep_kernel<64>, dim3(pg), dim3(256), 0, st, dO, O, D, T * Hq, V, T * Hkv, (unsigned*)(consts + 2), (unsigned*)(consts + 11), (unsigned*)(consts + 3));
+        if (hd == 128) sb_launch(at_bwd_prep_kernel<128>, dim3(pg), dim3(256), 0, st, dO, O, D, T * Hq, V, T * Hkv, (unsigned*)norm_do, (unsigned*)am_do, (unsigned*)norm_v);
+        else sb_launch(at_bwd_prep_kernel<64>, dim3(pg), dim3(256), 0, st, dO, O, D, T * Hq, V, T * Hkv, (unsigned*)norm_do, (unsigned*)am_do, (unsigned*)norm_v);
         c->launches++;
     }
     // from here on the launches depend on the boundaries
@@ -567,13 +574,14 @@ static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, cons
     float* LT = bb + n_ds; float* DT = LT + row_floats;
     {
         const AfSeqTab seqs = {n, c->attn_seq_starts};
-        sb_launch(at_bwd_prep2_kernel, dim3(dim3(tc_ew_blocks(c, n_q / 8), 2)), dim3(256), 0, st, (const float4*)dO, n_q / 4, (uint2*)hdo, (uint2*)(hdo + n_q), consts + 11,
-                                                                            consts, consts + 2, scale, lse, D, LT, DT, seqs, Hq, Smax, slot_pitch, hd == 64 ? 1 : 0);
+        sb_launch(at_bwd_prep2_kernel, dim3(dim3(tc_ew_blocks(c, n_q / 8), 2)), dim3(256), 0, st, (const float4*)dO, n_q / 4, (uint2*)hdo, (uint2*)(hdo + n_q), am_do,
+                                                                            consts, norm_do, norm_v, scale, lse, D, LT, DT, seqs, Hq, Smax, slot_pitch, hd == 64 ? 1 : 0);
         c->launches++;
     }
     __half* a = (__half*)bb;
-    AbCall call = {p[0].h1, p[0].h2, hdo, hdo + n_q, p[1].h1, p[1].h2, p[2].h1, p[2].h2, p[0].amax, p[1].amax, p[2].amax, consts + 11, consts + 1, LT, DT,
-                   a, a + n_ds, dK, dV, dq_gemm ? nullptr : dQ, accumulate_kv, Sp, T, Hq, Hkv};
+    AbCall call = {p[0].h1, p[0].h2, hdo, hdo + n_q, p[1].h1, p[1].h2, p[2].h1, p[2].h2, p[0].amax, p[1].amax, p[2].amax, am_do, consts + 1, LT, DT,
+                   a, a + n_ds, dK, dV, dq_gemm ? nullptr : dQ, accumulate_kv, Sp, T, Hq, Hkv, nullptr, nullptr, nullptr};
+    if (hd == 64 && !accumulate_kv) { call.amax_dq = sb_amax_take(c, dQ, n_q); call.amax_dk = sb_amax_take(c, dK, n_kv); call.amax_dv = sb_amax_take(c, dV, n_kv); }
     bool ok = sb_attention_fused_dkv(c, call, hd) == 0;
     if (ok && dq_gemm) {
         void* main_stream = c->pub.stream;

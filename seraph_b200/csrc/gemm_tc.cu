@@ -151,7 +151,7 @@ unsigned* sb_item_counter(sb_ctx_t* c) {
 extern "C" void sb_parts_open(sb_ctx_t* c) {
     c->parts_gen++; c->parts_open = 1;
     c->hint_n = 0; c->hint_npending = 0;
-    if (c->parts_cache && !c->hint_pool) {
+    if (!c->hint_pool) {
         c->hint_tab = (decltype(c->hint_tab))calloc(SB_HINT_CAP, sizeof *c->hint_tab);
         if (!c->hint_tab || cudaMalloc((void**)&c->hint_pool, SB_HINT_CAP * sizeof(float)) != cudaSuccess) { cudaGetLastError(); c->hint_pool = NULL; }
         c->hint_cap = c->hint_pool ? SB_HINT_CAP : 0;
@@ -160,10 +160,10 @@ extern "C" void sb_parts_open(sb_ctx_t* c) {
 }
 extern "C" void sb_parts_close(sb_ctx_t* c) { c->parts_gen++; c->parts_open = 0; c->hint_n = 0; c->hint_npending = 0; }
 extern "C" void sb_amax_announce(sb_ctx_t* c, const float* out, size_t n) {
-    if (!c->parts_open || !c->parts_cache || !c->hint_pool) return;
-    if (c->hint_npending >= 4) {                       // announcements nobody took (a launcher without the feature): the oldest goes
-        for (int i = 1; i < 4; i++) c->hint_pending[i - 1] = c->hint_pending[i];
-        c->hint_npending = 3;
+    if (!c->parts_open || !c->hint_pool) return;
+    if (c->hint_npending >= SB_HINT_PENDING) {         // announcements nobody took (a launcher without the feature): the oldest goes
+        for (int i = 1; i < SB_HINT_PENDING; i++) c->hint_pending[i - 1] = c->hint_pending[i];
+        c->hint_npending = SB_HINT_PENDING - 1;
     }
     c->hint_pending[c->hint_npending].ptr = out; c->hint_pending[c->hint_npending].n = n; c->hint_npending++;
 }

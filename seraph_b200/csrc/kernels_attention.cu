@@ -329,6 +329,7 @@ void sb_attention(sb_ctx_t* c, const float* Q, const float* K, const float* V, f
     if (T <= 0 || Hq <= 0 || Hkv <= 0 || hd <= 0) return;
     if (hd > 256 || Hq < Hkv) { sb_set_status(c, SB_ERR_SIZE); return; }
     c->attn_seq_starts = seq_starts;
+    sb_parts_invalidate(c, out);
     if (sb_attention_tc_forward(c, Q, K, V, out, lse, T, Hq, Hkv, hd) == 0) return;      // tensor-core path took it
     sb_resolve_seq_index(c);
     float scale = 1.0f / sqrtf((float)hd);
@@ -351,6 +352,7 @@ void sb_attention_backward(sb_ctx_t* c, const float* Q, const float* K, const fl
     if (T <= 0 || Hq <= 0 || Hkv <= 0 || hd <= 0) return;
     if (hd > 256) { sb_set_status(c, SB_ERR_SIZE); return; }
     c->attn_seq_starts = seq_starts;
+    sb_parts_invalidate(c, dQ); sb_parts_invalidate(c, dK); sb_parts_invalidate(c, dV);
     if (sb_attention_tc_backward(c, Q, K, V, O, lse, dO, dQ, dK, dV, accumulate_kv, T, Hq, Hkv, hd) == 0) return;
     sb_resolve_seq_index(c);
     float scale = 1.0f / sqrtf((float)hd);

@@ -259,6 +259,64 @@ __global__ void __launch_bounds__(EW_THREADS) rope_kernel(const float* qin, floa
     sb_block_amax(amk, amax_k);
 }
 
+// The same rotation with the FP16 operand parts of q, k and v written at once (v passes through unrotated): what would be a rotation pass and
+// a split pass over the three tensors.  A rotated pair is at most sqrt(2) times the larger of its two values, so max |x| of the input, left by
+// the kernel that wrote it, bounds the result and sets the scale.  f32: the rotated q and k are written as FP32 too (in place).
+__global__ void __launch_bounds__(EW_THREADS) rope_parts_kernel(float4* q, float4* k, const float4* __restrict__ v, uint2* __restrict__ hq, uint2* __restrict__ hk,
+                                                                uint2* __restrict__ hv, const uint32_t* __restrict__ pos_ids, const float2* __restrict__ tab,
+                                                                int T, int Hq, int Hkv, int hd, int backward, const float* am_q, const float* am_k, const float* am_v,
+                                                                float* bound_q, float* bound_k, int f32, unsigned keep) {
+    sb_pdl_enter();
+    const float bq = fminf(1.41422f * sb_word(am_q), 3.0e38f), bk = fminf(1.41422f * sb_word(am_k), 3.0e38f);
+    if (blockIdx.x == 0 && threadIdx.x == 0) { *bound_q = bq; *bound_k = bk; }
+    const float sq = sb_pow2(sb_f16_shift(bq)), sk = sb_pow2(sb_f16_shift(bk)), sv = sb_pow2(sb_f16_shift(sb_word(am_v)));
+    const uint32_t quads = (uint32_t)hd >> 2, rq = (uint32_t)Hq * quads, rk = (uint32_t)Hkv * quads, row_quads = rq + rk + (hv ? rk : 0u);
+    const uint32_t total = (uint32_t)T * row_quads, nth = gridDim.x * blockDim.x;
+    const size_t nq4 = (size_t)T * rq, nk4 = (size_t)T * rk;
+    for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; base < total; base += nth * ROPE_UNROLL) {
+        float4 x[ROPE_UNROLL], cs[ROPE_UNROLL];
+        size_t at[ROPE_UNROLL];
+        int which[ROPE_UNROLL];               // 0 q, 1 k, 2 v, 3 nothing
+#pragma unroll
+        for (int u = 0; u < ROPE_UNROLL; u++) {
+            const uint32_t i = base + u * nth;
+            which[u] = 3;
+            if (i < total) {
+                const uint32_t t = i / row_quads, rem = i - t * row_quads;
+                which[u] = rem < rq ? 0 : rem < rq + rk ? 1 : 2;
+                const uint32_t w = which[u] == 0 ? rem : which[u] == 1 ? rem - rq : rem - rq - rk;
+                at[u] = (size_t)t * (which[u] == 0 ? rq : rk) + w;
+                x[u] = which[u] == 0 ? q[at[u]] : which[u] == 1 ? k[at[u]] : v[at[u]];
+                if (which[u] < 2) cs[u] = ((const float4*)tab)[(size_t)pos_ids[t] * quads + w % quads];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < ROPE_UNROLL; u++) {
+            if (which[u] == 3) continue;
+            float4 r = x[u];
+            float sc = sv;
+            uint2* h = hv; size_t n4 = nk4;
+            if (which[u] < 2) {
+                if (!backward) {
+                    r.x = x[u].x * cs[u].x - x[u].y * cs[u].y; r.y = x[u].x * cs[u].y + x[u].y * cs[u].x;
+                    r.z = x[u].z * cs[u].z - x[u].w * cs[u].w; r.w = x[u].z * cs[u].w + x[u].w * cs[u].z;
+                } else {
+                    r.x = x[u].x * cs[u].x + x[u].y * cs[u].y; r.y = -x[u].x * cs[u].y + x[u].y * cs[u].x;
+                    r.z = x[u].z * cs[u].z + x[u].w * cs[u].w; r.w = -x[u].z * cs[u].w + x[u].w * cs[u].z;
+                }
+                const bool isq = which[u] == 0;
+                if (f32) { if (isq) q[at[u]] = r; else k[at[u]] = r; }
+                sc = isq ? sq : sk; h = isq ? hq : hk; if (isq) n4 = nq4;
+            }
+            if (h) {
+                uint2 a, b;
+                sb_split2(r.x * sc, r.y * sc, a.x, b.x, keep); sb_split2(r.z * sc, r.w * sc, a.y, b.y, keep);
+                h[at[u]] = a; h[n4 + at[u]] = b;
+            }
+        }
+    }
+}
+
 // Adapters between their compact form (A [r,in], B [out,r]) and the working copies of rank R (A [R,in], B [out,R]): blockIdx.y = adapter,
 // blockIdx.z = layer.  Only the live part moves; the padding of the working copies stays zero.
 struct LoraShapes { int n, r, R; int in[7], out[7]; size_t off[7], off_pad[7], per_layer, per_layer_pad; };
@@ -430,6 +488,29 @@ void sb_rope(sb_ctx_t* c, const float* in, float* out, const uint32_t* pos_ids, 
 }
 
 // q and k rotated in place by one launch when the fast path applies, else by two calls of sb_rope
+// q and k rotated in place and, with v, handed on as parts; 0: not done (the maxima of all three have to be known).  Without an arena for the
+// parts the words of q and k still get the same bounds, so that whoever splits them gets the same parts.
+int sb_rope_parts(sb_ctx_t* c, float* q, float* k, const float* v, const uint32_t* pos_ids, int T, int Hq, int Hkv, int hd, float theta, int max_pos, int backward, int f32) {
+    const double nq = (double)T * (Hq + 2 * Hkv) * (hd / 4);
+    if (T <= 0 || (hd & 7) || !aligned16(q) || !aligned16(k) || !aligned16(v) || nq >= 2147483648.0) return 0;
+    const size_t n_q = (size_t)T * Hq * hd, n_k = (size_t)T * Hkv * hd;
+    const float* aq = sb_amax_lookup(c, q, n_q); const float* ak = sb_amax_lookup(c, k, n_k); float* av = sb_amax_lookup(c, v, n_k);
+    if (!aq || !ak || !av || !rope_ensure_table(c, hd, theta, max_pos)) return 0;
+    sb_amax_announce(c, q, n_q); sb_amax_announce(c, k, n_k);
+    float* wq = (float*)sb_amax_take(c, q, n_q); float* wk = (float*)sb_amax_take(c, k, n_k);      // from here on the words of the rotated tensors
+    if (!wq || !wk) { sb_amax_forget(c, q); sb_amax_forget(c, k); return 0; }
+    void *hq, *hk, *hv; float* own; int fresh;
+    if (sb_parts_find(c, q, n_q, &hq, &own, &fresh)) sb_parts_set_amax(c, q, wq); else { hq = NULL; f32 = 1; }
+    if (sb_parts_find(c, k, n_k, &hk, &own, &fresh)) sb_parts_set_amax(c, k, wk); else { hk = NULL; f32 = 1; }
+    if (sb_parts_find(c, v, n_k, &hv, &own, &fresh)) sb_parts_set_amax(c, v, av); else hv = NULL;
+    int tk = sb_tick_begin(c, SB_CLS_ROPE);
+    const size_t work = ((size_t)nq + ROPE_UNROLL - 1) / ROPE_UNROLL;
+    sb_launch(rope_parts_kernel, dim3(ew_grid(c, work)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (float4*)q, (float4*)k, (const float4*)v, (uint2*)hq, (uint2*)hk,
+              (uint2*)hv, pos_ids, (const float2*)c->rope_tab, T, Hq, Hkv, hd, backward, aq, ak, (const float*)av, wq, wk, f32, sb_parts_keep(c));
+    sb_tick_end(c, tk, 0.0, (f32 ? 12.0 : 8.0) * T * (Hq + Hkv) * hd + 8.0 * T * Hkv * hd);
+    c->launches++;
+    return 1;
+}
 void sb_rope2(sb_ctx_t* c, float* q, float* k, const uint32_t* pos_ids, int T, int Hq, int Hkv, int hd, float theta, int max_pos, int backward) {
     if (T <= 0) return;
     const double nq = (double)T * (Hq + Hkv) * (hd / 4);

@@ -55,6 +55,7 @@ typedef struct {
 
 typedef struct { const float* ptr; size_t n, cur, off; unsigned gen; int kind; float* amax_ptr; } sb_parts_entry_t;   /* n: registered floats, cur: floats of the parts held */
 
+#define SB_HINT_PENDING 12
 typedef struct sb_ctx {
     cuda_train_context_t pub;        /* MUST stay first */
     uint32_t magic;
@@ -74,7 +75,7 @@ typedef struct sb_ctx {
     /* largest magnitudes left by the kernels that produce GEMM operands (announced by the step driver, valid inside one step):
        the operand preparation then skips its own pass over the tensor */
     struct { const float* ptr; size_t n; } *hint_tab; int hint_n, hint_cap; float* hint_pool;
-    struct { const float* ptr; size_t n; } hint_pending[4]; int hint_npending;
+    struct { const float* ptr; size_t n; } hint_pending[SB_HINT_PENDING]; int hint_npending;
     void* cs_pending; int cs_defer, cs_store;      /* dscale sums waiting for their common launch */
     int weights_fixed, in_evaluate; unsigned weights_gen;      /* the weights' parts outlive the call while weights_gen stands */
     unsigned parts_gen; int parts_open; int parts_cache;   /* parts_cache 0: off (switch, or the arena did not fit) */
@@ -206,6 +207,7 @@ void sb_swiglu_backward(sb_ctx_t*, const float* gate, const float* up, const flo
 /* The same two, writing `out` (dgate, dup) only as the FP16 parts of registered tensors, scaled by bounds formed from the largest
    magnitudes their producers left for the inputs; 1 = done, 0 = not possible here (no parts, no hints): call the plain one */
 int  sb_swiglu_parts(sb_ctx_t*, const float* gate, const float* up, float* out, size_t n);
+int  sb_attention_reads_parts(sb_ctx_t*, int Hq, int Hkv, int hd);      /* 1: forward and backward attention run on FP16 parts of q, k, v */
 int  sb_rmsnorm_parts(sb_ctx_t*, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps);      /* bound: sqrt(cols) max|w| */
 int  sb_swiglu_backward_parts(sb_ctx_t*, const float* gate, const float* up, const float* dout, float* dgate, float* dup, size_t n);
 void sb_amax_forget(sb_ctx_t*, const float* x);      /* x is written by something that leaves no maximum: earlier hints for it are void */
@@ -232,6 +234,7 @@ void sb_parts_set_amax(sb_ctx_t*, const float* x, float* word);
 /* 1: x[n] is registered and the step is open; *h = its two parts (h, h + n), *amax its scale word, *fresh = parts must be made now */
 int sb_parts_find(sb_ctx_t*, const float* x, size_t n, void** h, float** amax, int* fresh);
 void sb_parts_invalidate(sb_ctx_t*, const float* x);      /* x is rewritten as plain FP32: parts held for it are stale */
+int  sb_rope_parts(sb_ctx_t*, float* q, float* k, const float* v, const uint32_t* pos_ids, int T, int Hq, int Hkv, int hd, float theta, int max_pos, int backward, int f32);
 void sb_rope2(sb_ctx_t*, float* q, float* k, const uint32_t* pos_ids, int T, int Hq, int Hkv, int hd, float theta, int max_pos, int backward);
 void sb_rope(sb_ctx_t*, const float* in, float* out, const uint32_t* pos_ids, int T, int H, int hd, float theta,
              int max_pos, int backward);

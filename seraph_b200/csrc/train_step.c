@@ -589,6 +589,7 @@ static int ensure_activations(sb_ctx_t* c, int T, int need_logits_grad) {
     }
     sb_parts_register(c, 1, c->hidden_norm, (size_t)T * c->d);
     sb_parts_register(c, 1, c->dlogits, (size_t)T * c->V);
+    sb_parts_register(c, 1, c->g_q, (size_t)T * c->qd); sb_parts_register(c, 1, c->g_k, (size_t)T * c->kvd); sb_parts_register(c, 1, c->g_v, (size_t)T * c->kvd);
     sb_parts_register(c, 1, c->g_gate, (size_t)T * c->F); sb_parts_register(c, 1, c->g_up, (size_t)T * c->F);      /* written as parts by the SwiGLU backward */
     return 0;
 }
@@ -802,6 +803,8 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
                          sb_gemm_reads_f16_parts(c, qd, d, T, 1, 0) && sb_gemm_reads_f16_parts(c, kvd, d, T, 1, 0);
     const int xf_parts = !c->nan_on && !(use_lora && (c->lora_mask & 0x30)) &&
                          sb_gemm_reads_f16_parts(c, T, F, d, 0, 1) && sb_gemm_reads_f16_parts(c, F, d, T, 1, 0);
+    /* q and k leave the rotation as the parts that attention reads (the row-wise qk_norm comes after it and keeps the plain pass) */
+    const int rope_parts = !c->qk_norm && sb_attention_reads_parts(c, c->Hq, c->Hkv, c->hd);
     const int hn_parts = !c->nan_on && sb_gemm_reads_f16_parts(c, T, c->V, d, 0, 1) && sb_gemm_reads_f16_parts(c, c->V, d, T, 1, 0);
     nan_mark(c, c->W, (size_t)c->V * d, nan_weight_idx(c));
     prepare_weights(c, T);
@@ -820,6 +823,7 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
         sb_gemm_keep_begin(c);
         float* yq = c->head_norm ? a->q_pre : a->q; float* yk = c->head_norm ? a->k_pre : a->k;
         sb_amax_announce(c, a->v, (size_t)T * kvd);           /* nothing rewrites v before attention splits it */
+        if (rope_parts && !c->head_norm) { sb_amax_announce(c, a->q, (size_t)T * qd); sb_amax_announce(c, a->k, (size_t)T * kvd); }
         if (!(use_lora && (c->lora_mask & 0x07))) {
             const sb_gemm_job_t jobs[3] = {{a->x_norm_attn, c->W + o->q, yq, T, qd, d, 0, 1, 0}, {a->x_norm_attn, c->W + o->k, yk, T, kvd, d, 0, 1, 0},
                                            {a->x_norm_attn, c->W + o->v, a->v, T, kvd, d, 0, 1, 0}};
@@ -835,11 +839,15 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
         sb_gemm_keep_end(c);
         if (c->head_norm) {       /* learned RMSNorm over each head (rows of head_dim), before RoPE */
             const float* wn = c->XW + (size_t)l * 2 * c->hd;
+            if (rope_parts) { sb_amax_announce(c, a->q, (size_t)T * qd); sb_amax_announce(c, a->k, (size_t)T * kvd); }
             sb_rmsnorm(c, a->q_pre, wn, a->q, T * c->Hq, c->hd, RMS_EPS);
             sb_rmsnorm(c, a->k_pre, wn + c->hd, a->k, T * c->Hkv, c->hd, RMS_EPS);
         }
-        if (!c->qk_norm) { sb_amax_announce(c, a->q, (size_t)T * qd); sb_amax_announce(c, a->k, (size_t)T * kvd); }
-        sb_rope2(c, a->q, a->k, c->pos_ids, T, c->Hq, c->Hkv, c->hd, theta, max_seq, 0);
+        if (!(rope_parts && sb_rope_parts(c, a->q, a->k, a->v, c->pos_ids, T, c->Hq, c->Hkv, c->hd, theta, max_seq, 0, 1))) {
+            sb_amax_forget(c, a->q); sb_amax_forget(c, a->k);
+            if (!c->qk_norm) { sb_amax_announce(c, a->q, (size_t)T * qd); sb_amax_announce(c, a->k, (size_t)T * kvd); }
+            sb_rope2(c, a->q, a->k, c->pos_ids, T, c->Hq, c->Hkv, c->hd, theta, max_seq, 0);
+        }
         if (c->qk_norm) {
             /* whole-row normalisation of q and k after RoPE (shaders/qk_norm.comp, src/train.c:4688-4689); the row statistic is kept for the backward pass */
             sb_qk_norm(c, a->q, a->q_rms, T, qd, RMS_EPS);
@@ -914,6 +922,10 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
     nan_mark(c, gh, (size_t)T * d, 5); nan_mark(c, gh, (size_t)T * d, 0);
     const int ffn_lora = !full && (c->lora_mask & 0x70);
     const int ffn_parts_bwd = !c->nan_on && !ffn_lora && sb_gemm_reads_f16_parts(c, T, d, F, 0, 0) && (!full || sb_gemm_reads_f16_parts(c, F, d, T, 1, 0));
+    /* 64-wide heads: the gradients of q, k and v leave the backward rotation as parts only (the attention kernels leave their maxima) */
+    const int rope_parts = !c->nan_on && !c->qk_norm && !c->head_norm && c->hd == 64 && sb_attention_reads_parts(c, c->Hq, c->Hkv, c->hd) &&
+                           sb_gemm_reads_f16_parts(c, T, d, qd, 0, 0) && sb_gemm_reads_f16_parts(c, T, d, kvd, 0, 0) &&
+                           (!full || (sb_gemm_reads_f16_parts(c, qd, d, T, 1, 0) && sb_gemm_reads_f16_parts(c, kvd, d, T, 1, 0)));
     for (int l = L - 1; l >= 0; l--) {
         const sb_layer_off_t* o = &c->off[l];
         sb_layer_act_t* a = &c->act[l];
@@ -959,6 +971,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
         sb_gemm_keep_end(c);
         if (grouped && !c->nan_on && l == 0 && !(c->lora_mask & 7)) goto layer_done;      /* below the first layer's o projection nothing is trained */
         nan_mark(c, c->g_attn, (size_t)T * qd, nan_bwd_base(c) + 5u * (uint32_t)l);
+        if (rope_parts) { sb_amax_announce(c, c->g_q, (size_t)T * qd); sb_amax_announce(c, c->g_k, (size_t)T * kvd); sb_amax_announce(c, c->g_v, (size_t)T * kvd); }
         sb_attention_backward(c, a->q, a->k, a->v, a->attn_out, a->lse, c->g_attn, c->g_q, c->g_k, c->g_v, 0,
                               c->seq_starts, c->seq_ids, B, T, c->Hq, c->Hkv, c->hd);
         if (c->qk_norm) {
@@ -966,8 +979,11 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
             sb_qk_norm_backward(c, a->q, a->q_rms, c->g_q, c->g_q, T, qd, RMS_EPS);
             sb_qk_norm_backward(c, a->k, a->k_rms, c->g_k, c->g_k, T, kvd, RMS_EPS);
         }
-        sb_amax_announce(c, c->g_q, (size_t)T * qd); sb_amax_announce(c, c->g_k, (size_t)T * kvd);
-        sb_rope2(c, c->g_q, c->g_k, c->pos_ids, T, c->Hq, c->Hkv, c->hd, theta, max_seq, 1);
+        if (!(rope_parts && sb_rope_parts(c, c->g_q, c->g_k, c->g_v, c->pos_ids, T, c->Hq, c->Hkv, c->hd, theta, max_seq, 1, !full && !grouped))) {
+            sb_amax_forget(c, c->g_q); sb_amax_forget(c, c->g_k);
+            sb_amax_announce(c, c->g_q, (size_t)T * qd); sb_amax_announce(c, c->g_k, (size_t)T * kvd);
+            sb_rope2(c, c->g_q, c->g_k, c->pos_ids, T, c->Hq, c->Hkv, c->hd, theta, max_seq, 1);
+        }
         if (c->nan_on) {
             const uint32_t nb = nan_bwd_base(c) + 5u * (uint32_t)l;
             nan_mark(c, c->g_q, (size_t)T * qd, nb + 1); nan_mark(c, c->g_k, (size_t)T * kvd, nb + 2); nan_mark(c, c->g_v, (size_t)T * kvd, nb + 3);
