@@ -122,7 +122,10 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_kernel(const float* __r
 // scale comes from a bound formed on the device from the largest magnitudes the inputs' producers left behind,
 //   |silu(g) u| <= max|g| max|u|,   |dup| = |d silu(g)| <= max|d| max|g|,   |dgate| = |d u silu'(g)| <= 1.1 max|d| max|u|
 // (silu' lies in [-0.1, 1.1]).  12 instead of 24 bytes per element forward, 20 instead of 44 backward, counting the split pass
-// that no longer runs.
+// that no longer runs.  A thread takes SW_UNROLL vectors, loaded together, and the blocks cover the array once: with a resident grid striding over
+// it, arrays of two to three strides (2048 tokens x 1408) left a quarter of the last one idle.
+#define SW_UNROLL 2
+static inline dim3 sw_grid(size_t n4) { return dim3((unsigned)((n4 + EW_THREADS * SW_UNROLL - 1) / (EW_THREADS * SW_UNROLL))); }
 __global__ void __launch_bounds__(EW_THREADS) swiglu_parts_kernel(const float4* __restrict__ gate, const float4* __restrict__ up,
                                                                   uint2* __restrict__ h1, uint2* __restrict__ h2, size_t n4,
                                                                   const float* __restrict__ amax_g, const float* __restrict__ amax_u,
@@ -131,8 +134,15 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_parts_kernel(const float4* 
     const float bound = fminf(sb_word(amax_g) * sb_word(amax_u), 3.0e38f);
     const float sc = sb_pow2(sb_f16_shift(bound));
     if (blockIdx.x == 0 && threadIdx.x == 0) *bound_out = bound;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
-        const float4 g = gate[i], u = up[i];
+    float4 gv[SW_UNROLL], uv[SW_UNROLL];
+    const size_t i0 = (size_t)blockIdx.x * (EW_THREADS * SW_UNROLL) + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < SW_UNROLL; k++) if (i0 + k * EW_THREADS < n4) { gv[k] = gate[i0 + k * EW_THREADS]; uv[k] = up[i0 + k * EW_THREADS]; }
+#pragma unroll
+    for (int k = 0; k < SW_UNROLL; k++) {
+        const size_t i = i0 + k * EW_THREADS;
+        if (i >= n4) break;
+        const float4 g = gv[k], u = uv[k];
         const float r0 = ew_apply<OP_SWIGLU>(g.x, u.x) * sc, r1 = ew_apply<OP_SWIGLU>(g.y, u.y) * sc;
         const float r2 = ew_apply<OP_SWIGLU>(g.z, u.z) * sc, r3 = ew_apply<OP_SWIGLU>(g.w, u.w) * sc;
         uint2 a, b;
@@ -152,8 +162,15 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_parts_kernel(const floa
     const float bg = fminf(1.1f * ad * sb_word(amax_u), 3.0e38f), bu = fminf(ad * sb_word(amax_g), 3.0e38f);
     const float sg_ = sb_pow2(sb_f16_shift(bg)), su = sb_pow2(sb_f16_shift(bu));
     if (blockIdx.x == 0 && threadIdx.x == 0) { *bound_dg = bg; *bound_du = bu; }
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
-        const float4 g = gate[i], u = up[i], d = dout[i];
+    float4 gv[SW_UNROLL], uv[SW_UNROLL], dv[SW_UNROLL];
+    const size_t i0 = (size_t)blockIdx.x * (EW_THREADS * SW_UNROLL) + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < SW_UNROLL; k++) if (i0 + k * EW_THREADS < n4) { gv[k] = gate[i0 + k * EW_THREADS]; uv[k] = up[i0 + k * EW_THREADS]; dv[k] = dout[i0 + k * EW_THREADS]; }
+#pragma unroll
+    for (int k = 0; k < SW_UNROLL; k++) {
+        const size_t i = i0 + k * EW_THREADS;
+        if (i >= n4) break;
+        const float4 g = gv[k], u = uv[k], d = dv[k];
         float4 dg, du;
         SWIGLU_BWD_ONE(g.x, u.x, d.x, dg.x, du.x) SWIGLU_BWD_ONE(g.y, u.y, d.y, dg.y, du.y)
         SWIGLU_BWD_ONE(g.z, u.z, d.z, dg.z, du.z) SWIGLU_BWD_ONE(g.w, u.w, d.w, dg.w, du.w)
@@ -262,56 +279,52 @@ __global__ void __launch_bounds__(EW_THREADS) rope_kernel(const float* qin, floa
 // The same rotation with the FP16 operand parts of q, k and v written at once (v passes through unrotated): what would be a rotation pass and
 // a split pass over the three tensors.  A rotated pair is at most sqrt(2) times the larger of its two values, so max |x| of the input, left by
 // the kernel that wrote it, bounds the result and sets the scale.  f32: the rotated q and k are written as FP32 too (in place).
+// One warp per token and tensor (blockIdx.y: q, k, v).  Heads of 64 and 128 (16 and 32 vectors) divide a warp's stride, so a lane's (cos, sin) pair
+// is the same for every vector of the row: one table read, then independent loads.  (Vectors dealt to threads over all three tensors, with a
+// division and a dependent table read each: 12.8 us at 2048 tokens of 3 x 8 x 64.)
+#define ROPE_ROW 4             // vectors of a row in flight per lane
 __global__ void __launch_bounds__(EW_THREADS) rope_parts_kernel(float4* q, float4* k, const float4* __restrict__ v, uint2* __restrict__ hq, uint2* __restrict__ hk,
                                                                 uint2* __restrict__ hv, const uint32_t* __restrict__ pos_ids, const float2* __restrict__ tab,
-                                                                int T, int Hq, int Hkv, int hd, int backward, const float* am_q, const float* am_k, const float* am_v,
+                                                                int T, int Hq, int Hkv, int quads, int backward, const float* am_q, const float* am_k, const float* am_v,
                                                                 float* bound_q, float* bound_k, int f32, unsigned keep) {
     sb_pdl_enter();
-    const float bq = fminf(1.41422f * sb_word(am_q), 3.0e38f), bk = fminf(1.41422f * sb_word(am_k), 3.0e38f);
-    if (blockIdx.x == 0 && threadIdx.x == 0) { *bound_q = bq; *bound_k = bk; }
-    const float sq = sb_pow2(sb_f16_shift(bq)), sk = sb_pow2(sb_f16_shift(bk)), sv = sb_pow2(sb_f16_shift(sb_word(am_v)));
-    const uint32_t quads = (uint32_t)hd >> 2, rq = (uint32_t)Hq * quads, rk = (uint32_t)Hkv * quads, row_quads = rq + rk + (hv ? rk : 0u);
-    const uint32_t total = (uint32_t)T * row_quads, nth = gridDim.x * blockDim.x;
-    const size_t nq4 = (size_t)T * rq, nk4 = (size_t)T * rk;
-    for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; base < total; base += nth * ROPE_UNROLL) {
-        float4 x[ROPE_UNROLL], cs[ROPE_UNROLL];
-        size_t at[ROPE_UNROLL];
-        int which[ROPE_UNROLL];               // 0 q, 1 k, 2 v, 3 nothing
+    const int which = blockIdx.y, lane = threadIdx.x & 31;
+    float bound = sb_word(which == 0 ? am_q : which == 1 ? am_k : am_v);
+    if (which < 2) {
+        bound = fminf(1.41422f * bound, 3.0e38f);
+        if (blockIdx.x == 0 && threadIdx.x == 0) *(which == 0 ? bound_q : bound_k) = bound;
+    }
+    const float sc = sb_pow2(sb_f16_shift(bound));
+    const int t = blockIdx.x * (EW_THREADS / 32) + (threadIdx.x >> 5), row = (which == 0 ? Hq : Hkv) * quads;
+    if (t >= T) return;
+    uint2* h = which == 0 ? hq : which == 1 ? hk : hv;
+    const size_t at = (size_t)t * row, n4 = (size_t)T * row;
+    float4* io = which == 0 ? q + at : k + at;
+    const float4* in = which == 2 ? v + at : io;
+    const float4 cs = which < 2 ? __ldg((const float4*)tab + (size_t)__ldg(pos_ids + t) * quads + (lane & (quads - 1))) : make_float4(1.f, 0.f, 1.f, 0.f);
+    for (int i0 = lane; i0 < row; i0 += 32 * ROPE_ROW) {
+        float4 x[ROPE_ROW];
 #pragma unroll
-        for (int u = 0; u < ROPE_UNROLL; u++) {
-            const uint32_t i = base + u * nth;
-            which[u] = 3;
-            if (i < total) {
-                const uint32_t t = i / row_quads, rem = i - t * row_quads;
-                which[u] = rem < rq ? 0 : rem < rq + rk ? 1 : 2;
-                const uint32_t w = which[u] == 0 ? rem : which[u] == 1 ? rem - rq : rem - rq - rk;
-                at[u] = (size_t)t * (which[u] == 0 ? rq : rk) + w;
-                x[u] = which[u] == 0 ? q[at[u]] : which[u] == 1 ? k[at[u]] : v[at[u]];
-                if (which[u] < 2) cs[u] = ((const float4*)tab)[(size_t)pos_ids[t] * quads + w % quads];
-            }
-        }
+        for (int u = 0; u < ROPE_ROW; u++) if (i0 + 32 * u < row) x[u] = in[i0 + 32 * u];
 #pragma unroll
-        for (int u = 0; u < ROPE_UNROLL; u++) {
-            if (which[u] == 3) continue;
+        for (int u = 0; u < ROPE_ROW; u++) {
+            const int i = i0 + 32 * u;
+            if (i >= row) break;
             float4 r = x[u];
-            float sc = sv;
-            uint2* h = hv; size_t n4 = nk4;
-            if (which[u] < 2) {
+            if (which < 2) {
                 if (!backward) {
-                    r.x = x[u].x * cs[u].x - x[u].y * cs[u].y; r.y = x[u].x * cs[u].y + x[u].y * cs[u].x;
-                    r.z = x[u].z * cs[u].z - x[u].w * cs[u].w; r.w = x[u].z * cs[u].w + x[u].w * cs[u].z;
+                    r.x = x[u].x * cs.x - x[u].y * cs.y; r.y = x[u].x * cs.y + x[u].y * cs.x;
+                    r.z = x[u].z * cs.z - x[u].w * cs.w; r.w = x[u].z * cs.w + x[u].w * cs.z;
                 } else {
-                    r.x = x[u].x * cs[u].x + x[u].y * cs[u].y; r.y = -x[u].x * cs[u].y + x[u].y * cs[u].x;
-                    r.z = x[u].z * cs[u].z + x[u].w * cs[u].w; r.w = -x[u].z * cs[u].w + x[u].w * cs[u].z;
+                    r.x = x[u].x * cs.x + x[u].y * cs.y; r.y = -x[u].x * cs.y + x[u].y * cs.x;
+                    r.z = x[u].z * cs.z + x[u].w * cs.w; r.w = -x[u].z * cs.w + x[u].w * cs.z;
                 }
-                const bool isq = which[u] == 0;
-                if (f32) { if (isq) q[at[u]] = r; else k[at[u]] = r; }
-                sc = isq ? sq : sk; h = isq ? hq : hk; if (isq) n4 = nq4;
+                if (f32) io[i] = r;
             }
             if (h) {
                 uint2 a, b;
                 sb_split2(r.x * sc, r.y * sc, a.x, b.x, keep); sb_split2(r.z * sc, r.w * sc, a.y, b.y, keep);
-                h[at[u]] = a; h[n4 + at[u]] = b;
+                h[at + i] = a; h[n4 + at + i] = b;
             }
         }
     }
@@ -416,7 +429,7 @@ int sb_swiglu_parts(sb_ctx_t* c, const float* gate, const float* up, float* out,
     if (!sb_parts_find(c, out, n, &h, &bound, &fresh)) return 0;
     sb_amax_forget(c, out);
     int tk = sb_tick_begin(c, SB_CLS_SWIGLU);
-    sb_launch(swiglu_parts_kernel, dim3(ew_grid(c, n / 4)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (const float4*)gate, (const float4*)up, (uint2*)h,
+    sb_launch(swiglu_parts_kernel, sw_grid(n / 4), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (const float4*)gate, (const float4*)up, (uint2*)h,
                                                                                          (uint2*)((uint16_t*)h + n), n / 4, ag, au, bound, sb_parts_keep(c));
     sb_tick_end(c, tk, 0.0, 12.0 * (double)n);
     c->launches++;
@@ -430,7 +443,7 @@ int sb_swiglu_backward_parts(sb_ctx_t* c, const float* gate, const float* up, co
     if (!sb_parts_find(c, dgate, n, &hg, &bg, &fresh) || !sb_parts_find(c, dup, n, &hu, &bu, &fresh)) return 0;
     sb_amax_forget(c, dgate); sb_amax_forget(c, dup);
     int tk = sb_tick_begin(c, SB_CLS_SWIGLU);
-    sb_launch(swiglu_bwd_parts_kernel, dim3(ew_grid(c, n / 4)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (const float4*)gate, (const float4*)up, (const float4*)dout, (uint2*)hg, (uint2*)((uint16_t*)hg + n), (uint2*)hu, (uint2*)((uint16_t*)hu + n),
+    sb_launch(swiglu_bwd_parts_kernel, sw_grid(n / 4), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (const float4*)gate, (const float4*)up, (const float4*)dout, (uint2*)hg, (uint2*)((uint16_t*)hg + n), (uint2*)hu, (uint2*)((uint16_t*)hu + n),
         n / 4, ag, au, ad, bg, bu, sb_parts_keep(c));
     sb_tick_end(c, tk, 0.0, 20.0 * (double)n);
     c->launches++;
@@ -491,8 +504,7 @@ void sb_rope(sb_ctx_t* c, const float* in, float* out, const uint32_t* pos_ids, 
 // q and k rotated in place and, with v, handed on as parts; 0: not done (the maxima of all three have to be known).  Without an arena for the
 // parts the words of q and k still get the same bounds, so that whoever splits them gets the same parts.
 int sb_rope_parts(sb_ctx_t* c, float* q, float* k, const float* v, const uint32_t* pos_ids, int T, int Hq, int Hkv, int hd, float theta, int max_pos, int backward, int f32) {
-    const double nq = (double)T * (Hq + 2 * Hkv) * (hd / 4);
-    if (T <= 0 || (hd & 7) || !aligned16(q) || !aligned16(k) || !aligned16(v) || nq >= 2147483648.0) return 0;
+    if (T <= 0 || (hd != 64 && hd != 128) || !aligned16(q) || !aligned16(k) || !aligned16(v)) return 0;
     const size_t n_q = (size_t)T * Hq * hd, n_k = (size_t)T * Hkv * hd;
     const float* aq = sb_amax_lookup(c, q, n_q); const float* ak = sb_amax_lookup(c, k, n_k); float* av = sb_amax_lookup(c, v, n_k);
     if (!aq || !ak || !av || !rope_ensure_table(c, hd, theta, max_pos)) return 0;
@@ -504,9 +516,8 @@ int sb_rope_parts(sb_ctx_t* c, float* q, float* k, const float* v, const uint32_
     if (sb_parts_find(c, k, n_k, &hk, &own, &fresh)) sb_parts_set_amax(c, k, wk); else { hk = NULL; f32 = 1; }
     if (sb_parts_find(c, v, n_k, &hv, &own, &fresh)) sb_parts_set_amax(c, v, av); else hv = NULL;
     int tk = sb_tick_begin(c, SB_CLS_ROPE);
-    const size_t work = ((size_t)nq + ROPE_UNROLL - 1) / ROPE_UNROLL;
-    sb_launch(rope_parts_kernel, dim3(ew_grid(c, work)), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (float4*)q, (float4*)k, (const float4*)v, (uint2*)hq, (uint2*)hk,
-              (uint2*)hv, pos_ids, (const float2*)c->rope_tab, T, Hq, Hkv, hd, backward, aq, ak, (const float*)av, wq, wk, f32, sb_parts_keep(c));
+    sb_launch(rope_parts_kernel, dim3((unsigned)((T + EW_THREADS / 32 - 1) / (EW_THREADS / 32)), hv ? 3 : 2), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (float4*)q, (float4*)k,
+              (const float4*)v, (uint2*)hq, (uint2*)hk, (uint2*)hv, pos_ids, (const float2*)c->rope_tab, T, Hq, Hkv, hd / 4, backward, aq, ak, (const float*)av, wq, wk, f32, sb_parts_keep(c));
     sb_tick_end(c, tk, 0.0, (f32 ? 12.0 : 8.0) * T * (Hq + Hkv) * hd + 8.0 * T * Hkv * hd);
     c->launches++;
     return 1;
