@@ -122,7 +122,6 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
                   const float* __restrict__ amax_do, const float* __restrict__ ds_bound,
                   const AfSeqTab seqs, int Sp, int Hq, int g, int nkb, int chunk, int accumulate, int slot_pitch, float scale, int* status,
                   unsigned* amax_dk, unsigned* amax_dv) {
-    sb_pdl_enter();
     constexpr int NH = HD / 64;
     constexpr int KV_PART = NH * 16384, ST_PART = NH * 4096;
     constexpr int COL_DK = 0, COL_DV = HD, COL_K = 2 * HD, COL_S0 = 3 * HD, COL_V = COL_S0 + 128;
@@ -146,13 +145,15 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
     const int kb = kb_lo + cr / in_chunk;
     const int rem = ci * chunk + cr % in_chunk;
     const int b = rem / Hkv, kvh = rem % Hkv;
-    const int t0 = (int)seqs.start[b], S = (int)seqs.start[b + 1] - t0;
     const int k0 = kb * AB_BK;
-    if (kb >= nkb || k0 >= S) return;
-    if (*(volatile int*)status != 0) return;
-    const int nq = (S + AB_BQ - 1) / AB_BQ, j0 = k0 / AB_BQ, per_head = nq - j0;
-    const int nsteps = g * per_head;
-    const int nchains = (nsteps + DRAIN - 1) / DRAIN;
+    int t0, S;
+    auto take = [&]() -> bool {                        // false: no keys for this CTA
+        sb_pdl_enter();
+        t0 = (int)seqs.start[b]; S = (int)seqs.start[b + 1] - t0;
+        return kb < nkb && k0 < S && *(volatile int*)status == 0;
+    };
+    const bool first = gridDim.x > AF_ONE_WAVE;
+    if (first && !take()) return;
     const int kvd = Hkv * HD;
 
     extern __shared__ uint8_t af_raw[];
@@ -185,7 +186,14 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if (!first && !take()) {
+        if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512));
+        return;
+    }
     bool ok = true;
+    const int nq = (S + AB_BQ - 1) / AB_BQ, j0 = k0 / AB_BQ, per_head = nq - j0;
+    const int nsteps = g * per_head;
+    const int nchains = (nsteps + DRAIN - 1) / DRAIN;
 
     if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(AB_REGS_LIGHT));
@@ -598,16 +606,20 @@ at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant_
                  const __grid_constant__ CUtensorMap mK1, const __grid_constant__ CUtensorMap mK2,
                  const AfSeqTab seqs, float* __restrict__ dQ, const float* __restrict__ ds_bound, const float* __restrict__ amax_k,
                  int Sp, int Hq, int g, int nqb_max, int* status, unsigned* amax_dq) {
-    sb_pdl_enter();
     constexpr int NH = HD / 64, OC = HD / 2;
     const int per_i = seqs.n * Hq;
     const int qb = nqb_max - 1 - (int)blockIdx.x / per_i;
     const int rem = (int)blockIdx.x % per_i;
     const int b = rem / Hq, h = rem % Hq;
-    const int t0 = (int)seqs.start[b], S = (int)seqs.start[b + 1] - t0;
-    if (qb * 128 >= S) return;
-    if (*(volatile int*)status != 0) return;
-    const int nkv = min((S + 63) / 64, 2 * qb + 2);
+    int t0, S, nkv;
+    auto take = [&]() -> bool {                         // false: no rows for this CTA
+        sb_pdl_enter();
+        t0 = (int)seqs.start[b]; S = (int)seqs.start[b + 1] - t0;
+        nkv = min((S + 63) / 64, 2 * qb + 2);
+        return qb * 128 < S && *(volatile int*)status == 0;
+    };
+    const bool first = gridDim.x > AF_ONE_WAVE;
+    if (first && !take()) return;
 
     extern __shared__ uint8_t af_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)af_raw + 1023) & ~(uintptr_t)1023);
@@ -630,6 +642,10 @@ at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if (!first && !take()) {
+        if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * HD));
+        return;
+    }
     bool ok = true;
     if (warp == 0) {
         // ---------------- TMA producer ----------------

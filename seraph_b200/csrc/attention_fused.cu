@@ -31,8 +31,6 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
                     const AfSeqTab seqs, float* __restrict__ O, float* __restrict__ lse,
                     const float* __restrict__ amax_q, const float* __restrict__ amax_k, const float* __restrict__ amax_v,
                     int Hq, int g, int nqb_max, float scale, int* status, float* bound_o, uint4* __restrict__ Oh, size_t n_o, unsigned keep) {
-    sb_pdl_enter();
-    if (bound_o && blockIdx.x == 0 && threadIdx.x == 0) *bound_o = sb_word(amax_v);
     constexpr int NH = HD / 64;                              // 64-column halves of the head dimension (one 128-byte row of halfs each)
     constexpr int Q_BYTES = NH * 32768, KV_STAGE = NH * 16384, Q_PART = NH * 16384, KV_PART = NH * 8192;
     constexpr int OFF_K = Q_BYTES, OFF_V = OFF_K + 2 * KV_STAGE, OFF_P = OFF_V + 2 * KV_STAGE, OFF_BAR = OFF_P + 32768;
@@ -44,10 +42,16 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
     const int qb = nqb_max - 1 - (int)blockIdx.x / per_i;
     const int rem = (int)blockIdx.x % per_i;
     const int b = rem / Hq, h = rem % Hq;
-    const int t0 = (int)seqs.start[b], S = (int)seqs.start[b + 1] - t0;
-    if (qb * AF_BQ >= S) return;
-    if (*(volatile int*)status != 0) return;                 // an earlier CTA gave up: do not queue behind its cause
-    const int nkv = min((S + AF_BKV - 1) / AF_BKV, 2 * qb + 2);
+    int t0, S, nkv;
+    auto take = [&]() -> bool {                              // false: no rows for this CTA
+        sb_pdl_enter();
+        if (bound_o && blockIdx.x == 0 && threadIdx.x == 0) *bound_o = sb_word(amax_v);
+        t0 = (int)seqs.start[b]; S = (int)seqs.start[b + 1] - t0;
+        nkv = min((S + AF_BKV - 1) / AF_BKV, 2 * qb + 2);
+        return qb * AF_BQ < S && *(volatile int*)status == 0;      // an earlier CTA gave up: do not queue behind its cause
+    };
+    const bool first = gridDim.x > AF_ONE_WAVE;
+    if (first && !take()) return;
     const int kvh = h / g;
     const int qd = Hq * HD;
 
@@ -90,6 +94,10 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if (!first && !take()) {
+        if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
+        return;
+    }
     bool ok = true;
 
     if (warp == 0) {

@@ -7,6 +7,9 @@
 #define AF_BQ 128
 #define AF_BKV 64
 #define AF_HD 128
+// Launches of one wave set up their barriers and tensor memory while the kernel before them drains, and only then wait for it (1 us of a launch of
+// ten); with more CTAs than SMs the setup overlaps other CTAs' work anyway, and CTAs without rows should leave at once.
+#define AF_ONE_WAVE 160
 #define AF_THREADS 512
 #define AF_MAXSEQ 240
 
