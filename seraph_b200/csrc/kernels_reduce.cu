@@ -9,6 +9,7 @@
 #include <cuda_fp16.h>
 #include <math.h>
 #include <stdio.h>
+#include <string.h>
 #include <stdint.h>
 #include "sb_internal.h"
 
@@ -567,36 +568,210 @@ __global__ void __launch_bounds__(RB_THREADS) qk_norm_row_kernel(float* __restri
 }
 
 // ---------------------------------------------------------------------------
-// Cross-entropy loss and gradient, packed.  One CTA per row: an online
-// (max,sum) pass over the logits, then one pass that writes the gradient:
-// 12 bytes per logit where the reference's three passes move 20.
+// Cross-entropy loss and gradient, packed.
 //   last token of a sequence -> zero row and zero loss
 //   loss = -(logit[target] - max - log(sum));  grad = (softmax - onehot)/num_valid
+// A cluster of CL CTAs holds one row of logits in shared memory, a slice of V / CL each: every logit is read once and exponentiated once, and
+// the maximum and the sum of the row are exchanged through distributed shared memory.  8 bytes per logit (4 when no gradient is asked for).
+// (An online maximum and sum, then a second read for the gradient: 12 bytes and two or more exponentials per logit.)
+// The gradient leaves as FP32 (`grad`), or as the two FP16 parts the LM-head backward products read (g1: h1 = fp16(g * part_scale),
+// h2 = fp16(g * part_scale - h1), laid out like grad): |g| <= inv_valid everywhere (softmax minus one-hot, over the number of predictions),
+// so the parts' scale is known before a single logit is read, *part_amax = inv_valid; or, both NULL, not at all.
 // ---------------------------------------------------------------------------
 #define CE_THREADS 512
-__global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(const float* __restrict__ logits, const uint32_t* __restrict__ targets,
+struct CeArgs {
+    const float* logits; const uint32_t* targets; float *grad, *loss_rows;
+    const uint32_t *pos_ids, *seq_ids, *seq_starts;
+    int T, V; float inv_valid; int* status; unsigned* amax_grad;
+    __half *g1, *g2; float part_scale; float* part_amax; unsigned keep;
+};
+// the CTAs of a cluster combine one value each: v of rank i lands in slot[i] of every CTA
+template <int CL>
+__device__ __forceinline__ void ce_exchange(float* slot, float v) {
+    if (CL == 1) { if (threadIdx.x == 0) slot[0] = v; __syncthreads(); return; }
+    if (threadIdx.x < CL) {
+        uint32_t rank, a;
+        asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(slot + rank)), "r"((uint32_t)threadIdx.x));
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <int CL>
+__global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(const __grid_constant__ CeArgs p) {
+    sb_pdl_enter();
+    extern __shared__ float4 row[];
+    __shared__ float red[CE_THREADS / 32], smax[CL], ssum[CL];
+    const int r = blockIdx.x / CL, rank = blockIdx.x % CL, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n4 = p.V / 4, per = (n4 + CL - 1) / CL, lo = min(n4, rank * per), n = min(n4, lo + per) - lo;
+    const float4* lr = (const float4*)(p.logits + (size_t)r * p.V) + lo;
+    const size_t out = (size_t)r * n4 + lo;
+    float4* gr = p.grad ? (float4*)p.grad + out : nullptr;
+    uint2* p1 = p.g1 ? (uint2*)p.g1 + out : nullptr; uint2* p2 = p.g1 ? (uint2*)p.g2 + out : nullptr;
+    if (p.g1 && blockIdx.x == 0 && threadIdx.x == 0) *p.part_amax = p.inv_valid;
+    const uint32_t s = p.seq_ids[r];
+    if ((int)p.pos_ids[r] >= (int)(p.seq_starts[s + 1] - p.seq_starts[s]) - 1) {
+        for (int i = threadIdx.x; i < n; i += CE_THREADS) {
+            if (p1) { p1[i] = make_uint2(0u, 0u); p2[i] = make_uint2(0u, 0u); }
+            else if (gr) gr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (rank == 0 && threadIdx.x == 0) p.loss_rows[r] = 0.f;
+        return;
+    }
+    uint32_t tg = p.targets[r];
+    if (tg >= (uint32_t)p.V) { if (threadIdx.x == 0) atomicExch(p.status, SB_ERR_TOKEN_RANGE); tg = 0; }
+    const float lt = p.logits[(size_t)r * p.V + tg];        // (grad may be the same array as logits)
+    if (CL > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    float m = -INFINITY;
+    for (int i0 = threadIdx.x; i0 < n; i0 += 4 * CE_THREADS) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) if (i0 + u * CE_THREADS < n) v[u] = __ldcs(lr + i0 + u * CE_THREADS);
+#pragma unroll
+        for (int u = 0; u < 4; u++) if (i0 + u * CE_THREADS < n) {
+            row[i0 + u * CE_THREADS] = v[u];
+            m = fmaxf(m, fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)));
+        }
+    }
+    m = warp_max(m);
+    if (lane == 0) red[warp] = m;
+    __syncthreads();
+    m = warp_max(red[lane & (CE_THREADS / 32 - 1)]);
+    if (CL > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");      // every CTA of the cluster is running: its shared memory may be written
+    ce_exchange<CL>(smax, m);
+    m = smax[0];
+#pragma unroll
+    for (int i = 1; i < CL; i++) m = fmaxf(m, smax[i]);
+    float sum = 0.f;
+    for (int i = threadIdx.x; i < n; i += CE_THREADS) {     // a thread reads back what it stored itself
+        float4 v = row[i];
+        v.x = expf(v.x - m); v.y = expf(v.y - m); v.z = expf(v.z - m); v.w = expf(v.w - m);
+        row[i] = v;
+        sum += (v.x + v.y) + (v.z + v.w);
+    }
+    sum = warp_sum(sum);
+    __syncthreads();                                        // red has been read
+    if (lane == 0) red[warp] = sum;
+    __syncthreads();
+    sum = red[0];
+#pragma unroll
+    for (int i = 1; i < CE_THREADS / 32; i++) sum += red[i];
+    ce_exchange<CL>(ssum, sum);
+    sum = ssum[0];
+#pragma unroll
+    for (int i = 1; i < CL; i++) sum += ssum[i];
+    if (rank == 0 && threadIdx.x == 0) p.loss_rows[r] = -((lt - m) - logf(sum));
+    if (!p1 && !gr) return;
+    const float inv = 1.0f / sum;
+    float am = 0.f;
+    for (int i = threadIdx.x; i < n; i += CE_THREADS) {
+        float4 g = row[i];
+        g.x *= inv; g.y *= inv; g.z *= inv; g.w *= inv;
+        const uint32_t b = (uint32_t)(lo + i) * 4;
+        if (tg - b < 4u) { if (tg == b) g.x -= 1.f; else if (tg == b + 1) g.y -= 1.f; else if (tg == b + 2) g.z -= 1.f; else g.w -= 1.f; }
+        g.x *= p.inv_valid; g.y *= p.inv_valid; g.z *= p.inv_valid; g.w *= p.inv_valid;
+        if (p1) {
+            uint2 h, l;
+            sb_split2(g.x * p.part_scale, g.y * p.part_scale, h.x, l.x, p.keep); sb_split2(g.z * p.part_scale, g.w * p.part_scale, h.y, l.y, p.keep);
+            p1[i] = h; p2[i] = l;
+        } else {
+            gr[i] = g;
+            am = sb_amax4(am, g);
+        }
+    }
+    sb_block_amax(am, p.amax_grad);
+}
+
+// Rows too long for that (a vocabulary of 152k is 608 KB a row): one CTA of 1024 threads per row and SM, an online (max, sum) pass in batches of 16
+// logits (one comparison and at most one rescaling each), then the gradient pass from the end of the row backwards, which finds what the rows in
+// flight (148 x 608 KB) still have in L2.  (Clusters of 8 and 16 CTAs with slices in shared memory read each logit once, but their phases and
+// the cluster's launch leave memory idle: 3.3 and 4.1 ms at 8192 x 151936, against 2.85 here and 2.96 for an
+// online pass of 512 threads that compared every logit.)
+#define CE_LONG 1024
+__global__ void __launch_bounds__(CE_LONG, 1) cross_entropy_long_kernel(const __grid_constant__ CeArgs p) {
+    sb_pdl_enter();
+    __shared__ float redm[32], reds[32];
+    const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = p.V / 4;
+    const float4* lr = (const float4*)(p.logits + (size_t)r * p.V);
+    const size_t out = (size_t)r * n;
+    float4* gr = p.grad ? (float4*)p.grad + out : nullptr;
+    uint2* p1 = p.g1 ? (uint2*)p.g1 + out : nullptr; uint2* p2 = p.g1 ? (uint2*)p.g2 + out : nullptr;
+    if (p.g1 && r == 0 && threadIdx.x == 0) *p.part_amax = p.inv_valid;
+    const uint32_t s = p.seq_ids[r];
+    if ((int)p.pos_ids[r] >= (int)(p.seq_starts[s + 1] - p.seq_starts[s]) - 1) {
+        for (int i = threadIdx.x; i < n; i += CE_LONG) {
+            if (p1) { p1[i] = make_uint2(0u, 0u); p2[i] = make_uint2(0u, 0u); }
+            else if (gr) gr[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (threadIdx.x == 0) p.loss_rows[r] = 0.f;
+        return;
+    }
+    uint32_t tg = p.targets[r];
+    if (tg >= (uint32_t)p.V) { if (threadIdx.x == 0) atomicExch(p.status, SB_ERR_TOKEN_RANGE); tg = 0; }
+    const float lt = p.logits[(size_t)r * p.V + tg];
+    float m = -INFINITY, sum = 0.f;
+    for (int i0 = threadIdx.x; i0 < n; i0 += 4 * CE_LONG) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = i0 + u * CE_LONG < n ? lr[i0 + u * CE_LONG] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        float bm = -INFINITY;
+#pragma unroll
+        for (int u = 0; u < 4; u++) bm = fmaxf(bm, fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)));
+        if (bm > m) { sum = m == -INFINITY ? sum : sum * expf(m - bm); m = bm; }
+#pragma unroll
+        for (int u = 0; u < 4; u++) if (i0 + u * CE_LONG < n) sum += (expf(v[u].x - m) + expf(v[u].y - m)) + (expf(v[u].z - m) + expf(v[u].w - m));
+    }
+    float wm = warp_max(m);
+    sum = warp_sum(m == -INFINITY ? sum : sum * expf(m - wm));
+    if (lane == 0) { redm[warp] = wm; reds[warp] = sum; }
+    __syncthreads();
+    m = warp_max(redm[lane]);
+    sum = warp_sum(redm[lane] == -INFINITY ? reds[lane] : reds[lane] * expf(redm[lane] - m));
+    if (threadIdx.x == 0) p.loss_rows[r] = -((lt - m) - logf(sum));
+    if (!p1 && !gr) return;
+    const float inv = 1.0f / sum;
+    float am = 0.f;
+    auto grad_of = [&](int i, float4 g) {
+        g.x = expf(g.x - m) * inv; g.y = expf(g.y - m) * inv; g.z = expf(g.z - m) * inv; g.w = expf(g.w - m) * inv;
+        const uint32_t b = (uint32_t)i * 4;
+        if (tg - b < 4u) { if (tg == b) g.x -= 1.f; else if (tg == b + 1) g.y -= 1.f; else if (tg == b + 2) g.z -= 1.f; else g.w -= 1.f; }
+        g.x *= p.inv_valid; g.y *= p.inv_valid; g.z *= p.inv_valid; g.w *= p.inv_valid;
+        if (p1) {
+            uint2 h, l;
+            sb_split2(g.x * p.part_scale, g.y * p.part_scale, h.x, l.x, p.keep); sb_split2(g.z * p.part_scale, g.w * p.part_scale, h.y, l.y, p.keep);
+            __stcs(p1 + i, h); __stcs(p2 + i, l);
+        } else {
+            gr[i] = g;
+            am = sb_amax4(am, g);
+        }
+    };
+    for (int j0 = threadIdx.x; j0 < n; j0 += 4 * CE_LONG) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) if (j0 + u * CE_LONG < n) v[u] = __ldcs(lr + (n - 1 - j0 - u * CE_LONG));
+#pragma unroll
+        for (int u = 0; u < 4; u++) if (j0 + u * CE_LONG < n) grad_of(n - 1 - j0 - u * CE_LONG, v[u]);
+    }
+    sb_block_amax(am, p.amax_grad);
+}
+
+// rows that are not a multiple of four logits or not aligned: one CTA per row, an online (max, sum) pass over the
+// logits, then one pass that writes the gradient
+__global__ void __launch_bounds__(CE_THREADS) cross_entropy_any_kernel(const float* __restrict__ logits, const uint32_t* __restrict__ targets,
                                                                    float* __restrict__ grad, float* __restrict__ loss_rows,
                                                                    const uint32_t* __restrict__ pos_ids, const uint32_t* __restrict__ seq_ids,
                                                                    const uint32_t* __restrict__ seq_starts,
-                                                                   int T, int V, float inv_valid, int vec, int* status, unsigned* amax_grad,
-                                                                   __half* __restrict__ g1, __half* __restrict__ g2, float part_scale, float* part_amax, unsigned keep) {
+                                                                   int T, int V, float inv_valid, int* status, unsigned* amax_grad) {
     sb_pdl_enter();
-    // g1 != NULL (vec only): the gradient leaves as the two FP16 parts the LM-head backward products read, h1 = fp16(g * part_scale),
-    // h2 = fp16(g * part_scale - h1), laid out like grad; nothing is written to grad.  |g| <= inv_valid everywhere (softmax minus
-    // one-hot, over the number of predictions), so the parts' scale is known before a single logit is read: *part_amax = inv_valid.
     __shared__ float redm[32], reds[32];
     float am = 0.f;
     int r = blockIdx.x;
     if (r >= T) return;
-    if (g1 && r == 0 && threadIdx.x == 0) *part_amax = inv_valid;
     const float* lr = logits + (size_t)r * V; float* gr = grad + (size_t)r * V;
-    uint2* p1 = g1 ? (uint2*)(g1 + (size_t)r * V) : NULL; uint2* p2 = g1 ? (uint2*)(g2 + (size_t)r * V) : NULL;
     uint32_t s = seq_ids[r];
     int seq_len = (int)(seq_starts[s + 1] - seq_starts[s]);
     if ((int)pos_ids[r] >= seq_len - 1) {
-        if (g1) for (int i = threadIdx.x; i < V / 4; i += blockDim.x) { p1[i] = make_uint2(0u, 0u); p2[i] = make_uint2(0u, 0u); }
-        else if (vec) for (int i = threadIdx.x; i < V / 4; i += blockDim.x) ((float4*)gr)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        else     for (int i = threadIdx.x; i < V; i += blockDim.x) gr[i] = 0.f;
+        if (grad) for (int i = threadIdx.x; i < V; i += blockDim.x) gr[i] = 0.f;
         if (threadIdx.x == 0) loss_rows[r] = 0.f;
         return;
     }
@@ -604,8 +779,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(const float* 
     if (tg >= (uint32_t)V) { if (threadIdx.x == 0) atomicExch(status, SB_ERR_TOKEN_RANGE); tg = 0; }
     float m = -INFINITY, sum = 0.f;
 #define CE_ONLINE(v) { float nv = (v); if (nv > m) { sum = sum * expf(m - nv) + 1.0f; m = nv; } else sum += expf(nv - m); }
-    if (vec) for (int i = threadIdx.x; i < V / 4; i += blockDim.x) { float4 v = ((const float4*)lr)[i]; CE_ONLINE(v.x) CE_ONLINE(v.y) CE_ONLINE(v.z) CE_ONLINE(v.w) }
-    else     for (int i = threadIdx.x; i < V; i += blockDim.x) CE_ONLINE(lr[i])
+    for (int i = threadIdx.x; i < V; i += blockDim.x) CE_ONLINE(lr[i])
     // combine (m,sum) pairs: warp, then block
     for (int o = 16; o > 0; o >>= 1) {
         float om = __shfl_xor_sync(0xffffffffu, m, o), os = __shfl_xor_sync(0xffffffffu, sum, o);
@@ -623,22 +797,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(const float* 
     }
     float inv = 1.0f / sum;
     if (threadIdx.x == 0) loss_rows[r] = -((lr[tg] - m) - logf(sum));
-    if (vec) for (int i = threadIdx.x; i < V / 4; i += blockDim.x) {
-        float4 v = ((const float4*)lr)[i], g;
-        g.x = expf(v.x - m) * inv; g.y = expf(v.y - m) * inv; g.z = expf(v.z - m) * inv; g.w = expf(v.w - m) * inv;
-        uint32_t b = (uint32_t)i * 4;
-        if (tg - b < 4u) { if (tg == b) g.x -= 1.f; else if (tg == b + 1) g.y -= 1.f; else if (tg == b + 2) g.z -= 1.f; else g.w -= 1.f; }
-        g.x *= inv_valid; g.y *= inv_valid; g.z *= inv_valid; g.w *= inv_valid;
-        if (g1) {
-            const float q0 = g.x * part_scale, q1 = g.y * part_scale, q2 = g.z * part_scale, q3 = g.w * part_scale;
-            uint2 h, l;
-            sb_split2(q0, q1, h.x, l.x, keep); sb_split2(q2, q3, h.y, l.y, keep);
-            p1[i] = h; p2[i] = l;
-        } else {
-            ((float4*)gr)[i] = g;
-            am = sb_amax4(am, g);
-        }
-    } else for (int i = threadIdx.x; i < V; i += blockDim.x) {
+    if (grad) for (int i = threadIdx.x; i < V; i += blockDim.x) {
         float g = expf(lr[i] - m) * inv;
         if ((uint32_t)i == tg) g -= 1.f;
         gr[i] = g * inv_valid;
@@ -728,7 +887,7 @@ __global__ void __launch_bounds__(EB_CHUNK) eb_place_kernel(const uint32_t* __re
                                                             const int* __restrict__ chunk_cnt, const int* __restrict__ start,
                                                             int* __restrict__ sorted_pos) {
     sb_pdl_enter();
-    __shared__ uint32_t s_tok[EB_CHUNK];
+    __shared__ __align__(16) uint32_t s_tok[EB_CHUNK];
     int t = blockIdx.x * EB_CHUNK + threadIdx.x;
     uint32_t id = t < T ? tok[t] : 0xffffffffu;
     s_tok[threadIdx.x] = id;
@@ -736,7 +895,10 @@ __global__ void __launch_bounds__(EB_CHUNK) eb_place_kernel(const uint32_t* __re
     if (t >= T || id >= (uint32_t)V) return;
     int rank = 0;
     for (int cb = 0; cb < (int)blockIdx.x; cb++) rank += chunk_cnt[(size_t)cb * V + id];   // earlier chunks
-    for (int j = 0; j < (int)threadIdx.x; j++) rank += (s_tok[j] == id);                   // earlier in this chunk
+    // earlier in this chunk: four tokens per read (one per read was most of the kernel's 16 us at 2048 tokens)
+    const int j4 = (int)threadIdx.x >> 2;
+    for (int j = 0; j < j4; j++) { const uint4 k = ((const uint4*)s_tok)[j]; rank += (k.x == id) + (k.y == id) + (k.z == id) + (k.w == id); }
+    for (int j = j4 * 4; j < (int)threadIdx.x; j++) rank += (s_tok[j] == id);
     sorted_pos[start[id] + rank] = t;
 }
 
@@ -1010,16 +1172,61 @@ void sb_qk_norm_backward(sb_ctx_t* c, const float* y, const float* rms, const fl
     c->launches++;
 }
 
+#define CE_MAX_SLICE (64 * 1024)      // bytes of a row in one CTA's shared memory
+// CTAs per row: slices of at most 64 KB, so that three or more CTAs share an SM, in clusters of one or two (four at 32 KB each: 0.63 instead of
+// 0.50 ms at 8192 x 32768); up to eight only when there are too few rows to fill the device.  0: the row is too long.
+static int ce_cluster(sb_ctx_t* c, int T, int V) {
+    int cl = 1;
+    if ((size_t)V * 4 > 64 * 1024) cl = 2;
+    while (cl < 8 && (long)T * cl <= (long)sm_count(c)) cl *= 2;
+    return (size_t)((V / 4 + cl - 1) / cl) * 16 <= CE_MAX_SLICE ? cl : 0;
+}
+extern "C++" {
+template <int CL>
+static bool ce_launch(sb_ctx_t* c, const CeArgs& a) {
+    const size_t smem = (size_t)((a.V / 4 + CL - 1) / CL) * 16;
+    static bool attr = false;
+    if (!attr) {
+        if (cudaFuncSetAttribute(cross_entropy_kernel<CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, CE_MAX_SLICE) != cudaSuccess) { cudaGetLastError(); return false; }
+        attr = true;
+    }
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDim = dim3((unsigned)a.T * CL); cfg.blockDim = dim3(CE_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = (cudaStream_t)c->pub.stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = CL; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = CL > 1 ? 2 : 1;
+    c->launches++;
+    return cudaLaunchKernelEx(&cfg, cross_entropy_kernel<CL>, a) == cudaSuccess;
+}
+static bool ce_launch_any(sb_ctx_t* c, const CeArgs& a) {
+    switch (ce_cluster(c, a.T, a.V)) {
+        case 1: return ce_launch<1>(c, a);
+        case 2: return ce_launch<2>(c, a);
+        case 4: return ce_launch<4>(c, a);
+        case 8: return ce_launch<8>(c, a);
+        default:
+            c->launches++;
+            return sb_launch(cross_entropy_long_kernel, dim3(a.T), dim3(CE_LONG), 0, (cudaStream_t)c->pub.stream, a) == cudaSuccess;
+    }
+}
+}
+// grad NULL: the loss alone
 void sb_cross_entropy(sb_ctx_t* c, const float* logits, const uint32_t* targets, float* grad, float* loss_rows,
                       const uint32_t* pos_ids, const uint32_t* seq_ids, const uint32_t* seq_starts, int T, int V, int num_valid) {
     if (T <= 0 || V <= 0) return;
-    int vec = (V % 4 == 0) && aligned16(logits) && aligned16(grad);
     int tk = sb_tick_begin(c, SB_CLS_CE);
-    sb_launch(cross_entropy_kernel, dim3(T), dim3(CE_THREADS), 0, (cudaStream_t)c->pub.stream, logits, targets, grad, loss_rows, pos_ids, seq_ids,
-                                                                          seq_starts, T, V, 1.0f / (float)num_valid, vec, c->d_status, sb_amax_take(c, grad, (size_t)T * V),
-                                                                          nullptr, nullptr, 0.f, nullptr, 0u);
-    sb_tick_end(c, tk, 0.0, 12.0 * T * V);
-    c->launches++;
+    const CeArgs a = {logits, targets, grad, loss_rows, pos_ids, seq_ids, seq_starts, T, V, 1.0f / (float)num_valid, c->d_status,
+                      grad ? sb_amax_take(c, grad, (size_t)T * V) : nullptr, nullptr, nullptr, 0.f, nullptr, 0u};
+    if (!((V % 4) == 0 && aligned16(logits) && (!grad || aligned16(grad)) && ce_launch_any(c, a))) {
+        sb_launch(cross_entropy_any_kernel, dim3(T), dim3(CE_THREADS), 0, (cudaStream_t)c->pub.stream, logits, targets, grad, loss_rows, pos_ids, seq_ids,
+                  seq_starts, T, V, a.inv_valid, c->d_status, a.amax_grad);
+        c->launches++;
+    }
+    sb_tick_end(c, tk, 0.0, (grad ? 8.0 : 4.0) * T * V);
 }
 
 // The same, with the gradient written only as the FP16 parts of the registered tensor `grad` (its FP32 array is not touched): the
@@ -1038,10 +1245,11 @@ int sb_cross_entropy_parts(sb_ctx_t* c, const float* logits, const uint32_t* tar
     int sh = ce_shift(inv_valid); sh = sh < -100 ? -100 : (sh > 100 ? 100 : sh);      // the rule the products apply to *amax
     const float sc = ldexpf(1.0f, sh);
     int tk = sb_tick_begin(c, SB_CLS_CE);
-    sb_launch(cross_entropy_kernel, dim3(T), dim3(CE_THREADS), 0, (cudaStream_t)c->pub.stream, logits, targets, grad, loss_rows, pos_ids, seq_ids, seq_starts, T, V,
-                                                                          inv_valid, 1, c->d_status, nullptr, (__half*)h, (__half*)h + (size_t)T * V, sc, amax, sb_parts_keep(c));
-    sb_tick_end(c, tk, 0.0, 12.0 * T * V);
-    c->launches++;
+    const CeArgs a = {logits, targets, nullptr, loss_rows, pos_ids, seq_ids, seq_starts, T, V, inv_valid, c->d_status, nullptr,
+                      (__half*)h, (__half*)h + (size_t)T * V, sc, amax, sb_parts_keep(c)};
+    const bool ok = ce_launch_any(c, a);
+    sb_tick_end(c, tk, 0.0, 8.0 * T * V);
+    if (!ok) sb_set_status(c, SB_ERR_CUDA);
     return 1;
 }
 
@@ -1077,7 +1285,7 @@ void sb_embedding_backward(sb_ctx_t* c, const uint32_t* tok, const float* g, flo
     size_t ints = sb_embedding_scratch_ints(T, V);
     int* base = (int*)sb_scratch(c, ints * sizeof(int));
     if (!base) return;
-    int *cnt = base, *start = cnt + V, *rows = start + V, *meta = rows + V, *sorted_pos = meta + 4, *chunk_cnt = sorted_pos + T;
+    int *cnt = base, *start = cnt + V, *rows = start + V, *meta = rows + V, *sorted_pos = meta + 4, *chunk_cnt = sorted_pos + T;      // sb_embedding_segments reads the same layout
     int tk = sb_tick_begin(c, SB_CLS_EMBED);
     cudaMemsetAsync(cnt, 0, (size_t)V * sizeof(int), s);
     cudaMemsetAsync(chunk_cnt, 0, (size_t)nchunk * V * sizeof(int), s);

@@ -1143,7 +1143,7 @@ static float step_body(train_state_t* st, int* tokens, int T, int* seq_starts, i
     if (!(ce_parts && sb_cross_entropy_parts(c, c->logits, c->targets, c->dlogits, c->loss_rows, c->pos_ids, c->seq_ids, c->seq_starts,
                                                           T, c->V, num_valid))) {
         if (train) sb_amax_announce(c, c->dlogits, (size_t)T * c->V);
-        sb_cross_entropy(c, c->logits, c->targets, c->dlogits, c->loss_rows, c->pos_ids, c->seq_ids, c->seq_starts, T, c->V, num_valid);
+        sb_cross_entropy(c, c->logits, c->targets, train ? c->dlogits : NULL, c->loss_rows, c->pos_ids, c->seq_ids, c->seq_starts, T, c->V, num_valid);
     }
     sb_reduce_sum(c, c->loss_rows, c->d_loss, (size_t)T);
 
