@@ -130,7 +130,7 @@ extern "C" void sb_parts_unregister(sb_ctx_t* c, int kind) {
 }
 #define SB_HINT_CAP 4096
 // a device word that is zero until the current step ends; NULL outside a step or when they are used up
-float* sb_zero_word(sb_ctx_t* c) {
+extern "C" float* sb_zero_word(sb_ctx_t* c) {
     if (!c->parts_open || !c->hint_pool || c->hint_n >= c->hint_cap) return NULL;
     c->hint_tab[c->hint_n].ptr = NULL; c->hint_tab[c->hint_n].n = 0;
     return c->hint_pool + c->hint_n++;
@@ -243,6 +243,15 @@ extern "C" int sb_parts_find(sb_ctx_t* c, const float* x, size_t n, void** hout,
     return 1;
 }
 
+extern "C" int sb_bound_out(sb_ctx_t* c, const float* x, size_t n, void** parts, float** word) {
+    int fresh;
+    sb_amax_forget(c, x);
+    if (sb_parts_find(c, x, n, parts, word, &fresh)) return 1;
+    *parts = NULL;
+    sb_amax_announce(c, x, n);
+    *word = (float*)sb_amax_take(c, x, n);
+    return *word ? 2 : 0;
+}
 extern "C" void sb_gemm_keep_begin(sb_ctx_t* c) { c->f16_keep = 1; }
 // the array at `p` is about to be rewritten inside a keep region: parts kept for it are stale
 extern "C" void sb_gemm_keep_forget(sb_ctx_t* c, const float* p) {

@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_kernel(const float* __r
 #define SW_UNROLL 2
 static inline dim3 sw_grid(size_t n4) { return dim3((unsigned)((n4 + EW_THREADS * SW_UNROLL - 1) / (EW_THREADS * SW_UNROLL))); }
 __global__ void __launch_bounds__(EW_THREADS) swiglu_parts_kernel(const float4* __restrict__ gate, const float4* __restrict__ up,
-                                                                  uint2* __restrict__ h1, uint2* __restrict__ h2, size_t n4,
+                                                                  float4* __restrict__ out, uint2* __restrict__ h1, uint2* __restrict__ h2, size_t n4,
                                                                   const float* __restrict__ amax_g, const float* __restrict__ amax_u,
                                                                   float* __restrict__ bound_out, unsigned keep) {
     sb_pdl_enter();
@@ -143,16 +143,16 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_parts_kernel(const float4* 
         const size_t i = i0 + k * EW_THREADS;
         if (i >= n4) break;
         const float4 g = gv[k], u = uv[k];
-        const float r0 = ew_apply<OP_SWIGLU>(g.x, u.x) * sc, r1 = ew_apply<OP_SWIGLU>(g.y, u.y) * sc;
-        const float r2 = ew_apply<OP_SWIGLU>(g.z, u.z) * sc, r3 = ew_apply<OP_SWIGLU>(g.w, u.w) * sc;
+        const float4 r = make_float4(ew_apply<OP_SWIGLU>(g.x, u.x), ew_apply<OP_SWIGLU>(g.y, u.y), ew_apply<OP_SWIGLU>(g.z, u.z), ew_apply<OP_SWIGLU>(g.w, u.w));
+        if (out) { out[i] = r; continue; }                       // no arena for the parts
         uint2 a, b;
-        sb_split2(r0, r1, a.x, b.x, keep); sb_split2(r2, r3, a.y, b.y, keep);
+        sb_split2(r.x * sc, r.y * sc, a.x, b.x, keep); sb_split2(r.z * sc, r.w * sc, a.y, b.y, keep);
         h1[i] = a; h2[i] = b;
     }
 }
 __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_parts_kernel(const float4* __restrict__ gate, const float4* __restrict__ up,
                                                                       const float4* __restrict__ dout,
-                                                                      uint2* __restrict__ dg1, uint2* __restrict__ dg2,
+                                                                      float4* __restrict__ dgo, float4* __restrict__ duo, uint2* __restrict__ dg1, uint2* __restrict__ dg2,
                                                                       uint2* __restrict__ du1, uint2* __restrict__ du2, size_t n4,
                                                                       const float* __restrict__ amax_g, const float* __restrict__ amax_u,
                                                                       const float* __restrict__ amax_d,
@@ -174,6 +174,7 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_parts_kernel(const floa
         float4 dg, du;
         SWIGLU_BWD_ONE(g.x, u.x, d.x, dg.x, du.x) SWIGLU_BWD_ONE(g.y, u.y, d.y, dg.y, du.y)
         SWIGLU_BWD_ONE(g.z, u.z, d.z, dg.z, du.z) SWIGLU_BWD_ONE(g.w, u.w, d.w, dg.w, du.w)
+        if (dgo) { dgo[i] = dg; duo[i] = du; continue; }
         uint2 a, b, e, f;
         sb_split2(dg.x * sg_, dg.y * sg_, a.x, b.x, keep); sb_split2(dg.z * sg_, dg.w * sg_, a.y, b.y, keep);
         sb_split2(du.x * su, du.y * su, e.x, f.x, keep); sb_split2(du.z * su, du.w * su, e.y, f.y, keep);
@@ -425,11 +426,10 @@ int sb_swiglu_parts(sb_ctx_t* c, const float* gate, const float* up, float* out,
     if (!n || (n & 7) || !aligned16(gate) || !aligned16(up)) return 0;
     float* ag = sb_amax_lookup(c, gate, n); float* au = sb_amax_lookup(c, up, n);
     if (!ag || !au) return 0;
-    void* h; float* bound; int fresh;
-    if (!sb_parts_find(c, out, n, &h, &bound, &fresh)) return 0;
-    sb_amax_forget(c, out);
+    void* h; float* bound;
+    if (!aligned16(out) || !sb_bound_out(c, out, n, &h, &bound)) return 0;
     int tk = sb_tick_begin(c, SB_CLS_SWIGLU);
-    sb_launch(swiglu_parts_kernel, sw_grid(n / 4), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (const float4*)gate, (const float4*)up, (uint2*)h,
+    sb_launch(swiglu_parts_kernel, sw_grid(n / 4), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (const float4*)gate, (const float4*)up, h ? (float4*)nullptr : (float4*)out, (uint2*)h,
                                                                                          (uint2*)((uint16_t*)h + n), n / 4, ag, au, bound, sb_parts_keep(c));
     sb_tick_end(c, tk, 0.0, 12.0 * (double)n);
     c->launches++;
@@ -439,11 +439,13 @@ int sb_swiglu_backward_parts(sb_ctx_t* c, const float* gate, const float* up, co
     if (!n || (n & 7) || !aligned16(gate) || !aligned16(up) || !aligned16(dout)) return 0;
     float* ag = sb_amax_lookup(c, gate, n); float* au = sb_amax_lookup(c, up, n); float* ad = sb_amax_lookup(c, dout, n);
     if (!ag || !au || !ad) return 0;
-    void *hg, *hu; float *bg, *bu; int fresh;
-    if (!sb_parts_find(c, dgate, n, &hg, &bg, &fresh) || !sb_parts_find(c, dup, n, &hu, &bu, &fresh)) return 0;
-    sb_amax_forget(c, dgate); sb_amax_forget(c, dup);
+    void *hg, *hu; float *bg, *bu;
+    if (!aligned16(dgate) || !aligned16(dup)) return 0;
+    const int kg = sb_bound_out(c, dgate, n, &hg, &bg), ku = sb_bound_out(c, dup, n, &hu, &bu);
+    if (!kg || kg != ku) { sb_amax_forget(c, dgate); sb_amax_forget(c, dup); return 0; }
+    float4 *og = hg ? nullptr : (float4*)dgate, *ou = hu ? nullptr : (float4*)dup;
     int tk = sb_tick_begin(c, SB_CLS_SWIGLU);
-    sb_launch(swiglu_bwd_parts_kernel, sw_grid(n / 4), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (const float4*)gate, (const float4*)up, (const float4*)dout, (uint2*)hg, (uint2*)((uint16_t*)hg + n), (uint2*)hu, (uint2*)((uint16_t*)hu + n),
+    sb_launch(swiglu_bwd_parts_kernel, sw_grid(n / 4), dim3(EW_THREADS), 0, (cudaStream_t)c->pub.stream, (const float4*)gate, (const float4*)up, (const float4*)dout, og, ou, (uint2*)hg, (uint2*)((uint16_t*)hg + n), (uint2*)hu, (uint2*)((uint16_t*)hu + n),
         n / 4, ag, au, ad, bg, bu, sb_parts_keep(c));
     sb_tick_end(c, tk, 0.0, 20.0 * (double)n);
     c->launches++;

@@ -138,11 +138,11 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_bwd_kernel(const float* __
 // ---------------------------------------------------------------------------
 template <int NV>
 __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                                  float* __restrict__ y, float* __restrict__ copy, int rows, int cols, float eps, unsigned* amax_out) {
+                                                                  float* __restrict__ y, float* __restrict__ copy, int rows, int cols, float eps, unsigned* amax_out, unsigned* inv_max) {
     sb_pdl_enter();
     const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int c4 = cols >> 2;
-    float am = 0.f;
+    float am = 0.f, im = 0.f;
     for (int r = warp; r < rows; r += nwarps) {
         const float4* xr = (const float4*)(x + (size_t)r * cols);
         float4 v[NV];
@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_kernel(const float* _
         }
         ss = warp_sum(ss);
         const float inv = 1.0f / sqrtf(ss / cols + eps);
+        im = fmaxf(im, inv);
         float4* yr = (float4*)(y + (size_t)r * cols);
 #pragma unroll
         for (int i = 0; i < NV; i++) {
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_kernel(const float* _
         }
     }
     sb_block_amax(am, amax_out);
+    if (inv_max && lane == 0 && im > 0.f) atomicMax(inv_max, __float_as_uint(im));
 }
 
 // Rows of exactly 128 columns (the learned per-head norm: rows = tokens x heads): one float4 per lane, four rows of a warp in
@@ -201,6 +203,16 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_w128_kernel(const float* _
 // registers.  The loads of the next group (x, dy, residual) are issued before the current group is reduced,
 // so memory requests are in flight during the two CTA-wide reductions (sum x^2 and sum dy*w*x of each row);
 // two CTAs share an SM.  One dscale partial row per CTA, summed in CTA order by colsum_partials_kernel.
+// With RnbOut the result leaves as FP16 operand parts beside FP32, for the products that read the gradient next.  Its bound: with g = dy o w and
+// xh = x / rms, dx = (g - xh mean(g o xh)) / rms + residual, |xh_i| <= sqrt(cols) and |mean(g o xh)| <= rms(g) <= max|g|, so
+//   |dx| <= max|residual| + (1 + sqrt(cols)) max(1/rms) max|w| max|dy|.
+// It is some 2^5 above the true maximum, which costs only values below 2^-13 of that maximum a part of their low halves (see sb_f16_shift).
+struct RnbOut {
+    uint2 *h1, *h2;                                   // NULL: only the bound is formed
+    const float *amax_dy, *amax_resid, *inv_max;      // amax_resid NULL: no residual
+    float* bound;                                     // NULL: neither parts nor bound
+    unsigned keep;
+};
 template <int NC, int ROWS>
 struct RnbSet { float4 v[ROWS][NC], g[ROWS][NC], q[ROWS][NC]; };
 
@@ -230,7 +242,7 @@ __device__ __forceinline__ float4 rnb_scale(const float4 (&scr)[NC], const float
 
 template <int NC, int ROWS>
 __device__ __forceinline__ void rnb_compute(const RnbSet<NC, ROWS>& s, const float4 (&scr)[NC], const float* __restrict__ w, float4 (&acc)[NC], float* dx, int r0, int rows,
-                                            int cols, int c4, float eps, float (*s_red)[2 * ROWS], float* s_tot, float& am) {
+                                            int cols, int c4, float eps, float (*s_red)[2 * ROWS], float* s_tot, float& am, const RnbOut& out, float osc) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     float part[2 * ROWS];
 #pragma unroll
@@ -271,6 +283,11 @@ __device__ __forceinline__ void rnb_compute(const RnbSet<NC, ROWS>& s, const flo
                 o.x = g.x * sc.x * inv - v.x * k + q.x; o.y = g.y * sc.y * inv - v.y * k + q.y;
                 o.z = g.z * sc.z * inv - v.z * k + q.z; o.w = g.w * sc.w * inv - v.w * k + q.w;
                 ((float4*)dx)[(size_t)(r0 + rr) * c4 + j] = o;
+                if (out.h1) {
+                    uint2 hh, hl;
+                    sb_split2(o.x * osc, o.y * osc, hh.x, hl.x, out.keep); sb_split2(o.z * osc, o.w * osc, hh.y, hl.y, out.keep);
+                    out.h1[(size_t)(r0 + rr) * c4 + j] = hh; out.h2[(size_t)(r0 + rr) * c4 + j] = hl;
+                }
                 am = sb_amax4(am, o);
             }
         }
@@ -280,11 +297,12 @@ __device__ __forceinline__ void rnb_compute(const RnbSet<NC, ROWS>& s, const flo
 template <int NC, int ROWS>
 __global__ void __launch_bounds__(RB_THREADS, 2) rmsnorm_bwd_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                                          const float* __restrict__ dy, const float* resid, float* dx,
-                                                                         float* __restrict__ partial, int rows, int cols, float eps, unsigned* amax_dx) {
+                                                                         float* __restrict__ partial, int rows, int cols, float eps, unsigned* amax_dx, const RnbOut out) {
     sb_pdl_enter();
     float am = 0.f;
     __shared__ float s_red[2][RB_THREADS / 32][2 * ROWS];
     __shared__ float s_tot[2][2 * ROWS];
+    __shared__ float s_w[RB_THREADS / 32];
     const int c4 = cols >> 2;
     float4 acc[NC], sc[NC];
 #pragma unroll
@@ -293,17 +311,30 @@ __global__ void __launch_bounds__(RB_THREADS, 2) rmsnorm_bwd_rows_kernel(const f
         const int j = threadIdx.x + RB_THREADS * i;
         sc[i] = j < c4 ? ((const float4*)w)[j] : acc[i];
     }
+    float osc = 1.f;
+    if (out.bound) {
+        float wm = 0.f;
+#pragma unroll
+        for (int i = 0; i < NC; i++) wm = sb_amax4(wm, sc[i]);
+        wm = warp_max(wm);
+        if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = wm;
+        __syncthreads();
+        wm = warp_max(s_w[threadIdx.x & (RB_THREADS / 32 - 1)]);
+        const float bound = fminf((out.amax_resid ? sb_word(out.amax_resid) : 0.f) + 1.0001f * (1.f + sqrtf((float)cols)) * sb_word(out.inv_max) * wm * sb_word(out.amax_dy), 3.0e38f);
+        osc = sb_pow2(sb_f16_shift(bound));
+        if (blockIdx.x == 0 && threadIdx.x == 0) *out.bound = bound;
+    }
     const int ngroups = (rows + ROWS - 1) / ROWS, stride = gridDim.x;
     RnbSet<NC, ROWS> a, b;
     int gidx = blockIdx.x;
     if (gidx < ngroups) rnb_load<NC, ROWS>(a, x, dy, resid, gidx * ROWS, rows, c4);
     while (gidx < ngroups) {
         if (gidx + stride < ngroups) rnb_load<NC, ROWS>(b, x, dy, resid, (gidx + stride) * ROWS, rows, c4);
-        rnb_compute<NC, ROWS>(a, sc, w, acc, dx, gidx * ROWS, rows, cols, c4, eps, s_red[0], s_tot[0], am);
+        rnb_compute<NC, ROWS>(a, sc, w, acc, dx, gidx * ROWS, rows, cols, c4, eps, s_red[0], s_tot[0], am, out, osc);
         gidx += stride;
         if (gidx >= ngroups) break;
         if (gidx + stride < ngroups) rnb_load<NC, ROWS>(a, x, dy, resid, (gidx + stride) * ROWS, rows, c4);
-        rnb_compute<NC, ROWS>(b, sc, w, acc, dx, gidx * ROWS, rows, cols, c4, eps, s_red[1], s_tot[1], am);
+        rnb_compute<NC, ROWS>(b, sc, w, acc, dx, gidx * ROWS, rows, cols, c4, eps, s_red[1], s_tot[1], am, out, osc);
         gidx += stride;
     }
 #pragma unroll
@@ -437,8 +468,8 @@ __global__ void __launch_bounds__(RB_THREADS) softmax_kernel(const float* __rest
 // exceed the row's sum of squares), so that bound sets the scale and no pass over y looks for its maximum or splits it again.
 template <int NV>
 __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                                        uint2* __restrict__ h1, uint2* __restrict__ h2, int rows, int cols, float eps,
-                                                                        float* __restrict__ bound_out, unsigned keep, float* __restrict__ copy) {
+                                                                        float* __restrict__ y, uint2* __restrict__ h1, uint2* __restrict__ h2, int rows, int cols, float eps,
+                                                                        float* __restrict__ bound_out, unsigned keep, float* __restrict__ copy, unsigned* inv_max) {
     sb_pdl_enter();
     const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int c4 = cols >> 2;
@@ -453,6 +484,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const fl
     const float bound = fminf(sqrtf((float)cols) * wm * 1.0001f, 3.0e38f);
     const float sc = sb_pow2(sb_f16_shift(bound));
     if (warp == 0 && lane == 0) *bound_out = bound;
+    float im = 0.f;
     for (int r = warp; r < rows; r += nwarps) {
         const float4* xr = (const float4*)(x + (size_t)r * cols);
         float4 v[NV];
@@ -466,6 +498,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const fl
         }
         ss = warp_sum(ss);
         const float inv = 1.0f / sqrtf(ss / cols + eps);
+        im = fmaxf(im, inv);
         uint2* o1 = h1 + (size_t)r * c4; uint2* o2 = h2 + (size_t)r * c4;
 #pragma unroll
         for (int i = 0; i < NV; i++) {
@@ -474,12 +507,14 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const fl
                 // the FP32 value first, exactly as the plain kernel forms it, then the scale (a power of two: exact)
                 const float4 s = ((const float4*)w)[j];
                 const float y0 = v[i].x * inv * s.x, y1 = v[i].y * inv * s.y, y2 = v[i].z * inv * s.z, y3 = v[i].w * inv * s.w;
+                if (y) { ((float4*)(y + (size_t)r * cols))[j] = make_float4(y0, y1, y2, y3); continue; }      // no arena for the parts
                 uint2 a, b;
                 sb_split2(y0 * sc, y1 * sc, a.x, b.x, keep); sb_split2(y2 * sc, y3 * sc, a.y, b.y, keep);
                 o1[j] = a; o2[j] = b;
             }
         }
     }
+    if (inv_max && lane == 0 && im > 0.f) atomicMax(inv_max, __float_as_uint(im));
 }
 template <int NV>
 __global__ void __launch_bounds__(RB_THREADS) qk_norm_warp_kernel(float* __restrict__ x, float* __restrict__ rms_out, int rows, int cols, float eps) {
@@ -608,7 +643,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(const __grid_
     const size_t out = (size_t)r * n4 + lo;
     float4* gr = p.grad ? (float4*)p.grad + out : nullptr;
     uint2* p1 = p.g1 ? (uint2*)p.g1 + out : nullptr; uint2* p2 = p.g1 ? (uint2*)p.g2 + out : nullptr;
-    if (p.g1 && blockIdx.x == 0 && threadIdx.x == 0) *p.part_amax = p.inv_valid;
+    if (p.part_amax && blockIdx.x == 0 && threadIdx.x == 0) *p.part_amax = p.inv_valid;
     const uint32_t s = p.seq_ids[r];
     if ((int)p.pos_ids[r] >= (int)(p.seq_starts[s + 1] - p.seq_starts[s]) - 1) {
         for (int i = threadIdx.x; i < n; i += CE_THREADS) {
@@ -696,7 +731,7 @@ __global__ void __launch_bounds__(CE_LONG, 1) cross_entropy_long_kernel(const __
     const size_t out = (size_t)r * n;
     float4* gr = p.grad ? (float4*)p.grad + out : nullptr;
     uint2* p1 = p.g1 ? (uint2*)p.g1 + out : nullptr; uint2* p2 = p.g1 ? (uint2*)p.g2 + out : nullptr;
-    if (p.g1 && r == 0 && threadIdx.x == 0) *p.part_amax = p.inv_valid;
+    if (p.part_amax && r == 0 && threadIdx.x == 0) *p.part_amax = p.inv_valid;
     const uint32_t s = p.seq_ids[r];
     if ((int)p.pos_ids[r] >= (int)(p.seq_starts[s + 1] - p.seq_starts[s]) - 1) {
         for (int i = threadIdx.x; i < n; i += CE_LONG) {
@@ -956,7 +991,9 @@ __global__ void __launch_bounds__(RB_THREADS) adamw_kernel(float* __restrict__ w
 extern "C" {
 
 // `copy` (may be NULL) receives the rows x as well: the residual stream that the layer's next product adds into, written while x is in registers
-void sb_rmsnorm_copy(sb_ctx_t* c, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps) {
+// inv_word (may be NULL): a word raised to the largest 1 / rms of the rows, for the bound of the backward pass; *inv_word = NULL on return when it was not formed
+void sb_rmsnorm_copy(sb_ctx_t* c, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps, float** inv_word) {
+    float* inv_max = inv_word ? *inv_word : NULL;
     if (rows <= 0 || cols <= 0) return;
     sb_parts_invalidate(c, y);
     int grid = rows < sm_count(c) * 8 ? rows : sm_count(c) * 8;
@@ -970,36 +1007,40 @@ void sb_rmsnorm_copy(sb_ctx_t* c, const float* x, const float* w, float* y, floa
         cudaStream_t st = (cudaStream_t)c->pub.stream;
         unsigned* am = sb_amax_take(c, y, (size_t)rows * cols);
         if (cols == 128 && rows >= 1024) {
+            if (inv_word) *inv_word = NULL;
             int g4 = (rows + 31) / 32; if (g4 > sm_count(c) * 4) g4 = sm_count(c) * 4;      // 8 warps x 4 rows per CTA and pass
             sb_launch(rmsnorm_w128_kernel, dim3(g4), dim3(RB_THREADS), 0, st, x, w, y, rows, eps, am);
         } else
-        if (cols <= 512)       sb_launch(rmsnorm_warp_kernel<4>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am);
-        else if (cols <= 1024) sb_launch(rmsnorm_warp_kernel<8>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am);
-        else if (cols <= 2048) sb_launch(rmsnorm_warp_kernel<16>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am);
-        else                   sb_launch(rmsnorm_warp_kernel<32>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am);
-    } else
+        if (cols <= 512)       sb_launch(rmsnorm_warp_kernel<4>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am, (unsigned*)inv_max);
+        else if (cols <= 1024) sb_launch(rmsnorm_warp_kernel<8>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am, (unsigned*)inv_max);
+        else if (cols <= 2048) sb_launch(rmsnorm_warp_kernel<16>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am, (unsigned*)inv_max);
+        else                   sb_launch(rmsnorm_warp_kernel<32>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am, (unsigned*)inv_max);
+    } else {
+    if (inv_word) *inv_word = NULL;
     sb_launch(rmsnorm_kernel, dim3(grid), dim3(RB_THREADS), 0, (cudaStream_t)c->pub.stream, x, w, y, rows, cols, eps, vec);
+    }
     sb_tick_end(c, tk, 0.0, (copy ? 12.0 : 8.0) * rows * cols);
     c->launches++;
 }
-void sb_rmsnorm(sb_ctx_t* c, const float* x, const float* w, float* y, int rows, int cols, float eps) { sb_rmsnorm_copy(c, x, w, y, NULL, rows, cols, eps); }
+void sb_rmsnorm(sb_ctx_t* c, const float* x, const float* w, float* y, int rows, int cols, float eps) { sb_rmsnorm_copy(c, x, w, y, NULL, rows, cols, eps, NULL); }
 
 // y only as the FP16 parts of the registered tensor `y`; 1 = done, 0 = not possible here (call sb_rmsnorm)
-int sb_rmsnorm_parts(sb_ctx_t* c, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps) {
+int sb_rmsnorm_parts(sb_ctx_t* c, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps, float** inv_word) {
+    float* inv_max = inv_word ? *inv_word : NULL;
     if (rows < 1 || cols <= 0 || (cols & 7) || cols > 4096 || !aligned16(x) || !aligned16(w) || (copy && !aligned16(copy))) return 0;
-    void* h; float* bound; int fresh;
+    void* h; float* bound;
     const size_t n = (size_t)rows * cols;
-    if (!sb_parts_find(c, y, n, &h, &bound, &fresh)) return 0;
-    sb_amax_forget(c, y);
+    if (!aligned16(y) || !sb_bound_out(c, y, n, &h, &bound)) return 0;
+    float* y32 = h ? NULL : y;
     int wgrid = (rows + 7) / 8;
     { int cap = sm_count(c) * 2, k = (wgrid + cap - 1) / cap; wgrid = (wgrid + k - 1) / k; }
     cudaStream_t st = (cudaStream_t)c->pub.stream;
     uint2* h1 = (uint2*)h; uint2* h2 = (uint2*)((uint16_t*)h + n);
     int tk = sb_tick_begin(c, SB_CLS_NORM_FWD);
-    if (cols <= 512)       sb_launch(rmsnorm_warp_parts_kernel<4>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy);
-    else if (cols <= 1024) sb_launch(rmsnorm_warp_parts_kernel<8>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy);
-    else if (cols <= 2048) sb_launch(rmsnorm_warp_parts_kernel<16>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy);
-    else                   sb_launch(rmsnorm_warp_parts_kernel<32>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy);
+    if (cols <= 512)       sb_launch(rmsnorm_warp_parts_kernel<4>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y32, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy, (unsigned*)inv_max);
+    else if (cols <= 1024) sb_launch(rmsnorm_warp_parts_kernel<8>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y32, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy, (unsigned*)inv_max);
+    else if (cols <= 2048) sb_launch(rmsnorm_warp_parts_kernel<16>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y32, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy, (unsigned*)inv_max);
+    else                   sb_launch(rmsnorm_warp_parts_kernel<32>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y32, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy, (unsigned*)inv_max);
     sb_tick_end(c, tk, 0.0, (copy ? 12.0 : 8.0) * rows * cols);
     c->launches++;
     return 1;
@@ -1082,12 +1123,13 @@ void sb_rmsnorm_backward_with_partials(sb_ctx_t* c, const float* x, const float*
     sb_tick_end(c, tk, 0.0, (resid ? 16.0 : 12.0) * rows * cols);
 }
 
-void sb_rmsnorm_backward(sb_ctx_t* c, const float* x, const float* w, const float* dy, const float* resid,
-                         float* dx_out, float* dscale, int rows, int cols, float eps) {
+static bool rn_rows_ok(int vec, int cols) { return vec && cols <= 4096; }
+static void rn_backward(sb_ctx_t* c, const float* x, const float* w, const float* dy, const float* resid,
+                        float* dx_out, float* dscale, int rows, int cols, float eps, const RnbOut& out, unsigned* exact) {
     if (rows <= 0 || cols <= 0) return;
     if (cols > RB_THREADS * 4 * RN_MAX_SWEEP || (cols % 4 != 0 && cols > RB_THREADS * RN_MAX_SWEEP * 4)) { sb_set_status(c, SB_ERR_SIZE); return; }
     int vec = (cols % 4 == 0) && aligned16(x) && aligned16(w) && aligned16(dy) && aligned16(dx_out) && (!resid || aligned16(resid));
-    if (vec && cols == 128 && rows >= 1024) {
+    if (vec && cols == 128 && rows >= 1024 && !out.bound) {
         // many short rows (the per-head norm): a warp per row
         int wgrid = (rows + 31) / 32; if (wgrid > 4 * sm_count(c)) wgrid = 4 * sm_count(c);
         float* partial = rn_partials(c, (size_t)wgrid * cols);
@@ -1101,7 +1143,7 @@ void sb_rmsnorm_backward(sb_ctx_t* c, const float* x, const float* w, const floa
         sb_tick_end(c, tk, 0.0, (resid ? 16.0 : 12.0) * rows * cols);
         return;
     }
-    if (vec && cols <= 4096) {
+    if (rn_rows_ok(vec, cols)) {
         // row groups with the next group's loads in flight, two CTAs per SM; one dscale partial per CTA, summed in CTA order.  Groups of two
         // rows, of one above 2048 columns (a thread then holds four chunks of a row, and two rows would not fit its registers).
         const int per = cols <= 2048 ? 2 : 1;
@@ -1110,10 +1152,10 @@ void sb_rmsnorm_backward(sb_ctx_t* c, const float* x, const float* w, const floa
         if (!partial) return;
         cudaStream_t st = (cudaStream_t)c->pub.stream;
         int tk = sb_tick_begin(c, SB_CLS_NORM_BWD);
-        unsigned* am = sb_amax_take(c, dx_out, (size_t)rows * cols);
-        if (cols <= 1024)      sb_launch(rmsnorm_bwd_rows_kernel<1, 2>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
-        else if (cols > 2048)  sb_launch(rmsnorm_bwd_rows_kernel<4, 1>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
-        else                   sb_launch(rmsnorm_bwd_rows_kernel<2, 2>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am);
+        unsigned* am = exact ? exact : sb_amax_take(c, dx_out, (size_t)rows * cols);
+        if (cols <= 1024)      sb_launch(rmsnorm_bwd_rows_kernel<1, 2>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am, out);
+        else if (cols > 2048)  sb_launch(rmsnorm_bwd_rows_kernel<4, 1>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am, out);
+        else                   sb_launch(rmsnorm_bwd_rows_kernel<2, 2>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, dy, resid, dx_out, partial, rows, cols, eps, am, out);
         c->launches++;
         if (dscale) rn_dscale(c, partial, dscale, wgrid, cols);
         sb_tick_end(c, tk, 0.0, (resid ? 16.0 : 12.0) * rows * cols);
@@ -1123,6 +1165,32 @@ void sb_rmsnorm_backward(sb_ctx_t* c, const float* x, const float* w, const floa
     float* partial = rn_partials(c, (size_t)grid * cols);
     if (!partial) return;
     sb_rmsnorm_backward_with_partials(c, x, w, dy, resid, dx_out, dscale, rows, cols, eps, partial, grid);
+}
+void sb_rmsnorm_backward(sb_ctx_t* c, const float* x, const float* w, const float* dy, const float* resid,
+                         float* dx_out, float* dscale, int rows, int cols, float eps) {
+    const RnbOut none = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0u};
+    sb_parts_invalidate(c, dx_out);
+    rn_backward(c, x, w, dy, resid, dx_out, dscale, rows, cols, eps, none, nullptr);
+}
+// The same, with dx handed on as operand parts under a bound where max|dy|, max|residual| and max(1/rms) are known (a pass over dx less);
+// *amax: in, the word with max|residual|; out, the word with max|dx| (NULL: not known).
+void sb_rmsnorm_backward_parts(sb_ctx_t* c, const float* x, const float* w, const float* dy, const float* resid,
+                               float* dx_out, float* dscale, int rows, int cols, float eps, const float* inv_max, float** amax) {
+    const size_t n = (size_t)rows * cols;
+    const int vec = (cols % 8 == 0) && aligned16(x) && aligned16(w) && aligned16(dy) && aligned16(dx_out) && (!resid || aligned16(resid));
+    RnbOut out = {nullptr, nullptr, sb_amax_lookup(c, dy, n), resid ? *amax : nullptr, inv_max, nullptr, sb_parts_keep(c)};
+    float* exact = rn_rows_ok(vec, cols) && inv_max && out.amax_dy && (!resid || *amax) ? sb_zero_word(c) : nullptr;
+    if (exact) { sb_amax_announce(c, dx_out, n); out.bound = (float*)sb_amax_take(c, dx_out, n); }
+    if (!out.bound) {
+        sb_amax_announce(c, dx_out, n);
+        sb_rmsnorm_backward(c, x, w, dy, resid, dx_out, dscale, rows, cols, eps);
+        *amax = sb_amax_lookup(c, dx_out, n);
+        return;
+    }
+    void* h; float* own; int fresh;
+    if (sb_parts_find(c, dx_out, n, &h, &own, &fresh)) { sb_parts_set_amax(c, dx_out, out.bound); out.h1 = (uint2*)h; out.h2 = (uint2*)((uint16_t*)h + n); }
+    rn_backward(c, x, w, dy, resid, dx_out, dscale, rows, cols, eps, out, (unsigned*)exact);
+    *amax = exact;
 }
 
 void sb_softmax(sb_ctx_t* c, const float* x, float* y, int rows, int cols) {
@@ -1239,14 +1307,14 @@ static __device__ __host__ inline int ce_shift(float amax) {
 int sb_cross_entropy_parts(sb_ctx_t* c, const float* logits, const uint32_t* targets, float* grad, float* loss_rows,
                            const uint32_t* pos_ids, const uint32_t* seq_ids, const uint32_t* seq_starts, int T, int V, int num_valid) {
     if (T <= 0 || V <= 0 || (V % 4) || !aligned16(logits) || num_valid <= 0) return 0;
-    void* h; float* amax; int fresh;
-    if (!sb_parts_find(c, grad, (size_t)T * V, &h, &amax, &fresh)) return 0;
+    void* h; float* amax;
+    if (!aligned16(grad) || !sb_bound_out(c, grad, (size_t)T * V, &h, &amax)) return 0;
     const float inv_valid = 1.0f / (float)num_valid;
     int sh = ce_shift(inv_valid); sh = sh < -100 ? -100 : (sh > 100 ? 100 : sh);      // the rule the products apply to *amax
     const float sc = ldexpf(1.0f, sh);
     int tk = sb_tick_begin(c, SB_CLS_CE);
-    const CeArgs a = {logits, targets, nullptr, loss_rows, pos_ids, seq_ids, seq_starts, T, V, inv_valid, c->d_status, nullptr,
-                      (__half*)h, (__half*)h + (size_t)T * V, sc, amax, sb_parts_keep(c)};
+    const CeArgs a = {logits, targets, h ? nullptr : grad, loss_rows, pos_ids, seq_ids, seq_starts, T, V, inv_valid, c->d_status, nullptr,
+                      (__half*)h, h ? (__half*)h + (size_t)T * V : nullptr, sc, amax, sb_parts_keep(c)};
     const bool ok = ce_launch_any(c, a);
     sb_tick_end(c, tk, 0.0, 8.0 * T * V);
     if (!ok) sb_set_status(c, SB_ERR_CUDA);

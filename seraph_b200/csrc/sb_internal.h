@@ -51,6 +51,7 @@ typedef struct {
     float *layer_in, *x_norm_attn, *q, *k, *v, *attn_out, *lse, *post_attn_in, *x_norm_ffn, *gate, *up, *ffn_hidden;
     float *q_rms, *k_rms;            /* per-token sqrt(mean(x^2)) of q and k before their whole-row normalisation (use_qk_norm) */
     float *q_pre, *k_pre;            /* q and k before the learned per-head RMSNorm (head_norm), kept for its backward */
+    float *inv_attn, *inv_ffn;      /* words of this step: max 1/rms of the rows each norm read, or NULL */
 } sb_layer_act_t;
 
 typedef struct { const float* ptr; size_t n, cur, off; unsigned gen; int kind; float* amax_ptr; } sb_parts_entry_t;   /* n: registered floats, cur: floats of the parts held */
@@ -76,6 +77,7 @@ typedef struct sb_ctx {
        the operand preparation then skips its own pass over the tensor */
     struct { const float* ptr; size_t n; } *hint_tab; int hint_n, hint_cap; float* hint_pool;
     struct { const float* ptr; size_t n; } hint_pending[SB_HINT_PENDING]; int hint_npending;
+    float* final_inv; float* ghid_amax;      /* words of this step: max 1/rms of the final norm, max |g_hidden| */
     void* cs_pending; int cs_defer, cs_store;      /* dscale sums waiting for their common launch */
     int weights_fixed, in_evaluate; unsigned weights_gen;      /* the weights' parts outlive the call while weights_gen stands */
     unsigned parts_gen; int parts_open; int parts_cache;   /* parts_cache 0: off (switch, or the arena did not fit) */
@@ -184,7 +186,9 @@ void sb_tick_end(sb_ctx_t* c, int slot, double flops, double bytes);
 /* ---- kernel launchers (raw pointers) ---- */
 void sb_embed_lookup(sb_ctx_t*, const uint32_t* tok, const float* E, float* out, int T, int d, int V);
 void sb_rmsnorm(sb_ctx_t*, const float* x, const float* w, float* y, int rows, int cols, float eps);
-void sb_rmsnorm_copy(sb_ctx_t*, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps);
+void sb_rmsnorm_copy(sb_ctx_t*, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps, float** inv_word);
+void sb_rmsnorm_backward_parts(sb_ctx_t*, const float* x, const float* w, const float* dy, const float* resid, float* dx_out, float* dscale, int rows, int cols, float eps,
+                               const float* inv_max, float** amax);
 void sb_colsum_defer(sb_ctx_t*, int on, int store, size_t floats);      /* dscale sums of sb_rmsnorm_backward in one launch at the flush */
 void sb_colsum_flush(sb_ctx_t*);
 void sb_colsum_free(sb_ctx_t*);
@@ -208,7 +212,7 @@ void sb_swiglu_backward(sb_ctx_t*, const float* gate, const float* up, const flo
    magnitudes their producers left for the inputs; 1 = done, 0 = not possible here (no parts, no hints): call the plain one */
 int  sb_swiglu_parts(sb_ctx_t*, const float* gate, const float* up, float* out, size_t n);
 int  sb_attention_reads_parts(sb_ctx_t*, int Hq, int Hkv, int hd);      /* 1: forward and backward attention run on FP16 parts of q, k, v */
-int  sb_rmsnorm_parts(sb_ctx_t*, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps);      /* bound: sqrt(cols) max|w| */
+int  sb_rmsnorm_parts(sb_ctx_t*, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps, float** inv_word);      /* bound: sqrt(cols) max|w| */
 int  sb_swiglu_backward_parts(sb_ctx_t*, const float* gate, const float* up, const float* dout, float* dgate, float* dup, size_t n);
 void sb_amax_forget(sb_ctx_t*, const float* x);      /* x is written by something that leaves no maximum: earlier hints for it are void */
 void sb_seq_index(sb_ctx_t*, const uint32_t* seq_starts, int B, int T, uint32_t* pos_ids, uint32_t* seq_ids);
@@ -230,6 +234,10 @@ void sb_parts_free(sb_ctx_t*);
 void sb_amax_announce(sb_ctx_t*, const float* out, size_t n);
 unsigned* sb_amax_take(sb_ctx_t*, const float* out, size_t n);
 float* sb_amax_lookup(sb_ctx_t*, const float* x, size_t n);
+/* where a kernel that bounds its output x[n] leaves it: the parts of the registered tensor x with *word beside them (1), or without an arena the
+   plain array and a word for whoever splits it (2; so both ways give the same bits); 0: neither, use the kernel without a bound */
+int sb_bound_out(sb_ctx_t*, const float* x, size_t n, void** parts, float** word);
+float* sb_zero_word(sb_ctx_t*);      /* a device word that is zero until the step ends; NULL outside a step */
 void sb_parts_set_amax(sb_ctx_t*, const float* x, float* word);
 /* 1: x[n] is registered and the step is open; *h = its two parts (h, h + n), *amax its scale word, *fresh = parts must be made now */
 int sb_parts_find(sb_ctx_t*, const float* x, size_t n, void** h, float** amax, int* fresh);
@@ -295,7 +303,6 @@ void sb_prof_end(sb_ctx_t*, int op, size_t flops, size_t bytes);
 }
 /* the `keep` mask of sb_split2 for operands of the plain products */
 static inline unsigned sb_parts_keep(const sb_ctx_t* c) { return c->pub.use_bf16 || c->gemm_mode == SB_GEMM_BF16 ? 0xffffe000u : 0xffffffffu; }
-float* sb_zero_word(sb_ctx_t* c);
 unsigned* sb_item_counter(sb_ctx_t* c);
 int sb_f16_slot(sb_ctx_t* c, const float* x, size_t n, int own, bool* fresh);
 #endif

@@ -589,6 +589,7 @@ static int ensure_activations(sb_ctx_t* c, int T, int need_logits_grad) {
     }
     sb_parts_register(c, 1, c->hidden_norm, (size_t)T * c->d);
     sb_parts_register(c, 1, c->dlogits, (size_t)T * c->V);
+    sb_parts_register(c, 1, c->g_hidden, (size_t)T * c->d);
     sb_parts_register(c, 1, c->g_q, (size_t)T * c->qd); sb_parts_register(c, 1, c->g_k, (size_t)T * c->kvd); sb_parts_register(c, 1, c->g_v, (size_t)T * c->kvd);
     sb_parts_register(c, 1, c->g_gate, (size_t)T * c->F); sb_parts_register(c, 1, c->g_up, (size_t)T * c->F);      /* written as parts by the SwiGLU backward */
     return 0;
@@ -791,7 +792,7 @@ static void prepare_weights(sb_ctx_t* c, int T) {
     if (k) sb_parts_prepare(c, x, n, k);
 }
 
-static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_lora) {
+static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_lora, int train) {
     const int d = c->d, F = c->F, qd = c->qd, kvd = c->kvd, L = c->L;
     const size_t Td = (size_t)T * d;
     /* producers that may write an operand only as FP16 parts: every product that reads it must take parts */
@@ -814,10 +815,11 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
         const sb_layer_off_t* o = &c->off[l];
         sb_layer_act_t* a = &c->act[l];
         float* next_in = (l + 1 < L) ? c->act[l + 1].layer_in : c->final_in;
+        a->inv_attn = train ? sb_zero_word(c) : NULL; a->inv_ffn = train ? sb_zero_word(c) : NULL;
         /* the norms also write the rows they read to where the residual stream goes on: the o and down projections add into that copy */
-        if (!(xa_parts && sb_rmsnorm_parts(c, a->layer_in, c->W + o->in_norm, a->x_norm_attn, a->post_attn_in, T, d, RMS_EPS))) {
+        if (!(xa_parts && sb_rmsnorm_parts(c, a->layer_in, c->W + o->in_norm, a->x_norm_attn, a->post_attn_in, T, d, RMS_EPS, &a->inv_attn))) {
             sb_amax_announce(c, a->x_norm_attn, Td);       /* producers of GEMM operands leave max |x| behind for the operand split */
-            sb_rmsnorm_copy(c, a->layer_in, c->W + o->in_norm, a->x_norm_attn, a->post_attn_in, T, d, RMS_EPS);
+            sb_rmsnorm_copy(c, a->layer_in, c->W + o->in_norm, a->x_norm_attn, a->post_attn_in, T, d, RMS_EPS, &a->inv_attn);
         }
         /* runs of products that share an operand keep its prepared parts (the adapters' scratch, rewritten in between, is dropped from the kept set at every write) */
         sb_gemm_keep_begin(c);
@@ -857,9 +859,9 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
         sb_attention(c, a->q, a->k, a->v, a->attn_out, a->lse, c->seq_starts, c->seq_ids, T, c->Hq, c->Hkv, c->hd);
         if (use_lora && c->lora_grouped) { const proj_t p = {3, c->W + o->o, a->post_attn_in, d, 1}; sb_gemm_keep_begin(c); lora_fwd_group(c, l, a->attn_out, &p, 1, T, qd); sb_gemm_keep_end(c); }
         else linear_fwd(c, use_lora, l, 3, a->attn_out, c->W + o->o, a->post_attn_in, T, qd, d, 1);
-        if (!(xf_parts && sb_rmsnorm_parts(c, a->post_attn_in, c->W + o->post_norm, a->x_norm_ffn, next_in, T, d, RMS_EPS))) {
+        if (!(xf_parts && sb_rmsnorm_parts(c, a->post_attn_in, c->W + o->post_norm, a->x_norm_ffn, next_in, T, d, RMS_EPS, &a->inv_ffn))) {
             sb_amax_announce(c, a->x_norm_ffn, Td);
-            sb_rmsnorm_copy(c, a->post_attn_in, c->W + o->post_norm, a->x_norm_ffn, next_in, T, d, RMS_EPS);
+            sb_rmsnorm_copy(c, a->post_attn_in, c->W + o->post_norm, a->x_norm_ffn, next_in, T, d, RMS_EPS, &a->inv_ffn);
         }
         sb_gemm_keep_begin(c);
         sb_amax_announce(c, a->gate, (size_t)T * F);        /* the products' epilogues leave max |gate|, max |up| for the bound below */
@@ -885,9 +887,10 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
         else linear_fwd(c, use_lora, l, 6, a->ffn_hidden, c->W + o->down, next_in, T, F, d, 1);
         nan_mark(c, next_in, Td, nan_fwd_base(c) + (uint32_t)l);
     }
-    if (!(hn_parts && sb_rmsnorm_parts(c, c->final_in, c->W + (size_t)c->V * d, c->hidden_norm, NULL, T, d, RMS_EPS))) {
+    c->final_inv = train ? sb_zero_word(c) : NULL;
+    if (!(hn_parts && sb_rmsnorm_parts(c, c->final_in, c->W + (size_t)c->V * d, c->hidden_norm, NULL, T, d, RMS_EPS, &c->final_inv))) {
         sb_amax_announce(c, c->hidden_norm, Td);
-        sb_rmsnorm(c, c->final_in, c->W + (size_t)c->V * d, c->hidden_norm, T, d, RMS_EPS);
+        sb_rmsnorm_copy(c, c->final_in, c->W + (size_t)c->V * d, c->hidden_norm, NULL, T, d, RMS_EPS, &c->final_inv);
     }
     nan_mark(c, c->hidden_norm, Td, 2); nan_mark(c, c->final_in, Td, 6);
     sb_gemm(c, c->hidden_norm, c->untied ? c->XW + extras_lm_off(c) : c->W, c->logits, T, c->V, d, 0, 1, 0);       /* tied LM head, or the separate one */
@@ -910,6 +913,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
     const size_t sms = (size_t)(c->pub.gpu_sm_count > 0 ? c->pub.gpu_sm_count : 148);
     sb_colsum_defer(c, full && !reduce, store, sms * ((size_t)(2 * L + 1) * 2 * ((size_t)d + 32) + (c->head_norm ? (size_t)2 * L * 4 * ((size_t)c->hd + 32) : 0)));
     sb_gemm_keep_begin(c);
+    sb_amax_announce(c, gx, (size_t)T * d);       /* the norms' backward bounds its result with max |gx| */
     {
         const sb_gemm_job_t jobs[2] = {{c->dlogits, c->untied ? c->XW + extras_lm_off(c) : c->W, gx, T, d, V, 0, 0, 0},
                                        {c->dlogits, c->hidden_norm, c->untied ? c->XG + extras_lm_off(c) : Gd, V, d, T, 1, 0, add}};
@@ -917,8 +921,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
     }
     sb_gemm_keep_end(c);
     nan_mark(c, c->dlogits, (size_t)T * V, 3); nan_mark(c, gx, (size_t)T * d, 4);
-    sb_amax_announce(c, gh, (size_t)T * d);
-    sb_rmsnorm_backward(c, c->final_in, c->W + (size_t)V * d, gx, NULL, gh, full ? Gd + (size_t)V * d : norm_sink, T, d, RMS_EPS);
+    sb_rmsnorm_backward_parts(c, c->final_in, c->W + (size_t)V * d, gx, NULL, gh, full ? Gd + (size_t)V * d : norm_sink, T, d, RMS_EPS, c->final_inv, &c->ghid_amax);
     nan_mark(c, gh, (size_t)T * d, 5); nan_mark(c, gh, (size_t)T * d, 0);
     const int ffn_lora = !full && (c->lora_mask & 0x70);
     const int ffn_parts_bwd = !c->nan_on && !ffn_lora && sb_gemm_reads_f16_parts(c, T, d, F, 0, 0) && (!full || sb_gemm_reads_f16_parts(c, F, d, T, 1, 0));
@@ -946,6 +949,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
             sb_swiglu_backward(c, a->gate, a->up, c->g_ffn, c->g_gate, c->g_up, (size_t)T * F);
         }
         sb_gemm_keep_begin(c);
+        sb_amax_announce(c, gx, (size_t)T * d);
         if (grouped) {
             const int ads[2] = {4, 5}; const float *dy[2] = {c->g_gate, c->g_up}, *w[2] = {c->W + o->gate, c->W + o->up};
             lora_bwd_group(c, l, ads, dy, w, 2, a->x_norm_ffn, gx, T, d);
@@ -956,8 +960,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
         }
         if (!full && !grouped) { lora_bwd(c, l, 4, c->g_gate, a->x_norm_ffn, gx, T); lora_bwd(c, l, 5, c->g_up, a->x_norm_ffn, gx, T); }
         sb_gemm_keep_end(c);
-        sb_amax_announce(c, gh, (size_t)T * d);
-        sb_rmsnorm_backward(c, a->post_attn_in, c->W + o->post_norm, gx, gh, gh, full ? Gd + o->post_norm : norm_sink, T, d, RMS_EPS);
+        sb_rmsnorm_backward_parts(c, a->post_attn_in, c->W + o->post_norm, gx, gh, gh, full ? Gd + o->post_norm : norm_sink, T, d, RMS_EPS, a->inv_ffn, &c->ghid_amax);
         /* attention */
         sb_gemm_keep_begin(c);
         if (grouped) {
@@ -997,6 +1000,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
             gq = c->g_q2; gk = c->g_k2;
         }
         sb_gemm_keep_begin(c);
+        sb_amax_announce(c, gx, (size_t)T * d);
         const int last = grouped && !c->nan_on && l == 0;      /* nothing below the first layer's projections is trained: their input gradient is not formed */
         if (grouped) {
             const int ads[3] = {0, 1, 2}; const float *dy[3] = {gq, gk, c->g_v}, *w[3] = {c->W + o->q, c->W + o->k, c->W + o->v};
@@ -1010,8 +1014,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
         if (!full && !grouped) { lora_bwd(c, l, 0, gq, a->x_norm_attn, gx, T); lora_bwd(c, l, 1, gk, a->x_norm_attn, gx, T); lora_bwd(c, l, 2, c->g_v, a->x_norm_attn, gx, T); }
         sb_gemm_keep_end(c);
         if (!last) {
-            sb_amax_announce(c, gh, (size_t)T * d);
-            sb_rmsnorm_backward(c, a->layer_in, c->W + o->in_norm, gx, gh, gh, full ? Gd + o->in_norm : norm_sink, T, d, RMS_EPS);
+            sb_rmsnorm_backward_parts(c, a->layer_in, c->W + o->in_norm, gx, gh, gh, full ? Gd + o->in_norm : norm_sink, T, d, RMS_EPS, a->inv_attn, &c->ghid_amax);
         }
     layer_done:
         nan_mark(c, gh, (size_t)T * d, nan_ghid_base(c) + (uint32_t)l);
@@ -1135,7 +1138,7 @@ static float step_body(train_state_t* st, int* tokens, int T, int* seq_starts, i
         else { sb_memset(c, c->LG, 0, c->n_lora * sizeof(float)); if (c->LGp != c->LG) sb_memset(c, c->LGp, 0, c->n_lora_pad * sizeof(float)); }
         if (full && c->XG && !store) sb_memset(c, c->XG, 0, c->n_extras * sizeof(float));
     }
-    forward_pass(c, T, max_seq, theta, use_lora);
+    forward_pass(c, T, max_seq, theta, use_lora, train);
     /* training: the gradient of the logits leaves the loss kernel as the FP16 parts the two LM-head backward products read (its
        FP32 form is never written); evaluation, the NaN guard (which inspects the FP32 array) and contexts without the parts arena
        take the plain kernel */
