@@ -311,6 +311,10 @@ __global__ void __launch_bounds__(RB_THREADS, 2) rmsnorm_bwd_rows_kernel(const f
         const int j = threadIdx.x + RB_THREADS * i;
         sc[i] = j < c4 ? ((const float4*)w)[j] : acc[i];
     }
+    const int ngroups = (rows + ROWS - 1) / ROWS, stride = gridDim.x;
+    RnbSet<NC, ROWS> a, b;
+    int gidx = blockIdx.x;
+    if (gidx < ngroups) rnb_load<NC, ROWS>(a, x, dy, resid, gidx * ROWS, rows, c4);
     float osc = 1.f;
     if (out.bound) {
         float wm = 0.f;
@@ -324,10 +328,6 @@ __global__ void __launch_bounds__(RB_THREADS, 2) rmsnorm_bwd_rows_kernel(const f
         osc = sb_pow2(sb_f16_shift(bound));
         if (blockIdx.x == 0 && threadIdx.x == 0) *out.bound = bound;
     }
-    const int ngroups = (rows + ROWS - 1) / ROWS, stride = gridDim.x;
-    RnbSet<NC, ROWS> a, b;
-    int gidx = blockIdx.x;
-    if (gidx < ngroups) rnb_load<NC, ROWS>(a, x, dy, resid, gidx * ROWS, rows, c4);
     while (gidx < ngroups) {
         if (gidx + stride < ngroups) rnb_load<NC, ROWS>(b, x, dy, resid, (gidx + stride) * ROWS, rows, c4);
         rnb_compute<NC, ROWS>(a, sc, w, acc, dx, gidx * ROWS, rows, cols, c4, eps, s_red[0], s_tot[0], am, out, osc);
@@ -464,6 +464,77 @@ __global__ void __launch_bounds__(RB_THREADS) softmax_kernel(const float* __rest
 // row because it overwrites x.  One warp per row, the row in registers (cols % 4 == 0, cols <= 128 * NV): 8 bytes
 // per element forward, 12 backward.  Other shapes: one CTA per row.
 // ---------------------------------------------------------------------------
+// RMSNorm of rows of 1028 to 4096 columns: a CTA per row, NC vectors of it per thread, the next row's loads in flight during this row's sum.  (A warp
+// per row needs 64 to 128 registers for the row alone, one or two CTAs per SM: 2.0 to 3.3 TB/s at 2048 and 4096 columns.)  The row leaves as FP32
+// (y) or as FP16 operand parts under the bound that rmsnorm_warp_parts_kernel explains; copy, inv_max and amax_out as there.
+template <int NC>
+__global__ void __launch_bounds__(RB_THREADS, 4) rmsnorm_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y,
+                                                                     uint2* __restrict__ h1, uint2* __restrict__ h2, float* __restrict__ copy, int rows, int cols, float eps,
+                                                                     float* bound_out, unsigned keep, unsigned* inv_max, unsigned* amax_out) {
+    sb_pdl_enter();
+    __shared__ float red[2][RB_THREADS / 32], s_w[RB_THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c4 = cols >> 2;
+    float4 s[NC], v[NC], nx[NC];
+    int r = blockIdx.x;
+#pragma unroll
+    for (int i = 0; i < NC; i++) {
+        const int j = threadIdx.x + RB_THREADS * i;
+        s[i] = j < c4 ? ((const float4*)w)[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[i] = j < c4 && r < rows ? ((const float4*)x)[(size_t)r * c4 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float sc = 1.f, im = 0.f, am = 0.f;
+    if (bound_out) {
+        float wm = 0.f;
+#pragma unroll
+        for (int i = 0; i < NC; i++) wm = sb_amax4(wm, s[i]);
+        wm = warp_max(wm);
+        if (lane == 0) s_w[warp] = wm;
+        __syncthreads();
+        wm = warp_max(s_w[threadIdx.x & (RB_THREADS / 32 - 1)]);
+        const float bound = fminf(sqrtf((float)cols) * wm * 1.0001f, 3.0e38f);
+        sc = sb_pow2(sb_f16_shift(bound));
+        if (blockIdx.x == 0 && threadIdx.x == 0) *bound_out = bound;
+    }
+    for (int it = 0; r < rows; r += gridDim.x, it++) {
+        const int rn = r + gridDim.x;
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < NC; i++) {
+            const int j = threadIdx.x + RB_THREADS * i;
+            if (j < c4 && rn < rows) nx[i] = ((const float4*)x)[(size_t)rn * c4 + j];
+            ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+        }
+        ss = warp_sum(ss);
+        if (lane == 0) red[it & 1][warp] = ss;
+        __syncthreads();                        // the other half of red is written next: one barrier a row is enough
+        ss = red[it & 1][0];
+#pragma unroll
+        for (int k = 1; k < RB_THREADS / 32; k++) ss += red[it & 1][k];
+        const float inv = 1.0f / sqrtf(ss / cols + eps);
+        im = fmaxf(im, inv);
+#pragma unroll
+        for (int i = 0; i < NC; i++) {
+            const int j = threadIdx.x + RB_THREADS * i;
+            if (j < c4) {
+                const size_t o = (size_t)r * c4 + j;
+                if (copy) ((float4*)copy)[o] = v[i];
+                const float4 q = make_float4(v[i].x * inv * s[i].x, v[i].y * inv * s[i].y, v[i].z * inv * s[i].z, v[i].w * inv * s[i].w);
+                if (h1) {
+                    uint2 a, b;
+                    sb_split2(q.x * sc, q.y * sc, a.x, b.x, keep); sb_split2(q.z * sc, q.w * sc, a.y, b.y, keep);
+                    h1[o] = a; h2[o] = b;
+                } else {
+                    ((float4*)y)[o] = q;
+                    am = sb_amax4(am, q);
+                }
+                v[i] = nx[i];
+            }
+        }
+    }
+    if (inv_max && threadIdx.x == 0 && im > 0.f) atomicMax(inv_max, __float_as_uint(im));
+    sb_block_amax(am, amax_out);
+}
+
 // The same rows with y written only as FP16 operand parts: every |y_i| = |x_i| rstd |w_i| is at most sqrt(cols) max|w| (x_i^2 cannot
 // exceed the row's sum of squares), so that bound sets the scale and no pass over y looks for its maximum or splits it again.
 template <int NV>
@@ -1013,8 +1084,11 @@ void sb_rmsnorm_copy(sb_ctx_t* c, const float* x, const float* w, float* y, floa
         } else
         if (cols <= 512)       sb_launch(rmsnorm_warp_kernel<4>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am, (unsigned*)inv_max);
         else if (cols <= 1024) sb_launch(rmsnorm_warp_kernel<8>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am, (unsigned*)inv_max);
-        else if (cols <= 2048) sb_launch(rmsnorm_warp_kernel<16>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am, (unsigned*)inv_max);
-        else                   sb_launch(rmsnorm_warp_kernel<32>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y, copy, rows, cols, eps, am, (unsigned*)inv_max);
+        else {
+            const int g = rows < 4 * sm_count(c) ? rows : 4 * sm_count(c);
+            if (cols <= 2048) sb_launch(rmsnorm_rows_kernel<2>, dim3(g), dim3(RB_THREADS), 0, st, x, w, y, nullptr, nullptr, copy, rows, cols, eps, nullptr, 0u, (unsigned*)inv_max, am);
+            else              sb_launch(rmsnorm_rows_kernel<4>, dim3(g), dim3(RB_THREADS), 0, st, x, w, y, nullptr, nullptr, copy, rows, cols, eps, nullptr, 0u, (unsigned*)inv_max, am);
+        }
     } else {
     if (inv_word) *inv_word = NULL;
     sb_launch(rmsnorm_kernel, dim3(grid), dim3(RB_THREADS), 0, (cudaStream_t)c->pub.stream, x, w, y, rows, cols, eps, vec);
@@ -1039,8 +1113,11 @@ int sb_rmsnorm_parts(sb_ctx_t* c, const float* x, const float* w, float* y, floa
     int tk = sb_tick_begin(c, SB_CLS_NORM_FWD);
     if (cols <= 512)       sb_launch(rmsnorm_warp_parts_kernel<4>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y32, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy, (unsigned*)inv_max);
     else if (cols <= 1024) sb_launch(rmsnorm_warp_parts_kernel<8>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y32, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy, (unsigned*)inv_max);
-    else if (cols <= 2048) sb_launch(rmsnorm_warp_parts_kernel<16>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y32, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy, (unsigned*)inv_max);
-    else                   sb_launch(rmsnorm_warp_parts_kernel<32>, dim3(wgrid), dim3(RB_THREADS), 0, st, x, w, y32, h1, h2, rows, cols, eps, bound, sb_parts_keep(c), copy, (unsigned*)inv_max);
+    else {
+        const int g = rows < 4 * sm_count(c) ? rows : 4 * sm_count(c);
+        if (cols <= 2048) sb_launch(rmsnorm_rows_kernel<2>, dim3(g), dim3(RB_THREADS), 0, st, x, w, y32, h ? h1 : nullptr, h2, copy, rows, cols, eps, bound, sb_parts_keep(c), (unsigned*)inv_max, nullptr);
+        else              sb_launch(rmsnorm_rows_kernel<4>, dim3(g), dim3(RB_THREADS), 0, st, x, w, y32, h ? h1 : nullptr, h2, copy, rows, cols, eps, bound, sb_parts_keep(c), (unsigned*)inv_max, nullptr);
+    }
     sb_tick_end(c, tk, 0.0, (copy ? 12.0 : 8.0) * rows * cols);
     c->launches++;
     return 1;

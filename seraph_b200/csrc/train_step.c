@@ -796,13 +796,13 @@ static void forward_pass(sb_ctx_t* c, int T, int max_seq, float theta, int use_l
     const int d = c->d, F = c->F, qd = c->qd, kvd = c->kvd, L = c->L;
     const size_t Td = (size_t)T * d;
     /* producers that may write an operand only as FP16 parts: every product that reads it must take parts */
-    const int ffn_lora = use_lora && (c->lora_mask & 0x70);
+    const int ffn_lora = use_lora && !c->lora_grouped && (c->lora_mask & 0x70);
     const int ffn_parts = !c->nan_on && !ffn_lora && sb_gemm_reads_f16_parts(c, T, d, F, 0, 1) && sb_gemm_reads_f16_parts(c, d, F, T, 1, 0);
-    /* the normalised rows are read by the projections and by their weight gradients only (adapters read them too: FP32 stays then) */
-    const int xa_parts = !c->nan_on && !(use_lora && (c->lora_mask & 0x07)) &&
+    /* the normalised rows are read by the projections and by their weight gradients only (adapters read them too: FP32 stays unless their products run in groups) */
+    const int xa_parts = !c->nan_on && !(use_lora && !c->lora_grouped && (c->lora_mask & 0x07)) &&
                          sb_gemm_reads_f16_parts(c, T, qd, d, 0, 1) && sb_gemm_reads_f16_parts(c, T, kvd, d, 0, 1) &&
                          sb_gemm_reads_f16_parts(c, qd, d, T, 1, 0) && sb_gemm_reads_f16_parts(c, kvd, d, T, 1, 0);
-    const int xf_parts = !c->nan_on && !(use_lora && (c->lora_mask & 0x30)) &&
+    const int xf_parts = !c->nan_on && !(use_lora && !c->lora_grouped && (c->lora_mask & 0x30)) &&
                          sb_gemm_reads_f16_parts(c, T, F, d, 0, 1) && sb_gemm_reads_f16_parts(c, F, d, T, 1, 0);
     /* q and k leave the rotation as the parts that attention reads (the row-wise qk_norm comes after it and keeps the plain pass) */
     const int rope_parts = !c->qk_norm && sb_attention_reads_parts(c, c->Hq, c->Hkv, c->hd);
@@ -923,7 +923,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
     nan_mark(c, c->dlogits, (size_t)T * V, 3); nan_mark(c, gx, (size_t)T * d, 4);
     sb_rmsnorm_backward_parts(c, c->final_in, c->W + (size_t)V * d, gx, NULL, gh, full ? Gd + (size_t)V * d : norm_sink, T, d, RMS_EPS, c->final_inv, &c->ghid_amax);
     nan_mark(c, gh, (size_t)T * d, 5); nan_mark(c, gh, (size_t)T * d, 0);
-    const int ffn_lora = !full && (c->lora_mask & 0x70);
+    const int ffn_lora = !full && !grouped && (c->lora_mask & 0x70);
     const int ffn_parts_bwd = !c->nan_on && !ffn_lora && sb_gemm_reads_f16_parts(c, T, d, F, 0, 0) && (!full || sb_gemm_reads_f16_parts(c, F, d, T, 1, 0));
     /* 64-wide heads: the gradients of q, k and v leave the backward rotation as parts only (the attention kernels leave their maxima) */
     const int rope_parts = !c->nan_on && !c->qk_norm && !c->head_norm && c->hd == 64 && sb_attention_reads_parts(c, c->Hq, c->Hkv, c->hd) &&
