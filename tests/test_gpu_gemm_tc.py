@@ -53,6 +53,25 @@ def test_tc_gemm_matches_oracle(ctx, M, N, K, tA, tB, acc, mode, pair):
     ctx.release(a, b, c)
 
 
+@pytest.mark.parametrize("tA,tB,acc", [(0, 1, 0), (0, 0, 1), (1, 0, 0), (1, 0, 1)])
+@pytest.mark.parametrize("M,N,K", [(8, 512, 1024), (61, 1408, 512), (264, 136, 72), (256, 128, 64), (512, 264, 1000), (2056, 8, 4096), (24, 16, 8192)])
+def test_grouped_kernel_at_tile_edges(ctx, M, N, K, tA, tB, acc):
+    """The persistent kernel of grouped products from eight rows or columns up: single and partial tiles of 256, a short last block of k, tiles cut
+    along k."""
+    r = np.random.default_rng(M + N + K)
+    A = r.standard_normal((K, M) if tA else (M, K)).astype(np.float32)
+    B = r.standard_normal((N, K) if tB else (K, N)).astype(np.float32)
+    C0 = r.standard_normal((M, N)).astype(np.float32)
+    ref = C0.copy()
+    O.lib().ref_matmul(A, B, ref, M, N, K, tA, tB, acc)
+    a, b, c = ctx.upload(A), ctx.upload(B), ctx.upload(C0)
+    ctx.lib.cuda_train_matmul_transpose(ctx.h, a.b, b.b, c.b, M, N, K, tA, tB, acc)
+    out = c.numpy(shape=(M, N))
+    ctx.check()
+    assert rel_l2(out, ref) < BOUND[4], rel_l2(out, ref)
+    ctx.release(a, b, c)
+
+
 def test_tc_gemm_long_k_and_reproducible(ctx):
     """K = 16384 (longer than the 8192-token reduction of the weight gradients): accumulation error stays in bound."""
     M, N, K = 256, 512, 16384

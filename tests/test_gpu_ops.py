@@ -89,6 +89,12 @@ def test_rmsnorm_forward_backward(ctx, rows, cols):
     ctx.release(bx, bw, bdy, by, bdx, bds, bds2)
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 1028), (700, 2048), (3, 3000), (700, 4096), (40, 4100)])
+def test_rmsnorm_wide_rows(ctx, rows, cols):
+    """A CTA per row up to 4096 columns (two or four vectors per thread), the general kernels beyond."""
+    test_rmsnorm_forward_backward(ctx, rows, cols)
+
+
 @pytest.mark.parametrize("n", [1, 5, 4096, 100003])
 def test_elementwise(ctx, n):
     r = rng(n)
@@ -329,6 +335,22 @@ def test_cross_entropy_packed(ctx, V):
     ctx.lib.cuda_train_reduce_sum(ctx.h, br.b, bsum.b, T)
     assert abs(bsum.numpy()[0] - O.lib().ref_reduce_sum(rows_ref, T)) < 1e-4
     ctx.release(bl, bt, bg, br, bs, bsum)
+
+
+@pytest.mark.parametrize("T,V", [(24, 1004), (24, 131076), (200, 8192), (200, 16388), (200, 32768), (200, 32772)])
+def test_cross_entropy_row_in_shared_memory(ctx, T, V):
+    """Rows held by one CTA, by clusters of two (long rows) and eight (few rows), and rows that are too long for that."""
+    ss = np.array([0, 7, T - 5, T], np.uint32)
+    r = rng(V + T)
+    logits = f32(3 * r.standard_normal((T, V)))
+    tgt = r.integers(0, V, T).astype(np.uint32)
+    g_ref, rows_ref = np.empty_like(logits), np.empty(T, np.float32)
+    O.lib().ref_cross_entropy_grad(logits, tgt, g_ref, rows_ref, ss, T, 3, V, T - 3)
+    bl, bt, bg, br, bs = ctx.upload(logits), ctx.upload(tgt), ctx.empty(logits.size), ctx.empty(T), ctx.upload(ss)
+    ctx.lib.cuda_train_cross_entropy_grad_packed(ctx.h, bl.b, bt.b, bg.b, br.b, bs.b, T, 3, V, T - 3)
+    ctx.check()
+    assert rel_l2(bg.numpy(), g_ref) < TOL and rel_l2(br.numpy(), rows_ref) < TOL
+    ctx.release(bl, bt, bg, br, bs)
 
 
 @pytest.mark.parametrize("T,d,V,mode", [(24, 64, 257, "uniform"), (3000, 96, 500, "uniform"), (2048, 512, 8192, "uniform"),

@@ -386,6 +386,35 @@ def test_c1_lora_step_on_tensor_cores_matches_oracle(ctx):
     assert outs[0][0] == outs[1][0] and np.array_equal(outs[0][1], outs[1][1])
 
 
+@pytest.mark.parametrize("rank,mask,exact", [(4, 0x7F, 1), (8, 0x05, 0), (20, 0x7F, 0)])
+def test_lora_step_with_grouped_adapters(ctx, rank, mask, exact):
+    """Adapters whose products run in groups with the projections: ranks below, at and between multiples of eight, over two steps (the second reads
+    the adapters that the first has moved)."""
+    from seraph_b200 import api
+    cfg = O.ModelCfg(V=512, d=256, L=2, Hq=4, Hkv=2, hd=64, F=512)
+    p = cfg.init_params(41)
+    tens, n = cfg.lora_tensors(rank, mask)
+    lo = (0.02 * np.random.default_rng(42).standard_normal(n)).astype(np.float32)
+    ss = [0, 300, 431, 1000]
+    tok = tokens_for(cfg, 1000, 43)
+    st = api.TrainState(cfg, p, lr=1e-2)
+    st.attach_lora(rank, 2.0 * rank, mask, lo)
+    assert ctx.lib.seraph_b200_set_lora_exact(ctx.h, exact) == 0
+    for _ in range(2):
+        ref = O.train_step(cfg, p, tok, ss, lora=lo, rank=rank, alpha=2.0 * rank, mask=mask, lora_exact=exact)
+        loss = api.step_lora_batch(ctx, st, tok, ss)
+        ctx.check()
+        ctx.lib.cuda_download_lora_weights(ctx.h, st.lora_ptr())
+        g = st.lora_get(1)
+        assert abs(loss - ref["loss"]) < 1e-5 * abs(ref["loss"])
+        for name, shp, off in tens:
+            k = int(np.prod(shp))
+            assert rel_l2(g[off:off + k], ref["grads"][off:off + k]) < TOL, name
+        lo = st.lora_get(0).copy()
+    assert ctx.lib.seraph_b200_set_lora_exact(ctx.h, 0) == 0
+    st.close()
+
+
 def test_operand_parts_kept_within_a_step_change_nothing(ctx):
     """The FP16 parts of weights and saved activations are made once per call and shared by the call's products, and the SwiGLU
     kernels write their outputs straight into that arena (scaled by a bound instead of the exact maximum, so those operands
