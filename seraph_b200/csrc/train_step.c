@@ -1028,7 +1028,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
     sb_colsum_defer(c, 0, 0, 0);
     if (full) {
         nan_mark(c, gh, (size_t)T * d, 8);
-        sb_embedding_backward(c, c->tokens, gh, Gd, T, d, V);
+        sb_embedding_backward_step(c, c->tokens, gh, Gd, T, d, V);
         nan_mark(c, Gd, (size_t)V * d, 9);
     }
     /* Every layer's gradients are with the all-reduce.  The last bucket (embedding with the LM head's share, and the final norm:

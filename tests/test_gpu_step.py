@@ -386,6 +386,18 @@ def test_c1_lora_step_on_tensor_cores_matches_oracle(ctx):
     assert outs[0][0] == outs[1][0] and np.array_equal(outs[0][1], outs[1][1])
 
 
+@pytest.mark.parametrize("ids,ss", [([2, 9, 100], [0, 7]), ([0, 5, 511], [0, 300, 431, 1030]), (None, [0, 2, 513])])
+def test_step_with_repeated_tokens(ctx, ids, ss):
+    """The embedding gradient of a step sums the rows of equal ids: a handful of tokens, long runs of a few, and mostly different ones."""
+    cfg = O.ModelCfg(V=512, d=128, L=1, Hq=2, Hkv=1, hd=64, F=256)
+    p = cfg.init_params(51, norm_jitter=0.1)
+    tok = tokens_for(cfg, ss[-1], 52) if ids is None else np.random.default_rng(53).choice(np.array(ids, np.int32), ss[-1])
+    ref = O.train_step(cfg, p, tok, ss)
+    got = run_full_step(ctx, cfg, p, tok, ss)
+    assert abs(got["loss"][0] - ref["loss"]) < 1e-5 * abs(ref["loss"])
+    check_grads(cfg, got["grads"], ref["grads"])
+
+
 @pytest.mark.parametrize("rank,mask,exact", [(4, 0x7F, 1), (8, 0x05, 0), (20, 0x7F, 0)])
 def test_lora_step_with_grouped_adapters(ctx, rank, mask, exact):
     """Adapters whose products run in groups with the projections: ranks below, at and between multiples of eight, over two steps (the second reads
