@@ -89,9 +89,9 @@ def test_rmsnorm_forward_backward(ctx, rows, cols):
     ctx.release(bx, bw, bdy, by, bdx, bds, bds2)
 
 
-@pytest.mark.parametrize("rows,cols", [(1, 1028), (700, 2048), (3, 3000), (700, 4096), (40, 4100)])
-def test_rmsnorm_wide_rows(ctx, rows, cols):
-    """A CTA per row up to 4096 columns (two or four vectors per thread), the general kernels beyond."""
+@pytest.mark.parametrize("rows,cols", [(700, 480), (511, 512), (512, 512), (1, 1028), (700, 2048), (3, 3000), (700, 4096), (40, 4100)])
+def test_rmsnorm_row_kernels(ctx, rows, cols):
+    """A warp per row up to 512 columns (backward), a CTA per row up to 4096 (two or four vectors per thread), the general kernels beyond."""
     test_rmsnorm_forward_backward(ctx, rows, cols)
 
 
