@@ -567,7 +567,7 @@ static int gg_operand(sb_ctx_t* c, GgOperand* ops, int* nops, const float* x, si
     GgOperand* o = &ops[*nops];
     o->x = x; o->n = n; o->slot = -1; o->kept = false;
     void* h; int fresh;
-    if (sb_parts_find(c, x, n, &h, &o->amax, &fresh)) { o->h = (__half*)h; o->fresh = fresh != 0; }
+    if (sb_parts_find(c, x, n, &h, &o->amax, &fresh)) { o->h = (__half*)h; o->fresh = fresh != 0; o->kept = fresh == SB_PARTS_MAKE_KEPT; }
     else {
         bool fr;
         const int s = sb_f16_slot(c, x, n, -1, &fr);
@@ -591,7 +591,7 @@ static void gg_prepare(sb_ctx_t* c, GgOperand* ops, int n) {
         GgOperand* o = &ops[i];
         if (o->fresh) {
             if (!any) { tk = sb_tick_begin(c, SB_CLS_GEMM_PREP); any = true; }
-            float* left = sb_amax_lookup(c, o->x, o->n);
+            float* left = o->kept ? NULL : sb_amax_lookup(c, o->x, o->n);
             if (left) {
                 o->amax = left;
                 if (o->slot >= 0) c->f16_slot[o->slot].amax = left; else sb_parts_set_amax(c, o->x, left);

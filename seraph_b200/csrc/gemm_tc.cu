@@ -158,7 +158,10 @@ extern "C" void sb_parts_open(sb_ctx_t* c) {
     }
     if (c->hint_pool) cudaMemsetAsync(c->hint_pool, 0, SB_HINT_CAP * sizeof(float), (cudaStream_t)c->pub.stream);
 }
-extern "C" void sb_parts_close(sb_ctx_t* c) { c->parts_gen++; c->parts_open = 0; c->hint_n = 0; c->hint_npending = 0; }
+extern "C" void sb_parts_close(sb_ctx_t* c) {
+    c->parts_gen++; c->parts_open = 0; c->hint_n = 0; c->hint_npending = 0;
+    if (c->status != SB_OK) c->weights_gen++;                         // a launch may be missing: parts that were looked up need not have been made
+}
 extern "C" void sb_amax_announce(sb_ctx_t* c, const float* out, size_t n) {
     if (!c->parts_open || !c->hint_pool) return;
     if (c->hint_npending >= SB_HINT_PENDING) {         // announcements nobody took (a launcher without the feature): the oldest goes
@@ -236,7 +239,7 @@ extern "C" int sb_parts_find(sb_ctx_t* c, const float* x, size_t n, void** hout,
     *hout = (__half*)c->parts_arena + e->off;
     // weights that nothing changes between calls (the frozen base of adapter training; any model inside one evaluation) keep their parts
     const unsigned gen = e->kind == 0 && c->weights_fixed ? 0x80000000u | (c->weights_gen << 1) | (sb_parts_keep(c) == 0xffffffffu ? 0u : 1u) : c->parts_gen & 0x7fffffffu;
-    *fresh = e->gen != gen || e->cur != n;
+    *fresh = e->gen == gen && e->cur == n ? 0 : gen & 0x80000000u ? SB_PARTS_MAKE_KEPT : SB_PARTS_MAKE;
     if (*fresh) e->amax_ptr = c->parts_amax + idx;
     *amax = e->amax_ptr;
     e->gen = gen; e->cur = n;

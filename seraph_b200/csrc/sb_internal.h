@@ -239,7 +239,10 @@ float* sb_amax_lookup(sb_ctx_t*, const float* x, size_t n);
 int sb_bound_out(sb_ctx_t*, const float* x, size_t n, void** parts, float** word);
 float* sb_zero_word(sb_ctx_t*);      /* a device word that is zero until the step ends; NULL outside a step */
 void sb_parts_set_amax(sb_ctx_t*, const float* x, float* word);
-/* 1: x[n] is registered and the step is open; *h = its two parts (h, h + n), *amax its scale word, *fresh = parts must be made now */
+/* 1: x[n] is registered and the step is open; *h = its two parts (h, h + n), *amax its scale word, *fresh: 0 when they hold x, else they must be
+   made now.  Parts that outlive the step (SB_PARTS_MAKE_KEPT) take *amax as it is: a word of the step's pool (sb_zero_word, sb_amax_lookup) is
+   another tensor's in the next step. */
+enum { SB_PARTS_MAKE = 1, SB_PARTS_MAKE_KEPT = 2 };
 int sb_parts_find(sb_ctx_t*, const float* x, size_t n, void** h, float** amax, int* fresh);
 void sb_parts_invalidate(sb_ctx_t*, const float* x);      /* x is rewritten as plain FP32: parts held for it are stale */
 int  sb_rope_parts(sb_ctx_t*, float* q, float* k, const float* v, const uint32_t* pos_ids, int T, int Hq, int Hkv, int hd, float theta, int max_pos, int backward, int f32);

@@ -427,6 +427,56 @@ def test_lora_step_with_grouped_adapters(ctx, rank, mask, exact):
     st.close()
 
 
+FROZEN = [("vocabulary not a multiple of 4", O.ModelCfg(V=515, d=256, L=2, Hq=4, Hkv=2, hd=64, F=512), [0, 300, 431, 640]),
+          ("narrow k and v", O.ModelCfg(V=512, d=256, L=2, Hq=4, Hkv=1, hd=64, F=512), [0, 11, 24])]
+
+
+@pytest.mark.parametrize("name,cfg,ss", FROZEN, ids=[f[0] for f in FROZEN])
+def test_lora_steps_whose_products_are_not_all_grouped(ctx, name, cfg, ss):
+    """One kind of product of the pass (the LM head; k and v) runs outside the grouped launches, so the frozen weights meet their first product without
+    having been prepared together: the parts a later step reads must carry their own scale."""
+    from seraph_b200 import api
+    rank, mask = 8, 0x7F
+    p = cfg.init_params(61)
+    tens, n = cfg.lora_tensors(rank, mask)
+    lo = (0.02 * np.random.default_rng(62).standard_normal(n)).astype(np.float32)
+    tok = tokens_for(cfg, ss[-1], 63)
+    st = api.TrainState(cfg, p, lr=1e-2)
+    st.attach_lora(rank, 2.0 * rank, mask, lo)
+    for step in range(3):
+        ref = O.train_step(cfg, p, tok, ss, lora=lo, rank=rank, alpha=2.0 * rank, mask=mask)
+        loss = api.step_lora_batch(ctx, st, tok, ss)
+        ctx.check()
+        ctx.lib.cuda_download_lora_weights(ctx.h, st.lora_ptr())
+        g = st.lora_get(1)
+        assert abs(loss - ref["loss"]) < 1e-5 * abs(ref["loss"]), (step, loss, ref["loss"])
+        for nm, shp, off in tens:
+            k = int(np.prod(shp))
+            assert rel_l2(g[off:off + k], ref["grads"][off:off + k]) < TOL, (step, nm)
+        lo = st.lora_get(0).copy()
+    st.close()
+
+
+@pytest.mark.parametrize("name,cfg,ss", FROZEN, ids=[f[0] for f in FROZEN])
+def test_evaluate_in_several_passes_whose_products_are_not_all_grouped(ctx, name, cfg, ss):
+    """The passes of one cuda_evaluate share the parts of the weights."""
+    import ctypes as C
+    from seraph_b200 import api
+    p = cfg.init_params(64, norm_jitter=0.1)
+    n = ss[-1]
+    val = tokens_for(cfg, 4 * n, 65)
+    offs = np.arange(0, 4 * n, n, dtype=np.int32)
+    ref = np.mean([O.train_step(cfg, p, np.ascontiguousarray(val[o:o + n]), [0, n])["loss"] for o in offs])
+    st = api.TrainState(cfg, p)
+    ppl = C.c_float(0)
+    assert ctx.lib.seraph_b200_set_eval_batch_tokens(ctx.h, n) == 0          # one sample fills a pass
+    got = ctx.lib.cuda_evaluate(st.h, val.ctypes.data, len(val), offs.ctypes.data, len(offs), n, 0, ctx.h, C.byref(ppl))
+    ctx.check()
+    assert ctx.lib.seraph_b200_set_eval_batch_tokens(ctx.h, 8192) == 0
+    assert abs(got - ref) < 1e-5 * ref, (got, ref)
+    st.close()
+
+
 def test_operand_parts_kept_within_a_step_change_nothing(ctx):
     """The FP16 parts of weights and saved activations are made once per call and shared by the call's products, and the SwiGLU
     kernels write their outputs straight into that arena (scaled by a bound instead of the exact maximum, so those operands
