@@ -1,0 +1,80 @@
+"""What a training step asks of the CUDA runtime besides its kernel launches: calls are counted by a small library that is loaded in front of the
+runtime, in a process of its own."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+SHIM = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stddef.h>
+static void* next(const char* name) { return dlsym(dlopen("libcudart.so.12", RTLD_NOW | RTLD_NOLOAD), name); }
+int n_malloc, n_memset;
+int cudaMalloc(void** p, size_t n) {
+    static int (*f)(void**, size_t);
+    if (!f) f = (int (*)(void**, size_t))next("cudaMalloc");
+    n_malloc++;
+    return f(p, n);
+}
+int cudaMemsetAsync(void* p, int v, size_t n, void* s) {
+    static int (*f)(void*, int, size_t, void*);
+    if (!f) f = (int (*)(void*, int, size_t, void*))next("cudaMemsetAsync");
+    n_memset++;
+    return f(p, v, n, s);
+}
+"""
+
+PRELUDE = """
+import ctypes as C, sys
+import numpy as np
+sys.path.insert(0, %r)
+import oracle_lib as O
+from seraph_b200 import api
+SHIM = C.CDLL(%r)
+def count(name): return C.c_int.in_dll(SHIM, name).value
+def lora_state(ctx, cfg, rank, mask):
+    ctx.lib.seraph_b200_reset_model(ctx.h)
+    st = api.TrainState(cfg, cfg.init_params(1))
+    n = cfg.lora_tensors(rank, mask)[1]
+    st.attach_lora(rank, 2.0 * rank, mask, (0.02 * np.random.default_rng(2).standard_normal(n)).astype(np.float32))
+    return st
+def step(ctx, cfg, st, T):
+    tok = np.random.default_rng(T).integers(0, cfg.V, T).astype(np.int32)
+    before = count("n_malloc"), count("n_memset")
+    assert api.step_lora_batch(ctx, st, tok, [0, T // 3, T]) > 0
+    ctx.check()
+    return count("n_malloc") - before[0], count("n_memset") - before[1]
+cfg = O.ModelCfg(V=512, d=256, L=2, Hq=4, Hkv=2, hd=64, F=512)
+ctx = api.Context(0)
+"""
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    d = tmp_path_factory.mktemp("shim")
+    (d / "shim.c").write_text(SHIM)
+    so = str(d / "shim.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", so, str(d / "shim.c"), "-ldl"], check=True)
+
+    def go(code):
+        r = subprocess.run([sys.executable, "-c", PRELUDE % (HERE, so) + code], env=dict(os.environ, LD_PRELOAD=so), capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        return r.stdout
+    return go
+
+
+def test_clearing_in_a_lora_step_does_not_grow_with_its_adapters(run):
+    out = run("""
+for mask in (0x05, 0x7F):
+    st = lora_state(ctx, cfg, 8, mask)
+    for _ in range(3): m = step(ctx, cfg, st, 512)[1]
+    print(m)
+    st.close()
+""").split()
+    few, many = (int(x) for x in out)
+    assert few > 0 and many == few, out
