@@ -620,7 +620,7 @@ extern "C" void sb_parts_prepare(sb_ctx_t* c, const float* const* x, const size_
         int k = 0;
         for (; i0 < count && k < TC_MULTI; i0++) {
             void* h; int fresh;
-            if (!sb_parts_find(c, x[i0], n[i0], &h, &ops[k].amax, &fresh)) return;      // no arena: every product prepares its own operands
+            if (!sb_parts_find(c, x[i0], n[i0], &h, &ops[k].amax, &fresh)) continue;      // no parts for it: its products prepare it
             ops[k].x = x[i0]; ops[k].n = n[i0]; ops[k].h = (__half*)h; ops[k].fresh = fresh != 0; ops[k].kept = fresh == SB_PARTS_MAKE_KEPT; ops[k].slot = -1;
             k++;
         }
