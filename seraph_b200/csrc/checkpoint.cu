@@ -194,7 +194,6 @@ extern "C" int seraph_b200_load_safetensors(cuda_train_context_t* ctx, train_sta
             if (fread(hbuf[b], 2, n, f) != n) { fprintf(stderr, "ERROR: Failed to read tensor data\n"); rc = SB_ERR_ARG; break; }
             cudaMemcpyAsync(dbuf[b], hbuf[b], n * 2, cudaMemcpyHostToDevice, st);
             cudaEventRecord(ev[b], st);
-            c->weights_gen++;
             unpack_bf16_kernel<<<blocks, 256, 0, st>>>(dbuf[b], c->W + seg[s].begin + o, n);
             c->launches++;
         }
@@ -229,7 +228,6 @@ extern "C" int sb_upload_bf16(sb_ctx_t* c, const uint16_t* src, float* dst, size
         memcpy(hbuf[b], src + o, m * 2);
         cudaMemcpyAsync(dbuf[b], hbuf[b], m * 2, cudaMemcpyHostToDevice, st);
         cudaEventRecord(ev[b], st);
-        c->weights_gen++;
         unpack_bf16_kernel<<<blocks, 256, 0, st>>>(dbuf[b], dst + o, m);
         c->launches++;
     }

@@ -150,18 +150,13 @@ void cuda_train_buffer_free(cuda_train_context_t* ctx, cuda_buffer_t* buf) {
     free(buf);
 }
 
-// the written buffer may be one of the published views of the weights: parts kept for them are stale
-static void weights_may_change(cuda_train_context_t* ctx) { sb_ctx_t* c = sb_priv(ctx); if (c) c->weights_gen++; }
-
 void cuda_train_buffer_upload(cuda_train_context_t* ctx, cuda_buffer_t* buf, const float* data, size_t count) {
     if (!ctx || !buf || !data) return;
-    weights_may_change(ctx);
     sb_check(sb_priv(ctx), cudaMemcpyAsync(buf->data, data, count * sizeof(float), cudaMemcpyHostToDevice,
                                            (cudaStream_t)ctx->stream), "upload");
 }
 void cuda_train_buffer_upload_u32(cuda_train_context_t* ctx, cuda_buffer_t* buf, const uint32_t* data, size_t count) {
     if (!ctx || !buf || !data) return;
-    weights_may_change(ctx);
     sb_check(sb_priv(ctx), cudaMemcpyAsync(buf->data, data, count * sizeof(uint32_t), cudaMemcpyHostToDevice,
                                            (cudaStream_t)ctx->stream), "upload_u32");
 }
@@ -177,7 +172,6 @@ void cuda_train_buffer_download(cuda_train_context_t* ctx, cuda_buffer_t* buf, f
 // `value` is a byte value, as with cudaMemsetAsync in the reference
 void cuda_train_fill_buffer_range(cuda_train_context_t* ctx, cuda_buffer_t* buf, size_t offset, uint32_t value, size_t bytes) {
     if (!ctx || !buf) return;
-    weights_may_change(ctx);
     sb_check(sb_priv(ctx), cudaMemsetAsync((char*)buf->data + offset, (int)value, bytes, (cudaStream_t)ctx->stream), "fill");
 }
 void cuda_train_fill_buffer(cuda_train_context_t* ctx, cuda_buffer_t* buf, uint32_t value, size_t bytes) {
@@ -185,7 +179,6 @@ void cuda_train_fill_buffer(cuda_train_context_t* ctx, cuda_buffer_t* buf, uint3
 }
 void cuda_train_copy_buffer(cuda_train_context_t* ctx, cuda_buffer_t* src, cuda_buffer_t* dst, size_t bytes) {
     if (!ctx || !src || !dst) return;
-    weights_may_change(ctx);
     sb_check(sb_priv(ctx), cudaMemcpyAsync(dst->data, src->data, bytes, cudaMemcpyDeviceToDevice,
                                            (cudaStream_t)ctx->stream), "copy_buffer");
 }

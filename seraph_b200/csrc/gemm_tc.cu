@@ -73,8 +73,8 @@ int sb_f16_slot(sb_ctx_t* c, const float* x, size_t n, int own, bool* fresh) {
 // Weights and the activations the forward pass saves for the backward pass are read by several products of one step
 // (a weight by its forward product and by the input gradient; a saved activation by the forward product and by the
 // weight gradient).  The step driver registers them; their parts live in one arena at fixed offsets and are made at
-// the first use inside a step.  Nothing is valid across steps (the caller may write any of these tensors between calls) but the parts of
-// weights that are fixed: c->weights_fixed, until weights_gen moves on (an upload, any call of the op-level interface).
+// the first use inside a step.  Nothing is valid across calls (the caller may write any of these tensors between them, through their published
+// addresses with code of its own); inside one cuda_evaluate the parts of weights stay from pass to pass, until weights_gen moves on.
 static size_t parts_hash_of(const float* p, int cap) { return (size_t)(((uintptr_t)p >> 8) * 0x9E3779B97F4A7C15ull >> 20) & (size_t)(cap - 1); }
 static void parts_rehash(sb_ctx_t* c) {
     for (int i = 0; i < c->parts_hash_cap; i++) c->parts_hash[i] = -1;
@@ -237,8 +237,8 @@ extern "C" int sb_parts_find(sb_ctx_t* c, const float* x, size_t n, void** hout,
     }
     sb_parts_entry_t* e = &c->parts_tab[idx];
     *hout = (__half*)c->parts_arena + e->off;
-    // weights that nothing changes between calls (the frozen base of adapter training; any model inside one evaluation) keep their parts
-    const unsigned gen = e->kind == 0 && c->weights_fixed ? 0x80000000u | (c->weights_gen << 1) | (sb_parts_keep(c) == 0xffffffffu ? 0u : 1u) : c->parts_gen & 0x7fffffffu;
+    // the passes of one cuda_evaluate share the parts of the weights
+    const unsigned gen = e->kind == 0 && c->in_evaluate ? 0x80000000u | c->weights_gen : c->parts_gen & 0x7fffffffu;
     *fresh = e->gen == gen && e->cur == n ? 0 : gen & 0x80000000u ? SB_PARTS_MAKE_KEPT : SB_PARTS_MAKE;
     if (*fresh) e->amax_ptr = c->parts_amax + idx;
     *amax = e->amax_ptr;

@@ -113,7 +113,7 @@ static int index_single(sb_ctx_t* c, int T, int len) {
     return 0;
 }
 
-#define CTX_OR_RETURN(ctx) sb_ctx_t* c = sb_priv(ctx); if (!c) { fprintf(stderr, "seraph_b200: invalid context\n"); return; } c->weights_gen++;      /* its output may be a view of the weights */
+#define CTX_OR_RETURN(ctx) sb_ctx_t* c = sb_priv(ctx); if (!c) { fprintf(stderr, "seraph_b200: invalid context\n"); return; }
 #define NEED(...) do { const void* ptrs_[] = {__VA_ARGS__}; for (size_t i_ = 0; i_ < sizeof(ptrs_) / sizeof(ptrs_[0]); i_++) \
         if (!ptrs_[i_]) { sb_set_status(c, SB_ERR_ARG); return; } } while (0)
 

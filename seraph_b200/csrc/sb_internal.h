@@ -79,7 +79,7 @@ typedef struct sb_ctx {
     struct { const float* ptr; size_t n; } hint_pending[SB_HINT_PENDING]; int hint_npending;
     float* final_inv; float* ghid_amax;      /* words of this step: max 1/rms of the final norm, max |g_hidden| */
     void* cs_pending; int cs_defer, cs_store;      /* dscale sums waiting for their common launch */
-    int weights_fixed, in_evaluate; unsigned weights_gen;      /* the weights' parts outlive the call while weights_gen stands */
+    int in_evaluate; unsigned weights_gen;      /* inside one cuda_evaluate the weights' parts stay while weights_gen stands */
     unsigned parts_gen; int parts_open; int parts_cache;   /* parts_cache 0: off (switch, or the arena did not fit) */
     int eval_batch_tokens;           /* cuda_evaluate packs samples up to this many tokens per forward pass; 0: one sample per pass */
     int attn_flash;                  /* 128-wide heads: 0 a launch per product over a score scratch; otherwise the forward is one kernel and the backward

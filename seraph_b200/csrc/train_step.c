@@ -307,7 +307,6 @@ static int ensure_model(sb_ctx_t* c, const train_state_t* st, int frozen_base) {
         sb_parts_register(c, 0, c->W + o->gate, (size_t)F * d); sb_parts_register(c, 0, c->W + o->up, (size_t)F * d);
         sb_parts_register(c, 0, c->W + o->down, (size_t)F * d);
     }
-    c->weights_gen++;
     if (st->full_weights) for_each_tensor(c, st->full_weights, up_tensor, NULL);
     else if (upload_base_from_model(c, (const seraph_model_t*)st->model)) { sb_set_status(c, SB_ERR_ARG); return 1; }
     publish_views(c);
@@ -327,7 +326,6 @@ static int ensure_extras(sb_ctx_t* c, int full) {
         }
         if (sb_check(c, cudaMalloc((void**)&c->XW, n * 4), "extra parameters")) { c->status = SB_ERR_OOM; return 1; }
         c->n_extras = n;
-        c->weights_gen++;
         cudaMemcpyAsync(c->XW, c->h_extras, n * 4, cudaMemcpyHostToDevice, S(c));
         if (c->untied) sb_parts_register(c, 0, c->XW + extras_lm_off(c), (size_t)c->V * c->d);
         if (sb_check(c, cudaStreamSynchronize(S(c)), "extra parameter upload")) return 1;
@@ -1102,7 +1100,6 @@ static float step_body(train_state_t* st, int* tokens, int T, int* seq_starts, i
     if (use_lora && ensure_lora(c, st->lora)) return -1.0f;
     if (ensure_extras(c, full && train)) return -1.0f;
     if (ensure_activations(c, T, train)) return -1.0f;
-    c->weights_fixed = c->frozen_base || c->in_evaluate;
     c->lora_grouped = 0;
     if (use_lora) {
         if (ensure_lora_working(c) || ensure_lora_grouped(c, T)) return -1.0f;
@@ -1285,7 +1282,7 @@ float cuda_evaluate(train_state_t* state, int* val_tokens, int num_val_tokens, i
     }
     int full = state->lora == NULL;
     int B = 0;
-    if (c) { c->weights_gen++; c->in_evaluate = 1; }      /* nothing changes the weights between the passes of this call */
+    if (c) { c->weights_gen++; c->in_evaluate = 1; }      /* nothing changes the weights between the passes of this call: they share their parts */
     if (budget > 0) ss[0] = 0;
     for (int s = 0; s < num_samples; s += stride) {
         int start = offsets[s], end = (s + 1 < num_samples) ? offsets[s + 1] : num_val_tokens;

@@ -477,6 +477,44 @@ def test_evaluate_in_several_passes_whose_products_are_not_all_grouped(ctx, name
     st.close()
 
 
+def test_writes_to_a_frozen_weight_through_its_published_address_take_effect(ctx):
+    """A host changes weights of the resident base between LoRA steps with code of its own, through the addresses the context publishes and with no call
+    of the library in between: the next step and the next evaluation read what is there."""
+    import torch
+    from perf import cases
+    from seraph_b200 import api
+    cfg, rank, mask, ss = O.ModelCfg(V=512, d=256, L=2, Hq=4, Hkv=2, hd=64, F=512), 8, 0x05, [0, 300, 431, 640]
+    p = cfg.init_params(66)
+    tens, n = cfg.lora_tensors(rank, mask)
+    lo = (0.02 * np.random.default_rng(67).standard_normal(n)).astype(np.float32)
+    tok = tokens_for(cfg, ss[-1], 68)
+    st = api.TrainState(cfg, p, lr=1e-2)
+    st.attach_lora(rank, 2.0 * rank, mask, lo)
+    offs = {name: (off, int(np.prod(shp))) for name, shp, off in cfg.tensors()}
+    for _ in range(3):
+        ref = O.train_step(cfg, p, tok, ss, lora=lo, rank=rank, alpha=2.0 * rank, mask=mask)
+        loss = api.step_lora_batch(ctx, st, tok, ss)
+        ctx.check()
+        assert abs(loss - ref["loss"]) < 1e-5 * abs(ref["loss"])
+        ctx.lib.cuda_download_lora_weights(ctx.h, st.lora_ptr())
+        g = st.lora_get(1)
+        for nm, shp, off in tens:
+            k = int(np.prod(shp))
+            assert rel_l2(g[off:off + k], ref["grads"][off:off + k]) < TOL, nm
+        lo = st.lora_get(0).copy()
+        head = cases._CtxHead.from_address(ctx.h)
+        for name, buf, factor in (("l0.q", head.q[0][0], -1.5), ("l1.down", head.down[0][1], 3.0), ("embed", head.embed[0], 0.5)):
+            off, k = offs[name]
+            cases.on_device(ctx, cases._address(buf), k).mul_(factor)
+            p[off:off + k] *= np.float32(factor)
+        torch.cuda.synchronize()
+    t = np.ascontiguousarray(tok[:300])
+    ev = ctx.lib.cuda_eval_forward(st.h, t.ctypes.data, 300, ctx.h)
+    ref = O.train_step(cfg, p, t, [0, 300], lora=lo, rank=rank, alpha=2.0 * rank, mask=mask)["loss"]
+    assert abs(ev - ref) < 1e-5 * ref
+    st.close()
+
+
 def test_operand_parts_kept_within_a_step_change_nothing(ctx):
     """The FP16 parts of weights and saved activations are made once per call and shared by the call's products, and the SwiGLU
     kernels write their outputs straight into that arena (scaled by a bound instead of the exact maximum, so those operands
