@@ -126,7 +126,7 @@ typedef struct sb_ctx {
        A and columns of B are zero, so the extra columns of X A^T are zero and the extra gradient rows / columns are never read. */
     int lora_R; size_t n_lora_pad; float *LWp, *LGp; int lora_pad_stale;
     float* lora_tmp; size_t lora_tmp_cap;
-    float* lora_h; size_t lora_h_cap; int lora_h_T;      /* X A^T of every layer and adapter, kept for the backward pass [T, lora_R] */
+    float* lora_h; size_t lora_h_cap; int lora_h_T;      /* X A^T of every layer and adapter, kept for the backward pass [T <= lora_h_T, lora_R] */
     int lora_grouped;                /* the step in flight runs its adapters' products in groups */
 
     /* activations */

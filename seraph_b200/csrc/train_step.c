@@ -502,8 +502,8 @@ static float* lora_h_of(const sb_ctx_t* c, int l, int a) {
     for (int b = 0; b < a; b++) i += (c->lora_mask >> b) & 1;
     return c->lora_h + ((size_t)l * lora_count_adapters(c) + i) * (((size_t)c->lora_h_T * c->lora_R + 63) & ~(size_t)63);
 }
-/* May this step run its adapters' products in groups?  Then X A^T of every adapter is kept for the backward pass (lora_h, sized here for T
- * tokens); otherwise the products run one after the other over lora_tmp. */
+/* May this step run its adapters' products in groups?  Then X A^T of every adapter is kept for the backward pass (lora_h: slots for as many tokens as
+ * the activations hold, so that steps of fewer tokens use them as they are); otherwise the products run one after the other over lora_tmp. */
 static int ensure_lora_grouped(sb_ctx_t* c, int T) {
     c->lora_grouped = 0;
     const int R = c->lora_R;
@@ -515,8 +515,9 @@ static int ensure_lora_grouped(sb_ctx_t* c, int T) {
             !sb_gemm_group_takes(c, R, in, T, 1, 0) || !sb_gemm_group_takes(c, T, in, R, 0, 0)) return 0;
     }
     const int n = lora_count_adapters(c);
-    const size_t one = ((size_t)T * R + 63) & ~(size_t)63, need = one * (size_t)n * (size_t)c->L;
-    if (c->lora_h_T != T) {
+    if (c->lora_h_T < T) {
+        const int cap = c->T_cap;                    /* >= T: the activations have been made */
+        const size_t one = ((size_t)cap * R + 63) & ~(size_t)63, need = one * (size_t)n * (size_t)c->L;
         sb_parts_unregister(c, 3);
         c->lora_h_T = 0;
         if (c->lora_h_cap < need) {
@@ -526,8 +527,8 @@ static int ensure_lora_grouped(sb_ctx_t* c, int T) {
             if (sb_check(c, cudaMalloc((void**)&c->lora_h, need * sizeof(float)), "lora activations")) { c->status = SB_ERR_OOM; return 1; }
             c->lora_h_cap = need;
         }
-        c->lora_h_T = T;
-        for (size_t i = 0; i < (size_t)n * (size_t)c->L; i++) sb_parts_register(c, 3, c->lora_h + i * one, (size_t)T * R);
+        c->lora_h_T = cap;
+        for (size_t i = 0; i < (size_t)n * (size_t)c->L; i++) sb_parts_register(c, 3, c->lora_h + i * one, (size_t)cap * R);
     }
     c->lora_grouped = 1;
     return 0;

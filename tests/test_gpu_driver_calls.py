@@ -78,3 +78,13 @@ for mask in (0x05, 0x7F):
 """).split()
     few, many = (int(x) for x in out)
     assert few > 0 and many == few, out
+
+
+def test_lora_steps_of_lengths_seen_before_allocate_nothing(run):
+    out = run("""
+st = lora_state(ctx, cfg, 16, 0x7F)
+print(*[step(ctx, cfg, st, T)[0] for _ in range(2) for T in (512, 300, 40, 411)])
+st.close()
+""").split()
+    calls = [int(x) for x in out]
+    assert calls[0] > 0 and calls[4:] == [0, 0, 0, 0], calls

@@ -427,6 +427,30 @@ def test_lora_step_with_grouped_adapters(ctx, rank, mask, exact):
     st.close()
 
 
+def test_lora_steps_of_changing_length(ctx):
+    """The rows X A^T kept for the backward pass have room for the longest batch seen; shorter and longer ones in between."""
+    from seraph_b200 import api
+    cfg, rank, mask = O.ModelCfg(V=512, d=256, L=2, Hq=4, Hkv=2, hd=64, F=512), 20, 0x7F
+    p = cfg.init_params(69)
+    tens, n = cfg.lora_tensors(rank, mask)
+    lo = (0.02 * np.random.default_rng(70).standard_normal(n)).astype(np.float32)
+    st = api.TrainState(cfg, p, lr=1e-2)
+    st.attach_lora(rank, 2.0 * rank, mask, lo)
+    for ss in ([0, 300, 641], [0, 77, 301], [0, 40], [0, 641], [0, 500, 811]):
+        tok = tokens_for(cfg, ss[-1], 71 + ss[-1])
+        ref = O.train_step(cfg, p, tok, ss, lora=lo, rank=rank, alpha=2.0 * rank, mask=mask)
+        loss = api.step_lora_batch(ctx, st, tok, ss)
+        ctx.check()
+        assert abs(loss - ref["loss"]) < 1e-5 * abs(ref["loss"])
+        ctx.lib.cuda_download_lora_weights(ctx.h, st.lora_ptr())
+        g = st.lora_get(1)
+        for nm, shp, off in tens:
+            k = int(np.prod(shp))
+            assert rel_l2(g[off:off + k], ref["grads"][off:off + k]) < TOL, (ss, nm)
+        lo = st.lora_get(0).copy()
+    st.close()
+
+
 FROZEN = [("vocabulary not a multiple of 4", O.ModelCfg(V=515, d=256, L=2, Hq=4, Hkv=2, hd=64, F=512), [0, 300, 431, 640]),
           ("narrow k and v", O.ModelCfg(V=512, d=256, L=2, Hq=4, Hkv=1, hd=64, F=512), [0, 11, 24])]
 
