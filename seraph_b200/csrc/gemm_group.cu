@@ -22,7 +22,7 @@
 //     warps are back at the next tile's chunks after about 2900 cycles, which is what the two accumulators hide of it.  (Whole rows through
 //     one buffer of 64 rows and store warps: 4900 cycles, a stall of 1.3 us a tile.)
 // NT = 3: FP32-accurate (hi hi + lo hi + hi lo).  NT = 1: hi parts only, the 11 leading significant bits (what a TF32 instruction reads of an
-// FP32 word, at twice its rate): the reduced-precision mode.
+// FP32 word, at twice its rate): the reduced-precision mode, for all but its smallest products (gg_single).
 #include <stdio.h>
 #include "gemm_tc.cuh"
 
@@ -550,6 +550,14 @@ bool gg_shape_ok(int M, int N, int K, int tA, int tB) {
     if (tA && tB) tA = tB = 0;
     return (tA ? (M & 7) == 0 : (K & 7) == 0) && (tB ? (K & 7) == 0 : (N & 7) == 0);
 }
+// In the single-pass mode a product of fewer than 32 rows or columns, or under 2^21 multiply-adds, stays FP32-accurate: that mode's TF32 kernel left
+// those to the FP32 cores, and so few operations gain nothing from two passes less.  The rank of an adapter counts as the multiple of 128 that it
+// was padded to there.  One such product and the launch takes three passes.
+static bool gg_single(const sb_gemm_job_t* b) {
+    int d[3] = {b->M, b->N, b->K};
+    if (b->rank) d[b->rank - 1] = (d[b->rank - 1] + 127) / 128 * 128;
+    return d[0] >= 32 && d[1] >= 32 && (double)d[0] * d[1] * d[2] >= (double)(1 << 21);
+}
 static bool gg_mode(const sb_ctx_t* c, int* nt) {
     const int mode = c->pub.use_bf16 ? SB_GEMM_BF16 : c->gemm_mode;
     *nt = mode == SB_GEMM_BF16 ? 1 : 3;
@@ -746,7 +754,9 @@ extern "C" int sb_gemm_group_try(sb_ctx_t* c, const sb_gemm_job_t* jobs, int njo
         int k = j + 1;
         while (k < njobs && k - j < GG_MAXS) k++;
         if (k < njobs) while (k > j + 1 && jobs[k].C == jobs[k - 1].C && jobs[k].acc) k--;      // a sum stays in one launch
-        ok = gg_run(c, jobs + j, k - j, nt);
+        int passes = nt;
+        for (int i = j; i < k; i++) if (!gg_single(&jobs[i])) passes = 3;
+        ok = gg_run(c, jobs + j, k - j, passes);
         j = k;
     }
     if (!keep) sb_gemm_keep_end(c);

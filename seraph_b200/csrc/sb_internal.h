@@ -270,7 +270,8 @@ void sb_nan_check(sb_ctx_t*, const float* x, size_t n, uint32_t* flags, uint32_t
 void sb_gemm(sb_ctx_t*, const float* A, const float* B, float* C, int M, int N, int K, int tA, int tB, int acc);
 /* Several products that do not depend on one another, as if by sb_gemm in this order; a product with the destination of the one before it and
    acc set is added to it.  On FP16 parts they run as one launch.  Jobs with a factor only where sb_gemm_group_takes says so. */
-typedef struct { const float *A, *B; float* C; int M, N, K, tA, tB, acc; float alpha; } sb_gemm_job_t;      /* alpha: factor of the product, 0 means 1 */
+typedef struct { const float *A, *B; float* C; int M, N, K, tA, tB, acc; float alpha; int rank; } sb_gemm_job_t;      /* alpha: factor of the product, 0 means 1; rank: which
+                                                                            of M, N, K (1, 2, 3) is the rank of an adapter, or 0 */
 void sb_gemm_group(sb_ctx_t*, const sb_gemm_job_t* jobs, int n);
 int  sb_gemm_group_try(sb_ctx_t*, const sb_gemm_job_t* jobs, int n);      /* 0: launched as a group */
 int  sb_gemm_group_takes(sb_ctx_t*, int M, int N, int K, int tA, int tB);

@@ -638,7 +638,7 @@ static void lora_fwd_group(sb_ctx_t* c, int l, const float* X, const proj_t* p, 
     lora_ref_t r;
     for (int i = 0; i < n; i++)
         if (lora_get(c, l, p[i].a, &r)) {
-            const sb_gemm_job_t j = {X, r.A, r.h, T, c->lora_R, in, 0, 1, 0, 1.f};
+            const sb_gemm_job_t j = {X, r.A, r.h, T, c->lora_R, in, 0, 1, 0, 1.f, 2};
             sb_amax_announce(c, r.h, (size_t)T * c->lora_R);
             jobs[k++] = j;
         }
@@ -647,7 +647,7 @@ static void lora_fwd_group(sb_ctx_t* c, int l, const float* X, const proj_t* p, 
     for (int i = 0; i < n; i++) {
         const sb_gemm_job_t j = {X, p[i].W, p[i].Y, T, p[i].out, in, 0, 1, p[i].acc, 1.f};
         jobs[k++] = j;
-        if (lora_get(c, l, p[i].a, &r)) { const sb_gemm_job_t b = {r.h, r.B, p[i].Y, T, p[i].out, c->lora_R, 0, 1, 1, s}; jobs[k++] = b; }
+        if (lora_get(c, l, p[i].a, &r)) { const sb_gemm_job_t b = {r.h, r.B, p[i].Y, T, p[i].out, c->lora_R, 0, 1, 1, s, 3}; jobs[k++] = b; }
     }
     sb_gemm_group(c, jobs, k);
 }
@@ -666,7 +666,7 @@ static void lora_bwd_group(sb_ctx_t* c, int l, const int* ads, const float* cons
     for (int i = 0; i < n; i++)
         if (lora_get(c, l, ads[i], &r)) {
             float* gh = c->lora_tmp + (size_t)i * one;
-            const sb_gemm_job_t j = {dY[i], r.B, gh, T, c->lora_R, r.out, 0, 0, 0, 1.f}, b = {dY[i], r.h, r.gB, r.out, c->lora_R, T, 1, 0, 1, s};
+            const sb_gemm_job_t j = {dY[i], r.B, gh, T, c->lora_R, r.out, 0, 0, 0, 1.f, 2}, b = {dY[i], r.h, r.gB, r.out, c->lora_R, T, 1, 0, 1, s, 2};
             sb_gemm_keep_forget(c, gh);
             sb_amax_announce(c, gh, (size_t)T * c->lora_R);
             jobs[k++] = j; jobs[k++] = b;
@@ -674,9 +674,9 @@ static void lora_bwd_group(sb_ctx_t* c, int l, const int* ads, const float* cons
     if (k) sb_gemm_group(c, jobs, k);
     k = 0;
     for (int i = 0; i < n; i++)
-        if (lora_get(c, l, ads[i], &r)) { const sb_gemm_job_t j = {c->lora_tmp + (size_t)i * one, X, r.gA, c->lora_R, r.in, T, 1, 0, 1, s}; jobs[k++] = j; }
+        if (lora_get(c, l, ads[i], &r)) { const sb_gemm_job_t j = {c->lora_tmp + (size_t)i * one, X, r.gA, c->lora_R, r.in, T, 1, 0, 1, s, 1}; jobs[k++] = j; }
     for (int i = 0; i < n && dX && c->lora_exact; i++)
-        if (lora_get(c, l, ads[i], &r)) { const sb_gemm_job_t j = {c->lora_tmp + (size_t)i * one, r.A, dX, T, r.in, c->lora_R, 0, 0, 1, s}; jobs[k++] = j; }
+        if (lora_get(c, l, ads[i], &r)) { const sb_gemm_job_t j = {c->lora_tmp + (size_t)i * one, r.A, dX, T, r.in, c->lora_R, 0, 0, 1, s, 3}; jobs[k++] = j; }
     if (k) sb_gemm_group(c, jobs, k);
 }
 

@@ -72,6 +72,27 @@ def test_grouped_kernel_at_tile_edges(ctx, M, N, K, tA, tB, acc):
     ctx.release(a, b, c)
 
 
+@pytest.mark.parametrize("tA,tB,acc", [(0, 1, 0), (0, 0, 1), (1, 0, 1)])
+@pytest.mark.parametrize("M,N,K,single", [(8, 512, 1024, 0), (24, 2048, 512, 0), (512, 16, 4096, 0), (64, 128, 248, 0), (64, 128, 256, 1), (32, 512, 128, 1)])
+def test_single_pass_mode_keeps_small_products_accurate(ctx, M, N, K, single, tA, tB, acc):
+    """use_bf16 / mode 2: operands of 11 significant bits from 32 rows and columns and 2^21 multiply-adds up, FP32 accuracy below."""
+    r = np.random.default_rng(M + N + K)
+    A = r.standard_normal((K, M) if tA else (M, K)).astype(np.float32)
+    B = r.standard_normal((N, K) if tB else (K, N)).astype(np.float32)
+    C0 = r.standard_normal((M, N)).astype(np.float32)
+    ref = C0.copy()
+    O.lib().ref_matmul(A, B, ref, M, N, K, tA, tB, acc)
+    a, b, c = ctx.upload(A), ctx.upload(B), ctx.upload(C0)
+    ctx.set_gemm_mode(2)
+    ctx.lib.cuda_train_matmul_transpose(ctx.h, a.b, b.b, c.b, M, N, K, tA, tB, acc)
+    out = c.numpy(shape=(M, N))
+    ctx.set_gemm_mode(4)
+    ctx.check()
+    e = rel_l2(out, ref)
+    assert (1e-4 < e < BOUND[1]) if single else e < BOUND[4], e
+    ctx.release(a, b, c)
+
+
 def test_tc_gemm_long_k_and_reproducible(ctx):
     """K = 16384 (longer than the 8192-token reduction of the weight gradients): accumulation error stays in bound."""
     M, N, K = 256, 512, 16384

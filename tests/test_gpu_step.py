@@ -451,6 +451,40 @@ def test_lora_steps_of_changing_length(ctx):
     st.close()
 
 
+@pytest.mark.parametrize("lora", [0, 1])
+@pytest.mark.parametrize("ss,tol", [([0, 11, 24], TOL), ([0, 300, 431, 640], 2e-2)])
+def test_single_pass_mode_step(ctx, ss, tol, lora):
+    """use_bf16: a step of fewer than 32 tokens stays FP32-accurate.  Longer ones run on operands cut to 11 bits, a relative error of at most 2^-10 in each
+    operand; a gradient is behind up to ten such products in a row (20 x 2^-10)."""
+    from seraph_b200 import api
+    cfg, rank, mask = O.ModelCfg(V=512, d=256, L=2, Hq=4, Hkv=2, hd=64, F=512), 16, 0x7F
+    p = cfg.init_params(72)
+    tok = tokens_for(cfg, ss[-1], 73)
+    st = api.TrainState(cfg, p)
+    ctx.lib.seraph_b200_set_gemm_mode(ctx.h, 2)
+    if lora:
+        tens, n = cfg.lora_tensors(rank, mask)
+        lo = (0.02 * np.random.default_rng(74).standard_normal(n)).astype(np.float32)
+        st.attach_lora(rank, 2.0 * rank, mask, lo)
+        ref = O.train_step(cfg, p, tok, ss, lora=lo, rank=rank, alpha=2.0 * rank, mask=mask)
+        loss = api.step_lora_batch(ctx, st, tok, ss)
+        ctx.lib.cuda_download_lora_weights(ctx.h, st.lora_ptr())
+        g = st.lora_get(1)
+    else:
+        tens = cfg.tensors()
+        ref = O.train_step(cfg, p, tok, ss)
+        loss = api.step_full_batch(ctx, st, tok, ss)
+        ctx.lib.cuda_download_gpu_gradients(ctx.h, st.h)
+        g = st.get(1)
+    ctx.set_gemm_mode(4)
+    ctx.check()
+    st.close()
+    assert abs(loss - ref["loss"]) < tol * abs(ref["loss"])
+    errs = [rel_l2(g[off:off + int(np.prod(shp))], ref["grads"][off:off + int(np.prod(shp))]) for _, shp, off in tens]
+    print("worst gradient:", max(errs))
+    assert max(errs) < tol, max(errs)
+
+
 FROZEN = [("vocabulary not a multiple of 4", O.ModelCfg(V=515, d=256, L=2, Hq=4, Hkv=2, hd=64, F=512), [0, 300, 431, 640]),
           ("narrow k and v", O.ModelCfg(V=512, d=256, L=2, Hq=4, Hkv=1, hd=64, F=512), [0, 11, 24])]
 
