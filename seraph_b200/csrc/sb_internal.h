@@ -133,8 +133,8 @@ typedef struct sb_ctx {
     int T_cap;
     sb_layer_act_t* act;             /* [L] */
     float* act_arena; size_t act_arena_bytes;
-    float *hidden, *hidden_norm, *final_in, *logits, *dlogits, *loss_rows;
-    float *g_hidden, *g_tmp, *g_xnorm, *g_q, *g_k, *g_v, *g_attn, *g_ffn, *g_gate, *g_up, *attn_delta;
+    float *hidden_norm, *final_in, *logits, *dlogits, *loss_rows;
+    float *g_hidden, *g_xnorm, *g_q, *g_k, *g_v, *g_attn, *g_ffn, *g_gate, *g_up;
     uint32_t *tokens, *targets, *seq_starts, *pos_ids, *seq_ids;
     int seq_cap, seq_starts_cap;
     int* h_seq; int h_seq_n, h_seq_cap;   /* host copy of the current batch's sequence starts (h_seq_n + 1 entries); 0 = unknown */

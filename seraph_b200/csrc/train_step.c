@@ -546,7 +546,7 @@ static void free_activations(sb_ctx_t* c) {
 
 static size_t r4(size_t n) { return (n + 63) & ~(size_t)63; }     /* keep every slot 256-byte aligned */
 
-static int ensure_activations(sb_ctx_t* c, int T, int need_logits_grad) {
+static int ensure_activations(sb_ctx_t* c, int T) {
     if (c->act_arena && c->T_cap >= T) return 0;
     cudaStreamSynchronize(S(c));
     free_activations(c);
@@ -554,9 +554,8 @@ static int ensure_activations(sb_ctx_t* c, int T, int need_logits_grad) {
     size_t TH = r4((size_t)T * c->Hq), TV = r4((size_t)T * c->V);
     size_t per_layer = 4 * Td + 2 * Tq + 2 * Tkv + TH + 3 * TF + 2 * r4((size_t)T);    /* layer_in x_norm_attn post_attn_in x_norm_ffn | q attn_out | k v | lse | gate up ffn_hidden */
     if (c->head_norm) per_layer += Tq + Tkv;                                          /* q_pre k_pre */
-    size_t shared = 3 * Td /* hidden_norm final_in (+1 spare) */ + 2 * TV + r4((size_t)T)
-                  + 3 * Td /* g_hidden g_tmp g_xnorm */ + 2 * Tq + 2 * Tkv + 3 * TF + (c->head_norm ? Tq + Tkv : 0);
-    (void)need_logits_grad;
+    size_t shared = 2 * Td /* hidden_norm final_in */ + 2 * TV + r4((size_t)T)
+                  + 2 * Td /* g_hidden g_xnorm */ + 2 * Tq + 2 * Tkv + 3 * TF + (c->head_norm ? Tq + Tkv : 0);
     size_t total = per_layer * (size_t)c->L + shared;
     if (sb_check(c, cudaMalloc((void**)&c->act_arena, total * sizeof(float)), "activation arena")) { c->status = SB_ERR_OOM; return 1; }
     c->act_arena_bytes = total * sizeof(float); c->T_cap = T;
@@ -571,9 +570,9 @@ static int ensure_activations(sb_ctx_t* c, int T, int need_logits_grad) {
         TAKE(a->gate, TF); TAKE(a->up, TF); TAKE(a->ffn_hidden, TF);
         if (c->head_norm) { TAKE(a->q_pre, Tq); TAKE(a->k_pre, Tkv); }
     }
-    TAKE(c->hidden_norm, Td); TAKE(c->final_in, Td); TAKE(c->hidden, Td);
+    TAKE(c->hidden_norm, Td); TAKE(c->final_in, Td);
     TAKE(c->logits, TV); TAKE(c->dlogits, TV); TAKE(c->loss_rows, r4((size_t)T));
-    TAKE(c->g_hidden, Td); TAKE(c->g_tmp, Td); TAKE(c->g_xnorm, Td);
+    TAKE(c->g_hidden, Td); TAKE(c->g_xnorm, Td);
     TAKE(c->g_q, Tq); TAKE(c->g_attn, Tq); TAKE(c->g_k, Tkv); TAKE(c->g_v, Tkv);
     TAKE(c->g_ffn, TF); TAKE(c->g_gate, TF); TAKE(c->g_up, TF);
     if (c->head_norm) { TAKE(c->g_q2, Tq); TAKE(c->g_k2, Tkv); }
@@ -904,8 +903,7 @@ typedef struct { int on, done, step; float lr, gscale; } early_adamw_t;
 static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, int full, int store, int reduce, early_adamw_t* early) {
     const int d = c->d, F = c->F, qd = c->qd, kvd = c->kvd, L = c->L, V = c->V;
     float* gh = c->g_hidden; float* gx = c->g_xnorm;
-    float* Gd = full ? c->G : NULL;
-    float* norm_sink = NULL;                     /* LoRA mode: norm-scale gradients are not formed */
+    float* Gd = full ? c->G : NULL;              /* LoRA mode: norm-scale gradients are not formed either */
     const int add = !store;
     const int grouped = !full && c->lora_grouped;
     /* the gradients of all norm scales are summed in one launch at the end, unless the layers' buckets are handed to the all-reduce as they come */
@@ -920,7 +918,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
     }
     sb_gemm_keep_end(c);
     nan_mark(c, c->dlogits, (size_t)T * V, 3); nan_mark(c, gx, (size_t)T * d, 4);
-    sb_rmsnorm_backward_parts(c, c->final_in, c->W + (size_t)V * d, gx, NULL, gh, full ? Gd + (size_t)V * d : norm_sink, T, d, RMS_EPS, c->final_inv, &c->ghid_amax);
+    sb_rmsnorm_backward_parts(c, c->final_in, c->W + (size_t)V * d, gx, NULL, gh, full ? Gd + (size_t)V * d : NULL, T, d, RMS_EPS, c->final_inv, &c->ghid_amax);
     nan_mark(c, gh, (size_t)T * d, 5); nan_mark(c, gh, (size_t)T * d, 0);
     const int ffn_lora = !full && !grouped && (c->lora_mask & 0x70);
     const int ffn_parts_bwd = !c->nan_on && !ffn_lora && sb_gemm_reads_f16_parts(c, T, d, F, 0, 0) && (!full || sb_gemm_reads_f16_parts(c, F, d, T, 1, 0));
@@ -959,7 +957,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
         }
         if (!full && !grouped) { lora_bwd(c, l, 4, c->g_gate, a->x_norm_ffn, gx, T); lora_bwd(c, l, 5, c->g_up, a->x_norm_ffn, gx, T); }
         sb_gemm_keep_end(c);
-        sb_rmsnorm_backward_parts(c, a->post_attn_in, c->W + o->post_norm, gx, gh, gh, full ? Gd + o->post_norm : norm_sink, T, d, RMS_EPS, a->inv_ffn, &c->ghid_amax);
+        sb_rmsnorm_backward_parts(c, a->post_attn_in, c->W + o->post_norm, gx, gh, gh, full ? Gd + o->post_norm : NULL, T, d, RMS_EPS, a->inv_ffn, &c->ghid_amax);
         /* attention */
         sb_gemm_keep_begin(c);
         if (grouped) {
@@ -994,8 +992,8 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
         if (c->head_norm) {
             const size_t xo = (size_t)l * 2 * c->hd;
             sb_amax_announce(c, c->g_q2, (size_t)T * qd); sb_amax_announce(c, c->g_k2, (size_t)T * kvd);
-            sb_rmsnorm_backward(c, a->q_pre, c->XW + xo, c->g_q, NULL, c->g_q2, full ? c->XG + xo : norm_sink, T * c->Hq, c->hd, RMS_EPS);
-            sb_rmsnorm_backward(c, a->k_pre, c->XW + xo + c->hd, c->g_k, NULL, c->g_k2, full ? c->XG + xo + c->hd : norm_sink, T * c->Hkv, c->hd, RMS_EPS);
+            sb_rmsnorm_backward(c, a->q_pre, c->XW + xo, c->g_q, NULL, c->g_q2, full ? c->XG + xo : NULL, T * c->Hq, c->hd, RMS_EPS);
+            sb_rmsnorm_backward(c, a->k_pre, c->XW + xo + c->hd, c->g_k, NULL, c->g_k2, full ? c->XG + xo + c->hd : NULL, T * c->Hkv, c->hd, RMS_EPS);
             gq = c->g_q2; gk = c->g_k2;
         }
         sb_gemm_keep_begin(c);
@@ -1013,7 +1011,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
         if (!full && !grouped) { lora_bwd(c, l, 0, gq, a->x_norm_attn, gx, T); lora_bwd(c, l, 1, gk, a->x_norm_attn, gx, T); lora_bwd(c, l, 2, c->g_v, a->x_norm_attn, gx, T); }
         sb_gemm_keep_end(c);
         if (!last) {
-            sb_rmsnorm_backward_parts(c, a->layer_in, c->W + o->in_norm, gx, gh, gh, full ? Gd + o->in_norm : norm_sink, T, d, RMS_EPS, a->inv_attn, &c->ghid_amax);
+            sb_rmsnorm_backward_parts(c, a->layer_in, c->W + o->in_norm, gx, gh, gh, full ? Gd + o->in_norm : NULL, T, d, RMS_EPS, a->inv_attn, &c->ghid_amax);
         }
     layer_done:
         nan_mark(c, gh, (size_t)T * d, nan_ghid_base(c) + (uint32_t)l);
@@ -1100,7 +1098,7 @@ static float step_body(train_state_t* st, int* tokens, int T, int* seq_starts, i
     if (ensure_model(c, st, full ? 0 : (use_lora ? 1 : c->frozen_base))) return -1.0f;
     if (use_lora && ensure_lora(c, st->lora)) return -1.0f;
     if (ensure_extras(c, full && train)) return -1.0f;
-    if (ensure_activations(c, T, train)) return -1.0f;
+    if (ensure_activations(c, T)) return -1.0f;
     c->lora_grouped = 0;
     if (use_lora) {
         if (ensure_lora_working(c) || ensure_lora_grouped(c, T)) return -1.0f;
