@@ -13,7 +13,8 @@ are all-reduced with NCCL while backward still runs.
 
 value  : tokens/s with the batch already resident in HBM (no host<->device copies in the timed region)
 e2e    : tokens/s through the public step call with host token buffers (upload + loss read-back inside)
-roofline / per_class : CUDA-event time per kernel class, recorded on the library's stream during the timed steps
+roofline / per_class : CUDA-event time per kernel class, recorded on the library's stream during the timed steps (the events keep
+         launches from overlapping, so that a small model's `value` is below its `e2e`)
 cpu_baseline / reference_cuda : the reference's own CPU path and its own CUDA backend, timed on this box (baselines only)
 """
 import argparse
@@ -50,13 +51,14 @@ METRIC = "train tokens/sec (fwd+bwd+AdamW)"
 
 
 def gemm_traffic(cfg, T, f16=True):
-    """DRAM bytes of one launch of the dominant kernel: the FFN gate projection (M = T, N = ffn, K = hidden).
-    One ncu capture of that launch at T = 4096, hidden 2048, ffn 6144 read 161.7 MB and wrote 83.5 MB of DRAM in the
-    default mode (1.33 times its algorithmic 4*(M*K + N*K + M*N) bytes; with TF32 parts 151.4 + 75.1 MB, 1.23 times);
-    a full-size launch is too long a capture, so that ratio is applied to the algorithmic bytes of the launch at this
-    workload's T."""
-    alg = 4.0 * (T * cfg.d + cfg.F * cfg.d + T * cfg.F)
-    return (1.33 if f16 else 1.23) * alg
+    """DRAM bytes of one launch of the dominant kernel, the FFN gate and up projections (M = T, N = ffn, K = hidden; gg_kernel runs
+    both in one launch).  One ncu capture of that launch at T = 4096, hidden 2048, ffn 6144 read 293.8 MB and wrote 172.6 MB of
+    DRAM (1.39 times its algorithmic 4*(M*K + 2*(N*K + M*N)) bytes).  The other modes run a launch per projection on
+    gemm_tc_kernel: 151.4 + 75.1 MB with TF32 parts, 1.23 times.  A full-size launch is too long a capture, so the ratio is applied to
+    the algorithmic bytes of the launch at this workload's T."""
+    products = 2 if f16 else 1
+    alg = 4.0 * (T * cfg.d + products * (cfg.F * cfg.d + T * cfg.F))
+    return (1.39 if f16 else 1.23) * alg
 
 
 def peaks():
@@ -540,8 +542,8 @@ def run_ours(args):
                                        if f16_mode else
                                        f"{pk_kind} bf16 sustained {pk['bf16_tflops_sustained']} TFLOP/s halved for TF32 operands") +
                                       "; achieved counts useful FLOPs (2MNK) per launch over the step's GEMM launches, operand preparation "
-                                      "included; the FP32-accurate modes issue 3x that on the tensor pipe; traffic = DRAM bytes of one FFN "
-                                      "gate-projection launch (ncu capture at T=4096 scaled by algorithmic bytes)",
+                                      "included; the FP32-accurate modes issue 3x that on the tensor pipe; traffic = DRAM bytes of one launch of the FFN "
+                                      "gate and up projections (ncu capture at T=4096 scaled by algorithmic bytes)",
                          "share_of_step": (g.get("ms_per_step", 0) / (ms / args.steps)) if g else None},
             "per_class": per_class,
         }
