@@ -574,11 +574,10 @@ def test_writes_to_a_frozen_weight_through_its_published_address_take_effect(ctx
 
 
 def test_operand_parts_kept_within_a_step_change_nothing(ctx):
-    """The FP16 parts of weights and saved activations are made once per call and shared by the call's products, and the SwiGLU
-    kernels write their outputs straight into that arena (scaled by a bound instead of the exact maximum, so those operands
-    round differently in their last bits).  Three optimizer steps (the weights move between them), then a step on fewer tokens
-    and one on the full batch again: losses, gradients and weights agree with the run in which every product prepares its own
-    operands to a few 1e-6 (both inside the parity bound), and the run with the arena repeats bit for bit."""
+    """The FP16 parts of weights and saved activations are made once per call and shared by the call's products, and the kernels
+    that know a bound of their output write it straight into that arena.  Three optimizer steps (the weights move between them), then
+    a step on fewer tokens and one on the full batch again: losses, gradients and weights are those of the run in which every product
+    prepares its own operands (under the same bounds), and the run with the arena repeats bit for bit."""
     from seraph_b200 import api
     cfg = C1
     p = cfg.init_params(77)
@@ -603,6 +602,7 @@ def test_operand_parts_kept_within_a_step_change_nothing(ctx):
     print(f"arena on vs off: gradients rel-L2 {eg:.2e}, weights {ew:.2e}")
     # two roundings of the same sums: each is within 2.5e-6 of the oracle, so they may differ from each other by their root sum
     assert eg < 6e-6 and ew < 2e-6, (eg, ew)
+    assert runs[0][0] == runs[1][0] and np.array_equal(runs[0][1], runs[1][1]) and np.array_equal(runs[0][2], runs[1][2])      # and they do not
     assert runs[0][0] == runs[2][0] and np.array_equal(runs[0][1], runs[2][1]) and np.array_equal(runs[0][2], runs[2][2])
     assert runs[0][0][0] != runs[0][0][2]          # the weights did move
 
