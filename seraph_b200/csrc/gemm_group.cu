@@ -17,6 +17,10 @@
 //   * work items are handed out at run time: one warp of the pair's leader takes the next item from a counter and passes it to the
 //     roles of both CTAs through a ring in shared memory.  Items are ordered longest first, so the schedule is a greedy one whatever the mix
 //     of products; the order of the additions inside a tile does not depend on it;
+//   * what a role does between two chunks is kept short, for a chunk is 768 (BN = 128) or 1536 cycles of the tensor core and the roles took longer: the
+//     epilogue's loop has its width as a constant, waits that are over read no clock, an item arrives decoded.  In all, with the schedule below and
+//     roles that wait for the preceding kernel only where they need it: 2048 x 8192 x 512 from 58.5 to 44.3 us, 64 x 128 x 512 (one tile) from
+//     8.4 to 6.2 us, 256 x 256 tiles at one pass from 0.88 to 0.45 us a chunk;
 //   * each epilogue warp sends its 32 rows out itself, 32 columns at a time, through two 4 KB buffers and tensor stores (or reductions).
 //     An SM writes about 32 bytes a cycle to L2, 4096 cycles for its half of a 256 x 256 tile; with buffers that are refilled as they drain the
 //     warps are back at the next tile's chunks after about 2900 cycles, which is what the two accumulators hide of it.  (Whole rows through
@@ -24,6 +28,7 @@
 // NT = 3: FP32-accurate (hi hi + lo hi + hi lo).  NT = 1: hi parts only, the 11 leading significant bits (what a TF32 instruction reads of an
 // FP32 word, at twice its rate): the reduced-precision mode, for all but its smallest products (gg_single).
 #include <stdio.h>
+#include <type_traits>
 #include "gemm_tc.cuh"
 
 #define GG_MAXP 10               // products per launch
@@ -32,7 +37,12 @@
 #define GG_RING 4                // items the slowest role may lag behind the scheduling warp
 #define GG_AHEAD 8               // k blocks left to load of an item when the next one is asked for: enough to hide the hand-over, not more, so
                                  // that items go to the pairs that really are free first
-#define GG_THREADS 512
+#define GG_THREADS 384          // warps 0-3: loads, instructions, items; 4-11: epilogue
+// Registers of a thread of the one and of the other: 128 accumulators, 32 words on their way and the addresses need more than the 184 that sixteen warps
+// leave an epilogue thread; with twelve it has 216, and a chunk of 256 columns is drained in 800 cycles instead of 1300 (spills).  Their sum is what
+// the CTA is launched with (384 x 168).
+#define GG_REGS_LIGHT 72
+#define GG_REGS_EPI 216
 #define GG_EMPTY_ARRIVALS 19     // roles that take an item: producer and 8 epilogue warps in both CTAs, the MMA warp in the leader
 
 struct __align__(64) GgSeg {
@@ -45,11 +55,11 @@ struct __align__(64) GgSeg {
 struct __align__(64) GgProb {
     CUtensorMap c;               // FP32 {N, M}, boxes of 32 columns x 32 rows, 128-byte swizzle
     unsigned* out_amax;          // largest |C| is left here (whole tiles; the fix-up leaves it for split ones), or NULL
-    int M, N, tiles_m, tiles_n, seg0, nseg, kb, acc;
+    int M, N, bn, tiles_m, tiles_n, seg0, nseg, kb, acc;      // bn: width of its tiles
 };
 struct GgRun { int item0, prob, tile0, split, slot0; };      // items item0 .. : tiles tile0 .. of the product, `split` pieces each
 struct GgParams {
-    int nruns, items, nsegs;
+    int nruns, items, nsegs, nprob;
     unsigned* counter; int* status;
     CUtensorMap partial;         // workspace of the split tiles: {BN, 256 rows per piece}, the same boxes
     GgRun run[GG_MAXE];
@@ -57,36 +67,47 @@ struct GgParams {
     GgSeg seg[GG_MAXS];
 };
 
+__device__ __forceinline__ bool gg_try_cluster(uint32_t addr, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred P;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}"
+                 : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+    return done != 0;
+}
 __device__ __forceinline__ bool gg_wait_cluster(uint64_t* bar, uint32_t parity) {      // as mbar_wait, for data written by the other CTA of the pair
-    uint32_t addr = smem_u32(bar), done = 0;
-    long long t0 = clock64();
+    const uint32_t addr = smem_u32(bar);
+    if (gg_try_cluster(addr, parity)) return true;
+    const long long t0 = clock64();
     for (;;) {
-        asm volatile("{\n\t.reg .pred P;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}"
-                     : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-        if (done) return true;
+        if (gg_try_cluster(addr, parity)) return true;
         if (clock64() - t0 > TC_SPIN_CYCLES) return false;
     }
 }
-__device__ __forceinline__ void gg_arrive_release(uint32_t bar_cluster) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
+// An item's hand-over: decoded once by the warp that takes it from the counter (1000 cycles of table look-ups and divisions), not by every role.  The words
+// travel with their own completion on the receiver's barrier (st.async), and a role gives a slot back without a release: it has only read the slot.
+// Arrivals with release semantics waited 3000 cycles each for whatever their thread had in flight, half of a short item.
+struct __align__(16) GgItem { int prob, mt, nt, kb0, kb1, slot, split, pad; };      // prob: -1 after the last item; slot: of the workspace, where split
+__device__ __forceinline__ void gg_send_item(uint32_t slot_cluster, uint32_t bar_cluster, const GgItem& v) {
+    asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], 32;" ::"r"(bar_cluster) : "memory");
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(slot_cluster), "r"(v.prob), "r"(v.mt), "r"(v.nt), "r"(v.kb0), "r"(bar_cluster) : "memory");
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(slot_cluster + 16), "r"(v.kb1), "r"(v.slot), "r"(v.split), "r"(0), "r"(bar_cluster) : "memory");
+}
+__device__ __forceinline__ void gg_arrive_relaxed(uint32_t bar_cluster) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
 }
 
 __device__ __forceinline__ void af_arrive_local(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 struct GgWork { int prob, m0, n0, nb0, kb0, kb1, slot; bool split; };
-template <int BN>
-__device__ __forceinline__ void gg_decode(const GgParams& p, int item, int rank, GgWork& w) {
+__device__ __forceinline__ void gg_decode(const GgParams& p, int item, GgItem& w) {
     int r = 0;
     while (r + 1 < p.nruns && p.run[r + 1].item0 <= item) r++;
     const GgRun& run = p.run[r];
     const GgProb& pr = p.prob[run.prob];
     const int local = item - run.item0;
     const int t = run.split > 1 ? local / run.split : local, piece = run.split > 1 ? local % run.split : 0;
-    int mt, nt;
-    tc_raster(run.tile0 + t, pr.tiles_m, pr.tiles_n, TC_GROUP_M / 2, &mt, &nt);
+    tc_raster(run.tile0 + t, pr.tiles_m, pr.tiles_n, TC_GROUP_M / 2, &w.mt, &w.nt);
     w.prob = run.prob;
-    w.m0 = mt * 256 + rank * 128; w.n0 = nt * BN; w.nb0 = w.n0 + rank * (BN / 2);
     w.split = run.split > 1;
     w.slot = run.slot0 + local;
     w.kb0 = 0; w.kb1 = pr.kb;
@@ -106,6 +127,9 @@ struct GgShape {
     static constexpr int STAGES = BN == 256 ? 5 : 8;
     static constexpr int NBUF = BN == 256 ? 2 : 1;                 // output staging: blocks of 32 rows x 32 columns per epilogue warp
     static constexpr int STG = 8 * NBUF * 4096;
+    // accumulators in tensor memory.  Between a chunk's last instruction and the return of its accumulator lie a commit, the drain and two arrivals,
+    // as long as a chunk of the narrow tile takes: with two of them its instructions waited (2048 x 8192 x 512: 58.7 us, with four 54.3).
+    static constexpr int NACC = 512 / BN;
     static constexpr int SMEM = STAGES * STAGE + STG + 1024 + 512;
 };
 
@@ -114,19 +138,19 @@ __global__ void __launch_bounds__(GG_THREADS, 1)
 gg_kernel(const __grid_constant__ GgParams p) {
     using Sh = GgShape<BN, NT>;
     constexpr int NP = Sh::NP, A_PART = Sh::A_PART, STAGE = Sh::STAGE, STAGES = Sh::STAGES;
-    constexpr uint32_t TMEM_COLS = 2 * BN;
-    constexpr int COLS = BN / 2;                                   // columns per epilogue thread
+    constexpr int NACC = Sh::NACC;
+    constexpr uint32_t TMEM_COLS = NACC * BN;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* stg = smem + STAGES * STAGE;
     uint64_t* full = (uint64_t*)(stg + Sh::STG);
     uint64_t* empty = full + STAGES;
-    uint64_t* acc_full = empty + STAGES;          // [2]
-    uint64_t* acc_empty = acc_full + 2;           // [2]
-    uint64_t* item_full = acc_empty + 2;          // [GG_RING]
+    uint64_t* acc_full = empty + STAGES;          // [NACC]
+    uint64_t* acc_empty = acc_full + NACC;        // [NACC]
+    uint64_t* item_full = acc_empty + NACC;       // [GG_RING]
     uint64_t* item_empty = item_full + GG_RING;   // [GG_RING] (the leader's are used)
     uint64_t* item_req = item_empty + GG_RING;    // 1: the leader's producer asks for the next item
-    int* item_slot = (int*)(item_req + 1);
+    GgItem* item_slot = (GgItem*)(((uintptr_t)(item_req + 1) + 15) & ~(uintptr_t)15);
     uint32_t* tmem_slot = (uint32_t*)(item_slot + GG_RING);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -134,7 +158,7 @@ gg_kernel(const __grid_constant__ GgParams p) {
     const bool leader = rank == 0;
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }
+        for (int b = 0; b < NACC; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }
         mbar_init(item_req, 1);
         for (int b = 0; b < GG_RING; b++) { mbar_init(&item_full[b], 1); mbar_init(&item_empty[b], GG_EMPTY_ARRIVALS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -142,6 +166,7 @@ gg_kernel(const __grid_constant__ GgParams p) {
     if (warp == 3 && lane < p.nsegs) {            // the tensor maps on their way to the cache
         asm volatile("prefetch.tensormap [%0];" ::"l"(&p.seg[lane].a) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&p.seg[lane].b) : "memory");
+        if (lane < p.nprob) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.prob[lane].c) : "memory");
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS));
@@ -150,33 +175,41 @@ gg_kernel(const __grid_constant__ GgParams p) {
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();                           // the peer's barriers exist before anything signals them
-    sb_pdl_enter();                               // up to here nothing was read that the kernel before may still write
+    // Every role waits for the kernel before this one where it first touches what that may still write: the operands, the scale words, the counter.
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     bool ok = true;
-    // the n-th item of this CTA's roles: the first is the pair's number, the others are waited for, read, and their slot handed back; -1 after the last
-    auto next_item = [&](int n, bool arrive) -> int {
-        if (n == 0) return (int)(blockIdx.x >> 1);
-        const int s = (n - 1) % GG_RING;
-        if (!gg_wait_cluster(&item_full[s], ((n - 1) / GG_RING) & 1)) { ok = false; return -1; }
-        const int item = *(volatile int*)&item_slot[s];
-        __syncwarp(__activemask());
-        if (arrive) gg_arrive_release(mapa_u32(smem_u32(&item_empty[s]), 0));
-        return item;
+    // the n-th item of this CTA's roles: the first is the pair's number, the others are waited for, read, and their slot handed back; false after the last
+    auto next_item = [&](int n, bool arrive, int rk, GgWork& w) -> bool {
+        GgItem it;
+        if (n == 0) gg_decode(p, (int)(blockIdx.x >> 1), it);
+        else {
+            const int s = (n - 1) % GG_RING;
+            if (!gg_wait_cluster(&item_full[s], ((n - 1) / GG_RING) & 1)) { ok = false; return false; }
+            const uint32_t a = smem_u32(&item_slot[s]);
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(it.prob), "=r"(it.mt), "=r"(it.nt), "=r"(it.kb0) : "r"(a) : "memory");
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(it.kb1), "=r"(it.slot), "=r"(it.split), "=r"(it.pad) : "r"(a + 16) : "memory");
+            __syncwarp(__activemask());
+            if (arrive && it.prob >= -1 && it.pad == 0) gg_arrive_relaxed(mapa_u32(smem_u32(&item_empty[s]), 0));      // (always so: the arrival waits for the words)
+            if (it.prob < 0) return false;
+        }
+        const int bn = p.prob[it.prob].bn;
+        w.prob = it.prob; w.kb0 = it.kb0; w.kb1 = it.kb1; w.slot = it.slot; w.split = it.split != 0;
+        w.m0 = it.mt * 256 + rk * 128; w.n0 = it.nt * bn; w.nb0 = w.n0 + rk * (bn / 2);
+        return true;
     };
 
     const bool is_epi = warp >= 4 && warp < 12;
     if (!is_epi) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REGS_LIGHT));
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(GG_REGS_LIGHT));
         if (warp == 0) {
             // ---------------- TMA producer ----------------
             if (elect_one()) {
                 uint32_t git = 0;
                 for (int n = 0; ok; n++) {
-                    const int item = next_item(n, true);
-                    if (item < 0) break;
                     GgWork w;
-                    gg_decode<BN>(p, item, (int)rank, w);
+                    if (!next_item(n, true, (int)rank, w)) break;
+                    if (n == 0) sb_pdl_enter();
                     const GgProb& pr = p.prob[w.prob];
                     int off = 0, left = w.kb1 - w.kb0;
                     const int ask = min(left, GG_AHEAD);
@@ -186,6 +219,8 @@ gg_kernel(const __grid_constant__ GgParams p) {
                         const int lo = max(w.kb0, off) - off, hi = min(w.kb1, off + g.kb) - off;
                         off += g.kb;
                         const bool amn = (g.mn & 1) != 0, bmn = (g.mn & 2) != 0;
+                        const int boxes = (pr.bn + 127) / 128;                        // of 64 columns: an MN-major B is fetched in whole lines
+                        const uint32_t bytes = (uint32_t)(A_PART + (bmn ? boxes * 8192 : pr.bn * 64)) * 2;
                         for (int kb = lo; kb < hi && ok; kb++) {
                             if (left-- == ask && leader) af_arrive_local(item_req);
                             for (int part = 0; part < NP; part++, git++) {
@@ -193,7 +228,7 @@ gg_kernel(const __grid_constant__ GgParams p) {
                                 ok = mbar_wait(&empty[s], ((git / STAGES) & 1) ^ 1);
                                 if (!ok) break;
                                 uint8_t* st = smem + s * STAGE;
-                                if (leader) mbar_expect_tx(&full[s], STAGE * 2);      // both CTAs' bytes land on the leader's barrier
+                                if (leader) mbar_expect_tx(&full[s], bytes);      // both CTAs' bytes land on the leader's barrier
                                 const uint32_t fb = mapa_u32(smem_u32(&full[s]), 0);
                                 if (amn) {
 #pragma unroll
@@ -201,7 +236,7 @@ gg_kernel(const __grid_constant__ GgParams p) {
                                 } else tma_load_3d_pair(st, &g.a, fb, kb * 64, w.m0, part);
                                 if (bmn) {
 #pragma unroll
-                                    for (int j = 0; j < BN / 128; j++) tma_load_3d_pair(st + A_PART + j * 8192, &g.b, fb, w.nb0 + 64 * j, kb * 64, part);
+                                    for (int j = 0; j < BN / 128; j++) if (j < boxes) tma_load_3d_pair(st + A_PART + j * 8192, &g.b, fb, w.nb0 + 64 * j, kb * 64, part);
                                 } else tma_load_3d_pair(st + A_PART, &g.b, fb, kb * 64, w.nb0, part);
                             }
                         }
@@ -214,10 +249,8 @@ gg_kernel(const __grid_constant__ GgParams p) {
             if (leader && elect_one()) {
                 uint32_t git = 0, gch = 0;
                 for (int n = 0; ok; n++) {
-                    const int item = next_item(n, true);
-                    if (item < 0) break;
                     GgWork w;
-                    gg_decode<BN>(p, item, 0, w);
+                    if (!next_item(n, true, 0, w)) break;
                     const GgProb& pr = p.prob[w.prob];
                     int off = 0;
                     for (int sg = pr.seg0; sg < pr.seg0 + pr.nseg && ok; sg++) {
@@ -225,32 +258,40 @@ gg_kernel(const __grid_constant__ GgParams p) {
                         const int lo = max(w.kb0, off) - off, hi = min(w.kb1, off + g.kb) - off;
                         off += g.kb;
                         const bool amn = (g.mn & 1) != 0, bmn = (g.mn & 2) != 0;
-                        const uint32_t idesc = (1u << 4) | ((amn ? 1u : 0u) << 15) | ((bmn ? 1u : 0u) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+                        const uint32_t idesc = (1u << 4) | ((amn ? 1u : 0u) << 15) | ((bmn ? 1u : 0u) << 16) | ((uint32_t)(pr.bn >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
                         const uint64_t adva = amn ? 128 : 2, advb = bmn ? 128 : 2;      // 16 k in 16-byte units
+                        const int K = g.K;
+                        auto step = [&](uint32_t tmem_d, uint64_t a1, uint64_t b1, uint64_t a2, uint64_t b2, uint32_t acc) {
+                            // consecutive instructions share an operand (hi hi, lo hi, hi lo): with the narrow tile, whose operand reads take as long
+                            // as its arithmetic, all of hi hi first was 40 % slower
+                            tc_mma_f16_pair(tmem_d, a1, b1, idesc, acc);
+                            if (NT == 3) {
+                                tc_mma_f16_pair(tmem_d, a2, b1, idesc, 1);
+                                tc_mma_f16_pair(tmem_d, a1, b2, idesc, 1);
+                            }
+                        };
                         for (int kb = lo; kb < hi && ok; kb++, git += NP, gch++) {
-                            const int buf = gch & 1, s = git % STAGES, s2 = (git + 1) % STAGES;
-                            ok = mbar_wait(&acc_empty[buf], ((gch >> 1) & 1) ^ 1) && mbar_wait(&full[s], (git / STAGES) & 1);
+                            const int buf = gch % NACC, s = git % STAGES, s2 = (git + 1) % STAGES;
+                            ok = mbar_wait(&acc_empty[buf], ((gch / NACC) & 1) ^ 1) && mbar_wait(&full[s], (git / STAGES) & 1);
                             if (!ok) break;
                             tc_fence_after();
                             const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BN);
                             const uint32_t sa = smem_u32(smem + s * STAGE), sb = sa + A_PART;
                             const uint64_t a1 = amn ? make_mn16_desc<64>(sa) : make_kmajor_desc<128>(sa);
                             const uint64_t b1 = bmn ? make_mn16_desc<64>(sb) : make_kmajor_desc<128>(sb);
-                            const int nkk = min(4, (g.K - kb * 64 + 15) >> 4);      // the rest of a short last block is zeros
                             if (NT == 3) {
-                                // consecutive instructions share an operand (hi hi, lo hi, hi lo): with the narrow tile, whose operand reads take as long
-                                // as its arithmetic, all of hi hi first was 40 % slower
                                 ok = mbar_wait(&full[s2], ((git + 1) / STAGES) & 1);
                                 if (!ok) break;
                                 tc_fence_after();
-                                const uint64_t a2 = a1 + (uint64_t)((s2 - s) * (STAGE >> 4)), b2 = b1 + (uint64_t)((s2 - s) * (STAGE >> 4));
-                                for (int kk = 0; kk < nkk; kk++) {
-                                    tc_mma_f16_pair(tmem_d, a1 + kk * adva, b1 + kk * advb, idesc, kk ? 1u : 0u);
-                                    tc_mma_f16_pair(tmem_d, a2 + kk * adva, b1 + kk * advb, idesc, 1);
-                                    tc_mma_f16_pair(tmem_d, a1 + kk * adva, b2 + kk * advb, idesc, 1);
-                                }
+                            }
+                            const uint64_t lo_off = NT == 3 ? (uint64_t)((s2 - s) * (STAGE >> 4)) : 0, a2 = a1 + lo_off, b2 = b1 + lo_off;
+                            const int left = K - kb * 64;
+                            if (left >= 64) {
+#pragma unroll
+                                for (int kk = 0; kk < 4; kk++) step(tmem_d, a1 + kk * adva, b1 + kk * advb, a2 + kk * adva, b2 + kk * advb, kk ? 1u : 0u);
                             } else {
-                                for (int kk = 0; kk < nkk; kk++) tc_mma_f16_pair(tmem_d, a1 + kk * adva, b1 + kk * advb, idesc, kk ? 1u : 0u);
+                                for (int kk = 0; kk < (left + 15) >> 4; kk++)      // the rest of a short last block is zeros
+                                    step(tmem_d, a1 + kk * adva, b1 + kk * advb, a2 + kk * adva, b2 + kk * advb, kk ? 1u : 0u);
                             }
                             tc_commit_pair(&empty[s]);
                             if (NT == 3) tc_commit_pair(&empty[s2]);
@@ -264,76 +305,93 @@ gg_kernel(const __grid_constant__ GgParams p) {
             // ---------------- scheduler: hands the next item to the roles of both CTAs ----------------
             if (leader && elect_one()) {
                 const int G = gridDim.x / 2;
-                const uint32_t slot1 = mapa_u32(smem_u32(item_slot), 1), full1 = mapa_u32(smem_u32(item_full), 1), full0 = mapa_u32(smem_u32(item_full), 0);
+                sb_pdl_wait();
+                const uint32_t slot0 = mapa_u32(smem_u32(item_slot), 0), slot1 = mapa_u32(smem_u32(item_slot), 1), full1 = mapa_u32(smem_u32(item_full), 1), full0 = mapa_u32(smem_u32(item_full), 0);
                 for (int n = 0; ok; n++) {
                     const int s = n % GG_RING;
                     ok = mbar_wait(item_req, n & 1) && gg_wait_cluster(&item_empty[s], ((n / GG_RING) & 1) ^ 1);
                     if (!ok) break;
                     const int item = G + (int)atomicAdd(p.counter, 1u);
-                    const int v = item < p.items ? item : -1;
-                    *(volatile int*)&item_slot[s] = v;
-                    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(slot1 + (uint32_t)(s * 4)), "r"(v) : "memory");
-                    gg_arrive_release(full0 + (uint32_t)(s * 8));
-                    gg_arrive_release(full1 + (uint32_t)(s * 8));
-                    if (v < 0) break;
+                    GgItem v;
+                    v.prob = -1; v.mt = v.nt = v.kb0 = v.kb1 = v.slot = v.split = 0;
+                    if (item < p.items) gg_decode(p, item, v);
+                    gg_send_item(slot0 + (uint32_t)(s * sizeof(GgItem)), full0 + (uint32_t)(s * 8), v);
+                    gg_send_item(slot1 + (uint32_t)(s * sizeof(GgItem)), full1 + (uint32_t)(s * 8), v);
+                    if (v.prob < 0) break;
                 }
                 if (!ok) atomicExch(p.status, SB_ERR_TIMEOUT);
             }
         }
     } else {
         // ---------------- epilogue: chunks from tensor memory, scaled, into register accumulators; tiles to the staging buffer ----------------
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TC_REGS_EPI));
-        const int q = warp & 3, col0 = ((warp - 4) >> 2) * COLS;
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(GG_REGS_EPI));
+        const int q = warp & 3, half = (warp - 4) >> 2;
         const uint32_t sbuf = smem_u32(stg + (warp - 4) * Sh::NBUF * 4096);
         uint32_t gch = 0, pieces = 0;
+        sb_pdl_wait();
+        // The factor of each segment, in the lane of its number (read once: at every item the two words took 1400 cycles).  It undoes the operands'
+        // power-of-two scales; where their product leaves the float range it takes two multiplications.
+        float my_s1 = 0.f, my_s2 = 0.f;
+        if (lane < p.nsegs) {
+            const GgSeg& g = p.seg[lane];
+            const int e = -tc_f16_shift(sb_word(g.amax_a)) - tc_f16_shift(sb_word(g.amax_b));
+            const bool far = e < -120 || e > 120;
+            my_s1 = (far ? tc_pow2(e / 2) : tc_pow2(e)) * g.alpha; my_s2 = far ? tc_pow2(e - e / 2) : 0.f;
+        }
+        __syncwarp();
         for (int n = 0; ok; n++) {
-            const int item = next_item(n, lane == 0);
-            if (item < 0) break;
             GgWork w;
-            gg_decode<BN>(p, item, (int)rank, w);
+            if (!next_item(n, lane == 0, (int)rank, w)) break;
             const GgProb& pr = p.prob[w.prob];
-            float accr[COLS];
+            const int groups = pr.bn / 64, col0 = half * groups * 32;      // 32 columns at a time, half of the tile's per warp
+            float accr[BN / 2];
 #pragma unroll
-            for (int j = 0; j < COLS; j++) accr[j] = 0.f;
+            for (int j = 0; j < BN / 2; j++) accr[j] = 0.f;
             int off = 0;
             for (int sg = pr.seg0; sg < pr.seg0 + pr.nseg && ok; sg++) {
                 const GgSeg& g = p.seg[sg];
                 const int lo = max(w.kb0, off) - off, hi = min(w.kb1, off + g.kb) - off;
                 off += g.kb;
                 if (lo >= hi) continue;
-                // undo the operands' power-of-two scales; their product may leave the float range, then it takes two multiplications
-                const int e = -tc_f16_shift(sb_word(g.amax_a)) - tc_f16_shift(sb_word(g.amax_b));
-                const bool far = e < -120 || e > 120;
-                const float s1 = (far ? tc_pow2(e / 2) : tc_pow2(e)) * g.alpha, s2 = far ? tc_pow2(e - e / 2) : 1.f;
+                const float s1 = __shfl_sync(0xffffffffu, my_s1, sg), s2 = __shfl_sync(0xffffffffu, my_s2, sg);
+                const bool far = s2 != 0.f;
+                // W: groups of 32 columns of this warp, a constant of the loop; 0: `groups` of them with scales that take two factors
+                auto drain = [&](auto w_t) {
+                constexpr int W = decltype(w_t)::value;
+                constexpr bool FAR = W == 0;
                 for (int kb = lo; kb < hi && ok; kb++, gch++) {
-                    const int buf = gch & 1;
-                    ok = mbar_wait(&acc_full[buf], (gch >> 1) & 1);
+                    const int buf = gch % NACC;
+                    ok = mbar_wait(&acc_full[buf], (gch / NACC) & 1);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + col0);
 #pragma unroll
-                    for (int gi = 0; gi < COLS / 32; gi++) {
+                    for (int gi = 0; gi < (FAR ? BN / 64 : W); gi++) {
+                        if (FAR && gi >= groups) continue;
                         uint32_t r[32];
                         tc_ld32(taddr + (uint32_t)(gi * 32), r);
-                        if (gi == COLS / 32 - 1) {
+                        if (gi == (FAR ? groups : W) - 1) {
                             tc_fence_before();
                             __syncwarp();
                             if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[buf]), 0));
                         }
-                        if (!far) {
 #pragma unroll
-                            for (int j = 0; j < 32; j++) accr[gi * 32 + j] = fmaf(__uint_as_float(r[j]), s1, accr[gi * 32 + j]);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 32; j++) accr[gi * 32 + j] += __uint_as_float(r[j]) * s1 * s2;
-                        }
+                        for (int j = 0; j < 32; j++) accr[gi * 32 + j] = FAR ? accr[gi * 32 + j] + __uint_as_float(r[j]) * s1 * s2 : fmaf(__uint_as_float(r[j]), s1, accr[gi * 32 + j]);
                     }
                 }
+                };
+                // A loop for each width, and one for far scales, chosen outside: with the choices inside, a chunk of 256 columns cost the warps 1250 cycles
+                // instead of 640 (moves between copies of the accumulators), more than the tensor core takes for the single-pass form of it.
+                if (far) drain(std::integral_constant<int, 0>());
+                else if (BN == 256 && groups == 4) drain(std::integral_constant<int, BN / 64>());
+                else if (BN == 256 && groups == 3) drain(std::integral_constant<int, BN == 256 ? 3 : 1>());
+                else if (groups == 2) drain(std::integral_constant<int, 2>());
+                else drain(std::integral_constant<int, 1>());
             }
             if (pr.out_amax && !w.split) {
                 float m = 0.f;
 #pragma unroll
-                for (int j = 0; j < COLS; j++) m = fmaxf(m, fabsf(accr[j]));
+                for (int j = 0; j < BN / 2; j++) m = fmaxf(m, fabsf(accr[j]));
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
                 if (lane == 0 && m > 0.f) atomicMax(pr.out_amax, __float_as_uint(m));
@@ -343,9 +401,9 @@ gg_kernel(const __grid_constant__ GgParams p) {
             const int x0 = (w.split ? 0 : w.n0) + col0, y0 = (w.split ? (w.slot * 2 + (int)rank) * 128 : w.m0) + q * 32;
             const bool inside = w.split || y0 < pr.M, accf = !w.split && pr.acc;
 #pragma unroll
-            for (int g = 0; g < COLS / 32; g++, pieces++) {
-                if (!inside || !(w.split || x0 + g * 32 < pr.N)) continue;
-                const uint32_t buf = sbuf + (pieces % Sh::NBUF) * 4096;
+            for (int g = 0; g < BN / 64; g++) {
+                if (g >= groups || !inside || !(w.split || x0 + g * 32 < pr.N)) continue;
+                const uint32_t buf = sbuf + (pieces++ % Sh::NBUF) * 4096;      // the buffers in turn, whatever was skipped: the wait leaves the other one's store pending
                 if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(Sh::NBUF - 1) : "memory");      // what was staged here before has been read
                 __syncwarp();
 #pragma unroll
@@ -374,7 +432,7 @@ gg_kernel(const __grid_constant__ GgParams p) {
 }
 
 // Adds the pieces of the split tiles into C in piece order: one thread per four columns of one row, all products of the launch.
-struct GgFixRun { float* C; long ldc; unsigned* out_amax; int M, N, tiles_m, tiles_n, acc, tile0, split, slot0, block0; };
+struct GgFixRun { float* C; long ldc; unsigned* out_amax; int M, N, bn, tiles_m, tiles_n, acc, tile0, split, slot0, block0; };
 struct GgFixParams { int n, blocks, bn; const float* partial; GgFixRun f[GG_MAXP]; };
 static __global__ void __launch_bounds__(256) gg_fixup_kernel(const __grid_constant__ GgFixParams p) {
     sb_pdl_enter();
@@ -389,8 +447,8 @@ static __global__ void __launch_bounds__(256) gg_fixup_kernel(const __grid_const
     int mt, nt;
     tc_raster(f.tile0 + t, f.tiles_m, f.tiles_n, TC_GROUP_M / 2, &mt, &nt);
     const int r = i / bn4, col = (i % bn4) * 4;
-    const int row = mt * 256 + rank * 128 + r, c0 = nt * p.bn + col;
-    if (row >= f.M || c0 >= f.N) return;                        // N is a multiple of 4: a group of columns is inside or outside
+    const int row = mt * 256 + rank * 128 + r, c0 = nt * f.bn + col;
+    if (row >= f.M || c0 >= f.N || col >= f.bn) return;         // N is a multiple of 4: a group of columns is inside or outside
     const size_t block = (size_t)128 * p.bn;
     const float* p0 = p.partial + ((size_t)(f.slot0 + t * f.split) * 2 + rank) * block + (size_t)r * p.bn + col;
     float4* cp = (float4*)(f.C + (size_t)row * f.ldc + c0);
@@ -411,20 +469,33 @@ static __global__ void __launch_bounds__(256) gg_fixup_kernel(const __grid_const
 }
 
 // --------------------------------------------------------------------------- the schedule of a group
-// Whole tiles of 256 x 256 or 256 x 128, the last of them cut into pieces of the k range when that shortens the launch.  The cost of an item is
-// its k blocks plus an epilogue that the next item's first two chunks hide part of; a launch is the greedy schedule of its items on the CTA
-// pairs.  The constants (microseconds per k block of 64 at BN = 256 and 128, per epilogue, for the fix-up launch) are measured.
+// Every product has a tile width and may be cut into pieces of its k range; the last tiles of a launch are cut when that shortens it.  The kernel comes in two
+// classes: tiles of 128, 192 and 256 columns (five stages, two accumulators), and of 64 and 128 (eight and four).  The widest tile costs least per
+// multiply-add; a narrower one pays where the wide tiles leave the last round mostly empty (2816 columns of 2048 rows are 96 tiles of 256 on 74
+// pairs, two rounds, or 128 of 192: two shorter ones) and where one product's long k would outlast all others (a weight gradient over 2048 tokens
+// beside an input gradient over 512 columns).  The cost of an item is its k blocks plus an epilogue that the next item's first two chunks hide
+// part of; a launch is the greedy schedule of its items on the CTA pairs.  The constants (microseconds per k block of 64, per epilogue, for the
+// fix-up launch) are measured.
 struct GgPlanRun { int prob, tile0, tiles, split; };
-struct GgPlan { int bn, nruns; GgPlanRun run[GG_MAXE]; };
+struct GgPlan { int bn, nruns, w[GG_MAXP]; GgPlanRun run[GG_MAXE]; };
 struct GgPlanKey { int nprob, nt, G; int mnk[GG_MAXP][3]; };
 struct GgPlanEntry { GgPlanKey key; GgPlan plan; bool valid; };
 #define GG_PLANS 128
+#define GG_NARROWER 1.03f                     // a plan with narrower tiles has to win by more than the constants are worth
 
-static const float gg_t_kb[2][2] = {{0.95f, 0.50f}, {0.36f, 0.25f}}, gg_t_epi[2] = {4.0f, 2.4f}, gg_t_fix = 3.5f;      // [nt == 1][bn == 128]
+struct GgWidth { int bn; float t_kb[2], t_epi; };      // t_kb: three passes, one pass
+static const GgWidth gg_wide[3] = {{256, {1.00f, 0.47f}, 4.3f}, {192, {0.82f, 0.43f}, 3.5f}, {128, {0.64f, 0.38f}, 2.6f}};
+static const GgWidth gg_narrow[2] = {{128, {0.52f, 0.31f}, 2.3f}, {64, {0.42f, 0.27f}, 2.0f}};
+static const float gg_t_fix = 3.0f, gg_t_fix_col = 2e-4f;      // the fix-up launch, and for each column of 256 rows that it adds
 
 struct GgSim { float t[64]; int c[64]; int n; };
 // `count` items of one cost, each to the pair that is free first
-static void gg_sim_add(GgSim* s, int count, float cost) {
+static void gg_sim_add(GgSim* s, int count, float cost, int G) {
+    if (count > 4 * G) {                                         // whole rounds first
+        const int rounds = count / G - 2;
+        for (int i = 0; i < s->n; i++) s->t[i] += rounds * cost;
+        count -= rounds * G;
+    }
     while (count > 0) {
         int lo = 0;
         for (int i = 1; i < s->n; i++) if (s->t[i] < s->t[lo]) lo = i;
@@ -440,73 +511,123 @@ static void gg_sim_add(GgSim* s, int count, float cost) {
     }
 }
 static int gg_tiles(const int* mnk, int bn) { return ((mnk[0] + 255) / 256) * ((mnk[1] + bn - 1) / bn); }
+// What a plan chooses for each product: its tiles' width (of the class's table) and the pieces every one of them is cut into.
+struct GgPick { unsigned char w[GG_MAXP], s[GG_MAXP]; };
+static bool gg_can_cut(int kb, int s) { const int per = (kb + s - 1) / s; return s == 1 || (per * (s - 1) < kb && per >= 2); }
+// The launch of these choices; tail: pieces of the tiles that its last round holds, taken from the shortest uncut products (1: they stay whole).
+// Returns its time and the runs, or -1 when there is no such plan or none below `limit` (0: no limit).
+static float gg_eval(const GgPlanKey* k, const GgWidth* tab, const GgPick* c, int tail, float limit, GgPlan* p) {
+    float cost[GG_MAXP];
+    int order[GG_MAXP], tiles[GG_MAXP], spl[GG_MAXP], cut[GG_MAXP], total = 0;
+    const int one = k->nt == 1;
+    for (int i = 0; i < k->nprob; i++) {
+        cost[i] = k->mnk[i][2] * tab[c->w[i]].t_kb[one] + tab[c->w[i]].t_epi;
+        int j = i;
+        for (; j > 0 && cost[order[j - 1]] < cost[i]; j--) order[j] = order[j - 1];
+        order[j] = i;
+        tiles[i] = gg_tiles(k->mnk[i], tab[c->w[i]].bn);
+        spl[i] = c->s[i];
+        if (!gg_can_cut(k->mnk[i][2], spl[i])) return -1.f;
+        cut[i] = spl[i] > 1 ? tiles[i] : 0;
+        total += tiles[i] * spl[i];
+    }
+    if (tail > 1) {
+        int left = total % k->G;
+        if (left == 0) return -1.f;
+        bool any = false;
+        for (int o = k->nprob - 1; o >= 0 && left > 0; o--) {
+            const int i = order[o];
+            if (spl[i] > 1) continue;
+            if (!gg_can_cut(k->mnk[i][2], tail)) return -1.f;
+            spl[i] = tail; cut[i] = tiles[i] < left ? tiles[i] : left; left -= cut[i]; any = true;
+        }
+        if (!any) return -1.f;
+    }
+    GgPlanRun pieces[GG_MAXP]; float pcost[GG_MAXP]; int np = 0;
+    GgSim sim;
+    sim.n = 1; sim.t[0] = 0.f; sim.c[0] = k->G;
+    p->nruns = 0;
+    for (int i = 0; i < k->nprob; i++) {
+        if (!cut[i]) continue;
+        const float pc = (k->mnk[i][2] + spl[i] - 1) / spl[i] * tab[c->w[i]].t_kb[one] + tab[c->w[i]].t_epi;
+        int j = np++;
+        for (; j > 0 && pcost[j - 1] < pc; j--) { pieces[j] = pieces[j - 1]; pcost[j] = pcost[j - 1]; }
+        pieces[j] = {i, tiles[i] - cut[i], cut[i], spl[i]}; pcost[j] = pc;
+    }
+    if (limit > 0.f) {                                           // the work spread evenly, or the longest item: no schedule is shorter
+        float work = 0.f, longest = np ? pcost[0] : 0.f;
+        for (int i = 0; i < k->nprob; i++) if (tiles[i] > cut[i]) { work += (tiles[i] - cut[i]) * cost[i]; if (cost[i] > longest) longest = cost[i]; }
+        for (int a = 0; a < np; a++) work += pieces[a].tiles * pieces[a].split * pcost[a];
+        if ((work > longest * k->G ? work / k->G : longest) + (np ? gg_t_fix : 0.f) >= limit) return -1.f;
+    }
+    // longest items first, whole or pieces
+    float slots = 0.f;
+    for (int o = 0, a = 0; o < k->nprob || a < np; ) {
+        if (a == np || (o < k->nprob && cost[order[o]] >= pcost[a])) {
+            const int i = order[o++];
+            if (tiles[i] == cut[i]) continue;
+            p->run[p->nruns++] = {i, 0, tiles[i] - cut[i], 1};
+            gg_sim_add(&sim, tiles[i] - cut[i], cost[i], k->G);
+        } else {
+            p->run[p->nruns++] = pieces[a];
+            gg_sim_add(&sim, pieces[a].tiles * pieces[a].split, pcost[a], k->G);
+            slots += (float)(pieces[a].tiles * pieces[a].split) * tab[c->w[pieces[a].prob]].bn;
+            a++;
+        }
+    }
+    float t = 0.f;
+    for (int i = 0; i < sim.n; i++) if (sim.t[i] > t) t = sim.t[i];
+    if (np) t = (t + gg_t_fix + slots * gg_t_fix_col) * 1.02f;
+    for (int i = 0; i < k->nprob; i++) p->w[i] = tab[c->w[i]].bn;
+    p->bn = tab[0].bn;
+    return t;
+}
 static void gg_make_plan(const GgPlanKey* k, GgPlan* best) {
+    // products of one shape share their choice
+    int kind_of[GG_MAXP], nk = 0;
+    for (int i = 0; i < k->nprob; i++) {
+        kind_of[i] = -1;
+        for (int j = 0; j < i && kind_of[i] < 0; j++) if (memcmp(k->mnk[i], k->mnk[j], sizeof k->mnk[i]) == 0) kind_of[i] = kind_of[j];
+        if (kind_of[i] < 0) kind_of[i] = nk++;
+    }
+    static const unsigned char pieces[6] = {1, 2, 3, 4, 6, 8}, tails[6] = {2, 3, 4, 5, 6, 8};
     float best_t = 0.f;
     best->nruns = 0;
-    for (int wide = 1; wide >= 0; wide--) {
-        const int bn = wide ? 256 : 128;
-        const float tk = gg_t_kb[k->nt == 1][!wide], te = gg_t_epi[!wide];
-        int order[GG_MAXP], total = 0;
-        for (int i = 0; i < k->nprob; i++) {
-            int j = i;
-            for (; j > 0 && k->mnk[order[j - 1]][2] < k->mnk[i][2]; j--) order[j] = order[j - 1];
-            order[j] = i;
-            total += gg_tiles(k->mnk[i], bn);
-        }
-        // what is cut: nothing; the last `cut` tiles of the last products into s pieces; or everything into pieces of at most q k blocks
-        for (int kind = 0; kind < 12; kind++) {
-            GgPlan p;
-            p.bn = bn; p.nruns = 0;
-            GgPlanRun pieces[GG_MAXP]; int np = 0;
-            int cut_left = 0, s_tail = 1, q = 0;
-            if (kind >= 1 && kind <= 6) {
-                static const int ss[6] = {2, 3, 4, 5, 6, 8};
-                s_tail = ss[kind - 1];
-                cut_left = total % k->G;
-                if (cut_left == 0) continue;
-            } else if (kind > 6) {
-                static const int qs[5] = {3, 5, 8, 12, 20};
-                q = qs[kind - 7];
-                if (total >= k->G) continue;
-            }
-            // the tail is taken from the products with the shortest k, last in the order
-            int cut[GG_MAXP], spl[GG_MAXP];
-            for (int i = 0; i < k->nprob; i++) { cut[i] = 0; spl[i] = 1; }
-            bool any = false, bad = false;
-            for (int o = k->nprob - 1; o >= 0; o--) {
-                const int i = order[o], t = gg_tiles(k->mnk[i], bn), kb = k->mnk[i][2];
-                int s = s_tail;
-                if (q) { s = (kb + q - 1) / q; if (s > 8) s = 8; }
-                const int per = (kb + s - 1) / s;
-                if (s > 1 && (per * (s - 1) >= kb || per < 2)) { if (q) { s = 1; } else if (cut_left > 0) { bad = true; break; } }
-                if (q) { if (s > 1) { cut[i] = t; spl[i] = s; any = true; } }
-                else if (cut_left > 0 && s > 1) { cut[i] = t < cut_left ? t : cut_left; spl[i] = s; cut_left -= cut[i]; any = true; }
-            }
-            if (bad || (kind > 0 && !any)) continue;
-            GgSim sim;
-            sim.n = 1; sim.t[0] = 0.f; sim.c[0] = k->G;
-            for (int o = 0; o < k->nprob; o++) {
-                const int i = order[o], t = gg_tiles(k->mnk[i], bn), kb = k->mnk[i][2];
-                if (t > cut[i]) {
-                    p.run[p.nruns++] = {i, 0, t - cut[i], 1};
-                    gg_sim_add(&sim, t - cut[i], kb * tk + te);
-                }
-                if (cut[i]) pieces[np++] = {i, t - cut[i], cut[i], spl[i]};
-            }
-            for (int a = 1; a < np; a++)                         // longest pieces first
-                for (int b = a; b > 0; b--) {
-                    const int ka = (k->mnk[pieces[b].prob][2] + pieces[b].split - 1) / pieces[b].split, kp = (k->mnk[pieces[b - 1].prob][2] + pieces[b - 1].split - 1) / pieces[b - 1].split;
-                    if (ka > kp) { GgPlanRun x = pieces[b]; pieces[b] = pieces[b - 1]; pieces[b - 1] = x; } else break;
-                }
-            for (int a = 0; a < np; a++) {
-                const int kb = k->mnk[pieces[a].prob][2], per = (kb + pieces[a].split - 1) / pieces[a].split;
-                p.run[p.nruns++] = pieces[a];
-                gg_sim_add(&sim, pieces[a].tiles * pieces[a].split, per * tk + te);
-            }
-            float t = 0.f;
-            for (int i = 0; i < sim.n; i++) if (sim.t[i] > t) t = sim.t[i];
-            if (np) t = (t + gg_t_fix) * 1.03f;
+    GgPlan p;
+    for (int cls = 0; cls < 2; cls++) {
+        const GgWidth* tab = cls ? gg_narrow : gg_wide;
+        const int nw = cls ? 2 : 3;
+        int total = 0;
+        for (int i = 0; i < k->nprob; i++) total += gg_tiles(k->mnk[i], tab[0].bn);
+        const bool many = total > 6 * k->G;                      // many rounds: no empty last one to speak of, and no product that outlasts the rest
+        for (int base = 0; base < (many ? 1 : nw); base++) {
+            GgPick c;
+            memset(&c, 0, sizeof c);
+            for (int i = 0; i < k->nprob; i++) { c.w[i] = (unsigned char)base; c.s[i] = 1; }
+            const float off = cls || base ? GG_NARROWER : 1.f;
+            float t = gg_eval(k, tab, &c, 1, 0.f, &p) * off;
             if (best->nruns == 0 || t < best_t) { *best = p; best_t = t; }
+            // one kind of product after the other to its best choice beside the others'
+            for (int sweep = 0; sweep < (many ? 0 : 2); sweep++) {
+                bool moved = false;
+                for (int kd = 0; kd < nk; kd++) {
+                    GgPick top = c;
+                    for (int w = 0; w < nw; w++)
+                        for (int q = 0; q < 6; q++) {
+                            GgPick v = c;
+                            for (int i = 0; i < k->nprob; i++) if (kind_of[i] == kd) { v.w[i] = (unsigned char)w; v.s[i] = pieces[q]; }
+                            if (memcmp(&v, &c, sizeof v) == 0) continue;
+                            const float tv = gg_eval(k, tab, &v, 1, t, &p) * (cls || w || base ? GG_NARROWER : 1.f);
+                            if (tv > 0.f && tv < t) { t = tv; top = v; moved = true; if (t < best_t) { *best = p; best_t = t; } }
+                        }
+                    c = top;
+                }
+                if (!moved) break;
+            }
+            for (int q = 0; q < 6; q++) {
+                const float tv = gg_eval(k, tab, &c, tails[q], best_t, &p) * off;
+                if (tv > 0.f && tv < best_t) { *best = p; best_t = tv; }
+            }
         }
     }
 }
@@ -528,7 +649,10 @@ static bool gg_launch_t(sb_ctx_t* c, const GgParams& p, int G) {
     static_assert(smem <= 232448, "shared memory of one CTA");
     static bool attr_set = false;
     if (!attr_set) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return false;
+        cudaFuncAttributes fa;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess || cudaFuncGetAttributes(&fa, kern) != cudaSuccess) return false;
+        // setmaxnreg.inc takes from the registers the CTA was launched with and would wait for good on a build that has fewer
+        if (fa.numRegs * GG_THREADS < GG_REGS_LIGHT * 128 + GG_REGS_EPI * 256) return false;
         attr_set = true;
     }
     cudaLaunchConfig_t cfg;
@@ -664,7 +788,7 @@ static bool gg_run(sb_ctx_t* c, const sb_gemm_job_t* jobs, int njobs, int nt) {
     memset(&p, 0, sizeof p);
     GgPlanKey key;
     memset(&key, 0, sizeof key);
-    int np = 0;
+    int np = 0, of[GG_MAXS];      // of: product of each job
     double flops = 0, bytes = 0;
     for (int j = 0; j < njobs; j++) {
         const sb_gemm_job_t* b = &jobs[j];
@@ -678,6 +802,7 @@ static bool gg_run(sb_ctx_t* c, const sb_gemm_job_t* jobs, int njobs, int nt) {
         GgProb* q = &p.prob[np - 1];
         p.seg[j].K = b->K; p.seg[j].alpha = b->alpha == 0.f ? 1.f : b->alpha; p.seg[j].kb = (b->K + 63) / 64;
         q->nseg++; q->kb += p.seg[j].kb;
+        of[j] = np - 1;
     }
     const int sms = c->pub.gpu_sm_count > 0 ? c->pub.gpu_sm_count : 148;
     key.nprob = np; key.nt = nt; key.G = max(1, (sms - (c->gemm_reserve_sms < sms ? c->gemm_reserve_sms : 0)) / 2);
@@ -693,14 +818,15 @@ static bool gg_run(sb_ctx_t* c, const sb_gemm_job_t* jobs, int njobs, int nt) {
         p.seg[j].mn = (tA ? 1 : 0) | (tB ? 0 : 2);
         p.seg[j].amax_a = oa->amax; p.seg[j].amax_b = ob->amax;
         if (!gg_map(c, &p.seg[j].a, oa->h, oa->n, b->M, b->K, tA != 0, 128) ||
-            !gg_map(c, &p.seg[j].b, ob->h, ob->n, b->N, b->K, !tB, bn / 2)) return false;
+            !gg_map(c, &p.seg[j].b, ob->h, ob->n, b->N, b->K, !tB, plan->w[of[j]] / 2)) return false;
     }
     GgFixParams fx;
     fx.n = fx.blocks = 0; fx.bn = bn;
     int slots = 0;
     for (int i = 0; i < np; i++) {
         GgProb* q = &p.prob[i];
-        q->tiles_m = (q->M + 255) / 256; q->tiles_n = (q->N + bn - 1) / bn;
+        q->bn = plan->w[i];
+        q->tiles_m = (q->M + 255) / 256; q->tiles_n = (q->N + q->bn - 1) / q->bn;
         float* C = jobs[q->seg0].C;
         if (!q->acc) q->out_amax = sb_amax_take(c, C, (size_t)q->M * q->N);      // an announced output: the epilogue leaves max |C|
         if (!gg_map_out(c, &q->c, C, q->M, q->N)) return false;
@@ -712,13 +838,13 @@ static bool gg_run(sb_ctx_t* c, const sb_gemm_job_t* jobs, int njobs, int nt) {
         p.items += pr->tiles * pr->split;
         if (pr->split > 1) {
             GgFixRun* f = &fx.f[fx.n++];
-            f->C = jobs[q->seg0].C; f->ldc = q->N; f->out_amax = q->out_amax; f->M = q->M; f->N = q->N; f->tiles_m = q->tiles_m; f->tiles_n = q->tiles_n;
+            f->C = jobs[q->seg0].C; f->ldc = q->N; f->out_amax = q->out_amax; f->M = q->M; f->N = q->N; f->bn = q->bn; f->tiles_m = q->tiles_m; f->tiles_n = q->tiles_n;
             f->acc = q->acc; f->tile0 = pr->tile0; f->split = pr->split; f->slot0 = slots; f->block0 = fx.blocks;
             fx.blocks += pr->tiles * 2;
             slots += pr->tiles * pr->split;
         }
     }
-    p.nruns = plan->nruns; p.nsegs = njobs;
+    p.nruns = plan->nruns; p.nsegs = njobs; p.nprob = np;
     float* partial = nullptr;
     if (slots) {
         partial = (float*)sb_gemm_stage(c, 4, (size_t)slots * 2 * 128 * bn * sizeof(float));

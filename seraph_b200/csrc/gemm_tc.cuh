@@ -102,13 +102,18 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 // bounded wait; returns false when `limit` clock cycles passed without the phase completing
+__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred P;\n\tmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}"
+                 : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+    return done != 0;
+}
 __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, long long limit) {
-    uint32_t addr = smem_u32(bar), done = 0;
-    long long t0 = clock64();
+    const uint32_t addr = smem_u32(bar);
+    if (mbar_try(addr, parity)) return true;      // most waits of a running pipeline are over already: no clock for those
+    const long long t0 = clock64();
     for (;;) {
-        asm volatile("{\n\t.reg .pred P;\n\tmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}"
-                     : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-        if (done) return true;
+        if (mbar_try(addr, parity)) return true;
         if (clock64() - t0 > limit) return false;
     }
 }
@@ -192,7 +197,6 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
                  : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-
 // shared-memory matrix descriptor, K-major operand, rows of SWZ bytes (64 or 128), 8-row groups contiguous
 template <int SWZ>
 __device__ __forceinline__ uint64_t make_kmajor_desc(uint32_t smem_addr) {

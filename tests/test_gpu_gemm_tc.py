@@ -72,6 +72,31 @@ def test_grouped_kernel_at_tile_edges(ctx, M, N, K, tA, tB, acc):
     ctx.release(a, b, c)
 
 
+@pytest.mark.parametrize("mode", [4, 2])
+@pytest.mark.parametrize("tA,tB,acc", [(0, 1, 0), (0, 0, 1), (1, 0, 1)])
+@pytest.mark.parametrize("M,N,K", [(64, 512, 512), (64, 520, 1408), (512, 520, 1408), (2048, 2816, 256), (5800, 520, 512), (5800, 1000, 512), (10240, 344, 64),
+                                   (18944, 88, 64), (4096, 2048, 136)])
+def test_grouped_kernel_widths_of_tiles(ctx, M, N, K, tA, tB, acc, mode):
+    """Tiles of 64, 128, 192 and 256 columns, whole and in pieces, with ragged last tiles; several items per CTA pair where a warp sends an odd number of
+    blocks of a tile out (88 columns are three of a half tile's four), so that its staging buffers change turns.  The bounds are those of every product."""
+    r = np.random.default_rng(M + 2 * N + 3 * K + tA)
+    A = r.standard_normal((K, M) if tA else (M, K)).astype(np.float32)
+    B = r.standard_normal((N, K) if tB else (K, N)).astype(np.float32)
+    C0 = r.standard_normal((M, N)).astype(np.float32)
+    ref = (A.T if tA else A).astype(np.float64) @ (B.T if tB else B).astype(np.float64) + (C0 if acc else 0)
+    a, b, c = ctx.upload(A), ctx.upload(B), ctx.upload(C0)
+    ctx.set_gemm_mode(mode)
+    ctx.lib.cuda_train_matmul_transpose(ctx.h, a.b, b.b, c.b, M, N, K, tA, tB, acc)
+    out = c.numpy(shape=(M, N))
+    ctx.set_gemm_mode(4)
+    ctx.check()
+    bound = BOUND[4] if mode == 4 else BOUND[1]
+    assert rel_l2(out, ref) < bound, rel_l2(out, ref)
+    for y in range(0, M, 256):                        # a wrong tile does not hide in the norm of the whole
+        assert rel_l2(out[y:y + 256], ref[y:y + 256]) < 2 * bound
+    ctx.release(a, b, c)
+
+
 @pytest.mark.parametrize("tA,tB,acc", [(0, 1, 0), (0, 0, 1), (1, 0, 1)])
 @pytest.mark.parametrize("M,N,K,single", [(8, 512, 1024, 0), (24, 2048, 512, 0), (512, 16, 4096, 0), (64, 128, 248, 0), (64, 128, 256, 1), (32, 512, 128, 1)])
 def test_single_pass_mode_keeps_small_products_accurate(ctx, M, N, K, single, tA, tB, acc):
