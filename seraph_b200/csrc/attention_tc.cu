@@ -369,37 +369,24 @@ static AtParts at_make_parts(sb_ctx_t* c, const float* x, size_t n, __half* h, f
     AtParts p = {h, h + n, amax};
     return p;
 }
-// The same for several tensors, in one maximum and one split launch; their words are consecutive from need[0].amax (zeroed: by the caller)
-struct AtNeed { const float* x; size_t n; __half* h; float* amax; };
-static void at_make_parts_multi(sb_ctx_t* c, const AtNeed* need, int count, AtParts* out, bool zeroed) {
-    TcMulti am, sp;
-    cudaStream_t st = (cudaStream_t)c->pub.stream;
-    am.n = sp.n = 0; am.chunks = sp.chunks = 0;
+// The same for several tensors together; guess: two words of the call's own for each
+struct AtNeed { const float* x; size_t n; __half* h; float* amax; float* guess; };
+static void at_make_parts_multi(sb_ctx_t* c, const AtNeed* need, int count, AtParts* out) {
+    TcMulti sp;
+    tc_multi_begin(&sp);
     for (int i = 0; i < count; i++) {
-        __half* h = need[i].h; float* amax = need[i].amax;
+        __half* h = need[i].h; float *amax = need[i].amax, *guess = need[i].guess;
         const float* x = need[i].x; const size_t n = need[i].n;
         void* kept; float* kept_amax; int fresh = 1;
-        const bool reg = sb_parts_find(c, x, n, &kept, &kept_amax, &fresh) != 0;
-        if (reg) { h = (__half*)kept; amax = kept_amax; }
+        if (sb_parts_find(c, x, n, &kept, &kept_amax, &fresh)) { h = (__half*)kept; amax = kept_amax; guess = sb_parts_guess(c, x); }
         if (fresh) {
             float* left = sb_amax_lookup(c, x, n);
             if (left) { amax = left; sb_parts_set_amax(c, x, left); }
-            else {
-                if (reg) cudaMemsetAsync(amax, 0, sizeof(float), st);
-                else if (!zeroed) { cudaMemsetAsync(need[0].amax, 0, count * sizeof(float), st); zeroed = true; }
-                tc_multi_add(&am, x, n, nullptr, amax);
-            }
-            tc_multi_add(&sp, x, n, h, amax);
+            tc_multi_add(&sp, x, n, h, amax, left ? nullptr : guess);
         }
         out[i] = {h, h + n, amax};
-        // large tensors one by one, so that the split finds most of what the maximum pass read in L2 (126 MB): three tensors of 134 MB
-        // prepared together cost 2 % of a forward and backward call at 8 x 2048 tokens, 16 heads of 128
-        if ((size_t)(am.chunks + sp.chunks) * TC_MULTI_CHUNK * 16 > ((size_t)64 << 20) || i + 1 == count) {
-            tc_multi_amax(c, am);
-            tc_multi_split(c, sp);
-            am.n = sp.n = 0; am.chunks = sp.chunks = 0;
-        }
     }
+    tc_multi_split(c, sp);
 }
 // per-(token, head) vector (lse or D, laid out [token][Hq]) as seen by a launch over heads head0, head0+step, ...
 static TcEpi at_epi(int mode, float scale, const float* vec, int tok0, int Hq, int head0, int head_step, const float* aux) {
@@ -455,9 +442,9 @@ static int at_forward_one_kernel(sb_ctx_t* c, const float* Q, const float* K, co
     if (!consts) return 1;
     int tk = sb_tick_begin(c, SB_CLS_ATTN_FWD);
     __half* hb = (__half*)(consts + 64);
-    const AtNeed need[3] = {{Q, n_q, hb, consts + 8}, {K, n_kv, hb + 2 * n_q, consts + 9}, {V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10}};
+    const AtNeed need[3] = {{Q, n_q, hb, consts + 8, consts + 16}, {K, n_kv, hb + 2 * n_q, consts + 9, consts + 18}, {V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10, consts + 20}};
     AtParts p[3];
-    at_make_parts_multi(c, need, 3, p, false);
+    at_make_parts_multi(c, need, 3, p);
     if (!at_have_seq(c, T)) { sb_tick_end(c, tk, 0.0, 0.0); return 1; }
     double fl = 0;
     for (int b = 0; b < c->h_seq_n; b++) { const double S = c->h_seq[b + 1] - c->h_seq[b]; fl += 2.0 * Hq * S * S * hd; }
@@ -543,11 +530,10 @@ static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, cons
     int tk = sb_tick_begin(c, SB_CLS_ATTN_BWD);
     // words that start from zero: inside a step from its pool, else cleared here (a launch)
     float *am_do = sb_zero_word(c), *norm_do = sb_zero_word(c), *norm_v = sb_zero_word(c);
-    const bool cleared = !norm_v;
-    if (cleared) { cudaMemsetAsync(consts, 0, 64 * sizeof(float), st); norm_do = consts + 2; norm_v = consts + 3; am_do = consts + 11; }
-    const AtNeed need[3] = {{Q, n_q, hb, consts + 8}, {K, n_kv, hb + 2 * n_q, consts + 9}, {V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10}};
+    if (!norm_v) { cudaMemsetAsync(consts, 0, 64 * sizeof(float), st); norm_do = consts + 2; norm_v = consts + 3; am_do = consts + 11; }
+    const AtNeed need[3] = {{Q, n_q, hb, consts + 8, consts + 16}, {K, n_kv, hb + 2 * n_q, consts + 9, consts + 18}, {V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10, consts + 20}};
     AtParts p[3];
-    at_make_parts_multi(c, need, 3, p, cleared);
+    at_make_parts_multi(c, need, 3, p);
     __half* hdo = hb + 2 * n_q + 4 * n_kv;
     {
         const int rpb = 8 * 4 * (128 / hd);                          // rows a CTA takes per pass

@@ -692,30 +692,28 @@ extern "C" int sb_gemm_group_takes(sb_ctx_t* c, int M, int N, int K, int tA, int
     return gg_mode(c, &nt) && gg_shape_ok(M, N, K, tA, tB) ? 1 : 0;
 }
 
-struct GgOperand { const float* x; size_t n; __half* h; float* amax; bool fresh, kept; int slot; };      // kept: the parts outlive the step
+struct GgOperand { const float* x; size_t n; __half* h; float* amax; float* guess; bool fresh, kept; int slot; };      // kept: the parts outlive the step
 // the parts of an operand: those a producer or an earlier product of the step left, or a slot to make them in
 static int gg_operand(sb_ctx_t* c, GgOperand* ops, int* nops, const float* x, size_t n) {
     for (int i = 0; i < *nops; i++) if (ops[i].x == x && ops[i].n == n) return i;
     GgOperand* o = &ops[*nops];
     o->x = x; o->n = n; o->slot = -1; o->kept = false;
     void* h; int fresh;
-    if (sb_parts_find(c, x, n, &h, &o->amax, &fresh)) { o->h = (__half*)h; o->fresh = fresh != 0; o->kept = fresh == SB_PARTS_MAKE_KEPT; }
+    if (sb_parts_find(c, x, n, &h, &o->amax, &fresh)) { o->h = (__half*)h; o->fresh = fresh != 0; o->kept = fresh == SB_PARTS_MAKE_KEPT; o->guess = sb_parts_guess(c, x); }
     else {
         bool fr;
         const int s = sb_f16_slot(c, x, n, -1, &fr);
         if (s < 0) return -1;
         o->h = (__half*)c->f16_slot[s].h; o->fresh = fr; o->slot = s;
         if (fr) c->f16_slot[s].amax = c->d_amax + s;
-        o->amax = c->f16_slot[s].amax;
+        o->amax = c->f16_slot[s].amax; o->guess = c->d_amax + SB_F16_SLOTS + 2 * s;
     }
     return (*nops)++;
 }
-// Parts of the operands that have none yet: one maximum launch for those whose producer left none, one split launch.  Large ones in runs that
-// fit L2, so that the split finds what the maximum pass read.
+// Parts of the operands that have none yet, in one launch for those whose producer left their maximum and three where some have none
 static void gg_prepare(sb_ctx_t* c, GgOperand* ops, int n) {
-    cudaStream_t st = (cudaStream_t)c->pub.stream;
-    TcMulti am, sp;
-    am.n = sp.n = 0; am.chunks = sp.chunks = 0;
+    TcMulti sp;
+    tc_multi_begin(&sp);
     double bytes = 0;
     int tk = -1;
     bool any = false;
@@ -724,24 +722,11 @@ static void gg_prepare(sb_ctx_t* c, GgOperand* ops, int n) {
         if (o->fresh) {
             if (!any) { tk = sb_tick_begin(c, SB_CLS_GEMM_PREP); any = true; }
             float* left = o->kept ? NULL : sb_amax_lookup(c, o->x, o->n);
-            if (left) {
-                o->amax = left;
-                if (o->slot >= 0) c->f16_slot[o->slot].amax = left; else sb_parts_set_amax(c, o->x, left);
-            } else {
-                float* word = o->kept ? NULL : sb_zero_word(c); // zero already; outside a step the operand's own word
-                if (word) { o->amax = word; if (o->slot >= 0) c->f16_slot[o->slot].amax = word; else sb_parts_set_amax(c, o->x, word); }
-                else cudaMemsetAsync(o->amax, 0, sizeof(float), st);
-                tc_multi_add(&am, o->x, o->n, nullptr, o->amax);
-                bytes += 4.0 * o->n;
-            }
-            tc_multi_add(&sp, o->x, o->n, o->h, o->amax);
+            if (left) { o->amax = left; if (o->slot >= 0) c->f16_slot[o->slot].amax = left; else sb_parts_set_amax(c, o->x, left); }
+            tc_multi_add(&sp, o->x, o->n, o->h, o->amax, left ? nullptr : o->guess);
             bytes += 8.0 * o->n;
         }
-        if (sp.n == TC_MULTI || (sp.n && (i + 1 == n || (size_t)(am.chunks + sp.chunks) * TC_MULTI_CHUNK * 16 > ((size_t)64 << 20)))) {
-            tc_multi_amax(c, am);
-            tc_multi_split(c, sp);
-            am.n = sp.n = 0; am.chunks = sp.chunks = 0;
-        }
+        if (sp.n == TC_MULTI || i + 1 == n) { tc_multi_split(c, sp); tc_multi_begin(&sp); }
     }
     if (any) sb_tick_end(c, tk, 0.0, bytes);
 }
@@ -753,7 +738,7 @@ extern "C" void sb_parts_prepare(sb_ctx_t* c, const float* const* x, const size_
         for (; i0 < count && k < TC_MULTI; i0++) {
             void* h; int fresh;
             if (!sb_parts_find(c, x[i0], n[i0], &h, &ops[k].amax, &fresh)) continue;      // no parts for it: its products prepare it
-            ops[k].x = x[i0]; ops[k].n = n[i0]; ops[k].h = (__half*)h; ops[k].fresh = fresh != 0; ops[k].kept = fresh == SB_PARTS_MAKE_KEPT; ops[k].slot = -1;
+            ops[k].x = x[i0]; ops[k].n = n[i0]; ops[k].h = (__half*)h; ops[k].fresh = fresh != 0; ops[k].kept = fresh == SB_PARTS_MAKE_KEPT; ops[k].slot = -1; ops[k].guess = sb_parts_guess(c, x[i0]);
             k++;
         }
         gg_prepare(c, ops, k);

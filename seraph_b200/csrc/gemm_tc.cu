@@ -45,7 +45,7 @@ static bool prep_operand(sb_ctx_t* c, const float* src, int rows, int K, bool km
 // first and the least recently used one is taken on a miss; outside, the call's own slot `own` is used.  *fresh: the
 // parts must be made.  Returns the slot index, -1 on allocation failure.
 int sb_f16_slot(sb_ctx_t* c, const float* x, size_t n, int own, bool* fresh) {
-    if (!c->d_amax && sb_check(c, cudaMalloc(&c->d_amax, SB_F16_SLOTS * sizeof(float)), "amax alloc")) return -1;
+    if (!c->d_amax && sb_check(c, cudaMalloc(&c->d_amax, 3 * SB_F16_SLOTS * sizeof(float)), "amax alloc")) return -1;
     int s = own;
     *fresh = true;
     if (c->f16_keep) {
@@ -191,6 +191,13 @@ extern "C" float* sb_amax_lookup(sb_ctx_t* c, const float* x, size_t n) {
         if (c->hint_tab[i].ptr == x) return c->hint_tab[i].n == n ? c->hint_pool + i : NULL;      // the latest writer decides
     return NULL;
 }
+// the two words beside a registered tensor's own that the preparation of its parts uses
+extern "C" float* sb_parts_guess(sb_ctx_t* c, const float* x) {
+    size_t h = parts_hash_of(x, c->parts_hash_cap);
+    int idx;
+    while ((idx = c->parts_hash[h]) >= 0 && c->parts_tab[idx].ptr != x) h = (h + 1) & (size_t)(c->parts_hash_cap - 1);
+    return idx >= 0 && c->parts_amax ? c->parts_amax + c->parts_amax_cap + 2 * idx : NULL;
+}
 extern "C" void sb_parts_set_amax(sb_ctx_t* c, const float* x, float* word) {
     if (!c->parts_cache || !c->parts_open || !c->parts_n) return;
     size_t h = parts_hash_of(x, c->parts_hash_cap);
@@ -226,7 +233,7 @@ extern "C" int sb_parts_find(sb_ctx_t* c, const float* x, size_t n, void** hout,
         cudaStreamSynchronize((cudaStream_t)c->pub.stream);
         if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || fr < bytes || fr - bytes < tot / 8 ||
             cudaMalloc(&c->parts_arena, bytes) != cudaSuccess ||
-            cudaMalloc((void**)&c->parts_amax, (size_t)c->parts_n * sizeof(float)) != cudaSuccess) {
+            cudaMalloc((void**)&c->parts_amax, 3 * (size_t)c->parts_n * sizeof(float)) != cudaSuccess) {
             cudaGetLastError();
             if (c->parts_arena) cudaFree(c->parts_arena);
             c->parts_arena = NULL; c->parts_amax = NULL;

@@ -909,53 +909,62 @@ static __global__ void __launch_bounds__(256) tc_split_f16_kernel(const float* _
     }
 }
 
-// The same two passes over up to TC_MULTI tensors in one launch each: the tensors are cut into chunks of TC_MULTI_CHUNK float4, a CTA takes
-// an equal run of chunks.  Preparing a small model's operands is launches, not bytes: one launch instead of one or two per tensor.
-#define TC_MULTI 64
+// FP16 parts of up to TC_MULTI tensors with one read of each.  The scale of a tensor whose largest magnitude nobody left is a guess: four times the largest
+// of 16384 scattered elements, taken as if it were the maximum.  The pass that writes the parts compares every element with it, and a third launch makes
+// the parts again, with the true maximum, of a tensor that has a larger one (a single outlier among many millions); for all others it ends at once.  Parts
+// are floating point, so a scale that is two bits low costs nothing above 2^-15 of the largest element (sb_split2), and the scale is a function of the
+// tensor alone.  Bytes bound it, 12 for each element: three tensors of
+// 8 x 2048 x 2048 floats take 139 us, 131 of them in the split at 6.1 TB/s (198 with a pass for the maximum before it); small tensors are launches:
+// the 57 weights of the 33M model (120 MB) take three, 50 us (twelve and 78 when maximum and split passes ran in batches that fit L2).
+#define TC_MULTI 96
 #define TC_MULTI_CHUNK 1024
-struct TcMultiJob { const float* x; __half* h; float* amax; uint32_t n4, first; };      // h: hi parts, lo parts behind them; first: its first chunk
-struct TcMulti { int n; uint32_t chunks; unsigned keep; TcMultiJob j[TC_MULTI]; };
-static inline void tc_multi_add(TcMulti* m, const float* x, size_t n, void* h, float* amax) {
+#define TC_SAMPLE 4096                        // float4s looked at for the guess: 16 a thread
+// h: hi parts, lo parts behind them; first: its first chunk; amax: the word the products read; guess: NULL when *amax is there already, else two words
+// of the tensor's own: the guess, and the largest magnitude above it (zero when there is none)
+struct TcMultiJob { const float* x; __half* h; float* amax; float* guess; uint32_t n4, first; };
+struct TcMulti { int n, guesses; uint32_t chunks; unsigned keep; TcMultiJob j[TC_MULTI]; };
+static inline void tc_multi_begin(TcMulti* m) { m->n = m->guesses = 0; m->chunks = 0; }
+static inline void tc_multi_add(TcMulti* m, const float* x, size_t n, void* h, float* amax, float* guess) {
     TcMultiJob* j = &m->j[m->n++];
-    j->x = x; j->h = (__half*)h; j->amax = amax; j->n4 = (uint32_t)(n / 4); j->first = m->chunks;
+    j->x = x; j->h = (__half*)h; j->amax = amax; j->guess = guess; j->n4 = (uint32_t)(n / 4); j->first = m->chunks;
     m->chunks += (j->n4 + TC_MULTI_CHUNK - 1) / TC_MULTI_CHUNK;
+    if (guess) m->guesses++;
 }
 __device__ __forceinline__ int tc_multi_find(const TcMulti& m, uint32_t chunk) {
     int lo = 0, hi = m.n - 1;
     while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (m.j[mid].first <= chunk) lo = mid; else hi = mid - 1; }
     return lo;
 }
-static __global__ void __launch_bounds__(256) tc_amax_multi_kernel(const __grid_constant__ TcMulti m) {
+// a CTA per tensor; a tensor of up to TC_SAMPLE float4s is read whole, and its maximum is no guess
+static __global__ void __launch_bounds__(256) tc_guess_kernel(const __grid_constant__ TcMulti m) {
     sb_pdl_enter();
     __shared__ float red[8];
-    const uint32_t per = (m.chunks + gridDim.x - 1) / gridDim.x;
-    uint32_t ck = blockIdx.x * per;
-    const uint32_t end = min(m.chunks, ck + per);
-    while (ck < end) {
-        const int jb = tc_multi_find(m, ck);
-        const TcMultiJob& j = m.j[jb];
-        const uint32_t last = min(end, jb + 1 < m.n ? m.j[jb + 1].first : m.chunks);
-        const float4* x = (const float4*)j.x;
-        float mx = 0.f;
-        for (; ck < last; ck++) {
-            const uint32_t base = (ck - j.first) * TC_MULTI_CHUNK + threadIdx.x;
-            float4 v[TC_MULTI_CHUNK / 256];
+    const TcMultiJob& j = m.j[blockIdx.x];
+    if (!j.guess) return;
+    const float4* x = (const float4*)j.x;
+    const uint32_t lines = j.n4 >> 3, step = lines / (TC_SAMPLE >> 3);      // lines of 8 float4s (scattered float4s took 10 us for 57 tensors, lines 6)
+    float4 v[TC_SAMPLE / 256];
 #pragma unroll
-            for (int u = 0; u < TC_MULTI_CHUNK / 256; u++) v[u] = base + u * 256 < j.n4 ? __ldg(x + base + u * 256) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = 0; u < TC_SAMPLE / 256; u++) {
+        const uint32_t i = threadIdx.x + u * 256;
+        // one line of each run of `step`, at a place that does not repeat with the rows' length
+        const uint32_t l = i >> 3, at = step > 1 ? ((l * step + ((l * 2654435761u) >> 8) % step) << 3) + (i & 7) : i;
+        v[u] = at < j.n4 ? __ldg(x + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float mx = 0.f;
 #pragma unroll
-            for (int u = 0; u < TC_MULTI_CHUNK / 256; u++) mx = sb_amax4(mx, v[u]);
-        }
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[w]);
-            if (mx > 0.f) atomicMax((unsigned*)j.amax, __float_as_uint(mx));
-        }
-        __syncthreads();
+    for (int u = 0; u < TC_SAMPLE / 256; u++) mx = sb_amax4(mx, v[u]);
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[w]);
+        if (j.n4 > TC_SAMPLE) mx *= 4.f;
+        j.guess[0] = mx; j.guess[1] = 0.f; *j.amax = mx;
     }
 }
-// walks each CTA's run backwards: what the maximum pass read last is still in L2
+// A CTA takes an equal run of chunks, and walks it backwards: what a producer wrote last is still in L2.
+template <bool REDO>
 static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid_constant__ TcMulti m) {
     sb_pdl_enter();
     const uint32_t per = (m.chunks + gridDim.x - 1) / gridDim.x;
@@ -965,9 +974,17 @@ static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid
         const int jb = tc_multi_find(m, ck - 1);
         const TcMultiJob& j = m.j[jb];
         const uint32_t stop = max(begin, j.first);
+        float top = INFINITY;                 // what no element may exceed
+        if (REDO) {
+            const float above = j.guess ? sb_word(j.guess + 1) : 0.f;
+            if (above == 0.f) { ck = stop; continue; }
+            top = above;
+            if (stop == j.first && threadIdx.x == 0) *j.amax = above;      // nobody reads it in this launch
+        } else if (j.guess) top = sb_word(j.guess);
         const float4* x = (const float4*)j.x;
         uint2* h1 = (uint2*)j.h; uint2* h2 = h1 + j.n4;
-        const float sc = tc_pow2(tc_f16_shift(sb_word(j.amax)));
+        const float sc = tc_pow2(tc_f16_shift(!REDO && !j.guess ? sb_word(j.amax) : top));
+        float mx = 0.f;
         while (ck > stop) {
             ck--;
             const uint32_t base = (ck - j.first) * TC_MULTI_CHUNK + threadIdx.x;
@@ -977,26 +994,26 @@ static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid
 #pragma unroll
             for (int u = 0; u < TC_MULTI_CHUNK / 256; u++) if (base + u * 256 < j.n4) {
                 uint2 a, b;
+                if (!REDO) mx = sb_amax4(mx, v[u]);
                 sb_split2(v[u].x * sc, v[u].y * sc, a.x, b.x, m.keep); sb_split2(v[u].z * sc, v[u].w * sc, a.y, b.y, m.keep);
                 h1[base + u * 256] = a; h2[base + u * 256] = b;
             }
         }
+        if (!REDO && mx > top) atomicMax((unsigned*)(j.guess + 1), __float_as_uint(mx));
     }
 }
 static inline unsigned tc_multi_grid(sb_ctx_t* c, const TcMulti& m) {
     const unsigned cap = (unsigned)(c->pub.gpu_sm_count > 0 ? c->pub.gpu_sm_count : 148) * 8;
     return m.chunks < cap ? (m.chunks ? m.chunks : 1) : cap;
 }
-static inline void tc_multi_amax(sb_ctx_t* c, const TcMulti& m) {      // the words are zero before
-    if (!m.n) return;
-    sb_launch(tc_amax_multi_kernel, dim3(tc_multi_grid(c, m)), dim3(256), 0, (cudaStream_t)c->pub.stream, m);
-    c->launches++;
-}
 static inline void tc_multi_split(sb_ctx_t* c, TcMulti& m) {
     if (!m.n) return;
+    cudaStream_t st = (cudaStream_t)c->pub.stream;
     m.keep = sb_parts_keep(c);
-    sb_launch(tc_split_multi_kernel, dim3(tc_multi_grid(c, m)), dim3(256), 0, (cudaStream_t)c->pub.stream, m);
-    c->launches++;
+    if (m.guesses) sb_launch(tc_guess_kernel, dim3((unsigned)m.n), dim3(256), 0, st, m);
+    sb_launch(tc_split_multi_kernel<false>, dim3(tc_multi_grid(c, m)), dim3(256), 0, st, m);
+    if (m.guesses) sb_launch(tc_split_multi_kernel<true>, dim3(tc_multi_grid(c, m)), dim3(256), 0, st, m);
+    c->launches += m.guesses ? 3 : 1;
 }
 
 // --------------------------------------------------------------------------- operand preparation kernels

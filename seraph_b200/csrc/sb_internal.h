@@ -63,7 +63,7 @@ typedef struct sb_ctx {
     int status;                      /* last host-side status */
     int* d_status;                   /* device status word (bounds checks, bounded waits) */
     int gemm_mode;                   /* SB_GEMM_* (use_bf16 in pub overrides to BF16) */
-    float* d_amax;                   /* FP16 split: max |x| of the operand held by each part slot */
+    float* d_amax;                   /* FP16 split: max |x| of the operand held by each part slot, then two words of each for its preparation */
     struct { void* h; size_t cap; const float* ptr; size_t n; unsigned stamp; int valid; float* amax; } f16_slot[SB_F16_SLOTS];   /* FP16 parts of GEMM operands: all but the last two kept across
                                         calls inside a keep region (train_step.c marks runs of GEMMs that share operands), the last two for one call */
     int f16_keep; unsigned f16_clock;
@@ -239,9 +239,10 @@ float* sb_amax_lookup(sb_ctx_t*, const float* x, size_t n);
 int sb_bound_out(sb_ctx_t*, const float* x, size_t n, void** parts, float** word);
 float* sb_zero_word(sb_ctx_t*);      /* a device word that is zero until the step ends; NULL outside a step */
 void sb_parts_set_amax(sb_ctx_t*, const float* x, float* word);
+float* sb_parts_guess(sb_ctx_t*, const float* x);
 /* 1: x[n] is registered and the step is open; *h = its two parts (h, h + n), *amax its scale word, *fresh: 0 when they hold x, else they must be
-   made now.  Parts that outlive the step (SB_PARTS_MAKE_KEPT) take *amax as it is: a word of the step's pool (sb_zero_word, sb_amax_lookup) is
-   another tensor's in the next step. */
+   made now.  Parts that outlive the step (SB_PARTS_MAKE_KEPT) take *amax as it is: a word of the step's pool (sb_amax_lookup) is another
+   tensor's in the next step. */
 enum { SB_PARTS_MAKE = 1, SB_PARTS_MAKE_KEPT = 2 };
 int sb_parts_find(sb_ctx_t*, const float* x, size_t n, void** h, float** amax, int* fresh);
 void sb_parts_invalidate(sb_ctx_t*, const float* x);      /* x is rewritten as plain FP32: parts held for it are stale */

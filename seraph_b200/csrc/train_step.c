@@ -757,14 +757,13 @@ static int nan_tripped(sb_ctx_t* c, const train_state_t* st, int T) {
     return any;
 }
 
-/* The FP16 parts of every weight matrix the pass reads, in a few launches (tensors that fit L2 together share a maximum and a split
-   launch) instead of one or two per matrix at its first product. */
-#define PREP_BATCH_FLOATS ((size_t)10 << 20)
+/* The FP16 parts of every weight matrix the pass reads (and of the adapters), in a few launches instead of some per matrix at its first product */
+#define PREP_BATCH 96
 static void prepare_weights(sb_ctx_t* c, int T) {
     const int d = c->d, F = c->F, qd = c->qd, kvd = c->kvd;
     if (!sb_gemm_group_takes(c, T, qd, d, 0, 1) || !sb_gemm_group_takes(c, T, kvd, d, 0, 1) || !sb_gemm_group_takes(c, T, F, d, 0, 1) ||
         !sb_gemm_group_takes(c, T, d, F, 0, 1) || !sb_gemm_group_takes(c, T, d, qd, 0, 1) || !sb_gemm_group_takes(c, T, c->V, d, 0, 1)) return;
-    const float* x[64]; size_t n[64], sum = 0; int k = 0;
+    const float* x[PREP_BATCH]; size_t n[PREP_BATCH]; int k = 0;
     for (int l = -1; l < c->L; l++) {
         const sb_layer_off_t* o = l >= 0 ? &c->off[l] : NULL;
         const float* w[7]; size_t m[7]; int nw = 0;
@@ -776,15 +775,15 @@ static void prepare_weights(sb_ctx_t* c, int T) {
             nw = 7;
         }
         for (int i = 0; i < nw; i++) {
-            if (k && (k == 64 || sum + m[i] > PREP_BATCH_FLOATS)) { sb_parts_prepare(c, x, n, k); k = 0; sum = 0; }
-            x[k] = w[i]; n[k] = m[i]; sum += m[i]; k++;
+            if (k == PREP_BATCH) { sb_parts_prepare(c, x, n, k); k = 0; }
+            x[k] = w[i]; n[k] = m[i]; k++;
         }
     }
     for (int l = 0; l < c->L && c->lora_grouped; l++)
         for (int a = 0; a < 7; a++) {
             lora_ref_t r;
             if (!lora_get(c, l, a, &r)) continue;
-            if (k > 62) { sb_parts_prepare(c, x, n, k); k = 0; }
+            if (k > PREP_BATCH - 2) { sb_parts_prepare(c, x, n, k); k = 0; }
             x[k] = r.A; n[k++] = (size_t)c->lora_R * r.in; x[k] = r.B; n[k++] = (size_t)r.out * c->lora_R;
         }
     if (k) sb_parts_prepare(c, x, n, k);

@@ -118,6 +118,32 @@ def test_single_pass_mode_keeps_small_products_accurate(ctx, M, N, K, single, tA
     ctx.release(a, b, c)
 
 
+@pytest.mark.parametrize("kind", ["normal", "outlier", "one element", "zeros", "inf", "nan"])
+@pytest.mark.parametrize("M,N,K", [(512, 256, 1024), (64, 128, 256), (1000, 264, 136)])
+def test_scale_of_the_parts_is_checked_against_every_element(ctx, M, N, K, kind):
+    """The scale of an operand's FP16 parts is guessed from 16384 of its elements; one above four times the largest of those (an element that few samples
+    hit, the only one that is not zero) must give the scale of the true maximum, and not the overflow of the guessed one.  Operands that are
+    looked at whole (64 x 256) have no guess."""
+    r = np.random.default_rng(M + K)
+    A, B = r.standard_normal((M, K)).astype(np.float32), r.standard_normal((N, K)).astype(np.float32)
+    if kind in ("one element", "zeros"):
+        A[:] = 0
+    for y, x in ([(M - 3, K - 5), (M // 2, 77)] if kind not in ("normal", "zeros") else []):
+        A[y, x] = {"outlier": 3.0e5, "one element": -7.25, "inf": np.inf, "nan": np.nan}[kind]
+    a, b, c = ctx.upload(A), ctx.upload(B), ctx.zeros(M * N)
+    ctx.lib.cuda_train_matmul_transpose(ctx.h, a.b, b.b, c.b, M, N, K, 0, 1, 0)
+    out = c.numpy(shape=(M, N))
+    ctx.check()
+    if kind in ("inf", "nan"):
+        assert not np.isfinite(out[[M - 3, M // 2]]).any() and (kind == "inf" or np.isfinite(np.delete(out, [M - 3, M // 2], 0)).all())
+    else:
+        # parts hold 22 bits of what is within 2^-17 of the largest element (3e5 is 2^18: elements near 1 keep 21) and 2^-39 of it below
+        ref = A.astype(np.float64) @ B.T.astype(np.float64)
+        for y in range(0, M, 64):
+            assert rel_l2(out[y:y + 64], ref[y:y + 64]) < BOUND[4] or not ref[y:y + 64].any() and not out[y:y + 64].any()
+    ctx.release(a, b, c)
+
+
 def test_tc_gemm_long_k_and_reproducible(ctx):
     """K = 16384 (longer than the 8192-token reduction of the weight gradients): accumulation error stays in bound."""
     M, N, K = 256, 512, 16384
