@@ -69,12 +69,6 @@
 // 64-wide heads: dK 0..63, dV 64..127, K 128..191, the score buffers 192..319, and there is room for the parts of V, 320..383, and for a second
 // set of accumulators, 384..511.
 
-// A from tensor memory (M 128 lanes, 16 halfs of k = 8 columns), B from shared memory
-__device__ __forceinline__ void ab_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                 ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void ab_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
@@ -85,10 +79,6 @@ __device__ __forceinline__ void ab_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                      "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
 __device__ __forceinline__ void ab_ld_wait2(uint32_t (&a)[16], uint32_t (&b)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" : AB_REGS16(a), AB_REGS16(b) :: "memory");
-}
-__device__ __forceinline__ void ab_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 __device__ __forceinline__ void ab_red4(float* p, float a, float b, float c, float d) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
@@ -250,9 +240,9 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
                                 for (int kk = 0; kk < 4; kk++) {
                                     const uint64_t adv = (uint64_t)(kk * 2);
                                     const uint32_t ta = tk + (uint32_t)((p * 4 + kk) * 16);
-                                    ab_mma_ts(d, ta, b1 + adv, idesc_s, (p | kk) ? 1u : 0u);
-                                    ab_mma_ts(d, ta + 8, b1 + adv, idesc_s, 1);
-                                    ab_mma_ts(d, ta, b2 + adv, idesc_s, 1);
+                                    af_mma_ts(d, ta, b1 + adv, idesc_s, (p | kk) ? 1u : 0u);
+                                    af_mma_ts(d, ta + 8, b1 + adv, idesc_s, 1);
+                                    af_mma_ts(d, ta, b2 + adv, idesc_s, 1);
                                 }
                             }
                         }
@@ -268,13 +258,12 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
                                     const uint64_t adv = (uint64_t)(kk * 2);
                                     if constexpr (V_TMEM) {
                                         const uint32_t ta = tmem_base + (uint32_t)(COL_V + kk * 16);
-                                        ab_mma_ts(d, ta, b1 + adv, idesc_s, kk ? 1u : 0u);
-                                        ab_mma_ts(d, ta + 8, b1 + adv, idesc_s, 1);
-                                        ab_mma_ts(d, ta, b2 + adv, idesc_s, 1);
+                                        af_mma_ts(d, ta, b1 + adv, idesc_s, kk ? 1u : 0u);
+                                        af_mma_ts(d, ta + 8, b1 + adv, idesc_s, 1);
+                                        af_mma_ts(d, ta, b2 + adv, idesc_s, 1);
                                     } else {
-                                        af_mma_f16(d, a1 + adv, b1 + adv, idesc_s, (p | kk) ? 1u : 0u);
+                                        af_mma_f16_two(d, a1 + adv, b1 + adv, b2 + adv, idesc_s, (p | kk) ? 1u : 0u);
                                         af_mma_f16(d, a2 + adv, b1 + adv, idesc_s, 1);
-                                        af_mma_f16(d, a1 + adv, b2 + adv, idesc_s, 1);
                                     }
                                 }
                             }
@@ -303,9 +292,9 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
 #pragma unroll
                             for (int kk = 0; kk < 2; kk++) {
                                 const uint64_t advb = (uint64_t)(kk * 128);
-                                ab_mma_ts(d, ta + kk * 16, b1 + advb, idesc_o, (first && kk == 0) ? 0u : 1u);
-                                ab_mma_ts(d, ta + kk * 16 + 8, b1 + advb, idesc_o, 1);
-                                ab_mma_ts(d, ta + kk * 16, b2 + advb, idesc_o, 1);
+                                af_mma_ts(d, ta + kk * 16, b1 + advb, idesc_o, (first && kk == 0) ? 0u : 1u);
+                                af_mma_ts(d, ta + kk * 16 + 8, b1 + advb, idesc_o, 1);
+                                af_mma_ts(d, ta + kk * 16, b2 + advb, idesc_o, 1);
                             }
                         }
                         tc_commit(&empty[s]);
@@ -459,8 +448,8 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
                 asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(h8[4]), "=r"(h8[5]), "=r"(h8[6]), "=r"(h8[7]) : "r"(kt + c1) : "memory");
                 asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(l8[0]), "=r"(l8[1]), "=r"(l8[2]), "=r"(l8[3]) : "r"(kt + KV_PART + c0) : "memory");
                 asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(l8[4]), "=r"(l8[5]), "=r"(l8[6]), "=r"(l8[7]) : "r"(kt + KV_PART + c1) : "memory");
-                ab_st8(kcol + (uint32_t)(kk * 16), h8);
-                ab_st8(kcol + (uint32_t)(kk * 16 + 8), l8);
+                af_st8(kcol + (uint32_t)(kk * 16), h8);
+                af_st8(kcol + (uint32_t)(kk * 16 + 8), l8);
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
@@ -541,10 +530,10 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
             if (nomask) columns(std::false_type{}); else columns(std::true_type{});
             // The parts of these 16 queries go back over the 16 columns their scores came from (all of them are in registers by now):
             // hi part in the first 8 columns, lo part in the next 8, which is where the MMA issuer looks for k-step `ch`.
-            ab_st8(tmem_base + lane_addr + (uint32_t)(COL_S0 + 64 * e + ch * 16), p1);
-            ab_st8(tmem_base + lane_addr + (uint32_t)(COL_S0 + 64 * e + ch * 16 + 8), p2);
-            ab_st8(tmem_base + lane_addr + (uint32_t)(COL_S0 + 64 * e + 32 + ch * 16), d1);
-            ab_st8(tmem_base + lane_addr + (uint32_t)(COL_S0 + 64 * e + 32 + ch * 16 + 8), d2);
+            af_st8(tmem_base + lane_addr + (uint32_t)(COL_S0 + 64 * e + ch * 16), p1);
+            af_st8(tmem_base + lane_addr + (uint32_t)(COL_S0 + 64 * e + ch * 16 + 8), p2);
+            af_st8(tmem_base + lane_addr + (uint32_t)(COL_S0 + 64 * e + 32 + ch * 16), d1);
+            af_st8(tmem_base + lane_addr + (uint32_t)(COL_S0 + 64 * e + 32 + ch * 16 + 8), d2);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();

@@ -39,6 +39,24 @@ __device__ __forceinline__ void af_mma_f16(uint32_t tmem_d, uint64_t adesc, uint
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
                  ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// The same A twice in a row: the first instruction leaves it in the tensor core's collector, the second takes it from there instead of reading 4 KB of
+// shared memory again.  That is what an instruction of few columns waits for: 128 x 32 x 16 is 16 cycles of arithmetic and 40 of reads.
+__device__ __forceinline__ void af_mma_f16_two(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint64_t bdesc2, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %5, 0;\n\tsetp.eq.b32 q, %4, %4;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16.collector::a::fill [%0], %1, %2, %4, p;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16.collector::a::lastuse [%0], %1, %3, %4, q;\n\t}"
+                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "l"(bdesc2), "r"(idesc), "r"(accumulate) : "memory");
+}
+// A from tensor memory (M 128 lanes, 16 halfs of k = 8 columns), B from shared memory
+__device__ __forceinline__ void af_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void af_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
 __device__ __forceinline__ void af_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }

@@ -244,6 +244,33 @@ def test_attention_head128_one_kernel_paths(ctx, ss, Hq, Hkv, flash):
     ctx.release(bq, bk, bv, bdo, bs)
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("lens,Hq,Hkv", [([700, 1, 31, 32, 33, 127, 128, 129, 300, 513] * 3, 8, 4), ([64] * 40, 8, 8), ([385] * 7, 16, 2)])
+def test_attention_forward_several_tiles_per_cta(ctx, lens, Hq, Hkv, hd):
+    """The forward kernel's CTAs take tiles of 128 queries in turn: more of them than SMs, of one to many blocks of keys (odd and even counts, so that the
+    rings change turns), rows that leave as whole groups of 32 beside the last rows of a sequence, query blocks without rows."""
+    ss = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint32)
+    T, B = int(ss[-1]), len(lens)
+    r = rng(T + Hq + hd)
+    Q, K, V = f32(r.standard_normal((T, Hq * hd))), f32(r.standard_normal((T, Hkv * hd))), f32(r.standard_normal((T, Hkv * hd)))
+    out_ref, lse_ref = np.empty_like(Q), np.empty((T, Hq), np.float32)
+    O.lib().ref_attention(Q, K, V, out_ref, lse_ref, ss, T, B, Hq, Hkv, hd)
+    bq, bk, bv, bs = ctx.upload(Q), ctx.upload(K), ctx.upload(V), ctx.upload(ss)
+    runs = []
+    for rep in range(2):
+        bout, blse = ctx.zeros(Q.size), ctx.zeros(T * Hq)
+        ctx.lib.cuda_train_batch_attention_packed(ctx.h, bq.b, bk.b, bv.b, bout.b, blse.b, bs.b, T, B, Hq, Hkv, hd, max(lens))
+        ctx.check()
+        runs.append((bout.numpy(), blse.numpy()))
+        ctx.release(bout, blse)
+    assert np.array_equal(runs[0][0], runs[1][0]) and np.array_equal(runs[0][1], runs[1][1])
+    out, lse = runs[0][0].reshape(Q.shape), runs[0][1].reshape(T, Hq)
+    assert rel_l2(out, out_ref) < TOL and rel_l2(lse, lse_ref) < TOL
+    for b in range(B):                                # a wrong row does not hide in the norm of the whole
+        assert rel_l2(out[ss[b]:ss[b + 1]], out_ref[ss[b]:ss[b + 1]]) < 2 * TOL
+    ctx.release(bq, bk, bv, bs)
+
+
 @pytest.mark.parametrize("ss,Hq,Hkv,hd", [([0, 1, 3, 66, 194, 450, 963], 4, 2, 64), (list(range(0, 301 * 7, 7)), 2, 1, 64), ([0, 61], 8, 8, 64),
                                           ([0, 128, 256, 1280], 8, 2, 64), ([0, 5, 133, 900, 901], 4, 2, 128), ([0, 17], 2, 2, 128)])
 def test_attention_on_chip_short_and_ragged(ctx, ss, Hq, Hkv, hd):
