@@ -93,6 +93,9 @@ __device__ __forceinline__ void ab_tma_store(const CUtensorMap* map, uint32_t sr
 __device__ __forceinline__ void ab_tma_add(const CUtensorMap* map, uint32_t src, int c0, int c1) {
     asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(c0), "r"(c1), "r"(src) : "memory");
 }
+__device__ __forceinline__ void ab_bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
 #define AB_BULK_COMMIT() asm volatile("cp.async.bulk.commit_group;" ::: "memory")
 #define AB_BULK_WAIT_READ(n) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(n) : "memory")
 #define AB_BULK_WAIT(n) asm volatile("cp.async.bulk.wait_group %0;" ::"n"(n) : "memory")
@@ -160,6 +163,7 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
     uint64_t* k_full = k_ready + 1;                    // 1: K in shared memory, on its way there
     uint64_t* ew_sync = k_full + 1;                    // 1: the elementwise warps have staged their rows of a step's dS^T tiles
     uint32_t* tmem_slot = (uint32_t*)(ew_sync + 1);
+    float* rows_s = (float*)(smem + AB_OFF_BAR(NH) + 256);      // per stage the log-sum-exp and D of its 32 queries
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -200,13 +204,17 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
                     af_tma_2d(smem + p * 16384, &mV1, kv_full, kvh * HD + p * 64, t0 + k0);
                     af_tma_2d(smem + KV_PART + p * 16384, &mV2, kv_full, kvh * HD + p * 64, t0 + k0);
                 }
+                const int slot0 = af_slot_row(slot_pitch, Hq, b, kvh * g, t0, S), slot_rows = slot_pitch > 0 ? slot_pitch : (S + 127) & ~127;
                 for (int t = 0; t < nsteps && ok; t++) {
                     const int s = t % AB_STAGES, u = t / AB_STAGES;
                     const int h = kvh * g + t / per_head, j = j0 + t % per_head;
                     ok = mbar_wait(&empty[s], (u & 1) ^ 1);
                     if (!ok) break;
                     uint8_t* st = smem + AB_KV_BYTES(NH) + s * AB_STAGE_BYTES(NH);
-                    mbar_expect_tx(&full[s], AB_STAGE_BYTES(NH));
+                    mbar_expect_tx(&full[s], AB_STAGE_BYTES(NH) + 256);
+                    const size_t row = (size_t)(slot0 + t / per_head * slot_rows) + j * AB_BQ;
+                    ab_bulk_load(rows_s + s * 64, LT + row, 128, &full[s]);
+                    ab_bulk_load(rows_s + s * 64 + 32, DT + row, 128, &full[s]);
                     for (int p = 0; p < NH; p++) {
                         af_tma_2d(st + p * 4096, &mQ1, &full[s], h * HD + p * 64, t0 + j * AB_BQ);
                         af_tma_2d(st + ST_PART + p * 4096, &mQ2, &full[s], h * HD + p * 64, t0 + j * AB_BQ);
@@ -488,20 +496,20 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
         for (int t = 0; t < nsteps && ok; t++) {
             const int e = t & 1;
             const int q0 = j * AB_BQ;
-            ok = mbar_wait(&sdp_full[e], (t >> 1) & 1);
+            ok = mbar_wait(&sdp_full[e], (t >> 1) & 1) && mbar_wait(&full[t % AB_STAGES], (t / AB_STAGES) & 1);
             if (!ok) break;
             tc_fence_after();
             const int hb = slot0 + hi * slot_rows;
             uint32_t sr[16], dr[16];
             ab_ld16(tmem_base + lane_addr + (uint32_t)(COL_S0 + 64 * e + ch * 16), sr);
             ab_ld16(tmem_base + lane_addr + (uint32_t)(COL_S0 + 64 * e + 32 + ch * 16), dr);
-            // log-sum-exp (times log2 e) and D of this warp's 16 queries: the same addresses for every lane
+            // log-sum-exp (times log2 e) and D of this warp's 16 queries, which came with the step's tiles: the same addresses for every lane (from global memory
+            // they were late by most of a step's 1400 cycles of arithmetic)
             float4 L4[4], D4[4];
             {
-                const size_t o = (size_t)hb + q0 + ch * 16;
-                const float4* lp = (const float4*)(LT + o); const float4* dp = (const float4*)(DT + o);
+                const float4* lp = (const float4*)(rows_s + t % AB_STAGES * 64 + ch * 16);
 #pragma unroll
-                for (int i = 0; i < 4; i++) { L4[i] = __ldg(lp + i); D4[i] = __ldg(dp + i); }
+                for (int i = 0; i < 4; i++) { L4[i] = lp[i]; D4[i] = lp[8 + i]; }
             }
             ab_ld_wait2(sr, dr);
             uint32_t p1[8], p2[8], d1[8], d2[8];
@@ -543,13 +551,13 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
             // then all eight warps meet and it hands this step's tiles to the TMA unit.
             {
                 const uint32_t buf = ews + (uint32_t)(e * 16384);
-                const uint32_t row = buf + (uint32_t)(r * 64 + ch * 32);
+                const uint32_t row = buf + (uint32_t)(r * 64), x0 = (uint32_t)((2 * ch) ^ ((r >> 1) & 3)) << 4, x1 = x0 ^ 16;      // 64-byte swizzle: without it four lanes of eight met in a bank
                 if (warp != 4 && sync_n > 0) {                  // (the issuer's warp waited for this phase when it handed the tiles over)
                     ok = mbar_wait(ew_sync, (sync_n - 1) & 1);
                     if (!ok) break;
                 }
-                ab_sts4(row, d1[0], d1[1], d1[2], d1[3]); ab_sts4(row + 16, d1[4], d1[5], d1[6], d1[7]);
-                ab_sts4(row + 8192, d2[0], d2[1], d2[2], d2[3]); ab_sts4(row + 8192 + 16, d2[4], d2[5], d2[6], d2[7]);
+                ab_sts4(row + x0, d1[0], d1[1], d1[2], d1[3]); ab_sts4(row + x1, d1[4], d1[5], d1[6], d1[7]);
+                ab_sts4(row + 8192 + x0, d2[0], d2[1], d2[2], d2[3]); ab_sts4(row + 8192 + x1, d2[4], d2[5], d2[6], d2[7]);
                 AB_FENCE_ASYNC();
                 __syncwarp();
                 if (issuer) AB_BULK_WAIT_READ(0);
@@ -756,7 +764,7 @@ static int ab_launch(sb_ctx_t* c, const AbCall& p) {
         !af_make_map(c, &mK1, p.k1, p.T, kvd, AB_BK) || !af_make_map(c, &mK2, p.k2, p.T, kvd, AB_BK) ||
         !af_make_map(c, &mV1, p.v1, p.T, kvd, AB_BK) || !af_make_map(c, &mV2, p.v2, p.T, kvd, AB_BK)) return 1;
     {
-        // dS^T parts: [rows of the head slots: keys][Sp queries] halfs, tiles of 32 queries x 128 keys, plain rows of 64 bytes in shared memory;
+        // dS^T parts: [rows of the head slots: keys][Sp queries] halfs, tiles of 32 queries x 128 keys, rows of 64 bytes with the 64-byte swizzle in shared memory;
         // dK, dV: [T][kvd] floats, tiles of 32 columns x 32 keys, 128-byte swizzle
         const cuuint64_t rows = af_slot_rows(slot_pitch, p.Hq, seqs.n, p.T);
         const cuuint64_t sd[2] = {(cuuint64_t)p.Sp, rows}, ss[1] = {(cuuint64_t)p.Sp * 2};
@@ -765,8 +773,8 @@ static int ab_launch(sb_ctx_t* c, const AbCall& p) {
         const cuuint32_t gbx[2] = {32u, 32u};
         const CUtensorMapL2promotion np = CU_TENSOR_MAP_L2_PROMOTION_NONE;
         if (rows > 0x7fffffffull || !tc_aligned16(p.dS1) || !tc_aligned16(p.dS2) ||
-            !tc_encode(c, &mS1, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.dS1, sd, ss, sbx, CU_TENSOR_MAP_SWIZZLE_NONE, np) ||
-            !tc_encode(c, &mS2, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.dS2, sd, ss, sbx, CU_TENSOR_MAP_SWIZZLE_NONE, np) ||
+            !tc_encode(c, &mS1, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.dS1, sd, ss, sbx, CU_TENSOR_MAP_SWIZZLE_64B, np) ||
+            !tc_encode(c, &mS2, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.dS2, sd, ss, sbx, CU_TENSOR_MAP_SWIZZLE_64B, np) ||
             !tc_encode(c, &mdK, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, p.dK, gd, gs, gbx, CU_TENSOR_MAP_SWIZZLE_128B, np) ||
             !tc_encode(c, &mdV, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, p.dV, gd, gs, gbx, CU_TENSOR_MAP_SWIZZLE_128B, np)) return 1;
         if (p.dQ && (!tc_encode(c, &mA1, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.dS1, sd, ss, abx, CU_TENSOR_MAP_SWIZZLE_128B) ||
