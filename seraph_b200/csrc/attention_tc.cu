@@ -549,7 +549,7 @@ static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, cons
     if (at_have_seq(c, T)) n = c->h_seq_n;
     for (int b = 0; b < n; b++) { const int S = c->h_seq[b + 1] - c->h_seq[b]; Smax = max(Smax, S); flops += 5.0 * Hq * (double)S * S * hd; }
     if (Smax <= 0) { sb_tick_end(c, tk, 0.0, 0.0); return 1; }
-    // Long sequences of 128-wide heads: dQ from the CTA-pair GEMM kernel (256-row tiles read K half as often), a launch per sequence.
+    // Long sequences of 128-wide heads: dQ from the kernel of grouped products (256-row tiles read K half as often).
     // Shorter ones and 64-wide heads: at_dq_bwd_kernel, one launch for all.  8 x 2048 tokens, 16 heads: 1.57 against 1.67 ms for the whole
     // call; 5 sequences of 1080 on average: equal; 33M model, 24 sequences of 240: a launch instead of 24.
     const bool dq_gemm = hd == 128 && (long)n * 1024 <= T;
@@ -569,23 +569,7 @@ static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, cons
                    a, a + n_ds, dK, dV, dq_gemm ? nullptr : dQ, accumulate_kv, Sp, T, Hq, Hkv, nullptr, nullptr, nullptr};
     if (hd == 64 && !accumulate_kv) { call.amax_dq = sb_amax_take(c, dQ, n_q); call.amax_dk = sb_amax_take(c, dK, n_kv); call.amax_dv = sb_amax_take(c, dV, n_kv); }
     bool ok = sb_attention_fused_dkv(c, call, hd) == 0;
-    if (ok && dq_gemm) {
-        void* main_stream = c->pub.stream;
-        const int ns = at_fork(c, n);
-        const long sb = (long)Sp * Sp;
-        for (int b = 0; b < n && ok; b++) {
-            const int t0 = c->h_seq[b], S = c->h_seq[b + 1] - t0;
-            if (S <= 0) continue;
-            if (ns > 1) c->pub.stream = c->side_stream[b % ns];
-            // all query heads of the sequence in one launch: head h reads slot b Hq + h of dS^T and K/V head h / g
-            const AtParts pds = {a + (size_t)b * Hq * sb, a + n_ds + (size_t)b * Hq * sb, consts + 1};
-            TcOperand kop = op_tokens_mn(K, p[1], t0, kvd, Hkv, hd, 0, 1);
-            kop.c2_div = g;
-            ok = ok && at_gemm(c, op_scratch(bb, pds, S, Sp, Hq, 1), kop, dQ + (size_t)t0 * qd, qd, (long)hd, S, hd, S, 0, Hq,
-                               TC_CAUSAL_K_UPTO_M, nullptr, pds.amax, p[1].amax);
-        }
-        at_join(c, ns, main_stream);
-    }
+    if (ok && dq_gemm) ok = sb_gemm_dq(c, a, n_ds, consts + 1, p[1].h1, (size_t)(p[1].h2 - p[1].h1), p[1].amax, dQ, c->h_seq, n, Sp, Hq, g) == 0;
     sb_tick_end(c, tk, flops, 0.0);
     if (!ok) sb_set_status(c, SB_ERR_CUDA);
     return ok ? 0 : 1;

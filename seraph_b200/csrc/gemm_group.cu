@@ -60,6 +60,7 @@ struct __align__(64) GgProb {
 struct GgRun { int item0, prob, tile0, split, slot0; };      // items item0 .. : tiles tile0 .. of the product, `split` pieces each
 struct GgParams {
     int nruns, items, nsegs, nprob;
+    int heads, group;            // BATCH: query heads, and those of one K/V head
     unsigned* counter; int* status;
     CUtensorMap partial;         // workspace of the split tiles: {BN, 256 rows per piece}, the same boxes
     GgRun run[GG_MAXE];
@@ -95,16 +96,26 @@ __device__ __forceinline__ void gg_arrive_relaxed(uint32_t bar_cluster) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
 }
 
+__device__ __forceinline__ void gg_load_4d_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(bar_cluster), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
 __device__ __forceinline__ void af_arrive_local(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-struct GgWork { int prob, m0, n0, nb0, kb0, kb1, slot; bool split; };
+struct GgWork { int prob, m0, n0, nb0, kb0, kb1, slot, head; bool split; };
+template <bool BATCH>
 __device__ __forceinline__ void gg_decode(const GgParams& p, int item, GgItem& w) {
     int r = 0;
     while (r + 1 < p.nruns && p.run[r + 1].item0 <= item) r++;
     const GgRun& run = p.run[r];
     const GgProb& pr = p.prob[run.prob];
     const int local = item - run.item0;
+    if constexpr (BATCH) {                                         // the lowest rows first: they have the most k
+        w.prob = run.prob; w.mt = pr.tiles_m - 1 - local / p.heads; w.nt = local % p.heads;
+        w.split = w.slot = w.kb0 = 0; w.kb1 = min(pr.kb, (w.mt + 1) * 4);
+        return;
+    }
     const int t = run.split > 1 ? local / run.split : local, piece = run.split > 1 ? local % run.split : 0;
     tc_raster(run.tile0 + t, pr.tiles_m, pr.tiles_n, TC_GROUP_M / 2, &w.mt, &w.nt);
     w.prob = run.prob;
@@ -133,7 +144,7 @@ struct GgShape {
     static constexpr int SMEM = STAGES * STAGE + STG + 1024 + 512;
 };
 
-template <int BN, int NT>
+template <int BN, int NT, bool BATCH>
 __global__ void __launch_bounds__(GG_THREADS, 1)
 gg_kernel(const __grid_constant__ GgParams p) {
     using Sh = GgShape<BN, NT>;
@@ -182,7 +193,7 @@ gg_kernel(const __grid_constant__ GgParams p) {
     // the n-th item of this CTA's roles: the first is the pair's number, the others are waited for, read, and their slot handed back; false after the last
     auto next_item = [&](int n, bool arrive, int rk, GgWork& w) -> bool {
         GgItem it;
-        if (n == 0) gg_decode(p, (int)(blockIdx.x >> 1), it);
+        if (n == 0) gg_decode<BATCH>(p, (int)(blockIdx.x >> 1), it);
         else {
             const int s = (n - 1) % GG_RING;
             if (!gg_wait_cluster(&item_full[s], ((n - 1) / GG_RING) & 1)) { ok = false; return false; }
@@ -195,7 +206,7 @@ gg_kernel(const __grid_constant__ GgParams p) {
         }
         const int bn = p.prob[it.prob].bn;
         w.prob = it.prob; w.kb0 = it.kb0; w.kb1 = it.kb1; w.slot = it.slot; w.split = it.split != 0;
-        w.m0 = it.mt * 256 + rk * 128; w.n0 = it.nt * bn; w.nb0 = w.n0 + rk * (bn / 2);
+        w.m0 = it.mt * 256 + rk * 128; w.n0 = it.nt * bn; w.nb0 = (BATCH ? it.nt / p.group * bn : w.n0) + rk * (bn / 2); w.head = it.nt;
         return true;
     };
 
@@ -232,7 +243,9 @@ gg_kernel(const __grid_constant__ GgParams p) {
                                 const uint32_t fb = mapa_u32(smem_u32(&full[s]), 0);
                                 if (amn) {
 #pragma unroll
-                                    for (int j = 0; j < 2; j++) tma_load_3d_pair(st + j * 8192, &g.a, fb, w.m0 + 64 * j, kb * 64, part);
+                                    for (int j = 0; j < 2; j++)
+                                        if constexpr (BATCH) gg_load_4d_pair(st + j * 8192, &g.a, fb, w.m0 + 64 * j, kb * 64, w.head, part);
+                                        else tma_load_3d_pair(st + j * 8192, &g.a, fb, w.m0 + 64 * j, kb * 64, part);
                                 } else tma_load_3d_pair(st, &g.a, fb, kb * 64, w.m0, part);
                                 if (bmn) {
 #pragma unroll
@@ -314,7 +327,7 @@ gg_kernel(const __grid_constant__ GgParams p) {
                     const int item = G + (int)atomicAdd(p.counter, 1u);
                     GgItem v;
                     v.prob = -1; v.mt = v.nt = v.kb0 = v.kb1 = v.slot = v.split = 0;
-                    if (item < p.items) gg_decode(p, item, v);
+                    if (item < p.items) gg_decode<BATCH>(p, item, v);
                     gg_send_item(slot0 + (uint32_t)(s * sizeof(GgItem)), full0 + (uint32_t)(s * 8), v);
                     gg_send_item(slot1 + (uint32_t)(s * sizeof(GgItem)), full1 + (uint32_t)(s * 8), v);
                     if (v.prob < 0) break;
@@ -642,9 +655,9 @@ static const GgPlan* gg_plan(sb_ctx_t* c, const GgPlanKey* key) {
     return &e->plan;
 }
 
-template <int BN, int NT>
+template <int BN, int NT, bool BATCH = false>
 static bool gg_launch_t(sb_ctx_t* c, const GgParams& p, int G) {
-    auto kern = gg_kernel<BN, NT>;
+    auto kern = gg_kernel<BN, NT, BATCH>;
     constexpr int smem = GgShape<BN, NT>::SMEM;
     static_assert(smem <= 232448, "shared memory of one CTA");
     static bool attr_set = false;
@@ -873,4 +886,52 @@ extern "C" int sb_gemm_group_try(sb_ctx_t* c, const sb_gemm_job_t* jobs, int njo
     if (!keep) sb_gemm_keep_end(c);
     if (!ok) sb_set_status(c, SB_ERR_CUDA);
     return 0;
+}
+
+// dQ = dS K of an attention backward: for every sequence and query head [S, 128] from the parts of dS^T ([slot = sequence, head][key][query], rows of Sp) and of
+// K.  The query rows of a tile of 256 need the keys up to its last row.  A product is a sequence; its tiles of all heads are items of one launch, which
+// takes GG_MAXP sequences.  (A launch per sequence of gemm_tc_kernel, two of them side by side: 8 x 2048 tokens, 16 heads, 296 us; the parts of dS
+// alone, 1.07 GB, take 164.)  starts: boundaries on the host.  0: launched.
+extern "C" int sb_gemm_dq(sb_ctx_t* c, const void* ds, size_t ds_part, const float* ds_bound, const void* k, size_t k_part, const float* amax_k, float* dQ,
+                          const int* starts, int nseq, int Sp, int Hq, int g) {
+    if (!tc_load_encode()) return 1;
+    const int qd = Hq * 128, kvd = qd / g;
+    const int sms = c->pub.gpu_sm_count > 0 ? c->pub.gpu_sm_count : 148, pairs = max(1, (sms - (c->gemm_reserve_sms < sms ? c->gemm_reserve_sms : 0)) / 2);
+    for (int b0 = 0; b0 < nseq; ) {
+        GgParams p;
+        memset(&p, 0, sizeof p);
+        int seq[GG_MAXP], n = 0;
+        for (; b0 < nseq && n < GG_MAXP; b0++) {                  // the longest first
+            const int S = starts[b0 + 1] - starts[b0];
+            if (S <= 0) continue;
+            int j = n++;
+            for (; j > 0 && starts[seq[j - 1] + 1] - starts[seq[j - 1]] < S; j--) seq[j] = seq[j - 1];
+            seq[j] = b0;
+        }
+        if (!n) break;
+        for (int i = 0; i < n; i++) {
+            const int t0 = starts[seq[i]], S = starts[seq[i] + 1] - t0;
+            GgSeg* sg = &p.seg[i];
+            GgProb* q = &p.prob[i];
+            sg->K = S; sg->kb = (S + 63) / 64; sg->alpha = 1.f; sg->mn = 3; sg->amax_a = ds_bound; sg->amax_b = amax_k;
+            q->M = S; q->N = qd; q->bn = 128; q->tiles_m = (S + 255) / 256; q->tiles_n = Hq; q->seg0 = i; q->nseg = 1; q->kb = sg->kb;
+            p.run[i].item0 = p.items; p.run[i].prob = i; p.run[i].split = 1;
+            p.items += q->tiles_m * Hq;
+            const cuuint64_t ad[4] = {(cuuint64_t)S, (cuuint64_t)S, (cuuint64_t)Hq, 2}, as[3] = {(cuuint64_t)Sp * 2, (cuuint64_t)Sp * Sp * 2, (cuuint64_t)ds_part * 2};
+            const cuuint32_t abox[4] = {64u, 64u, 1u, 1u}, one[4] = {1u, 1u, 1u, 1u};
+            if (g_tc_encode(&sg->a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, (void*)((const __half*)ds + (size_t)seq[i] * Hq * Sp * Sp), ad, as, abox, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return 1;
+            const cuuint64_t bd[3] = {(cuuint64_t)kvd, (cuuint64_t)S, 2}, bs[2] = {(cuuint64_t)kvd * 2, (cuuint64_t)k_part * 2};
+            const cuuint32_t bbox[3] = {64u, 64u, 1u};
+            if (!tc_encode(c, &sg->b, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (const __half*)k + (size_t)t0 * kvd, bd, bs, bbox, CU_TENSOR_MAP_SWIZZLE_128B) ||
+                !gg_map_out(c, &q->c, dQ + (size_t)t0 * qd, S, qd)) return 1;
+        }
+        p.nruns = p.nsegs = p.nprob = n;
+        p.heads = Hq; p.group = g;
+        p.counter = sb_item_counter(c);
+        if (!p.counter) return 1;
+        p.status = c->d_status;
+        if (!gg_launch_t<128, 3, true>(c, p, p.items < pairs ? p.items : pairs)) return 1;
+    }
+    return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }

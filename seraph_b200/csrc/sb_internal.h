@@ -276,6 +276,8 @@ typedef struct { const float *A, *B; float* C; int M, N, K, tA, tB, acc; float a
 void sb_gemm_group(sb_ctx_t*, const sb_gemm_job_t* jobs, int n);
 int  sb_gemm_group_try(sb_ctx_t*, const sb_gemm_job_t* jobs, int n);      /* 0: launched as a group */
 int  sb_gemm_group_takes(sb_ctx_t*, int M, int N, int K, int tA, int tB);
+int  sb_gemm_dq(sb_ctx_t*, const void* ds, size_t ds_part, const float* ds_bound, const void* k, size_t k_part, const float* amax_k, float* dQ,
+                const int* starts, int nseq, int Sp, int Hq, int g);
 void sb_parts_prepare(sb_ctx_t*, const float* const* x, const size_t* n, int count);
 int  sb_gemm_reads_f16_parts(sb_ctx_t*, int M, int N, int K, int tA, int tB);      /* 1: that product takes prepared FP16 parts of its operands */
 void sb_gemm_simt(sb_ctx_t*, const float* A, const float* B, float* C, int M, int N, int K, int tA, int tB, int acc);
