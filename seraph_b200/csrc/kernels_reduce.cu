@@ -357,26 +357,9 @@ __global__ void __launch_bounds__(RB_THREADS, 2) rmsnorm_bwd_warp_kernel(const f
     __shared__ float4 s_acc[RB_THREADS / 32][32 * NV];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, c4 = cols >> 2, stride = gridDim.x * (RB_THREADS / 32);
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 sc[NV], acc[NV];
-    float wm = 0.f, am = 0.f;
-#pragma unroll
-    for (int i = 0; i < NV; i++) {
-        const int j = lane + 32 * i;
-        sc[i] = j < c4 ? ((const float4*)w)[j] : zero;
-        acc[i] = zero;
-        wm = sb_amax4(wm, sc[i]);
-    }
-    float osc = 1.f;
-    if (out.bound) {
-        wm = warp_max(wm);
-        const float bound = fminf((out.amax_resid ? sb_word(out.amax_resid) : 0.f) + 1.0001f * (1.f + sqrtf((float)cols)) * sb_word(out.inv_max) * wm * sb_word(out.amax_dy), 3.0e38f);
-        osc = sb_pow2(sb_f16_shift(bound));
-        if (blockIdx.x == 0 && threadIdx.x == 0) *out.bound = bound;
-    }
-    for (int r = blockIdx.x * (RB_THREADS / 32) + wib; r < rows; r += stride) {
+    float4 acc[NV], v[NV], g[NV], q[NV];
+    auto load = [&](int r) {
         const size_t o0 = (size_t)r * c4;
-        float4 v[NV], g[NV], q[NV];
-        float ss = 0.f, cp = 0.f;
 #pragma unroll
         for (int i = 0; i < NV; i++) {
             const int j = lane + 32 * i;
@@ -385,8 +368,31 @@ __global__ void __launch_bounds__(RB_THREADS, 2) rmsnorm_bwd_warp_kernel(const f
             g[i] = in ? ((const float4*)dy)[o0 + j] : zero;
             q[i] = in && resid ? ((const float4*)resid)[o0 + j] : zero;
         }
+    };
+    const int r0 = blockIdx.x * (RB_THREADS / 32) + wib;
+    if (r0 < rows) load(r0);              // on its way while the scales and the words are looked at
+    float wm = 0.f, am = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        const int j = lane + 32 * i;
+        acc[i] = zero;
+        wm = sb_amax4(wm, j < c4 ? ((const float4*)w)[j] : zero);      // (read again from cache below)
+    }
+    float osc = 1.f;
+    if (out.bound) {
+        wm = warp_max(wm);
+        const float bound = fminf((out.amax_resid ? sb_word(out.amax_resid) : 0.f) + 1.0001f * (1.f + sqrtf((float)cols)) * sb_word(out.inv_max) * wm * sb_word(out.amax_dy), 3.0e38f);
+        osc = sb_pow2(sb_f16_shift(bound));
+        if (blockIdx.x == 0 && threadIdx.x == 0) *out.bound = bound;
+    }
+    for (int r = r0; r < rows; r += stride) {
+        const size_t o0 = (size_t)r * c4;
+        if (r != r0) load(r);
+        float ss = 0.f, cp = 0.f;
+        float4 sc[NV];
 #pragma unroll
         for (int i = 0; i < NV; i++) {
+            sc[i] = lane + 32 * i < c4 ? __ldg((const float4*)w + lane + 32 * i) : zero;
             ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
             cp += g[i].x * sc[i].x * v[i].x + g[i].y * sc[i].y * v[i].y + g[i].z * sc[i].z * v[i].z + g[i].w * sc[i].w * v[i].w;
         }
@@ -618,13 +624,24 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const fl
                                                                         float* __restrict__ y, uint2* __restrict__ h1, uint2* __restrict__ h2, int rows, int cols, float eps,
                                                                         float* __restrict__ bound_out, unsigned keep, float* __restrict__ copy, unsigned* inv_max) {
     sb_pdl_enter();
+    constexpr bool KEEP = NV <= 4;        // the scales stay in registers; wider rows read them again from cache
     const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int c4 = cols >> 2;
-    float wm = 0.f;                       // (w is read again from cache in the output loop: keeping it would double the registers)
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v[NV], s[KEEP ? NV : 1];
+    auto load = [&](int r) {
+        const float4* xr = (const float4*)(x + (size_t)r * cols);
+#pragma unroll
+        for (int i = 0; i < NV; i++) v[i] = lane + 32 * i < c4 ? xr[lane + 32 * i] : zero;
+    };
+    if (warp < rows) load(warp);          // on its way while the scales are looked at
+    float wm = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; i++) {
         const int j = lane + 32 * i;
-        if (j < c4) wm = sb_amax4(wm, ((const float4*)w)[j]);
+        const float4 q = j < c4 ? ((const float4*)w)[j] : zero;
+        if constexpr (KEEP) s[i] = q;
+        wm = sb_amax4(wm, q);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffu, wm, o));
@@ -633,13 +650,11 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const fl
     if (warp == 0 && lane == 0) *bound_out = bound;
     float im = 0.f;
     for (int r = warp; r < rows; r += nwarps) {
-        const float4* xr = (const float4*)(x + (size_t)r * cols);
-        float4 v[NV];
+        if (r != warp) load(r);
         float ss = 0.f;
 #pragma unroll
         for (int i = 0; i < NV; i++) {
-            int j = lane + 32 * i;
-            v[i] = j < c4 ? xr[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const int j = lane + 32 * i;
             if (copy && j < c4) ((float4*)(copy + (size_t)r * cols))[j] = v[i];
             ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
         }
@@ -652,8 +667,8 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const fl
             int j = lane + 32 * i;
             if (j < c4) {
                 // the FP32 value first, exactly as the plain kernel forms it, then the scale (a power of two: exact)
-                const float4 s = ((const float4*)w)[j];
-                const float y0 = v[i].x * inv * s.x, y1 = v[i].y * inv * s.y, y2 = v[i].z * inv * s.z, y3 = v[i].w * inv * s.w;
+                const float4 q = KEEP ? s[KEEP ? i : 0] : ((const float4*)w)[j];
+                const float y0 = v[i].x * inv * q.x, y1 = v[i].y * inv * q.y, y2 = v[i].z * inv * q.z, y3 = v[i].w * inv * q.w;
                 if (y) { ((float4*)(y + (size_t)r * cols))[j] = make_float4(y0, y1, y2, y3); continue; }      // no arena for the parts
                 uint2 a, b;
                 sb_split2(y0 * sc, y1 * sc, a.x, b.x, keep); sb_split2(y2 * sc, y3 * sc, a.y, b.y, keep);
@@ -661,7 +676,7 @@ __global__ void __launch_bounds__(RB_THREADS) rmsnorm_warp_parts_kernel(const fl
             }
         }
     }
-    if (inv_max && lane == 0 && im > 0.f) atomicMax(inv_max, __float_as_uint(im));
+    sb_block_amax(im, inv_max);           // (a word that all warps raise one by one: 5800 of them took longer than the rows)
 }
 template <int NV>
 __global__ void __launch_bounds__(RB_THREADS) qk_norm_warp_kernel(float* __restrict__ x, float* __restrict__ rms_out, int rows, int cols, float eps) {
@@ -1228,8 +1243,10 @@ int sb_rmsnorm_parts(sb_ctx_t* c, const float* x, const float* w, float* y, floa
     const size_t n = (size_t)rows * cols;
     if (!aligned16(y) || !sb_bound_out(c, y, n, &h, &bound)) return 0;
     float* y32 = h ? NULL : y;
+    // a row per warp: what a row costs is the way to memory and back.  5800 x 512 in a step: 8.4 us, 15 with three rows one after the other in two CTAs an
+    // SM and an atomic a warp; 2048 x 512: 5.0 (6.5)
     int wgrid = (rows + 7) / 8;
-    { int cap = sm_count(c) * 2, k = (wgrid + cap - 1) / cap; wgrid = (wgrid + k - 1) / k; }
+    if (wgrid > sm_count(c) * 16) wgrid = sm_count(c) * 16;
     cudaStream_t st = (cudaStream_t)c->pub.stream;
     uint2* h1 = (uint2*)h; uint2* h2 = (uint2*)((uint16_t*)h + n);
     int tk = sb_tick_begin(c, SB_CLS_NORM_FWD);
