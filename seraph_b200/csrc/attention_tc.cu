@@ -202,17 +202,20 @@ __global__ void at_delta_kernel(const float* __restrict__ dO, const float* __res
 
 // D for 64- and 128-wide heads, together with what the FP16 split of dO and the bound of dS need from the same rows: the largest |dO|
 // (amax) and the largest row norms of dO (norm_do; blockIdx.y == 0) and of V (norm_v; blockIdx.y == 1), all raised with integer atomicMax
-// on the float bits (order-free; zeroed before).  HD/4 lanes per (t,h) row, four passes of rows in flight.
+// on the float bits (order-free; zeroed before).  HD/4 lanes per (t,h) row, four passes of rows in flight.  h1: where the kernel that wrote dO left its
+// largest magnitude (*known), the parts of dO are written on the way, and the second step does not read it again.
 template <int HD>
 __global__ void __launch_bounds__(256) at_bwd_prep_kernel(const float* __restrict__ dO, const float* __restrict__ O, float* __restrict__ D, int n_do,
                                                           const float* __restrict__ V, int n_v,
-                                                          unsigned* __restrict__ norm_do, unsigned* __restrict__ amax, unsigned* __restrict__ norm_v) {
+                                                          unsigned* __restrict__ norm_do, unsigned* __restrict__ amax, unsigned* __restrict__ norm_v,
+                                                          const float* __restrict__ known, uint2* __restrict__ h1, uint2* __restrict__ h2) {
     sb_pdl_enter();
     constexpr int LPR = HD / 4, RPW = 32 / LPR;
     const int lane = threadIdx.x & 31, sub = lane / LPR, l = lane % LPR, nwarps = (gridDim.x * blockDim.x) >> 5;
     const bool is_v = blockIdx.y != 0;
     const int n = is_v ? n_v : n_do;
     float bn = 0.f, ba = 0.f;
+    const float sc = h1 ? tc_pow2(tc_f16_shift(sb_word(known))) : 0.f;
     for (int r0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (4 * RPW); r0 < n; r0 += nwarps * (4 * RPW)) {
         float d[4], n2[4];
 #pragma unroll
@@ -225,7 +228,11 @@ __global__ void __launch_bounds__(256) at_bwd_prep_kernel(const float* __restric
                 if (!is_v) {
                     const float4 o = __ldcs((const float4*)(O + (size_t)r * HD) + l);      // dO is read again by the next kernel, O is not
                     d[i] = g.x * o.x + g.y * o.y + g.z * o.z + g.w * o.w;
-                    ba = sb_amax4(ba, g);
+                    if (h1) {
+                        uint2 a, b;
+                        sb_split2(g.x * sc, g.y * sc, a.x, b.x); sb_split2(g.z * sc, g.w * sc, a.y, b.y);
+                        h1[(size_t)r * LPR + l] = a; h2[(size_t)r * LPR + l] = b;
+                    } else ba = sb_amax4(ba, g);
                 }
             }
         }
@@ -238,11 +245,12 @@ __global__ void __launch_bounds__(256) at_bwd_prep_kernel(const float* __restric
         }
     }
     sb_block_amax(sqrtf(bn), is_v ? norm_v : norm_do);
+    if (h1) return;
     __syncthreads();
     if (!is_v) sb_block_amax(ba, amax);
 }
-// Second step, once those maxima are known.  blockIdx.y == 0: the FP16 parts of dO; also the constants (consts[0] = 1, consts[1] = the
-// bound of dS as in at_consts_kernel).  blockIdx.y == 1: lse and D, [token][head], moved to the rows of the (sequence, head) slots (zeros up
+// Second step, once those maxima are known.  blockIdx.y == 0 (h1 given): the FP16 parts of dO; also the constants (consts[0] = 1, consts[1] = the
+// bound of dS as in at_consts_kernel).  The other blocks: lse and D, [token][head], moved to the rows of the (sequence, head) slots (zeros up
 // to a multiple of 32 queries) in the form the backward's elementwise warps use: 14 - lse log2(e) for 128-wide heads (the
 // probabilities are formed times 2^14, by the exponent), -lse for 64-wide ones (those have the issue slots to multiply by log2(e) and 2^14
 // after the subtraction, which keeps the rounding of the large terms out of the exponent), and D times the factor that takes
@@ -253,8 +261,8 @@ __global__ void __launch_bounds__(256) at_bwd_prep2_kernel(const float4* __restr
                                                            const AfSeqTab seqs, int Hq, int Smax, int slot_pitch, int natural) {
     sb_pdl_enter();
     const float bound = 2.0f * sb_word(norm_do) * sb_word(norm_v) * scale;
-    if (blockIdx.y == 0) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) { consts[0] = 1.0f; consts[1] = bound; }
+    if (blockIdx.y == 0 && blockIdx.x == 0 && threadIdx.x == 0) { consts[0] = 1.0f; consts[1] = bound; }
+    if (h1 && blockIdx.y == 0) {
         const float sc = tc_pow2(tc_f16_shift(sb_word(amax)));
         const size_t nth = (size_t)gridDim.x * blockDim.x;
         for (size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n4; i0 += 2 * nth) {
@@ -529,8 +537,9 @@ static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, cons
     cudaStream_t st = (cudaStream_t)c->pub.stream;
     int tk = sb_tick_begin(c, SB_CLS_ATTN_BWD);
     // words that start from zero: inside a step from its pool, else cleared here (a launch)
-    float *am_do = sb_zero_word(c), *norm_do = sb_zero_word(c), *norm_v = sb_zero_word(c);
-    if (!norm_v) { cudaMemsetAsync(consts, 0, 64 * sizeof(float), st); norm_do = consts + 2; norm_v = consts + 3; am_do = consts + 11; }
+    float* left = sb_amax_lookup(c, dO, n_q);                        // the product that wrote dO may have left its largest magnitude
+    float *am_do = left ? left : sb_zero_word(c), *norm_do = sb_zero_word(c), *norm_v = sb_zero_word(c);
+    if (!norm_v) { cudaMemsetAsync(consts, 0, 64 * sizeof(float), st); norm_do = consts + 2; norm_v = consts + 3; am_do = left ? left : consts + 11; }
     const AtNeed need[3] = {{Q, n_q, hb, consts + 8, consts + 16}, {K, n_kv, hb + 2 * n_q, consts + 9, consts + 18}, {V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10, consts + 20}};
     AtParts p[3];
     at_make_parts_multi(c, need, 3, p);
@@ -539,8 +548,9 @@ static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, cons
         const int rpb = 8 * 4 * (128 / hd);                          // rows a CTA takes per pass
         const int cap = c->pub.gpu_sm_count * 8, want = (T * Hq + rpb - 1) / rpb;
         const dim3 pg(want < cap ? want : cap, 2);
-        if (hd == 128) sb_launch(at_bwd_prep_kernel<128>, dim3(pg), dim3(256), 0, st, dO, O, D, T * Hq, V, T * Hkv, (unsigned*)norm_do, (unsigned*)am_do, (unsigned*)norm_v);
-        else sb_launch(at_bwd_prep_kernel<64>, dim3(pg), dim3(256), 0, st, dO, O, D, T * Hq, V, T * Hkv, (unsigned*)norm_do, (unsigned*)am_do, (unsigned*)norm_v);
+        uint2 *h1 = left ? (uint2*)hdo : nullptr, *h2 = (uint2*)(hdo + n_q);
+        if (hd == 128) sb_launch(at_bwd_prep_kernel<128>, dim3(pg), dim3(256), 0, st, dO, O, D, T * Hq, V, T * Hkv, (unsigned*)norm_do, (unsigned*)am_do, (unsigned*)norm_v, left, h1, h2);
+        else sb_launch(at_bwd_prep_kernel<64>, dim3(pg), dim3(256), 0, st, dO, O, D, T * Hq, V, T * Hkv, (unsigned*)norm_do, (unsigned*)am_do, (unsigned*)norm_v, left, h1, h2);
         c->launches++;
     }
     // from here on the launches depend on the boundaries
@@ -560,7 +570,9 @@ static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, cons
     float* LT = bb + n_ds; float* DT = LT + row_floats;
     {
         const AfSeqTab seqs = {n, c->attn_seq_starts};
-        sb_launch(at_bwd_prep2_kernel, dim3(dim3(tc_ew_blocks(c, n_q / 8), 2)), dim3(256), 0, st, (const float4*)dO, n_q / 4, (uint2*)hdo, (uint2*)(hdo + n_q), am_do,
+        const int rows_blocks = (int)(((long)n * ((Smax + 31) / 32) * Hq + 7) / 8);      // a warp for 32 rows
+        const dim3 pg = left ? dim3((unsigned)max(1, min(rows_blocks, c->pub.gpu_sm_count * 8))) : dim3(tc_ew_blocks(c, n_q / 8), 2);
+        sb_launch(at_bwd_prep2_kernel, pg, dim3(256), 0, st, (const float4*)dO, n_q / 4, left ? (uint2*)nullptr : (uint2*)hdo, (uint2*)(hdo + n_q), am_do,
                                                                             consts, norm_do, norm_v, scale, lse, D, LT, DT, seqs, Hq, Smax, slot_pitch, hd == 64 ? 1 : 0);
         c->launches++;
     }

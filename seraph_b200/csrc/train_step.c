@@ -959,6 +959,7 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
         sb_rmsnorm_backward_parts(c, a->post_attn_in, c->W + o->post_norm, gx, gh, gh, full ? Gd + o->post_norm : NULL, T, d, RMS_EPS, a->inv_ffn, &c->ghid_amax);
         /* attention */
         sb_gemm_keep_begin(c);
+        if (full || (grouped && !c->lora_exact)) sb_amax_announce(c, c->g_attn, (size_t)T * qd);      /* attention's backward scales its parts by it (an exact adapter adds to it afterwards) */
         if (grouped) {
             const int ad = 3; const float *dy = gh, *w = c->W + o->o;
             lora_bwd_group(c, l, &ad, &dy, &w, 1, a->attn_out, l > 0 || (c->lora_mask & 7) ? c->g_attn : NULL, T, qd);
