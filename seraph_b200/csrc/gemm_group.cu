@@ -43,7 +43,7 @@
 // the CTA is launched with (384 x 168).
 #define GG_REGS_LIGHT 72
 #define GG_REGS_EPI 216
-#define GG_EMPTY_ARRIVALS 19     // roles that take an item: producer and 8 epilogue warps in both CTAs, the MMA warp in the leader
+#define GG_EMPTY_ARRIVALS 21     // roles that take an item: 2 producers and 8 epilogue warps in both CTAs, the MMA warp in the leader
 
 struct __align__(64) GgSeg {
     CUtensorMap a, b;            // parts: K-major {K, rows, part}, MN-major {rows, K, part}
@@ -213,44 +213,50 @@ gg_kernel(const __grid_constant__ GgParams p) {
     const bool is_epi = warp >= 4 && warp < 12;
     if (!is_epi) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(GG_REGS_LIGHT));
-        if (warp == 0) {
-            // ---------------- TMA producer ----------------
+        if (warp == 0 || warp == 3) {
+            // ---------------- TMA producers: warp 0 fetches A, asks for items and announces the bytes, warp 3 fetches B ----------------
+            // (one thread for both took 430 cycles a stage, as long as the tensor core has for half a chunk of the narrow tile)
             if (elect_one()) {
-                uint32_t git = 0;
+                const bool is_a = warp == 0;
+                const uint32_t full0 = mapa_u32(smem_u32(full), 0);      // both CTAs' bytes land on the leader's barriers
+                int s = 0;
+                uint32_t par = 1;
                 for (int n = 0; ok; n++) {
                     GgWork w;
                     if (!next_item(n, true, (int)rank, w)) break;
                     if (n == 0) sb_pdl_enter();
                     const GgProb& pr = p.prob[w.prob];
                     int off = 0, left = w.kb1 - w.kb0;
-                    const int ask = min(left, GG_AHEAD);
-                    if (left == 0 && leader) af_arrive_local(item_req);
+                    const int ask = is_a && leader ? min(left, GG_AHEAD) : -1;
+                    if (left == 0 && ask == 0) af_arrive_local(item_req);
                     for (int sg = pr.seg0; sg < pr.seg0 + pr.nseg && ok; sg++) {
                         const GgSeg& g = p.seg[sg];
                         const int lo = max(w.kb0, off) - off, hi = min(w.kb1, off + g.kb) - off;
                         off += g.kb;
-                        const bool amn = (g.mn & 1) != 0, bmn = (g.mn & 2) != 0;
-                        const int boxes = (pr.bn + 127) / 128;                        // of 64 columns: an MN-major B is fetched in whole lines
-                        const uint32_t bytes = (uint32_t)(A_PART + (bmn ? boxes * 8192 : pr.bn * 64)) * 2;
+                        const bool mn = (g.mn & (is_a ? 1 : 2)) != 0;
+                        const int boxes = is_a ? 2 : (pr.bn + 127) / 128;             // of 64 rows: an MN-major operand is fetched in whole lines
+                        const uint32_t bytes = (uint32_t)(A_PART + ((g.mn & 2) ? (pr.bn + 127) / 128 * 8192 : pr.bn * 64)) * 2;
+                        const CUtensorMap* map = is_a ? &g.a : &g.b;
+                        const int row = is_a ? w.m0 : w.nb0;
+                        uint8_t* base = is_a ? smem : smem + A_PART;
                         for (int kb = lo; kb < hi && ok; kb++) {
-                            if (left-- == ask && leader) af_arrive_local(item_req);
-                            for (int part = 0; part < NP; part++, git++) {
-                                const int s = git % STAGES;
-                                ok = mbar_wait(&empty[s], ((git / STAGES) & 1) ^ 1);
+                            if (left-- == ask) af_arrive_local(item_req);
+                            for (int part = 0; part < NP; part++) {
+                                ok = mbar_wait(&empty[s], par);
                                 if (!ok) break;
-                                uint8_t* st = smem + s * STAGE;
-                                if (leader) mbar_expect_tx(&full[s], bytes);      // both CTAs' bytes land on the leader's barrier
-                                const uint32_t fb = mapa_u32(smem_u32(&full[s]), 0);
-                                if (amn) {
+                                if (is_a && leader) mbar_expect_tx(&full[s], bytes);
+                                uint8_t* st = base + s * STAGE;
+                                const uint32_t fb = full0 + (uint32_t)(s * 8);
+                                if (!mn) tma_load_3d_pair(st, map, fb, kb * 64, row, part);
+                                else {
 #pragma unroll
-                                    for (int j = 0; j < 2; j++)
-                                        if constexpr (BATCH) gg_load_4d_pair(st + j * 8192, &g.a, fb, w.m0 + 64 * j, kb * 64, w.head, part);
-                                        else tma_load_3d_pair(st + j * 8192, &g.a, fb, w.m0 + 64 * j, kb * 64, part);
-                                } else tma_load_3d_pair(st, &g.a, fb, kb * 64, w.m0, part);
-                                if (bmn) {
-#pragma unroll
-                                    for (int j = 0; j < BN / 128; j++) if (j < boxes) tma_load_3d_pair(st + A_PART + j * 8192, &g.b, fb, w.nb0 + 64 * j, kb * 64, part);
-                                } else tma_load_3d_pair(st + A_PART, &g.b, fb, kb * 64, w.nb0, part);
+                                    for (int j = 0; j < 2; j++) {
+                                        if (j >= boxes) continue;
+                                        if (BATCH && is_a) gg_load_4d_pair(st + j * 8192, map, fb, row + 64 * j, kb * 64, w.head, part);
+                                        else tma_load_3d_pair(st + j * 8192, map, fb, row + 64 * j, kb * 64, part);
+                                    }
+                                }
+                                if (++s == STAGES) { s = 0; par ^= 1; }
                             }
                         }
                     }
