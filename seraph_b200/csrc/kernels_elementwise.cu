@@ -216,6 +216,21 @@ __global__ void seq_index_kernel(const uint32_t* __restrict__ ss, int B, int T, 
     seq_ids[t] = (uint32_t)lo;
 }
 
+// A batch as it was uploaded, T tokens, T targets, B + 1 boundaries, to where a step reads it, with the same tables (B < T)
+__global__ void batch_index_kernel(const uint32_t* __restrict__ upload, int B, int T, uint32_t* tokens, uint32_t* targets, uint32_t* seq_starts, uint32_t* pos_ids, uint32_t* seq_ids) {
+    sb_pdl_enter();
+    const uint32_t* ss = upload + 2 * (size_t)T;
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= T) return;
+    tokens[t] = upload[t]; targets[t] = upload[(size_t)T + t];
+    if (t <= B) seq_starts[t] = ss[t];
+    int lo = 0, hi = B;
+    while (lo < hi) { int mid = (lo + hi) >> 1; if ((int)ss[mid + 1] <= t) lo = mid + 1; else hi = mid; }
+    if (lo >= B) lo = B - 1;
+    pos_ids[t] = (uint32_t)(t - (int)ss[lo]);
+    seq_ids[t] = (uint32_t)lo;
+}
+
 // cos/sin table [max_pos, hd/2] built with the same FP32 expression the
 // reference evaluates per element: angle = pos * (1/powf(theta, 2p/hd)).
 __global__ void rope_table_kernel(float2* tab, int max_pos, int half, int hd, float theta) {
@@ -471,6 +486,11 @@ void sb_embed_lookup(sb_ctx_t* c, const uint32_t* tok, const float* E, float* ou
 void sb_seq_index(sb_ctx_t* c, const uint32_t* seq_starts, int B, int T, uint32_t* pos_ids, uint32_t* seq_ids) {
     if (T <= 0) return;
     sb_launch(seq_index_kernel, dim3((T + 255) / 256), dim3(256), 0, (cudaStream_t)c->pub.stream, seq_starts, B, T, pos_ids, seq_ids);
+    c->launches++;
+}
+
+void sb_batch_index(sb_ctx_t* c, const uint32_t* upload, int B, int T, uint32_t* tokens, uint32_t* targets, uint32_t* seq_starts, uint32_t* pos_ids, uint32_t* seq_ids) {
+    sb_launch(batch_index_kernel, dim3((T + 255) / 256), dim3(256), 0, (cudaStream_t)c->pub.stream, upload, B, T, tokens, targets, seq_starts, pos_ids, seq_ids);
     c->launches++;
 }
 

@@ -137,6 +137,7 @@ typedef struct sb_ctx {
     float *g_hidden, *g_xnorm, *g_q, *g_k, *g_v, *g_attn, *g_ffn, *g_gate, *g_up;
     uint32_t *tokens, *targets, *seq_starts, *pos_ids, *seq_ids;
     int seq_cap, seq_starts_cap;
+    uint32_t* upload; size_t upload_cap;   /* a step's tokens, targets and boundaries as they arrive, in one copy */
     int* h_seq; int h_seq_n, h_seq_cap;   /* host copy of the current batch's sequence starts (h_seq_n + 1 entries); 0 = unknown */
     /* boundaries of an op-level packed attention call on their way to the host (ops.cu), and the tables it did not make yet */
     void* seq_copy_stream; void* seq_copy_ev[2]; int* h_seq_pin; int h_seq_pin_cap; int seq_pending;
@@ -215,6 +216,7 @@ int  sb_attention_reads_parts(sb_ctx_t*, int Hq, int Hkv, int hd);      /* 1: fo
 int  sb_rmsnorm_parts(sb_ctx_t*, const float* x, const float* w, float* y, float* copy, int rows, int cols, float eps, float** inv_word);      /* bound: sqrt(cols) max|w| */
 int  sb_swiglu_backward_parts(sb_ctx_t*, const float* gate, const float* up, const float* dout, float* dgate, float* dup, size_t n);
 void sb_amax_forget(sb_ctx_t*, const float* x);      /* x is written by something that leaves no maximum: earlier hints for it are void */
+void sb_batch_index(sb_ctx_t*, const uint32_t* upload, int B, int T, uint32_t* tokens, uint32_t* targets, uint32_t* seq_starts, uint32_t* pos_ids, uint32_t* seq_ids);
 void sb_seq_index(sb_ctx_t*, const uint32_t* seq_starts, int B, int T, uint32_t* pos_ids, uint32_t* seq_ids);
 /* Between begin and end the FP16 parts of GEMM operands are kept and reused by later calls on the same array; the caller
  * guarantees that no operand array is written inside the region. */

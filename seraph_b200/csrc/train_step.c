@@ -1048,8 +1048,16 @@ static void backward_pass(sb_ctx_t* c, int T, int B, int max_seq, float theta, i
  * sequence has target 0 (src/train_cuda.c:2030-2043); staged in pinned memory */
 static int upload_batch(sb_ctx_t* c, const int* tokens, int T, const int* seq_starts, int B, int* max_seq_out) {
     if (sb_ensure_tokens(c, T, B)) return 1;
-    size_t words = (size_t)2 * T + (size_t)B + 1 + 4;
-    if (ensure_pinned(c, words * sizeof(uint32_t) + 64)) return 1;
+    const size_t words = (size_t)2 * T + (size_t)B + 1;
+    if (ensure_pinned(c, (words + 4 + (c->in_evaluate ? (size_t)T : 0)) * sizeof(uint32_t) + 64)) return 1;
+    if (c->upload_cap < words) {
+        cudaStreamSynchronize(S(c));
+        if (c->upload) cudaFree(c->upload);
+        c->upload = NULL; c->upload_cap = 0;
+        const size_t cap = words < 4096 ? 4096 : words;
+        if (sb_check(c, cudaMalloc((void**)&c->upload, cap * sizeof(uint32_t)), "token upload")) { c->status = SB_ERR_OOM; return 1; }
+        c->upload_cap = cap;
+    }
     uint32_t* h_tok = (uint32_t*)c->h_pinned; uint32_t* h_tgt = h_tok + T; uint32_t* h_ss = h_tgt + T;
     int max_seq = 0;
     for (int b = 0; b < B; b++) {
@@ -1064,15 +1072,16 @@ static int upload_batch(sb_ctx_t* c, const int* tokens, int T, const int* seq_st
     }
     if (seq_starts[0] != 0 || seq_starts[B] != T) { sb_set_status(c, SB_ERR_ARG); return 1; }
     for (int b = 0; b <= B; b++) h_ss[b] = (uint32_t)seq_starts[b];
-    cudaMemcpyAsync(c->tokens, h_tok, (size_t)T * 4, cudaMemcpyHostToDevice, S(c));
-    cudaMemcpyAsync(c->targets, h_tgt, (size_t)T * 4, cudaMemcpyHostToDevice, S(c));
-    cudaMemcpyAsync(c->seq_starts, h_ss, (size_t)(B + 1) * 4, cudaMemcpyHostToDevice, S(c));
-    sb_seq_index(c, c->seq_starts, B, T, c->pos_ids, c->seq_ids);
+    /* one copy, dealt out by the kernel that makes the tables (a copy each cost 3 to 7 us of an idle device) */
+    cudaMemcpyAsync(c->upload, h_tok, words * 4, cudaMemcpyHostToDevice, S(c));
+    sb_batch_index(c, c->upload, B, T, c->tokens, c->targets, c->seq_starts, c->pos_ids, c->seq_ids);
     sb_set_host_seq(c, seq_starts, B);
     *max_seq_out = max_seq;
     return 0;
 }
 
+/* the per-token losses of an evaluation pass in the pinned staging buffer, behind the batch */
+static float* eval_rows(const sb_ctx_t* c, int T, int B) { return (float*)((uint32_t*)c->h_pinned + (size_t)2 * T + (size_t)B + 1); }
 static float lr_for_step(const train_state_t* st, int accum) {
     /* 100-step linear warm-up, then divided by the accumulation count (src/train_cuda.c:2298-2303) */
     float lr = st->learning_rate;
@@ -1200,6 +1209,7 @@ static float step_body(train_state_t* st, int* tokens, int T, int* seq_starts, i
     if (train && c->dp_world > 1 && seraph_dp_wait(ctx, c->dp_timeout_ms) != SB_OK) return -1.0f;
     float* h_loss = (float*)((char*)c->h_pinned + c->h_pinned_bytes - 64);
     cudaMemcpyAsync(h_loss, c->d_loss, sizeof(float), cudaMemcpyDeviceToHost, S(c));
+    if (c->in_evaluate) cudaMemcpyAsync(eval_rows(c, T, B), c->loss_rows, (size_t)T * sizeof(float), cudaMemcpyDeviceToHost, S(c));      /* eval_flush reads them */
     if (sb_check(c, cudaStreamSynchronize(S(c)), "training step")) return -1.0f;
     float loss = *h_loss / (float)num_valid;
     if (train && st->debug_nan_check && (isnan(loss) || isinf(loss))) { st->nan_detected = 1; return NAN; }
@@ -1242,14 +1252,14 @@ float cuda_eval_forward(train_state_t* state, int* tokens, int num_tokens, cuda_
 
 /* One packed forward pass over the samples gathered in pk[0..T) / ss[0..B]: every sample's mean loss is added to *total
  * (and counted in *valid) from the per-token losses of the pass, summed per sample on the host in token order. */
-static void eval_flush(train_state_t* state, cuda_train_context_t* ctx, int* pk, int* ss, int B, int full, float* rows,
-                       double* total, int* valid) {
+static void eval_flush(train_state_t* state, cuda_train_context_t* ctx, int* pk, int* ss, int B, int full, double* total, int* valid) {
     sb_ctx_t* c = sb_priv(ctx);
     int T = ss[B];
     if (B <= 0 || T <= 0) return;
     float loss = step_common(state, pk, T, ss, B, ctx, full, 0, 0);
     if (loss < 0.0f || isnan(loss)) return;
-    if (cudaMemcpy(rows, c->loss_rows, (size_t)T * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) { cudaGetLastError(); return; }
+    if (T - B <= 0) return;                              /* no pass was run */
+    const float* rows = eval_rows(c, T, B);
     for (int b = 0; b < B; b++) {
         double sum = 0.0;
         int n = ss[b + 1] - ss[b];
@@ -1271,13 +1281,12 @@ float cuda_evaluate(train_state_t* state, int* val_tokens, int num_val_tokens, i
     int stride = num_samples > max_eval ? num_samples / max_eval : 1;
     int budget = c ? c->eval_batch_tokens : 0;
     double total = 0.0; int valid = 0;
-    int* pk = NULL; int* ss = NULL; float* rows = NULL;
+    int* pk = NULL; int* ss = NULL;
     if (budget > 0) {
         if (budget < max_seq_len) budget = max_seq_len;
         pk = (int*)malloc((size_t)budget * sizeof(int));
         ss = (int*)malloc((EVAL_MAX_SEQS + 1) * sizeof(int));
-        rows = (float*)malloc((size_t)budget * sizeof(float));
-        if (!pk || !ss || !rows) { free(pk); free(ss); free(rows); pk = NULL; budget = 0; }
+        if (!pk || !ss) { free(pk); free(ss); pk = NULL; budget = 0; }
     }
     int full = state->lora == NULL;
     int B = 0;
@@ -1293,14 +1302,14 @@ float cuda_evaluate(train_state_t* state, int* val_tokens, int num_val_tokens, i
             if (loss >= 0.0f && !isnan(loss)) { total += loss; valid++; }
             continue;
         }
-        if (B == EVAL_MAX_SEQS || ss[B] + n > budget) { eval_flush(state, ctx, pk, ss, B, full, rows, &total, &valid); B = 0; }
+        if (B == EVAL_MAX_SEQS || ss[B] + n > budget) { eval_flush(state, ctx, pk, ss, B, full, &total, &valid); B = 0; }
         memcpy(pk + ss[B], &val_tokens[start], (size_t)n * sizeof(int));
         ss[B + 1] = ss[B] + n;
         B++;
     }
     if (budget > 0) {
-        eval_flush(state, ctx, pk, ss, B, full, rows, &total, &valid);
-        free(pk); free(ss); free(rows);
+        eval_flush(state, ctx, pk, ss, B, full, &total, &valid);
+        free(pk); free(ss);
     }
     if (c) c->in_evaluate = 0;
     float avg = valid > 0 ? (float)(total / valid) : -1.0f;
@@ -1421,6 +1430,7 @@ void cuda_train_free(cuda_train_context_t* ctx) {
     free_activations(c);
     free_model(c);
     if (c->tokens) cudaFree(c->tokens);
+    if (c->upload) cudaFree(c->upload);
     if (c->seq_starts) cudaFree(c->seq_starts);
     if (c->scratch) cudaFree(c->scratch);
     for (int i = 0; i < 5; i++) if (c->gemm_stage[i]) cudaFree(c->gemm_stage[i]);
