@@ -215,25 +215,30 @@ __global__ void __launch_bounds__(256) at_bwd_prep_kernel(const float* __restric
     const bool is_v = blockIdx.y != 0;
     const int n = is_v ? n_v : n_do;
     float bn = 0.f, ba = 0.f;
-    const float sc = h1 ? tc_pow2(tc_f16_shift(sb_word(known))) : 0.f;
     for (int r0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (4 * RPW); r0 < n; r0 += nwarps * (4 * RPW)) {
         float d[4], n2[4];
+        float4 g[4], o[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            d[i] = 0.f; n2[i] = 0.f;
             const int r = r0 + i * RPW + sub;
+            g[i] = o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (r < n) {
-                const float4 g = __ldg((const float4*)((is_v ? V : dO) + (size_t)r * HD) + l);
-                n2[i] = g.x * g.x + g.y * g.y + g.z * g.z + g.w * g.w;
-                if (!is_v) {
-                    const float4 o = __ldcs((const float4*)(O + (size_t)r * HD) + l);      // dO is read again by the next kernel, O is not
-                    d[i] = g.x * o.x + g.y * o.y + g.z * o.z + g.w * o.w;
-                    if (h1) {
-                        uint2 a, b;
-                        sb_split2(g.x * sc, g.y * sc, a.x, b.x); sb_split2(g.z * sc, g.w * sc, a.y, b.y);
-                        h1[(size_t)r * LPR + l] = a; h2[(size_t)r * LPR + l] = b;
-                    } else ba = sb_amax4(ba, g);
-                }
+                g[i] = __ldg((const float4*)((is_v ? V : dO) + (size_t)r * HD) + l);
+                if (!is_v) o[i] = __ldcs((const float4*)(O + (size_t)r * HD) + l);      // dO may be read again by the next kernel, O is not
+            }
+        }
+        const float sc = h1 && !is_v ? tc_pow2(tc_f16_shift(sb_word(known))) : 0.f;      // after the loads: it is no shorter on its way
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = r0 + i * RPW + sub;
+            n2[i] = g[i].x * g[i].x + g[i].y * g[i].y + g[i].z * g[i].z + g[i].w * g[i].w;
+            d[i] = g[i].x * o[i].x + g[i].y * o[i].y + g[i].z * o[i].z + g[i].w * o[i].w;
+            if (is_v) continue;
+            if (!h1) ba = sb_amax4(ba, g[i]);
+            else if (r < n) {
+                uint2 a, b;
+                sb_split2(g[i].x * sc, g[i].y * sc, a.x, b.x); sb_split2(g[i].z * sc, g[i].w * sc, a.y, b.y);
+                h1[(size_t)r * LPR + l] = a; h2[(size_t)r * LPR + l] = b;
             }
         }
 #pragma unroll
