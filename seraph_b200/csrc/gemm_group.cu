@@ -505,7 +505,8 @@ struct GgPlanEntry { GgPlanKey key; GgPlan plan; bool valid; };
 struct GgWidth { int bn; float t_kb[2], t_epi; };      // t_kb: three passes, one pass
 static const GgWidth gg_wide[3] = {{256, {1.00f, 0.47f}, 4.3f}, {192, {0.82f, 0.43f}, 3.5f}, {128, {0.64f, 0.38f}, 2.6f}};
 static const GgWidth gg_narrow[2] = {{128, {0.52f, 0.31f}, 2.3f}, {64, {0.42f, 0.27f}, 2.0f}};
-static const float gg_t_fix = 3.0f, gg_t_fix_col = 2e-4f;      // the fix-up launch, and for each column of 256 rows that it adds
+// the fix-up launch, and for each column of 256 rows that is written for it and read: in L2, and beyond 16 MB (512 x 256 columns: 130 us)
+static const float gg_t_fix = 3.0f, gg_t_fix_col = 2.5e-4f, gg_t_fix_far = 8e-4f, gg_fix_near = 16384.f;
 
 struct GgSim { float t[64]; int c[64]; int n; };
 // `count` items of one cost, each to the pair that is free first
@@ -596,7 +597,7 @@ static float gg_eval(const GgPlanKey* k, const GgWidth* tab, const GgPick* c, in
     }
     float t = 0.f;
     for (int i = 0; i < sim.n; i++) if (sim.t[i] > t) t = sim.t[i];
-    if (np) t = (t + gg_t_fix + slots * gg_t_fix_col) * 1.02f;
+    if (np) t = (t + gg_t_fix + slots * gg_t_fix_col + (slots > gg_fix_near ? (slots - gg_fix_near) * (gg_t_fix_far - gg_t_fix_col) : 0.f)) * 1.02f;
     for (int i = 0; i < k->nprob; i++) p->w[i] = tab[c->w[i]].bn;
     p->bn = tab[0].bn;
     return t;
@@ -626,6 +627,13 @@ static void gg_make_plan(const GgPlanKey* k, GgPlan* best) {
             const float off = cls || base ? GG_NARROWER : 1.f;
             float t = gg_eval(k, tab, &c, 1, 0.f, &p) * off;
             if (best->nruns == 0 || t < best_t) { *best = p; best_t = t; }
+            auto cut_tail = [&]() {
+                for (int q = 0; q < 6; q++) {
+                    const float tv = gg_eval(k, tab, &c, tails[q], best_t, &p) * off;
+                    if (tv > 0.f && tv < best_t) { *best = p; best_t = tv; }
+                }
+            };
+            cut_tail();
             // one kind of product after the other to its best choice beside the others'
             for (int sweep = 0; sweep < (many ? 0 : 2); sweep++) {
                 bool moved = false;
@@ -643,10 +651,7 @@ static void gg_make_plan(const GgPlanKey* k, GgPlan* best) {
                 }
                 if (!moved) break;
             }
-            for (int q = 0; q < 6; q++) {
-                const float tv = gg_eval(k, tab, &c, tails[q], best_t, &p) * off;
-                if (tv > 0.f && tv < best_t) { *best = p; best_t = tv; }
-            }
+            if (!many) cut_tail();
         }
     }
 }
