@@ -590,20 +590,25 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
 // dQ = dS K.  One CTA owns 128 queries of one (sequence, query head) and walks over the keys up to the diagonal in blocks of 64:
 // dS^T parts ([key][query], read MN-major as the 128-row A operand) and K parts (MN-major B operand) through a ring of stages, twelve
 // MMAs per block into one of two tensor-memory accumulators, which eight warps add into registers (round-to-nearest FP32).  All
-// sequences and heads in one launch, longest query blocks first.
+// sequences and heads in one launch, longest query blocks first.  32 rows of a sequence leave through tensor stores, staged where the ring was
+// (a thread's own stores touch 32 lines an instruction).  Bound by the bytes of dS and K that an SM takes in.
 #define AQ_THREADS 320
-#define AQ_STAGES 3
+// 64-wide heads, more CTAs than SMs: two stages, so that two CTAs share an SM and one loads and starts while the other ends (24 sequences of 383
+// tokens, 8 heads: backward call 155 -> 146 us, 8 x 2048: 517 -> 500).  A grid of one wave keeps three: launched early, beside what still runs,
+// small CTAs would share an SM while others idle (8 x 256: 47 -> 49 us).
+#define AQ_STAGES(NH, GRID) ((NH) == 1 && (GRID) > AF_ONE_WAVE ? 2 : 3)
 #define AQ_A_BYTES 32768                                // dS^T: 2 parts x 64 keys x 128 queries
 #define AQ_STAGE_BYTES(NH) (AQ_A_BYTES + (NH) * 16384)  // and K: 2 parts x 64 keys x head size
-#define AQ_SMEM(NH) (AQ_STAGES * AQ_STAGE_BYTES(NH) + 1024 + 256)
+#define AQ_SMEM(NH, STAGES) ((STAGES) * AQ_STAGE_BYTES(NH) + 1024 + 256)
 
 template <int HD>
-__global__ void __launch_bounds__(AQ_THREADS, 1)
+__global__ void __launch_bounds__(AQ_THREADS, HD == 64 ? 2 : 1)
 at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant__ CUtensorMap mS2,
-                 const __grid_constant__ CUtensorMap mK1, const __grid_constant__ CUtensorMap mK2,
+                 const __grid_constant__ CUtensorMap mK1, const __grid_constant__ CUtensorMap mK2, const __grid_constant__ CUtensorMap mdQ,
                  const AfSeqTab seqs, float* __restrict__ dQ, const float* __restrict__ ds_bound, const float* __restrict__ amax_k,
                  int Sp, int Hq, int g, int nqb_max, int* status, unsigned* amax_dq) {
     constexpr int NH = HD / 64, OC = HD / 2;
+    const int stages = AQ_STAGES(NH, gridDim.x);
     const int per_i = seqs.n * Hq;
     const int qb = nqb_max - 1 - (int)blockIdx.x / per_i;
     const int rem = (int)blockIdx.x % per_i;
@@ -620,14 +625,14 @@ at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant_
 
     extern __shared__ uint8_t af_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)af_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* full = (uint64_t*)(smem + AQ_STAGES * AQ_STAGE_BYTES(NH));
-    uint64_t* empty = full + AQ_STAGES;
-    uint64_t* acc_full = empty + AQ_STAGES;             // 2
+    uint64_t* full = (uint64_t*)(smem + stages * AQ_STAGE_BYTES(NH));
+    uint64_t* empty = full + stages;
+    uint64_t* acc_full = empty + stages;             // 2
     uint64_t* acc_empty = acc_full + 2;                 // 2
     uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < AQ_STAGES; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < stages; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
         for (int i = 0; i < 2; i++) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -648,9 +653,8 @@ at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant_
         // ---------------- TMA producer ----------------
         if (elect_one()) {
             const int y0 = af_slot_row(0, Hq, b, h, t0, S);
-            for (int j = 0; j < nkv && ok; j++) {
-                const int s = j % AQ_STAGES;
-                ok = mbar_wait(&empty[s], ((j / AQ_STAGES) & 1) ^ 1);
+            for (int j = 0, s = 0, turn = 0; j < nkv && ok; j++, s = s + 1 < stages ? s + 1 : 0, turn += s == 0) {
+                ok = mbar_wait(&empty[s], (turn & 1) ^ 1);
                 if (!ok) break;
                 uint8_t* st = smem + s * AQ_STAGE_BYTES(NH);
                 mbar_expect_tx(&full[s], AQ_STAGE_BYTES(NH));
@@ -669,9 +673,9 @@ at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant_
         // ---------------- MMA issuer ----------------
         if (elect_one()) {
             const uint32_t idesc = (1u << 4) | (1u << 15) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-            for (int j = 0; j < nkv && ok; j++) {
-                const int s = j % AQ_STAGES, e = j & 1;
-                ok = mbar_wait(&full[s], (j / AQ_STAGES) & 1) && mbar_wait(&acc_empty[e], ((j >> 1) & 1) ^ 1);
+            for (int j = 0, s = 0, turn = 0; j < nkv && ok; j++, s = s + 1 < stages ? s + 1 : 0, turn += s == 0) {
+                const int e = j & 1;
+                ok = mbar_wait(&full[s], turn & 1) && mbar_wait(&acc_empty[e], ((j >> 1) & 1) ^ 1);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t st = smem_u32(smem + s * AQ_STAGE_BYTES(NH));
@@ -717,13 +721,34 @@ at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant_
                 if constexpr (OC == 64) o[32 + i] += __uint_as_float(t2[i]);
             }
         }
+        ok = __all_sync(0xffffffffu, ok);
         float am = 0.f;
-        if (ok && qi < S) {
+        if (ok) {
             const float f1 = tc_pow2(-tc_f16_shift(sb_word(ds_bound))), f2 = tc_pow2(-tc_f16_shift(sb_word(amax_k)));
+#pragma unroll
+            for (int i = 0; i < OC; i++) o[i] = o[i] * f1 * f2;
+        }
+        if (ok && qb * 128 + q * 32 + 32 <= S) {
+            // 32 rows of the sequence: as tiles, through the ring (every load has been consumed)
+#pragma unroll
+            for (int c = 0; c < NH; c++) {
+                const uint32_t buf = smem_u32(smem) + (uint32_t)(((warp - 2) * NH + c) * 4096);
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const float4 v = make_float4(o[c * 32 + 4 * i], o[c * 32 + 4 * i + 1], o[c * 32 + 4 * i + 2], o[c * 32 + 4 * i + 3]);
+                    ab_sts4(buf + (uint32_t)(lane * 128 + ((i ^ (lane & 7)) << 4)), __float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
+                    am = sb_amax4(am, v);
+                }
+                AB_FENCE_ASYNC();
+                __syncwarp();
+                if (lane == 0) ab_tma_store(&mdQ, buf, h * HD + ch * OC + c * 32, t0 + qb * 128 + q * 32);
+            }
+            if (lane == 0) { AB_BULK_COMMIT(); AB_BULK_WAIT_READ(0); }
+        } else if (ok && qi < S) {
             float4* dst = (float4*)(dQ + (size_t)(t0 + qi) * Hq * HD + (size_t)h * HD + ch * OC);
 #pragma unroll
             for (int i = 0; i < OC / 4; i++) {
-                const float4 v = make_float4(o[4 * i] * f1 * f2, o[4 * i + 1] * f1 * f2, o[4 * i + 2] * f1 * f2, o[4 * i + 3] * f1 * f2);
+                const float4 v = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
                 dst[i] = v;
                 am = sb_amax4(am, v);
             }
@@ -749,7 +774,7 @@ static int ab_launch(sb_ctx_t* c, const AbCall& p) {
     static bool attr_done = false;
     if (!attr_done) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AB_SMEM(NH)) != cudaSuccess ||
-            cudaFuncSetAttribute(at_dq_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, AQ_SMEM(NH)) != cudaSuccess) { cudaGetLastError(); return 1; }
+            cudaFuncSetAttribute(at_dq_bwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, AQ_SMEM(NH, 3)) != cudaSuccess) { cudaGetLastError(); return 1; }
         attr_done = true;
     }
     const AfSeqTab seqs = {c->h_seq_n, c->attn_seq_starts};
@@ -758,7 +783,7 @@ static int ab_launch(sb_ctx_t* c, const AbCall& p) {
     if (Smax <= 0 || Smax > p.Sp) return 1;
     const int qd = p.Hq * HD, kvd = p.Hkv * HD, nkb = (Smax + AB_BK - 1) / AB_BK, g = p.Hq / p.Hkv;
     const int slot_pitch = p.dQ ? 0 : p.Sp;
-    CUtensorMap mQ1, mQ2, mD1, mD2, mK1, mK2, mV1, mV2, mS1, mS2, mdK, mdV, mA1, mA2, mB1, mB2;
+    CUtensorMap mQ1, mQ2, mD1, mD2, mK1, mK2, mV1, mV2, mS1, mS2, mdK, mdV, mdQ, mA1, mA2, mB1, mB2;
     if (!af_make_map(c, &mQ1, p.q1, p.T, qd, AB_BQ) || !af_make_map(c, &mQ2, p.q2, p.T, qd, AB_BQ) ||
         !af_make_map(c, &mD1, p.do1, p.T, qd, AB_BQ) || !af_make_map(c, &mD2, p.do2, p.T, qd, AB_BQ) ||
         !af_make_map(c, &mK1, p.k1, p.T, kvd, AB_BK) || !af_make_map(c, &mK2, p.k2, p.T, kvd, AB_BK) ||
@@ -777,7 +802,9 @@ static int ab_launch(sb_ctx_t* c, const AbCall& p) {
             !tc_encode(c, &mS2, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.dS2, sd, ss, sbx, CU_TENSOR_MAP_SWIZZLE_64B, np) ||
             !tc_encode(c, &mdK, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, p.dK, gd, gs, gbx, CU_TENSOR_MAP_SWIZZLE_128B, np) ||
             !tc_encode(c, &mdV, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, p.dV, gd, gs, gbx, CU_TENSOR_MAP_SWIZZLE_128B, np)) return 1;
-        if (p.dQ && (!tc_encode(c, &mA1, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.dS1, sd, ss, abx, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        const cuuint64_t qdim[2] = {(cuuint64_t)qd, (cuuint64_t)p.T}, qst[1] = {(cuuint64_t)qd * 4};
+        if (p.dQ && (!tc_encode(c, &mdQ, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, p.dQ, qdim, qst, gbx, CU_TENSOR_MAP_SWIZZLE_128B, np) ||
+                     !tc_encode(c, &mA1, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.dS1, sd, ss, abx, CU_TENSOR_MAP_SWIZZLE_128B) ||
                      !tc_encode(c, &mA2, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.dS2, sd, ss, abx, CU_TENSOR_MAP_SWIZZLE_128B) ||
                      !af_make_map(c, &mB1, p.k1, p.T, kvd, 64) || !af_make_map(c, &mB2, p.k2, p.T, kvd, 64))) return 1;
     }
@@ -792,7 +819,7 @@ static int ab_launch(sb_ctx_t* c, const AbCall& p) {
         p.amax_q, p.amax_k, p.amax_v, p.amax_do, p.ds_bound, seqs, p.Sp, p.Hq, g, nkb, chunk, p.accumulate, slot_pitch, 1.0f / sqrtf((float)HD), c->d_status, p.amax_dk, p.amax_dv);
     c->launches++;
     if (p.dQ) {
-        sb_launch(at_dq_bwd_kernel<HD>, dim3((unsigned)qblocks), dim3(AQ_THREADS), AQ_SMEM(NH), st, mA1, mA2, mB1, mB2, seqs, p.dQ, p.ds_bound, p.amax_k, p.Sp, p.Hq, g, nkb, c->d_status, p.amax_dq);
+        sb_launch(at_dq_bwd_kernel<HD>, dim3((unsigned)qblocks), dim3(AQ_THREADS), AQ_SMEM(NH, AQ_STAGES(NH, qblocks)), st, mA1, mA2, mB1, mB2, mdQ, seqs, p.dQ, p.ds_bound, p.amax_k, p.Sp, p.Hq, g, nkb, c->d_status, p.amax_dq);
         c->launches++;
     }
     return cudaGetLastError() == cudaSuccess ? 0 : 1;

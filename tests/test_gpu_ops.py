@@ -297,6 +297,33 @@ def test_attention_on_chip_short_and_ragged(ctx, ss, Hq, Hkv, hd):
     ctx.release(bq, bk, bv, bdo, bs, bout, blse, bdq, bdk, bdv)
 
 
+@pytest.mark.parametrize("lens,Hq,Hkv,hd", [([383, 31, 129, 256, 97] * 9, 4, 2, 64), ([1100, 1023, 1024, 1025, 900, 1311, 1, 1500, 1217, 1088, 1152, 1153], 1, 1, 128)])
+def test_attention_backward_dq_of_many_sequences(ctx, lens, Hq, Hkv, hd):
+    """dQ in one launch: at 64 more tiles than SMs (two CTAs an SM on two stages, rows in tiles of 32 beside the last rows of a sequence), at 128 long
+    sequences, more of them than one launch of the grouped kernel takes.  The bound of a sequence is twice that of the whole."""
+    ss = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint32)
+    T, B = int(ss[-1]), len(lens)
+    r = rng(T + Hq + hd)
+    Q, K, V = f32(r.standard_normal((T, Hq * hd))), f32(r.standard_normal((T, Hkv * hd))), f32(r.standard_normal((T, Hkv * hd)))
+    dO, dK0 = f32(r.standard_normal(Q.shape)), f32(np.zeros(K.shape))
+    out_ref, lse_ref, dQ_ref, dK_ref, dV_ref = np.empty_like(Q), np.empty((T, Hq), np.float32), np.empty_like(Q), dK0.copy(), dK0.copy()
+    O.lib().ref_attention(Q, K, V, out_ref, lse_ref, ss, T, B, Hq, Hkv, hd)
+    O.lib().ref_attention_backward(Q, K, V, dO, dQ_ref, dK_ref, dV_ref, ss, T, B, Hq, Hkv, hd)
+    bq, bk, bv, bdo, bs = ctx.upload(Q), ctx.upload(K), ctx.upload(V), ctx.upload(dO), ctx.upload(ss)
+    bout, blse, bdq, bdk, bdv = ctx.zeros(Q.size), ctx.zeros(T * Hq), ctx.empty(Q.size), ctx.upload(dK0), ctx.upload(dK0)
+    ctx.lib.cuda_train_batch_attention_packed(ctx.h, bq.b, bk.b, bv.b, bout.b, blse.b, bs.b, T, B, Hq, Hkv, hd, max(lens))
+    ctx.lib.cuda_train_batch_attention_backward_packed(ctx.h, bq.b, bk.b, bv.b, bout.b, blse.b, bdo.b, bdq.b, bdk.b, bdv.b, bs.b,
+                                                       T, B, Hq, Hkv, hd, max(lens))
+    ctx.check()
+    dQ = bdq.numpy().reshape(Q.shape)
+    for got, ref in zip((dQ, bdk.numpy().reshape(K.shape), bdv.numpy().reshape(K.shape)), (dQ_ref, dK_ref, dV_ref)):
+        assert rel_l2(got, ref) < TOL
+    for b in range(B):
+        if lens[b] > 1:                               # (of one row dS is zero but for rounding)
+            assert rel_l2(dQ[ss[b]:ss[b + 1]], dQ_ref[ss[b]:ss[b + 1]]) < 2 * TOL
+    ctx.release(bq, bk, bv, bdo, bs, bout, blse, bdq, bdk, bdv)
+
+
 def test_attention_unpacked_single_sequence(ctx):
     T, Hq, Hkv, hd = 70, 4, 4, 32
     r = rng(70)
