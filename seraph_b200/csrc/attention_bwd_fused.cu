@@ -113,7 +113,7 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
                   __half* __restrict__ dS1, __half* __restrict__ dS2, float* __restrict__ dK, float* __restrict__ dV,
                   const float* __restrict__ amax_q, const float* __restrict__ amax_k, const float* __restrict__ amax_v,
                   const float* __restrict__ amax_do, const float* __restrict__ ds_bound,
-                  const AfSeqTab seqs, int Sp, int Hq, int g, int nkb, int chunk, int accumulate, int slot_pitch, float scale, int* status,
+                  const AfSeqTab seqs, int Sp, int Hq, int g, int nkb, int chunk, int accumulate, int upper, float scale, int* status,
                   unsigned* amax_dk, unsigned* amax_dv) {
     constexpr int NH = HD / 64;
     constexpr int KV_PART = NH * 16384, ST_PART = NH * 4096;
@@ -204,7 +204,7 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
                     af_tma_2d(smem + p * 16384, &mV1, kv_full, kvh * HD + p * 64, t0 + k0);
                     af_tma_2d(smem + KV_PART + p * 16384, &mV2, kv_full, kvh * HD + p * 64, t0 + k0);
                 }
-                const int slot0 = af_slot_row(slot_pitch, Hq, b, kvh * g, t0, S), slot_rows = slot_pitch > 0 ? slot_pitch : (S + 127) & ~127;
+                const int slot0 = af_slot_row(Hq, b, kvh * g, t0, S), slot_rows = (S + 127) & ~127;
                 for (int t = 0; t < nsteps && ok; t++) {
                     const int s = t % AB_STAGES, u = t / AB_STAGES;
                     const int h = kvh * g + t / per_head, j = j0 + t % per_head;
@@ -465,7 +465,7 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
             if (lane == 0) af_arrive(k_ready);
         }
         ok = ok && mbar_wait(k_ready, 0);                       // every warp has its rows of K out of the staging area
-        const int slot0 = af_slot_row(slot_pitch, Hq, b, kvh * g, t0, S), slot_rows = slot_pitch > 0 ? slot_pitch : (S + 127) & ~127;      // this K/V head's slots
+        const int slot0 = af_slot_row(Hq, b, kvh * g, t0, S), slot_rows = (S + 127) & ~127;      // this K/V head's slots
         const uint32_t ews = smem_u32(smem + AB_OFF_EWS(NH));
         const bool issuer = warp == 4 && lane == 0;            // hands the staged tiles to the TMA unit
         // Columns before this key block that the dQ product reads together with it (its query tiles are 256 wide): zeros, stored
@@ -474,7 +474,7 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
         // before it arrives it makes sure that everything it handed over earlier has been read.  So a completed phase n tells every
         // warp that the tiles handed over in phases < n are read out: a buffer is written again one phase after the next.
         int sync_n = 0;
-        if (slot_pitch > 0 && (k0 & 255) != 0 && ok) {
+        if (upper && (k0 & 255) != 0 && ok) {
             ab_sts4(ews + 16384 + (uint32_t)((warp - 4) * 1024 + lane * 32), 0, 0, 0, 0);
             ab_sts4(ews + 16384 + (uint32_t)((warp - 4) * 1024 + lane * 32 + 16), 0, 0, 0, 0);
             AB_FENCE_ASYNC();
@@ -652,7 +652,7 @@ at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant_
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (elect_one()) {
-            const int y0 = af_slot_row(0, Hq, b, h, t0, S);
+            const int y0 = af_slot_row(Hq, b, h, t0, S);
             for (int j = 0, s = 0, turn = 0; j < nkv && ok; j++, s = s + 1 < stages ? s + 1 : 0, turn += s == 0) {
                 ok = mbar_wait(&empty[s], (turn & 1) ^ 1);
                 if (!ok) break;
@@ -782,7 +782,7 @@ static int ab_launch(sb_ctx_t* c, const AbCall& p) {
     for (int b = 0; b < c->h_seq_n; b++) Smax = max(Smax, c->h_seq[b + 1] - c->h_seq[b]);
     if (Smax <= 0 || Smax > p.Sp) return 1;
     const int qd = p.Hq * HD, kvd = p.Hkv * HD, nkb = (Smax + AB_BK - 1) / AB_BK, g = p.Hq / p.Hkv;
-    const int slot_pitch = p.dQ ? 0 : p.Sp;
+    const int upper = !p.dQ;                             // the product over tiles of 256 queries reads 128 columns left of odd key blocks: zeros
     CUtensorMap mQ1, mQ2, mD1, mD2, mK1, mK2, mV1, mV2, mS1, mS2, mdK, mdV, mdQ, mA1, mA2, mB1, mB2;
     if (!af_make_map(c, &mQ1, p.q1, p.T, qd, AB_BQ) || !af_make_map(c, &mQ2, p.q2, p.T, qd, AB_BQ) ||
         !af_make_map(c, &mD1, p.do1, p.T, qd, AB_BQ) || !af_make_map(c, &mD2, p.do2, p.T, qd, AB_BQ) ||
@@ -791,7 +791,7 @@ static int ab_launch(sb_ctx_t* c, const AbCall& p) {
     {
         // dS^T parts: [rows of the head slots: keys][Sp queries] halfs, tiles of 32 queries x 128 keys, rows of 64 bytes with the 64-byte swizzle in shared memory;
         // dK, dV: [T][kvd] floats, tiles of 32 columns x 32 keys, 128-byte swizzle
-        const cuuint64_t rows = af_slot_rows(slot_pitch, p.Hq, seqs.n, p.T);
+        const cuuint64_t rows = af_slot_rows(p.Hq, seqs.n, p.T);
         const cuuint64_t sd[2] = {(cuuint64_t)p.Sp, rows}, ss[1] = {(cuuint64_t)p.Sp * 2};
         const cuuint32_t sbx[2] = {32u, 128u}, abx[2] = {64u, 64u};
         const cuuint64_t gd[2] = {(cuuint64_t)kvd, (cuuint64_t)p.T}, gs[1] = {(cuuint64_t)kvd * 4};
@@ -816,7 +816,7 @@ static int ab_launch(sb_ctx_t* c, const AbCall& p) {
     if (qblocks > 0x7fffffffL) return 1;
     cudaStream_t st = (cudaStream_t)c->pub.stream;
     sb_launch(kern, dim3((unsigned)blocks), dim3(AB_THREADS), AB_SMEM(NH), st, mQ1, mQ2, mD1, mD2, mK1, mK2, mV1, mV2, mS1, mS2, mdK, mdV, p.LT, p.DT, (__half*)p.dS1, (__half*)p.dS2, p.dK, p.dV,
-        p.amax_q, p.amax_k, p.amax_v, p.amax_do, p.ds_bound, seqs, p.Sp, p.Hq, g, nkb, chunk, p.accumulate, slot_pitch, 1.0f / sqrtf((float)HD), c->d_status, p.amax_dk, p.amax_dv);
+        p.amax_q, p.amax_k, p.amax_v, p.amax_do, p.ds_bound, seqs, p.Sp, p.Hq, g, nkb, chunk, p.accumulate, upper, 1.0f / sqrtf((float)HD), c->d_status, p.amax_dk, p.amax_dv);
     c->launches++;
     if (p.dQ) {
         sb_launch(at_dq_bwd_kernel<HD>, dim3((unsigned)qblocks), dim3(AQ_THREADS), AQ_SMEM(NH, AQ_STAGES(NH, qblocks)), st, mA1, mA2, mB1, mB2, mdQ, seqs, p.dQ, p.ds_bound, p.amax_k, p.Sp, p.Hq, g, nkb, c->d_status, p.amax_dq);
@@ -827,7 +827,7 @@ static int ab_launch(sb_ctx_t* c, const AbCall& p) {
 
 // See AbCall for the operands.  Returns 0 when launched, 1 when this path does not take the call.
 int sb_attention_fused_dkv(sb_ctx_t* c, const AbCall& p, int hd) {
-    if ((p.Sp % (p.dQ ? 128 : 256)) || p.Hkv <= 0 || p.Hq % p.Hkv || !tc_load_encode()) return 1;
+    if (p.Sp % 128 || p.Hkv <= 0 || p.Hq % p.Hkv || !tc_load_encode()) return 1;
     if (c->h_seq_n <= 0 || !c->attn_seq_starts) return 1;
     if (!tc_aligned16(p.dK) || !tc_aligned16(p.dV) || !tc_aligned16(p.dQ)) return 1;
     if (hd == 128) return ab_launch<128>(c, p);

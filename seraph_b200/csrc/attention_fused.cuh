@@ -18,13 +18,13 @@ struct AfSeqs { int n; int start[AF_MAXSEQ + 1]; };
 struct AfSeqTab { int n; const uint32_t* start; };      // sequence boundaries in device memory, n + 1 of them
 
 // First row of (sequence b, head h) in the backward's per-head scratch (rows of dS^T are keys; of LT and DT the row's one value).
-// pitch > 0: every slot has `pitch` rows.  pitch == 0: slots have the sequence's own length rounded up to 128, so that short sequences
+// Slots have the sequence's own length rounded up to 128, so that short sequences
 // packed beside a long one cost what they need; 128 (t0 / 128 + b) is at least the sum of the rounded lengths before sequence b.
-__host__ __device__ __forceinline__ int af_slot_row(int pitch, int Hq, int b, int h, int t0, int S) {
-    return pitch > 0 ? (b * Hq + h) * pitch : Hq * (((t0 >> 7) + b) << 7) + h * ((S + 127) & ~127);
+__host__ __device__ __forceinline__ int af_slot_row(int Hq, int b, int h, int t0, int S) {
+    return Hq * (((t0 >> 7) + b) << 7) + h * ((S + 127) & ~127);
 }
-static inline size_t af_slot_rows(int pitch, int Hq, int n, int T) {
-    return pitch > 0 ? (size_t)n * Hq * pitch : (size_t)Hq * ((((size_t)T >> 7) + n + 1) << 7);
+static inline size_t af_slot_rows(int Hq, int n, int T) {
+    return (size_t)Hq * ((((size_t)T >> 7) + n + 1) << 7);
 }
 
 #define AF_Q_BYTES 65536
@@ -130,8 +130,8 @@ static inline bool af_make_map(sb_ctx_t* c, CUtensorMap* m, const void* base, in
 // The backward with dK and dV kept on chip.  q, do, k, v: the FP16 parts of Q, dO [T, Hq*hd] and K, V [T, Hkv*hd]; amax_*: the device words
 // their scales derive from; ds_bound: the device word that bounds |dS|.  dS1/dS2: the parts of dS^T, laid out
 // [slot of (sequence, head): af_slot_row][Sp] (key rows, query columns).  LT, DT: the log-sum-exp and D, one value per row of the
-// slots (row = query), in the form at_bwd_prep2_kernel writes.  accumulate: dK and dV are added into, else written.  dQ given: dQ = dS K follows in a second launch
-// (Sp a multiple of 128, slots of the sequences' own lengths); NULL: the caller forms it (Sp a multiple of 256, slots of Sp rows).
+// slots (row = query), in the form at_bwd_prep2_kernel writes.  accumulate: dK and dV are added into, else written.  dQ given: dQ = dS K follows in a second launch;
+// NULL: the caller forms it in tiles of 256 queries, and the columns such a tile reads above the diagonal are cleared.  Sp a multiple of 128.
 struct AbCall {
     const void *q1, *q2, *do1, *do2, *k1, *k2, *v1, *v2;
     const float *amax_q, *amax_k, *amax_v, *amax_do, *ds_bound, *LT, *DT;

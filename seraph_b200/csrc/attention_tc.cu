@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(256) at_bwd_prep_kernel(const float* __restric
 __global__ void __launch_bounds__(256) at_bwd_prep2_kernel(const float4* __restrict__ dO, size_t n4, uint2* __restrict__ h1, uint2* __restrict__ h2,
                                                            const float* __restrict__ amax, float* consts, const float* __restrict__ norm_do, const float* __restrict__ norm_v, float scale,
                                                            const float* __restrict__ lse, const float* __restrict__ D, float* __restrict__ LT, float* __restrict__ DT,
-                                                           const AfSeqTab seqs, int Hq, int Smax, int slot_pitch, int natural) {
+                                                           const AfSeqTab seqs, int Hq, int Smax, int natural) {
     sb_pdl_enter();
     const float bound = 2.0f * sb_word(norm_do) * sb_word(norm_v) * scale;
     if (blockIdx.y == 0 && blockIdx.x == 0 && threadIdx.x == 0) { consts[0] = 1.0f; consts[1] = bound; }
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(256) at_bwd_prep2_kernel(const float4* __restr
         if (q - lane >= S) continue;
         float a = 0.f, d = 0.f;
         if (q < S) { const float L = __ldg(&lse[(size_t)(t0 + q) * Hq + h]); a = natural ? -L : 14.f - L * 1.4426950408889634f; d = __ldg(&D[(size_t)(t0 + q) * Hq + h]) * dsc; }
-        const size_t o = (size_t)af_slot_row(slot_pitch, Hq, b, h, t0, S) + q;
+        const size_t o = (size_t)af_slot_row(Hq, b, h, t0, S) + q;
         LT[o] = a; DT[o] = d;
     }
 }
@@ -564,12 +564,13 @@ static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, cons
     if (at_have_seq(c, T)) n = c->h_seq_n;
     for (int b = 0; b < n; b++) { const int S = c->h_seq[b + 1] - c->h_seq[b]; Smax = max(Smax, S); flops += 5.0 * Hq * (double)S * S * hd; }
     if (Smax <= 0) { sb_tick_end(c, tk, 0.0, 0.0); return 1; }
-    // Long sequences of 128-wide heads: dQ from the kernel of grouped products (256-row tiles read K half as often).
-    // Shorter ones and 64-wide heads: at_dq_bwd_kernel, one launch for all.  8 x 2048 tokens, 16 heads: 1.57 against 1.67 ms for the whole
-    // call; 5 sequences of 1080 on average: equal; 33M model, 24 sequences of 240: a launch instead of 24.
-    const bool dq_gemm = hd == 128 && (long)n * 1024 <= T;
-    const int Sp = round_up(Smax, dq_gemm ? AT_ROWTILE : 128), slot_pitch = dq_gemm ? Sp : 0;
-    const size_t rows = af_slot_rows(slot_pitch, Hq, n, T), n_ds = rows * (size_t)Sp, row_floats = (rows + 63) & ~(size_t)63;
+    // Long sequences of 128-wide heads: dQ from the kernel of grouped products (256-row tiles read K half as often).  Shorter ones, where much of a
+    // 256-row tile is above the diagonal, and 64-wide heads: at_dq_bwd_kernel.  The whole call, 16 heads, by this kernel and by the products: 8 x 2048 tokens
+    // 1543 and 1415 us, 16 x 1024 909 and 860, 20 of 384 on average 385 and 375, 32 of 260 372 and 368, 60 x 256 498 and 503, 60 of 130 355 and 365.
+    // Of few heads, ten sequences a launch do not fill the chip: one launch of at_dq_bwd_kernel does.
+    const bool dq_gemm = hd == 128 && ((long)n * 1024 <= T || ((long)n * 320 <= T && (n <= 10 || Hq >= 8)));
+    const int Sp = round_up(Smax, 128);
+    const size_t rows = af_slot_rows(Hq, n, T), n_ds = rows * (size_t)Sp, row_floats = (rows + 63) & ~(size_t)63;
     float* bb = (float*)sb_gemm_stage(c, 3, n_ds * 4 + 2 * row_floats * sizeof(float));
     if (!bb) { sb_tick_end(c, tk, 0.0, 0.0); return 1; }
     float* LT = bb + n_ds; float* DT = LT + row_floats;
@@ -578,7 +579,7 @@ static int at_backward_on_chip(sb_ctx_t* c, const float* Q, const float* K, cons
         const int rows_blocks = (int)(((long)n * ((Smax + 31) / 32) * Hq + 7) / 8);      // a warp for 32 rows
         const dim3 pg = left ? dim3((unsigned)max(1, min(rows_blocks, c->pub.gpu_sm_count * 8))) : dim3(tc_ew_blocks(c, n_q / 8), 2);
         sb_launch(at_bwd_prep2_kernel, pg, dim3(256), 0, st, (const float4*)dO, n_q / 4, left ? (uint2*)nullptr : (uint2*)hdo, (uint2*)(hdo + n_q), am_do,
-                                                                            consts, norm_do, norm_v, scale, lse, D, LT, DT, seqs, Hq, Smax, slot_pitch, hd == 64 ? 1 : 0);
+                                                                            consts, norm_do, norm_v, scale, lse, D, LT, DT, seqs, Hq, Smax, hd == 64 ? 1 : 0);
         c->launches++;
     }
     __half* a = (__half*)bb;

@@ -30,6 +30,7 @@
 #include <stdio.h>
 #include <type_traits>
 #include "gemm_tc.cuh"
+#include "attention_fused.cuh"
 
 #define GG_MAXP 10               // products per launch
 #define GG_MAXS 10               // segments per launch
@@ -134,7 +135,7 @@ struct GgShape {
     static constexpr int A_PART = 128 * 128, B_PART = (BN / 2) * 128;
     static constexpr int STAGE = A_PART + B_PART;                  // one part of both operands
     // A load takes about a microsecond under load: 1.5 (BN = 256) to 3 (BN = 128) chunks of MMA time ahead of the one being multiplied.  With the
-    // narrow tile six stages and two buffers per warp were 13 % slower than eight and one.
+    // narrow tile six stages and two buffers per warp take 0.97 to 1.03 of the time of eight and one.
     static constexpr int STAGES = BN == 256 ? 5 : 8;
     static constexpr int NBUF = BN == 256 ? 2 : 1;                 // output staging: blocks of 32 rows x 32 columns per epilogue warp
     static constexpr int STG = 8 * NBUF * 4096;
@@ -899,10 +900,10 @@ extern "C" int sb_gemm_group_try(sb_ctx_t* c, const sb_gemm_job_t* jobs, int njo
     return 0;
 }
 
-// dQ = dS K of an attention backward: for every sequence and query head [S, 128] from the parts of dS^T ([slot = sequence, head][key][query], rows of Sp) and of
-// K.  The query rows of a tile of 256 need the keys up to its last row.  A product is a sequence; its tiles of all heads are items of one launch, which
-// takes GG_MAXP sequences.  (A launch per sequence of gemm_tc_kernel, two of them side by side: 8 x 2048 tokens, 16 heads, 296 us; the parts of dS
-// alone, 1.07 GB, take 164.)  starts: boundaries on the host.  0: launched.
+// dQ = dS K of an attention backward: for every sequence and query head [S, 128] from the parts of dS^T ([slot of (sequence, head): af_slot_row][key][query], rows of Sp) and
+// of K.  The query rows of a tile of 256 need the keys up to its last row.  A product is a sequence; its tiles of all heads are items of one launch, which
+// takes GG_MAXP sequences.  (A launch per sequence of gemm_tc_kernel, two of them side by side: 8 x 2048 tokens, 16 heads, 296 us; this 250,
+// of which the parts of dS alone, 1.07 GB, take 164.)  starts: boundaries on the host.  0: launched.
 extern "C" int sb_gemm_dq(sb_ctx_t* c, const void* ds, size_t ds_part, const float* ds_bound, const void* k, size_t k_part, const float* amax_k, float* dQ,
                           const int* starts, int nseq, int Sp, int Hq, int g) {
     if (!tc_load_encode()) return 1;
@@ -928,9 +929,9 @@ extern "C" int sb_gemm_dq(sb_ctx_t* c, const void* ds, size_t ds_part, const flo
             q->M = S; q->N = qd; q->bn = 128; q->tiles_m = (S + 255) / 256; q->tiles_n = Hq; q->seg0 = i; q->nseg = 1; q->kb = sg->kb;
             p.run[i].item0 = p.items; p.run[i].prob = i; p.run[i].split = 1;
             p.items += q->tiles_m * Hq;
-            const cuuint64_t ad[4] = {(cuuint64_t)S, (cuuint64_t)S, (cuuint64_t)Hq, 2}, as[3] = {(cuuint64_t)Sp * 2, (cuuint64_t)Sp * Sp * 2, (cuuint64_t)ds_part * 2};
+            const cuuint64_t ad[4] = {(cuuint64_t)S, (cuuint64_t)S, (cuuint64_t)Hq, 2}, as[3] = {(cuuint64_t)Sp * 2, (cuuint64_t)((S + 127) & ~127) * Sp * 2, (cuuint64_t)ds_part * 2};
             const cuuint32_t abox[4] = {64u, 64u, 1u, 1u}, one[4] = {1u, 1u, 1u, 1u};
-            if (g_tc_encode(&sg->a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, (void*)((const __half*)ds + (size_t)seq[i] * Hq * Sp * Sp), ad, as, abox, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            if (g_tc_encode(&sg->a, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, (void*)((const __half*)ds + (size_t)af_slot_row(Hq, seq[i], 0, t0, S) * Sp), ad, as, abox, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return 1;
             const cuuint64_t bd[3] = {(cuuint64_t)kvd, (cuuint64_t)S, 2}, bs[2] = {(cuuint64_t)kvd * 2, (cuuint64_t)k_part * 2};
             const cuuint32_t bbox[3] = {64u, 64u, 1u};

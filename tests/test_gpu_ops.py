@@ -297,10 +297,11 @@ def test_attention_on_chip_short_and_ragged(ctx, ss, Hq, Hkv, hd):
     ctx.release(bq, bk, bv, bdo, bs, bout, blse, bdq, bdk, bdv)
 
 
-@pytest.mark.parametrize("lens,Hq,Hkv,hd", [([383, 31, 129, 256, 97] * 9, 4, 2, 64), ([1100, 1023, 1024, 1025, 900, 1311, 1, 1500, 1217, 1088, 1152, 1153], 1, 1, 128)])
+@pytest.mark.parametrize("lens,Hq,Hkv,hd", [([383, 31, 129, 256, 97] * 9, 4, 2, 64), ([1100, 1023, 1024, 1025, 900, 1311, 1, 1500, 1217, 1088, 1152, 1153], 1, 1, 128),
+                                             ([383, 700, 129, 256, 1, 640, 511] * 2, 8, 4, 128)])
 def test_attention_backward_dq_of_many_sequences(ctx, lens, Hq, Hkv, hd):
-    """dQ in one launch: at 64 more tiles than SMs (two CTAs an SM on two stages, rows in tiles of 32 beside the last rows of a sequence), at 128 long
-    sequences, more of them than one launch of the grouped kernel takes.  The bound of a sequence is twice that of the whole."""
+    """dQ in one launch: at 64 more tiles than SMs (two CTAs an SM on two stages, rows in tiles of 32 beside the last rows of a sequence), at 128
+    sequences of 320 tokens and more on average, more of them than one launch of the grouped kernel takes.  The bound of a sequence is twice that of the whole."""
     ss = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint32)
     T, B = int(ss[-1]), len(lens)
     r = rng(T + Hq + hd)
