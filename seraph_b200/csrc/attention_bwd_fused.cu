@@ -22,8 +22,8 @@
 // performed in L2).  A dK/dV element is only ever touched by the one CTA that owns its key, one chain's additions have
 // been performed before the next chain's are issued, and the output is zeroed (or holds the caller's values) before the
 // launch: the result does not depend on scheduling and is the same bits on every run.
-// dS^T also leaves the chip, as FP16 parts laid out [head slot = (sequence, K/V head, group member)][key][query]: dQ = dS K is one more product on the
-// GEMM kernel (M = queries, K = keys up to the diagonal, A read MN-major).  P never reaches memory, dS is written once
+// dS^T also leaves the chip, as FP16 parts laid out [head slot = (sequence, K/V head, group member)][key][query]: dQ = dS K is one more launch, of the
+// grouped kernel (long 128-wide sequences) or of at_dq_bwd_kernel below (keys up to the diagonal, A read MN-major).  P never reaches memory, dS is written once
 // and read once: 8 bytes per score element instead of the 20 of the score-materialising path.
 //
 // Everything that leaves the CTA goes through shared memory and the TMA unit.  With one key row per thread (the layout
