@@ -908,18 +908,20 @@ static __global__ void __launch_bounds__(256) tc_split_f16_kernel(const float* _
     }
 }
 
-// FP16 parts of up to TC_MULTI tensors with one read of each.  The scale of a tensor whose largest magnitude nobody left is a guess: four times the largest
-// of 16384 scattered elements, taken as if it were the maximum.  The pass that writes the parts compares every element with it, and a third launch makes
-// the parts again, with the true maximum, of a tensor that has a larger one (a single outlier among many millions); for all others it ends at once.  Parts
-// are floating point, so a scale that is two bits low costs nothing above 2^-15 of the largest element (sb_split2), and the scale is a function of the
-// tensor alone.  Bytes bound it, 12 for each element: three tensors of
+// FP16 parts of up to TC_MULTI tensors with one read of each.  The scale of a tensor whose largest magnitude nobody left is a guess: that of the largest
+// of 16384 scattered elements, which the true maximum is never below.  It brings the sample's largest to [2^14, 2^15), and FP16 holds 65504: room for elements
+// two to four times as large.  The pass that writes the parts compares every element with that, and a third launch makes the parts again, with the
+// scale of the true maximum, of a tensor that has a larger one; for all others it ends at once.  So an element keeps the bits that the scale of the
+// true maximum would give it, or one more, and the scale is a function of the tensor alone.
+// The word that goes with the parts tells their scale; it is no bound of a tensor whose scale was guessed.  Bytes bound it, 12 for each element: three tensors of
 // 8 x 2048 x 2048 floats take 139 us, 131 of them in the split at 6.1 TB/s (198 with a pass for the maximum before it); small tensors are launches:
 // the 57 weights of the 33M model (120 MB) take three, 50 us (twelve and 78 when maximum and split passes ran in batches that fit L2).
 #define TC_MULTI 96
 #define TC_MULTI_CHUNK 1024
 #define TC_SAMPLE 4096                        // float4s looked at for the guess: 16 a thread
+#define TC_NO_SCALE 0x1p-100f                 // maxima below this are not scaled (sb_f16_shift)
 // h: hi parts, lo parts behind them; first: its first chunk; amax: the word the products read; guess: NULL when *amax is there already, else two words
-// of the tensor's own: the guess, and the largest magnitude above it (zero when there is none)
+// of the tensor's own: the guess, and the true maximum where the guess does not do (else zero)
 struct TcMultiJob { const float* x; __half* h; float* amax; float* guess; uint32_t n4, first; };
 struct TcMulti { int n, guesses; uint32_t chunks; unsigned keep; TcMultiJob j[TC_MULTI]; };
 static inline void tc_multi_begin(TcMulti* m) { m->n = m->guesses = 0; m->chunks = 0; }
@@ -958,7 +960,6 @@ static __global__ void __launch_bounds__(256) tc_guess_kernel(const __grid_const
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[w]);
-        if (j.n4 > TC_SAMPLE) mx *= 4.f;
         j.guess[0] = mx; j.guess[1] = 0.f; *j.amax = mx;
     }
 }
@@ -973,16 +974,15 @@ static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid
         const int jb = tc_multi_find(m, ck - 1);
         const TcMultiJob& j = m.j[jb];
         const uint32_t stop = max(begin, j.first);
-        float top = INFINITY;                 // what no element may exceed
+        float top;                            // the scale's word
         if (REDO) {
-            const float above = j.guess ? sb_word(j.guess + 1) : 0.f;
-            if (above == 0.f) { ck = stop; continue; }
-            top = above;
-            if (stop == j.first && threadIdx.x == 0) *j.amax = above;      // nobody reads it in this launch
-        } else if (j.guess) top = sb_word(j.guess);
+            top = j.guess ? sb_word(j.guess + 1) : 0.f;
+            if (top == 0.f) { ck = stop; continue; }
+            if (stop == j.first && threadIdx.x == 0) *j.amax = top;        // nobody reads it in this launch
+        } else top = sb_word(j.guess ? j.guess : j.amax);
         const float4* x = (const float4*)j.x;
         uint2* h1 = (uint2*)j.h; uint2* h2 = h1 + j.n4;
-        const float sc = tc_pow2(tc_f16_shift(!REDO && !j.guess ? sb_word(j.amax) : top));
+        const float sc = tc_pow2(tc_f16_shift(top));
         float mx = 0.f;
         while (ck > stop) {
             ck--;
@@ -998,7 +998,8 @@ static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid
                 h1[base + u * 256] = a; h2[base + u * 256] = b;
             }
         }
-        if (!REDO && mx > top) atomicMax((unsigned*)(j.guess + 1), __float_as_uint(mx));
+        // beyond FP16's range; or a sample of (nearly) nothing but zeros, which is not scaled, beside elements that would be
+        if (!REDO && j.guess && (mx * sc > 65504.f || (top < TC_NO_SCALE && mx >= TC_NO_SCALE))) atomicMax((unsigned*)(j.guess + 1), __float_as_uint(mx));
     }
 }
 static inline unsigned tc_multi_grid(sb_ctx_t* c, const TcMulti& m) {

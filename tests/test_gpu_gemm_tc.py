@@ -121,9 +121,8 @@ def test_single_pass_mode_keeps_small_products_accurate(ctx, M, N, K, single, tA
 @pytest.mark.parametrize("kind", ["normal", "outlier", "one element", "zeros", "inf", "nan"])
 @pytest.mark.parametrize("M,N,K", [(512, 256, 1024), (64, 128, 256), (1000, 264, 136)])
 def test_scale_of_the_parts_is_checked_against_every_element(ctx, M, N, K, kind):
-    """The scale of an operand's FP16 parts is guessed from 16384 of its elements; one above four times the largest of those (an element that few samples
-    hit, the only one that is not zero) must give the scale of the true maximum, and not the overflow of the guessed one.  Operands that are
-    looked at whole (64 x 256) have no guess."""
+    """The scale of an operand's FP16 parts is guessed from 16384 of its elements; one that FP16 cannot hold under it (an element that few samples
+    hit, the only one that is not zero) must give the scale of the true maximum, and not the overflow of the guessed one."""
     r = np.random.default_rng(M + K)
     A, B = r.standard_normal((M, K)).astype(np.float32), r.standard_normal((N, K)).astype(np.float32)
     if kind in ("one element", "zeros"):
@@ -141,6 +140,29 @@ def test_scale_of_the_parts_is_checked_against_every_element(ctx, M, N, K, kind)
         ref = A.astype(np.float64) @ B.T.astype(np.float64)
         for y in range(0, M, 64):
             assert rel_l2(out[y:y + 64], ref[y:y + 64]) < BOUND[4] or not ref[y:y + 64].any() and not out[y:y + 64].any()
+    ctx.release(a, b, c)
+
+
+@pytest.mark.parametrize("M,peak,unit", [(8, 1.0, 1.0), (8, 1.99, 1.0), (120, 1.0, 1.0), (4096, 1.0, 1.0), (4096, 1.99, 1.0), (4096, 2.6, 1.0), (4096, 3.9, 1.0),
+                                         (4096, 7.0, 1.0), (4096, 1.0, 2.0 ** -60), (4096, 3.9, 2.0 ** -60), (4096, 2.0 ** 80, 1.0)])
+def test_parts_keep_the_bits_of_the_true_scale(ctx, M, peak, unit):
+    """An operand times the identity is its two parts, added: under the scale of its true maximum, 2^s with max 2^s in [2^14, 2^15), each element is within
+    2^-23 of itself (hi and lo part, 11 bits each, rounded to nearest) or within half of FP16's smallest step, 2^-25, whichever is larger.  No guess of
+    that scale may cost more.  The largest element lies where a sample of 16384 need not see it, among others below 1."""
+    K = 256
+    r = np.random.default_rng(M)
+    A = (r.choice([-1, 1], (M, K)) * 2.0 ** r.uniform(-34, 0, (M, K))).astype(np.float32)
+    A[M - 3, K - 5] = peak
+    A *= np.float32(unit)
+    top = float(np.abs(A).max())
+    a, b, c = ctx.upload(A), ctx.upload(np.eye(K, dtype=np.float32)), ctx.zeros(M * K)
+    ctx.lib.cuda_train_matmul_transpose(ctx.h, a.b, b.b, c.b, M, K, K, 0, 1, 0)
+    out = c.numpy(shape=(M, K)).astype(np.float64)
+    ctx.check()
+    s = 14 - int(np.floor(np.log2(top)))
+    bound = np.maximum(np.abs(A) * 2.0 ** -23, 2.0 ** (-25 - s))
+    worst = float((np.abs(out - A) / bound).max())
+    assert worst <= 1.0, worst
     ctx.release(a, b, c)
 
 
