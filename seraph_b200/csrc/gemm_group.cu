@@ -735,7 +735,7 @@ static int gg_operand(sb_ctx_t* c, GgOperand* ops, int* nops, const float* x, si
     }
     return (*nops)++;
 }
-// Parts of the operands that have none yet, in one launch for those whose producer left their maximum and three where some have none
+// Parts of the operands that have none yet: one launch, or three where some larger ones have no known maximum
 static void gg_prepare(sb_ctx_t* c, GgOperand* ops, int n) {
     TcMulti sp;
     tc_multi_begin(&sp);
@@ -755,7 +755,7 @@ static void gg_prepare(sb_ctx_t* c, GgOperand* ops, int n) {
     }
     if (any) sb_tick_end(c, tk, 0.0, bytes);
 }
-// Parts of registered tensors (weights) ahead of the products that read them: one pair of launches instead of one or two per tensor
+// Parts of registered tensors (weights) ahead of the products that read them: one to three launches instead of as many per tensor
 extern "C" void sb_parts_prepare(sb_ctx_t* c, const float* const* x, const size_t* n, int count) {
     GgOperand ops[TC_MULTI];
     for (int i0 = 0; i0 < count; ) {

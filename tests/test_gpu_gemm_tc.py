@@ -143,13 +143,15 @@ def test_scale_of_the_parts_is_checked_against_every_element(ctx, M, N, K, kind)
     ctx.release(a, b, c)
 
 
-@pytest.mark.parametrize("M,peak,unit", [(8, 1.0, 1.0), (8, 1.99, 1.0), (120, 1.0, 1.0), (4096, 1.0, 1.0), (4096, 1.99, 1.0), (4096, 2.6, 1.0), (4096, 3.9, 1.0),
-                                         (4096, 7.0, 1.0), (4096, 1.0, 2.0 ** -60), (4096, 3.9, 2.0 ** -60), (4096, 2.0 ** 80, 1.0)])
-def test_parts_keep_the_bits_of_the_true_scale(ctx, M, peak, unit):
+@pytest.mark.parametrize("M,K,peak,unit", [(8, 256, 1.0, 1.0), (120, 256, 1.99, 1.0), (512, 64, 1.99, 1.0), (520, 64, 1.0, 1.0), (512, 256, 3.9, 1.0), (513, 256, 1.99, 1.0),
+                                           (1024, 256, 2.0 ** 80, 1.0), (1024, 256, 1.99, 2.0 ** -60), (1025, 256, 1.0, 1.0), (4096, 256, 1.0, 1.0), (4096, 256, 1.99, 1.0),
+                                           (4096, 256, 2.6, 1.0), (4096, 256, 3.9, 1.0), (4096, 256, 7.0, 1.0), (4096, 256, 1.0, 2.0 ** -60), (4096, 256, 3.9, 2.0 ** -60),
+                                           (4096, 256, 2.0 ** 80, 1.0)])
+def test_parts_keep_the_bits_of_the_true_scale(ctx, M, K, peak, unit):
     """An operand times the identity is its two parts, added: under the scale of its true maximum, 2^s with max 2^s in [2^14, 2^15), each element is within
     2^-23 of itself (hi and lo part, 11 bits each, rounded to nearest) or within half of FP16's smallest step, 2^-25, whichever is larger.  No guess of
-    that scale may cost more.  The largest element lies where a sample of 16384 need not see it, among others below 1."""
-    K = 256
+    that scale may cost more.  The largest element lies where a sample of 16384 need not see it, among others below 1.  Up to 1024 x 256 elements one launch
+    of clusters of one to eight CTAs prepares an operand, 8192 float4s a CTA."""
     r = np.random.default_rng(M)
     A = (r.choice([-1, 1], (M, K)) * 2.0 ** r.uniform(-34, 0, (M, K))).astype(np.float32)
     A[M - 3, K - 5] = peak

@@ -297,6 +297,26 @@ def test_attention_on_chip_short_and_ragged(ctx, ss, Hq, Hkv, hd):
     ctx.release(bq, bk, bv, bdo, bs, bout, blse, bdq, bdk, bdv)
 
 
+@pytest.mark.parametrize("S,Hq,Hkv,hd", [(16, 8, 8, 64), (61, 16, 8, 128), (128, 16, 16, 128)])
+def test_attention_of_few_tokens_is_few_launches(ctx, S, Hq, Hkv, hd):
+    """Operands of up to 262144 elements are prepared in one launch a direction: the forward is two, the backward five (a pass for the maxima, one for the
+    parts and the kernels made it three and six once)."""
+    r = rng(S)
+    Q, K, V, dO = (f32(r.standard_normal((S, h * hd))) for h in (Hq, Hkv, Hkv, Hq))
+    b = [ctx.upload(x) for x in (Q, K, V, dO, np.array([0, S], np.uint32))] + [ctx.zeros(n) for n in (Q.size, S * Hq, Q.size, K.size, V.size)]
+    bq, bk, bv, bdo, bs, bout, blse, bdq, bdk, bdv = b
+    counts = []
+    for rep in range(2):                              # the first call may make tables
+        n0 = ctx.launches()
+        ctx.lib.cuda_train_batch_attention_packed(ctx.h, bq.b, bk.b, bv.b, bout.b, blse.b, bs.b, S, 1, Hq, Hkv, hd, S)
+        n1 = ctx.launches()
+        ctx.lib.cuda_train_batch_attention_backward_packed(ctx.h, bq.b, bk.b, bv.b, bout.b, blse.b, bdo.b, bdq.b, bdk.b, bdv.b, bs.b, S, 1, Hq, Hkv, hd, S)
+        ctx.check()
+        counts.append((n1 - n0, ctx.launches() - n1))
+    assert counts[1][0] <= 2 and counts[1][1] <= 5, counts
+    ctx.release(*b)
+
+
 @pytest.mark.parametrize("lens,Hq,Hkv,hd", [([383, 31, 129, 256, 97] * 9, 4, 2, 64), ([1100, 1023, 1024, 1025, 900, 1311, 1, 1500, 1217, 1088, 1152, 1153], 1, 1, 128),
                                              ([383, 700, 129, 256, 1, 640, 511] * 2, 8, 4, 128)])
 def test_attention_backward_dq_of_many_sequences(ctx, lens, Hq, Hkv, hd):
