@@ -718,24 +718,30 @@ static int af_launch_fwd(sb_ctx_t* c, const void* q1, const void* q2, const void
     const long blocks = (long)nqb * seqs.n * Hq;
     if (blocks > 0x7fffffffL) return 1;
     const size_t n_o = (size_t)T * qd;
-    void* oh; float* own; int fresh;
-    float* bound_o = (float*)sb_amax_take(c, O, n_o);
-    if (sb_parts_find(c, O, n_o, &oh, &own, &fresh)) sb_parts_set_amax(c, O, (float*)amax_v); else oh = nullptr;      // O of a training step is an operand
     CUtensorMap mO, mH1, mH2;
     {
         const cuuint64_t dims[2] = {(cuuint64_t)qd, (cuuint64_t)T}, pitch[1] = {(cuuint64_t)qd * 4};
         const cuuint32_t box[2] = {32u, 32u};
         if (!tc_encode(c, &mO, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, O, dims, pitch, box, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE)) return 1;
-        mH1 = mH2 = mO;
-        if (oh && (!af_make_map(c, &mH1, oh, T, qd, 32) || !af_make_map(c, &mH2, (__half*)oh + n_o, T, qd, 32))) return 1;
     }
     unsigned* counter = sb_item_counter(c);
     if (!counter) return 1;
-    const int sms = c->pub.gpu_sm_count > 0 ? c->pub.gpu_sm_count : 148;
-    sb_launch(kern, dim3((unsigned)(blocks < sms ? blocks : sms)), dim3(AF_THREADS), smem, (cudaStream_t)c->pub.stream, mQ1, mQ2, mK1, mK2, mV1, mV2, mO, mH1, mH2, seqs, O, lse, amax_q, amax_k, amax_v, Hq, Hq / Hkv, nqb, (int)blocks,
-        counter, 1.0f / sqrtf((float)HD), c->d_status, bound_o, (uint4*)oh, n_o, sb_parts_keep(c));
-    c->launches++;
-    return cudaGetLastError() == cudaSuccess ? 0 : 1;
+    // From here on the step's tables say that the kernel leaves the maximum and the parts of O (an operand of a training step).  Where it is not
+    // launched after all, they must not: the kernels that then form O write neither.
+    void* oh; float* own; int fresh;
+    float* bound_o = (float*)sb_amax_take(c, O, n_o);
+    if (sb_parts_find(c, O, n_o, &oh, &own, &fresh)) sb_parts_set_amax(c, O, (float*)amax_v); else oh = nullptr;
+    mH1 = mH2 = mO;
+    bool ok = !oh || (af_make_map(c, &mH1, oh, T, qd, 32) && af_make_map(c, &mH2, (__half*)oh + n_o, T, qd, 32));
+    if (ok) {
+        const int sms = c->pub.gpu_sm_count > 0 ? c->pub.gpu_sm_count : 148;
+        sb_launch(kern, dim3((unsigned)(blocks < sms ? blocks : sms)), dim3(AF_THREADS), smem, (cudaStream_t)c->pub.stream, mQ1, mQ2, mK1, mK2, mV1, mV2, mO, mH1, mH2, seqs, O, lse, amax_q, amax_k, amax_v, Hq, Hq / Hkv, nqb, (int)blocks,
+            counter, 1.0f / sqrtf((float)HD), c->d_status, bound_o, (uint4*)oh, n_o, sb_parts_keep(c));
+        c->launches++;
+        ok = cudaGetLastError() == cudaSuccess;
+    }
+    if (!ok) { sb_amax_forget(c, O); sb_parts_invalidate(c, O); }
+    return ok ? 0 : 1;
 }
 // q1/q2, k1/k2, v1/v2: the FP16 parts of Q [T, Hq*hd], K and V [T, Hkv*hd]; amax_*: the device words their scales derive from.
 // Returns 0 when the kernel was launched, 1 when this path does not take the call.
