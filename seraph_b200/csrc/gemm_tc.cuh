@@ -920,12 +920,14 @@ static __global__ void __launch_bounds__(256) tc_split_f16_kernel(const float* _
 #define TC_MULTI_CHUNK 1024
 #define TC_SAMPLE 4096                        // float4s looked at for the guess: 16 a thread
 #define TC_NO_SCALE 0x1p-100f                 // maxima below this are not scaled (sb_f16_shift)
+#define TC_SPANS 64                           // at most, of a tensor: tc_peaks_kernel
+#define TC_PEAKS_CHUNKS 1024                  // 16 MB of tensors: up to here a second read costs less than the launch that repeats a guess
 // h: hi parts, lo parts behind them; first: its first chunk; amax: the word the products read; guess: NULL when *amax is there already, else two words
 // of the tensor's own: the guess, and the true maximum where the guess does not do (else zero)
 struct TcMultiJob { const float* x; __half* h; float* amax; float* guess; uint32_t n4, first; };
-// unknown: tensors without a known maximum; guesses: those of them whose scale is a guess; longest: the largest n4
-struct TcMulti { int n, unknown, guesses; uint32_t chunks, longest; unsigned keep; TcMultiJob j[TC_MULTI]; };
-static inline void tc_multi_begin(TcMulti* m) { m->n = m->unknown = m->guesses = 0; m->chunks = m->longest = 0; }
+// unknown: tensors without a known maximum; guesses: those of them whose scale is a guess; longest: the largest n4; spans, peaks: see tc_peaks_kernel
+struct TcMulti { int n, unknown, guesses, spans; uint32_t chunks, longest; unsigned keep; float* peaks; TcMultiJob j[TC_MULTI]; };
+static inline void tc_multi_begin(TcMulti* m) { m->n = m->unknown = m->guesses = m->spans = 0; m->chunks = m->longest = 0; m->peaks = nullptr; }
 static inline void tc_multi_add(TcMulti* m, const float* x, size_t n, void* h, float* amax, float* guess) {
     TcMultiJob* j = &m->j[m->n++];
     j->x = x; j->h = (__half*)h; j->amax = amax; j->guess = guess; j->n4 = (uint32_t)(n / 4); j->first = m->chunks;
@@ -965,8 +967,35 @@ static __global__ void __launch_bounds__(256) tc_guess_kernel(const __grid_const
         j.guess[0] = mx; j.guess[1] = 0.f; *j.amax = mx;
     }
 }
-// A CTA takes an equal run of chunks, and walks it backwards: what a producer wrote last is still in L2.
-template <bool REDO>
+// The largest element of each of `spans` equal spans of a tensor, for preparations whose second read comes from L2: two launches and no guess.  Isolated
+// attention, one call alone, backward of 512 tokens, 8 heads of 64: 54.4 us, 57 with the guess and its repeat; 256 tokens, 16 heads of 128: 52.0 and 53.9.
+static __global__ void __launch_bounds__(256) tc_peaks_kernel(const __grid_constant__ TcMulti m) {
+    sb_pdl_enter();
+    __shared__ float red[8];
+    const TcMultiJob& j = m.j[blockIdx.y];
+    if (!j.guess) return;
+    const float4* x = (const float4*)j.x;
+    const uint32_t span = (j.n4 + m.spans - 1) / m.spans, end = min(j.n4, (blockIdx.x + 1) * span);
+    float mx = 0.f;
+    for (uint32_t i = blockIdx.x * span + threadIdx.x; i < end; i += 8 * 256) {
+        float4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = i + u * 256 < end ? __ldg(x + i + u * 256) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 8; u++) mx = sb_amax4(mx, v[u]);
+    }
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[w]);
+        m.peaks[blockIdx.y * m.spans + blockIdx.x] = mx;
+    }
+}
+// A CTA takes an equal run of chunks, and walks it backwards: what a producer wrote last is still in L2.  The scale comes from the tensor's word or
+// guess (TC_FIRST), from the word that TC_FIRST left where its guess did not do (TC_REDO), or from the peaks of its spans (TC_PEAKS).
+enum { TC_FIRST, TC_REDO, TC_PEAKS };
+template <int MODE>
 static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid_constant__ TcMulti m) {
     sb_pdl_enter();
     const uint32_t per = (m.chunks + gridDim.x - 1) / gridDim.x;
@@ -977,11 +1006,15 @@ static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid
         const TcMultiJob& j = m.j[jb];
         const uint32_t stop = max(begin, j.first);
         float top;                            // the scale's word
-        if (REDO) {
-            top = j.guess ? sb_word(j.guess + 1) : 0.f;
-            if (top == 0.f) { ck = stop; continue; }
-            if (stop == j.first && threadIdx.x == 0) *j.amax = top;        // nobody reads it in this launch
-        } else top = sb_word(j.guess ? j.guess : j.amax);
+        if (MODE == TC_FIRST || !j.guess) top = sb_word(j.guess ? j.guess : j.amax);
+        else if (MODE == TC_REDO) top = sb_word(j.guess + 1);
+        else {
+            top = 0.f;
+            for (int i = threadIdx.x & 31; i < m.spans; i += 32) top = fmaxf(top, sb_word(m.peaks + jb * m.spans + i));
+            for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        }
+        if (MODE == TC_REDO && (!j.guess || top == 0.f)) { ck = stop; continue; }
+        if (MODE != TC_FIRST && j.guess && stop == j.first && threadIdx.x == 0) *j.amax = top;      // nobody reads it in this launch
         const float4* x = (const float4*)j.x;
         uint2* h1 = (uint2*)j.h; uint2* h2 = h1 + j.n4;
         const float sc = tc_pow2(tc_f16_shift(top));
@@ -995,13 +1028,13 @@ static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid
 #pragma unroll
             for (int u = 0; u < TC_MULTI_CHUNK / 256; u++) if (base + u * 256 < j.n4) {
                 uint2 a, b;
-                if (!REDO) mx = sb_amax4(mx, v[u]);
+                if (MODE == TC_FIRST) mx = sb_amax4(mx, v[u]);
                 sb_split2(v[u].x * sc, v[u].y * sc, a.x, b.x, m.keep); sb_split2(v[u].z * sc, v[u].w * sc, a.y, b.y, m.keep);
                 h1[base + u * 256] = a; h2[base + u * 256] = b;
             }
         }
         // beyond FP16's range; or a sample of (nearly) nothing but zeros, which is not scaled, beside elements that would be
-        if (!REDO && j.guess && (mx * sc > 65504.f || (top < TC_NO_SCALE && mx >= TC_NO_SCALE))) atomicMax((unsigned*)(j.guess + 1), __float_as_uint(mx));
+        if (MODE == TC_FIRST && j.guess && (mx * sc > 65504.f || (top < TC_NO_SCALE && mx >= TC_NO_SCALE))) atomicMax((unsigned*)(j.guess + 1), __float_as_uint(mx));
     }
 }
 // Small tensors, each read once by a cluster that holds it in registers: the maximum, exchanged through the cluster's shared memory, and the parts in one
@@ -1080,9 +1113,20 @@ static inline void tc_multi_split(sb_ctx_t* c, TcMulti& m) {
     cudaStream_t st = (cudaStream_t)c->pub.stream;
     m.keep = sb_parts_keep(c);
     if (m.unknown && tc_multi_small(c, m)) return;
+    if (m.guesses && m.chunks <= TC_PEAKS_CHUNKS) {
+        if (!c->d_peaks && cudaMalloc((void**)&c->d_peaks, TC_SPANS * TC_MULTI * sizeof(float)) != cudaSuccess) { cudaGetLastError(); c->d_peaks = NULL; }      // then by the guess
+        m.peaks = c->d_peaks;
+        m.spans = max(1, min(TC_SPANS, 592 / m.n));
+    }
+    if (m.peaks) {
+        sb_launch(tc_peaks_kernel, dim3((unsigned)m.spans, (unsigned)m.n), dim3(256), 0, st, m);
+        sb_launch(tc_split_multi_kernel<TC_PEAKS>, dim3(tc_multi_grid(c, m)), dim3(256), 0, st, m);
+        c->launches += 2;
+        return;
+    }
     if (m.unknown) sb_launch(tc_guess_kernel, dim3((unsigned)m.n), dim3(256), 0, st, m);
-    sb_launch(tc_split_multi_kernel<false>, dim3(tc_multi_grid(c, m)), dim3(256), 0, st, m);
-    if (m.guesses) sb_launch(tc_split_multi_kernel<true>, dim3(tc_multi_grid(c, m)), dim3(256), 0, st, m);
+    sb_launch(tc_split_multi_kernel<TC_FIRST>, dim3(tc_multi_grid(c, m)), dim3(256), 0, st, m);
+    if (m.guesses) sb_launch(tc_split_multi_kernel<TC_REDO>, dim3(tc_multi_grid(c, m)), dim3(256), 0, st, m);
     c->launches += 1 + (m.unknown != 0) + (m.guesses != 0);
 }
 

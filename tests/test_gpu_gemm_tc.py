@@ -119,7 +119,7 @@ def test_single_pass_mode_keeps_small_products_accurate(ctx, M, N, K, single, tA
 
 
 @pytest.mark.parametrize("kind", ["normal", "outlier", "one element", "zeros", "inf", "nan"])
-@pytest.mark.parametrize("M,N,K", [(512, 256, 1024), (64, 128, 256), (1000, 264, 136)])
+@pytest.mark.parametrize("M,N,K", [(512, 256, 1024), (64, 128, 256), (1000, 264, 136), (4200, 264, 1024)])
 def test_scale_of_the_parts_is_checked_against_every_element(ctx, M, N, K, kind):
     """The scale of an operand's FP16 parts is guessed from 16384 of its elements; one that FP16 cannot hold under it (an element that few samples
     hit, the only one that is not zero) must give the scale of the true maximum, and not the overflow of the guessed one."""
@@ -144,14 +144,14 @@ def test_scale_of_the_parts_is_checked_against_every_element(ctx, M, N, K, kind)
 
 
 @pytest.mark.parametrize("M,K,peak,unit", [(8, 256, 1.0, 1.0), (120, 256, 1.99, 1.0), (512, 64, 1.99, 1.0), (520, 64, 1.0, 1.0), (512, 256, 3.9, 1.0), (513, 256, 1.99, 1.0),
-                                           (1024, 256, 2.0 ** 80, 1.0), (1024, 256, 1.99, 2.0 ** -60), (1025, 256, 1.0, 1.0), (4096, 256, 1.0, 1.0), (4096, 256, 1.99, 1.0),
-                                           (4096, 256, 2.6, 1.0), (4096, 256, 3.9, 1.0), (4096, 256, 7.0, 1.0), (4096, 256, 1.0, 2.0 ** -60), (4096, 256, 3.9, 2.0 ** -60),
-                                           (4096, 256, 2.0 ** 80, 1.0)])
+                                           (1024, 256, 2.0 ** 80, 1.0), (1024, 256, 1.99, 2.0 ** -60), (1025, 256, 1.0, 1.0), (4096, 256, 3.9, 1.0), (4097, 256, 1.99, 2.0 ** -60),
+                                           (4096, 256, 2.0 ** 80, 1.0)] +
+                         [(4200, 1024, p, u) for p in (1.0, 1.99, 2.6, 3.9, 7.0) for u in (1.0, 2.0 ** -60)] + [(4200, 1024, 2.0 ** 80, 1.0)])
 def test_parts_keep_the_bits_of_the_true_scale(ctx, M, K, peak, unit):
     """An operand times the identity is its two parts, added: under the scale of its true maximum, 2^s with max 2^s in [2^14, 2^15), each element is within
     2^-23 of itself (hi and lo part, 11 bits each, rounded to nearest) or within half of FP16's smallest step, 2^-25, whichever is larger.  No guess of
     that scale may cost more.  The largest element lies where a sample of 16384 need not see it, among others below 1.  Up to 1024 x 256 elements one launch
-    of clusters of one to eight CTAs prepares an operand, 8192 float4s a CTA."""
+    of clusters of one to eight CTAs prepares an operand, 8192 float4s a CTA; up to 16 MB the maximum is found first; beyond that it is guessed."""
     r = np.random.default_rng(M)
     A = (r.choice([-1, 1], (M, K)) * 2.0 ** r.uniform(-34, 0, (M, K))).astype(np.float32)
     A[M - 3, K - 5] = peak
