@@ -117,7 +117,8 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
         // ---------------- tiles and TMA loads ----------------
         if (elect_one()) {
             const int per_i = seqs.n * Hq;
-            int tile = *(volatile int*)status == 0 ? (int)blockIdx.x : tiles;      // an earlier CTA gave up: do not queue behind its cause
+            const int gave_up = *(volatile int*)status;        // an earlier CTA did: do not queue behind its cause (on its way together with the boundaries)
+            int tile = (int)blockIdx.x;
             uint32_t gk = 0;                                   // blocks so far
             for (int n = 0; ok; n++) {
                 // tiles with the most keys first, the query heads of one K/V head side by side; some have no rows
@@ -128,8 +129,9 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
                     const int rem = tile % per_i, b = rem / Hq;
                     t.qb = nqb_max - 1 - tile / per_i; t.h = rem % Hq;
                     t.t0 = (int)seqs.start[b]; t.S = (int)seqs.start[b + 1] - t.t0;
-                    if (t.qb * AF_BQ < t.S) break;
+                    if (t.qb * AF_BQ < t.S || gave_up) break;
                 }
+                if (gave_up) t.qb = -1;
                 ok = mbar_wait(&tile_empty[n & 1], ((n >> 1) & 1) ^ 1);
                 if (!ok) break;
                 tile_s[n & 1] = t;
@@ -705,18 +707,11 @@ static int af_launch_fwd(sb_ctx_t* c, const void* q1, const void* q2, const void
             fa.numRegs * AF_THREADS < 128 * (AF_REGS_LIGHT + 2 * AF_REGS_SOFTMAX + AF_REGS_O)) { cudaGetLastError(); return 1; }      // (setmaxnreg.inc would wait for good)
         attr_done = true;
     }
-    int Smax = 0;
-    for (int b = 0; b < c->h_seq_n; b++) Smax = max(Smax, c->h_seq[b + 1] - c->h_seq[b]);
-    if (Smax <= 0) return 1;
-    const AfSeqTab seqs = {c->h_seq_n, c->attn_seq_starts};
-    const int nqb = (Smax + AF_BQ - 1) / AF_BQ;
     const int qd = Hq * HD, kvd = Hkv * HD;
     CUtensorMap mQ1, mQ2, mK1, mK2, mV1, mV2;
     if (!af_make_map(c, &mQ1, q1, T, qd, AF_BQ) || !af_make_map(c, &mQ2, q2, T, qd, AF_BQ) ||
         !af_make_map(c, &mK1, k1, T, kvd, AF_BKV) || !af_make_map(c, &mK2, k2, T, kvd, AF_BKV) ||
         !af_make_map(c, &mV1, v1, T, kvd, AF_BKV) || !af_make_map(c, &mV2, v2, T, kvd, AF_BKV)) return 1;
-    const long blocks = (long)nqb * seqs.n * Hq;
-    if (blocks > 0x7fffffffL) return 1;
     const size_t n_o = (size_t)T * qd;
     CUtensorMap mO, mH1, mH2;
     {
@@ -726,6 +721,15 @@ static int af_launch_fwd(sb_ctx_t* c, const void* q1, const void* q2, const void
     }
     unsigned* counter = sb_item_counter(c);
     if (!counter) return 1;
+    sb_resolve_host_seq(c);                                  // only now: a single call's boundaries are on their way to the host while the maps are made
+    if (c->h_seq_n <= 0 || !c->h_seq || c->h_seq[c->h_seq_n] != T) return 1;
+    int Smax = 0;
+    for (int b = 0; b < c->h_seq_n; b++) Smax = max(Smax, c->h_seq[b + 1] - c->h_seq[b]);
+    if (Smax <= 0) return 1;
+    const AfSeqTab seqs = {c->h_seq_n, c->attn_seq_starts};
+    const int nqb = (Smax + AF_BQ - 1) / AF_BQ;
+    const long blocks = (long)nqb * seqs.n * Hq;
+    if (blocks > 0x7fffffffL) return 1;
     // From here on the step's tables say that the kernel leaves the maximum and the parts of O (an operand of a training step).  Where it is not
     // launched after all, they must not: the kernels that then form O write neither.
     void* oh; float* own; int fresh;
@@ -748,7 +752,7 @@ static int af_launch_fwd(sb_ctx_t* c, const void* q1, const void* q2, const void
 extern "C" int sb_attention_fused_forward(sb_ctx_t* c, const void* q1, const void* q2, const void* k1, const void* k2,
                                           const void* v1, const void* v2, const float* amax_q, const float* amax_k, const float* amax_v,
                                           float* O, float* lse, int T, int Hq, int Hkv, int hd) {
-    if (c->h_seq_n <= 0 || !c->attn_seq_starts || Hq % Hkv || !tc_aligned16(O) || !tc_load_encode()) return 1;
+    if (!c->attn_seq_starts || Hq % Hkv || !tc_aligned16(O) || !tc_load_encode()) return 1;
     if (hd == 128) return af_launch_fwd<128>(c, q1, q2, k1, k2, v1, v2, amax_q, amax_k, amax_v, O, lse, T, Hq, Hkv);
     if (hd == 64) return af_launch_fwd<64>(c, q1, q2, k1, k2, v1, v2, amax_q, amax_k, amax_v, O, lse, T, Hq, Hkv);
     return 1;

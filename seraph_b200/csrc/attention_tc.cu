@@ -458,10 +458,9 @@ static int at_forward_one_kernel(sb_ctx_t* c, const float* Q, const float* K, co
     const AtNeed need[3] = {{Q, n_q, hb, consts + 8, consts + 16}, {K, n_kv, hb + 2 * n_q, consts + 9, consts + 18}, {V, n_kv, hb + 2 * n_q + 2 * n_kv, consts + 10, consts + 20}};
     AtParts p[3];
     at_make_parts_multi(c, need, 3, p);
-    if (!at_have_seq(c, T)) { sb_tick_end(c, tk, 0.0, 0.0); return 1; }
-    double fl = 0;
-    for (int b = 0; b < c->h_seq_n; b++) { const double S = c->h_seq[b + 1] - c->h_seq[b]; fl += 2.0 * Hq * S * S * hd; }
     const int rc = sb_attention_fused_forward(c, p[0].h1, p[0].h2, p[1].h1, p[1].h2, p[2].h1, p[2].h2, p[0].amax, p[1].amax, p[2].amax, O, lse, T, Hq, Hkv, hd);
+    double fl = 0;
+    for (int b = 0; rc == 0 && b < c->h_seq_n; b++) { const double S = c->h_seq[b + 1] - c->h_seq[b]; fl += 2.0 * Hq * S * S * hd; }
     sb_tick_end(c, tk, fl, 0.0);
     return rc;
 }
