@@ -191,18 +191,24 @@ gg_kernel(const __grid_constant__ GgParams p) {
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     bool ok = true;
-    // the n-th item of this CTA's roles: the first is the pair's number, the others are waited for, read, and their slot handed back; false after the last
-    auto next_item = [&](int n, bool arrive, int rk, GgWork& w) -> bool {
+    // the n-th item of this CTA's roles: the first is the pair's number, the others are waited for, read, and their slot handed back; false after the last.
+    // The arrival that hands a slot back is relaxed; it follows the reads because it depends on the words they brought.  A role that is a warp
+    // (`whole`) votes on them, so that its one arrival depends on every lane's.
+    auto next_item = [&](int n, bool whole, int rk, GgWork& w) -> bool {
         GgItem it;
         if (n == 0) gg_decode<BATCH>(p, (int)(blockIdx.x >> 1), it);
         else {
             const int s = (n - 1) % GG_RING;
-            if (!gg_wait_cluster(&item_full[s], ((n - 1) / GG_RING) & 1)) { ok = false; return false; }
-            const uint32_t a = smem_u32(&item_slot[s]);
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(it.prob), "=r"(it.mt), "=r"(it.nt), "=r"(it.kb0) : "r"(a) : "memory");
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(it.kb1), "=r"(it.slot), "=r"(it.split), "=r"(it.pad) : "r"(a + 16) : "memory");
-            __syncwarp(__activemask());
-            if (arrive && it.prob >= -1 && it.pad == 0) gg_arrive_relaxed(mapa_u32(smem_u32(&item_empty[s]), 0));      // (always so: the arrival waits for the words)
+            it.prob = -2; it.pad = 0;             // the wait ran out
+            if (gg_wait_cluster(&item_full[s], ((n - 1) / GG_RING) & 1)) {
+                const uint32_t a = smem_u32(&item_slot[s]);
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(it.prob), "=r"(it.mt), "=r"(it.nt), "=r"(it.kb0) : "r"(a) : "memory");
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(it.kb1), "=r"(it.slot), "=r"(it.split), "=r"(it.pad) : "r"(a + 16) : "memory");
+            }
+            bool read = it.prob >= -1 && it.pad == 0;      // so whenever the words have come
+            if (whole) read = __all_sync(0xffffffffu, read);
+            if (!read) { ok = false; return false; }
+            if (!whole || lane == 0) gg_arrive_relaxed(mapa_u32(smem_u32(&item_empty[s]), 0));
             if (it.prob < 0) return false;
         }
         const int bn = p.prob[it.prob].bn;
@@ -224,7 +230,7 @@ gg_kernel(const __grid_constant__ GgParams p) {
                 uint32_t par = 1;
                 for (int n = 0; ok; n++) {
                     GgWork w;
-                    if (!next_item(n, true, (int)rank, w)) break;
+                    if (!next_item(n, false, (int)rank, w)) break;
                     if (n == 0) sb_pdl_enter();
                     const GgProb& pr = p.prob[w.prob];
                     int off = 0, left = w.kb1 - w.kb0;
@@ -270,7 +276,7 @@ gg_kernel(const __grid_constant__ GgParams p) {
                 uint32_t git = 0, gch = 0;
                 for (int n = 0; ok; n++) {
                     GgWork w;
-                    if (!next_item(n, true, 0, w)) break;
+                    if (!next_item(n, false, 0, w)) break;
                     const GgProb& pr = p.prob[w.prob];
                     int off = 0;
                     for (int sg = pr.seg0; sg < pr.seg0 + pr.nseg && ok; sg++) {
@@ -361,7 +367,7 @@ gg_kernel(const __grid_constant__ GgParams p) {
         __syncwarp();
         for (int n = 0; ok; n++) {
             GgWork w;
-            if (!next_item(n, lane == 0, (int)rank, w)) break;
+            if (!next_item(n, true, (int)rank, w)) break;
             const GgProb& pr = p.prob[w.prob];
             const int groups = pr.bn / 64, col0 = half * groups * 32;      // 32 columns at a time, half of the tile's per warp
             float accr[BN / 2];
