@@ -238,22 +238,24 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
     } else if (warp >= 4 && warp < 12) {
         // ---------------- softmax: half a query row (32 of the block's keys) per thread ----------------
         // The two warps of a lane quarter meet at a named barrier in every block, once before they leave, and learn there whether the other one's waits
-        // ran out: both meet the same number of times, whichever of them gives up.
+        // ran out: both meet the same number of times, whichever of them gives up.  A warp that gives up leaves the number of the meeting it does so at: the other
+        // one may look only after that warp has gone on to the next meeting, and must not leave before it.
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(AF_REGS_SOFTMAX));
         const int q = warp & 3, half = (warp - 4) >> 2, r = q * 32 + lane;
         const uint32_t lanes = tmem_base + ((uint32_t)(q * 32) << 16);
         const float cs = tc_pow2(-tc_f16_shift(sb_word(amax_q))) * tc_pow2(-tc_f16_shift(sb_word(amax_k))) * (scale * 1.4426950408889634f);
-        auto meet = [&]() {
-            if (!ok && lane == 0) bad[q * 2 + half] = 1;
+        auto meet = [&](uint32_t id) {                         // id: as many meetings before this one, the same in both warps
+            if (!ok && lane == 0) bad[q * 2 + half] = (int)id + 1;
             __syncwarp();
             asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
-            if (bad[q * 2 + (half ^ 1)]) ok = false;
+            const int other = bad[q * 2 + (half ^ 1)];
+            if (other != 0 && other <= (int)id + 1) ok = false;
         };
         uint32_t gk = 0, gh = 0;                               // blocks so far, slots of half_s used so far
         for (int n = 0;; n++) {
             AfTile t;
             int nkv;
-            if (!next_tile(n, lane == 0, t, nkv)) { meet(); break; }
+            if (!next_tile(n, lane == 0, t, nkv)) { meet(gh); break; }
             const int qi = t.qb * AF_BQ + r;                   // position of this row inside the sequence
             float m = -INFINITY, l = 0.f;
             // This row's parts of Q from shared memory (128-byte-swizzled tiles) into tensor memory, where an instruction of 64 columns reads them without
@@ -305,7 +307,7 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
                 const float mine = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * cs;      // cs > 0
                 ok = ok && mbar_wait(&h_empty[hi & 1], ((hi >> 1) & 1) ^ 1);
                 half_s[hs + half * 128 + r] = mine;
-                meet();
+                meet(hi);
                 if (!ok) break;
                 if (lane == 0) af_arrive(&h_full[hi & 1]);
                 const float m_new = fmaxf(m, fmaxf(mine, half_s[hs + (half ^ 1) * 128 + r]));      // finite from block 0 on: key 0 counts for every row
@@ -339,7 +341,7 @@ at_fused_fwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
             const uint32_t hi = gh + (uint32_t)nkv, hs = (hi & 1) * 256;
             ok = ok && mbar_wait(&h_empty[hi & 1], ((hi >> 1) & 1) ^ 1);
             if (half) half_s[hs + 128 + r] = l;
-            meet();
+            meet(hi);
             if (!ok) break;
             if (!half) {
                 l += half_s[hs + 128 + r];
