@@ -143,7 +143,8 @@ at_dkv_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_constant
     auto take = [&]() -> bool {                        // false: no keys for this CTA
         sb_pdl_enter();
         t0 = (int)seqs.start[b]; S = (int)seqs.start[b + 1] - t0;
-        return kb < nkb && k0 < S && *(volatile int*)status == 0;
+        const bool gave_up = __syncthreads_or(*(volatile int*)status != 0);      // an earlier CTA did (it may do so while this one reads: all threads decide alike)
+        return kb < nkb && k0 < S && !gave_up;
     };
     const bool first = gridDim.x > AF_ONE_WAVE;
     if (first && !take()) return;
@@ -618,7 +619,8 @@ at_dq_bwd_kernel(const __grid_constant__ CUtensorMap mS1, const __grid_constant_
         sb_pdl_enter();
         t0 = (int)seqs.start[b]; S = (int)seqs.start[b + 1] - t0;
         nkv = min((S + 63) / 64, 2 * qb + 2);
-        return qb * 128 < S && *(volatile int*)status == 0;
+        const bool gave_up = __syncthreads_or(*(volatile int*)status != 0);      // as above
+        return qb * 128 < S && !gave_up;
     };
     const bool first = gridDim.x > AF_ONE_WAVE;
     if (first && !take()) return;

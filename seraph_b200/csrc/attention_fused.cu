@@ -510,7 +510,7 @@ at_score_bwd_kernel(const __grid_constant__ CUtensorMap mQ1, const __grid_consta
     const int hb = nb > 0 ? hi : (b * g + h % g) * (Hq / g) + h / g;
     const int t0 = seqs.start[b], S = seqs.start[b + 1] - t0;
     if (qb * AF_BQ >= S) return;
-    if (*(volatile int*)status != 0) return;
+    if (__syncthreads_or(*(volatile int*)status != 0)) return;            // all threads or none, also while another CTA sets it
     const int nkv = min((S + AF_BKV - 1) / AF_BKV, 2 * qb + 2);           // key blocks that hold scores
     const int nz = min(Sp / AF_BKV, 4 * (qb / 2 + 1));                    // key blocks that are written
     const int kvh = h / g;

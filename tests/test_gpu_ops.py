@@ -297,6 +297,36 @@ def test_attention_on_chip_short_and_ragged(ctx, ss, Hq, Hkv, hd):
     ctx.release(bq, bk, bv, bdo, bs, bout, blse, bdq, bdk, bdv)
 
 
+@pytest.mark.parametrize("lens,Hq,Hkv,hd", [([200], 4, 2, 64), ([200], 4, 2, 128), ([130] * 48, 8, 8, 64), ([130] * 48, 8, 8, 128)])
+def test_attention_after_a_wait_that_ran_out(ctx, lens, Hq, Hkv, hd):
+    """While the status word says that a wait ran out, the kernels that keep scores on chip leave at once, whole CTAs of them, before and after they have taken
+    tensor memory (one wave of CTAs sets up first), and the context stays usable: the same calls are right once the status has been read."""
+    ss = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint32)
+    T, B, longest = int(ss[-1]), len(lens), max(lens)
+    r = rng(T + hd)
+    Q, K, V, dO = (f32(r.standard_normal((T, h * hd))) for h in (Hq, Hkv, Hkv, Hq))
+    out_ref, lse_ref, dQ_ref, dK_ref, dV_ref = np.empty_like(Q), np.empty((T, Hq), np.float32), np.empty_like(Q), np.zeros_like(K), np.zeros_like(V)
+    O.lib().ref_attention(Q, K, V, out_ref, lse_ref, ss, T, B, Hq, Hkv, hd)
+    O.lib().ref_attention_backward(Q, K, V, dO, dQ_ref, dK_ref, dV_ref, ss, T, B, Hq, Hkv, hd)
+    bq, bk, bv, bdo, bs = ctx.upload(Q), ctx.upload(K), ctx.upload(V), ctx.upload(dO), ctx.upload(ss)
+    bout, blse, bdq, bdk, bdv = ctx.zeros(Q.size), ctx.zeros(T * Hq), ctx.zeros(Q.size), ctx.zeros(K.size), ctx.zeros(V.size)
+    for ran_out in (1, 0):
+        for flash in (1, 2) if hd == 128 else (1,):
+            if ran_out:
+                assert ctx.lib.seraph_b200_selftest_bounded_wait(ctx.h, 10_000, None) == 0
+            ctx.set_attn_flash(flash)
+            for x in (bdk, bdv):
+                ctx.lib.cuda_train_fill_buffer(ctx.h, x.b, 0, x.nbytes)
+            ctx.lib.cuda_train_batch_attention_packed(ctx.h, bq.b, bk.b, bv.b, bout.b, blse.b, bs.b, T, B, Hq, Hkv, hd, longest)
+            ctx.lib.cuda_train_batch_attention_backward_packed(ctx.h, bq.b, bk.b, bv.b, bout.b, blse.b, bdo.b, bdq.b, bdk.b, bdv.b, bs.b, T, B, Hq, Hkv, hd, longest)
+            ctx.set_attn_flash(1)
+            assert ctx.status() == (5 if ran_out else 0)
+            if not ran_out:
+                for got, ref in zip((bout, blse, bdq, bdk, bdv), (out_ref, lse_ref, dQ_ref, dK_ref, dV_ref)):
+                    assert rel_l2(got.numpy(), ref) < TOL
+    ctx.release(bq, bk, bv, bdo, bs, bout, blse, bdq, bdk, bdv)
+
+
 @pytest.mark.parametrize("S,Hq,Hkv,hd", [(16, 8, 8, 64), (61, 16, 8, 128), (128, 16, 16, 128)])
 def test_attention_of_few_tokens_is_few_launches(ctx, S, Hq, Hkv, hd):
     """Operands of up to 262144 elements are prepared in one launch a direction: the forward is two, the backward five (a pass for the maxima, one for the
