@@ -31,10 +31,9 @@
 #include <type_traits>
 #include "gemm_tc.cuh"
 #include "attention_fused.cuh"
+#include "gemm_plan.h"
 
-#define GG_MAXP 10               // products per launch
 #define GG_MAXS 10               // segments per launch
-#define GG_MAXE (2 * GG_MAXP)    // runs of items: whole tiles, then pieces, of each product
 #define GG_RING 4                // items the slowest role may lag behind the scheduling warp
 #define GG_AHEAD 8               // k blocks left to load of an item when the next one is asked for: enough to hide the hand-over, not more, so
                                  // that items go to the pairs that really are free first
@@ -494,183 +493,10 @@ static __global__ void __launch_bounds__(256) gg_fixup_kernel(const __grid_const
     }
 }
 
-// --------------------------------------------------------------------------- the schedule of a group
-// Every product has a tile width and may be cut into pieces of its k range; the last tiles of a launch are cut when that shortens it.  The kernel comes in two
-// classes: tiles of 128, 192 and 256 columns (five stages, two accumulators), and of 64 and 128 (eight and four).  The widest tile costs least per
-// multiply-add; a narrower one pays where the wide tiles leave the last round mostly empty (2816 columns of 2048 rows are 96 tiles of 256 on 74
-// pairs, two rounds, or 128 of 192: two shorter ones) and where one product's long k would outlast all others (a weight gradient over 2048 tokens
-// beside an input gradient over 512 columns).  The cost of an item is its k blocks plus an epilogue that the next item's first two chunks hide
-// part of; a launch is the greedy schedule of its items on the CTA pairs.  The constants (microseconds per k block of 64, per epilogue, for the
-// fix-up launch) are measured.
-struct GgPlanRun { int prob, tile0, tiles, split; };
-struct GgPlan { int bn, nruns, w[GG_MAXP]; GgPlanRun run[GG_MAXE]; };
-struct GgPlanKey { int nprob, nt, G; int mnk[GG_MAXP][3]; };
-struct GgPlanEntry { GgPlanKey key; GgPlan plan; bool valid; };
-#define GG_PLANS 128
-#define GG_NARROWER 1.03f                     // a plan with narrower tiles has to win by more than the constants are worth
-
-struct GgWidth { int bn; float t_kb[2], t_epi; };      // t_kb: three passes, one pass
-static const GgWidth gg_wide[3] = {{256, {1.00f, 0.47f}, 4.3f}, {192, {0.82f, 0.43f}, 3.5f}, {128, {0.64f, 0.38f}, 2.6f}};
-static const GgWidth gg_narrow[2] = {{128, {0.52f, 0.31f}, 2.3f}, {64, {0.42f, 0.27f}, 2.0f}};
-// the fix-up launch, and for each column of 256 rows that is written for it and read: in L2, and beyond 16 MB (512 x 256 columns: 130 us)
-static const float gg_t_fix = 3.0f, gg_t_fix_col = 2.5e-4f, gg_t_fix_far = 8e-4f, gg_fix_near = 16384.f;
-
-struct GgSim { float t[64]; int c[64]; int n; };
-// `count` items of one cost, each to the pair that is free first
-static void gg_sim_add(GgSim* s, int count, float cost, int G) {
-    if (count > 4 * G) {                                         // whole rounds first
-        const int rounds = count / G - 2;
-        for (int i = 0; i < s->n; i++) s->t[i] += rounds * cost;
-        count -= rounds * G;
-    }
-    while (count > 0) {
-        int lo = 0;
-        for (int i = 1; i < s->n; i++) if (s->t[i] < s->t[lo]) lo = i;
-        const int a = count < s->c[lo] ? count : s->c[lo];
-        const float nt = s->t[lo] + cost;
-        count -= a; s->c[lo] -= a;
-        int hit = -1;
-        for (int i = 0; i < s->n; i++) if (s->t[i] == nt || (s->n >= 60 && s->t[i] > nt - 0.5f * cost && s->t[i] < nt + 0.5f * cost)) { hit = i; break; }
-        if (hit >= 0) s->c[hit] += a;
-        else if (s->c[lo] == 0) { s->t[lo] = nt; s->c[lo] = a; continue; }
-        else { s->t[s->n] = nt; s->c[s->n] = a; s->n++; }
-        if (s->c[lo] == 0) { s->n--; s->t[lo] = s->t[s->n]; s->c[lo] = s->c[s->n]; }
-    }
-}
-static int gg_tiles(const int* mnk, int bn) { return ((mnk[0] + 255) / 256) * ((mnk[1] + bn - 1) / bn); }
-// What a plan chooses for each product: its tiles' width (of the class's table) and the pieces every one of them is cut into.
-struct GgPick { unsigned char w[GG_MAXP], s[GG_MAXP]; };
-static bool gg_can_cut(int kb, int s) { const int per = (kb + s - 1) / s; return s == 1 || (per * (s - 1) < kb && per >= 2); }
-// The launch of these choices; tail: pieces of the tiles that its last round holds, taken from the shortest uncut products (1: they stay whole).
-// Returns its time and the runs, or -1 when there is no such plan or none below `limit` (0: no limit).
-static float gg_eval(const GgPlanKey* k, const GgWidth* tab, const GgPick* c, int tail, float limit, GgPlan* p) {
-    float cost[GG_MAXP];
-    int order[GG_MAXP], tiles[GG_MAXP], spl[GG_MAXP], cut[GG_MAXP], total = 0;
-    const int one = k->nt == 1;
-    for (int i = 0; i < k->nprob; i++) {
-        cost[i] = k->mnk[i][2] * tab[c->w[i]].t_kb[one] + tab[c->w[i]].t_epi;
-        int j = i;
-        for (; j > 0 && cost[order[j - 1]] < cost[i]; j--) order[j] = order[j - 1];
-        order[j] = i;
-        tiles[i] = gg_tiles(k->mnk[i], tab[c->w[i]].bn);
-        spl[i] = c->s[i];
-        if (!gg_can_cut(k->mnk[i][2], spl[i])) return -1.f;
-        cut[i] = spl[i] > 1 ? tiles[i] : 0;
-        total += tiles[i] * spl[i];
-    }
-    if (tail > 1) {
-        int left = total % k->G;
-        if (left == 0) return -1.f;
-        bool any = false;
-        for (int o = k->nprob - 1; o >= 0 && left > 0; o--) {
-            const int i = order[o];
-            if (spl[i] > 1) continue;
-            if (!gg_can_cut(k->mnk[i][2], tail)) return -1.f;
-            spl[i] = tail; cut[i] = tiles[i] < left ? tiles[i] : left; left -= cut[i]; any = true;
-        }
-        if (!any) return -1.f;
-    }
-    GgPlanRun pieces[GG_MAXP]; float pcost[GG_MAXP]; int np = 0;
-    GgSim sim;
-    sim.n = 1; sim.t[0] = 0.f; sim.c[0] = k->G;
-    p->nruns = 0;
-    for (int i = 0; i < k->nprob; i++) {
-        if (!cut[i]) continue;
-        const float pc = (k->mnk[i][2] + spl[i] - 1) / spl[i] * tab[c->w[i]].t_kb[one] + tab[c->w[i]].t_epi;
-        int j = np++;
-        for (; j > 0 && pcost[j - 1] < pc; j--) { pieces[j] = pieces[j - 1]; pcost[j] = pcost[j - 1]; }
-        pieces[j] = {i, tiles[i] - cut[i], cut[i], spl[i]}; pcost[j] = pc;
-    }
-    if (limit > 0.f) {                                           // the work spread evenly, or the longest item: no schedule is shorter
-        float work = 0.f, longest = np ? pcost[0] : 0.f;
-        for (int i = 0; i < k->nprob; i++) if (tiles[i] > cut[i]) { work += (tiles[i] - cut[i]) * cost[i]; if (cost[i] > longest) longest = cost[i]; }
-        for (int a = 0; a < np; a++) work += pieces[a].tiles * pieces[a].split * pcost[a];
-        if ((work > longest * k->G ? work / k->G : longest) + (np ? gg_t_fix : 0.f) >= limit) return -1.f;
-    }
-    // longest items first, whole or pieces
-    float slots = 0.f;
-    for (int o = 0, a = 0; o < k->nprob || a < np; ) {
-        if (a == np || (o < k->nprob && cost[order[o]] >= pcost[a])) {
-            const int i = order[o++];
-            if (tiles[i] == cut[i]) continue;
-            p->run[p->nruns++] = {i, 0, tiles[i] - cut[i], 1};
-            gg_sim_add(&sim, tiles[i] - cut[i], cost[i], k->G);
-        } else {
-            p->run[p->nruns++] = pieces[a];
-            gg_sim_add(&sim, pieces[a].tiles * pieces[a].split, pcost[a], k->G);
-            slots += (float)(pieces[a].tiles * pieces[a].split) * tab[c->w[pieces[a].prob]].bn;
-            a++;
-        }
-    }
-    float t = 0.f;
-    for (int i = 0; i < sim.n; i++) if (sim.t[i] > t) t = sim.t[i];
-    if (np) t = (t + gg_t_fix + slots * gg_t_fix_col + (slots > gg_fix_near ? (slots - gg_fix_near) * (gg_t_fix_far - gg_t_fix_col) : 0.f)) * 1.02f;
-    for (int i = 0; i < k->nprob; i++) p->w[i] = tab[c->w[i]].bn;
-    p->bn = tab[0].bn;
-    return t;
-}
-static void gg_make_plan(const GgPlanKey* k, GgPlan* best) {
-    // products of one shape share their choice
-    int kind_of[GG_MAXP], nk = 0;
-    for (int i = 0; i < k->nprob; i++) {
-        kind_of[i] = -1;
-        for (int j = 0; j < i && kind_of[i] < 0; j++) if (memcmp(k->mnk[i], k->mnk[j], sizeof k->mnk[i]) == 0) kind_of[i] = kind_of[j];
-        if (kind_of[i] < 0) kind_of[i] = nk++;
-    }
-    static const unsigned char pieces[6] = {1, 2, 3, 4, 6, 8}, tails[6] = {2, 3, 4, 5, 6, 8};
-    float best_t = 0.f;
-    best->nruns = 0;
-    GgPlan p;
-    for (int cls = 0; cls < 2; cls++) {
-        const GgWidth* tab = cls ? gg_narrow : gg_wide;
-        const int nw = cls ? 2 : 3;
-        int total = 0;
-        for (int i = 0; i < k->nprob; i++) total += gg_tiles(k->mnk[i], tab[0].bn);
-        const bool many = total > 6 * k->G;                      // many rounds: no empty last one to speak of, and no product that outlasts the rest
-        for (int base = 0; base < (many ? 1 : nw); base++) {
-            GgPick c;
-            memset(&c, 0, sizeof c);
-            for (int i = 0; i < k->nprob; i++) { c.w[i] = (unsigned char)base; c.s[i] = 1; }
-            const float off = cls || base ? GG_NARROWER : 1.f;
-            float t = gg_eval(k, tab, &c, 1, 0.f, &p) * off;
-            if (best->nruns == 0 || t < best_t) { *best = p; best_t = t; }
-            auto cut_tail = [&]() {
-                for (int q = 0; q < 6; q++) {
-                    const float tv = gg_eval(k, tab, &c, tails[q], best_t, &p) * off;
-                    if (tv > 0.f && tv < best_t) { *best = p; best_t = tv; }
-                }
-            };
-            cut_tail();
-            // one kind of product after the other to its best choice beside the others'
-            for (int sweep = 0; sweep < (many ? 0 : 2); sweep++) {
-                bool moved = false;
-                for (int kd = 0; kd < nk; kd++) {
-                    GgPick top = c;
-                    for (int w = 0; w < nw; w++)
-                        for (int q = 0; q < 6; q++) {
-                            GgPick v = c;
-                            for (int i = 0; i < k->nprob; i++) if (kind_of[i] == kd) { v.w[i] = (unsigned char)w; v.s[i] = pieces[q]; }
-                            if (memcmp(&v, &c, sizeof v) == 0) continue;
-                            const float tv = gg_eval(k, tab, &v, 1, t, &p) * (cls || w || base ? GG_NARROWER : 1.f);
-                            if (tv > 0.f && tv < t) { t = tv; top = v; moved = true; if (t < best_t) { *best = p; best_t = t; } }
-                        }
-                    c = top;
-                }
-                if (!moved) break;
-            }
-            if (!many) cut_tail();
-        }
-    }
-}
+// the schedule of a group (gemm_plan.h)
 static const GgPlan* gg_plan(sb_ctx_t* c, const GgPlanKey* key) {
-    if (!c->gg_plans) c->gg_plans = calloc(GG_PLANS + 1, sizeof(GgPlanEntry));
-    if (!c->gg_plans) return nullptr;
-    uint64_t h = 1469598103934665603ull;
-    const int* w = (const int*)key;
-    for (size_t i = 0; i < sizeof *key / sizeof(int); i++) { h ^= (uint64_t)(uint32_t)w[i]; h *= 0x9E3779B97F4A7C15ull; h ^= h >> 29; }
-    GgPlanEntry* e = (GgPlanEntry*)c->gg_plans + h % GG_PLANS;
-    if (!e->valid || memcmp(&e->key, key, sizeof *key) != 0) { gg_make_plan(key, &e->plan); e->key = *key; e->valid = true; }
-    return &e->plan;
+    if (!c->gg_plans) c->gg_plans = calloc(1, sizeof(GgPlanTable));
+    return c->gg_plans ? gg_plan_find((GgPlanTable*)c->gg_plans, key) : nullptr;
 }
 
 template <int BN, int NT, bool BATCH = false>
@@ -821,8 +647,8 @@ static bool gg_run(sb_ctx_t* c, const sb_gemm_job_t* jobs, int njobs, int nt) {
         of[j] = np - 1;
     }
     const int sms = c->pub.gpu_sm_count > 0 ? c->pub.gpu_sm_count : 148;
-    key.nprob = np; key.nt = nt; key.G = max(1, (sms - (c->gemm_reserve_sms < sms ? c->gemm_reserve_sms : 0)) / 2);
-    for (int i = 0; i < np; i++) { key.mnk[i][0] = p.prob[i].M; key.mnk[i][1] = p.prob[i].N; key.mnk[i][2] = p.prob[i].kb; }
+    key.nt = nt; key.G = max(1, (sms - (c->gemm_reserve_sms < sms ? c->gemm_reserve_sms : 0)) / 2);
+    for (int i = 0; i < np; i++) gg_key_add(&key, p.prob[i].M, p.prob[i].N, p.prob[i].kb);
     const GgPlan* plan = gg_plan(c, &key);
     if (!plan) return false;
     const int bn = plan->bn;
