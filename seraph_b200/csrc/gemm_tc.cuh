@@ -912,7 +912,7 @@ static __global__ void __launch_bounds__(256) tc_split_f16_kernel(const float* _
 // of 16384 scattered elements, which the true maximum is never below.  It brings the sample's largest to [2^14, 2^15), and FP16 holds 65504: room for elements
 // two to four times as large.  The pass that writes the parts compares every element with that, and a third launch makes the parts again, with the
 // scale of the true maximum, of a tensor that has a larger one; for all others it ends at once.  So an element keeps the bits that the scale of the
-// true maximum would give it, or one more, and the scale is a function of the tensor alone.
+// true maximum would give it, or one more.  The scale is a function of the tensor alone: preparations that find the maximum first (below) choose the same.
 // The word that goes with the parts tells their scale; it is no bound of a tensor whose scale was guessed.  Bytes bound it, 12 for each element: three tensors of
 // 8 x 2048 x 2048 floats take 139 us, 131 of them in the split at 6.1 TB/s (198 with a pass for the maximum before it); small tensors are launches:
 // the 57 weights of the 33M model (120 MB) take three, 50 us (twelve and 78 when maximum and split passes ran in batches that fit L2).
@@ -940,34 +940,48 @@ __device__ __forceinline__ int tc_multi_find(const TcMulti& m, uint32_t chunk) {
     while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (m.j[mid].first <= chunk) lo = mid; else hi = mid - 1; }
     return lo;
 }
-// a CTA per tensor; a tensor of up to TC_SAMPLE float4s is read whole, and its maximum is no guess
+// The sample of a tensor: TC_SAMPLE float4s, one line of eight from each of equal runs of lines at a place that does not repeat with the rows' length
+// (scattered float4s took 10 us for 57 tensors, lines 6); a tensor of up to that many is its own sample.  The largest element of this thread's share.
+template <int THREADS>
+__device__ __forceinline__ float tc_sample_share(const float4* x, uint32_t n4) {
+    const uint32_t lines = n4 >> 3, step = lines / (TC_SAMPLE >> 3);
+    float4 v[TC_SAMPLE / THREADS];
+#pragma unroll
+    for (int u = 0; u < TC_SAMPLE / THREADS; u++) {
+        const uint32_t i = threadIdx.x + u * THREADS;
+        const uint32_t l = i >> 3, at = step > 1 ? ((l * step + ((l * 2654435761u) >> 8) % step) << 3) + (i & 7) : i;
+        v[u] = at < n4 ? __ldg(x + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float mx = 0.f;
+#pragma unroll
+    for (int u = 0; u < TC_SAMPLE / THREADS; u++) mx = sb_amax4(mx, v[u]);
+    return mx;
+}
+template <int THREADS>
+__device__ __forceinline__ float tc_cta_max(float mx, float* red) {      // red: THREADS / 32 floats; all threads get it
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    mx = red[0];
+#pragma unroll
+    for (int w = 1; w < THREADS / 32; w++) mx = fmaxf(mx, red[w]);
+    return mx;
+}
+// Does FP16 hold `mx` under the scale that the sample's largest element gives?  (A sample of nearly nothing but zeros is not scaled.)
+__device__ __forceinline__ bool tc_sample_does(float sample, float mx) {
+    return mx * tc_pow2(tc_f16_shift(sample)) <= 65504.f && (sample >= TC_NO_SCALE || mx < TC_NO_SCALE);
+}
+// a CTA per tensor
 static __global__ void __launch_bounds__(256) tc_guess_kernel(const __grid_constant__ TcMulti m) {
     sb_pdl_enter();
     __shared__ float red[8];
     const TcMultiJob& j = m.j[blockIdx.x];
     if (!j.guess) return;
-    const float4* x = (const float4*)j.x;
-    const uint32_t lines = j.n4 >> 3, step = lines / (TC_SAMPLE >> 3);      // lines of 8 float4s (scattered float4s took 10 us for 57 tensors, lines 6)
-    float4 v[TC_SAMPLE / 256];
-#pragma unroll
-    for (int u = 0; u < TC_SAMPLE / 256; u++) {
-        const uint32_t i = threadIdx.x + u * 256;
-        // one line of each run of `step`, at a place that does not repeat with the rows' length
-        const uint32_t l = i >> 3, at = step > 1 ? ((l * step + ((l * 2654435761u) >> 8) % step) << 3) + (i & 7) : i;
-        v[u] = at < j.n4 ? __ldg(x + at) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    float mx = 0.f;
-#pragma unroll
-    for (int u = 0; u < TC_SAMPLE / 256; u++) mx = sb_amax4(mx, v[u]);
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[w]);
-        j.guess[0] = mx; j.guess[1] = 0.f; *j.amax = mx;
-    }
+    const float mx = tc_cta_max<256>(tc_sample_share<256>((const float4*)j.x, j.n4), red);
+    if (threadIdx.x == 0) { j.guess[0] = mx; j.guess[1] = 0.f; *j.amax = mx; }
 }
-// The largest element of each of `spans` equal spans of a tensor, for preparations whose second read comes from L2: two launches and no guess.  Isolated
+// The largest element of each of `spans` equal spans of a tensor, and of its sample, for preparations whose second read comes from L2: the next launch knows
+// what the scale is, and no third one has to repeat anything.  Isolated
 // attention, one call alone, backward of 512 tokens, 8 heads of 64: 54.4 us, 57 with the guess and its repeat; 256 tokens, 16 heads of 128: 52.0 and 53.9.
 static __global__ void __launch_bounds__(256) tc_peaks_kernel(const __grid_constant__ TcMulti m) {
     sb_pdl_enter();
@@ -975,25 +989,23 @@ static __global__ void __launch_bounds__(256) tc_peaks_kernel(const __grid_const
     const TcMultiJob& j = m.j[blockIdx.y];
     if (!j.guess) return;
     const float4* x = (const float4*)j.x;
-    const uint32_t span = (j.n4 + m.spans - 1) / m.spans, end = min(j.n4, (blockIdx.x + 1) * span);
     float mx = 0.f;
-    for (uint32_t i = blockIdx.x * span + threadIdx.x; i < end; i += 8 * 256) {
-        float4 v[8];
+    if (blockIdx.x == m.spans) mx = tc_sample_share<256>(x, j.n4);
+    else {
+        const uint32_t span = (j.n4 + m.spans - 1) / m.spans, end = min(j.n4, (blockIdx.x + 1) * span);
+        for (uint32_t i = blockIdx.x * span + threadIdx.x; i < end; i += 8 * 256) {
+            float4 v[8];
 #pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = i + u * 256 < end ? __ldg(x + i + u * 256) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int u = 0; u < 8; u++) v[u] = i + u * 256 < end ? __ldg(x + i + u * 256) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int u = 0; u < 8; u++) mx = sb_amax4(mx, v[u]);
+            for (int u = 0; u < 8; u++) mx = sb_amax4(mx, v[u]);
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; w++) mx = fmaxf(mx, red[w]);
-        m.peaks[blockIdx.y * m.spans + blockIdx.x] = mx;
-    }
+    mx = tc_cta_max<256>(mx, red);
+    if (threadIdx.x == 0) *(blockIdx.x == m.spans ? j.guess : m.peaks + blockIdx.y * m.spans + blockIdx.x) = mx;
 }
 // A CTA takes an equal run of chunks, and walks it backwards: what a producer wrote last is still in L2.  The scale comes from the tensor's word or
-// guess (TC_FIRST), from the word that TC_FIRST left where its guess did not do (TC_REDO), or from the peaks of its spans (TC_PEAKS).
+// guess (TC_FIRST), from the word that TC_FIRST left where its guess did not do (TC_REDO), or from the sample and the peaks of its spans (TC_PEAKS).
 enum { TC_FIRST, TC_REDO, TC_PEAKS };
 template <int MODE>
 static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid_constant__ TcMulti m) {
@@ -1012,6 +1024,8 @@ static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid
             top = 0.f;
             for (int i = threadIdx.x & 31; i < m.spans; i += 32) top = fmaxf(top, sb_word(m.peaks + jb * m.spans + i));
             for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            const float sample = sb_word(j.guess);
+            if (tc_sample_does(sample, top)) top = sample;
         }
         if (MODE == TC_REDO && (!j.guess || top == 0.f)) { ck = stop; continue; }
         if (MODE != TC_FIRST && j.guess && stop == j.first && threadIdx.x == 0) *j.amax = top;      // nobody reads it in this launch
@@ -1033,8 +1047,7 @@ static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid
                 h1[base + u * 256] = a; h2[base + u * 256] = b;
             }
         }
-        // beyond FP16's range; or a sample of (nearly) nothing but zeros, which is not scaled, beside elements that would be
-        if (MODE == TC_FIRST && j.guess && (mx * sc > 65504.f || (top < TC_NO_SCALE && mx >= TC_NO_SCALE))) atomicMax((unsigned*)(j.guess + 1), __float_as_uint(mx));
+        if (MODE == TC_FIRST && j.guess && !tc_sample_does(top, mx)) atomicMax((unsigned*)(j.guess + 1), __float_as_uint(mx));
     }
 }
 // Small tensors, each read once by a cluster that holds it in registers: the maximum, exchanged through the cluster's shared memory, and the parts in one
@@ -1042,10 +1055,13 @@ static __global__ void __launch_bounds__(256) tc_split_multi_kernel(const __grid
 // tokens, 16 heads of 128, 47.9 and 44.8.  The rule: every tensor fits the registers of eight CTAs, and all CTAs fit one wave.  Two float4s a
 // thread where that is enough (shorter code to fetch: 16 tokens, 16 heads of 128, cold, 5.3 us against 6.1 with sixteen), else sixteen.
 #define TC_SMALL_THREADS 512
+__device__ __forceinline__ float tc_peer_word(const float* p, uint32_t rank) {      // of another CTA of the cluster
+    float v; asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(mapa_u32(smem_u32(p), rank)) : "memory"); return v;
+}
 template <int U>                              // float4s a thread
 static __global__ void __launch_bounds__(TC_SMALL_THREADS) tc_small_kernel(const __grid_constant__ TcMulti m, int ctas) {
     sb_pdl_enter();
-    __shared__ float red[TC_SMALL_THREADS / 32], peak;
+    __shared__ float red[2][TC_SMALL_THREADS / 32], tops[2];      // tops: the largest element of this CTA's, and (the first CTA's) of the sample
     const TcMultiJob& j = m.j[blockIdx.x / ctas];
     const uint32_t base = blockIdx.x % ctas * (U * TC_SMALL_THREADS) + threadIdx.x;
     const float4* x = (const float4*)j.x;
@@ -1054,24 +1070,20 @@ static __global__ void __launch_bounds__(TC_SMALL_THREADS) tc_small_kernel(const
     for (int u = 0; u < U; u++) v[u] = base + u * TC_SMALL_THREADS < j.n4 ? __ldg(x + base + u * TC_SMALL_THREADS) : make_float4(0.f, 0.f, 0.f, 0.f);
     float top;
     if (j.guess) {
+        const bool sampled = j.n4 > TC_SAMPLE;
+        float sample = 0.f;
+        if (sampled && blockIdx.x % ctas == 0) sample = tc_cta_max<TC_SMALL_THREADS>(tc_sample_share<TC_SMALL_THREADS>(x, j.n4), red[1]);
         float mx = 0.f;
 #pragma unroll
         for (int u = 0; u < U; u++) mx = sb_amax4(mx, v[u]);
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-        __syncthreads();
-        top = red[0];
-#pragma unroll
-        for (int w = 1; w < TC_SMALL_THREADS / 32; w++) top = fmaxf(top, red[w]);
+        top = tc_cta_max<TC_SMALL_THREADS>(mx, red[0]);
         if (ctas > 1) {
-            if (threadIdx.x == 0) peak = top;
+            if (threadIdx.x == 0) { tops[0] = top; tops[1] = sample; }
             cluster_sync_all();
-            for (int r = 0; r < ctas; r++) {
-                float o;
-                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(o) : "r"(mapa_u32(smem_u32(&peak), (uint32_t)r)) : "memory");
-                top = fmaxf(top, o);
-            }
+            for (int r = 0; r < ctas; r++) top = fmaxf(top, tc_peer_word(&tops[0], (uint32_t)r));
+            sample = tc_peer_word(&tops[1], 0);
         }
+        if (sampled && tc_sample_does(sample, top)) top = sample;
         if (blockIdx.x % ctas == 0 && threadIdx.x == 0) *j.amax = top;
     } else top = sb_word(j.amax);
     const float sc = tc_pow2(tc_f16_shift(top));
@@ -1119,7 +1131,7 @@ static inline void tc_multi_split(sb_ctx_t* c, TcMulti& m) {
         m.spans = max(1, min(TC_SPANS, 592 / m.n));
     }
     if (m.peaks) {
-        sb_launch(tc_peaks_kernel, dim3((unsigned)m.spans, (unsigned)m.n), dim3(256), 0, st, m);
+        sb_launch(tc_peaks_kernel, dim3((unsigned)m.spans + 1, (unsigned)m.n), dim3(256), 0, st, m);
         sb_launch(tc_split_multi_kernel<TC_PEAKS>, dim3(tc_multi_grid(c, m)), dim3(256), 0, st, m);
         c->launches += 2;
         return;

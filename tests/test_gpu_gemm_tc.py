@@ -168,6 +168,25 @@ def test_parts_keep_the_bits_of_the_true_scale(ctx, M, K, peak, unit):
     ctx.release(a, b, c)
 
 
+@pytest.mark.parametrize("peak", [1.0, 1.99, 3.9, 7.0])
+@pytest.mark.parametrize("M", [120, 520, 1032])
+def test_parts_do_not_depend_on_the_way_they_are_made(ctx, M, peak):
+    """The same operand beside a small one (one launch, or the maximum first: from 1025 rows on) and beside one of 18 MB (the scale from a sample): the same parts."""
+    K, N = 256, 17408
+    r = np.random.default_rng(M)
+    A = (r.choice([-1, 1], (M, K)) * 2.0 ** r.uniform(-34, 0, (M, K))).astype(np.float32)
+    A[M - 3, K - 5] = peak
+    E = np.zeros((N, K), np.float32)
+    E[:K] = np.eye(K)
+    a, e, c, cl = ctx.upload(A), ctx.upload(E), ctx.zeros(M * K), ctx.zeros(M * N)
+    ctx.lib.cuda_train_matmul_transpose(ctx.h, a.b, e.b, c.b, M, K, K, 0, 1, 0)
+    ctx.lib.cuda_train_matmul_transpose(ctx.h, a.b, e.b, cl.b, M, N, K, 0, 1, 0)
+    out, large = c.numpy(shape=(M, K)), cl.numpy(shape=(M, N))
+    ctx.check()
+    assert np.array_equal(out, large[:, :K]) and not large[:, K:].any()
+    ctx.release(a, e, c, cl)
+
+
 def test_tc_gemm_long_k_and_reproducible(ctx):
     """K = 16384 (longer than the 8192-token reduction of the weight gradients): accumulation error stays in bound."""
     M, N, K = 256, 512, 16384
