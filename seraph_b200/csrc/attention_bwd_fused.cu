@@ -33,8 +33,8 @@
 // and one thread stores them as two tiles of 128 keys x 32 queries (a store per warp cost the issuing lane 500 cycles a step: the
 // TMA unit takes few, large requests), each drain warp stages 32 rows x 32 columns of a chain at a time
 // (128-byte swizzle, conflict-free for row-per-lane writes) and adds it with a TMA reduction, and the log-sum-exp and the row
-// dot products D are read from copies transposed to [sequence][head][query] (at_bwd_prep2_kernel), 16 consecutive queries as
-// four 16-byte loads from one address for the whole warp.  A key block that reaches past its sequence's end keeps the
+// dot products D come from copies transposed to [sequence][head][query] (at_bwd_prep2_kernel): a bulk copy brings a step's 32 of each
+// beside its tiles, and a warp reads its 16 as four 16-byte loads from one address.  A key block that reaches past its sequence's end keeps the
 // per-thread reductions, so that no CTA ever adds (even a zero) into a row of the next sequence.
 //
 // Warps (16): 0 TMA producer, 1 MMA issuer (owns the tensor-memory allocation), 4-11 elementwise (a lane quarter and half of
