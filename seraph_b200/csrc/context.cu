@@ -103,8 +103,9 @@ cuda_train_context_t* cuda_train_init(int device_id) {
     p->parallel_block_size = 256; p->attention_block_size = 256; p->attention_num_warps = 8;
     if (cudaMalloc(&c->d_status, 4 * sizeof(int)) != cudaSuccess) { cudaStreamDestroy(s); free(c); return NULL; }
     cudaMemset(c->d_status, 0, 4 * sizeof(int));
-    cudaMalloc(&c->d_loss, 16 * sizeof(float));
+    if (cudaMalloc(&c->d_loss, (16 + SB_PEAK_WORDS) * sizeof(float)) != cudaSuccess) { cudaFree(c->d_status); cudaStreamDestroy(s); free(c); return NULL; }
     c->d_gnorm = c->d_loss + 8;
+    c->d_peaks = c->d_loss + 16;
     cudaMemset(c->d_loss, 0, 16 * sizeof(float));
     return p;
 }

@@ -1126,7 +1126,7 @@ static inline void tc_multi_split(sb_ctx_t* c, TcMulti& m) {
     m.keep = sb_parts_keep(c);
     if (m.unknown && tc_multi_small(c, m)) return;
     if (m.guesses && m.chunks <= TC_PEAKS_CHUNKS) {
-        if (!c->d_peaks && cudaMalloc((void**)&c->d_peaks, TC_SPANS * TC_MULTI * sizeof(float)) != cudaSuccess) { cudaGetLastError(); c->d_peaks = NULL; }      // then by the guess
+        static_assert(TC_SPANS * TC_MULTI <= SB_PEAK_WORDS, "a word for each span of each tensor");
         m.peaks = c->d_peaks;
         m.spans = max(1, min(TC_SPANS, 592 / m.n));
     }

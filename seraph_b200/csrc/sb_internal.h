@@ -18,6 +18,7 @@ extern "C" {
 #define SB_MAGIC 0x53423230u   /* "SB20" */
 #define SB_F16_KEPT 22          /* operand-part slots kept across the products of a keep region */
 #define SB_F16_SLOTS 24         /* plus one per operand for products outside a region */
+#define SB_PEAK_WORDS 6144
 
 /* status codes (seraph_b200_last_status) */
 enum {
@@ -64,7 +65,7 @@ typedef struct sb_ctx {
     int* d_status;                   /* device status word (bounds checks, bounded waits) */
     int gemm_mode;                   /* SB_GEMM_* (use_bf16 in pub overrides to BF16) */
     float* d_amax;                   /* FP16 split: max |x| of the operand held by each part slot, then two words of each for its preparation */
-    float* d_peaks;                  /* largest magnitudes of spans of tensors, between the two launches of a preparation */
+    float* d_peaks;                  /* [SB_PEAK_WORDS] largest magnitudes of spans of tensors, between the two launches of a preparation */
     struct { void* h; size_t cap; const float* ptr; size_t n; unsigned stamp; int valid; float* amax; } f16_slot[SB_F16_SLOTS];   /* FP16 parts of GEMM operands: all but the last two kept across
                                         calls inside a keep region (train_step.c marks runs of GEMMs that share operands), the last two for one call */
     int f16_keep; unsigned f16_clock;

@@ -1447,7 +1447,6 @@ void cuda_train_free(cuda_train_context_t* ctx) {
     if (c->h_seq_pin) cudaFreeHost(c->h_seq_pin);
     sb_parts_free(c); sb_colsum_free(c);
     if (c->d_amax) cudaFree(c->d_amax);
-    if (c->d_peaks) cudaFree(c->d_peaks);
     for (int i = 0; i < SB_F16_SLOTS; i++) if (c->f16_slot[i].h) cudaFree(c->f16_slot[i].h);
     if (c->d_status) cudaFree(c->d_status);
     if (c->d_loss) cudaFree(c->d_loss);

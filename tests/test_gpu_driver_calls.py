@@ -88,3 +88,17 @@ st.close()
 """).split()
     calls = [int(x) for x in out]
     assert calls[0] > 0 and calls[4:] == [0, 0, 0, 0], calls
+
+
+def test_a_smaller_product_than_the_last_allocates_nothing(run):
+    """Operands are prepared in one, two or three launches by their size; whichever way it is, a call that follows a larger one needs no more memory."""
+    out = run("""
+for M, K in ((8192, 1024), (4096, 512), (512, 256)):
+    a, b, c = ctx.zeros(M * K), ctx.zeros(K * K), ctx.zeros(M * K)
+    before = count("n_malloc")
+    ctx.lib.cuda_train_matmul_transpose(ctx.h, a.b, b.b, c.b, M, K, K, 0, 1, 0)
+    ctx.check()
+    print(count("n_malloc") - before)
+    ctx.release(a, b, c)
+""").split()
+    assert int(out[0]) > 0 and out[1:] == ["0", "0"], out
