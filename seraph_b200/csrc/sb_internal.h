@@ -364,7 +364,8 @@ static __device__ __forceinline__ float sb_amax4(float m, float4 v) {
 /* FP16 operand parts: an operand whose largest magnitude (or a bound of it) is `amax` is scaled by 2^s with amax 2^s in
    [2^14, 2^15) (s = 0 for an all-zero operand) and every scaled value x is stored as hi = fp16(x), lo = fp16(x - hi).  Both parts
    are floating point, so a bound that is loose by 2^k only moves the few values below 2^-(18-k) of the largest into fp16's
-   subnormal range; the bound must be a true upper bound, or hi overflows. */
+   subnormal range; the bound must be a true upper bound, or hi overflows.  (A tensor that is looked at whole may take a smaller word, the largest of
+   a sample, where FP16's room above 2^15 holds the rest: gemm_tc.cuh.) */
 static __device__ __forceinline__ int sb_f16_shift(float amax) {
     const int e = (int)((__float_as_uint(amax) >> 23) & 255u) - 127;
     if (amax == 0.f || e < -100) return 0;
